@@ -2,8 +2,9 @@
 //
 // Reference: cuvs::neighbors::refine (cpp/src/neighbors/refine/refine_device.cuh:30-138, C entry
 // c/src/neighbors/refine.cpp) -- there an IVF-Flat scan over a fake one-list-per-query index; here
-// one warp per query: the lanes split the dimensions of each candidate vector (coalesced row reads),
-// a shuffle tree sums the partial distances and the warp keeps the k best in its register top-k.
+// one to eight warps per query: groups of 1 to 32 lanes read a candidate's row with the widest loads its
+// alignment allows, a shuffle tree sums the partial distances and every warp keeps its k best in its
+// register top-k (merged through shared memory where a query has several warps).
 // Candidates equal to INT64_MAX (the search's "no such neighbour" marker) or outside the dataset
 // are ignored.  Results are sorted best first.
 //   L2Expanded / L2Unexpanded : sum (q - x)^2        L2Sqrt*: its square root
@@ -12,6 +13,8 @@
 #include "ivf_pq.hpp"
 #include "topk.cuh"
 
+#include <algorithm>
+
 namespace cuvs::neighbors {
 
 using namespace cuvs_b200;
@@ -19,93 +22,211 @@ using ivf_pq::elem_t;
 
 namespace {
 
-template <typename T>
-__device__ __forceinline__ float ld_as_float(const T* p, uint32_t i);
-template <> __device__ __forceinline__ float ld_as_float<float>(const float* p, uint32_t i) { return p[i]; }
-template <> __device__ __forceinline__ float ld_as_float<__half>(const __half* p, uint32_t i) { return __half2float(p[i]); }
-template <> __device__ __forceinline__ float ld_as_float<int8_t>(const int8_t* p, uint32_t i) { return float(p[i]); }
-template <> __device__ __forceinline__ float ld_as_float<uint8_t>(const uint8_t* p, uint32_t i) { return float(p[i]); }
-
 enum { REF_L2 = 0, REF_L2SQRT = 1, REF_IP = 2, REF_COS = 3 };
 
-template <typename T, int KPL>
-__global__ void refine_kernel(const T* __restrict__ dataset, int64_t n_rows, uint32_t dim,
-                              const T* __restrict__ queries, uint32_t n_queries,
-                              const int64_t* __restrict__ candidates, uint32_t n_cand, uint32_t k,
-                              int mode, int64_t* __restrict__ indices, float* __restrict__ distances)
+// How a row is read: 16-byte loads where every row starts on a 16-byte boundary, 4-byte loads where every
+// row starts on a 4-byte boundary, else (16- and 8-bit elements in odd row lengths) aligned 4-byte words
+// shifted into place.
+enum { ROW_VEC16 = 0, ROW_WORD = 1, ROW_SHIFT = 2 };
+
+template <typename T>
+__device__ __forceinline__ void word_to_floats(uint32_t w, float* f);
+template <> __device__ __forceinline__ void word_to_floats<float>(uint32_t w, float* f) { f[0] = __uint_as_float(w); }
+template <> __device__ __forceinline__ void word_to_floats<__half>(uint32_t w, float* f)
 {
-  extern __shared__ float s_query[];  // [warps per block][dim]
-  const uint32_t wib  = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const uint32_t q    = blockIdx.x * (blockDim.x >> 5) + wib;
-  if (q >= n_queries) { return; }
-  float* sq     = s_query + size_t(wib) * dim;
-  const T* qrow = queries + size_t(q) * dim;
-  float qn      = 0.0f;
-  for (uint32_t d = lane; d < dim; d += 32) {
-    const float v = ld_as_float<T>(qrow, d);
-    sq[d]         = v;
-    qn            = __fmaf_rn(v, v, qn);
-  }
+  const float2 v = __half22float2(*reinterpret_cast<const __half2*>(&w));
+  f[0]           = v.x;
+  f[1]           = v.y;
+}
+template <> __device__ __forceinline__ void word_to_floats<int8_t>(uint32_t w, float* f)
+{
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) { qn += __shfl_xor_sync(kFullMask, qn, o); }
-  __syncwarp();
+  for (int i = 0; i < 4; i++) { f[i] = float(int8_t((w >> (8 * i)) & 0xFFu)); }
+}
+template <> __device__ __forceinline__ void word_to_floats<uint8_t>(uint32_t w, float* f)
+{
+#pragma unroll
+  for (int i = 0; i < 4; i++) { f[i] = float((w >> (8 * i)) & 0xFFu); }
+}
+__device__ __forceinline__ float elem_to_float(float x) { return x; }
+__device__ __forceinline__ float elem_to_float(__half x) { return __half2float(x); }
+__device__ __forceinline__ float elem_to_float(int8_t x) { return float(x); }
+__device__ __forceinline__ float elem_to_float(uint8_t x) { return float(x); }
+
+// Step v of a row's words: four words (ROW_VEC16) or one.
+template <typename T, int ROW>
+__device__ __forceinline__ void load_step(const T* row, uint32_t v, uint32_t row_bytes, uint32_t* w)
+{
+  if constexpr (ROW == ROW_VEC16) {
+    const uint4 x = __ldg(reinterpret_cast<const uint4*>(row) + v);
+    w[0] = x.x;
+    w[1] = x.y;
+    w[2] = x.z;
+    w[3] = x.w;
+  } else if constexpr (ROW == ROW_WORD) {
+    w[0] = __ldg(reinterpret_cast<const uint32_t*>(row) + v);
+  } else {
+    // bytes [4v, 4v + 4) of a row that starts anywhere: the aligned word that holds the first of them and,
+    // if the row reaches into it, the next one
+    const uintptr_t a  = reinterpret_cast<uintptr_t>(row) + 4u * v;
+    const uint32_t mis = uint32_t(a & 3u);
+    const uint32_t* p  = reinterpret_cast<const uint32_t*>(a - mis);
+    const uint32_t lo  = __ldg(p);
+    const uint32_t hi  = mis != 0u && 4u * v + 4u - mis < row_bytes ? __ldg(p + 1) : 0u;
+    w[0]               = __funnelshift_r(lo, hi, 8u * mis);
+  }
+}
+
+// What bounds it: latency of rows of a few hundred bytes at random places, i.e. bytes in flight.  One warp
+// per query with element-wise loads moved 0.65 TB/s on 4,000 x 200 candidates of 768 halves (1.32 ms);
+// 16-byte loads, four rows per group of lanes in flight and several warps per query: 2.6 TB/s (0.33 ms).
+template <typename T, int KPL, int ROW>
+__global__ void __launch_bounds__(256, 4)
+refine_kernel(const T* __restrict__ dataset, int64_t n_rows, uint32_t dim,
+              const T* __restrict__ queries, uint32_t n_queries,
+              const int64_t* __restrict__ candidates, uint32_t n_cand, uint32_t k,
+              int mode, uint32_t log_lanes, uint32_t log_wpq, uint32_t q_floats,
+              int64_t* __restrict__ indices, float* __restrict__ distances)
+{
+  constexpr uint32_t kWords = ROW == ROW_VEC16 ? 4u : 1u;          // 4-byte words per load step
+  constexpr uint32_t kPerWord = 4u / uint32_t(sizeof(T));
+  constexpr uint32_t kElems = kWords * kPerWord;
+  constexpr int kRows       = 4;
+  // [queries per block][q_floats] queries, zero-padded to whole load steps, then the merge buffers
+  extern __shared__ __align__(16) float s_query[];
+  const uint32_t wib  = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const uint32_t wpq  = 1u << log_wpq;                               // warps per query
+  const uint32_t qib  = wib >> log_wpq, part = wib & (wpq - 1u);
+  const uint32_t qpb  = (blockDim.x >> 5) >> log_wpq;
+  const uint32_t q    = blockIdx.x * qpb + qib;
+  const bool active   = q < n_queries;
+  float* sq           = s_query + size_t(qib) * q_floats;
+  if (active) {
+    const T* qrow = queries + size_t(q) * dim;
+    for (uint32_t d = part * 32u + lane; d < q_floats; d += wpq * 32u) {
+      sq[d] = d < dim ? elem_to_float(qrow[d]) : 0.0f;
+    }
+  }
+  __syncthreads();
   warp_topk<KPL> queue;
   queue.init(int(k));
-  const int64_t* cand = candidates + size_t(q) * n_cand;
-  for (uint32_t c0 = 0; c0 < n_cand; c0 += 32) {
-    // every lane ends up with the score of candidate c0 + lane
-    float my_score = INFINITY;
-    bool my_valid  = false;
-    const uint32_t n_here = min(32u, n_cand - c0);
-    // four candidates at a time, so that their rows are in flight together (each candidate's own
-    // summation order is unchanged)
-    for (uint32_t j = 0; j < n_here; j += 4) {
-      const T* x[4];
-      bool ok[4];  // uniform across the warp
-      float acc[4] = {0.0f, 0.0f, 0.0f, 0.0f}, xn[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+  const int64_t* cand      = candidates + size_t(active ? q : 0u) * n_cand;
+  const uint32_t lanes     = 1u << log_lanes;                        // lanes that share a row
+  const uint32_t rows      = 32u >> log_lanes;                       // rows a warp reads at a time
+  const uint32_t group     = lane >> log_lanes, gl = lane & (lanes - 1u);
+  const uint32_t row_bytes = dim * uint32_t(sizeof(T));
+  const uint32_t n_steps   = (dim + kElems - 1u) / kElems;
+  if (active) {
+    float qn = 0.0f;
+    if (mode == REF_COS) {
+      for (uint32_t d = lane; d < dim; d += 32) { qn = __fmaf_rn(sq[d], sq[d], qn); }
 #pragma unroll
-      for (int u = 0; u < 4; u++) {
-        const int64_t id = j + u < n_here ? cand[c0 + j + u] : int64_t(-1);
-        ok[u]            = id >= 0 && id < n_rows;
-        x[u]             = dataset + size_t(ok[u] ? id : 0) * dim;
-      }
-      for (uint32_t d = lane; d < dim; d += 32) {
-        const float qv = sq[d];
+      for (int o = 16; o > 0; o >>= 1) { qn += __shfl_xor_sync(kFullMask, qn, o); }
+    }
+    for (uint32_t c0 = part * 32u; c0 < n_cand; c0 += wpq * 32u) {
+      const uint32_t n_here = min(32u, n_cand - c0);
+      int64_t my_id         = -1;
+      if (lane < n_here) { my_id = cand[c0 + lane]; }
+      if (my_id >= n_rows) { my_id = -1; }
+      float my_score = INFINITY;
+      // four rows per group of lanes at a time, so that their loads are in flight together
+      for (uint32_t j = 0; j < n_here; j += kRows * rows) {
+        const T* x[kRows];
+        bool ok[kRows];
+        float acc[kRows] = {}, xn[kRows] = {};
 #pragma unroll
-        for (int u = 0; u < 4; u++) {
-          if (!ok[u]) { continue; }
-          const float xv = ld_as_float<T>(x[u], d);
-          if (mode == REF_IP) {
-            acc[u] = __fmaf_rn(qv, xv, acc[u]);
-          } else if (mode == REF_COS) {
-            acc[u] = __fmaf_rn(qv, xv, acc[u]);
-            xn[u]  = __fmaf_rn(xv, xv, xn[u]);
+        for (int u = 0; u < kRows; u++) {
+          const uint32_t c = j + uint32_t(u) * rows + group;         // may pass 31: the shuffle wraps, ok[] masks
+          const int64_t id = int64_t(shfl_u64(uint64_t(my_id), int(c & 31u)));
+          ok[u]            = c < n_here && id >= 0;
+          x[u]             = dataset + size_t(ok[u] ? id : 0) * dim;
+        }
+#pragma unroll 3
+        for (uint32_t v = gl; v < n_steps; v += lanes) {
+          uint32_t w[kRows][kWords];
+#pragma unroll
+          for (int u = 0; u < kRows; u++) {
+            if (ok[u]) {
+              load_step<T, ROW>(x[u], v, row_bytes, w[u]);
+            } else {
+#pragma unroll
+              for (uint32_t i = 0; i < kWords; i++) { w[u][i] = 0u; }
+            }
+          }
+          float qv[kElems];
+          if constexpr (kElems % 4 == 0) {
+#pragma unroll
+            for (uint32_t e = 0; e < kElems; e += 4) {
+              const float4 t = *reinterpret_cast<const float4*>(sq + v * kElems + e);
+              qv[e] = t.x;
+              qv[e + 1] = t.y;
+              qv[e + 2] = t.z;
+              qv[e + 3] = t.w;
+            }
           } else {
-            const float t = qv - xv;
-            acc[u]        = __fmaf_rn(t, t, acc[u]);
+#pragma unroll
+            for (uint32_t e = 0; e < kElems; e++) { qv[e] = sq[v * kElems + e]; }
+          }
+#pragma unroll
+          for (int u = 0; u < kRows; u++) {
+            float xv[kElems];
+#pragma unroll
+            for (uint32_t i = 0; i < kWords; i++) { word_to_floats<T>(w[u][i], xv + i * kPerWord); }
+            if constexpr (ROW == ROW_SHIFT) {
+              // the last word of a row may carry bytes of the next one
+#pragma unroll
+              for (uint32_t e = 0; e < kElems; e++) {
+                if (v * kElems + e >= dim) { xv[e] = 0.0f; }
+              }
+            }
+            if (mode == REF_IP) {
+#pragma unroll
+              for (uint32_t e = 0; e < kElems; e++) { acc[u] = __fmaf_rn(qv[e], xv[e], acc[u]); }
+            } else if (mode == REF_COS) {
+#pragma unroll
+              for (uint32_t e = 0; e < kElems; e++) {
+                acc[u] = __fmaf_rn(qv[e], xv[e], acc[u]);
+                xn[u]  = __fmaf_rn(xv[e], xv[e], xn[u]);
+              }
+            } else {
+#pragma unroll
+              for (uint32_t e = 0; e < kElems; e++) {
+                const float t = qv[e] - xv[e];
+                acc[u]        = __fmaf_rn(t, t, acc[u]);
+              }
+            }
           }
         }
-      }
 #pragma unroll
-      for (int u = 0; u < 4; u++) {
-        if (!ok[u]) { continue; }
-        float a = acc[u], b = xn[u];
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-          a += __shfl_xor_sync(kFullMask, a, o);
-          b += __shfl_xor_sync(kFullMask, b, o);
-        }
-        float score = a;                       // smaller is better
-        if (mode == REF_IP) { score = -a; }
-        if (mode == REF_COS) { score = 1.0f - a / (sqrtf(qn) * sqrtf(b) + 1e-30f); }
-        if (lane == j + uint32_t(u)) {
-          my_score = score;
-          my_valid = true;
+        for (int u = 0; u < kRows; u++) {
+          float a = acc[u], b = xn[u];
+          for (uint32_t o = lanes >> 1; o > 0; o >>= 1) {
+            a += __shfl_xor_sync(kFullMask, a, int(o));
+            if (mode == REF_COS) { b += __shfl_xor_sync(kFullMask, b, int(o)); }
+          }
+          float score = a;                       // smaller is better
+          if (mode == REF_IP) { score = -a; }
+          if (mode == REF_COS) { score = 1.0f - a / (sqrtf(qn) * sqrtf(b) + 1e-30f); }
+          // candidate j + u * rows + g was summed by group g: hand it to the lane of that number
+          const uint32_t first = j + uint32_t(u) * rows;
+          const float mine     = __shfl_sync(kFullMask, score, int(((lane - first) & (rows - 1u)) << log_lanes));
+          if (lane >= first && lane < first + rows) { my_score = mine; }
         }
       }
+      queue.offer(make_key(my_score, c0 + lane), my_id >= 0);
     }
-    queue.offer(make_key(my_score, c0 + lane), my_valid);
   }
+  if (wpq > 1u) {
+    uint64_t* s_merge = reinterpret_cast<uint64_t*>(s_query + size_t(qpb) * q_floats) + size_t(qib) * wpq * k;
+    if (part != 0u) { queue.store(s_merge + size_t(part) * k, int(k)); }
+    __syncthreads();
+    if (part != 0u) { return; }
+    for (uint32_t t0 = k; t0 < wpq * k; t0 += 32) {
+      const uint32_t t = t0 + lane;
+      queue.offer(t < wpq * k ? s_merge[t] : kEmptyKey, t < wpq * k);
+    }
+  }
+  if (!active) { return; }
 #pragma unroll
   for (int r = 0; r < KPL; r++) {
     const uint32_t pos = uint32_t(r) * 32u + lane;
@@ -124,29 +245,62 @@ __global__ void refine_kernel(const T* __restrict__ dataset, int64_t n_rows, uin
   }
 }
 
+template <typename T, int ROW>
+void launch_refine_rows(raft::resources& res, const T* dataset, int64_t n_rows, uint32_t dim,
+                        const T* queries, uint32_t n_queries, const int64_t* candidates, uint32_t n_cand,
+                        uint32_t k, int mode, int64_t* indices, float* distances)
+{
+  constexpr uint32_t kElems = (ROW == ROW_VEC16 ? 16u : 4u) / uint32_t(sizeof(T));
+  const uint32_t n_steps    = ceildiv(dim, kElems);
+  // Lanes per row: as few as still leave a lane at most eight loads of the row, so that a warp reads
+  // several rows at a time (a 128-byte row: one lane, 32 rows; 768 halves: 16 lanes, 2 rows: 332 us against
+  // 355 us with the whole warp on a row).
+  uint32_t log_lanes = 0;
+  while (log_lanes < 5 && (8u << log_lanes) < n_steps) { log_lanes++; }
+  // Warps per query: enough for 64 per SM (24 and 200: 15-25% slower), at most one per 32 candidates.
+  uint32_t log_wpq = 0;
+  while (log_wpq < 3 && (size_t(n_queries) << log_wpq) < size_t(res.sm_count) * 64 && (32u << log_wpq) < n_cand) {
+    log_wpq++;
+  }
+  const uint32_t warps    = std::max(4u, 1u << log_wpq);
+  const uint32_t qpb      = warps >> log_wpq;
+  const uint32_t q_floats = round_up(n_steps * kElems, 4u);
+  size_t smem             = size_t(qpb) * q_floats * 4 + (log_wpq > 0 ? size_t(warps) * k * 8 : 0);
+  auto go = [&](auto kernel) {
+    if (smem > 48 * 1024) {
+      CUVS_EXPECTS(smem <= size_t(res.smem_optin) - 1024, "refine: dim = %u is too large", dim);
+      ensure_dynamic_smem(reinterpret_cast<const void*>(kernel), smem);
+    }
+    kernel<<<ceildiv(n_queries, qpb), warps * 32, smem, res.stream>>>(
+      dataset, n_rows, dim, queries, n_queries, candidates, n_cand, k, mode, log_lanes, log_wpq, q_floats, indices,
+      distances);
+    CUDA_TRY(cudaGetLastError());
+  };
+  if (k <= 32) {
+    go(refine_kernel<T, 1, ROW>);
+  } else if (k <= 64) {
+    go(refine_kernel<T, 2, ROW>);
+  } else {
+    go(refine_kernel<T, 4, ROW>);
+  }
+  res.launches++;
+}
+
 template <typename T>
 void launch_refine(raft::resources& res, const void* dataset, int64_t n_rows, uint32_t dim,
                    const void* queries, uint32_t n_queries, const int64_t* candidates, uint32_t n_cand,
                    uint32_t k, int mode, int64_t* indices, float* distances)
 {
-  const int warps   = 4;
-  const size_t smem = size_t(warps) * dim * 4;
-  CUVS_EXPECTS(smem <= 48 * 1024, "refine: dim = %u is too large", dim);
-  const int blocks = int(ceildiv<uint32_t>(n_queries, warps));
-  const T* ds      = static_cast<const T*>(dataset);
-  const T* qs      = static_cast<const T*>(queries);
-  if (k <= 32) {
-    refine_kernel<T, 1><<<blocks, warps * 32, smem, res.stream>>>(ds, n_rows, dim, qs, n_queries, candidates,
-                                                                  n_cand, k, mode, indices, distances);
-  } else if (k <= 64) {
-    refine_kernel<T, 2><<<blocks, warps * 32, smem, res.stream>>>(ds, n_rows, dim, qs, n_queries, candidates,
-                                                                  n_cand, k, mode, indices, distances);
-  } else {
-    refine_kernel<T, 4><<<blocks, warps * 32, smem, res.stream>>>(ds, n_rows, dim, qs, n_queries, candidates,
-                                                                  n_cand, k, mode, indices, distances);
+  const T* ds          = static_cast<const T*>(dataset);
+  const T* qs          = static_cast<const T*>(queries);
+  const uintptr_t bits = reinterpret_cast<uintptr_t>(dataset) | (size_t(dim) * sizeof(T));
+  if ((bits & 15u) == 0) {
+    launch_refine_rows<T, ROW_VEC16>(res, ds, n_rows, dim, qs, n_queries, candidates, n_cand, k, mode, indices, distances);
+  } else if (sizeof(T) == 4 || (bits & 3u) == 0) {
+    launch_refine_rows<T, ROW_WORD>(res, ds, n_rows, dim, qs, n_queries, candidates, n_cand, k, mode, indices, distances);
+  } else if constexpr (sizeof(T) < 4) {
+    launch_refine_rows<T, ROW_SHIFT>(res, ds, n_rows, dim, qs, n_queries, candidates, n_cand, k, mode, indices, distances);
   }
-  CUDA_TRY(cudaGetLastError());
-  res.launches++;
 }
 
 }  // namespace
