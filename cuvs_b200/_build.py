@@ -26,6 +26,7 @@ UNITS = [("resources.cu", "resources.o", []), ("index.cu", "index.o", []),
          ("coarse.cu", "coarse.o", []), ("coarse_tc.cu", "coarse_tc.o", []), ("search.cu", "search.o", []),
          ("build.cu", "build.o", []), ("c_api.cu", "c_api.o", []),
          ("no_alloc.cu", "no_alloc.o", []), ("refine.cu", "refine.o", []),
+         ("filter_scan.cu", "filter_scan.o", []), ("rescore.cu", "rescore.o", []),
          ("dynamic_batching.cu", "dynamic_batching.o", []), ("mg.cu", "mg.o", []),
          ("c_api_mg.cu", "c_api_mg.o", [])]
 UNITS += [("scan_inst.cu", f"scan_{b}.o", [f"-DPQ_BITS={b}"]) for b in (4, 5, 6, 7, 8)]

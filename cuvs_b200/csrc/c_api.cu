@@ -762,7 +762,7 @@ extern "C" cuvsError_t cuvsB200SetCoarseWaitTest(uint32_t spin_limit, uint32_t s
 extern "C" cuvsError_t cuvsB200SetScanCodebookHome(int home)
 {
   return translate_exceptions([=] {
-    CUVS_EXPECTS(home >= 0 && home <= 3, "home must be 0, 1, 2 or 3");
+    CUVS_EXPECTS(home >= 0 && home <= 4, "home must be 0, 1, 2, 3 or 4");
     ivf_pq::set_scan_codebook_home(home);
   });
 }

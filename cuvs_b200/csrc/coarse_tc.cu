@@ -34,6 +34,7 @@
 //      fails is queued.
 //   4. coarse_fallback_kernel: queued queries (rare) are redone exactly over all lists.
 #include "search_internal.hpp"
+#include "tc_ptx.cuh"
 #include "topk.cuh"
 
 #include <cuda.h>
@@ -68,9 +69,6 @@ constexpr int kEpiWarps = 16;
 constexpr int kThreads  = (2 + kEpiWarps) * 32;  // warp 0 TMA, warp 1 MMA, warps 2..17 epilogue
 constexpr uint32_t kStageBytes = (2 * kBM + 2 * kBN) * kBK * 4;  // 48 KB
 constexpr uint32_t kSmemBytes  = kStages * kStageBytes + 1024 /*align*/ + 256 /*barriers*/;
-constexpr uint32_t kSpinLimit  = 1u << 21;  // bounded waits (each try_wait sleeps up to ~1 us)
-
-enum { ERR_NONE = 0, ERR_TIMEOUT = 1 };
 
 
 // ------------------------------------------------------------------------------------------------
@@ -153,66 +151,6 @@ __global__ void max_row_sumsq_scaled_kernel(const float* __restrict__ rows, uint
   if (lane == 0) { atomicMax(out_bits, __float_as_uint(ss)); }
 }
 
-// ------------------------------------------------------------------------------------------------
-// PTX wrappers
-// ------------------------------------------------------------------------------------------------
-__device__ __forceinline__ uint32_t smem_u32(const void* p)
-{
-  return uint32_t(__cvta_generic_to_shared(p));
-}
-__device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count)
-{
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count));
-}
-__device__ __forceinline__ void mbar_arrive(uint32_t bar)
-{
-  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
-}
-__device__ __forceinline__ void mbar_arrive_expect_tx(uint32_t bar, uint32_t bytes)
-{
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
-}
-// Bounded wait: false on time-out.
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, uint32_t limit)
-{
-  for (uint32_t it = 0; it < limit; it++) {
-    uint32_t done;
-    asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, 1000;\n\t"
-      "selp.u32 %0, 1, 0, p;\n\t}"
-      : "=r"(done)
-      : "r"(bar), "r"(parity)
-      : "memory");
-    if (done) { return true; }
-  }
-  return false;
-}
-__device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, uint32_t bar, int x,
-                                            int y)
-{
-  asm volatile(
-    "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
-    ::"r"(dst), "l"(map), "r"(bar), "r"(x), "r"(y)
-    : "memory");
-}
-__device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void tc_commit(uint32_t bar)
-{
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar)
-               : "memory");
-}
-__device__ __forceinline__ void tc_mma_tf32(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b,
-                                            uint32_t idesc, uint32_t accumulate)
-{
-  asm volatile(
-    "{\n\t.reg .pred p;\n\t"
-    "setp.ne.b32 p, %4, 0;\n\t"
-    "tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, p;\n\t}"
-    ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
-    : "memory");
-}
 // Shared-memory matrix descriptor of a K-major tile stored as rows of 64 bytes with the 64-byte
 // swizzle: 8-row groups 512 bytes apart.
 __device__ __forceinline__ uint64_t make_desc(uint32_t saddr)
@@ -226,22 +164,6 @@ __device__ __forceinline__ uint64_t make_desc(uint32_t saddr)
   return d;
 }
 static_assert(kBK * 4 == 64, "descriptor and tensor maps are written for 64-byte rows");
-__device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32])
-{
-  asm volatile(
-    "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
-    "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
-    "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
-    : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-      "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]),
-      "=r"(r[15]), "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]),
-      "=r"(r[22]), "=r"(r[23]), "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]),
-      "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
-    : "r"(taddr)
-    : "memory");
-  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-}
-
 // ------------------------------------------------------------------------------------------------
 // the GEMM + candidate kernel
 // ------------------------------------------------------------------------------------------------
@@ -807,41 +729,6 @@ constexpr uint32_t kFinMaxHalfTiles = 512;
 constexpr uint32_t kFinMaxC         = 64;
 constexpr uint32_t kFinRows         = 64;  // most rows rescored per round (all selected lists at once)
 
-// 64 values per warp, value e = r * 32 + lane in register a<r>: full bitonic sort.
-template <typename T, bool Desc>
-__device__ __forceinline__ void warp_sort64(T& a0, T& a1)
-{
-  const uint32_t lane = threadIdx.x & 31u;
-  auto shfl = [](T v, int j) {
-    if constexpr (sizeof(T) == 8) {
-      const uint32_t lo = __shfl_xor_sync(kFullMask, uint32_t(v), j);
-      const uint32_t hi = __shfl_xor_sync(kFullMask, uint32_t(uint64_t(v) >> 32), j);
-      return T((uint64_t(hi) << 32) | lo);
-    } else {
-      return T(__shfl_xor_sync(kFullMask, v, j));
-    }
-  };
-#pragma unroll
-  for (uint32_t k = 2; k <= 64; k <<= 1) {
-#pragma unroll
-    for (uint32_t j = k >> 1; j > 0; j >>= 1) {
-      if (j == 32) {  // k == 64: partner is the other register of the same lane, ascending block
-        const T lo = a0 < a1 ? a0 : a1, hi = a0 < a1 ? a1 : a0;
-        a0 = Desc ? hi : lo;
-        a1 = Desc ? lo : hi;
-      } else {
-        const T o0 = shfl(a0, int(j)), o1 = shfl(a1, int(j));
-        // value index e = r * 32 + lane; block direction from bit k of e (k == 64: one block)
-        const bool up0 = ((lane & k) == 0) || k >= 32;         // r = 0: bit 5 of e is 0
-        const bool up1 = k == 64 || (k < 32 && (lane & k) == 0);  // r = 1: bit 5 of e is 1
-        const bool low = (lane & j) == 0;
-        const bool min0 = (low == up0) != Desc, min1 = (low == up1) != Desc;
-        a0 = min0 ? (a0 < o0 ? a0 : o0) : (a0 < o0 ? o0 : a0);
-        a1 = min1 ? (a1 < o1 ? a1 : o1) : (a1 < o1 ? o1 : a1);
-      }
-    }
-  }
-}
 // (a0, a1) sorted descending, `other` = 64 values sorted descending in shared memory: afterwards
 // (a0, a1) = the 64 largest of the union, sorted descending.
 __device__ __forceinline__ void warp_merge_top64_desc(uint32_t& a0, uint32_t& a1, const uint32_t* other)
@@ -1233,41 +1120,10 @@ coarse_fallback_kernel(const uint32_t* __restrict__ redo_list, const uint32_t* _
 // ------------------------------------------------------------------------------------------------
 // host side
 // ------------------------------------------------------------------------------------------------
-using encode_fn_t = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
-                                 const cuuint64_t*, const cuuint32_t*, const cuuint32_t*,
-                                 CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion,
-                                 CUtensorMapFloatOOBfill);
-
-encode_fn_t get_encode_fn()
-{
-  static encode_fn_t fn = nullptr;
-  static std::once_flag once;
-  std::call_once(once, [] {
-    void* p = nullptr;
-    cudaDriverEntryPointQueryResult qres;
-    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &qres) == cudaSuccess &&
-        qres == cudaDriverEntryPointSuccess) {
-      fn = reinterpret_cast<encode_fn_t>(p);
-    }
-  });
-  CUVS_EXPECTS(fn != nullptr, "cuTensorMapEncodeTiled is not available in this driver");
-  return fn;
-}
-
 // 2-D fp32 row-major [rows, cols] tensor, box [box_rows, kBK columns], 64-byte swizzle, zero fill.
 CUtensorMap make_map(const float* ptr, uint64_t rows, uint64_t cols, uint32_t box_rows)
 {
-  CUtensorMap m;
-  const cuuint64_t dims[2]    = {cols, rows};
-  const cuuint64_t strides[1] = {cols * 4};
-  const cuuint32_t box[2]     = {kBK, box_rows};
-  const cuuint32_t elem[2]    = {1, 1};
-  CUresult r = get_encode_fn()(&m, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<float*>(ptr), dims,
-                               strides, box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                               CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  CUVS_EXPECTS(r == CUDA_SUCCESS, "cuTensorMapEncodeTiled failed with code %d", int(r));
-  return m;
+  return make_map_2d(CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, ptr, rows, cols, box_rows, kBK, CU_TENSOR_MAP_SWIZZLE_64B);
 }
 
 uint32_t margin_for(uint32_t n_probes) { return std::max<uint32_t>(16, n_probes / 4); }
@@ -1295,6 +1151,31 @@ tc_fault& tc_fault_ref()
 }
 
 }  // namespace
+
+CUtensorMap make_map_2d(CUtensorMapDataType type, uint32_t elem_bytes, const void* ptr, uint64_t rows, uint64_t cols,
+                        uint32_t box_rows, uint32_t box_cols, CUtensorMapSwizzle swizzle)
+{
+  using encode_fn_t = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
+                                   const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
+                                   CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+  static const encode_fn_t fn = [] {
+    void* p = nullptr;
+    cudaDriverEntryPointQueryResult qres;
+    const bool found = cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &qres) == cudaSuccess &&
+                       qres == cudaDriverEntryPointSuccess;
+    return found ? reinterpret_cast<encode_fn_t>(p) : nullptr;
+  }();
+  CUVS_EXPECTS(fn != nullptr, "cuTensorMapEncodeTiled is not available in this driver");
+  CUtensorMap m;
+  const cuuint64_t dims[2]    = {cols, rows};
+  const cuuint64_t strides[1] = {cols * elem_bytes};
+  const cuuint32_t box[2]     = {box_cols, box_rows};
+  const cuuint32_t elem[2]    = {1, 1};
+  CUresult r = fn(&m, type, 2, const_cast<void*>(ptr), dims, strides, box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle,
+                  CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  CUVS_EXPECTS(r == CUDA_SUCCESS, "cuTensorMapEncodeTiled failed with code %d", int(r));
+  return m;
+}
 
 void set_coarse_tc_products(int products) { tc_products_ref() = products; }
 void set_coarse_tc_resident(bool on) { tc_resident_ref() = on; }

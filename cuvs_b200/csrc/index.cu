@@ -9,6 +9,7 @@
 // codes u8 [ceil(size/32), n_pieces, 32, 16] and ids i64 [size].
 // The reader accepts any well-formed v1.0/2.0 header and checks element size and element count
 // of every record against what the format calls for.
+#include "filter_scan.hpp"
 #include "ivf_pq.hpp"
 #include "search_internal.hpp"
 
@@ -222,6 +223,25 @@ void index<int64_t>::recompute_internal_state(cudaStream_t stream)
   const bool norm_column = metric_ == DistanceType::L2Expanded || metric_ == DistanceType::L2SqrtExpanded;
   prepare_tc_centers(stream, centers_.data(), n_lists_, dim_ext(), norm_column ? dim_ : dim_ext(),
                      centers_hi_.data(), centers_lo_.data(), &centers_max_norm_, &centers_ext_scale_);
+  // codebooks in half precision for the fine search's tensor-core pass
+  if (codebook_kind_ == codebook_gen::PER_SUBSPACE) {
+    const uint32_t len = pq_len();
+    filter_.len_pad    = len <= 2 ? len : (len <= 4 ? 4u : round_up(len, 8u));
+    const size_t n     = round_up<size_t>(size_t(pq_dim_) * pq_book_size() * filter_.len_pad, 8);
+    if (filter_.book.size() != n) {
+      filter_.book.resize(n);
+      CUDA_TRY(cudaMemsetAsync(filter_.book.data(), 0, n * sizeof(__half), stream));
+    }
+    dev_array<float> tmp(size_t(pq_dim_) * 2 + 3);
+    make_filter_book(pq_centers_.data(), pq_dim_, len, filter_.len_pad, pq_book_size(), filter_.book.data(), tmp.data(),
+                     tmp.data() + 3, stream);
+    float h[3];
+    CUDA_TRY(cudaMemcpyAsync(h, tmp.data(), 12, cudaMemcpyDeviceToHost, stream));
+    CUDA_TRY(cudaStreamSynchronize(stream));
+    filter_.rmax     = std::sqrt(h[0]);
+    filter_.comp_max = h[1];
+    filter_.scale    = h[2];
+  }
 }
 
 // ------------------------------------------------------------------------------------------------

@@ -10,9 +10,11 @@
 //   scan_kernel ............... compute_similarity (scan.cuh)
 //   final_merge_kernel ........ cross-probe select_k (:646-655) + postprocess_distances
 //                               (ivf_common.cuh:175-252) + postprocess_neighbors (:112-169), fused
+#include "filter_scan.hpp"
 #include "ivf_pq.hpp"
 #include "scan.cuh"
 #include "search_internal.hpp"
+#include "tc_ptx.cuh"
 #include "topk.cuh"
 
 #include <algorithm>
@@ -274,12 +276,15 @@ __global__ void copy_u32_kernel(uint32_t* __restrict__ dst, const uint32_t* __re
 
 // Counters for the benchmark: sum over pairs, and over distinct probed lists, of ceil(size / 32).
 __global__ void scan_stats_kernel(const uint32_t* __restrict__ list_count,
-                                  const uint32_t* __restrict__ list_sizes, uint32_t n_lists,
+                                  const uint32_t* __restrict__ list_sizes, uint32_t n_lists, uint32_t n_segments,
                                   unsigned long long* __restrict__ stats)
 {
   const uint32_t l = blockIdx.x * blockDim.x + threadIdx.x;
   unsigned long long a = 0, b = 0;
-  const uint32_t cnt = l < n_lists ? list_count[l] + list_count[n_lists + l] : 0u;  // both segments
+  uint32_t cnt = 0;
+  if (l < n_lists) {
+    for (uint32_t i = 0; i < n_segments; i++) { cnt += list_count[size_t(i) * n_lists + l]; }
+  }
   if (cnt > 0) {
     const unsigned long long g = (list_sizes[l] + 31u) >> 5;
     a = g * cnt;
@@ -383,19 +388,6 @@ __global__ void fill_u32_kernel(uint32_t* p, size_t n, uint32_t v)
 // ------------------------------------------------------------------------------------------------
 // final selection across probes + post-processing
 // ------------------------------------------------------------------------------------------------
-__device__ __forceinline__ float postprocess_distance(float score, int metric, float scale)
-{
-  switch (metric) {
-    case 0: return scale != 1.0f ? __fmul_rn(score, __fmul_rn(scale, scale)) : score;
-    case 1: return scale != 1.0f ? __fmul_rn(__fsqrt_rn(score), scale) : __fsqrt_rn(score);
-    case 6: return __fmul_rn(score, __fmul_rn(__fmul_rn(-1.0f, scale), scale));
-    default: {
-      const float f = __fmul_rn(scale, scale);
-      return f != 1.0f ? __fmul_rn(score, f) : score;
-    }
-  }
-}
-
 // One warp per query: k smallest of the n_probes * k keys, then id translation
 // (binary search of the sample index in chunk_index, as find_chunk_ix does) and distance scaling.
 template <int KPL>
@@ -599,7 +591,8 @@ int& scan_codebook_home()
 {
   // 0 = choose, 1 = never tensor memory (shared or global memory instead), 2 = choose, but never an
   // instantiation made for one exact shape (tests compare it with the general kernel), 3 = behave as
-  // if no look-up table fitted shared memory (the variant with the table in global memory)
+  // if no look-up table fitted shared memory (the variant with the table in global memory), 4 = the two-step
+  // path (filter_scan.hpp) wherever it applies, whatever the size of the batch
   static int home = 0;
   return home;
 }
@@ -723,6 +716,45 @@ void check_search_params(const raft::resources& res, const search_params& params
   (void)plan_scan(res, idx, lut_kind, !is_l2, k > 128 ? 1 : k);  // throws when no plan exists
 }
 
+// Error model of the bounds (see rescore.cu for what each term stands for).
+static void set_error_model(rescore_params& rp, const operand_params& fp, int lut_kind, bool out_half, float rmax)
+{
+  const double half = std::ldexp(1.0, -11), ulp = std::ldexp(1.0, -24), tiny = std::ldexp(1.0, -25);
+  const double K    = double(fp.k_chunks) * 8.0;
+  rp.rmax  = rmax * 1.00001f;
+  rp.kappa = float((K + 32.0) * std::ldexp(1.0, -22) * 1.1);
+  rp.e1    = float(half * 1.03);
+  rp.e0    = float(2.0 * std::sqrt(K) * tiny / double(fp.scale));
+  // table entries: their fp32 chain, then one rounding to the table type
+  double up   = (double(fp.pq_len) + 4.0) * ulp, down = up;
+  double zero = 0.0;  // absolute error of an entry near zero
+  if (lut_kind == LUT_F16) {
+    up += half;
+    down += half;
+    zero = tiny;
+  } else if (lut_kind == LUT_FP8) {
+    up += 0.0626;     // three mantissa bits, read back at the middle of their interval
+    down += 0.0556;
+    zero = std::ldexp(1.0, -15) * 1.07;
+  }
+  // sums in the internal type
+  const double unit = out_half ? half : ulp;
+  const double sum  = std::expm1(double(fp.pq_dim + 2) * std::log1p(unit)) * 1.02;
+  rp.delta_hi = float((1.0 + up) * (1.0 + sum) - 1.0) * 1.0001f;
+  rp.delta_lo = float(1.0 - (1.0 - down) * (1.0 - sum)) * 1.0001f;
+  rp.eta      = float(double(fp.pq_dim) * (zero + (out_half ? 2.0 * tiny : 0.0)) * 1.2);
+  rp.sum_limit = out_half ? 6.0e4f : INFINITY;
+  rp.sharpen   = lut_kind == LUT_FP8 || out_half;
+  rp.saturates = lut_kind == LUT_FP8;
+  // inner product: every term is bounded by |q| (|c| + rmax)
+  rp.ip_gemm = float(2.0 * half * 1.03 + double(rp.kappa) + K * ulp);
+  rp.ip_lut  = float((3.0 * fp.rot_dim + double(fp.pq_dim) + 8.0) * ulp + (lut_kind == LUT_F16 ? half * 1.01 : 0.0));
+  if (fp.is_ip) {
+    rp.sum_limit = lut_kind == LUT_F16 ? 6.0e4f : INFINITY;
+    if (rp.cosine) { rp.eta += 5.0e-7f; }
+  }
+}
+
 void search_any(raft::resources& res, const search_params& params, const index<int64_t>& idx,
                 const void* queries, elem_t qtype, uint32_t n_queries, uint32_t k,
                 int64_t* neighbors, float* distances, const uint32_t* given_probes, bitset_view filter)
@@ -765,7 +797,19 @@ void search_any(raft::resources& res, const search_params& params, const index<i
   // worst-case samples per query: the n_probes largest lists (ivf_pq_search.cuh:934-940)
   const uint32_t max_samples =
     round_up<uint32_t>(std::max<uint32_t>(uint32_t(idx.accum_sorted_sizes()[n_probes]), k), 128);
-  if (store_all) {
+  // the two-step path (filter_scan.hpp) where it applies; a test override of the table's home asks for the
+  // look-up-table kernels
+  filter_plan fplan{};
+  const uint32_t max_groups = uint32_t(ceildiv<uint64_t>(uint64_t(idx.accum_sorted_sizes()[n_probes]) + 31ull * n_probes, 32));
+  // (below some 4,000 pairs, and for k > 128, the look-up-table scan is as fast or faster: 162 against 178 us for 100
+  // queries of 20 probes, 632 against 754 us for 500 queries with k = 1000)
+  const int home = scan_codebook_home();
+  if (home == 4 || (home == 0 && uint64_t(batch) * n_probes > 4096 && k <= 128)) {
+    // bounds of one internal batch: within 2 GiB
+    batch = uint32_t(std::max<uint64_t>(1, std::min<uint64_t>(batch, (1ull << 31) / (uint64_t(max_groups) * 16))));
+    fplan = plan_filter(res, idx, lut_kind, out_half, is_ip, k, n_probes, batch);
+  }
+  if (store_all && !fplan.use) {
     // keep the score matrix of one internal batch within 1 GiB
     const uint64_t cap_q = std::max<uint64_t>(1, (1ull << 30) / (uint64_t(max_samples) * 4));
     batch                = uint32_t(std::min<uint64_t>(batch, cap_q));
@@ -785,12 +829,24 @@ void search_any(raft::resources& res, const search_params& params, const index<i
   const size_t o_rq      = lay.add(size_t(batch) * idx.rot_dim() * 4);
   const size_t o_probes  = lay.add(n_pairs_max * 4);
   const size_t o_chunk   = lay.add(n_pairs_max * 4);
-  const size_t o_order   = lay.add(n_pairs_max * 32);
+  const bool f_use       = fplan.use;
+  const bool f_small     = n_pairs_max <= 4096 && !res.stats_enabled;  // every pair its own tile, nothing ordered by list
+  const size_t n_tiles   = f_use ? size_t(max_filter_tiles(idx, n_pairs_max, f_small)) : 0;
+  const size_t o_groups  = lay.add(f_use ? n_pairs_max * 4 : 0);
+  const size_t o_rec     = lay.add(f_use ? n_pairs_max * 16 : 0);
+  const size_t o_norm    = lay.add(f_use ? n_pairs_max * 4 : 0);
+  const size_t o_tiles   = lay.add(n_tiles * sizeof(filter_tile));
+  const size_t o_units   = lay.add(f_use ? size_t(batch) * max_groups * 16 : 0);
+  const size_t o_qscale  = lay.add(f_use && is_ip ? size_t(batch) * 4 : 0);
+  const uint32_t f_data  = f_use ? ceildiv(idx.pq_dim() * idx.filter_model().len_pad, 8u) : 0;
+  const uint32_t f_chunks = round_up(f_data + 1u, 2u);  // 16-byte chunks of an operand row
+  const size_t o_operand = lay.add(f_use ? n_pairs_max * f_chunks * 16 : 0);
+  const size_t o_order   = lay.add(f_use ? 0 : n_pairs_max * 32);
   const size_t o_count   = lay.add((size_t(n_lists) * 2 + 1) * 4);  // two segments of buckets, one per list each
   const size_t o_kth     = lay.add(size_t(batch) * 4);
   const size_t o_counter = lay.add(256);
-  const size_t o_keys    = lay.add(store_all ? size_t(batch) * k * 8 : n_pairs_max * k * 8);
-  const size_t o_all     = lay.add(store_all ? size_t(batch) * max_samples * 4 : 0);
+  const size_t o_keys    = lay.add(f_use ? 0 : (store_all ? size_t(batch) * k * 8 : n_pairs_max * k * 8));
+  const size_t o_all     = lay.add(store_all && !f_use ? size_t(batch) * max_samples * 4 : 0);
   // half-precision scores tie in large groups, which the tensor-core path's guard (made for fp32
   // scores) does not settle: the fp16 coarse search runs on the exact SIMT path
   const bool use_tc = !coarse_h && coarse_mode() != 1 && coarse_tc_usable(n_lists, n_probes, cdim_ext);
@@ -801,7 +857,7 @@ void search_any(raft::resources& res, const search_params& params, const index<i
   const size_t o_coarse  = lay.add(coarse_ws);
   // tables in global memory: one per CTA of the (smaller) grid of that variant
   const uint32_t glut_grid = uint32_t(std::min<size_t>(n_pairs_max, size_t(res.sm_count) * 4));
-  const size_t o_glut      = lay.add(plan.lut_global ? size_t(glut_grid) * plan.lut_bytes : 0);
+  const size_t o_glut      = lay.add(plan.lut_global && !f_use ? size_t(glut_grid) * plan.lut_bytes : 0);
   res.ws.reserve(lay.total());
   char* ws = res.ws.base();
   auto* d_fq      = reinterpret_cast<float*>(ws + o_fq);
@@ -864,6 +920,134 @@ void search_any(raft::resources& res, const search_params& params, const index<i
     nvtx_range worker_scope("ivf_pq::search-worker(n_queries = %u, n_probes = %u, k = %u, dim = %zu)", nq, n_probes,
                             k, size_t(idx.dim()));
     if (stats) { res.stats_mark(ev, 2); }
+    if (f_use) {
+      auto* d_groups = reinterpret_cast<uint32_t*>(ws + o_groups);
+      auto* d_rec     = reinterpret_cast<float4*>(ws + o_rec);
+      auto* d_norm    = reinterpret_cast<float*>(ws + o_norm);
+      auto* d_tiles   = reinterpret_cast<filter_tile*>(ws + o_tiles);
+      auto* d_units   = reinterpret_cast<float4*>(ws + o_units);
+      auto* d_qscale  = reinterpret_cast<float*>(ws + o_qscale);
+      auto* d_operand = reinterpret_cast<__half*>(ws + o_operand);
+      // 3. tiles, and the query operand of every pair, ordered by list; d_counter: pairs, tiles, error word
+      CUDA_TRY(cudaMemsetAsync(d_counter, 0, 16, stream));
+      if (f_small) {
+        launch_tiles_small(d_probes, idx.list_sizes(), idx.row_offsets(), n_lists, nq, n_probes, d_chunk, d_groups, d_tiles,
+                           d_counter, stream);
+        res.launches++;
+      } else {
+        CUDA_TRY(cudaMemsetAsync(d_count, 0, size_t(n_lists) * 4, stream));
+        launch_count_pairs(d_probes, idx.list_sizes(), n_lists, nq, n_probes, d_chunk, d_groups, d_count, stream);
+        if (stats) {
+          scan_stats_kernel<<<ceildiv<uint32_t>(n_lists, 256), 256, 0, stream>>>(d_count, idx.list_sizes(), n_lists, 1,
+                                                                                 res.d_stats);
+          res.stat_pairs += n_pairs;
+        }
+        launch_tiles(idx.list_sizes(), idx.row_offsets(), n_lists, d_count, d_tiles, d_counter, stream);
+        res.launches += 2;
+      }
+      if (is_ip) {
+        launch_query_scale(d_rq, nq, idx.rot_dim(), d_qscale, stream);
+        res.launches++;
+      }
+      const auto& fm = idx.filter_model();
+      operand_params op{};
+      op.rot_q       = d_rq;
+      op.centers     = idx.centers_rot();
+      op.q_scale     = d_qscale;
+      op.pq_dim      = idx.pq_dim();
+      op.pq_len      = idx.pq_len();
+      op.rot_dim     = idx.rot_dim();
+      op.len_pad     = fm.len_pad;
+      op.data_chunks = f_data;
+      op.k_chunks    = f_chunks;
+      op.vec_rows    = fm.len_pad == idx.pq_len() && idx.rot_dim() % 8 == 0;
+      op.is_ip       = is_ip;
+      op.scale       = fm.scale;
+      op.inv_scale2  = 1.0f / (fm.scale * fm.scale);
+      op.entry_limit = lut_kind == LUT_F16 || out_half ? 6.0e4f : (lut_kind == LUT_FP8 ? 1.2e5f : INFINITY);
+      op.rcomp_max   = fm.comp_max;
+      launch_pair_operands(op, d_probes, idx.list_sizes(), n_lists, d_groups, n_pairs, n_probes, max_groups,
+                           f_small ? nullptr : d_count, d_operand, d_rec, d_norm, stream);
+      res.launches++;
+      if (stats) { res.stats_mark(ev, 3); }
+      // 4. bounds
+      filter_params fp{};
+      fp.book         = fm.book.data();
+      fp.codes        = idx.codes();
+      fp.ids          = idx.ids();
+      fp.filter_bits  = filter.bits;
+      fp.filter_nbits = filter.n_bits;
+      fp.book_bytes   = uint32_t(fm.book.size() * sizeof(__half));
+      fp.book_size    = idx.pq_book_size();
+      fp.pq_dim       = idx.pq_dim();
+      fp.pq_bits      = idx.pq_bits();
+      fp.n_pieces     = idx.n_pieces();
+      fp.len_pad      = fm.len_pad;
+      fp.data_chunks  = f_data;
+      fp.k_chunks     = f_chunks;
+      fp.is_ip        = is_ip;
+      fp.tiles        = d_tiles;
+      fp.n_tiles      = d_counter + 1;
+      fp.pair_rec     = d_rec;
+      fp.units        = d_units;
+      fp.n_stages     = fplan.n_stages;
+      fp.error        = d_counter + 2;
+      fp.spin_limit   = kSpinLimit;
+      launch_filter(fp, d_operand, n_pairs, int(std::min<size_t>(size_t(res.sm_count), n_tiles)), fplan.filter_smem, stream);
+      res.launches++;
+      if (stats) { res.stats_mark(ev, 4); }
+      // 5. exact scores of what the bounds leave, top-k, ids and distances
+      rescore_params rp{};
+      rp.rot_q        = d_rq;
+      rp.centers      = idx.centers_rot();
+      rp.pq_centers   = idx.pq_centers();
+      rp.codes        = idx.codes();
+      rp.ids          = idx.ids();
+      rp.row_off      = idx.row_offsets();
+      rp.list_sizes   = idx.list_sizes();
+      rp.probes       = d_probes;
+      rp.chunk_index  = d_chunk;
+      rp.group_index  = d_groups;
+      rp.units        = d_units;
+      rp.pair_norm    = d_norm;
+      rp.error        = d_counter + 2;
+      rp.filter_bits  = filter.bits;
+      rp.filter_nbits = filter.n_bits;
+      rp.n_lists      = n_lists;
+      rp.n_queries    = nq;
+      rp.n_probes     = n_probes;
+      rp.k            = k;
+      rp.max_groups   = max_groups;
+      rp.pq_dim       = idx.pq_dim();
+      rp.pq_len       = idx.pq_len();
+      rp.pq_bits      = idx.pq_bits();
+      rp.rot_dim      = idx.rot_dim();
+      rp.n_pieces     = idx.n_pieces();
+      rp.book_size    = idx.pq_book_size();
+      rp.groups       = fplan.groups;
+      rp.group_threads = fplan.group_threads;
+      rp.list_cap     = fplan.list_cap;
+      rp.group_bytes  = fplan.group_bytes;
+      rp.book_bytes   = fplan.book_bytes;
+      rp.cap          = fplan.cap;
+      rp.tops         = fplan.tops;
+      rp.claim        = d_counter + 3;
+      rp.cosine       = cosine;
+      rp.metric       = int(metric);
+      rp.post_scale   = scale;
+      set_error_model(rp, op, lut_kind, out_half, fm.rmax);
+      rp.neighbors    = neighbors + size_t(q0) * k;
+      rp.distances    = distances + size_t(q0) * k;
+      launch_rescore(rp, lut_kind, out_half, is_ip,
+                     int(std::min<uint32_t>(uint32_t(res.sm_count), ceildiv(nq, fplan.groups))),
+                     fplan.rescore_smem, stream);
+      res.launches++;
+      if (stats) {
+        res.stats_mark(ev, 5);
+        res.pending.push_back(ev);
+      }
+      continue;
+    }
     // 3. sample offsets + work list of the scan
     const bool sorted_pairs = stats || n_pairs > 4096;
     if (!sorted_pairs) {
@@ -881,7 +1065,7 @@ void search_any(raft::resources& res, const search_params& params, const index<i
         d_probes, idx.list_sizes(), n_lists, nq, n_probes, d_chunk, d_count);
       if (stats) {
         scan_stats_kernel<<<ceildiv<uint32_t>(n_lists, 256), 256, 0, stream>>>(d_count, idx.list_sizes(),
-                                                                                n_lists, res.d_stats);
+                                                                                n_lists, 2, res.d_stats);
         res.stat_pairs += n_pairs;
       }
       // d_counter[0] = 0 (work counter), d_counter[1] = d_count[2 * n_lists] = number of work items

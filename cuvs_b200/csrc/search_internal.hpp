@@ -3,7 +3,25 @@
 
 #include "ivf_pq.hpp"
 
+#include <cuda.h>
+
 namespace cuvs::neighbors::ivf_pq {
+
+#ifdef __CUDACC__
+// Score -> reported distance (postprocess_distances, cpp/src/neighbors/ivf_common.cuh:175-252).
+__device__ __forceinline__ float postprocess_distance(float score, int metric, float scale)
+{
+  switch (metric) {
+    case 0: return scale != 1.0f ? __fmul_rn(score, __fmul_rn(scale, scale)) : score;
+    case 1: return scale != 1.0f ? __fmul_rn(__fsqrt_rn(score), scale) : __fsqrt_rn(score);
+    case 6: return __fmul_rn(score, __fmul_rn(__fmul_rn(-1.0f, scale), scale));
+    default: {
+      const float f = __fmul_rn(scale, scale);
+      return f != 1.0f ? __fmul_rn(score, f) : score;
+    }
+  }
+}
+#endif
 
 struct scan_plan {
   uint32_t n_groups, group_threads, pqc_in_smem, pqc_bytes, group_bytes, lut_bytes, base_bytes,
@@ -31,6 +49,9 @@ void select_rows(raft::resources& res, const float* rows, uint32_t n_rows, uint3
 // select_clusters; `centers_hi/lo` are the TF32 split of `centers`, `cmax` the largest row norm.
 // `exact_operands`: every operand is exact in TF32 and every partial sum in fp32 (small integers):
 // one product per K step, and the guard allows for no split error.
+// TMA descriptor of a row-major [rows, cols] matrix, box [box_rows, box_cols], zero fill outside (coarse_tc.cu).
+CUtensorMap make_map_2d(CUtensorMapDataType type, uint32_t elem_bytes, const void* ptr, uint64_t rows, uint64_t cols,
+                        uint32_t box_rows, uint32_t box_cols, CUtensorMapSwizzle swizzle);
 bool coarse_tc_usable(uint32_t n_lists, uint32_t n_probes, uint32_t dim_ext);
 size_t coarse_tc_workspace_bytes(uint32_t n_queries, uint32_t n_lists, uint32_t dim_ext);
 // Prepares `hi` / `lo` (TF32 split of the centre rows) with column `ext_col` (the |c|^2 column of L2

@@ -173,4 +173,40 @@ struct warp_topk {
   }
 };
 
+// 64 values per warp, value e = r * 32 + lane in register a<r>: full bitonic sort.
+template <typename T, bool Desc>
+__device__ __forceinline__ void warp_sort64(T& a0, T& a1)
+{
+  const uint32_t lane = threadIdx.x & 31u;
+  auto shfl = [](T v, int j) {
+    if constexpr (sizeof(T) == 8) {
+      const uint32_t lo = __shfl_xor_sync(kFullMask, uint32_t(v), j);
+      const uint32_t hi = __shfl_xor_sync(kFullMask, uint32_t(uint64_t(v) >> 32), j);
+      return T((uint64_t(hi) << 32) | lo);
+    } else {
+      return T(__shfl_xor_sync(kFullMask, v, j));
+    }
+  };
+#pragma unroll
+  for (uint32_t k = 2; k <= 64; k <<= 1) {
+#pragma unroll
+    for (uint32_t j = k >> 1; j > 0; j >>= 1) {
+      if (j == 32) {  // k == 64: partner is the other register of the same lane, ascending block
+        const T lo = a0 < a1 ? a0 : a1, hi = a0 < a1 ? a1 : a0;
+        a0 = Desc ? hi : lo;
+        a1 = Desc ? lo : hi;
+      } else {
+        const T o0 = shfl(a0, int(j)), o1 = shfl(a1, int(j));
+        // value index e = r * 32 + lane; block direction from bit k of e (k == 64: one block)
+        const bool up0 = ((lane & k) == 0) || k >= 32;         // r = 0: bit 5 of e is 0
+        const bool up1 = k == 64 || (k < 32 && (lane & k) == 0);  // r = 1: bit 5 of e is 1
+        const bool low = (lane & j) == 0;
+        const bool min0 = (low == up0) != Desc, min1 = (low == up1) != Desc;
+        a0 = min0 ? (a0 < o0 ? a0 : o0) : (a0 < o0 ? o0 : a0);
+        a1 = min1 ? (a1 < o1 ? a1 : o1) : (a1 < o1 ? o1 : a1);
+      }
+    }
+  }
+}
+
 }  // namespace cuvs_b200

@@ -90,6 +90,8 @@ class workspace {
   void reserve(size_t bytes)
   {
     if (bytes <= cap_) { return; }
+    // a second, slightly larger request is usual (sizes depend on the index's longest lists): an eighth of slack
+    if (cap_ != 0) { bytes += bytes / 8; }
     release();
     CUDA_TRY(cudaMalloc(&base_, bytes));
     cap_ = bytes;

@@ -280,6 +280,16 @@ class index<int64_t> {
     const float* rotation;  // [rot_dim, dim]
   };
   half_operands half_coarse_operands(cudaStream_t stream) const;
+  // Operand of the fine search's tensor-core pass, made with the other derived state: the per-subspace
+  // codebooks in half precision, [pq_dim][book][len_pad] (len_pad: pq_len rounded up to 1, 2, 4 or a
+  // multiple of 8), multiplied by the power of two `scale`; `rmax` bounds the norm of a decoded
+  // residual, `comp_max` its components.  Empty for PER_CLUSTER codebooks.
+  struct filter_operand {
+    dev_array<__half> book;
+    uint32_t len_pad = 0;
+    float scale = 1.0f, rmax = 0.0f, comp_max = 0.0f;
+  };
+  const filter_operand& filter_model() const { return filter_; }
 
   // (Re)create the arenas for the given list sizes; contents are zero codes / -1 ids.
   void allocate_lists(const std::vector<uint32_t>& sizes, cudaStream_t stream);
@@ -294,6 +304,7 @@ class index<int64_t> {
   mutable dev_array<float> centers_i8f_, rotation_i8f_;
   mutable dev_array<float> centers_h_, rotation_h_;
   mutable float centers_i8f_max_norm_ = 0.0f;
+  filter_operand filter_;
   dev_array<uint32_t> list_sizes_;
   dev_array<uint64_t> row_off_;
   dev_array<uint8_t> codes_;

@@ -1,0 +1,104 @@
+"""The two-step fine search (tensor-core bounds, then exact scores of what they leave), forced on at every size,
+against the CPU oracle: ids and distance bits."""
+import numpy as np
+import pytest
+
+from test_search_gpu import LUT, assert_parity, build_case, gpu_search
+
+pytestmark = pytest.mark.gpu
+torch = pytest.importorskip("torch")
+
+
+@pytest.fixture(autouse=True)
+def two_step():
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    from cuvs_b200 import _lib as L
+    L.check(L.load().cuvsB200SetScanCodebookHome(4))
+    yield
+    L.check(L.load().cuvsB200SetScanCodebookHome(0))
+
+
+@pytest.fixture(scope="module")
+def ivf():
+    from cuvs_b200 import ivf_pq
+    return ivf_pq
+
+
+def check(ivf, O, ix, path, q, k, p, lut, internal, tol=1e-5):
+    d, i = gpu_search(ivf, ivf.load(path), q, k, p, lut, internal)
+    do, io = O.search(ix, q, k, n_probes=p, lut_dtype=LUT[lut][1], internal_dtype=LUT[internal][1])
+    assert_parity(d, i, do, io, tol)
+
+
+# code widths x components per subspace (padded to 1, 2, 4 or a multiple of 8 in the operand)
+@pytest.mark.parametrize("bits,dim,pq_dim", [(8, 16, 16), (8, 96, 48), (8, 57, 19), (8, 32, 8), (8, 40, 8), (8, 64, 8),
+                                             (8, 96, 8), (4, 16, 16), (4, 64, 32), (4, 32, 8), (4, 48, 6), (4, 90, 10),
+                                             (5, 32, 16), (6, 48, 12), (7, 80, 16), (6, 100, 8)])
+@pytest.mark.parametrize("metric", [0, 6])
+def test_code_widths_and_lengths(ivf, oracle_mod, tmp_path, bits, dim, pq_dim, metric):
+    x, q, ix, path = build_case(oracle_mod, tmp_path, "w", n=1500, dim=dim, n_lists=12, pq_dim=pq_dim, pq_bits=bits,
+                                metric=metric, nq=40)
+    for lut in ("f32", "f16"):
+        check(ivf, oracle_mod, ix, path, q, 10, 5, lut, "f32", 1e-5 if lut == "f32" else 1e-2)
+
+
+@pytest.mark.parametrize("metric,lut,internal", [(0, "f32", "f32"), (1, "f16", "f32"), (0, "fp8", "f32"), (0, "f16", "f16"),
+                                                 (0, "fp8", "f16"), (2, "f32", "f32"), (2, "f16", "f32"), (6, "f16", "f32")])
+@pytest.mark.parametrize("k", [1, 16, 17, 64, 65, 100, 128, 300])
+def test_k_and_types(ivf, oracle_mod, tmp_path, metric, lut, internal, k):
+    x, q, ix, path = build_case(oracle_mod, tmp_path, "k", n=4000, dim=48, n_lists=16, pq_dim=24, metric=metric, nq=24)
+    check(ivf, oracle_mod, ix, path, q, k, 6, lut, internal, 1e-5 if lut == "f32" else 1e-2)
+
+
+@pytest.mark.parametrize("n_queries", [1, 16, 17, 128, 129, 400])
+def test_list_sizes_and_queries_per_list(ivf, oracle_mod, tmp_path, n_queries):
+    """Lists around the edges of groups (32 rows) and tiles (256 rows), empty ones among them, each probed by every
+    query: one tile of pairs, its edges, and several."""
+    O = oracle_mod
+    x, q, ix, path = build_case(O, tmp_path, "r", n=2000, n_lists=12, nq=n_queries)
+    sizes = [0, 1, 31, 32, 33, 0, 255, 256, 257, 64, 700, 5]
+    rng = np.random.default_rng(0)
+    codes, ids, nxt = [], [], 0
+    for s in sizes:
+        c = rng.integers(0, 256, size=(s, ix.pq_dim), dtype=np.uint8)
+        codes.append(O.pack_list(c, 8) if s else np.zeros(0, np.uint8))
+        ids.append(np.arange(nxt, nxt + s, dtype=np.int64) * 3 + 7)
+        nxt += s
+    ix.list_sizes = np.array(sizes, dtype=np.uint32)
+    ix.list_codes, ix.list_ids, ix._flat = codes, ids, None
+    ix.save(path)
+    for p in (1, 5, 12):
+        check(ivf, O, ix, path, q, 20, p, "f32", "f32")
+
+
+def test_filter_and_few_candidates(ivf, oracle_mod, tmp_path):
+    """A bitset that lets a handful of rows through: fewer than k results, padded."""
+    x, q, ix, path = build_case(oracle_mod, tmp_path, "f", n=3000, n_lists=16, nq=200)
+    g = ivf.load(path)
+    for keep in (3, 200, 2500):
+        allowed = np.zeros(3008, bool)
+        allowed[np.random.default_rng(keep).choice(3000, keep, replace=False)] = True
+        words = np.packbits(allowed, bitorder="little").view(np.uint32)
+        sp = ivf.SearchParams(n_probes=8)
+        d, i = ivf.search(sp, g, torch.from_numpy(q).cuda(), 10, filter=torch.from_numpy(words).cuda())
+        d, i = d.cpu().numpy(), i.cpu().numpy()
+        do, io = oracle_mod.search(ix, q, 10, n_probes=8, bitset=words)
+        assert_parity(d, i, do, io, 1e-5)
+
+
+@pytest.mark.parametrize("scale", [1e-6, 1.0, 300.0, 1e6])
+def test_data_scale(ivf, oracle_mod, tmp_path, scale):
+    """Operands are scaled into half precision: tiny and huge data, tables whose entries overflow their type, and queries
+    far outside the data (differences that half precision cannot hold)."""
+    O = oracle_mod
+    from conftest import make_mixture
+    x = (make_mixture(2000, 32, 30, 0.15, 0) * scale).astype(np.float32)
+    q = (make_mixture(48, 32, 30, 0.15, 1) * scale).astype(np.float32)
+    q[5] *= 3000.0
+    q[6] *= 1e-4
+    ix = O.build_index(x, 16, pq_dim=16, pq_bits=8, kmeans_iters=3)
+    path = str(tmp_path / "s.ivfpq")
+    ix.save(path)
+    for lut in ("f32", "fp8") + (("f16",) if scale < 1e3 else ()):
+        check(ivf, O, ix, path, q, 10, 6, lut, "f32", 1e-5 if lut == "f32" else 1e-2)
