@@ -20,226 +20,463 @@ using namespace cuvs_b200;
 
 namespace {
 
-constexpr int kTile   = 64;  // queries x lists per block
-constexpr int kTileK  = 16;
 constexpr uint32_t kMaxProbes = 4096;
 
-// scores[q, l] for a chunk of queries; block = 16x16 threads, 4x4 outputs per thread.
-__global__ void __launch_bounds__(256)
-coarse_scores_kernel(const float* __restrict__ centers, const float* __restrict__ fq, uint32_t n_lists,
-                     uint32_t n_queries, uint32_t dim_ext, float alpha, int half_scores,
-                     float* __restrict__ scores)
+__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c)
 {
-  __shared__ float s_c[kTileK][kTile + 1];
-  __shared__ float s_q[kTileK][kTile + 1];
-  const uint32_t l0 = blockIdx.x * kTile, q0 = blockIdx.y * kTile;
-  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-  float acc[4][4];
+  uint64_t d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
+}
+
+// out[i, j] = alpha * sum over ascending k of b[j, k] * a[i, k], one fused multiply-add chain per output (the chain that
+// defines a coarse score, a rotation, a label).  kArgmin: instead of storing, best[i] = min over j of
+// (ordered score << 32 | j), "lowest score, then lowest id".
+// What bounds it: the FMA pipe, and shared-memory wavefronts close behind.  128 x 128 outputs per block, 8 x 8 per thread
+// as packed pairs of columns (fma.rn.f32x2: two chains per instruction); the row operand sits in shared memory
+// duplicated, so that no register is spent on pairing, and the next eight k are on their way while eight are used.
+// 10,000 x 4,000 x 136: 487 us with 64 x 64 outputs per block and scalar FMAs, 358 us so.  kVec: rows of both operands are
+// 16-byte aligned and k is a multiple of four.
+constexpr uint32_t kTile = 128, kTileK = 8;
+template <bool kVec, bool kArgmin>
+__global__ void __launch_bounds__(256, 2)
+exact_gemm_kernel(const float* __restrict__ b, uint32_t n_cols, const float* __restrict__ a, uint32_t n_rows, uint32_t kdim,
+                  float alpha, int half_scores, float* __restrict__ out, unsigned long long* __restrict__ best)
+{
+  __shared__ __align__(16) float2 s_a[2][kTileK][kTile + 2];
+  __shared__ __align__(16) float s_b[2][kTileK][kTile + 4];
+  const uint32_t j0 = blockIdx.x * kTile, i0 = blockIdx.y * kTile;
+  const uint32_t tid = threadIdx.x, tx = tid & 15u, ty = tid >> 4;
+  // one row and four k of either operand per thread
+  const uint32_t lrow = tid >> 1, lk = (tid & 1u) * 4u;
+  const bool in_a = i0 + lrow < n_rows, in_b = j0 + lrow < n_cols;
+  const float* pa = a + size_t(i0 + lrow) * kdim + lk;
+  const float* pb = b + size_t(j0 + lrow) * kdim + lk;
+  float ra[4], rb[4];
+  auto load = [&](uint32_t k0) {
+    if constexpr (kVec) {
+      const float4 z = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+      const float4 x = in_a && k0 + lk < kdim ? __ldg(reinterpret_cast<const float4*>(pa + k0)) : z;
+      const float4 y = in_b && k0 + lk < kdim ? __ldg(reinterpret_cast<const float4*>(pb + k0)) : z;
+      ra[0] = x.x; ra[1] = x.y; ra[2] = x.z; ra[3] = x.w;
+      rb[0] = y.x; rb[1] = y.y; rb[2] = y.z; rb[3] = y.w;
+    } else {
 #pragma unroll
-  for (int i = 0; i < 4; i++) {
-#pragma unroll
-    for (int j = 0; j < 4; j++) { acc[i][j] = 0.0f; }
-  }
-  for (uint32_t k0 = 0; k0 < dim_ext; k0 += kTileK) {
-    for (int i = threadIdx.x; i < kTile * kTileK; i += 256) {
-      const int row = i / kTileK, kk = i % kTileK;
-      const uint32_t k = k0 + kk;
-      const uint32_t l = l0 + row, q = q0 + row;
-      s_c[kk][row] = (l < n_lists && k < dim_ext) ? centers[size_t(l) * dim_ext + k] : 0.0f;
-      s_q[kk][row] = (q < n_queries && k < dim_ext) ? fq[size_t(q) * dim_ext + k] : 0.0f;
-    }
-    __syncthreads();
-    const int kmax = min(kTileK, int(dim_ext - k0));
-    for (int kk = 0; kk < kmax; kk++) {
-      float c[4], f[4];
-#pragma unroll
-      for (int j = 0; j < 4; j++) { c[j] = s_c[kk][tx + 16 * j]; }
-#pragma unroll
-      for (int i = 0; i < 4; i++) { f[i] = s_q[kk][ty + 16 * i]; }
-#pragma unroll
-      for (int i = 0; i < 4; i++) {
-#pragma unroll
-        for (int j = 0; j < 4; j++) { acc[i][j] = __fmaf_rn(c[j], f[i], acc[i][j]); }
+      for (uint32_t e = 0; e < 4; e++) {
+        const bool in = k0 + lk + e < kdim;
+        ra[e]         = in && in_a ? __ldg(pa + k0 + e) : 0.0f;
+        rb[e]         = in && in_b ? __ldg(pb + k0 + e) : 0.0f;
       }
     }
-    __syncthreads();
+  };
+  auto store = [&](uint32_t buf) {
+#pragma unroll
+    for (uint32_t e = 0; e < 4; e++) {
+      s_a[buf][lk + e][lrow] = make_float2(ra[e], ra[e]);
+      s_b[buf][lk + e][lrow] = rb[e];
+    }
+  };
+  // rows ty * 4 + {0..3} and 64 + ..., columns tx * 4 + {0..3} and 64 + ...
+  uint64_t acc[8][4];
+#pragma unroll
+  for (int i = 0; i < 8; i++) {
+#pragma unroll
+    for (int j = 0; j < 4; j++) { acc[i][j] = 0ull; }
+  }
+  load(0);
+  store(0);
+  __syncthreads();
+  uint32_t buf = 0;
+  for (uint32_t k0 = 0; k0 < kdim; k0 += kTileK, buf ^= 1u) {
+    const bool more = k0 + kTileK < kdim;
+    if (more) { load(k0 + kTileK); }
+    // (a partial last tile stops at kdim: a product with zero would leave the chain's value alone, except for -0 and
+    // infinities)
+    const uint32_t kn = min(kTileK, kdim - k0);
+    auto step = [&](uint32_t k) {
+      const ulonglong2* qa = reinterpret_cast<const ulonglong2*>(&s_a[buf][k][ty * 4u]);
+      const ulonglong2* qb = reinterpret_cast<const ulonglong2*>(&s_a[buf][k][64u + ty * 4u]);
+      const ulonglong2 x0 = qa[0], x1 = qa[1], x2 = qb[0], x3 = qb[1];
+      const ulonglong2 c0 = *reinterpret_cast<const ulonglong2*>(&s_b[buf][k][tx * 4u]);
+      const ulonglong2 c1 = *reinterpret_cast<const ulonglong2*>(&s_b[buf][k][64u + tx * 4u]);
+      const uint64_t x[8] = {x0.x, x0.y, x1.x, x1.y, x2.x, x2.y, x3.x, x3.y};
+      const uint64_t c[4] = {c0.x, c0.y, c1.x, c1.y};
+#pragma unroll
+      for (int i = 0; i < 8; i++) {
+#pragma unroll
+        for (int j = 0; j < 4; j++) { acc[i][j] = fma2(c[j], x[i], acc[i][j]); }
+      }
+    };
+    if (kn == kTileK) {
+#pragma unroll
+      for (uint32_t k = 0; k < kTileK; k++) { step(k); }
+    } else {
+      for (uint32_t k = 0; k < kn; k++) { step(k); }
+    }
+    if (more) {
+      store(buf ^ 1u);
+      __syncthreads();
+    }
   }
 #pragma unroll
-  for (int i = 0; i < 4; i++) {
-    const uint32_t q = q0 + ty + 16 * i;
-    if (q >= n_queries) { continue; }
+  for (int i = 0; i < 8; i++) {
+    const uint32_t row = i0 + (i < 4 ? ty * 4u + i : 64u + ty * 4u + (i - 4));
+    [[maybe_unused]] unsigned long long m = ~0ull;
 #pragma unroll
-    for (int j = 0; j < 4; j++) {
-      const uint32_t l = l0 + tx + 16 * j;
-      if (l < n_lists) {
-        float v = __fmul_rn(alpha, acc[i][j]);
+    for (int h = 0; h < 2; h++) {
+      const uint32_t col = j0 + h * 64u + tx * 4u;
+      float v[4];
+#pragma unroll
+      for (int e = 0; e < 4; e++) {
+        const uint64_t pair = acc[i][h * 2 + (e >> 1)];
+        v[e] = __fmul_rn(alpha, __uint_as_float(uint32_t((e & 1) ? (pair >> 32) : pair)));
         // fp16 coarse search: the score is a half-precision number
+        if (half_scores) { v[e] = __half2float(__float2half_rn(v[e])); }
+      }
+      if constexpr (kArgmin) {
+#pragma unroll
+        for (int e = 0; e < 4; e++) {
+          const unsigned long long key = ((unsigned long long)float_to_ordered(v[e]) << 32) | (col + e);
+          if (col + e < n_cols) { m = key < m ? key : m; }
+        }
+      } else if (row < n_rows) {
+        float* o = out + size_t(row) * n_cols + col;
+        if (n_cols % 4 == 0 && col < n_cols) {
+          *reinterpret_cast<float4*>(o) = make_float4(v[0], v[1], v[2], v[3]);
+        } else {
+#pragma unroll
+          for (int e = 0; e < 4; e++) {
+            if (col + e < n_cols) { o[e] = v[e]; }
+          }
+        }
+      }
+    }
+    if constexpr (kArgmin) {
+      // the 16 threads sharing a row sit in one half-warp: reduce before touching memory
+#pragma unroll
+      for (int d = 8; d > 0; d >>= 1) {
+        const unsigned long long o = __shfl_xor_sync(kFullMask, m, d);
+        m = o < m ? o : m;
+      }
+      if (tx == 0 && row < n_rows) { atomicMin(best + row, m); }
+    }
+  }
+}
+
+// The same product for a few rows (at most kFewRows), where the tiles above would leave the chip empty and the time is
+// the latency of one block (1 x 1,024 x 136: 16 us so, 5.4 us here): 32 columns per block, their rows of `b` staged whole
+// in shared memory (every load in flight at once; odd row length against bank conflicts), warp = up to kFewRows / 4
+// rows of `a`, lane = column.
+constexpr uint32_t kFewRows = 16;
+__global__ void __launch_bounds__(128)
+few_rows_kernel(const float* __restrict__ b, uint32_t n_cols, const float* __restrict__ a, uint32_t n_rows, uint32_t kdim,
+                float alpha, int half_scores, float* __restrict__ out)
+{
+  extern __shared__ float s_few[];  // [32][kdim | 1], then [n_rows][kdim]
+  constexpr uint32_t kPer = kFewRows / 4;
+  const uint32_t j0 = blockIdx.x * 32u, tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
+  const uint32_t ld = kdim | 1u;
+  float* s_a        = s_few + 32u * ld;
+  const uint32_t nc = min(32u, n_cols - j0);
+  const float* src  = b + size_t(j0) * kdim;
+#pragma unroll 8
+  for (uint32_t i = tid; i < nc * kdim; i += 128u) {
+    const uint32_t r = i / kdim;
+    s_few[r * ld + (i - r * kdim)] = __ldg(src + i);
+  }
+  for (uint32_t i = tid; i < n_rows * kdim; i += 128u) { s_a[i] = __ldg(a + i); }
+  __syncthreads();
+  float acc[kPer] = {};
+  const float* c  = s_few + lane * ld;
+  if (warp < n_rows) {
+#pragma unroll 4
+    for (uint32_t k = 0; k < kdim; k++) {
+      const float cv = c[k];
+#pragma unroll
+      for (uint32_t r = 0; r < kPer; r++) {
+        if (warp + 4u * r < n_rows) { acc[r] = __fmaf_rn(cv, s_a[(warp + 4u * r) * kdim + k], acc[r]); }
+      }
+    }
+  }
+  if (lane < nc) {
+#pragma unroll
+    for (uint32_t r = 0; r < kPer; r++) {
+      if (warp + 4u * r < n_rows) {
+        float v = __fmul_rn(alpha, acc[r]);
         if (half_scores) { v = __half2float(__float2half_rn(v)); }
-        scores[size_t(q) * n_lists + l] = v;
+        out[size_t(warp + 4u * r) * n_cols + j0 + lane] = v;
       }
     }
   }
 }
 
-// One block per query: exact n_probes smallest (score, id) of a row, written in ascending order.
-// Radix select on the order-preserving image of the score (4 passes of 8 bits), one gather pass,
-// then a bitonic sort of the selected keys in shared memory.
-__global__ void __launch_bounds__(256)
-select_probes_kernel(const float* __restrict__ scores, uint32_t n_lists, uint32_t n_probes,
-                     uint32_t cap /* power of two >= n_probes */, uint32_t* __restrict__ probes,
-                     float* __restrict__ scores_out)
+template <bool kArgmin>
+void launch_exact_gemm(const float* b, uint32_t n_cols, const float* a, uint32_t n_rows, uint32_t kdim, float alpha,
+                       bool half_scores, float* out, unsigned long long* best, cudaStream_t stream)
 {
-  extern __shared__ uint64_t s_keys[];  // [cap]
-  __shared__ uint32_t s_hist[256];
-  __shared__ uint32_t s_prefix, s_remaining, s_count, s_eq_taken;
-  const uint32_t q   = blockIdx.x;
-  const float* row   = scores + size_t(q) * n_lists;
-  const uint32_t tid = threadIdx.x;
+  if constexpr (!kArgmin) {
+    const size_t smem = (size_t(32) * (kdim | 1u) + size_t(n_rows) * kdim) * 4;
+    if (n_rows <= kFewRows && smem <= 200 * 1024) {
+      ensure_dynamic_smem(reinterpret_cast<const void*>(few_rows_kernel), smem);
+      few_rows_kernel<<<ceildiv(n_cols, 32u), 128, smem, stream>>>(b, n_cols, a, n_rows, kdim, alpha, half_scores, out);
+      CUDA_TRY(cudaGetLastError());
+      return;
+    }
+  }
+  // grid.y is limited to 65535 blocks of rows
+  const uint32_t most = 65535u * kTile;
+  for (uint32_t r0 = 0; r0 < n_rows; r0 += most) {
+    const uint32_t nr = std::min(most, n_rows - r0);
+    const dim3 grid(ceildiv(n_cols, kTile), ceildiv(nr, kTile));
+    const float* ar = a + size_t(r0) * kdim;
+    float* o        = out ? out + size_t(r0) * n_cols : nullptr;
+    unsigned long long* bs = best ? best + r0 : nullptr;
+    const bool vec = kdim % 4 == 0 && ((reinterpret_cast<uintptr_t>(b) | reinterpret_cast<uintptr_t>(ar)) & 15u) == 0;
+    if (vec) {
+      exact_gemm_kernel<true, kArgmin><<<grid, 256, 0, stream>>>(b, n_cols, ar, nr, kdim, alpha, half_scores, o, bs);
+    } else {
+      exact_gemm_kernel<false, kArgmin><<<grid, 256, 0, stream>>>(b, n_cols, ar, nr, kdim, alpha, half_scores, o, bs);
+    }
+    CUDA_TRY(cudaGetLastError());
+  }
+}
 
-  if (tid == 0) {
-    s_prefix    = 0;
-    s_remaining = n_probes;
+// The digit (0..255) at which the running count of `hist` reaches `rem`, and how many of that digit are wanted; one whole
+// warp calls it.
+__device__ __forceinline__ void find_digit(const uint32_t* hist, uint32_t rem, uint32_t& digit, uint32_t& left)
+{
+  const uint32_t lane = threadIdx.x & 31u;
+  uint32_t c[8], sum = 0;
+#pragma unroll
+  for (int i = 0; i < 8; i++) {
+    c[i] = hist[lane * 8u + i];
+    sum += c[i];
   }
-  // radix select: after the passes s_prefix is the ordered image T of the n_probes-th smallest score
-  for (int pass = 0; pass < 4; pass++) {
-    const int shift = 24 - 8 * pass;
-    s_hist[tid]     = 0;
-    __syncthreads();
-    const uint32_t prefix = s_prefix;
-    const uint32_t mask   = pass == 0 ? 0u : (0xFFFFFFFFu << (shift + 8));
-    for (uint32_t l = tid; l < n_lists; l += 256) {
-      const uint32_t o = float_to_ordered(row[l]);
-      if ((o & mask) == prefix) { atomicAdd(&s_hist[(o >> shift) & 0xFFu], 1u); }
-    }
-    __syncthreads();
-    if (tid == 0) {
-      uint32_t rem = s_remaining, d = 0;
-      for (; d < 256; d++) {
-        const uint32_t c = s_hist[d];
-        if (c >= rem) { break; }
-        rem -= c;
-      }
-      s_prefix    = prefix | (d << shift);
-      s_remaining = rem;  // how many elements are wanted among those sharing the new prefix
-    }
-    __syncthreads();
+  uint32_t inc = sum;
+#pragma unroll
+  for (int d = 1; d < 32; d <<= 1) {
+    const uint32_t o = __shfl_up_sync(kFullMask, inc, d);
+    if (lane >= uint32_t(d)) { inc += o; }
   }
-  const uint32_t T       = s_prefix;
-  const uint32_t want_eq = s_remaining;  // elements equal to T that belong to the selection
-  if (tid == 0) {
-    s_count    = 0;
-    s_eq_taken = 0;
-  }
-  for (uint32_t i = tid; i < cap; i += 256) { s_keys[i] = kEmptyKey; }
-  __syncthreads();
-  // gather: everything below T, plus the want_eq lowest-numbered lists equal to T
-  for (uint32_t base = 0; base < n_lists; base += 256) {
-    const uint32_t l = base + tid;
-    uint32_t o       = 0xFFFFFFFFu;
-    if (l < n_lists) { o = float_to_ordered(row[l]); }
-    if (l < n_lists && o < T) { s_keys[atomicAdd(&s_count, 1u)] = (uint64_t(o) << 32) | l; }
-    // ties at T are taken in list order: ballot keeps order inside a warp, warps take turns
-    const bool eq = l < n_lists && o == T;
-    if (__syncthreads_or(eq)) {
-      for (int w = 0; w < 8; w++) {
-        if (int(tid >> 5) == w) {
-          const unsigned m = __ballot_sync(kFullMask, eq);
-          if (m) {
-            const uint32_t start = s_eq_taken;
-            const uint32_t rank  = start + __popc(m & ((1u << (tid & 31)) - 1u));
-            if (eq && rank < want_eq) { s_keys[atomicAdd(&s_count, 1u)] = (uint64_t(o) << 32) | l; }
-            __syncwarp();
-            if ((tid & 31) == 0) { s_eq_taken = start + __popc(m); }
-          }
-        }
-        __syncthreads();
-      }
+  const unsigned reach = __ballot_sync(kFullMask, inc >= rem);
+  digit = 255u;
+  left  = rem;
+  if (reach == 0u) { return; }
+  const int src = __ffs(reach) - 1;
+  uint32_t d = lane * 8u, r = rem - (inc - sum);
+#pragma unroll
+  for (int i = 0; i < 7; i++) {
+    if (d == lane * 8u + i && c[i] < r) {
+      r -= c[i];
+      d++;
     }
   }
-  __syncthreads();
-  // bitonic sort of cap keys
-  for (uint32_t size = 2; size <= cap; size <<= 1) {
+  digit = __shfl_sync(kFullMask, d, src);
+  left  = __shfl_sync(kFullMask, r, src);
+}
+
+// Sorts the first n2 (a power of two) keys ascending; the whole block calls it after a barrier.
+__device__ __forceinline__ void block_sort_keys(uint64_t* keys, uint32_t n2)
+{
+  for (uint32_t size = 2; size <= n2; size <<= 1) {
     for (uint32_t stride = size >> 1; stride > 0; stride >>= 1) {
-      for (uint32_t i = tid; i < cap / 2; i += 256) {
+      for (uint32_t i = threadIdx.x; i < n2 / 2; i += blockDim.x) {
         const uint32_t lo = 2 * i - (i & (stride - 1));
         const uint32_t hi = lo + stride;
         const bool up     = (lo & size) == 0;
-        const uint64_t a = s_keys[lo], b = s_keys[hi];
+        const uint64_t a = keys[lo], b = keys[hi];
         if ((a > b) == up) {
-          s_keys[lo] = b;
-          s_keys[hi] = a;
+          keys[lo] = b;
+          keys[hi] = a;
         }
       }
       __syncthreads();
     }
   }
-  for (uint32_t p = tid; p < n_probes; p += 256) {
-    const uint64_t key                  = s_keys[p];
-    probes[size_t(q) * n_probes + p]    = uint32_t(key);
-    if (scores_out) { scores_out[size_t(q) * n_probes + p] = ordered_to_float(uint32_t(key >> 32)); }
+}
+
+// One block per row: the exact `want` smallest (score, position), written in ascending order.  A row holds row_len scores,
+// or row_ends[(row + 1) * ends_stride - 1] of them; where that is less than `want` the rest of the result is empty
+// (score NaN).
+//
+// First way: every thread keeps the kTops smallest scores of its strided part of the row; at least `want` scores are at or
+// below the want-th smallest of the kThreads * kTops kept ones, and few others are (expected 1.2 `want` at 64 of 256,
+// 1.4 at 128; 1.1 at 1,000 of 1,024 x 2), so two reads of the row find them all: keys (score, position) into shared
+// memory, one sort.  A radix select reads the row five times, and its first histogram is one bucket's serial atomics
+// (scores share their exponent): 252 us against 111 us for 64 of 4,000 scores in 10,000 rows, 280 against 85 us for 1,000 of
+// 15,000 in 500 rows.
+// Second way (more ties at the threshold than the buffer holds): radix select on the order-preserving image of the score
+// (4 passes of 8 bits), one gather pass, then the sort.
+template <uint32_t kThreads, uint32_t kTops>
+__global__ void __launch_bounds__(kThreads)
+select_kernel(const float* __restrict__ scores, uint32_t row_stride, uint32_t row_len, const uint32_t* __restrict__ row_ends,
+              uint32_t ends_stride, uint32_t want, uint32_t cap /* keys of shared memory */, uint32_t* __restrict__ out_idx,
+              float* __restrict__ out_scores)
+{
+  extern __shared__ uint64_t s_keys[];  // [cap]
+  __shared__ uint32_t s_hist[256];
+  __shared__ uint32_t s_prefix, s_remaining, s_count, s_eq_taken;
+  const uint32_t q   = blockIdx.x;
+  const float* row   = scores + size_t(q) * row_stride;
+  const uint32_t tid = threadIdx.x;
+  const uint32_t len = row_ends ? row_ends[size_t(q + 1) * ends_stride - 1] : row_len;
+  const uint32_t n4  = row_stride % 4 == 0 ? len / 4 : 0u;  // rows start on 16-byte boundaries
+  // every score of the row with its position
+  auto for_row = [&](auto&& fn) {
+    const float4* r4 = reinterpret_cast<const float4*>(row);
+#pragma unroll 4
+    for (uint32_t i = tid; i < n4; i += kThreads) {
+      const float4 v = __ldg(r4 + i);
+      fn(float_to_ordered(v.x), 4 * i);
+      fn(float_to_ordered(v.y), 4 * i + 1);
+      fn(float_to_ordered(v.z), 4 * i + 2);
+      fn(float_to_ordered(v.w), 4 * i + 3);
+    }
+#pragma unroll 4
+    for (uint32_t i = 4 * n4 + tid; i < len; i += kThreads) { fn(float_to_ordered(__ldg(row + i)), i); }
+  };
+
+  uint32_t n_sort = 0;
+  {
+    uint32_t best[kTops];
+#pragma unroll
+    for (uint32_t i = 0; i < kTops; i++) { best[i] = 0xFFFFFFFFu; }
+    for_row([&](uint32_t o, uint32_t) {
+#pragma unroll
+      for (uint32_t i = kTops - 1; i > 0; i--) { best[i] = min(best[i], max(best[i - 1], o)); }
+      best[0] = min(best[0], o);
+    });
+    // 24 bits of the want-th smallest of the kept scores, rounded up
+    uint32_t lo = 0;
+    for (int bit = 31; bit >= 8; bit--) {
+      const uint32_t c = lo | (1u << bit);
+      uint32_t n       = 0;
+#pragma unroll
+      for (uint32_t i = 0; i < kTops; i++) { n += uint32_t(__syncthreads_count(best[i] < c)); }
+      if (n < want) { lo = c; }
+    }
+    const uint32_t T = lo | 0xFFu;
+    if (tid == 0) { s_count = 0; }
+    __syncthreads();
+    if (best[0] <= T) {  // (a thread whose smallest score is above the threshold has nothing)
+      for_row([&](uint32_t o, uint32_t l) {
+        if (o <= T) {
+          const uint32_t slot = atomicAdd(&s_count, 1u);
+          if (slot < cap) { s_keys[slot] = (uint64_t(o) << 32) | l; }
+        }
+      });
+    }
+    __syncthreads();
+    const uint32_t n = s_count;
+    if (n <= cap) {
+      n_sort = 64;
+      while (n_sort < n || n_sort < want) { n_sort <<= 1; }
+      for (uint32_t i = n + tid; i < n_sort; i += kThreads) { s_keys[i] = kEmptyKey; }
+    }
+    __syncthreads();
+  }
+  if (n_sort == 0) {
+    n_sort = 64;
+    while (n_sort < want) { n_sort <<= 1; }
+    if (tid == 0) {
+      s_prefix    = 0;
+      s_remaining = want;
+    }
+    // radix select: after the passes s_prefix is the ordered image T of the want-th smallest score
+    for (int pass = 0; pass < 4; pass++) {
+      const int shift = 24 - 8 * pass;
+      if (tid < 256) { s_hist[tid] = 0; }
+      __syncthreads();
+      const uint32_t prefix = s_prefix;
+      const uint32_t mask   = pass == 0 ? 0u : (0xFFFFFFFFu << (shift + 8));
+      for_row([&](uint32_t o, uint32_t) {
+        if ((o & mask) == prefix) { atomicAdd(&s_hist[(o >> shift) & 0xFFu], 1u); }
+      });
+      __syncthreads();
+      if (tid < 32) {
+        uint32_t d, left;
+        find_digit(s_hist, s_remaining, d, left);
+        if (tid == 0) {
+          s_prefix    = prefix | (d << shift);
+          s_remaining = left;  // how many elements are wanted among those sharing the new prefix
+        }
+      }
+      __syncthreads();
+    }
+    const uint32_t T       = s_prefix;
+    const uint32_t want_eq = s_remaining;  // elements equal to T that belong to the selection
+    if (tid == 0) {
+      s_count    = 0;
+      s_eq_taken = 0;
+    }
+    for (uint32_t i = tid; i < n_sort; i += kThreads) { s_keys[i] = kEmptyKey; }
+    __syncthreads();
+    // gather: everything below T, plus the want_eq lowest positions equal to T
+    for (uint32_t base = 0; base < len; base += kThreads) {
+      const uint32_t l = base + tid;
+      uint32_t o       = 0xFFFFFFFFu;
+      if (l < len) { o = float_to_ordered(row[l]); }
+      if (l < len && o < T) { s_keys[atomicAdd(&s_count, 1u)] = (uint64_t(o) << 32) | l; }
+      // ties at T are taken in order: ballot keeps order inside a warp, warps take turns
+      const bool eq = l < len && o == T;
+      if (__syncthreads_or(eq)) {
+        for (uint32_t w = 0; w < kThreads / 32; w++) {
+          if ((tid >> 5) == w) {
+            const unsigned m = __ballot_sync(kFullMask, eq);
+            if (m) {
+              const uint32_t start = s_eq_taken;
+              const uint32_t rank  = start + __popc(m & ((1u << (tid & 31)) - 1u));
+              if (eq && rank < want_eq) { s_keys[atomicAdd(&s_count, 1u)] = (uint64_t(o) << 32) | l; }
+              __syncwarp();
+              if ((tid & 31) == 0) { s_eq_taken = start + __popc(m); }
+            }
+          }
+          __syncthreads();
+        }
+      }
+    }
+    __syncthreads();
+  }
+  if (n_sort == 64) {
+    if (tid < 32) {
+      uint64_t a0 = s_keys[tid], a1 = s_keys[tid + 32];
+      warp_sort64<uint64_t, false>(a0, a1);
+      s_keys[tid]      = a0;
+      s_keys[tid + 32] = a1;
+    }
+    __syncthreads();
+  } else {
+    block_sort_keys(s_keys, n_sort);
+  }
+  for (uint32_t p = tid; p < want; p += kThreads) {
+    const uint64_t key             = s_keys[p];
+    out_idx[size_t(q) * want + p] = uint32_t(key);
+    if (out_scores) { out_scores[size_t(q) * want + p] = ordered_to_float(uint32_t(key >> 32)); }
   }
 }
 
-// Same product as coarse_scores_kernel, but the epilogue keeps only the per-row minimum:
-// atomicMin on (ordered score << 32 | list id) implements "lowest score, then lowest id".
-__global__ void __launch_bounds__(256)
-assign_nearest_kernel(const float* __restrict__ centers, const float* __restrict__ x, uint32_t n_lists,
-                      uint32_t n_rows, uint32_t dim_ext, float alpha, unsigned long long* __restrict__ best)
+// Threads and scores kept per thread: `want` stays below two thirds of what the block keeps, where the scores taken beyond
+// the wanted ones are few; the buffer holds them with room to spare (a power of two, as the sort needs).
+void launch_select(const float* scores, uint32_t n_rows, uint32_t row_stride, uint32_t row_len, const uint32_t* row_ends,
+                   uint32_t ends_stride, uint32_t want, uint32_t* out_idx, float* out_scores, cudaStream_t stream)
 {
-  __shared__ float s_c[kTileK][kTile + 1];
-  __shared__ float s_q[kTileK][kTile + 1];
-  const uint32_t l0 = blockIdx.x * kTile, q0 = blockIdx.y * kTile;
-  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-  float acc[4][4];
-#pragma unroll
-  for (int i = 0; i < 4; i++) {
-#pragma unroll
-    for (int j = 0; j < 4; j++) { acc[i][j] = 0.0f; }
-  }
-  for (uint32_t k0 = 0; k0 < dim_ext; k0 += kTileK) {
-    for (int i = threadIdx.x; i < kTile * kTileK; i += 256) {
-      const int row = i / kTileK, kk = i % kTileK;
-      const uint32_t k = k0 + kk;
-      const uint32_t l = l0 + row, q = q0 + row;
-      s_c[kk][row] = (l < n_lists && k < dim_ext) ? centers[size_t(l) * dim_ext + k] : 0.0f;
-      s_q[kk][row] = (q < n_rows && k < dim_ext) ? x[size_t(q) * dim_ext + k] : 0.0f;
-    }
-    __syncthreads();
-    const int kmax = min(kTileK, int(dim_ext - k0));
-    for (int kk = 0; kk < kmax; kk++) {
-      float c[4], f[4];
-#pragma unroll
-      for (int j = 0; j < 4; j++) { c[j] = s_c[kk][tx + 16 * j]; }
-#pragma unroll
-      for (int i = 0; i < 4; i++) { f[i] = s_q[kk][ty + 16 * i]; }
-#pragma unroll
-      for (int i = 0; i < 4; i++) {
-#pragma unroll
-        for (int j = 0; j < 4; j++) { acc[i][j] = __fmaf_rn(c[j], f[i], acc[i][j]); }
-      }
-    }
-    __syncthreads();
-  }
-#pragma unroll
-  for (int i = 0; i < 4; i++) {
-    const uint32_t q = q0 + ty + 16 * i;
-    unsigned long long m = ~0ull;
-#pragma unroll
-    for (int j = 0; j < 4; j++) {
-      const uint32_t l = l0 + tx + 16 * j;
-      if (l < n_lists) {
-        const unsigned long long key =
-          ((unsigned long long)float_to_ordered(__fmul_rn(alpha, acc[i][j])) << 32) | l;
-        m = key < m ? key : m;
-      }
-    }
-    // the 16 threads sharing a row sit in one half-warp: reduce before touching memory
-#pragma unroll
-    for (int d = 8; d > 0; d >>= 1) {
-      const unsigned long long o = __shfl_xor_sync(kFullMask, m, d);
-      m = o < m ? o : m;
-    }
-    if (tx == 0 && q < n_rows) { atomicMin(best + q, m); }
+  uint32_t cap = 64;
+  while (cap < want + (want <= 1024 ? want / 2 : want / 4) || (want <= 160 && cap < 3 * want)) { cap <<= 1; }
+  auto go = [&](auto kernel, int threads) {
+    const size_t smem = size_t(cap) * 8;
+    if (smem > 48 * 1024) { ensure_dynamic_smem(reinterpret_cast<const void*>(kernel), smem); }
+    kernel<<<n_rows, threads, smem, stream>>>(scores, row_stride, row_len, row_ends, ends_stride, want, cap, out_idx,
+                                              out_scores);
+    CUDA_TRY(cudaGetLastError());
+  };
+  if (want <= 160) {
+    go(select_kernel<256, 1>, 256);
+  } else if (want <= 384) {
+    go(select_kernel<256, 2>, 256);
+  } else if (want <= 1200) {
+    go(select_kernel<1024, 2>, 1024);
+  } else {
+    go(select_kernel<1024, 8>, 1024);
   }
 }
 
@@ -256,7 +493,9 @@ uint32_t chunk_queries(uint32_t n_queries, uint32_t n_lists)
   const uint64_t target = 64ull << 20;
   uint64_t c            = std::max<uint64_t>(kTile, target / (uint64_t(n_lists) * 4));
   c                     = (c / kTile) * kTile;
-  return uint32_t(std::min<uint64_t>(c, round_up<uint32_t>(n_queries, kTile)));
+  // equal chunks: a short last one would be a nearly empty wave
+  const uint32_t n = uint32_t(ceildiv<uint64_t>(n_queries, c));
+  return round_up<uint32_t>(ceildiv(n_queries, n), kTile);
 }
 
 }  // namespace
@@ -278,32 +517,23 @@ void select_clusters(raft::resources& res, const float* centers, uint32_t n_list
   const uint32_t chunk = chunk_queries(n_queries, n_lists);
   CUVS_EXPECTS(workspace_bytes >= size_t(chunk) * n_lists * 4, "coarse workspace too small");
   float* scores = static_cast<float*>(workspace);
-  uint32_t cap  = 1;
-  while (cap < n_probes) { cap <<= 1; }
-  cap = std::max<uint32_t>(cap, 2);
   for (uint32_t q0 = 0; q0 < n_queries; q0 += chunk) {
     const uint32_t nq = std::min(chunk, n_queries - q0);
-    dim3 grid(ceildiv<uint32_t>(n_lists, kTile), ceildiv<uint32_t>(nq, kTile));
-    coarse_scores_kernel<<<grid, 256, 0, res.stream>>>(centers, fq + size_t(q0) * dim_ext, n_lists,
-                                                       nq, dim_ext, alpha, half_scores ? 1 : 0, scores);
-    select_probes_kernel<<<nq, 256, size_t(cap) * 8, res.stream>>>(
-      scores, n_lists, n_probes, cap, probes + size_t(q0) * n_probes,
-      scores_out ? scores_out + size_t(q0) * n_probes : nullptr);
+    launch_exact_gemm<false>(centers, n_lists, fq + size_t(q0) * dim_ext, nq, dim_ext, alpha, half_scores, scores, nullptr,
+                             res.stream);
+    launch_select(scores, nq, n_lists, n_lists, nullptr, 0, n_probes, probes + size_t(q0) * n_probes,
+                  scores_out ? scores_out + size_t(q0) * n_probes : nullptr, res.stream);
     CUDA_TRY(cudaGetLastError());
     res.launches += 2;
   }
 }
 
 void select_rows(raft::resources& res, const float* rows, uint32_t n_rows, uint32_t row_len, uint32_t k,
-                 uint32_t* out_idx, float* out_scores)
+                 uint32_t* out_idx, float* out_scores, const uint32_t* row_ends, uint32_t ends_stride)
 {
   CUVS_EXPECTS(k <= kMaxProbes && k <= row_len, "select_rows: k = %u out of range", k);
   if (n_rows == 0) { return; }
-  uint32_t cap = 2;
-  while (cap < k) { cap <<= 1; }
-  select_probes_kernel<<<n_rows, 256, size_t(cap) * 8, res.stream>>>(rows, row_len, k, cap, out_idx,
-                                                                     out_scores);
-  CUDA_TRY(cudaGetLastError());
+  launch_select(rows, n_rows, row_len, row_len, row_ends, ends_stride, k, out_idx, out_scores, res.stream);
   res.launches++;
 }
 
@@ -313,14 +543,7 @@ void assign_nearest(raft::resources& res, const float* centers, uint32_t n_lists
 {
   if (n_rows == 0) { return; }
   CUDA_TRY(cudaMemsetAsync(best, 0xFF, size_t(n_rows) * 8, res.stream));
-  // grid.y is limited to 65535 blocks of 64 rows
-  const uint32_t max_rows = 65535u * kTile;
-  for (uint32_t r0 = 0; r0 < n_rows; r0 += max_rows) {
-    const uint32_t nr = std::min(max_rows, n_rows - r0);
-    dim3 grid(ceildiv<uint32_t>(n_lists, kTile), ceildiv<uint32_t>(nr, kTile));
-    assign_nearest_kernel<<<grid, 256, 0, res.stream>>>(centers, x_ext + size_t(r0) * dim_ext, n_lists,
-                                                        nr, dim_ext, alpha, best + r0);
-  }
+  launch_exact_gemm<true>(centers, n_lists, x_ext, n_rows, dim_ext, alpha, false, nullptr, best, res.stream);
   unpack_labels_kernel<<<ceildiv<uint32_t>(n_rows, 256), 256, 0, res.stream>>>(best, n_rows, labels);
   CUDA_TRY(cudaGetLastError());
   res.launches += 2;

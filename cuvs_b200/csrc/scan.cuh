@@ -1081,7 +1081,7 @@ __global__ void __launch_bounds__(1024, 1) scan_kernel(const scan_params p)
           valid = id >= 0 && uint64_t(id) < p.filter_nbits && ((p.filter_bits[id >> 5] >> (id & 31)) & 1u);
         }
         if constexpr (kStoreAll) {
-          if (valid) { p.all_scores[size_t(q) * p.max_samples + sample_offset + row] = score; }
+          if (row < n) { p.all_scores[size_t(q) * p.max_samples + sample_offset + row] = valid ? score : INFINITY; }
         } else {
           const uint32_t ord   = float_to_ordered(score);
           const uint64_t key   = (uint64_t(ord) << 32) | (sample_offset + row);
@@ -1267,7 +1267,7 @@ __global__ void __launch_bounds__(256) scan_glut_kernel(const scan_params p)
         valid = id >= 0 && uint64_t(id) < p.filter_nbits && ((p.filter_bits[id >> 5] >> (id & 31)) & 1u);
       }
       if constexpr (kStoreAll) {
-        if (valid) { p.all_scores[size_t(q) * p.max_samples + sample_offset + row] = score; }
+        if (row < n) { p.all_scores[size_t(q) * p.max_samples + sample_offset + row] = valid ? score : INFINITY; }
       } else {
         const uint32_t ord = float_to_ordered(score);
         queue.offer((uint64_t(ord) << 32) | (sample_offset + row), valid && ord <= thr0);

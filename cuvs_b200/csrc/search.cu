@@ -379,12 +379,6 @@ __global__ void small_batch_pairs_kernel(const uint32_t* __restrict__ probes,
   if (lane == 0) { query_kth[q] = kEmptyScore; }
 }
 
-__global__ void fill_u32_kernel(uint32_t* p, size_t n, uint32_t v)
-{
-  size_t i = blockIdx.x * size_t(blockDim.x) + threadIdx.x;
-  if (i < n) { p[i] = v; }
-}
-
 // ------------------------------------------------------------------------------------------------
 // final selection across probes + post-processing
 // ------------------------------------------------------------------------------------------------
@@ -477,12 +471,6 @@ __global__ void translate_selected_kernel(const float* __restrict__ sel_scores,
   }
   neighbors[i] = id;
   distances[i] = postprocess_distance(score, metric, scale);
-}
-
-__global__ void fill_f32_kernel(float* p, size_t n, float v)
-{
-  size_t i = blockIdx.x * size_t(blockDim.x) + threadIdx.x;
-  if (i < n) { p[i] = v; }
 }
 
 // knn_merge_parts (cpp/src/neighbors/detail/knn_merge_parts.cuh:24-97): one warp per query.
@@ -1079,11 +1067,6 @@ void search_any(raft::resources& res, const search_params& params, const index<i
 
     if (stats) { res.stats_mark(ev, 3); }
     // 4. LUT + scan + per-pair top-k
-    if (store_all) {
-      const size_t n_all = size_t(nq) * max_samples;
-      fill_f32_kernel<<<unsigned(ceildiv<size_t>(n_all, 256)), 256, 0, stream>>>(d_all, n_all, INFINITY);
-      res.launches++;
-    }
     {
       scan_params sp{};
       sp.pq_centers     = idx.pq_centers();
@@ -1153,7 +1136,8 @@ void search_any(raft::resources& res, const search_params& params, const index<i
     if (store_all) {
       auto* sel_scores = reinterpret_cast<float*>(d_keys);
       auto* sel_idx    = reinterpret_cast<uint32_t*>(d_keys) + size_t(nq) * k;
-      select_rows(res, d_all, nq, max_samples, k, sel_idx, sel_scores);
+      // (a row of scores ends where the query's last probe does; the scan writes every one of them)
+      select_rows(res, d_all, nq, max_samples, k, sel_idx, sel_scores, d_chunk, n_probes);
       translate_selected_kernel<<<unsigned(ceildiv<uint64_t>(uint64_t(nq) * k, 256)), 256, 0, stream>>>(
         sel_scores, sel_idx, d_probes, d_chunk, idx.row_offsets(), idx.ids(), nq, n_probes, k,
         int(metric), scale, neighbors + size_t(q0) * k, distances + size_t(q0) * k);

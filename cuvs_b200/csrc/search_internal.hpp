@@ -41,9 +41,10 @@ void select_clusters(raft::resources& res, const float* centers, uint32_t n_list
                      uint32_t* probes, float* scores_out, void* workspace, size_t workspace_bytes,
                      bool half_scores = false);
 
-// Per row the k smallest (value, position), ascending (radix select + sort; k <= 4096).
+// Per row the k smallest (value, position), ascending (k <= 4096).  `row_ends` (optional): row r holds only
+// row_ends[(r + 1) * ends_stride - 1] values; results beyond them have a NaN score.
 void select_rows(raft::resources& res, const float* rows, uint32_t n_rows, uint32_t row_len, uint32_t k,
-                 uint32_t* out_idx, float* out_scores);
+                 uint32_t* out_idx, float* out_scores, const uint32_t* row_ends = nullptr, uint32_t ends_stride = 0);
 
 // Tensor-core coarse stage (coarse_tc.cu): same contract and bit-identical probes as
 // select_clusters; `centers_hi/lo` are the TF32 split of `centers`, `cmax` the largest row norm.
