@@ -27,6 +27,7 @@ UNITS = [("resources.cu", "resources.o", []), ("index.cu", "index.o", []),
          ("build.cu", "build.o", []), ("c_api.cu", "c_api.o", []),
          ("no_alloc.cu", "no_alloc.o", []), ("refine.cu", "refine.o", []),
          ("filter_scan.cu", "filter_scan.o", []), ("rescore.cu", "rescore.o", []),
+         ("label_tc.cu", "label_tc.o", []),
          ("dynamic_batching.cu", "dynamic_batching.o", []), ("mg.cu", "mg.o", []),
          ("c_api_mg.cu", "c_api_mg.o", [])]
 UNITS += [("scan_inst.cu", f"scan_{b}.o", [f"-DPQ_BITS={b}"]) for b in (4, 5, 6, 7, 8)]

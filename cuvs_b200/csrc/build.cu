@@ -375,7 +375,281 @@ __global__ void train_codebooks_kernel(const float* __restrict__ resid, uint32_t
 // ------------------------------------------------------------------------------------------------
 // encoder
 // ------------------------------------------------------------------------------------------------
-// One warp per vector (taken in `order`): residual into shared memory, per-subspace argmin over the
+__device__ __forceinline__ uint64_t sub2(uint64_t a, uint64_t b)
+{
+  uint64_t d;
+  asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b)
+{
+  uint64_t d;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c)
+{
+  uint64_t d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
+}
+__device__ __forceinline__ uint64_t dup2(float x)
+{
+  uint64_t v;
+  asm("mov.b64 %0, {%1, %1};" : "=l"(v) : "f"(x));
+  return v;
+}
+__device__ __forceinline__ float lo2(uint64_t v) { return __uint_as_float(uint32_t(v)); }
+__device__ __forceinline__ float hi2(uint64_t v) { return __uint_as_float(uint32_t(v >> 32)); }
+__device__ __forceinline__ float min3(float a, float b, float c)
+{
+  float d;
+  asm("min.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
+  return d;
+}
+
+// Differences of the rows (taken in `order`) to the centres of their lists.  One thread per component.
+__global__ void difference_kernel(const float* __restrict__ x_ext, const uint32_t* __restrict__ labels,
+                                  const uint32_t* __restrict__ order, const float* __restrict__ centers, uint32_t n, uint32_t dim,
+                                  uint32_t dim_ext, float* __restrict__ out)
+{
+  const uint64_t t = blockIdx.x * uint64_t(blockDim.x) + threadIdx.x;
+  if (t >= uint64_t(n) * dim) { return; }
+  const uint32_t i = uint32_t(t / dim), k = uint32_t(t - uint64_t(i) * dim);
+  const uint32_t row = order ? order[i] : i;
+  out[t] = __fsub_rn(x_ext[size_t(row) * dim_ext + k], centers[size_t(labels[row]) * dim_ext + k]);
+}
+
+// Codes of per-subspace codebooks, one byte each: codes[i * out_stride + j] = the codeword of subspace j with the smallest
+// squared distance (a fused multiply-add chain over its components), lowest code on ties.  Vector i is row order[i]
+// of x, minus the centre of its list where `centers` is given.
+// What bounds it: the FMA pipe, at four operations per vector and codeword of two components.  Thread = four vectors, so that a
+// codeword read from shared memory (broadcast) serves four; two codewords per instruction (fp32x2); the minimum of
+// eight distances is compared with the best so far, and only the winning eight are looked at one by one.
+// One warp per vector with the codebook read through L1 took 24.8 ms for 1 M rows of 48 x 8 bits.
+// kLen: components per subspace, 0 = any number.
+constexpr uint32_t kEncVecs = 4;
+template <uint32_t kLen>
+__host__ __device__ constexpr uint32_t enc_subspaces() { return kLen == 0 || kLen > 4 ? 1u : (kLen > 2 ? 2u : 4u); }
+template <uint32_t kLen>
+__global__ void __launch_bounds__(256)
+encode_subspaces_kernel(const float* __restrict__ x, uint32_t x_stride, const uint32_t* __restrict__ order,
+                        const uint32_t* __restrict__ labels, const float* __restrict__ centers, uint32_t c_stride, uint32_t n,
+                        const float* __restrict__ pq_centers, uint32_t pq_dim, uint32_t len_rt, uint32_t book, int in_smem,
+                        uint8_t* __restrict__ codes, uint32_t out_stride)
+{
+  extern __shared__ __align__(16) float s_book[];
+  constexpr uint32_t kSub = enc_subspaces<kLen>();
+  constexpr uint32_t kEnt = kLen == 0 || kLen > 4 ? 4u : 8u;  // codewords per step
+  const uint32_t len = kLen > 0 ? kLen : len_rt;
+  const uint32_t j0 = blockIdx.y * kSub, nj = min(kSub, pq_dim - j0);
+  if (in_smem) {
+    const float4* src = reinterpret_cast<const float4*>(pq_centers + size_t(j0) * len * book);
+    float4* dst       = reinterpret_cast<float4*>(s_book);
+    for (uint32_t i = threadIdx.x; i < nj * len * book / 4; i += 256) { dst[i] = __ldg(src + i); }
+    __syncthreads();
+  }
+  const float* book0 = in_smem ? s_book : pq_centers + size_t(j0) * len * book;
+  const float* xr[kEncVecs];
+  const float* cr[kEncVecs];
+  uint32_t code[kEncVecs];
+  const uint32_t i0 = blockIdx.x * (256u * kEncVecs) + threadIdx.x;
+#pragma unroll
+  for (uint32_t v = 0; v < kEncVecs; v++) {
+    const uint32_t i   = min(i0 + v * 256u, n - 1u);
+    const uint32_t row = order ? order[i] : i;
+    xr[v]              = x + size_t(row) * x_stride + j0 * len;
+    cr[v]              = centers ? centers + size_t(labels[row]) * c_stride + j0 * len : nullptr;
+    code[v]            = 0u;
+  }
+  auto component = [&](uint32_t v, uint32_t k) {
+    const float a = __ldg(xr[v] + k);
+    return centers ? __fsub_rn(a, __ldg(cr[v] + k)) : a;
+  };
+  // the first of kEnt codewords at `b` whose distance is the smallest one found
+  auto pick = [&](const float* b, float best, auto&& comp) {
+    uint32_t first = 0;
+    for (int e = int(kEnt) - 1; e >= 0; e--) {
+      float d2 = 0.0f;
+      for (uint32_t k = 0; k < len; k++) {
+        const float t = __fsub_rn(comp(k), b[size_t(k) * book + e]);
+        d2            = __fmaf_rn(t, t, d2);
+      }
+      if (d2 == best) { first = uint32_t(e); }
+    }
+    return first;
+  };
+#pragma unroll
+  for (uint32_t s = 0; s < kSub; s++) {
+    if (s >= nj) { break; }
+    const float* bk = book0 + size_t(s) * len * book;
+    float best[kEncVecs];
+    uint32_t at[kEncVecs];
+#pragma unroll
+    for (uint32_t v = 0; v < kEncVecs; v++) {
+      best[v] = INFINITY;
+      at[v]   = 0u;
+    }
+    auto reduce = [&](uint32_t v, const uint64_t (&d)[kEnt / 2], uint32_t b0) {
+      float m = min3(lo2(d[0]), hi2(d[0]), fminf(lo2(d[1]), hi2(d[1])));
+      if constexpr (kEnt == 8) {
+        m = min3(m, lo2(d[2]), hi2(d[2]));
+        m = min3(m, lo2(d[3]), hi2(d[3]));
+      }
+      if (m < best[v]) {
+        best[v] = m;
+        at[v]   = b0;
+      }
+    };
+    if constexpr (kLen > 0) {
+      float r[kEncVecs][kLen];
+#pragma unroll
+      for (uint32_t v = 0; v < kEncVecs; v++) {
+#pragma unroll
+        for (uint32_t k = 0; k < kLen; k++) { r[v][k] = component(v, s * kLen + k); }
+      }
+#pragma unroll 1
+      for (uint32_t b0 = 0; b0 < book; b0 += kEnt) {
+        uint64_t c[kLen][kEnt / 2];
+#pragma unroll
+        for (uint32_t k = 0; k < kLen; k++) {
+#pragma unroll
+          for (uint32_t e = 0; e < kEnt / 4; e++) {
+            const ulonglong2 y = *reinterpret_cast<const ulonglong2*>(bk + k * book + b0 + 4 * e);
+            c[k][2 * e]        = y.x;
+            c[k][2 * e + 1]    = y.y;
+          }
+        }
+#pragma unroll
+        for (uint32_t v = 0; v < kEncVecs; v++) {
+          uint64_t d[kEnt / 2];
+#pragma unroll
+          for (uint32_t k = 0; k < kLen; k++) {
+            const uint64_t rr = dup2(r[v][k]);
+#pragma unroll
+            for (uint32_t e = 0; e < kEnt / 2; e++) {
+              const uint64_t t = sub2(rr, c[k][e]);
+              d[e]             = k == 0 ? mul2(t, t) : fma2(t, t, d[e]);  // the chain starts from +0
+            }
+          }
+          reduce(v, d, b0);
+        }
+      }
+#pragma unroll
+      for (uint32_t v = 0; v < kEncVecs; v++) {
+        // (no finite distance at all: code 0)
+        if (best[v] < INFINITY) {
+          uint32_t first = 0;
+#pragma unroll
+          for (int e = int(kEnt) - 1; e >= 0; e--) {
+            float d2 = 0.0f;
+#pragma unroll
+            for (uint32_t k = 0; k < kLen; k++) {
+              const float t = __fsub_rn(r[v][k], bk[k * book + at[v] + e]);
+              d2            = __fmaf_rn(t, t, d2);
+            }
+            if (d2 == best[v]) { first = uint32_t(e); }
+          }
+          code[v] |= (at[v] + first) << (8u * s);
+        }
+      }
+    } else {
+      for (uint32_t b0 = 0; b0 < book; b0 += kEnt) {
+        uint64_t d[kEncVecs][kEnt / 2];
+#pragma unroll
+        for (uint32_t v = 0; v < kEncVecs; v++) { d[v][0] = d[v][1] = 0ull; }
+        for (uint32_t k = 0; k < len; k++) {
+          const ulonglong2 y = *reinterpret_cast<const ulonglong2*>(bk + size_t(k) * book + b0);
+#pragma unroll
+          for (uint32_t v = 0; v < kEncVecs; v++) {
+            const uint64_t rr = dup2(component(v, k));
+            const uint64_t t0 = sub2(rr, y.x), t1 = sub2(rr, y.y);
+            d[v][0] = fma2(t0, t0, d[v][0]);
+            d[v][1] = fma2(t1, t1, d[v][1]);
+          }
+        }
+#pragma unroll
+        for (uint32_t v = 0; v < kEncVecs; v++) { reduce(v, d[v], b0); }
+      }
+#pragma unroll
+      for (uint32_t v = 0; v < kEncVecs; v++) {
+        if (best[v] < INFINITY) { code[v] = at[v] + pick(bk + at[v], best[v], [&](uint32_t k) { return component(v, k); }); }
+      }
+    }
+  }
+#pragma unroll
+  for (uint32_t v = 0; v < kEncVecs; v++) {
+    const uint32_t i = i0 + v * 256u;
+    if (i >= n) { continue; }
+    uint8_t* o = codes + size_t(i) * out_stride + j0;
+    if (kSub == 4 && nj == 4 && (reinterpret_cast<uintptr_t>(o) & 3u) == 0) {
+      *reinterpret_cast<uint32_t*>(o) = code[v];
+    } else {
+      for (uint32_t s = 0; s < nj; s++) { o[s] = uint8_t(code[v] >> (8u * s)); }
+    }
+  }
+}
+
+// Byte codes of vectors taken in `order` -> interleaved list slots (and ids).  A warp handles 32 vectors and one 16-byte
+// piece at a time: neighbours in a list are neighbours in the warp, so its stores are runs of 16-byte pieces.
+__global__ void place_interleaved_kernel(const uint8_t* __restrict__ codes, const uint32_t* __restrict__ labels,
+                                         const uint32_t* __restrict__ order, const uint32_t* __restrict__ slots, uint32_t n,
+                                         uint32_t pq_dim, uint32_t bits, uint32_t n_pieces, const uint64_t* __restrict__ row_off,
+                                         uint8_t* __restrict__ list_codes, int64_t* __restrict__ ids_out,
+                                         const int64_t* __restrict__ src_ids, int64_t id_base)
+{
+  const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, n_warps = blockDim.x >> 5;
+  const uint32_t i = blockIdx.x * 32u + lane;
+  if (i >= n) { return; }
+  const uint32_t row  = order ? order[i] : i;
+  const uint64_t arow = row_off[labels[row]] + slots[i];
+  const uint8_t* src  = codes + size_t(i) * pq_dim;
+  const uint32_t cpp  = 128u / bits;
+  for (uint32_t p = warp; p < n_pieces; p += n_warps) {
+    uint32_t w[4] = {0u, 0u, 0u, 0u};
+    if (bits == 8u && p * 16u + 16u <= pq_dim && pq_dim % 16u == 0u) {
+      const uint4 v = *reinterpret_cast<const uint4*>(src + p * 16u);
+      w[0] = v.x; w[1] = v.y; w[2] = v.z; w[3] = v.w;
+    } else {
+      const uint32_t nc = min(cpp, pq_dim - p * cpp);
+      for (uint32_t t = 0; t < nc; t++) {
+        const uint32_t code = src[p * cpp + t], bit = t * bits;
+        w[bit >> 5] |= code << (bit & 31u);
+        if ((bit & 31u) + bits > 32u) { w[(bit >> 5) + 1u] |= code >> (32u - (bit & 31u)); }
+      }
+    }
+    *reinterpret_cast<uint4*>(list_codes + (((arow >> 5) * n_pieces + p) * 32u + (arow & 31u)) * 16u) = make_uint4(w[0], w[1], w[2], w[3]);
+  }
+  if (warp == 0) { ids_out[arow] = src_ids ? src_ids[row] : id_base + int64_t(row); }
+}
+
+// Byte codes -> rows of a bit stream: plain output rows, or slots of FLAT lists (row_off given).  One thread per byte.
+__global__ void place_flat_kernel(const uint8_t* __restrict__ codes, const uint32_t* __restrict__ labels,
+                                  const uint32_t* __restrict__ order, const uint32_t* __restrict__ slots, uint32_t n,
+                                  uint32_t pq_dim, uint32_t bits, uint32_t row_bytes, const uint64_t* __restrict__ row_off,
+                                  uint8_t* __restrict__ out, int64_t* __restrict__ ids_out,
+                                  const int64_t* __restrict__ src_ids, int64_t id_base)
+{
+  const uint64_t t = blockIdx.x * uint64_t(blockDim.x) + threadIdx.x;
+  if (t >= uint64_t(n) * row_bytes) { return; }
+  const uint32_t i = uint32_t(t / row_bytes), byte = uint32_t(t - uint64_t(i) * row_bytes);
+  const uint32_t row = order ? order[i] : i;
+  const uint8_t* src = codes + size_t(i) * pq_dim;
+  uint32_t v         = 0;
+  for (uint32_t j = (byte * 8u) / bits; j < pq_dim && j * bits < byte * 8u + 8u; j++) {
+    const int shift     = int(j * bits) - int(byte * 8u);
+    const uint32_t code = src[j];
+    v |= shift >= 0 ? (code << shift) : (code >> (-shift));
+  }
+  uint64_t at = row;
+  if (row_off) {
+    at = row_off[labels[row]] + slots[i];
+    if (byte == 0) { ids_out[at] = src_ids ? src_ids[row] : id_base + int64_t(row); }
+  }
+  out[at * row_bytes + byte] = uint8_t(v & 0xFFu);
+}
+
+// Codebooks per cluster: one warp per vector (taken in `order`): residual into shared memory, per-subspace argmin over the
 // codebook split across lanes, then the lanes pack the codes.
 //   interleaved != 0: write into the list arena at row (row_off[label] + slot[i]); ids too.
 //   interleaved == 0: write a flat little-endian bit stream of ceil(pq_dim*bits/8) bytes per vector.
@@ -383,7 +657,7 @@ __global__ void encode_kernel(const float* __restrict__ x_ext, const uint32_t* _
                               const uint32_t* __restrict__ order, const uint32_t* __restrict__ slots,
                               uint32_t n, const float* __restrict__ centers,
                               const float* __restrict__ rot, int identity,
-                              const float* __restrict__ pq_centers, int per_cluster, uint32_t dim,
+                              const float* __restrict__ pq_centers, uint32_t dim,
                               uint32_t dim_ext, uint32_t rot_dim, uint32_t pq_dim, uint32_t len,
                               uint32_t bits, int interleaved, const uint64_t* __restrict__ row_off,
                               uint8_t* __restrict__ codes_out, int64_t* __restrict__ ids_out,
@@ -418,9 +692,8 @@ __global__ void encode_kernel(const float* __restrict__ x_ext, const uint32_t* _
     s_res[r] = acc;
   }
   __syncwarp();
-  const float* pqc0 = per_cluster ? pq_centers + size_t(label) * len * book : pq_centers;
+  const float* pqc = pq_centers + size_t(label) * len * book;
   for (uint32_t j = 0; j < pq_dim; j++) {
-    const float* pqc = pqc0 + (per_cluster ? 0 : size_t(j) * len * book);
     float best       = INFINITY;
     uint32_t best_b  = 0xFFFFFFFFu;
     for (uint32_t b = lane; b < book; b += 32) {
@@ -669,16 +942,10 @@ __global__ void relocate_lists_kernel(const uint8_t* __restrict__ old_codes, con
   for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) { new_ids[new_off[l] + i] = old_ids[old_off[l] + i]; }
 }
 
-__global__ void add_u32_kernel(uint32_t* a, const uint32_t* b, uint32_t n)
-{
-  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) { a[i] += b[i]; }
-}
-
 uint64_t chunk_rows_for(uint32_t dim_ext)
 {
-  const uint64_t budget = 1ull << 30;  // bytes of converted rows per chunk
-  return std::max<uint64_t>(1024, std::min<uint64_t>(1u << 20, budget / (uint64_t(dim_ext) * 4)));
+  const uint64_t budget = 1ull << 29;  // bytes of converted rows per chunk
+  return std::max<uint64_t>(1024, std::min<uint64_t>(1u << 19, budget / (uint64_t(dim_ext) * 4)));
 }
 
 // balanced k-means defaults of the reference (cpp/include/cuvs/cluster/kmeans.hpp:181-204)
@@ -697,65 +964,66 @@ label_ctx labeling_of(DistanceType m)
   return {-2.0f, -0.5f, m == DistanceType::CosineExpanded};
 }
 
-// Labelling of many rows against one set of centres.  Where the shape allows, the tensor-core coarse
-// path does it (probe selection with n_probes = 1: exact rescoring and guard make its answer the
-// defining one, ties to the lowest list id) -- an order of magnitude faster than the SIMT product on
-// the 10^5 .. 10^6 lists of the large configurations; otherwise the SIMT kernel.
+// Labelling of many rows against one set of centres: on the tensor cores (label_tc.cu) where there is enough work to fill
+// them, else by the exact product.  Works in memory that the caller provides, on any number of rows.
 class nearest_labeler {
  public:
-  // `dim`: index of the |c|^2 column of the centre rows (rows carry -0.5 there)
-  nearest_labeler(raft::resources& res, const float* centers, uint32_t n_lists, uint32_t dim, uint32_t dim_ext,
-                  float alpha)
-    : res_(res), centers_(centers), n_lists_(n_lists), dim_ext_(dim_ext), ext_col_(dim), alpha_(alpha)
+  static size_t bytes(const raft::resources& res, uint64_t n_rows, uint32_t n_lists, uint32_t dim)
   {
-    use_tc_ = coarse_tc_usable(n_lists, 1, dim_ext);
-    if (!use_tc_) { return; }
-    const size_t nc = size_t(n_lists) * dim_ext;
-    hi_.resize(nc);
-    lo_.resize(nc);
-    prepare_tc_centers(res.stream, centers, n_lists, dim_ext, ext_col_, hi_.data(), lo_.data(), &cmax_, &ext_scale_);
-    res.launches += 2;
+    const uint32_t batch = batch_of(n_rows);
+    return label_tc_usable(batch, n_lists)
+             ? round_up<size_t>(label_model_bytes(n_lists, dim), 256) + label_workspace_bytes(res, batch, n_lists, dim)
+             : size_t(batch) * 8;
   }
-  // labels[i] = nearest list of row i of x_ext [n_rows, dim_ext]; `best` is scratch of n_rows * 8 bytes
-  void run(const float* x_ext, uint32_t n_rows, uint32_t* labels, unsigned long long* best)
+  // `dim`: index of the |c|^2 column of the centre rows (rows carry -0.5 there); n_rows: the most that run() is given
+  nearest_labeler(raft::resources& res, const float* centers, uint32_t n_lists, uint32_t dim, uint32_t dim_ext,
+                  float alpha, uint64_t n_rows, void* mem)
+    : res_(res), centers_(centers), n_lists_(n_lists), dim_(dim), dim_ext_(dim_ext), batch_(batch_of(n_rows)), alpha_(alpha),
+      use_tc_(label_tc_usable(batch_, n_lists)), mem_(static_cast<char*>(mem))
   {
-    if (!use_tc_) {
-      assign_nearest(res_, centers_, n_lists_, dim_ext_, alpha_, x_ext, n_rows, labels, best);
-      return;
-    }
-    const uint32_t batch = std::min<uint32_t>(n_rows, 16384);
-    const size_t need    = coarse_tc_workspace_bytes(batch, n_lists_, dim_ext_);
-    if (ws_.size() < need) { ws_.resize(need); }
-    for (uint32_t r0 = 0; r0 < n_rows; r0 += batch) {
-      const uint32_t nr = std::min(batch, n_rows - r0);
-      select_clusters_tc(res_, centers_, hi_.data(), lo_.data(), cmax_, n_lists_, dim_ext_, alpha_,
-                         x_ext + size_t(r0) * dim_ext_, nr, 1, labels + r0, nullptr, ws_.data(), ws_.size(), false,
-                         ext_col_, ext_scale_);
+    refresh();
+  }
+  // the centres have changed
+  void refresh()
+  {
+    if (!use_tc_) { return; }
+    prepare_label_model(res_.stream, centers_, n_lists_, dim_, dim_ext_, mem_);
+    res_.launches += 2;
+  }
+  // labels[i] = nearest list of row i of x_ext [n_rows, dim_ext]
+  void run(const float* x_ext, uint64_t n_rows, uint32_t* labels)
+  {
+    for (uint64_t r0 = 0; r0 < n_rows; r0 += batch_) {
+      const uint32_t nr = uint32_t(std::min<uint64_t>(batch_, n_rows - r0));
+      const float* x    = x_ext + r0 * dim_ext_;
+      if (use_tc_) {
+        label_rows_tc(res_, centers_, mem_, n_lists_, dim_, dim_ext_, alpha_, x, nr, labels + r0,
+                      mem_ + round_up<size_t>(label_model_bytes(n_lists_, dim_), 256));
+      } else {
+        assign_nearest(res_, centers_, n_lists_, dim_ext_, alpha_, x, nr, labels + r0, reinterpret_cast<unsigned long long*>(mem_));
+      }
     }
   }
 
  private:
+  static uint32_t batch_of(uint64_t n_rows) { return uint32_t(std::min<uint64_t>(n_rows, 1u << 19)); }
   raft::resources& res_;
   const float* centers_;
-  uint32_t n_lists_, dim_ext_, ext_col_;
+  uint32_t n_lists_, dim_, dim_ext_, batch_;
   float alpha_;
-  bool use_tc_     = false;
-  float cmax_      = 0.0f;
-  float ext_scale_ = 1.0f;
-  dev_array<float> hi_, lo_;
-  dev_array<uint8_t> ws_;
+  bool use_tc_;
+  char* mem_;
 };
 
 // Host rows -> device staging (no-op for device data).
 const void* stage_rows(raft::resources& res, const void* data, elem_t t, uint64_t r0, uint64_t nr,
-                       uint32_t dim, bool on_device, dev_array<uint8_t>& staging)
+                       uint32_t dim, bool on_device, void* staging)
 {
   const size_t es = elem_size(t);
   const char* src = static_cast<const char*>(data) + r0 * dim * es;
   if (on_device) { return src; }
-  if (staging.size() < nr * dim * es) { staging.resize(nr * dim * es); }
-  CUDA_TRY(cudaMemcpyAsync(staging.data(), src, nr * dim * es, cudaMemcpyHostToDevice, res.stream));
-  return staging.data();
+  CUDA_TRY(cudaMemcpyAsync(staging, src, nr * dim * es, cudaMemcpyHostToDevice, res.stream));
+  return staging;
 }
 
 void make_rotation(uint32_t rot_dim, uint32_t dim, bool force_random, std::vector<float>& out)
@@ -789,28 +1057,102 @@ void make_rotation(uint32_t rot_dim, uint32_t dim, bool force_random, std::vecto
   }
 }
 
+// Scratch of launch_encode for up to n vectors: byte codes, and with a rotation the differences before and after it.
+size_t encode_scratch_bytes(const index<int64_t>& idx, uint64_t n)
+{
+  if (idx.codebook_kind() == codebook_gen::PER_CLUSTER) { return 0; }
+  ws_layout lay;
+  lay.add(n * idx.pq_dim());
+  if (!idx.rotation_is_identity()) {
+    lay.add(n * idx.dim() * 4);
+    lay.add(n * idx.rot_dim() * 4);
+  }
+  return lay.total();
+}
+
+// `to_lists`: write slots of the index's lists (and ids); else plain rows of codes_out.
 void launch_encode(raft::resources& res, const index<int64_t>& idx, const float* x_ext,
                    const uint32_t* labels, const uint32_t* order, const uint32_t* slots, uint32_t n,
-                   bool interleaved, uint8_t* codes_out, int64_t* ids_out, const int64_t* src_ids,
-                   int64_t id_base)
+                   bool to_lists, uint8_t* codes_out, int64_t* ids_out, const int64_t* src_ids,
+                   int64_t id_base, void* scratch)
 {
   if (n == 0) { return; }
-  const uint32_t warps = 4;
-  const uint32_t per_warp_floats = round_up<uint32_t>(idx.dim(), 4) + round_up<uint32_t>(idx.rot_dim(), 4) +
-                                   round_up<uint32_t>(idx.pq_dim(), 16) / 4;
-  const size_t smem = size_t(warps) * per_warp_floats * 4;
-  CUVS_EXPECTS(smem <= 48 * 1024, "dim = %u is too large for the encoder", idx.dim());
-  encode_kernel<<<ceildiv(n, warps), warps * 32, smem, res.stream>>>(
-    x_ext, labels, order, slots, n, idx.centers(), idx.rotation_matrix(), idx.rotation_is_identity(),
-    idx.pq_centers(), idx.codebook_kind() == codebook_gen::PER_CLUSTER, idx.dim(), idx.dim_ext(),
-    idx.rot_dim(), idx.pq_dim(), idx.pq_len(), idx.pq_bits(),
-    // 0: rows of a plain output matrix; 1: slots of interleaved lists; 2: slots of flat lists
-    interleaved ? (idx.codes_layout() == list_layout::FLAT ? 2 : 1) : 0, idx.row_offsets(), codes_out,
-    ids_out, src_ids, id_base, ceildiv(idx.pq_dim() * idx.pq_bits(), 8u));
+  const uint32_t row_bytes = ceildiv(idx.pq_dim() * idx.pq_bits(), 8u);
+  const bool flat          = !to_lists || idx.codes_layout() == list_layout::FLAT;
+  if (idx.codebook_kind() == codebook_gen::PER_CLUSTER) {
+    const uint32_t warps = 4;
+    const uint32_t per_warp_floats = round_up<uint32_t>(idx.dim(), 4) + round_up<uint32_t>(idx.rot_dim(), 4) +
+                                     round_up<uint32_t>(idx.pq_dim(), 16) / 4;
+    const size_t smem = size_t(warps) * per_warp_floats * 4;
+    CUVS_EXPECTS(smem <= 48 * 1024, "dim = %u is too large for the encoder", idx.dim());
+    encode_kernel<<<ceildiv(n, warps), warps * 32, smem, res.stream>>>(
+      x_ext, labels, order, slots, n, idx.centers(), idx.rotation_matrix(), idx.rotation_is_identity(),
+      idx.pq_centers(), idx.dim(), idx.dim_ext(), idx.rot_dim(), idx.pq_dim(), idx.pq_len(), idx.pq_bits(),
+      // 0: rows of a plain output matrix; 1: slots of interleaved lists; 2: slots of flat lists
+      to_lists ? (flat ? 2 : 1) : 0, idx.row_offsets(), codes_out, ids_out, src_ids, id_base, row_bytes);
+    CUDA_TRY(cudaGetLastError());
+    res.launches++;
+    return;
+  }
+  const uint32_t dim = idx.dim(), dim_ext = idx.dim_ext(), rot_dim = idx.rot_dim(), len = idx.pq_len();
+  const uint32_t pq_dim = idx.pq_dim(), book = idx.pq_book_size();
+  ws_layout lay;
+  char* ws     = static_cast<char*>(scratch);
+  auto* bytes  = reinterpret_cast<uint8_t*>(ws + lay.add(size_t(n) * pq_dim));
+  // plain rows of 8-bit codes are the byte codes themselves
+  const bool direct = !to_lists && idx.pq_bits() == 8;
+  if (direct) { bytes = codes_out; }
+  const float* x        = x_ext;
+  uint32_t x_stride     = dim_ext;
+  const float* c        = idx.centers();
+  const uint32_t* x_order = order;
+  if (!idx.rotation_is_identity()) {
+    auto* diff  = reinterpret_cast<float*>(ws + lay.add(size_t(n) * dim * 4));
+    auto* resid = reinterpret_cast<float*>(ws + lay.add(size_t(n) * rot_dim * 4));
+    difference_kernel<<<unsigned(ceildiv<uint64_t>(uint64_t(n) * dim, 256)), 256, 0, res.stream>>>(
+      x_ext, labels, order, idx.centers(), n, dim, dim_ext, diff);
+    exact_rows_product(res, idx.rotation_matrix(), rot_dim, diff, n, dim, resid);
+    res.launches++;
+    x        = resid;
+    x_stride = rot_dim;
+    c        = nullptr;
+    x_order  = nullptr;
+  }
+  auto go = [&](auto lenc) {
+    constexpr uint32_t kLen = decltype(lenc)::value;
+    constexpr uint32_t kSub = enc_subspaces<kLen>();
+    const size_t need  = size_t(kSub) * len * book * 4;
+    const bool in_smem = need <= 96 * 1024;
+    if (in_smem) { ensure_dynamic_smem(reinterpret_cast<const void*>(encode_subspaces_kernel<kLen>), need); }
+    const dim3 grid(ceildiv(n, 256u * kEncVecs), ceildiv(pq_dim, kSub));
+    encode_subspaces_kernel<kLen><<<grid, 256, in_smem ? need : 0, res.stream>>>(
+      x, x_stride, x_order, labels, c, dim_ext, n, idx.pq_centers(), pq_dim, len, book, in_smem, bytes, pq_dim);
+    CUDA_TRY(cudaGetLastError());
+  };
+  using std::integral_constant;
+  switch (len) {
+    case 1: go(integral_constant<uint32_t, 1>{}); break;
+    case 2: go(integral_constant<uint32_t, 2>{}); break;
+    case 3: go(integral_constant<uint32_t, 3>{}); break;
+    case 4: go(integral_constant<uint32_t, 4>{}); break;
+    case 8: go(integral_constant<uint32_t, 8>{}); break;
+    default: go(integral_constant<uint32_t, 0>{});
+  }
+  res.launches++;
+  if (direct) { return; }
+  if (flat) {
+    place_flat_kernel<<<unsigned(ceildiv<uint64_t>(uint64_t(n) * row_bytes, 256)), 256, 0, res.stream>>>(
+      bytes, labels, order, slots, n, pq_dim, idx.pq_bits(), row_bytes, to_lists ? idx.row_offsets() : nullptr, codes_out,
+      ids_out, src_ids, id_base);
+  } else {
+    const uint32_t warps = std::min<uint32_t>(8, idx.n_pieces());
+    place_interleaved_kernel<<<ceildiv(n, 32u), warps * 32, 0, res.stream>>>(bytes, labels, order, slots, n, pq_dim, idx.pq_bits(),
+                                                                            idx.n_pieces(), idx.row_offsets(), codes_out,
+                                                                            ids_out, src_ids, id_base);
+  }
   CUDA_TRY(cudaGetLastError());
   res.launches++;
 }
-
 
 // Re-create the arenas for `new_sizes`, keeping the first min(old, new) rows (codes and ids) of every list.
 void resize_lists(raft::resources& res, index<int64_t>* idx, const std::vector<uint32_t>& new_sizes)
@@ -823,6 +1165,10 @@ void resize_lists(raft::resources& res, index<int64_t>* idx, const std::vector<u
     keep[l] = std::min(idx->host_list_sizes()[l], new_sizes[l]);
     any |= keep[l] > 0;
   }
+  if (!any) {
+    idx->allocate_lists(new_sizes, stream);
+    return;
+  }
   dev_array<uint8_t> old_codes = std::move(idx->codes_);
   dev_array<int64_t> old_ids   = std::move(idx->ids_);
   dev_array<uint64_t> old_off(size_t(n_lists) + 1);
@@ -830,13 +1176,11 @@ void resize_lists(raft::resources& res, index<int64_t>* idx, const std::vector<u
   CUDA_TRY(cudaMemcpyAsync(old_off.data(), idx->row_offsets(), (size_t(n_lists) + 1) * 8, cudaMemcpyDeviceToDevice, stream));
   CUDA_TRY(cudaMemcpyAsync(keep_d.data(), keep.data(), size_t(n_lists) * 4, cudaMemcpyHostToDevice, stream));
   idx->allocate_lists(new_sizes, stream);
-  if (any) {
-    relocate_lists_kernel<<<n_lists, 128, 0, stream>>>(old_codes.data(), old_ids.data(), old_off.data(),
-                                                       keep_d.data(), idx->row_offsets(),
-                                                       idx->list_row_bytes(), idx->codes(), idx->ids());
-    CUDA_TRY(cudaGetLastError());
-    res.launches++;
-  }
+  relocate_lists_kernel<<<n_lists, 128, 0, stream>>>(old_codes.data(), old_ids.data(), old_off.data(),
+                                                     keep_d.data(), idx->row_offsets(),
+                                                     idx->list_row_bytes(), idx->codes(), idx->ids());
+  CUDA_TRY(cudaGetLastError());
+  res.launches++;
   res.sync();  // the old arenas are released on return
 }
 
@@ -888,6 +1232,7 @@ void set_model(raft::resources& res, index<int64_t>* idx, const float* pq_center
                            size_t(idx->rot_dim()) * idx->dim() * 4, cudaMemcpyDefault, res.stream));
   res.sync();
   idx->allocate_lists(std::vector<uint32_t>(idx->n_lists(), 0), res.stream);
+  idx->recompute_model_state(res.stream);
 }
 
 namespace {
@@ -1023,6 +1368,7 @@ void extend_list(raft::resources& res, index<int64_t>* idx, const void* new_vect
   const label_ctx lc = labeling_of(idx->metric());
   dev_array<float> x_ext(size_t(n_rows) * idx->dim_ext());
   dev_array<uint32_t> labels(n_rows), slots(n_rows);
+  dev_array<uint8_t> scratch(encode_scratch_bytes(*idx, n_rows));
   to_float_ext(res, new_vectors, dtype, n_rows, 1, idx->dim(), idx->dim_ext(), lc.pad, lc.normalize,
                x_ext.data());
   fill_u32_kernel<<<ceildiv(n_rows, 256u), 256, 0, res.stream>>>(labels.data(), n_rows, label);
@@ -1031,7 +1377,7 @@ void extend_list(raft::resources& res, index<int64_t>* idx, const void* new_vect
   res.launches += 3;
   // ids were written by extend_list_prepare: the encoder gets the same array, so it rewrites them
   launch_encode(res, *idx, x_ext.data(), labels.data(), nullptr, slots.data(), n_rows, true, idx->codes(),
-                idx->ids(), new_indices, 0);
+                idx->ids(), new_indices, 0, scratch.data());
   res.sync();
 }
 
@@ -1071,25 +1417,54 @@ void extend_any(raft::resources& res, const void* new_vectors, elem_t dtype, int
   const label_ctx lc   = labeling_of(idx->metric());
   const uint64_t chunk = std::min<uint64_t>(n, chunk_rows_for(dim_ext));
 
-  dev_array<uint8_t> staging;
-  dev_array<float> x_ext(chunk * dim_ext);
-  dev_array<unsigned long long> best(chunk);
-  dev_array<uint32_t> labels(n);
-  dev_array<uint32_t> counts(n_lists);
-  CUDA_TRY(cudaMemsetAsync(counts.data(), 0, size_t(n_lists) * 4, stream));
+  int end_bit = 1;
+  while ((1ull << end_bit) < n_lists) { end_bit++; }
+  size_t cub_bytes = 0;
+  cub::DeviceRadixSort::SortPairs(nullptr, cub_bytes, static_cast<uint32_t*>(nullptr), static_cast<uint32_t*>(nullptr),
+                                  static_cast<uint32_t*>(nullptr), static_cast<uint32_t*>(nullptr), int(chunk), 0, end_bit, stream);
+  // one grow-only scratch buffer of the handle for everything below (a dozen allocations and releases per call took as
+  // long as the work on 300,000 rows)
+  ws_layout lay;
+  const size_t row_bytes = size_t(dim) * elem_size(dtype);
+  const size_t o_x       = lay.add(chunk * dim_ext * 4);
+  const size_t o_labels  = lay.add(n * 4);
+  const size_t o_counts  = lay.add(size_t(n_lists) * 4);
+  const size_t o_fill    = lay.add(size_t(n_lists) * 4);
+  const size_t o_iota    = lay.add(chunk * 4);
+  const size_t o_order   = lay.add(chunk * 4);
+  const size_t o_sorted  = lay.add(chunk * 4);
+  const size_t o_slots   = lay.add(chunk * 4);
+  const size_t o_cub     = lay.add(cub_bytes);
+  const size_t o_staging = lay.add(on_device ? 0 : chunk * row_bytes);
+  const size_t o_ids     = lay.add(on_device || !new_indices ? 0 : chunk * 8);
+  // (labelling and encoding take turns)
+  const size_t o_work    = lay.add(std::max(nearest_labeler::bytes(res, chunk, n_lists, dim), encode_scratch_bytes(*idx, chunk)));
+  res.scratch.reserve(lay.total());
+  char* ws        = res.scratch.base();
+  auto* x_ext     = reinterpret_cast<float*>(ws + o_x);
+  auto* labels    = reinterpret_cast<uint32_t*>(ws + o_labels);
+  auto* counts    = reinterpret_cast<uint32_t*>(ws + o_counts);
+  auto* fill      = reinterpret_cast<uint32_t*>(ws + o_fill);  // rows already placed in each list
+  auto* iota      = reinterpret_cast<uint32_t*>(ws + o_iota);
+  auto* order     = reinterpret_cast<uint32_t*>(ws + o_order);
+  auto* sorted    = reinterpret_cast<uint32_t*>(ws + o_sorted);
+  auto* slots     = reinterpret_cast<uint32_t*>(ws + o_slots);
+  void* staging   = ws + o_staging;
+  CUDA_TRY(cudaMemsetAsync(counts, 0, size_t(n_lists) * 4, stream));
 
   // pass 1: labels + histogram
-  nearest_labeler labeler(res, idx->centers(), n_lists, dim, dim_ext, lc.alpha);
-  for (uint64_t r0 = 0; r0 < n; r0 += chunk) {
-    const uint64_t nr = std::min(chunk, n - r0);
-    const void* src   = stage_rows(res, new_vectors, dtype, r0, nr, dim, on_device, staging);
-    to_float_ext(res, src, dtype, nr, 1, dim, dim_ext, lc.pad, lc.normalize, x_ext.data());
-    labeler.run(x_ext.data(), uint32_t(nr), labels.data() + r0, best.data());
-    if (!on_device) { res.sync(); }
+  {
+    nearest_labeler labeler(res, idx->centers(), n_lists, dim, dim_ext, lc.alpha, chunk, ws + o_work);
+    for (uint64_t r0 = 0; r0 < n; r0 += chunk) {
+      const uint64_t nr = std::min(chunk, n - r0);
+      const void* src   = stage_rows(res, new_vectors, dtype, r0, nr, dim, on_device, staging);
+      to_float_ext(res, src, dtype, nr, 1, dim, dim_ext, lc.pad, lc.normalize, x_ext);
+      labeler.run(x_ext, nr, labels + r0);
+    }
   }
-  histogram_kernel<<<unsigned(ceildiv<uint64_t>(n, 256)), 256, 0, stream>>>(labels.data(), n, counts.data());
+  histogram_kernel<<<unsigned(ceildiv<uint64_t>(n, 256)), 256, 0, stream>>>(labels, n, counts);
   std::vector<uint32_t> h_counts(n_lists);
-  CUDA_TRY(cudaMemcpyAsync(h_counts.data(), counts.data(), size_t(n_lists) * 4, cudaMemcpyDeviceToHost, stream));
+  CUDA_TRY(cudaMemcpyAsync(h_counts.data(), counts, size_t(n_lists) * 4, cudaMemcpyDeviceToHost, stream));
   res.sync();
 
   // new arenas, old payload moved over
@@ -1102,39 +1477,32 @@ void extend_any(raft::resources& res, const void* new_vectors, elem_t dtype, int
   resize_lists(res, idx, new_sizes);
 
   // pass 2: per chunk, order rows by list (stable), give each its slot, encode
-  dev_array<uint32_t> fill(n_lists);  // rows already placed in each list
-  CUDA_TRY(cudaMemcpyAsync(fill.data(), old_sizes.data(), size_t(n_lists) * 4, cudaMemcpyHostToDevice, stream));
-  dev_array<uint32_t> iota(chunk), order(chunk), sorted_labels(chunk), slots(chunk), chunk_counts(n_lists);
-  size_t cub_bytes = 0;
-  int end_bit      = 1;
-  while ((1ull << end_bit) < n_lists) { end_bit++; }
-  cub::DeviceRadixSort::SortPairs(nullptr, cub_bytes, labels.data(), sorted_labels.data(), iota.data(),
-                                  order.data(), int(chunk), 0, end_bit, stream);
-  dev_array<uint8_t> cub_tmp(cub_bytes);
+  CUDA_TRY(cudaMemcpyAsync(fill, old_sizes.data(), size_t(n_lists) * 4, cudaMemcpyHostToDevice, stream));
   for (uint64_t r0 = 0; r0 < n; r0 += chunk) {
     const uint32_t nr = uint32_t(std::min(chunk, n - r0));
-    const void* src   = stage_rows(res, new_vectors, dtype, r0, nr, dim, on_device, staging);
-    to_float_ext(res, src, dtype, nr, 1, dim, dim_ext, lc.pad, lc.normalize, x_ext.data());
-    iota_kernel<<<ceildiv(nr, 256u), 256, 0, stream>>>(iota.data(), nr);
-    cub::DeviceRadixSort::SortPairs(cub_tmp.data(), cub_bytes, labels.data() + r0, sorted_labels.data(),
-                                    iota.data(), order.data(), int(nr), 0, end_bit, stream);
-    slots_kernel<<<ceildiv(nr, 256u), 256, 0, stream>>>(sorted_labels.data(), nr, fill.data(), slots.data());
-    const int64_t* ids_chunk = new_indices ? new_indices + r0 : nullptr;
-    dev_array<int64_t> ids_staging;
-    if (new_indices && !on_device) {
-      ids_staging.resize(nr);
-      CUDA_TRY(cudaMemcpyAsync(ids_staging.data(), new_indices + r0, size_t(nr) * 8, cudaMemcpyHostToDevice, stream));
-      ids_chunk = ids_staging.data();
+    if (n > chunk) {  // (else the rows of pass 1 are still there)
+      const void* src = stage_rows(res, new_vectors, dtype, r0, nr, dim, on_device, staging);
+      to_float_ext(res, src, dtype, nr, 1, dim, dim_ext, lc.pad, lc.normalize, x_ext);
     }
-    launch_encode(res, *idx, x_ext.data(), labels.data() + r0, order.data(), slots.data(), nr, true,
-                  idx->codes(), idx->ids(), ids_chunk, int64_t(r0));
-    CUDA_TRY(cudaMemsetAsync(chunk_counts.data(), 0, size_t(n_lists) * 4, stream));
-    histogram_kernel<<<ceildiv(nr, 256u), 256, 0, stream>>>(labels.data() + r0, nr, chunk_counts.data());
-    add_u32_kernel<<<ceildiv(n_lists, 256u), 256, 0, stream>>>(fill.data(), chunk_counts.data(), n_lists);
+    iota_kernel<<<ceildiv(nr, 256u), 256, 0, stream>>>(iota, nr);
+    cub::DeviceRadixSort::SortPairs(ws + o_cub, cub_bytes, labels + r0, sorted, iota, order, int(nr), 0, end_bit, stream);
+    slots_kernel<<<ceildiv(nr, 256u), 256, 0, stream>>>(sorted, nr, fill, slots);
+    const int64_t* ids_chunk = new_indices ? new_indices + r0 : nullptr;
+    if (new_indices && !on_device) {
+      CUDA_TRY(cudaMemcpyAsync(ws + o_ids, new_indices + r0, size_t(nr) * 8, cudaMemcpyHostToDevice, stream));
+      ids_chunk = reinterpret_cast<const int64_t*>(ws + o_ids);
+    }
+    launch_encode(res, *idx, x_ext, labels + r0, order, slots, nr, true, idx->codes(), idx->ids(), ids_chunk, int64_t(r0),
+                  ws + o_work);
+    if (r0 + chunk < n) {
+      // rows of the chunk are placed
+      histogram_kernel<<<ceildiv(nr, 256u), 256, 0, stream>>>(labels + r0, nr, fill);
+      res.launches++;
+    }
     CUDA_TRY(cudaGetLastError());
-    res.launches += 5;
-    res.sync();  // staging buffers are reused by the next chunk
+    res.launches += 3;
   }
+  res.sync();
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -1150,18 +1518,23 @@ void transform_any(raft::resources& res, const index<int64_t>& idx, const void* 
   const label_ctx lc   = labeling_of(idx.metric());
   const uint64_t chunk = std::min<uint64_t>(n, chunk_rows_for(dim_ext));
   const uint32_t flat  = ceildiv(idx.pq_dim() * idx.pq_bits(), 8u);
-  dev_array<float> x_ext(chunk * dim_ext);
-  dev_array<unsigned long long> best(chunk);
-  nearest_labeler labeler(res, idx.centers(), idx.n_lists(), dim, dim_ext, lc.alpha);
+  ws_layout lay;
+  const size_t o_x     = lay.add(chunk * dim_ext * 4);
+  const size_t o_label = lay.add(nearest_labeler::bytes(res, chunk, idx.n_lists(), dim));
+  const size_t o_enc   = lay.add(encode_scratch_bytes(idx, chunk));
+  res.scratch.reserve(lay.total());
+  char* ws    = res.scratch.base();
+  auto* x_ext = reinterpret_cast<float*>(ws + o_x);
+  nearest_labeler labeler(res, idx.centers(), idx.n_lists(), dim, dim_ext, lc.alpha, chunk, ws + o_label);
   for (uint64_t r0 = 0; r0 < n; r0 += chunk) {
     const uint32_t nr = uint32_t(std::min(chunk, n - r0));
     const char* src   = static_cast<const char*>(dataset) + r0 * dim * elem_size(dtype);
-    to_float_ext(res, src, dtype, nr, 1, dim, dim_ext, lc.pad, lc.normalize, x_ext.data());
-    labeler.run(x_ext.data(), nr, out_labels + r0, best.data());
-    launch_encode(res, idx, x_ext.data(), out_labels + r0, nullptr, nullptr, nr, false,
-                  out_codes + r0 * flat, nullptr, nullptr, 0);
-    res.sync();
+    to_float_ext(res, src, dtype, nr, 1, dim, dim_ext, lc.pad, lc.normalize, x_ext);
+    labeler.run(x_ext, nr, out_labels + r0);
+    launch_encode(res, idx, x_ext, out_labels + r0, nullptr, nullptr, nr, false, out_codes + r0 * flat, nullptr, nullptr, 0,
+                  ws + o_enc);
   }
+  res.sync();
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -1205,16 +1578,17 @@ void build_any(raft::resources& res, const index_params& params, const void* dat
 
   // ---- coarse k-means ----
   dev_array<uint32_t> labels(n_train);
-  dev_array<unsigned long long> best(n_train);
+  dev_array<uint8_t> label_mem(nearest_labeler::bytes(res, n_train, n_lists, dim));
   dev_array<float> sums(size_t(n_lists) * dim);
   dev_array<uint32_t> counts(n_lists);
   init_centers_kernel<<<n_lists, 128, 0, stream>>>(train.data(), n_train, n_lists, dim_ext, idx.centers());
   center_norms_kernel<<<ceildiv(n_lists, 128u), 128, 0, stream>>>(idx.centers(), n_lists, dim, dim_ext);
   res.launches += 2;
   const uint32_t iters = std::max<uint32_t>(1, params.kmeans_n_iters);
+  nearest_labeler labeler(res, idx.centers(), n_lists, dim, dim_ext, lc.alpha, n_train, label_mem.data());
   for (uint32_t it = 0; it < iters; it++) {
-    nearest_labeler(res, idx.centers(), n_lists, dim, dim_ext, lc.alpha)
-      .run(train.data(), uint32_t(n_train), labels.data(), best.data());
+    labeler.refresh();
+    labeler.run(train.data(), n_train, labels.data());
     CUDA_TRY(cudaMemsetAsync(sums.data(), 0, sums.size() * 4, stream));
     CUDA_TRY(cudaMemsetAsync(counts.data(), 0, size_t(n_lists) * 4, stream));
     accumulate_kernel<<<unsigned(ceildiv<uint64_t>(n_train * 32, 256)), 256, 0, stream>>>(
@@ -1262,8 +1636,8 @@ void build_any(raft::resources& res, const index_params& params, const void* dat
       }
     }
   }
-  nearest_labeler(res, idx.centers(), n_lists, dim, dim_ext, lc.alpha)
-    .run(train.data(), uint32_t(n_train), labels.data(), best.data());
+  labeler.refresh();
+  labeler.run(train.data(), n_train, labels.data());
 
   // ---- rotation, rotated centers ----
   {
@@ -1275,7 +1649,8 @@ void build_any(raft::resources& res, const index_params& params, const void* dat
   rotate_centers_kernel<<<unsigned(ceildiv<uint64_t>(uint64_t(n_lists) * rot_dim, 256)), 256, 0, stream>>>(
     idx.centers(), idx.rotation_matrix(), n_lists, dim, dim_ext, rot_dim, idx.centers_rot());
   res.launches++;
-  idx.allocate_lists(std::vector<uint32_t>(n_lists, 0), stream);  // also detects an identity rotation
+  idx.allocate_lists(std::vector<uint32_t>(n_lists, 0), stream);
+  idx.detect_identity_rotation(stream);
 
   // ---- PQ codebooks ----
   {
@@ -1330,6 +1705,8 @@ void build_any(raft::resources& res, const index_params& params, const void* dat
     res.launches++;
     res.sync();
   }
+
+  idx.recompute_model_state(stream);
 
   // ---- fill ----
   if (params.add_data_on_build) {

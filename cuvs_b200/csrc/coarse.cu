@@ -41,16 +41,22 @@ constexpr uint32_t kTile = 128, kTileK = 8;
 template <bool kVec, bool kArgmin>
 __global__ void __launch_bounds__(256, 2)
 exact_gemm_kernel(const float* __restrict__ b, uint32_t n_cols, const float* __restrict__ a, uint32_t n_rows, uint32_t kdim,
-                  float alpha, int half_scores, float* __restrict__ out, unsigned long long* __restrict__ best)
+                  float alpha, int half_scores, float* __restrict__ out, unsigned long long* __restrict__ best,
+                  const uint32_t* __restrict__ row_list, const uint32_t* __restrict__ n_listed)
 {
   __shared__ __align__(16) float2 s_a[2][kTileK][kTile + 2];
   __shared__ __align__(16) float s_b[2][kTileK][kTile + 4];
   const uint32_t j0 = blockIdx.x * kTile, i0 = blockIdx.y * kTile;
   const uint32_t tid = threadIdx.x, tx = tid & 15u, ty = tid >> 4;
+  // `row_list` (optional): the rows of `a` (and of `best`) to do, *n_listed of them
+  if (row_list != nullptr) {
+    n_rows = min(n_rows, __ldg(n_listed));
+    if (i0 >= n_rows) { return; }
+  }
   // one row and four k of either operand per thread
   const uint32_t lrow = tid >> 1, lk = (tid & 1u) * 4u;
   const bool in_a = i0 + lrow < n_rows, in_b = j0 + lrow < n_cols;
-  const float* pa = a + size_t(i0 + lrow) * kdim + lk;
+  const float* pa = a + size_t(row_list != nullptr && in_a ? __ldg(row_list + i0 + lrow) : i0 + lrow) * kdim + lk;
   const float* pb = b + size_t(j0 + lrow) * kdim + lk;
   float ra[4], rb[4];
   auto load = [&](uint32_t k0) {
@@ -158,7 +164,7 @@ exact_gemm_kernel(const float* __restrict__ b, uint32_t n_cols, const float* __r
         const unsigned long long o = __shfl_xor_sync(kFullMask, m, d);
         m = o < m ? o : m;
       }
-      if (tx == 0 && row < n_rows) { atomicMin(best + row, m); }
+      if (tx == 0 && row < n_rows) { atomicMin(best + (row_list != nullptr ? __ldg(row_list + row) : row), m); }
     }
   }
 }
@@ -212,7 +218,8 @@ few_rows_kernel(const float* __restrict__ b, uint32_t n_cols, const float* __res
 
 template <bool kArgmin>
 void launch_exact_gemm(const float* b, uint32_t n_cols, const float* a, uint32_t n_rows, uint32_t kdim, float alpha,
-                       bool half_scores, float* out, unsigned long long* best, cudaStream_t stream)
+                       bool half_scores, float* out, unsigned long long* best, cudaStream_t stream,
+                       const uint32_t* row_list = nullptr, const uint32_t* n_listed = nullptr)
 {
   if constexpr (!kArgmin) {
     const size_t smem = (size_t(32) * (kdim | 1u) + size_t(n_rows) * kdim) * 4;
@@ -233,9 +240,9 @@ void launch_exact_gemm(const float* b, uint32_t n_cols, const float* a, uint32_t
     unsigned long long* bs = best ? best + r0 : nullptr;
     const bool vec = kdim % 4 == 0 && ((reinterpret_cast<uintptr_t>(b) | reinterpret_cast<uintptr_t>(ar)) & 15u) == 0;
     if (vec) {
-      exact_gemm_kernel<true, kArgmin><<<grid, 256, 0, stream>>>(b, n_cols, ar, nr, kdim, alpha, half_scores, o, bs);
+      exact_gemm_kernel<true, kArgmin><<<grid, 256, 0, stream>>>(b, n_cols, ar, nr, kdim, alpha, half_scores, o, bs, row_list, n_listed);
     } else {
-      exact_gemm_kernel<false, kArgmin><<<grid, 256, 0, stream>>>(b, n_cols, ar, nr, kdim, alpha, half_scores, o, bs);
+      exact_gemm_kernel<false, kArgmin><<<grid, 256, 0, stream>>>(b, n_cols, ar, nr, kdim, alpha, half_scores, o, bs, row_list, n_listed);
     }
     CUDA_TRY(cudaGetLastError());
   }
@@ -481,10 +488,13 @@ void launch_select(const float* scores, uint32_t n_rows, uint32_t row_stride, ui
 }
 
 __global__ void unpack_labels_kernel(const unsigned long long* __restrict__ best, uint32_t n,
+                                     const uint32_t* __restrict__ row_list, const uint32_t* __restrict__ n_listed,
                                      uint32_t* __restrict__ labels)
 {
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) { labels[i] = uint32_t(best[i]); }
+  if (i >= (row_list != nullptr ? min(n, __ldg(n_listed)) : n)) { return; }
+  const uint32_t r = row_list != nullptr ? __ldg(row_list + i) : i;
+  labels[r]        = uint32_t(best[r]);
 }
 
 uint32_t chunk_queries(uint32_t n_queries, uint32_t n_lists)
@@ -537,6 +547,14 @@ void select_rows(raft::resources& res, const float* rows, uint32_t n_rows, uint3
   res.launches++;
 }
 
+void exact_rows_product(raft::resources& res, const float* b, uint32_t n_cols, const float* a, uint32_t n_rows, uint32_t k,
+                        float* out)
+{
+  if (n_rows == 0) { return; }
+  launch_exact_gemm<false>(b, n_cols, a, n_rows, k, 1.0f, false, out, nullptr, res.stream);
+  res.launches++;
+}
+
 void assign_nearest(raft::resources& res, const float* centers, uint32_t n_lists, uint32_t dim_ext,
                     float alpha, const float* x_ext, uint32_t n_rows, uint32_t* labels,
                     unsigned long long* best)
@@ -544,7 +562,19 @@ void assign_nearest(raft::resources& res, const float* centers, uint32_t n_lists
   if (n_rows == 0) { return; }
   CUDA_TRY(cudaMemsetAsync(best, 0xFF, size_t(n_rows) * 8, res.stream));
   launch_exact_gemm<true>(centers, n_lists, x_ext, n_rows, dim_ext, alpha, false, nullptr, best, res.stream);
-  unpack_labels_kernel<<<ceildiv<uint32_t>(n_rows, 256), 256, 0, res.stream>>>(best, n_rows, labels);
+  unpack_labels_kernel<<<ceildiv<uint32_t>(n_rows, 256), 256, 0, res.stream>>>(best, n_rows, nullptr, nullptr, labels);
+  CUDA_TRY(cudaGetLastError());
+  res.launches += 2;
+}
+
+void assign_nearest_listed(raft::resources& res, const float* centers, uint32_t n_lists, uint32_t dim_ext, float alpha,
+                           const float* x_ext, uint32_t n_rows, const uint32_t* row_list, const uint32_t* n_listed,
+                           uint32_t* labels, unsigned long long* best)
+{
+  CUVS_EXPECTS(n_rows <= 65535u * kTile, "too many rows");
+  CUDA_TRY(cudaMemsetAsync(best, 0xFF, size_t(n_rows) * 8, res.stream));
+  launch_exact_gemm<true>(centers, n_lists, x_ext, n_rows, dim_ext, alpha, false, nullptr, best, res.stream, row_list, n_listed);
+  unpack_labels_kernel<<<ceildiv<uint32_t>(n_rows, 256), 256, 0, res.stream>>>(best, n_rows, row_list, n_listed, labels);
   CUDA_TRY(cudaGetLastError());
   res.launches += 2;
 }

@@ -171,8 +171,9 @@ void index<int64_t>::allocate_lists(const std::vector<uint32_t>& sizes, cudaStre
     h_row_off_[l + 1] = h_row_off_[l] + round_up<uint64_t>(sizes[l], kIndexGroupSize);
   }
   const uint64_t rows = h_row_off_.back();
-  codes_.resize(round_up<uint64_t>(std::max<uint64_t>(rows, 32) * list_row_bytes(), 16));
-  ids_.resize(std::max<uint64_t>(rows, 32));
+  // (an index that is emptied and filled again keeps its arenas until it is destroyed or needs larger ones)
+  codes_.resize_within(round_up<uint64_t>(std::max<uint64_t>(rows, 32) * list_row_bytes(), 16));
+  ids_.resize_within(std::max<uint64_t>(rows, 32));
   CUDA_TRY(cudaMemsetAsync(codes_.data(), 0, codes_.size(), stream));
   fill_i64_kernel<<<ceildiv<size_t>(ids_.size(), 256), 256, 0, stream>>>(ids_.data(), ids_.size(),
                                                                           kInvalidRecord);
@@ -180,11 +181,11 @@ void index<int64_t>::allocate_lists(const std::vector<uint32_t>& sizes, cudaStre
                            cudaMemcpyHostToDevice, stream));
   CUDA_TRY(cudaMemcpyAsync(row_off_.data(), h_row_off_.data(), (size_t(n_lists_) + 1) * 8,
                            cudaMemcpyHostToDevice, stream));
+  recompute_list_state();
   CUDA_TRY(cudaStreamSynchronize(stream));
-  recompute_internal_state(stream);
 }
 
-void index<int64_t>::recompute_internal_state(cudaStream_t stream)
+void index<int64_t>::recompute_list_state()
 {
   // ivf_common.cuh:255-290: prefix sums of the list sizes sorted in descending order
   std::vector<uint32_t> sorted(h_list_sizes_);
@@ -194,6 +195,10 @@ void index<int64_t>::recompute_internal_state(cudaStream_t stream)
     accum_sorted_sizes_[l + 1] = accum_sorted_sizes_[l] + sorted[l];
   }
   size_ = accum_sorted_sizes_.back();
+}
+
+void index<int64_t>::detect_identity_rotation(cudaStream_t stream)
+{
   // an identity rotation lets search skip the rotation product (the result is bit-identical)
   std::vector<float> rot(size_t(rot_dim()) * dim_);
   CUDA_TRY(cudaMemcpyAsync(rot.data(), rotation_.data(), rot.size() * 4, cudaMemcpyDeviceToHost,
@@ -209,6 +214,11 @@ void index<int64_t>::recompute_internal_state(cudaStream_t stream)
     }
   }
   rotation_is_identity_ = ident;
+}
+
+void index<int64_t>::recompute_model_state(cudaStream_t stream)
+{
+  detect_identity_rotation(stream);
   centers_i8f_.reset();  // rebuilt from the current model on next use
   rotation_i8f_.reset();
   centers_h_.reset();
@@ -685,7 +695,7 @@ void deserialize(raft::resources& res, std::istream& is, index<int64_t>* out, in
     if (hids.size() >= stage_rows) { flush(); }
   }
   flush();
-  idx.recompute_internal_state(res.stream);
+  idx.recompute_model_state(res.stream);
   *out = std::move(idx);
 }
 

@@ -1,0 +1,554 @@
+// Nearest list of many rows on the tensor cores, exact: labels[i] = argmin over lists l of (score, l) with the score's
+// defining fp32 chain (coarse.cu) -- what k-means steps, extend and transform need.
+//
+// Reference: kmeans_balanced::predict (cpp/src/cluster/detail/kmeans_balanced.cuh:100-160).
+//
+// The probe selection of coarse_tc.cu with n_probes = 1 answers the same question, but keeps eight keys of every 64
+// lists in global memory and finishes with a block per row: 12 of 23 ms for 1 M rows x 16,384 lists.  For the nearest list
+// alone, one maximum per 64 lists is enough:
+//   1. operands in half precision (the same 11 significant bits as TF32 at twice the rate): rows q 2^e, lists c / cp, with
+//      cp the power of two above the largest |c|; -a against the two halfs of |c|^2 / (2 cp^2) in two more columns, so that
+//      the accumulator holds F (q.c - |c|^2 / 2), F = 2^e / cp, within (-0.5, 0.5).  `eps` of a row bounds how far that
+//      is from the exact value, the rounding of the keys below included.
+//   2. label_tc_kernel: a persistent CTA takes a tile of 128 rows against all (or a share) of the lists, 256 at a time.
+//      Per row and 64 lists of a tile the epilogue keeps the largest value as a packed key (value in fixed point, low bits
+//      the column: see coarse_tc.cu) and the second largest; across the tiles, per row and column quarter, the four
+//      largest of the former with their lists, and the largest of the latter.  Three float additions and three min / max per
+//      value: the epilogue's integer pipe and the tensor pipe are about equally busy.
+//   3. label_finish_kernel: lists within 2 eps of the largest value are rescored with the defining chain; one candidate needs
+//      no rescoring.  Where a list that was not kept might be within 2 eps, the row is redone exactly over all lists.
+// Every wait is bounded: on a time-out the kernel raises the error word and returns, and all rows are redone.
+#include "search_internal.hpp"
+#include "tc_ptx.cuh"
+#include "topk.cuh"
+
+#include <algorithm>
+
+namespace cuvs::neighbors::ivf_pq {
+
+using namespace cuvs_b200;
+
+namespace {
+
+constexpr uint32_t kRows = 128, kLists = 256, kBlockK = 64, kUnit = 64, kKeep = 4;
+constexpr uint32_t kEpiWarps = 16;
+constexpr uint32_t kThreads  = (2 + kEpiWarps) * 32;  // warp 0 TMA, warp 1 MMA, warps 2..17 epilogue
+constexpr uint32_t kABlock = kRows * kBlockK * 2, kBBlock = kLists * kBlockK * 2;  // 16 and 32 KB
+constexpr uint32_t kMaxStages = 6;
+constexpr uint32_t kRoom      = 6 * kBBlock;          // shared memory for operands: 192 KB
+
+// model words: [0] bits of the largest of |c|^2 and the norm column, [1] the power of two cp, [2] largest |c| / cp
+__global__ void center_stats_kernel(const float* __restrict__ centers, uint32_t n_lists, uint32_t dim, uint32_t dim_ext,
+                                    uint32_t* __restrict__ words)
+{
+  const uint32_t l    = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const uint32_t lane = threadIdx.x & 31u;
+  if (l >= n_lists) { return; }
+  const float* c = centers + size_t(l) * dim_ext;
+  float ss       = 0.0f;
+  for (uint32_t k = lane; k < dim; k += 32) { ss = __fmaf_rn(c[k], c[k], ss); }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) { ss += __shfl_xor_sync(kFullMask, ss, o); }
+  if (lane == 0) { atomicMax(words, __float_as_uint(fmaxf(ss, fabsf(c[dim])) * 1.0001f)); }
+}
+
+// cp = the smallest power of two that is at least sqrt(largest squared norm)
+__device__ __forceinline__ float center_scale(const uint32_t* words, float& bn)
+{
+  const float nrm = sqrtf(__uint_as_float(__ldg(words)));
+  const int E     = int((__float_as_uint(nrm) >> 23) & 0xFFu);   // nrm in [2^(E-127), 2^(E-126))
+  const bool fine = E >= 64 && E <= 190;
+  const float cp  = fine ? __uint_as_float(uint32_t(E + 1) << 23) : 1.0f;
+  bn              = fine ? nrm / cp * 1.0001f : INFINITY;       // out of range: no bound holds, every row is redone
+  return cp;
+}
+
+__global__ void center_operand_kernel(const float* __restrict__ centers, uint32_t n_lists, uint32_t dim, uint32_t dim_ext,
+                                      uint32_t width, const uint32_t* __restrict__ words, __half* __restrict__ out)
+{
+  const size_t i = blockIdx.x * size_t(blockDim.x) + threadIdx.x;
+  if (i >= size_t(n_lists) * width) { return; }
+  const uint32_t l = uint32_t(i / width), k = uint32_t(i - size_t(l) * width);
+  float bn;
+  const float inv = 1.0f / center_scale(words, bn);
+  const float* c  = centers + size_t(l) * dim_ext;
+  float v         = 0.0f;
+  if (k < dim) {
+    v = c[k] * inv;
+  } else if (k < dim + 2) {
+    const float n  = 0.5f * c[dim] * inv * inv;
+    const float hi = __half2float(__float2half_rn(n));
+    v              = k == dim ? hi : n - hi;
+  }
+  out[i] = __float2half_rn(v);
+}
+
+// One warp per row: the operand row, and eps (infinite: the row has to be redone).
+__global__ void row_operand_kernel(const float* __restrict__ x, uint32_t n_rows, uint32_t dim, uint32_t dim_ext,
+                                   uint32_t width, const uint32_t* __restrict__ words, __half* __restrict__ out,
+                                   float* __restrict__ eps)
+{
+  const uint32_t r    = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const uint32_t lane = threadIdx.x & 31u;
+  if (r >= n_rows) { return; }
+  float bn;
+  const float cp = center_scale(words, bn);
+  const float* q = x + size_t(r) * dim_ext;
+  float ss       = 0.0f;
+  for (uint32_t k = lane; k < dim; k += 32) { ss = __fmaf_rn(q[k], q[k], ss); }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) { ss += __shfl_xor_sync(kFullMask, ss, o); }
+  const float qn = sqrtf(ss) * 1.0001f;
+  // 2^e (|q| + cp / 2) in [0.25, 0.5)
+  const float b     = (qn + 0.5f * cp) * 1.01f;
+  const int E       = int((__float_as_uint(b) >> 23) & 0xFFu);
+  const bool fine   = E >= 2 && E <= 250;
+  const float scale = fine ? __uint_as_float(uint32_t(252 - E) << 23) : 0.0f;
+  const float a     = scale * cp;
+  __half2* dst      = reinterpret_cast<__half2*>(out + size_t(r) * width);
+  for (uint32_t k2 = lane; k2 < width / 2; k2 += 32) {
+    float v[2];
+#pragma unroll
+    for (uint32_t e = 0; e < 2; e++) {
+      const uint32_t k = 2 * k2 + e;
+      v[e]             = k < dim ? q[k] * scale : (k < dim + 2 ? -a : 0.0f);
+    }
+    dst[k2] = __floats2half2_rn(v[0], v[1]);
+  }
+  if (lane == 0) {
+    const float an = qn * scale, w = float(width);
+    // operands rounded to half precision (relative, and absolute near zero), accumulation, the exact chain's own
+    // rounding, the key's
+    float e = 9.9e-4f * an * bn + sqrtf(w) * 3.0e-8f * (an + bn) + (w + 24.0f) * 2.4e-7f + float(dim_ext) * 1.2e-7f + 7.7e-6f;
+    if (!fine || !(a >= 6.2e-5f)) { e = INFINITY; }
+    eps[r] = e;
+  }
+}
+
+struct label_params {
+  uint32_t n_rows, n_lists, k_steps /* of 16 halfs */, k_blocks;
+  uint32_t n_tiles, tiles_per_split, n_items, splits;
+  uint32_t a_resident, n_stages;
+  uint4* keys;       // [splits, n_rows, 4] largest keys of a column quarter
+  uint4* lists;      // their lists
+  uint32_t* bounds;  // [splits, n_rows, 4] key of the largest value that a 64-list unit of a tile dropped
+  uint32_t* error;
+  uint32_t spin_limit;
+};
+
+__global__ void __launch_bounds__(kThreads, 1)
+label_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, const label_params p)
+{
+  extern __shared__ uint8_t smem_raw[];
+  const uint32_t raw_a  = smem_u32(smem_raw);
+  const uint32_t base_a = (raw_a + 1023u) & ~1023u;
+  uint8_t* base_p       = smem_raw + (base_a - raw_a);
+  uint64_t* bars        = reinterpret_cast<uint64_t*>(base_p + kRoom);
+  const uint32_t bar_full   = smem_u32(bars);
+  const uint32_t bar_empty  = bar_full + kMaxStages * 8;
+  const uint32_t bar_tfull  = bar_empty + kMaxStages * 8;
+  const uint32_t bar_tempty = bar_tfull + 2 * 8;
+  const uint32_t bar_afull  = bar_tempty + 2 * 8;
+  const uint32_t bar_aempty = bar_afull + 8;
+  uint32_t* tmem_slot       = reinterpret_cast<uint32_t*>(bars + 2 * kMaxStages + 6);
+  // [row tile, when resident][stages: list block, then row block when not]
+  const uint32_t a_bytes    = p.a_resident ? p.k_blocks * kABlock : 0u;
+  const uint32_t stage_size = kBBlock + (p.a_resident ? 0u : kABlock);
+  const uint32_t stage_base = base_a + a_bytes;
+  const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
+
+  if (threadIdx.x == 0) {
+    for (uint32_t s = 0; s < p.n_stages; s++) {
+      mbar_init(bar_full + s * 8, 1);
+      mbar_init(bar_empty + s * 8, 1);
+    }
+    for (uint32_t a = 0; a < 2; a++) {
+      mbar_init(bar_tfull + a * 8, 1);
+      mbar_init(bar_tempty + a * 8, kEpiWarps);
+    }
+    mbar_init(bar_afull, 1);
+    mbar_init(bar_aempty, 1);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == 1) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(smem_u32(tmem_slot))
+                 : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem_base = *reinterpret_cast<volatile uint32_t*>(tmem_slot);
+  bool ok = true;
+  // the list tiles of an item
+  auto tiles_of = [&](uint32_t item, uint32_t& t0, uint32_t& t1) {
+    const uint32_t s = item % p.splits;
+    t0               = s * p.tiles_per_split;
+    t1               = min(p.n_tiles, t0 + p.tiles_per_split);
+  };
+
+  if (warp == 0) {
+    // ---------------- TMA producer ----------------
+    if (lane == 0) {
+      uint32_t stage = 0, phase = 0, n_a = 0;
+      for (uint32_t item = blockIdx.x; ok && item < p.n_items; item += gridDim.x) {
+        const int row0 = int((item / p.splits) * kRows);
+        uint32_t t0, t1;
+        tiles_of(item, t0, t1);
+        if (p.a_resident) {
+          if (!mbar_wait(bar_aempty, (n_a & 1u) ^ 1u, p.spin_limit)) {
+            ok = false;
+            break;
+          }
+          n_a++;
+          mbar_arrive_expect_tx(bar_afull, a_bytes);
+          for (uint32_t kb = 0; kb < p.k_blocks; kb++) {
+            tma_load_2d(base_a + kb * kABlock, &map_a, bar_afull, int(kb * kBlockK), row0);
+          }
+        }
+        for (uint32_t t = t0; ok && t < t1; t++) {
+          for (uint32_t kb = 0; kb < p.k_blocks; kb++) {
+            if (!mbar_wait(bar_empty + stage * 8, phase ^ 1u, p.spin_limit)) {
+              ok = false;
+              break;
+            }
+            const uint32_t dst = stage_base + stage * stage_size, bar = bar_full + stage * 8;
+            mbar_arrive_expect_tx(bar, stage_size);
+            tma_load_2d(dst, &map_b, bar, int(kb * kBlockK), int(t * kLists));
+            if (!p.a_resident) { tma_load_2d(dst + kBBlock, &map_a, bar, int(kb * kBlockK), row0); }
+            if (++stage == p.n_stages) {
+              stage = 0;
+              phase ^= 1u;
+            }
+          }
+        }
+      }
+    }
+    __syncwarp();
+  } else if (warp == 1) {
+    // ---------------- MMA issuer ----------------
+    if (lane == 0) {
+      // fp32 accumulate, half x half, both K-major, M = 128, N = 256
+      constexpr uint32_t idesc = (1u << 4) | ((kLists >> 3) << 17) | ((kRows >> 4) << 24);
+      uint32_t stage = 0, phase = 0, n_a = 0, it = 0;
+      for (uint32_t item = blockIdx.x; ok && item < p.n_items; item += gridDim.x) {
+        uint32_t t0, t1;
+        tiles_of(item, t0, t1);
+        if (p.a_resident) {
+          if (!mbar_wait(bar_afull, n_a & 1u, p.spin_limit)) {
+            ok = false;
+            break;
+          }
+          n_a++;
+        }
+        for (uint32_t t = t0; ok && t < t1; t++, it++) {
+          const uint32_t acc = it & 1u;
+          if (!mbar_wait(bar_tempty + acc * 8, ((it >> 1) & 1u) ^ 1u, p.spin_limit)) {
+            ok = false;
+            break;
+          }
+          tc_fence_after();
+          const uint32_t tmem_d = tmem_base + acc * kLists;
+          for (uint32_t kb = 0; kb < p.k_blocks; kb++) {
+            if (!mbar_wait(bar_full + stage * 8, phase, p.spin_limit)) {
+              ok = false;
+              break;
+            }
+            tc_fence_after();
+            const uint32_t sa  = stage_base + stage * stage_size;
+            const uint64_t da  = make_desc_sw128(p.a_resident ? base_a + kb * kABlock : sa + kBBlock);
+            const uint64_t db  = make_desc_sw128(sa);
+            const uint32_t nk  = min(4u, p.k_steps - kb * 4u);
+#pragma unroll
+            for (uint32_t k = 0; k < 4; k++) {
+              if (k >= nk) { break; }
+              tc_mma_f16(tmem_d, da + k * 2u, db + k * 2u, idesc, (kb | k) != 0u);  // 32 bytes of K per step
+            }
+            tc_commit(bar_empty + stage * 8);
+            if (++stage == p.n_stages) {
+              stage = 0;
+              phase ^= 1u;
+            }
+          }
+          if (ok) { tc_commit(bar_tfull + acc * 8); }
+        }
+        if (ok && p.a_resident) { tc_commit(bar_aempty); }  // the row tile may be replaced once these MMAs are done
+      }
+    }
+    __syncwarp();
+  } else {
+    // ---------------- epilogue: thread = row, warp = (lane quarter, 64 columns) ----------------
+    const uint32_t quarter = warp & 3u, unit = (warp - 2) >> 2;
+    uint32_t it            = 0;
+    for (uint32_t item = blockIdx.x; ok && item < p.n_items; item += gridDim.x) {
+      uint32_t t0, t1;
+      tiles_of(item, t0, t1);
+      uint32_t key[kKeep] = {0u, 0u, 0u, 0u}, list[kKeep] = {0u, 0u, 0u, 0u}, bound = 0u;
+      for (uint32_t t = t0; t < t1; t++, it++) {
+        const uint32_t acc = it & 1u;
+        if (ok && !mbar_wait(bar_tfull + acc * 8, (it >> 1) & 1u, p.spin_limit)) { ok = false; }
+        if (__any_sync(kFullMask, !ok)) {
+          ok = false;
+          break;
+        }
+        tc_fence_after();
+        const uint32_t n0 = t * kLists + unit * kUnit;
+        uint32_t l0 = 0u, l1 = 0u;
+        auto chunk = [&](auto second, auto full) {
+          constexpr uint32_t c = decltype(second)::value ? 32u : 0u;
+          uint32_t x[32];
+          tmem_ld32(tmem_base + ((quarter * 32u) << 16) + acc * kLists + unit * kUnit + c, x);
+#pragma unroll
+          for (uint32_t e = 0; e < 32; e++) {
+            // value rounded to a multiple of 2^-16, + 1.5 + tag 2^-23: bits that sort, low 7 the tag 63 - column
+            float f = __fadd_rn(__uint_as_float(x[e]), 192.0f);
+            f       = __fadd_rn(f, -192.0f);
+            f       = __fadd_rn(f, 1.5f + float(63u - c - e) * 0x1p-23f);
+            uint32_t k = __float_as_uint(f);
+            if constexpr (!decltype(full)::value) {
+              if (n0 + c + e >= p.n_lists) { k = 0u; }
+            }
+            l1 = max(l1, min(l0, k));
+            l0 = max(l0, k);
+          }
+        };
+        if (n0 + kUnit <= p.n_lists) {
+          chunk(std::false_type{}, std::true_type{});
+          chunk(std::true_type{}, std::true_type{});
+        } else {
+          chunk(std::false_type{}, std::false_type{});
+          chunk(std::true_type{}, std::false_type{});
+        }
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) { mbar_arrive(bar_tempty + acc * 8); }
+        bound = max(bound, l1);
+        if (l0 > key[kKeep - 1]) {
+          key[kKeep - 1]  = l0;
+          list[kKeep - 1] = n0 + (63u - (l0 & 127u));
+#pragma unroll
+          for (int i = int(kKeep) - 1; i > 0; i--) {
+            if (key[i] > key[i - 1]) {
+              const uint32_t a = key[i], b = list[i];
+              key[i]      = key[i - 1];
+              list[i]     = list[i - 1];
+              key[i - 1]  = a;
+              list[i - 1] = b;
+            }
+          }
+        }
+      }
+      const uint32_t row = (item / p.splits) * kRows + quarter * 32u + lane;
+      if (ok && row < p.n_rows) {
+        const size_t at = (size_t(item % p.splits) * p.n_rows + row) * 4u + unit;
+        p.keys[at]      = make_uint4(key[0], key[1], key[2], key[3]);
+        p.lists[at]     = make_uint4(list[0], list[1], list[2], list[3]);
+        p.bounds[at]    = bound;
+      }
+    }
+  }
+  if (!ok) { atomicExch(p.error, ERR_TIMEOUT); }
+
+  tc_fence_before();
+  if (__syncthreads_or(!ok)) {
+    // a time-out: give copies and MMAs that are still in flight time to finish before their memory is released
+    for (int i = 0; i < 64; i++) { __nanosleep(1000); }
+    __syncthreads();
+  }
+  if (warp == 1) {
+    tc_fence_after();
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(tmem_base) : "memory");
+  }
+}
+
+__device__ __forceinline__ float key_value(uint32_t key)
+{
+  return key >= 0x00800000u ? __fadd_rn(__uint_as_float(key & ~127u), -1.5f) : -INFINITY;
+}
+
+// Four lanes per row: lane u reads what column quarter u kept (of every split).
+__global__ void __launch_bounds__(256)
+label_finish_kernel(const uint4* __restrict__ keys, const uint4* __restrict__ lists, const uint32_t* __restrict__ bounds,
+                    uint32_t splits, uint32_t n_rows, const float* __restrict__ eps, const uint32_t* __restrict__ error,
+                    const float* __restrict__ x, const float* __restrict__ centers, uint32_t dim_ext, float alpha,
+                    uint32_t* __restrict__ labels, uint32_t* __restrict__ redo, uint32_t* __restrict__ n_redo)
+{
+  const uint32_t r = (blockIdx.x * 256u + threadIdx.x) >> 2, u = threadIdx.x & 3u;
+  const unsigned mask = 0xFu << (threadIdx.x & 28u);
+  if (r >= n_rows) { return; }
+  float top = -INFINITY, out = -INFINITY;  // largest value kept, largest that may have been dropped
+  for (uint32_t s = 0; s < splits; s++) {
+    const size_t at = (size_t(s) * n_rows + r) * 4u + u;
+    const uint4 k   = __ldg(keys + at);
+    top             = fmaxf(top, key_value(k.x));
+    out             = fmaxf(out, fmaxf(key_value(k.w), key_value(__ldg(bounds + at))));
+  }
+#pragma unroll
+  for (int o = 2; o > 0; o >>= 1) {
+    top = fmaxf(top, __shfl_xor_sync(mask, top, o));
+    out = fmaxf(out, __shfl_xor_sync(mask, out, o));
+  }
+  const float t = top - 2.0f * __ldg(eps + r);
+  // (negated: an infinite or undefined bound is not proof)
+  if (*error != 0u || !(out < t)) {
+    if (u == 0) { redo[atomicAdd(n_redo, 1u)] = r; }
+    return;
+  }
+  // candidates
+  uint32_t n = 0, only = 0xFFFFFFFFu;
+  for (uint32_t s = 0; s < splits; s++) {
+    const size_t at = (size_t(s) * n_rows + r) * 4u + u;
+    const uint4 k   = __ldg(keys + at);
+    if (key_value(k.x) >= t) {
+      const uint4 l = __ldg(lists + at);
+      n += 1u + (key_value(k.y) >= t ? 1u : 0u) + (key_value(k.z) >= t ? 1u : 0u);
+      only = l.x;
+    }
+  }
+  uint32_t all = n;
+#pragma unroll
+  for (int o = 2; o > 0; o >>= 1) { all += __shfl_xor_sync(mask, all, o); }
+  if (all == 1u) {
+    if (n == 1u) { labels[r] = only; }
+    return;
+  }
+  // each lane rescores its own (rarely more than one) with the defining chain
+  const float* q = x + size_t(r) * dim_ext;
+  uint64_t best  = kEmptyKey;
+  if (n > 0) {
+    for (uint32_t s = 0; s < splits; s++) {
+      const size_t at     = (size_t(s) * n_rows + r) * 4u + u;
+      const uint4 k       = __ldg(keys + at), l = __ldg(lists + at);
+      const uint32_t kk[3] = {k.x, k.y, k.z}, ll[3] = {l.x, l.y, l.z};
+#pragma unroll
+      for (int i = 0; i < 3; i++) {
+        if (key_value(kk[i]) < t) { continue; }
+        const float4* c = reinterpret_cast<const float4*>(centers + size_t(ll[i]) * dim_ext);
+        float acc       = 0.0f;
+        for (uint32_t k4 = 0; k4 < dim_ext / 4; k4++) {  // dim_ext is a multiple of 8
+          const float4 cv = __ldg(c + k4), qv = __ldg(reinterpret_cast<const float4*>(q) + k4);
+          acc             = __fmaf_rn(cv.x, qv.x, acc);
+          acc             = __fmaf_rn(cv.y, qv.y, acc);
+          acc             = __fmaf_rn(cv.z, qv.z, acc);
+          acc             = __fmaf_rn(cv.w, qv.w, acc);
+        }
+        const uint64_t key = make_key(__fmul_rn(alpha, acc), ll[i]);
+        best               = key < best ? key : best;
+      }
+    }
+  }
+#pragma unroll
+  for (int o = 2; o > 0; o >>= 1) {
+    const uint32_t hi = __shfl_xor_sync(mask, uint32_t(best >> 32), o), lo = __shfl_xor_sync(mask, uint32_t(best), o);
+    const uint64_t other = (uint64_t(hi) << 32) | lo;
+    best                 = other < best ? other : best;
+  }
+  if (u == 0) { labels[r] = uint32_t(best); }
+}
+
+uint32_t operand_width(uint32_t dim) { return round_up(dim + 2u, 16u); }
+
+}  // namespace
+
+// Below some 16 M products a whole exact pass costs less than these launches; fewer than 256 lists are not one tile.
+bool label_tc_usable(uint32_t n_rows, uint32_t n_lists)
+{
+  return n_lists >= 256 && uint64_t(n_rows) * n_lists >= (1ull << 24);
+}
+
+size_t label_model_bytes(uint32_t n_lists, uint32_t dim) { return size_t(n_lists) * operand_width(dim) * 2 + 256; }
+
+void prepare_label_model(cudaStream_t stream, const float* centers, uint32_t n_lists, uint32_t dim, uint32_t dim_ext, void* model)
+{
+  auto* words = static_cast<uint32_t*>(model);
+  auto* b     = reinterpret_cast<__half*>(static_cast<char*>(model) + 256);
+  CUDA_TRY(cudaMemsetAsync(words, 0, 16, stream));
+  center_stats_kernel<<<ceildiv<uint32_t>(n_lists * 32u, 256u), 256, 0, stream>>>(centers, n_lists, dim, dim_ext, words);
+  const size_t n = size_t(n_lists) * operand_width(dim);
+  center_operand_kernel<<<unsigned(ceildiv<size_t>(n, 256)), 256, 0, stream>>>(centers, n_lists, dim, dim_ext,
+                                                                              operand_width(dim), words, b);
+  CUDA_TRY(cudaGetLastError());
+}
+
+namespace {
+struct label_layout {
+  uint32_t splits, tiles_per_split;
+  size_t o_a, o_eps, o_keys, o_lists, o_bounds, o_redo, o_words, o_best, total;
+};
+label_layout layout_for(uint32_t n_rows, uint32_t n_lists, uint32_t dim, int sm_count)
+{
+  label_layout y{};
+  const uint32_t row_tiles = ceildiv(n_rows, kRows), n_tiles = ceildiv(n_lists, kLists);
+  // few row tiles: the lists are shared out, so that there are about four items per SM
+  y.splits = 1;
+  while (y.splits < n_tiles && row_tiles * y.splits < 4u * uint32_t(sm_count) && y.splits < 16) { y.splits <<= 1; }
+  y.splits          = std::min(y.splits, n_tiles);
+  y.tiles_per_split = ceildiv(n_tiles, y.splits);
+  y.splits          = ceildiv(n_tiles, y.tiles_per_split);
+  const size_t recs = size_t(y.splits) * n_rows * 4;
+  ws_layout lay;
+  y.o_a      = lay.add(size_t(n_rows) * operand_width(dim) * 2);
+  y.o_eps    = lay.add(size_t(n_rows) * 4);
+  y.o_keys   = lay.add(recs * 16);
+  y.o_lists  = lay.add(recs * 16);
+  y.o_bounds = lay.add(recs * 4);
+  y.o_redo   = lay.add(size_t(n_rows) * 4);
+  y.o_words  = lay.add(256);
+  y.o_best   = lay.add(size_t(n_rows) * 8);
+  y.total    = lay.total();
+  return y;
+}
+}  // namespace
+
+size_t label_workspace_bytes(const raft::resources& res, uint32_t n_rows, uint32_t n_lists, uint32_t dim)
+{
+  return layout_for(n_rows, n_lists, dim, res.sm_count).total;
+}
+
+void label_rows_tc(raft::resources& res, const float* centers, const void* model, uint32_t n_lists, uint32_t dim,
+                   uint32_t dim_ext, float alpha, const float* x_ext, uint32_t n_rows, uint32_t* labels, void* workspace)
+{
+  if (n_rows == 0) { return; }
+  const label_layout y = layout_for(n_rows, n_lists, dim, res.sm_count);
+  const uint32_t width = operand_width(dim);
+  char* ws             = static_cast<char*>(workspace);
+  auto* a              = reinterpret_cast<__half*>(ws + y.o_a);
+  auto* eps            = reinterpret_cast<float*>(ws + y.o_eps);
+  auto* words          = reinterpret_cast<uint32_t*>(ws + y.o_words);  // error, rows to redo
+  auto* redo           = reinterpret_cast<uint32_t*>(ws + y.o_redo);
+  auto* best           = reinterpret_cast<unsigned long long*>(ws + y.o_best);
+  const auto* b        = reinterpret_cast<const __half*>(static_cast<const char*>(model) + 256);
+  cudaStream_t stream  = res.stream;
+  CUDA_TRY(cudaMemsetAsync(words, 0, 8, stream));
+  row_operand_kernel<<<ceildiv<uint32_t>(n_rows, 8u), 256, 0, stream>>>(x_ext, n_rows, dim, dim_ext, width,
+                                                                        static_cast<const uint32_t*>(model), a, eps);
+  label_params p{};
+  p.n_rows          = n_rows;
+  p.n_lists         = n_lists;
+  p.k_steps         = width / 16;
+  p.k_blocks        = ceildiv(width, kBlockK);
+  p.n_tiles         = ceildiv(n_lists, kLists);
+  p.tiles_per_split = y.tiles_per_split;
+  p.splits          = y.splits;
+  p.n_items         = ceildiv(n_rows, kRows) * y.splits;
+  // the row tile stays in shared memory where that leaves at least three list stages (dim <= 382)
+  p.a_resident = p.k_blocks * kABlock + 3 * kBBlock <= kRoom;
+  p.n_stages   = p.a_resident ? std::min(kMaxStages, (kRoom - p.k_blocks * kABlock) / kBBlock) : kRoom / (kABlock + kBBlock);
+  p.keys       = reinterpret_cast<uint4*>(ws + y.o_keys);
+  p.lists      = reinterpret_cast<uint4*>(ws + y.o_lists);
+  p.bounds     = reinterpret_cast<uint32_t*>(ws + y.o_bounds);
+  p.error      = words;
+  p.spin_limit = kSpinLimit;
+  const CUtensorMap ma = make_map_2d(CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, a, n_rows, width, kRows, kBlockK, CU_TENSOR_MAP_SWIZZLE_128B);
+  const CUtensorMap mb = make_map_2d(CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, b, n_lists, width, kLists, kBlockK, CU_TENSOR_MAP_SWIZZLE_128B);
+  const size_t smem    = kRoom + 1024 + 256;
+  ensure_dynamic_smem(reinterpret_cast<const void*>(label_tc_kernel), smem);
+  label_tc_kernel<<<std::min(uint32_t(res.sm_count), p.n_items), kThreads, smem, stream>>>(ma, mb, p);
+  label_finish_kernel<<<ceildiv(n_rows, 64u), 256, 0, stream>>>(p.keys, p.lists, p.bounds, p.splits, n_rows, eps, words, x_ext,
+                                                                centers, dim_ext, alpha, labels, redo, words + 1);
+  CUDA_TRY(cudaGetLastError());
+  assign_nearest_listed(res, centers, n_lists, dim_ext, alpha, x_ext, n_rows, redo, words + 1, labels, best);
+  res.launches += 3;
+}
+
+}  // namespace cuvs::neighbors::ivf_pq

@@ -94,4 +94,22 @@ void assign_nearest(raft::resources& res, const float* centers, uint32_t n_lists
                     float alpha, const float* x_ext, uint32_t n_rows, uint32_t* labels,
                     unsigned long long* best);
 
+// The same for the rows named in row_list[0 .. *n_listed) (both on the device); other labels stay as they are.
+void assign_nearest_listed(raft::resources& res, const float* centers, uint32_t n_lists, uint32_t dim_ext, float alpha,
+                           const float* x_ext, uint32_t n_rows, const uint32_t* row_list, const uint32_t* n_listed,
+                           uint32_t* labels, unsigned long long* best);
+// out[i, j] = sum over ascending k of b[j, k] * a[i, k], one fp32 fused multiply-add chain each.
+void exact_rows_product(raft::resources& res, const float* b, uint32_t n_cols, const float* a, uint32_t n_rows, uint32_t k,
+                        float* out);
+
+// The same labels on the tensor cores (label_tc.cu).  `model`: label_model_bytes of device memory that
+// prepare_label_model fills from the centres; `workspace`: label_workspace_bytes.  Nothing synchronises.
+bool label_tc_usable(uint32_t n_rows, uint32_t n_lists);
+size_t label_model_bytes(uint32_t n_lists, uint32_t dim);
+void prepare_label_model(cudaStream_t stream, const float* centers, uint32_t n_lists, uint32_t dim, uint32_t dim_ext,
+                         void* model);
+size_t label_workspace_bytes(const raft::resources& res, uint32_t n_rows, uint32_t n_lists, uint32_t dim);
+void label_rows_tc(raft::resources& res, const float* centers, const void* model, uint32_t n_lists, uint32_t dim,
+                   uint32_t dim_ext, float alpha, const float* x_ext, uint32_t n_rows, uint32_t* labels, void* workspace);
+
 }  // namespace cuvs::neighbors::ivf_pq

@@ -134,7 +134,8 @@ struct resources {
   int sm_count          = 0;
   int smem_optin        = 0;        // max dynamic shared memory per block (opt-in)
   int cc_major          = 0;
-  workspace ws;
+  workspace ws;       // search
+  workspace scratch;  // extend and transform (bounded by their chunk size and the labels of the rows given)
   // small pinned host word for an occasional device->host scalar
   uint32_t* pinned = nullptr;
   // counters read by the benchmark ("how many kernels of ours ran")

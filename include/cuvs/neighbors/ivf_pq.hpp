@@ -160,19 +160,22 @@ class dev_array {
   dev_array() = default;
   explicit dev_array(size_t n) { resize(n); }
   ~dev_array() { reset(); }
-  dev_array(dev_array&& o) noexcept : p_(o.p_), n_(o.n_)
+  dev_array(dev_array&& o) noexcept : p_(o.p_), n_(o.n_), cap_(o.cap_)
   {
-    o.p_ = nullptr;
-    o.n_ = 0;
+    o.p_   = nullptr;
+    o.n_   = 0;
+    o.cap_ = 0;
   }
   dev_array& operator=(dev_array&& o) noexcept
   {
     if (this != &o) {
       reset();
-      p_   = o.p_;
-      n_   = o.n_;
-      o.p_ = nullptr;
-      o.n_ = 0;
+      p_     = o.p_;
+      n_     = o.n_;
+      cap_   = o.cap_;
+      o.p_   = nullptr;
+      o.n_   = 0;
+      o.cap_ = 0;
     }
     return *this;
   }
@@ -182,20 +185,29 @@ class dev_array {
   {
     reset();
     if (n) { CUDA_TRY(cudaMalloc(&p_, n * sizeof(T))); }
+    n_   = n;
+    cap_ = n;
+  }
+  // as resize, but keeps the allocation where it is large enough
+  void resize_within(size_t n)
+  {
+    if (n > cap_) { resize(n); }
     n_ = n;
   }
   void reset()
   {
     if (p_) { cudaFree(p_); }
-    p_ = nullptr;
-    n_ = 0;
+    p_   = nullptr;
+    n_   = 0;
+    cap_ = 0;
   }
   T* data() const { return p_; }
   size_t size() const { return n_; }
 
  private:
-  T* p_     = nullptr;
-  size_t n_ = 0;
+  T* p_       = nullptr;
+  size_t n_   = 0;
+  size_t cap_ = 0;
 };
 
 template <typename IdxT>
@@ -293,8 +305,10 @@ class index<int64_t> {
 
   // (Re)create the arenas for the given list sizes; contents are zero codes / -1 ids.
   void allocate_lists(const std::vector<uint32_t>& sizes, cudaStream_t stream);
-  // Recompute host-side derived state after the model arrays or list sizes changed.
-  void recompute_internal_state(cudaStream_t stream);
+  // Derived state: of the list sizes (allocate_lists does it), and of the model arrays (to be called when they changed).
+  void recompute_list_state();
+  void recompute_model_state(cudaStream_t stream);
+  void detect_identity_rotation(cudaStream_t stream);  // part of recompute_model_state
 
   // model arrays are public to the builder / loader
   dev_array<float> pq_centers_, centers_, centers_rot_, rotation_;

@@ -1,0 +1,87 @@
+"""Labels and codes of `transform` against a float64 statement: the labelling on the tensor cores (and the exact pass below
+its size), and the encoder for every number of components per subspace."""
+import numpy as np
+import pytest
+
+from conftest import make_mixture
+
+pytestmark = pytest.mark.gpu
+torch = pytest.importorskip("torch")
+
+
+@pytest.fixture(scope="module")
+def ivf():
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    from cuvs_b200 import ivf_pq
+    return ivf_pq
+
+
+def model(ivf, dim, n_lists, pq_dim, bits, metric="sqeuclidean", scale=1.0, seed=0):
+    rng = np.random.default_rng(seed)
+    length = -(-dim // pq_dim)
+    rot_dim = pq_dim * length
+    centers = (make_mixture(n_lists, dim, 40, 0.3, seed) * scale).astype(np.float32)
+    books = (rng.standard_normal((pq_dim, length, 1 << bits)) * 0.2 * scale).astype(np.float32)
+    rot = np.eye(dim) if rot_dim == dim else np.linalg.qr(rng.standard_normal((rot_dim, rot_dim)))[0][:, :dim]
+    rot = rot.astype(np.float32)
+    to = lambda a: torch.from_numpy(np.ascontiguousarray(a)).cuda()  # noqa: E731
+    index = ivf.build_precomputed(ivf.IndexParams(n_lists=n_lists, pq_dim=pq_dim, pq_bits=bits, metric=metric), dim,
+                                  to(books), to(centers), to(centers @ rot.T), to(rot))
+    return index, centers, books, rot
+
+
+def check_labels(labels, x, centers):
+    x64, c64 = torch.from_numpy(x).cuda().double(), torch.from_numpy(centers).cuda().double()
+    d = torch.cdist(x64, c64)
+    best = d.min(1).values
+    got = d.gather(1, labels.to(torch.int64).unsqueeze(1)).squeeze(1)
+    # the label's squared distance is the smallest up to the rounding of an fp32 chain over |x||c|
+    tol = 1e-5 * (x64.norm(dim=1) + c64.norm(dim=1).max()) ** 2
+    assert bool((got ** 2 <= best ** 2 + tol).all())
+    assert float((got == best).double().mean()) > 0.99
+
+
+# edges of the 128-row and 256-list tiles, one and several K blocks, row tile resident (dim <= 382) and not, few rows (lists
+# shared between SMs), and sizes below the tensor-core path
+@pytest.mark.parametrize("n,dim,n_lists", [(65536, 14, 256), (70001, 61, 257), (20000, 62, 1000), (16387, 126, 2049),
+                                           (9000, 127, 5000), (20001, 384, 1023), (17000, 768, 1100), (100, 32, 300)])
+@pytest.mark.parametrize("scale", [1.0, 3e4])
+def test_labels(ivf, n, dim, n_lists, scale):
+    pq_dim = 8 if dim >= 8 else 1
+    index, centers, _, _ = model(ivf, dim, n_lists, pq_dim, 8, scale=scale)
+    x = (make_mixture(n, dim, 40, 0.3, 5) * scale).astype(np.float32)
+    x[3] = centers[7]            # exactly a centre
+    x[4] *= 1e-3                 # far from the scale of the others
+    x[5] *= 1e5
+    labels, _ = ivf.transform(index, torch.from_numpy(x).cuda())
+    check_labels(labels, x, centers)
+
+
+def test_equal_centres_take_the_lowest_list(ivf):
+    index, centers, books, rot = model(ivf, 32, 512, 16, 8)
+    centers[100:356] = centers[44]          # ties inside and across tiles: all rows near them are redone exactly
+    to = lambda a: torch.from_numpy(np.ascontiguousarray(a)).cuda()  # noqa: E731
+    index = ivf.build_precomputed(ivf.IndexParams(n_lists=512, pq_dim=16), 32, to(books), to(centers),
+                                  to(centers @ rot.T), to(rot))
+    x = make_mixture(40000, 32, 40, 0.3, 3)
+    x[:300] = centers[44] + 1e-3
+    labels = ivf.transform(index, to(x))[0].to(torch.int64)
+    assert bool((labels[:300] == 44).all()) and not bool(((labels >= 100) & (labels < 356)).any())
+
+
+@pytest.mark.parametrize("bits,pq_dim,length", [(8, 16, 1), (8, 24, 2), (8, 6, 2), (8, 10, 3), (8, 5, 4), (4, 8, 5), (8, 4, 8),
+                                                (5, 8, 2), (6, 12, 4), (7, 8, 16), (8, 2, 130), (4, 64, 2)])
+@pytest.mark.parametrize("n", [1, 1025])
+def test_codes(ivf, bits, pq_dim, length, n):
+    dim = pq_dim * length
+    index, centers, books, _ = model(ivf, dim, 20, pq_dim, bits)
+    x = make_mixture(n, dim, 40, 0.3, 9)
+    labels, packed = ivf.transform(index, torch.from_numpy(x).cuda())
+    labels, packed = labels.cpu().numpy().astype(np.int64), packed.cpu().numpy()
+    stream = np.unpackbits(packed, axis=1, bitorder="little")[:, :pq_dim * bits].reshape(n, pq_dim, bits)
+    codes = (stream * (1 << np.arange(bits))).sum(2)
+    r = (x - centers[labels]).astype(np.float32).reshape(n, pq_dim, length)
+    d = ((r[:, :, :, None].astype(np.float64) - books[None]) ** 2).sum(2)
+    got = np.take_along_axis(d, codes[:, :, None], 2)[:, :, 0]
+    assert (got <= d.min(2) * (1 + 1e-5) + 1e-9).all() and (codes == d.argmin(2)).mean() > 0.999
