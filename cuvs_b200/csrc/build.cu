@@ -988,7 +988,7 @@ class nearest_labeler {
   {
     if (!use_tc_) { return; }
     prepare_label_model(res_.stream, centers_, n_lists_, dim_, dim_ext_, mem_);
-    res_.launches += 2;
+    res_.launches += 3;
   }
   // labels[i] = nearest list of row i of x_ext [n_rows, dim_ext]
   void run(const float* x_ext, uint64_t n_rows, uint32_t* labels)

@@ -6,17 +6,21 @@
 // The probe selection of coarse_tc.cu with n_probes = 1 answers the same question, but keeps eight keys of every 64
 // lists in global memory and finishes with a block per row: 12 of 23 ms for 1 M rows x 16,384 lists.  For the nearest list
 // alone, one maximum per 64 lists is enough:
-//   1. operands in half precision (the same 11 significant bits as TF32 at twice the rate): rows q 2^e, lists c / cp, with
-//      cp the power of two above the largest |c|; -a against the two halfs of |c|^2 / (2 cp^2) in two more columns, so that
-//      the accumulator holds F (q.c - |c|^2 / 2), F = 2^e / cp, within (-0.5, 0.5).  `eps` of a row bounds how far that
-//      is from the exact value, the rounding of the keys below included.
+//   1. operands in half precision (the same 11 significant bits as TF32 at twice the rate), relative to the mean m of the
+//      centres: rows (q - m) 2^e, lists (c - m) / cp, with cp the power of two above the largest |c - m|; two more
+//      columns carry |c|^2 / 2 - m.c + |m|^2 / 2, so that the accumulator holds F (score + a constant of the row), F = 2^e /
+//      cp, within (-0.5, 0.5).  `eps` of a row bounds how far that is from the exact value: the measured norms of what
+//      rounding took from row and lists, accumulation, the defining chain's own rounding, the rounding of the keys.
+//      Where the epilogue is the longer part (up to 190 dimensions) the row operand comes as two halfs, hi + lo, and two
+//      products: its rounding drops out of eps at no cost in time.
 //   2. label_tc_kernel: a persistent CTA takes a tile of 128 rows against all (or a share) of the lists, 256 at a time.
-//      Per row and 64 lists of a tile the epilogue keeps the largest value as a packed key (value in fixed point, low bits
-//      the column: see coarse_tc.cu) and the second largest; across the tiles, per row and column quarter, the four
-//      largest of the former with their lists, and the largest of the latter.  Three float additions and three min / max per
-//      value: the epilogue's integer pipe and the tensor pipe are about equally busy.
-//   3. label_finish_kernel: lists within 2 eps of the largest value are rescored with the defining chain; one candidate needs
-//      no rescoring.  Where a list that was not kept might be within 2 eps, the row is redone exactly over all lists.
+//      Per row and unit of 64 lists the epilogue finds the largest value as a packed key (value in fixed point, low bits
+//      the column: see coarse_tc.cu) and the second largest; across the tiles it keeps, per row and column quarter, the
+//      units with the four largest.  Three float additions and three min / max per value, which bound the kernel.
+//   3. label_finish_kernel: units within 2 eps of the largest value are looked at.  One such unit whose second value is
+//      outside: that is the label.  Several: their lists are rescored with the defining chain.  Units whose second value
+//      is inside too go to label_units_kernel, which rescores all 64 lists of them.  If the fourth unit kept is inside,
+//      a fifth might be: the row is redone exactly over all lists.
 // Every wait is bounded: on a time-out the kernel raises the error word and returns, and all rows are redone.
 #include "search_internal.hpp"
 #include "tc_ptx.cuh"
@@ -37,89 +41,174 @@ constexpr uint32_t kABlock = kRows * kBlockK * 2, kBBlock = kLists * kBlockK * 2
 constexpr uint32_t kMaxStages = 6;
 constexpr uint32_t kRoom      = 6 * kBBlock;          // shared memory for operands: 192 KB
 
-// model words: [0] bits of the largest of |c|^2 and the norm column, [1] the power of two cp, [2] largest |c| / cp
-__global__ void center_stats_kernel(const float* __restrict__ centers, uint32_t n_lists, uint32_t dim, uint32_t dim_ext,
-                                    uint32_t* __restrict__ words)
+// Model: words {bits of the largest max(|c - m|^2, 2 |norm column|), of the largest |c|^2 or norm column, of the largest
+// squared norm of what rounding took from a list}, the sum of the centres at kMeanAt, the list operand at operand_at(dim).
+constexpr uint32_t kMeanAt = 256;
+__host__ __device__ __forceinline__ size_t operand_at(uint32_t dim) { return kMeanAt + round_up<size_t>(size_t(dim) * 4, 256); }
+
+__global__ void center_sum_kernel(const float* __restrict__ centers, uint32_t n_lists, uint32_t dim, uint32_t dim_ext,
+                                  float* __restrict__ sum)
 {
-  const uint32_t l    = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const uint32_t lane = threadIdx.x & 31u;
-  if (l >= n_lists) { return; }
-  const float* c = centers + size_t(l) * dim_ext;
-  float ss       = 0.0f;
-  for (uint32_t k = lane; k < dim; k += 32) { ss = __fmaf_rn(c[k], c[k], ss); }
+  // block (32 dimensions, 8 list lanes); blockIdx.y: a share of the lists
+  __shared__ float s_part[8][33];
+  const uint32_t k = blockIdx.x * 32u + threadIdx.x;
+  float acc        = 0.0f;
+  if (k < dim) {
+#pragma unroll 8
+    for (uint32_t l = blockIdx.y * 8u + threadIdx.y; l < n_lists; l += gridDim.y * 8u) { acc += centers[size_t(l) * dim_ext + k]; }
+  }
+  s_part[threadIdx.y][threadIdx.x] = acc;
+  __syncthreads();
+  if (threadIdx.y == 0 && k < dim) {
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) { ss += __shfl_xor_sync(kFullMask, ss, o); }
-  if (lane == 0) { atomicMax(words, __float_as_uint(fmaxf(ss, fabsf(c[dim])) * 1.0001f)); }
+    for (uint32_t y = 1; y < 8; y++) { acc += s_part[y][threadIdx.x]; }
+    atomicAdd(sum + k, acc);
+  }
 }
 
-// cp = the smallest power of two that is at least sqrt(largest squared norm)
+// |c|^2 / 2 - m.c + |m|^2 / 2 of a list, by one warp (any m gives valid results: it only has to be the same everywhere)
+__device__ __forceinline__ void list_norms(const float* c, const float* sum, float inv_n, uint32_t dim, float& cc, float& dd, double& norm)
+{
+  const uint32_t lane = threadIdx.x & 31u;
+  double mc = 0.0, mm = 0.0;
+  cc = dd = 0.0f;
+  for (uint32_t k = lane; k < dim; k += 32) {
+    const float m = sum[k] * inv_n, v = c[k], d = v - m;
+    mc += double(m) * v;
+    mm += double(m) * m;
+    cc = __fmaf_rn(v, v, cc);
+    dd = __fmaf_rn(d, d, dd);
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    mc += __shfl_xor_sync(kFullMask, mc, o);
+    mm += __shfl_xor_sync(kFullMask, mm, o);
+    cc += __shfl_xor_sync(kFullMask, cc, o);
+    dd += __shfl_xor_sync(kFullMask, dd, o);
+  }
+  norm = 0.5 * double(c[dim]) - mc + 0.5 * mm;
+}
+
+__global__ void center_stats_kernel(const float* __restrict__ centers, uint32_t n_lists, uint32_t dim, uint32_t dim_ext,
+                                    const float* __restrict__ sum, uint32_t* __restrict__ words)
+{
+  const uint32_t l = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  if (l >= n_lists) { return; }
+  const float* c = centers + size_t(l) * dim_ext;
+  float cc, dd;
+  double norm;
+  list_norms(c, sum, 1.0f / float(n_lists), dim, cc, dd, norm);
+  if ((threadIdx.x & 31u) == 0) {
+    atomicMax(words, __float_as_uint(fmaxf(dd, 2.0f * fabsf(float(norm))) * 1.0001f));
+    atomicMax(words + 1, __float_as_uint(fmaxf(cc, fabsf(c[dim])) * 1.0001f));
+  }
+}
+
+// cp = a power of two above sqrt(largest squared norm); bn = that norm / cp, infinite where no bound holds
 __device__ __forceinline__ float center_scale(const uint32_t* words, float& bn)
 {
   const float nrm = sqrtf(__uint_as_float(__ldg(words)));
   const int E     = int((__float_as_uint(nrm) >> 23) & 0xFFu);   // nrm in [2^(E-127), 2^(E-126))
   const bool fine = E >= 64 && E <= 190;
   const float cp  = fine ? __uint_as_float(uint32_t(E + 1) << 23) : 1.0f;
-  bn              = fine ? nrm / cp * 1.0001f : INFINITY;       // out of range: no bound holds, every row is redone
+  bn              = fine ? nrm / cp * 1.0001f : INFINITY;
   return cp;
 }
 
+// One warp per list.
 __global__ void center_operand_kernel(const float* __restrict__ centers, uint32_t n_lists, uint32_t dim, uint32_t dim_ext,
-                                      uint32_t width, const uint32_t* __restrict__ words, __half* __restrict__ out)
+                                      uint32_t width, const float* __restrict__ sum, uint32_t* __restrict__ words,
+                                      __half* __restrict__ out)
 {
-  const size_t i = blockIdx.x * size_t(blockDim.x) + threadIdx.x;
-  if (i >= size_t(n_lists) * width) { return; }
-  const uint32_t l = uint32_t(i / width), k = uint32_t(i - size_t(l) * width);
-  float bn;
-  const float inv = 1.0f / center_scale(words, bn);
-  const float* c  = centers + size_t(l) * dim_ext;
-  float v         = 0.0f;
-  if (k < dim) {
-    v = c[k] * inv;
-  } else if (k < dim + 2) {
-    const float n  = 0.5f * c[dim] * inv * inv;
-    const float hi = __half2float(__float2half_rn(n));
-    v              = k == dim ? hi : n - hi;
+  const uint32_t l = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31u;
+  if (l >= n_lists) { return; }
+  float bn, cc, dd;
+  const float inv   = 1.0f / center_scale(words, bn);
+  const float inv_n = 1.0f / float(n_lists);
+  const float* c    = centers + size_t(l) * dim_ext;
+  double norm;
+  list_norms(c, sum, inv_n, dim, cc, dd, norm);
+  const float nf = float(norm * double(inv) * double(inv));
+  const float hi = __half2float(__float2half_rn(nf));
+  __half* dst    = out + size_t(l) * width;
+  float lost     = 0.0f;
+  for (uint32_t k = lane; k < width; k += 32) {
+    const float v  = k < dim ? (c[k] - sum[k] * inv_n) * inv : (k == dim ? hi : (k == dim + 1 ? nf - hi : 0.0f));
+    const __half h = __float2half_rn(v);
+    dst[k]         = h;
+    if (k < dim) {
+      const float d = v - __half2float(h);
+      lost          = __fmaf_rn(d, d, lost);
+    }
   }
-  out[i] = __float2half_rn(v);
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) { lost += __shfl_xor_sync(kFullMask, lost, o); }
+  if (lane == 0) { atomicMax(words + 2, __float_as_uint(lost * 1.001f)); }
 }
 
-// One warp per row: the operand row, and eps (infinite: the row has to be redone).
-__global__ void row_operand_kernel(const float* __restrict__ x, uint32_t n_rows, uint32_t dim, uint32_t dim_ext,
-                                   uint32_t width, const uint32_t* __restrict__ words, __half* __restrict__ out,
-                                   float* __restrict__ eps)
+// One warp per row: the operand row (kSplit: hi, then lo, `width` halfs each), and eps (infinite: redo the row).
+template <bool kSplit>
+__global__ void row_operand_kernel(const float* __restrict__ x, uint32_t n_rows, uint32_t n_lists, uint32_t dim, uint32_t dim_ext,
+                                   uint32_t width, const float* __restrict__ sum, const uint32_t* __restrict__ words,
+                                   __half* __restrict__ out, float* __restrict__ eps)
 {
   const uint32_t r    = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const uint32_t lane = threadIdx.x & 31u;
   if (r >= n_rows) { return; }
   float bn;
-  const float cp = center_scale(words, bn);
-  const float* q = x + size_t(r) * dim_ext;
-  float ss       = 0.0f;
-  for (uint32_t k = lane; k < dim; k += 32) { ss = __fmaf_rn(q[k], q[k], ss); }
+  const float cp    = center_scale(words, bn);
+  const float inv_n = 1.0f / float(n_lists);
+  const float* q    = x + size_t(r) * dim_ext;
+  float ss = 0.0f, qq = 0.0f;
+  for (uint32_t k = lane; k < dim; k += 32) {
+    const float v = q[k], d = v - sum[k] * inv_n;
+    ss = __fmaf_rn(d, d, ss);
+    qq = __fmaf_rn(v, v, qq);
+  }
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) { ss += __shfl_xor_sync(kFullMask, ss, o); }
-  const float qn = sqrtf(ss) * 1.0001f;
-  // 2^e (|q| + cp / 2) in [0.25, 0.5)
-  const float b     = (qn + 0.5f * cp) * 1.01f;
+  for (int o = 16; o > 0; o >>= 1) {
+    ss += __shfl_xor_sync(kFullMask, ss, o);
+    qq += __shfl_xor_sync(kFullMask, qq, o);
+  }
+  const float dn = sqrtf(ss) * 1.0001f, qn = sqrtf(qq) * 1.0001f;
+  // 2^e (|q - m| + cp / 2) in [0.25, 0.5)
+  const float b     = (dn + 0.5f * cp) * 1.01f;
   const int E       = int((__float_as_uint(b) >> 23) & 0xFFu);
   const bool fine   = E >= 2 && E <= 250;
   const float scale = fine ? __uint_as_float(uint32_t(252 - E) << 23) : 0.0f;
   const float a     = scale * cp;
-  __half2* dst      = reinterpret_cast<__half2*>(out + size_t(r) * width);
+  __half2* dst      = reinterpret_cast<__half2*>(out + size_t(r) * width * (kSplit ? 2u : 1u));
+  float lost        = 0.0f;
   for (uint32_t k2 = lane; k2 < width / 2; k2 += 32) {
     float v[2];
 #pragma unroll
     for (uint32_t e = 0; e < 2; e++) {
       const uint32_t k = 2 * k2 + e;
-      v[e]             = k < dim ? q[k] * scale : (k < dim + 2 ? -a : 0.0f);
+      v[e]             = k < dim ? (q[k] - sum[k] * inv_n) * scale : (k < dim + 2 ? -a : 0.0f);
     }
-    dst[k2] = __floats2half2_rn(v[0], v[1]);
+    const __half2 h = __floats2half2_rn(v[0], v[1]);
+    float2 f        = __half22float2(h);
+    dst[k2]         = h;
+    f               = make_float2(v[0] - f.x, v[1] - f.y);
+    if constexpr (kSplit) {
+      const __half2 lo     = __floats2half2_rn(f.x, f.y);
+      const float2 g       = __half22float2(lo);
+      dst[width / 2 + k2] = lo;
+      f                    = make_float2(f.x - g.x, f.y - g.y);
+    }
+    lost = __fmaf_rn(f.x, f.x, lost);
+    lost = __fmaf_rn(f.y, f.y, lost);
   }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) { lost += __shfl_xor_sync(kFullMask, lost, o); }
   if (lane == 0) {
-    const float an = qn * scale, w = float(width);
-    // operands rounded to half precision (relative, and absolute near zero), accumulation, the exact chain's own
-    // rounding, the key's
-    float e = 9.9e-4f * an * bn + sqrtf(w) * 3.0e-8f * (an + bn) + (w + 24.0f) * 2.4e-7f + float(dim_ext) * 1.2e-7f + 7.7e-6f;
+    const float an = dn * scale, w = float(width);
+    const float bl = sqrtf(__uint_as_float(__ldg(words + 2))), cn = sqrtf(__uint_as_float(__ldg(words + 1)));
+    const float orig = qn * cn + 0.5f * cn * cn;  // bounds every partial sum of the defining chain
+    float e = (sqrtf(lost) * (bn + bl) + an * bl) * 1.01f       // rounding of the operands
+              + (w + 24.0f) * (kSplit ? 1.8e-7f : 1.2e-7f)      // accumulation of sums below 0.5 by the tensor core
+              + (scale / cp) * orig * (float(dim_ext) + 4.0f) * 1.2e-7f  // the defining chain, and q - m
+              + 8.2e-6f;                                        // norm columns, keys
     if (!fine || !(a >= 6.2e-5f)) { e = INFINITY; }
     eps[r] = e;
   }
@@ -128,10 +217,10 @@ __global__ void row_operand_kernel(const float* __restrict__ x, uint32_t n_rows,
 struct label_params {
   uint32_t n_rows, n_lists, k_steps /* of 16 halfs */, k_blocks;
   uint32_t n_tiles, tiles_per_split, n_items, splits;
-  uint32_t a_resident, n_stages;
+  uint32_t a_resident, n_stages, products, width;
   uint4* keys;       // [splits, n_rows, 4] largest keys of a column quarter
+  uint4* seconds;    // second largest keys of their units
   uint4* lists;      // their lists
-  uint32_t* bounds;  // [splits, n_rows, 4] key of the largest value that a 64-list unit of a tile dropped
   uint32_t* error;
   uint32_t spin_limit;
 };
@@ -152,7 +241,7 @@ label_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
   const uint32_t bar_aempty = bar_afull + 8;
   uint32_t* tmem_slot       = reinterpret_cast<uint32_t*>(bars + 2 * kMaxStages + 6);
   // [row tile, when resident][stages: list block, then row block when not]
-  const uint32_t a_bytes    = p.a_resident ? p.k_blocks * kABlock : 0u;
+  const uint32_t a_bytes    = p.a_resident ? p.products * p.k_blocks * kABlock : 0u;
   const uint32_t stage_size = kBBlock + (p.a_resident ? 0u : kABlock);
   const uint32_t stage_base = base_a + a_bytes;
   const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
@@ -202,8 +291,10 @@ label_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
           }
           n_a++;
           mbar_arrive_expect_tx(bar_afull, a_bytes);
-          for (uint32_t kb = 0; kb < p.k_blocks; kb++) {
-            tma_load_2d(base_a + kb * kABlock, &map_a, bar_afull, int(kb * kBlockK), row0);
+          for (uint32_t i = 0; i < p.products; i++) {
+            for (uint32_t kb = 0; kb < p.k_blocks; kb++) {
+              tma_load_2d(base_a + (i * p.k_blocks + kb) * kABlock, &map_a, bar_afull, int(i * p.width + kb * kBlockK), row0);
+            }
           }
         }
         for (uint32_t t = t0; ok && t < t1; t++) {
@@ -264,6 +355,14 @@ label_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
               if (k >= nk) { break; }
               tc_mma_f16(tmem_d, da + k * 2u, db + k * 2u, idesc, (kb | k) != 0u);  // 32 bytes of K per step
             }
+            if (p.products == 2u) {
+              const uint64_t dl = make_desc_sw128(base_a + (p.k_blocks + kb) * kABlock);
+#pragma unroll
+              for (uint32_t k = 0; k < 4; k++) {
+                if (k >= nk) { break; }
+                tc_mma_f16(tmem_d, dl + k * 2u, db + k * 2u, idesc, 1u);
+              }
+            }
             tc_commit(bar_empty + stage * 8);
             if (++stage == p.n_stages) {
               stage = 0;
@@ -283,7 +382,7 @@ label_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
     for (uint32_t item = blockIdx.x; ok && item < p.n_items; item += gridDim.x) {
       uint32_t t0, t1;
       tiles_of(item, t0, t1);
-      uint32_t key[kKeep] = {0u, 0u, 0u, 0u}, list[kKeep] = {0u, 0u, 0u, 0u}, bound = 0u;
+      uint32_t key[kKeep] = {0u, 0u, 0u, 0u}, second[kKeep] = {0u, 0u, 0u, 0u}, list[kKeep] = {0u, 0u, 0u, 0u};
       for (uint32_t t = t0; t < t1; t++, it++) {
         const uint32_t acc = it & 1u;
         if (ok && !mbar_wait(bar_tfull + acc * 8, (it >> 1) & 1u, p.spin_limit)) { ok = false; }
@@ -322,18 +421,20 @@ label_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
         tc_fence_before();
         __syncwarp();
         if (lane == 0) { mbar_arrive(bar_tempty + acc * 8); }
-        bound = max(bound, l1);
         if (l0 > key[kKeep - 1]) {
-          key[kKeep - 1]  = l0;
+          key[kKeep - 1]    = l0;
+          second[kKeep - 1] = l1;
           list[kKeep - 1] = n0 + (63u - (l0 & 127u));
 #pragma unroll
           for (int i = int(kKeep) - 1; i > 0; i--) {
             if (key[i] > key[i - 1]) {
-              const uint32_t a = key[i], b = list[i];
-              key[i]      = key[i - 1];
-              list[i]     = list[i - 1];
-              key[i - 1]  = a;
-              list[i - 1] = b;
+              const uint32_t a = key[i], b = list[i], c = second[i];
+              key[i]        = key[i - 1];
+              list[i]       = list[i - 1];
+              second[i]     = second[i - 1];
+              key[i - 1]    = a;
+              list[i - 1]   = b;
+              second[i - 1] = c;
             }
           }
         }
@@ -343,7 +444,7 @@ label_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
         const size_t at = (size_t(item % p.splits) * p.n_rows + row) * 4u + unit;
         p.keys[at]      = make_uint4(key[0], key[1], key[2], key[3]);
         p.lists[at]     = make_uint4(list[0], list[1], list[2], list[3]);
-        p.bounds[at]    = bound;
+        p.seconds[at]   = make_uint4(second[0], second[1], second[2], second[3]);
       }
     }
   }
@@ -366,73 +467,92 @@ __device__ __forceinline__ float key_value(uint32_t key)
   return key >= 0x00800000u ? __fadd_rn(__uint_as_float(key & ~127u), -1.5f) : -INFINITY;
 }
 
-// Four lanes per row: lane u reads what column quarter u kept (of every split).
+struct label_records {
+  const uint4* keys;
+  const uint4* seconds;
+  const uint4* lists;
+  const float* eps;
+  const uint32_t* error;
+  uint32_t splits, n_rows, n_lists;
+};
+
+// the defining chain of one list
+__device__ __forceinline__ uint64_t exact_key(const float* q, const float* centers, uint32_t list, uint32_t dim_ext, float alpha)
+{
+  const float4* c = reinterpret_cast<const float4*>(centers + size_t(list) * dim_ext);
+  float acc       = 0.0f;
+#pragma unroll 4
+  for (uint32_t k4 = 0; k4 < dim_ext / 4; k4++) {  // dim_ext is a multiple of 8
+    const float4 cv = __ldg(c + k4), qv = __ldg(reinterpret_cast<const float4*>(q) + k4);
+    acc             = __fmaf_rn(cv.x, qv.x, acc);
+    acc             = __fmaf_rn(cv.y, qv.y, acc);
+    acc             = __fmaf_rn(cv.z, qv.z, acc);
+    acc             = __fmaf_rn(cv.w, qv.w, acc);
+  }
+  return make_key(__fmul_rn(alpha, acc), list);
+}
+
+// Four lanes per row: lane u reads what column quarter u kept (of every split).  Rows for the other two passes are
+// listed: redo[0 .. counts[0]) from the front, whole units from the back (counts[1] of them).
 __global__ void __launch_bounds__(256)
-label_finish_kernel(const uint4* __restrict__ keys, const uint4* __restrict__ lists, const uint32_t* __restrict__ bounds,
-                    uint32_t splits, uint32_t n_rows, const float* __restrict__ eps, const uint32_t* __restrict__ error,
-                    const float* __restrict__ x, const float* __restrict__ centers, uint32_t dim_ext, float alpha,
-                    uint32_t* __restrict__ labels, uint32_t* __restrict__ redo, uint32_t* __restrict__ n_redo)
+label_finish_kernel(const label_records p, const float* __restrict__ x, const float* __restrict__ centers, uint32_t dim_ext,
+                    float alpha, uint32_t* __restrict__ labels, uint32_t* __restrict__ redo, uint32_t* __restrict__ counts)
 {
   const uint32_t r = (blockIdx.x * 256u + threadIdx.x) >> 2, u = threadIdx.x & 3u;
   const unsigned mask = 0xFu << (threadIdx.x & 28u);
-  if (r >= n_rows) { return; }
-  float top = -INFINITY, out = -INFINITY;  // largest value kept, largest that may have been dropped
-  for (uint32_t s = 0; s < splits; s++) {
-    const size_t at = (size_t(s) * n_rows + r) * 4u + u;
-    const uint4 k   = __ldg(keys + at);
-    top             = fmaxf(top, key_value(k.x));
-    out             = fmaxf(out, fmaxf(key_value(k.w), key_value(__ldg(bounds + at))));
+  if (r >= p.n_rows) { return; }
+  float top = -INFINITY, out = -INFINITY;  // largest value, largest that bounds units not kept
+  for (uint32_t s = 0; s < p.splits; s++) {
+    const uint4 k = __ldg(p.keys + (size_t(s) * p.n_rows + r) * 4u + u);
+    top           = fmaxf(top, key_value(k.x));
+    out           = fmaxf(out, key_value(k.w));
   }
 #pragma unroll
   for (int o = 2; o > 0; o >>= 1) {
     top = fmaxf(top, __shfl_xor_sync(mask, top, o));
     out = fmaxf(out, __shfl_xor_sync(mask, out, o));
   }
-  const float t = top - 2.0f * __ldg(eps + r);
+  const float t = top - 2.0f * __ldg(p.eps + r);
   // (negated: an infinite or undefined bound is not proof)
-  if (*error != 0u || !(out < t)) {
-    if (u == 0) { redo[atomicAdd(n_redo, 1u)] = r; }
+  if (*p.error != 0u || !(out < t)) {
+    if (u == 0) { redo[atomicAdd(counts, 1u)] = r; }
     return;
   }
-  // candidates
   uint32_t n = 0, only = 0xFFFFFFFFu;
-  for (uint32_t s = 0; s < splits; s++) {
-    const size_t at = (size_t(s) * n_rows + r) * 4u + u;
-    const uint4 k   = __ldg(keys + at);
+  bool more  = false;
+  for (uint32_t s = 0; s < p.splits; s++) {
+    const size_t at = (size_t(s) * p.n_rows + r) * 4u + u;
+    const uint4 k   = __ldg(p.keys + at);
     if (key_value(k.x) >= t) {
-      const uint4 l = __ldg(lists + at);
+      const uint4 b = __ldg(p.seconds + at);
+      only          = __ldg(&p.lists[at].x);
       n += 1u + (key_value(k.y) >= t ? 1u : 0u) + (key_value(k.z) >= t ? 1u : 0u);
-      only = l.x;
+      more = more || key_value(b.x) >= t || (key_value(k.y) >= t && key_value(b.y) >= t) ||
+             (key_value(k.z) >= t && key_value(b.z) >= t);
     }
   }
   uint32_t all = n;
 #pragma unroll
   for (int o = 2; o > 0; o >>= 1) { all += __shfl_xor_sync(mask, all, o); }
+  if (__any_sync(mask, more)) {
+    if (u == 0) { redo[p.n_rows - 1u - atomicAdd(counts + 1, 1u)] = r; }
+    return;
+  }
   if (all == 1u) {
     if (n == 1u) { labels[r] = only; }
     return;
   }
-  // each lane rescores its own (rarely more than one) with the defining chain
-  const float* q = x + size_t(r) * dim_ext;
-  uint64_t best  = kEmptyKey;
+  // each lane rescores its own (rarely more than one)
+  uint64_t best = kEmptyKey;
   if (n > 0) {
-    for (uint32_t s = 0; s < splits; s++) {
-      const size_t at     = (size_t(s) * n_rows + r) * 4u + u;
-      const uint4 k       = __ldg(keys + at), l = __ldg(lists + at);
+    for (uint32_t s = 0; s < p.splits; s++) {
+      const size_t at      = (size_t(s) * p.n_rows + r) * 4u + u;
+      const uint4 k        = __ldg(p.keys + at), l = __ldg(p.lists + at);
       const uint32_t kk[3] = {k.x, k.y, k.z}, ll[3] = {l.x, l.y, l.z};
 #pragma unroll
       for (int i = 0; i < 3; i++) {
         if (key_value(kk[i]) < t) { continue; }
-        const float4* c = reinterpret_cast<const float4*>(centers + size_t(ll[i]) * dim_ext);
-        float acc       = 0.0f;
-        for (uint32_t k4 = 0; k4 < dim_ext / 4; k4++) {  // dim_ext is a multiple of 8
-          const float4 cv = __ldg(c + k4), qv = __ldg(reinterpret_cast<const float4*>(q) + k4);
-          acc             = __fmaf_rn(cv.x, qv.x, acc);
-          acc             = __fmaf_rn(cv.y, qv.y, acc);
-          acc             = __fmaf_rn(cv.z, qv.z, acc);
-          acc             = __fmaf_rn(cv.w, qv.w, acc);
-        }
-        const uint64_t key = make_key(__fmul_rn(alpha, acc), ll[i]);
+        const uint64_t key = exact_key(x + size_t(r) * dim_ext, centers, ll[i], dim_ext, alpha);
         best               = key < best ? key : best;
       }
     }
@@ -446,7 +566,55 @@ label_finish_kernel(const uint4* __restrict__ keys, const uint4* __restrict__ li
   if (u == 0) { labels[r] = uint32_t(best); }
 }
 
+// Rows with units whose second value is within reach: one warp per row rescores every list of such units, and the single
+// lists of the others.
+__global__ void __launch_bounds__(256)
+label_units_kernel(const label_records p, const float* __restrict__ x, const float* __restrict__ centers, uint32_t dim_ext,
+                   float alpha, uint32_t* __restrict__ labels, const uint32_t* __restrict__ redo, const uint32_t* __restrict__ counts)
+{
+  const uint32_t lane = threadIdx.x & 31u;
+  const uint32_t n    = __ldg(counts + 1);
+  for (uint32_t i = (blockIdx.x * 256u + threadIdx.x) >> 5; i < n; i += gridDim.x * 8u) {
+    const uint32_t r = redo[p.n_rows - 1u - i];
+    const float* q   = x + size_t(r) * dim_ext;
+    // lane 4 u + j: unit j of column quarter u
+    const uint32_t* keys = reinterpret_cast<const uint32_t*>(p.keys);
+    auto at = [&](uint32_t s) { return (size_t(s) * p.n_rows + r) * 16u + (lane & 15u); };
+    float top = -INFINITY;
+    for (uint32_t s = 0; s < p.splits; s++) { top = fmaxf(top, key_value(__ldg(keys + at(s)))); }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) { top = fmaxf(top, __shfl_xor_sync(kFullMask, top, o)); }
+    const float t = top - 2.0f * __ldg(p.eps + r);
+    uint64_t best = kEmptyKey;
+    for (uint32_t s = 0; s < p.splits; s++) {
+      const bool in       = lane < 16u && key_value(__ldg(keys + at(s))) >= t;
+      const bool whole    = in && key_value(__ldg(reinterpret_cast<const uint32_t*>(p.seconds) + at(s))) >= t;
+      const uint32_t list = in ? __ldg(reinterpret_cast<const uint32_t*>(p.lists) + at(s)) : 0u;
+      if (in && !whole) {
+        const uint64_t key = exact_key(q, centers, list, dim_ext, alpha);
+        best               = key < best ? key : best;
+      }
+      unsigned m = __ballot_sync(kFullMask, whole);
+      while (m) {
+        const uint32_t base = __shfl_sync(kFullMask, list, __ffs(m) - 1) & ~(kUnit - 1u);
+        m &= m - 1;
+        for (uint32_t l = base + lane; l < min(base + kUnit, p.n_lists); l += 32) {
+          const uint64_t key = exact_key(q, centers, l, dim_ext, alpha);
+          best               = key < best ? key : best;
+        }
+      }
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      const uint64_t other = shfl_u64(best, int(lane) ^ o);
+      best                 = other < best ? other : best;
+    }
+    if (lane == 0) { labels[r] = uint32_t(best); }
+  }
+}
+
 uint32_t operand_width(uint32_t dim) { return round_up(dim + 2u, 16u); }
+uint32_t operand_products(uint32_t dim) { return ceildiv(operand_width(dim), kBlockK) <= 3u ? 2u : 1u; }
 
 }  // namespace
 
@@ -456,24 +624,26 @@ bool label_tc_usable(uint32_t n_rows, uint32_t n_lists)
   return n_lists >= 256 && uint64_t(n_rows) * n_lists >= (1ull << 24);
 }
 
-size_t label_model_bytes(uint32_t n_lists, uint32_t dim) { return size_t(n_lists) * operand_width(dim) * 2 + 256; }
+size_t label_model_bytes(uint32_t n_lists, uint32_t dim) { return operand_at(dim) + size_t(n_lists) * operand_width(dim) * 2; }
 
 void prepare_label_model(cudaStream_t stream, const float* centers, uint32_t n_lists, uint32_t dim, uint32_t dim_ext, void* model)
 {
   auto* words = static_cast<uint32_t*>(model);
-  auto* b     = reinterpret_cast<__half*>(static_cast<char*>(model) + 256);
-  CUDA_TRY(cudaMemsetAsync(words, 0, 16, stream));
-  center_stats_kernel<<<ceildiv<uint32_t>(n_lists * 32u, 256u), 256, 0, stream>>>(centers, n_lists, dim, dim_ext, words);
-  const size_t n = size_t(n_lists) * operand_width(dim);
-  center_operand_kernel<<<unsigned(ceildiv<size_t>(n, 256)), 256, 0, stream>>>(centers, n_lists, dim, dim_ext,
-                                                                              operand_width(dim), words, b);
+  auto* sum   = reinterpret_cast<float*>(static_cast<char*>(model) + kMeanAt);
+  auto* b     = reinterpret_cast<__half*>(static_cast<char*>(model) + operand_at(dim));
+  CUDA_TRY(cudaMemsetAsync(model, 0, operand_at(dim), stream));
+  const uint32_t shares = std::min<uint32_t>(64, ceildiv(n_lists, 64u));
+  center_sum_kernel<<<dim3(ceildiv(dim, 32u), shares), dim3(32, 8), 0, stream>>>(centers, n_lists, dim, dim_ext, sum);
+  center_stats_kernel<<<ceildiv<uint32_t>(n_lists, 8u), 256, 0, stream>>>(centers, n_lists, dim, dim_ext, sum, words);
+  center_operand_kernel<<<ceildiv<uint32_t>(n_lists, 8u), 256, 0, stream>>>(centers, n_lists, dim, dim_ext, operand_width(dim), sum,
+                                                                           words, b);
   CUDA_TRY(cudaGetLastError());
 }
 
 namespace {
 struct label_layout {
   uint32_t splits, tiles_per_split;
-  size_t o_a, o_eps, o_keys, o_lists, o_bounds, o_redo, o_words, o_best, total;
+  size_t o_a, o_eps, o_keys, o_seconds, o_lists, o_redo, o_words, o_best, total;
 };
 label_layout layout_for(uint32_t n_rows, uint32_t n_lists, uint32_t dim, int sm_count)
 {
@@ -487,11 +657,11 @@ label_layout layout_for(uint32_t n_rows, uint32_t n_lists, uint32_t dim, int sm_
   y.splits          = ceildiv(n_tiles, y.tiles_per_split);
   const size_t recs = size_t(y.splits) * n_rows * 4;
   ws_layout lay;
-  y.o_a      = lay.add(size_t(n_rows) * operand_width(dim) * 2);
+  y.o_a      = lay.add(size_t(n_rows) * operand_width(dim) * operand_products(dim) * 2);
   y.o_eps    = lay.add(size_t(n_rows) * 4);
   y.o_keys   = lay.add(recs * 16);
   y.o_lists  = lay.add(recs * 16);
-  y.o_bounds = lay.add(recs * 4);
+  y.o_seconds = lay.add(recs * 16);
   y.o_redo   = lay.add(size_t(n_rows) * 4);
   y.o_words  = lay.add(256);
   y.o_best   = lay.add(size_t(n_rows) * 8);
@@ -517,11 +687,18 @@ void label_rows_tc(raft::resources& res, const float* centers, const void* model
   auto* words          = reinterpret_cast<uint32_t*>(ws + y.o_words);  // error, rows to redo
   auto* redo           = reinterpret_cast<uint32_t*>(ws + y.o_redo);
   auto* best           = reinterpret_cast<unsigned long long*>(ws + y.o_best);
-  const auto* b        = reinterpret_cast<const __half*>(static_cast<const char*>(model) + 256);
+  const auto* stats    = static_cast<const uint32_t*>(model);
+  const auto* sum      = reinterpret_cast<const float*>(static_cast<const char*>(model) + kMeanAt);
+  const auto* b        = reinterpret_cast<const __half*>(static_cast<const char*>(model) + operand_at(dim));
   cudaStream_t stream  = res.stream;
-  CUDA_TRY(cudaMemsetAsync(words, 0, 8, stream));
-  row_operand_kernel<<<ceildiv<uint32_t>(n_rows, 8u), 256, 0, stream>>>(x_ext, n_rows, dim, dim_ext, width,
-                                                                        static_cast<const uint32_t*>(model), a, eps);
+  CUDA_TRY(cudaMemsetAsync(words, 0, 12, stream));
+  const uint32_t products = operand_products(dim);
+  const uint32_t blocks   = ceildiv<uint32_t>(n_rows, 8u);
+  if (products == 2) {
+    row_operand_kernel<true><<<blocks, 256, 0, stream>>>(x_ext, n_rows, n_lists, dim, dim_ext, width, sum, stats, a, eps);
+  } else {
+    row_operand_kernel<false><<<blocks, 256, 0, stream>>>(x_ext, n_rows, n_lists, dim, dim_ext, width, sum, stats, a, eps);
+  }
   label_params p{};
   p.n_rows          = n_rows;
   p.n_lists         = n_lists;
@@ -531,24 +708,30 @@ void label_rows_tc(raft::resources& res, const float* centers, const void* model
   p.tiles_per_split = y.tiles_per_split;
   p.splits          = y.splits;
   p.n_items         = ceildiv(n_rows, kRows) * y.splits;
-  // the row tile stays in shared memory where that leaves at least three list stages (dim <= 382)
-  p.a_resident = p.k_blocks * kABlock + 3 * kBBlock <= kRoom;
-  p.n_stages   = p.a_resident ? std::min(kMaxStages, (kRoom - p.k_blocks * kABlock) / kBBlock) : kRoom / (kABlock + kBBlock);
+  // the row tile stays in shared memory where that leaves at least three list stages
+  const uint32_t a_size = products * p.k_blocks * kABlock;
+  p.products   = products;
+  p.width      = width;
+  p.a_resident = a_size + 3 * kBBlock <= kRoom;
+  CUVS_EXPECTS(p.a_resident || products == 1, "internal error: split row operands are resident");
+  p.n_stages   = p.a_resident ? std::min(kMaxStages, (kRoom - a_size) / kBBlock) : kRoom / (kABlock + kBBlock);
   p.keys       = reinterpret_cast<uint4*>(ws + y.o_keys);
   p.lists      = reinterpret_cast<uint4*>(ws + y.o_lists);
-  p.bounds     = reinterpret_cast<uint32_t*>(ws + y.o_bounds);
+  p.seconds    = reinterpret_cast<uint4*>(ws + y.o_seconds);
   p.error      = words;
   p.spin_limit = kSpinLimit;
-  const CUtensorMap ma = make_map_2d(CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, a, n_rows, width, kRows, kBlockK, CU_TENSOR_MAP_SWIZZLE_128B);
+  const CUtensorMap ma = make_map_2d(CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, a, n_rows, uint64_t(width) * products, kRows, kBlockK, CU_TENSOR_MAP_SWIZZLE_128B);
   const CUtensorMap mb = make_map_2d(CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, b, n_lists, width, kLists, kBlockK, CU_TENSOR_MAP_SWIZZLE_128B);
   const size_t smem    = kRoom + 1024 + 256;
   ensure_dynamic_smem(reinterpret_cast<const void*>(label_tc_kernel), smem);
   label_tc_kernel<<<std::min(uint32_t(res.sm_count), p.n_items), kThreads, smem, stream>>>(ma, mb, p);
-  label_finish_kernel<<<ceildiv(n_rows, 64u), 256, 0, stream>>>(p.keys, p.lists, p.bounds, p.splits, n_rows, eps, words, x_ext,
-                                                                centers, dim_ext, alpha, labels, redo, words + 1);
+  const label_records rec{p.keys, p.seconds, p.lists, eps, words, p.splits, n_rows, n_lists};
+  label_finish_kernel<<<ceildiv(n_rows, 64u), 256, 0, stream>>>(rec, x_ext, centers, dim_ext, alpha, labels, redo, words + 1);
+  label_units_kernel<<<std::min<uint32_t>(uint32_t(res.sm_count) * 8, blocks), 256, 0, stream>>>(rec, x_ext, centers, dim_ext, alpha,
+                                                                                               labels, redo, words + 1);
   CUDA_TRY(cudaGetLastError());
   assign_nearest_listed(res, centers, n_lists, dim_ext, alpha, x_ext, n_rows, redo, words + 1, labels, best);
-  res.launches += 3;
+  res.launches += 4;
 }
 
 }  // namespace cuvs::neighbors::ivf_pq
