@@ -29,13 +29,20 @@ __device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c)
   return d;
 }
 
+__device__ __forceinline__ uint64_t dup2(float x)
+{
+  uint64_t v;
+  asm("mov.b64 %0, {%1, %1};" : "=l"(v) : "f"(x));
+  return v;
+}
+
 // out[i, j] = alpha * sum over ascending k of b[j, k] * a[i, k], one fused multiply-add chain per output (the chain that
 // defines a coarse score, a rotation, a label).  kArgmin: instead of storing, best[i] = min over j of
 // (ordered score << 32 | j), "lowest score, then lowest id".
 // What bounds it: the FMA pipe, and shared-memory wavefronts close behind.  128 x 128 outputs per block, 8 x 8 per thread
-// as packed pairs of columns (fma.rn.f32x2: two chains per instruction); the row operand sits in shared memory
-// duplicated, so that no register is spent on pairing, and the next eight k are on their way while eight are used.
-// 10,000 x 4,000 x 136: 487 us with 64 x 64 outputs per block and scalar FMAs, 358 us so.  kVec: rows of both operands are
+// as packed pairs of columns (fma.rn.f32x2: two chains per instruction), a warp 4 x 8 threads so that its loads are
+// 64 and 128 distinct bytes; the next eight k are on their way while eight are used.
+// 10,000 x 4,000 x 136: 487 us with 64 x 64 outputs per block and scalar FMAs, 238 us so.  kVec: rows of both operands are
 // 16-byte aligned and k is a multiple of four.
 constexpr uint32_t kTile = 128, kTileK = 8;
 template <bool kVec, bool kArgmin>
@@ -44,10 +51,11 @@ exact_gemm_kernel(const float* __restrict__ b, uint32_t n_cols, const float* __r
                   float alpha, int half_scores, float* __restrict__ out, unsigned long long* __restrict__ best,
                   const uint32_t* __restrict__ row_list, const uint32_t* __restrict__ n_listed)
 {
-  __shared__ __align__(16) float2 s_a[2][kTileK][kTile + 2];
+  __shared__ __align__(16) float s_a[2][kTileK][kTile + 4];
   __shared__ __align__(16) float s_b[2][kTileK][kTile + 4];
   const uint32_t j0 = blockIdx.x * kTile, i0 = blockIdx.y * kTile;
-  const uint32_t tid = threadIdx.x, tx = tid & 15u, ty = tid >> 4;
+  const uint32_t tid = threadIdx.x;
+  const uint32_t tx = ((tid >> 5) & 1u) * 8u + (tid & 7u), ty = (tid >> 6) * 4u + ((tid >> 3) & 3u);
   // `row_list` (optional): the rows of `a` (and of `best`) to do, *n_listed of them
   if (row_list != nullptr) {
     n_rows = min(n_rows, __ldg(n_listed));
@@ -78,7 +86,7 @@ exact_gemm_kernel(const float* __restrict__ b, uint32_t n_cols, const float* __r
   auto store = [&](uint32_t buf) {
 #pragma unroll
     for (uint32_t e = 0; e < 4; e++) {
-      s_a[buf][lk + e][lrow] = make_float2(ra[e], ra[e]);
+      s_a[buf][lk + e][lrow] = ra[e];
       s_b[buf][lk + e][lrow] = rb[e];
     }
   };
@@ -100,12 +108,11 @@ exact_gemm_kernel(const float* __restrict__ b, uint32_t n_cols, const float* __r
     // infinities)
     const uint32_t kn = min(kTileK, kdim - k0);
     auto step = [&](uint32_t k) {
-      const ulonglong2* qa = reinterpret_cast<const ulonglong2*>(&s_a[buf][k][ty * 4u]);
-      const ulonglong2* qb = reinterpret_cast<const ulonglong2*>(&s_a[buf][k][64u + ty * 4u]);
-      const ulonglong2 x0 = qa[0], x1 = qa[1], x2 = qb[0], x3 = qb[1];
+      const float4 x0 = *reinterpret_cast<const float4*>(&s_a[buf][k][ty * 4u]);
+      const float4 x1 = *reinterpret_cast<const float4*>(&s_a[buf][k][64u + ty * 4u]);
       const ulonglong2 c0 = *reinterpret_cast<const ulonglong2*>(&s_b[buf][k][tx * 4u]);
       const ulonglong2 c1 = *reinterpret_cast<const ulonglong2*>(&s_b[buf][k][64u + tx * 4u]);
-      const uint64_t x[8] = {x0.x, x0.y, x1.x, x1.y, x2.x, x2.y, x3.x, x3.y};
+      const uint64_t x[8] = {dup2(x0.x), dup2(x0.y), dup2(x0.z), dup2(x0.w), dup2(x1.x), dup2(x1.y), dup2(x1.z), dup2(x1.w)};
       const uint64_t c[4] = {c0.x, c0.y, c1.x, c1.y};
 #pragma unroll
       for (int i = 0; i < 8; i++) {
@@ -158,13 +165,13 @@ exact_gemm_kernel(const float* __restrict__ b, uint32_t n_cols, const float* __r
       }
     }
     if constexpr (kArgmin) {
-      // the 16 threads sharing a row sit in one half-warp: reduce before touching memory
+      // eight lanes of a warp share a row: reduce before touching memory
 #pragma unroll
-      for (int d = 8; d > 0; d >>= 1) {
+      for (int d = 4; d > 0; d >>= 1) {
         const unsigned long long o = __shfl_xor_sync(kFullMask, m, d);
         m = o < m ? o : m;
       }
-      if (tx == 0 && row < n_rows) { atomicMin(best + (row_list != nullptr ? __ldg(row_list + row) : row), m); }
+      if ((tid & 7u) == 0 && row < n_rows) { atomicMin(best + (row_list != nullptr ? __ldg(row_list + row) : row), m); }
     }
   }
 }

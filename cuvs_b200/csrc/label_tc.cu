@@ -393,10 +393,8 @@ label_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
         tc_fence_after();
         const uint32_t n0 = t * kLists + unit * kUnit;
         uint32_t l0 = 0u, l1 = 0u;
-        auto chunk = [&](auto second, auto full) {
+        auto chunk = [&](const uint32_t (&x)[32], auto second, auto full) {
           constexpr uint32_t c = decltype(second)::value ? 32u : 0u;
-          uint32_t x[32];
-          tmem_ld32(tmem_base + ((quarter * 32u) << 16) + acc * kLists + unit * kUnit + c, x);
 #pragma unroll
           for (uint32_t e = 0; e < 32; e++) {
             // value rounded to a multiple of 2^-16, + 1.5 + tag 2^-23: bits that sort, low 7 the tag 63 - column
@@ -411,12 +409,19 @@ label_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
             l0 = max(l0, k);
           }
         };
+        // (the second half is on its way while the first is looked at)
+        const uint32_t tm = tmem_base + ((quarter * 32u) << 16) + acc * kLists + unit * kUnit;
+        uint32_t x0[32], x1[32];
+        tmem_ld32(tm, x0);
+        tmem_ld32_async(tm + 32u, x1);
         if (n0 + kUnit <= p.n_lists) {
-          chunk(std::false_type{}, std::true_type{});
-          chunk(std::true_type{}, std::true_type{});
+          chunk(x0, std::false_type{}, std::true_type{});
+          tmem_ld_wait(x1);
+          chunk(x1, std::true_type{}, std::true_type{});
         } else {
-          chunk(std::false_type{}, std::false_type{});
-          chunk(std::true_type{}, std::false_type{});
+          chunk(x0, std::false_type{}, std::false_type{});
+          tmem_ld_wait(x1);
+          chunk(x1, std::true_type{}, std::false_type{});
         }
         tc_fence_before();
         __syncwarp();
