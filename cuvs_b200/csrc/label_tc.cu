@@ -346,22 +346,30 @@ label_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
               break;
             }
             tc_fence_after();
-            const uint32_t sa  = stage_base + stage * stage_size;
-            const uint64_t da  = make_desc_sw128(p.a_resident ? base_a + kb * kABlock : sa + kBBlock);
-            const uint64_t db  = make_desc_sw128(sa);
-            const uint32_t nk  = min(4u, p.k_steps - kb * 4u);
-#pragma unroll
-            for (uint32_t k = 0; k < 4; k++) {
-              if (k >= nk) { break; }
-              tc_mma_f16(tmem_d, da + k * 2u, db + k * 2u, idesc, (kb | k) != 0u);  // 32 bytes of K per step
+            const uint32_t sa = stage_base + stage * stage_size;
+            const uint32_t la = desc_sw128_lo(p.a_resident ? base_a + kb * kABlock : sa + kBBlock);
+            const uint32_t lb = desc_sw128_lo(sa);
+            const uint32_t nk = p.k_steps - kb * 4u;  // 32 bytes of K (2 descriptor units) per step
+            if (kb == 0) {
+              tc_mma_f16_lo<false>(tmem_d, la, lb, idesc);
+            } else {
+              tc_mma_f16_lo<true>(tmem_d, la, lb, idesc);
             }
-            if (p.products == 2u) {
-              const uint64_t dl = make_desc_sw128(base_a + (p.k_blocks + kb) * kABlock);
-#pragma unroll
-              for (uint32_t k = 0; k < 4; k++) {
-                if (k >= nk) { break; }
-                tc_mma_f16(tmem_d, dl + k * 2u, db + k * 2u, idesc, 1u);
+            auto rest = [&](uint32_t a) {
+              if (nk >= 4u) {
+                tc_mma_f16_lo<true>(tmem_d, a + 2u, lb + 2u, idesc);
+                tc_mma_f16_lo<true>(tmem_d, a + 4u, lb + 4u, idesc);
+                tc_mma_f16_lo<true>(tmem_d, a + 6u, lb + 6u, idesc);
+              } else {
+                if (nk >= 2u) { tc_mma_f16_lo<true>(tmem_d, a + 2u, lb + 2u, idesc); }
+                if (nk >= 3u) { tc_mma_f16_lo<true>(tmem_d, a + 4u, lb + 4u, idesc); }
               }
+            };
+            rest(la);
+            if (p.products == 2u) {
+              const uint32_t ll = la + p.k_blocks * (kABlock >> 4);
+              tc_mma_f16_lo<true>(tmem_d, ll, lb, idesc);
+              rest(ll);
             }
             tc_commit(bar_empty + stage * 8);
             if (++stage == p.n_stages) {

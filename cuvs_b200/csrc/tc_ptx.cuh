@@ -91,6 +91,22 @@ __device__ __forceinline__ uint64_t make_desc_sw128(uint32_t saddr)
   d |= uint64_t(2) << 61;                  // 128-byte swizzle
   return d;
 }
+// Low word of the descriptor above; its high word is the same for every tile.
+__device__ __forceinline__ uint32_t desc_sw128_lo(uint32_t saddr) { return ((saddr & 0x3FFFFu) >> 4) | (1u << 16); }
+// One step of 16 halfs with descriptors given by their low words: few instructions in front of every MMA, since the one
+// thread that issues them shares its scheduler with busy epilogue warps.
+template <bool kAccumulate>
+__device__ __forceinline__ void tc_mma_f16_lo(uint32_t tmem_d, uint32_t lo_a, uint32_t lo_b, uint32_t idesc)
+{
+  constexpr uint32_t kHi = (1024u >> 4) | (1u << 14) | (2u << 29);
+  asm volatile(
+    "{\n\t.reg .pred p;\n\t.reg .b64 a, b;\n\t"
+    "setp.ne.b32 p, %5, 0;\n\t"
+    "mov.b64 a, {%1, %4};\n\tmov.b64 b, {%2, %4};\n\t"
+    "tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %3, p;\n\t}"
+    ::"r"(tmem_d), "r"(lo_a), "r"(lo_b), "r"(idesc), "r"(kHi), "n"(kAccumulate ? 1 : 0)
+    : "memory");
+}
 // The load alone; tmem_ld_wait makes its registers valid.
 __device__ __forceinline__ void tmem_ld32_async(uint32_t taddr, uint32_t (&r)[32])
 {
