@@ -17,6 +17,16 @@ _NP_DL = {np.dtype(np.float32): (L.kDLFloat, 32), np.dtype(np.float16): (L.kDLFl
           np.dtype(np.int32): (L.kDLInt, 32)}
 
 
+# the raw handle of torch's current stream, without building a Stream object where torch offers that
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+
+
+def _current_stream() -> int:
+    if _raw_stream is not None:
+        return _raw_stream(torch.cuda.current_device())
+    return torch.cuda.current_stream().cuda_stream
+
+
 class Resources:
     """Mirror of ``cuvs.common.Resources``: owns a ``cuvsResources_t`` bound to the current device.
 
@@ -35,8 +45,7 @@ class Resources:
 
     def use_current_stream(self):
         if self._fixed_stream is None:
-            s = torch.cuda.current_stream().cuda_stream
-            L.check(self._lib.cuvsStreamSet(self.handle, C.c_void_p(s)))
+            L.check(self._lib.cuvsStreamSet(self.handle, _current_stream()))
 
     def sync(self):
         L.check(self._lib.cuvsStreamSync(self.handle))
@@ -64,52 +73,57 @@ def default_resources() -> Resources:
     return r
 
 
+# ndim | dtype code << 32 | bits << 40 | lanes << 48, as the words of a DLTensor hold them
+_TORCH_WORD = {t: (code << 32) | (bits << 40) | (1 << 48) for t, (code, bits) in _TORCH_DL.items()}
+_NP_WORD = {t: (code << 32) | (bits << 40) | (1 << 48) for t, (code, bits) in _NP_DL.items()}
+_WORDS = {n: C.c_int64 * (8 + 2 * n) for n in range(5)}
+
+
 class DLTensorRef:
-    """A DLManagedTensor describing (not owning) a torch tensor or a numpy array."""
+    """A DLManagedTensor describing (not owning) a torch tensor or a numpy array.
+
+    The structure, its shape and its strides are one array of 64-bit words, filled by one call: three of these are made
+    for every search, and field-by-field ctypes assignments took longer than the launches."""
+
+    __slots__ = ("_keep", "_words")
 
     def __init__(self, obj, strided: bool = False):
         """`strided`: describe a non-contiguous torch tensor by its strides (only entry points that
         say so accept one) instead of refusing it."""
-        strides = None
+        strides = ()
         if isinstance(obj, torch.Tensor):
             if not obj.is_contiguous():
                 if not strided:
                     raise ValueError("Expected a row-major matrix")
                 strides = tuple(obj.stride())
-            code, bits = _TORCH_DL[obj.dtype]
+            word = _TORCH_WORD[obj.dtype]
             if obj.is_cuda:
-                dev = L.DLDevice(L.kDLCUDA, obj.device.index or 0)
-            elif obj.is_pinned():
-                dev = L.DLDevice(L.kDLCUDAHost, 0)
+                dev = L.kDLCUDA | ((obj.get_device() or 0) << 32)
             else:
-                dev = L.DLDevice(L.kDLCPU, 0)
+                dev = L.kDLCUDAHost if obj.is_pinned() else L.kDLCPU
             ptr, shape = obj.data_ptr(), tuple(obj.shape)
         elif isinstance(obj, np.ndarray):
             if not obj.flags.c_contiguous:
                 raise ValueError("Expected a row-major matrix")
-            code, bits = _NP_DL[obj.dtype]
-            dev = L.DLDevice(L.kDLCPU, 0)
-            ptr, shape = obj.ctypes.data, tuple(obj.shape)
+            word = _NP_WORD[obj.dtype]
+            dev, ptr, shape = L.kDLCPU, obj.ctypes.data, obj.shape
         else:
             raise TypeError(f"unsupported array type {type(obj)}")
+        n = len(shape)
         self._keep = obj
-        self._shape = (C.c_int64 * max(1, len(shape)))(*shape)
-        self.managed = L.DLManagedTensor()
-        t = self.managed.dl_tensor
-        t.data = C.c_void_p(ptr)
-        t.device = dev
-        t.ndim = len(shape)
-        t.dtype = L.DLDataType(code, bits, 1)
-        t.shape = C.cast(self._shape, C.POINTER(C.c_int64))
-        if strides is None:
-            t.strides = None
-        else:
-            self._strides = (C.c_int64 * len(strides))(*strides)
-            t.strides = C.cast(self._strides, C.POINTER(C.c_int64))
-        t.byte_offset = 0
+        words = (_WORDS.get(n) or C.c_int64 * (8 + 2 * n))(ptr, dev, word | n, 0, 0, 0, 0, 0, *shape, *strides)
+        at = C.addressof(words)
+        words[3] = at + 64
+        if strides:
+            words[4] = at + 64 + 8 * n
+        self._words = words
+
+    @property
+    def managed(self):
+        return L.DLManagedTensor.from_buffer(self._words)
 
     def ref(self):
-        return C.byref(self.managed)
+        return C.byref(L.DLManagedTensor.from_buffer(self._words))
 
 
 _TYPESTR = {(L.kDLFloat, 32): "<f4", (L.kDLUInt, 32): "<u4", (L.kDLInt, 64): "<i8",

@@ -1111,7 +1111,7 @@ void launch_encode(raft::resources& res, const index<int64_t>& idx, const float*
     auto* resid = reinterpret_cast<float*>(ws + lay.add(size_t(n) * rot_dim * 4));
     difference_kernel<<<unsigned(ceildiv<uint64_t>(uint64_t(n) * dim, 256)), 256, 0, res.stream>>>(
       x_ext, labels, order, idx.centers(), n, dim, dim_ext, diff);
-    exact_rows_product(res, idx.rotation_matrix(), rot_dim, diff, n, dim, resid);
+    exact_rows_product(res, idx.rotation_matrix(), rot_dim, diff, n, dim, dim, 1.0f, resid);
     res.launches++;
     x        = resid;
     x_stride = rot_dim;

@@ -47,8 +47,8 @@ __device__ __forceinline__ uint64_t dup2(float x)
 constexpr uint32_t kTile = 128, kTileK = 8;
 template <bool kVec, bool kArgmin>
 __global__ void __launch_bounds__(256, 2)
-exact_gemm_kernel(const float* __restrict__ b, uint32_t n_cols, const float* __restrict__ a, uint32_t n_rows, uint32_t kdim,
-                  float alpha, int half_scores, float* __restrict__ out, unsigned long long* __restrict__ best,
+exact_gemm_kernel(const float* __restrict__ b, uint32_t n_cols, const float* __restrict__ a, uint32_t n_rows, uint32_t a_stride,
+                  uint32_t kdim, float alpha, int half_scores, float* __restrict__ out, unsigned long long* __restrict__ best,
                   const uint32_t* __restrict__ row_list, const uint32_t* __restrict__ n_listed)
 {
   __shared__ __align__(16) float s_a[2][kTileK][kTile + 4];
@@ -64,7 +64,7 @@ exact_gemm_kernel(const float* __restrict__ b, uint32_t n_cols, const float* __r
   // one row and four k of either operand per thread
   const uint32_t lrow = tid >> 1, lk = (tid & 1u) * 4u;
   const bool in_a = i0 + lrow < n_rows, in_b = j0 + lrow < n_cols;
-  const float* pa = a + size_t(row_list != nullptr && in_a ? __ldg(row_list + i0 + lrow) : i0 + lrow) * kdim + lk;
+  const float* pa = a + size_t(row_list != nullptr && in_a ? __ldg(row_list + i0 + lrow) : i0 + lrow) * a_stride + lk;
   const float* pb = b + size_t(j0 + lrow) * kdim + lk;
   float ra[4], rb[4];
   auto load = [&](uint32_t k0) {
@@ -182,8 +182,8 @@ exact_gemm_kernel(const float* __restrict__ b, uint32_t n_cols, const float* __r
 // rows of `a`, lane = column.
 constexpr uint32_t kFewRows = 16;
 __global__ void __launch_bounds__(128)
-few_rows_kernel(const float* __restrict__ b, uint32_t n_cols, const float* __restrict__ a, uint32_t n_rows, uint32_t kdim,
-                float alpha, int half_scores, float* __restrict__ out)
+few_rows_kernel(const float* __restrict__ b, uint32_t n_cols, const float* __restrict__ a, uint32_t n_rows, uint32_t a_stride,
+                uint32_t kdim, float alpha, int half_scores, float* __restrict__ out)
 {
   extern __shared__ float s_few[];  // [32][kdim | 1], then [n_rows][kdim]
   constexpr uint32_t kPer = kFewRows / 4;
@@ -197,7 +197,10 @@ few_rows_kernel(const float* __restrict__ b, uint32_t n_cols, const float* __res
     const uint32_t r = i / kdim;
     s_few[r * ld + (i - r * kdim)] = __ldg(src + i);
   }
-  for (uint32_t i = tid; i < n_rows * kdim; i += 128u) { s_a[i] = __ldg(a + i); }
+  for (uint32_t i = tid; i < n_rows * kdim; i += 128u) {
+    const uint32_t r = i / kdim;
+    s_a[i]           = __ldg(a + size_t(r) * a_stride + (i - r * kdim));
+  }
   __syncthreads();
   float acc[kPer] = {};
   const float* c  = s_few + lane * ld;
@@ -224,7 +227,7 @@ few_rows_kernel(const float* __restrict__ b, uint32_t n_cols, const float* __res
 }
 
 template <bool kArgmin>
-void launch_exact_gemm(const float* b, uint32_t n_cols, const float* a, uint32_t n_rows, uint32_t kdim, float alpha,
+void launch_exact_gemm(const float* b, uint32_t n_cols, const float* a, uint32_t n_rows, uint32_t a_stride, uint32_t kdim, float alpha,
                        bool half_scores, float* out, unsigned long long* best, cudaStream_t stream,
                        const uint32_t* row_list = nullptr, const uint32_t* n_listed = nullptr)
 {
@@ -232,7 +235,7 @@ void launch_exact_gemm(const float* b, uint32_t n_cols, const float* a, uint32_t
     const size_t smem = (size_t(32) * (kdim | 1u) + size_t(n_rows) * kdim) * 4;
     if (n_rows <= kFewRows && smem <= 200 * 1024) {
       ensure_dynamic_smem(reinterpret_cast<const void*>(few_rows_kernel), smem);
-      few_rows_kernel<<<ceildiv(n_cols, 32u), 128, smem, stream>>>(b, n_cols, a, n_rows, kdim, alpha, half_scores, out);
+      few_rows_kernel<<<ceildiv(n_cols, 32u), 128, smem, stream>>>(b, n_cols, a, n_rows, a_stride, kdim, alpha, half_scores, out);
       CUDA_TRY(cudaGetLastError());
       return;
     }
@@ -242,51 +245,17 @@ void launch_exact_gemm(const float* b, uint32_t n_cols, const float* a, uint32_t
   for (uint32_t r0 = 0; r0 < n_rows; r0 += most) {
     const uint32_t nr = std::min(most, n_rows - r0);
     const dim3 grid(ceildiv(n_cols, kTile), ceildiv(nr, kTile));
-    const float* ar = a + size_t(r0) * kdim;
+    const float* ar = a + size_t(r0) * a_stride;
     float* o        = out ? out + size_t(r0) * n_cols : nullptr;
     unsigned long long* bs = best ? best + r0 : nullptr;
-    const bool vec = kdim % 4 == 0 && ((reinterpret_cast<uintptr_t>(b) | reinterpret_cast<uintptr_t>(ar)) & 15u) == 0;
+    const bool vec = kdim % 4 == 0 && a_stride % 4 == 0 && ((reinterpret_cast<uintptr_t>(b) | reinterpret_cast<uintptr_t>(ar)) & 15u) == 0;
     if (vec) {
-      exact_gemm_kernel<true, kArgmin><<<grid, 256, 0, stream>>>(b, n_cols, ar, nr, kdim, alpha, half_scores, o, bs, row_list, n_listed);
+      exact_gemm_kernel<true, kArgmin><<<grid, 256, 0, stream>>>(b, n_cols, ar, nr, a_stride, kdim, alpha, half_scores, o, bs, row_list, n_listed);
     } else {
-      exact_gemm_kernel<false, kArgmin><<<grid, 256, 0, stream>>>(b, n_cols, ar, nr, kdim, alpha, half_scores, o, bs, row_list, n_listed);
+      exact_gemm_kernel<false, kArgmin><<<grid, 256, 0, stream>>>(b, n_cols, ar, nr, a_stride, kdim, alpha, half_scores, o, bs, row_list, n_listed);
     }
     CUDA_TRY(cudaGetLastError());
   }
-}
-
-// The digit (0..255) at which the running count of `hist` reaches `rem`, and how many of that digit are wanted; one whole
-// warp calls it.
-__device__ __forceinline__ void find_digit(const uint32_t* hist, uint32_t rem, uint32_t& digit, uint32_t& left)
-{
-  const uint32_t lane = threadIdx.x & 31u;
-  uint32_t c[8], sum = 0;
-#pragma unroll
-  for (int i = 0; i < 8; i++) {
-    c[i] = hist[lane * 8u + i];
-    sum += c[i];
-  }
-  uint32_t inc = sum;
-#pragma unroll
-  for (int d = 1; d < 32; d <<= 1) {
-    const uint32_t o = __shfl_up_sync(kFullMask, inc, d);
-    if (lane >= uint32_t(d)) { inc += o; }
-  }
-  const unsigned reach = __ballot_sync(kFullMask, inc >= rem);
-  digit = 255u;
-  left  = rem;
-  if (reach == 0u) { return; }
-  const int src = __ffs(reach) - 1;
-  uint32_t d = lane * 8u, r = rem - (inc - sum);
-#pragma unroll
-  for (int i = 0; i < 7; i++) {
-    if (d == lane * 8u + i && c[i] < r) {
-      r -= c[i];
-      d++;
-    }
-  }
-  digit = __shfl_sync(kFullMask, d, src);
-  left  = __shfl_sync(kFullMask, r, src);
 }
 
 // Sorts the first n2 (a power of two) keys ascending; the whole block calls it after a barrier.
@@ -536,7 +505,7 @@ void select_clusters(raft::resources& res, const float* centers, uint32_t n_list
   float* scores = static_cast<float*>(workspace);
   for (uint32_t q0 = 0; q0 < n_queries; q0 += chunk) {
     const uint32_t nq = std::min(chunk, n_queries - q0);
-    launch_exact_gemm<false>(centers, n_lists, fq + size_t(q0) * dim_ext, nq, dim_ext, alpha, half_scores, scores, nullptr,
+    launch_exact_gemm<false>(centers, n_lists, fq + size_t(q0) * dim_ext, nq, dim_ext, dim_ext, alpha, half_scores, scores, nullptr,
                              res.stream);
     launch_select(scores, nq, n_lists, n_lists, nullptr, 0, n_probes, probes + size_t(q0) * n_probes,
                   scores_out ? scores_out + size_t(q0) * n_probes : nullptr, res.stream);
@@ -554,11 +523,11 @@ void select_rows(raft::resources& res, const float* rows, uint32_t n_rows, uint3
   res.launches++;
 }
 
-void exact_rows_product(raft::resources& res, const float* b, uint32_t n_cols, const float* a, uint32_t n_rows, uint32_t k,
-                        float* out)
+void exact_rows_product(raft::resources& res, const float* b, uint32_t n_cols, const float* a, uint32_t n_rows, uint32_t a_stride,
+                        uint32_t k, float alpha, float* out)
 {
   if (n_rows == 0) { return; }
-  launch_exact_gemm<false>(b, n_cols, a, n_rows, k, 1.0f, false, out, nullptr, res.stream);
+  launch_exact_gemm<false>(b, n_cols, a, n_rows, a_stride, k, alpha, false, out, nullptr, res.stream);
   res.launches++;
 }
 
@@ -568,7 +537,7 @@ void assign_nearest(raft::resources& res, const float* centers, uint32_t n_lists
 {
   if (n_rows == 0) { return; }
   CUDA_TRY(cudaMemsetAsync(best, 0xFF, size_t(n_rows) * 8, res.stream));
-  launch_exact_gemm<true>(centers, n_lists, x_ext, n_rows, dim_ext, alpha, false, nullptr, best, res.stream);
+  launch_exact_gemm<true>(centers, n_lists, x_ext, n_rows, dim_ext, dim_ext, alpha, false, nullptr, best, res.stream);
   unpack_labels_kernel<<<ceildiv<uint32_t>(n_rows, 256), 256, 0, res.stream>>>(best, n_rows, nullptr, nullptr, labels);
   CUDA_TRY(cudaGetLastError());
   res.launches += 2;
@@ -580,7 +549,7 @@ void assign_nearest_listed(raft::resources& res, const float* centers, uint32_t 
 {
   CUVS_EXPECTS(n_rows <= 65535u * kTile, "too many rows");
   CUDA_TRY(cudaMemsetAsync(best, 0xFF, size_t(n_rows) * 8, res.stream));
-  launch_exact_gemm<true>(centers, n_lists, x_ext, n_rows, dim_ext, alpha, false, nullptr, best, res.stream, row_list, n_listed);
+  launch_exact_gemm<true>(centers, n_lists, x_ext, n_rows, dim_ext, dim_ext, alpha, false, nullptr, best, res.stream, row_list, n_listed);
   unpack_labels_kernel<<<ceildiv<uint32_t>(n_rows, 256), 256, 0, res.stream>>>(best, n_rows, row_list, n_listed, labels);
   CUDA_TRY(cudaGetLastError());
   res.launches += 2;

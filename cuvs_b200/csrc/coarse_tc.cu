@@ -102,8 +102,9 @@ __global__ void split_tf32_kernel(const float* __restrict__ in, size_t n, uint32
 // (see there); the finish kernels undo the scale (row_scale[q] = 2^e, exact).  Then the TF32 split.
 __global__ void split_queries_kernel(const float* __restrict__ fq, uint32_t n_queries, uint32_t dim_ext,
                                      uint32_t ext_col, float col_scale, float cmax, float* __restrict__ hi,
-                                     float* __restrict__ lo, float* __restrict__ row_scale)
+                                     float* __restrict__ lo, float* __restrict__ row_scale, uint32_t* __restrict__ words)
 {
+  if (blockIdx.x == 0 && threadIdx.x < 4) { words[threadIdx.x] = 0u; }  // error, queries redone, redo and would-fail counters
   const uint32_t q    = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const uint32_t lane = threadIdx.x & 31u;
   if (q >= n_queries) { return; }
@@ -592,19 +593,14 @@ coarse_finish_kernel(const uint32_t* __restrict__ cand_key, const uint32_t* __re
       if ((o & mask) == prefix) { atomicAdd(&s_hist[(o >> shift) & 0xFFu], 1u); }
     }
     __syncthreads();
-    if (tid == 0) {
-      uint32_t rem = s_remaining, d = 0;
-      for (; d < 256; d++) {
-        const uint32_t c = s_hist[d];
-        if (c >= rem) { break; }
-        rem -= c;
+    if (tid < 32) {
+      // (fewer valid candidates than C: the last digit and as many as there are, so that everything is taken)
+      uint32_t d, left;
+      const bool all = !find_digit(s_hist, s_remaining, d, left);
+      if (tid == 0) {
+        s_prefix    = prefix | (d << shift);
+        s_remaining = all ? 0xFFFFFFFFu : left;
       }
-      if (d == 256) {  // fewer valid candidates than C: take everything
-        d   = 255;
-        rem = 0xFFFFFFFFu;
-      }
-      s_prefix    = prefix | (d << shift);
-      s_remaining = rem;
     }
     __syncthreads();
   }
@@ -1009,8 +1005,9 @@ coarse_fallback_kernel(const uint32_t* __restrict__ redo_list, const uint32_t* _
                        uint32_t dim_ext, float alpha, uint32_t n_probes, uint32_t cap,
                        float* __restrict__ scratch /* [gridDim.x, n_lists] */,
                        uint32_t* __restrict__ probes, float* __restrict__ scores_out,
-                       uint32_t* __restrict__ n_fallback, const uint32_t* __restrict__ error_word)
+                       uint32_t* __restrict__ words, volatile uint32_t* __restrict__ host_words, uint32_t host_seq)
 {
+  const uint32_t* error_word = words;
   extern __shared__ uint64_t s_keys[];  // [cap], then the query
   float* s_q = reinterpret_cast<float*>(s_keys + cap);
   __shared__ uint32_t s_hist[256];
@@ -1020,7 +1017,18 @@ coarse_fallback_kernel(const uint32_t* __restrict__ redo_list, const uint32_t* _
   // after a time-out of the GEMM nothing it produced is trusted: all queries are redone here
   const bool redo_all   = *error_word != 0u;
   const uint32_t n_redo = redo_all ? n_queries : min(*redo_count, n_queries);
-  if (blockIdx.x == 0 && tid == 0) { *n_fallback = n_redo; }
+  if (blockIdx.x == 0 && tid == 0) {
+    words[1] = n_redo;
+    if (host_words != nullptr) {
+      // the batch's verdict straight into the handle's pinned words (a copy and an event cost the host 8 us per call)
+      host_words[0] = words[0];
+      host_words[1] = n_redo;
+      host_words[2] = words[2];
+      host_words[3] = words[3];
+      __threadfence_system();
+      host_words[4] = host_seq;
+    }
+  }
   for (uint32_t ri = blockIdx.x; ri < n_redo; ri += gridDim.x) {
     const uint32_t q = redo_all ? ri : redo_list[ri];
     for (uint32_t i = tid; i < dim_ext; i += 256) { s_q[i] = fq[size_t(q) * dim_ext + i]; }
@@ -1051,15 +1059,13 @@ coarse_fallback_kernel(const uint32_t* __restrict__ redo_list, const uint32_t* _
         if ((o & mask) == prefix) { atomicAdd(&s_hist[(o >> shift) & 0xFFu], 1u); }
       }
       __syncthreads();
-      if (tid == 0) {
-        uint32_t rem = s_remaining, d = 0;
-        for (; d < 256; d++) {
-          const uint32_t c = s_hist[d];
-          if (c >= rem) { break; }
-          rem -= c;
+      if (tid < 32) {
+        uint32_t d, left;
+        find_digit(s_hist, s_remaining, d, left);
+        if (tid == 0) {
+          s_prefix    = prefix | (d << shift);
+          s_remaining = left;
         }
-        s_prefix    = prefix | (d << shift);
-        s_remaining = rem;
       }
       __syncthreads();
     }
@@ -1289,8 +1295,7 @@ void select_clusters_tc(raft::resources& res, const float* centers, const float*
 
   if (ext_scale == 1.0f) { ext_col = dim_ext; }
   split_queries_kernel<<<ceildiv<uint32_t>(n_queries * 32u, 256u), 256, 0, stream>>>(
-    fq, n_queries, dim_ext, ext_col, ext_scale, cmax, fq_hi, fq_lo, row_scale);
-  CUDA_TRY(cudaMemsetAsync(words, 0, 16, stream));  // error, queries redone, redo counter, would-fail counter
+    fq, n_queries, dim_ext, ext_col, ext_scale, cmax, fq_hi, fq_lo, row_scale, words);
 
   const CUtensorMap m_a_hi = make_map(fq_hi, n_queries, dim_ext, kBM);
   const CUtensorMap m_a_lo = make_map(fq_lo, n_queries, dim_ext, kBM);
@@ -1385,22 +1390,22 @@ void select_clusters_tc(raft::resources& res, const float* centers, const float*
   ensure_dynamic_smem(reinterpret_cast<const void*>(coarse_fallback_scores_kernel), fs_smem);
   coarse_fallback_scores_kernel<<<ceildiv<uint32_t>(n_lists, 256u), 256, fs_smem, stream>>>(
     redo_list, words + 2, centers, fq, n_queries, n_lists, dim_ext, alpha, scratch, kFbSlots, words);
-  coarse_fallback_kernel<<<kFbSlots, 256, fb_smem, stream>>>(redo_list, words + 2, centers, fq, n_queries, n_lists,
-                                                       dim_ext, alpha, n_probes, cap_fb, scratch, probes,
-                                                       scores_out, words + 1, words);
-  CUDA_TRY(cudaGetLastError());
-  res.launches += 5;
+  // the error word and how many queries this batch redid exactly: written to pinned memory by the kernel, looked at
+  // before a later batch and at the handle's next synchronisation
+  uint32_t* host_words = nullptr;
   if (!res.tc_redo_pending) {
-    // the error word and how many queries this batch redid exactly: read back without waiting, looked
-    // at before a later batch and at the handle's next synchronisation
-    if (!res.tc_redo_event) { CUDA_TRY(cudaEventCreateWithFlags(&res.tc_redo_event, cudaEventDisableTiming)); }
-    CUDA_TRY(cudaMemcpyAsync(res.pinned + 8, words, 16, cudaMemcpyDeviceToHost, stream));
-    CUDA_TRY(cudaEventRecord(res.tc_redo_event, stream));
+    host_words           = res.pinned + 8;
     res.tc_redo_queries  = n_queries;
     res.tc_redo_n_probes = n_probes;
-    res.tc_redo_adapts  = !exact_operands && tc_products_ref() == 0;
-    res.tc_redo_pending = true;
+    res.tc_redo_adapts   = !exact_operands && tc_products_ref() == 0;
+    res.tc_redo_pending  = true;
+    res.tc_redo_seq++;
   }
+  coarse_fallback_kernel<<<kFbSlots, 256, fb_smem, stream>>>(redo_list, words + 2, centers, fq, n_queries, n_lists,
+                                                       dim_ext, alpha, n_probes, cap_fb, scratch, probes,
+                                                       scores_out, words, host_words, res.tc_redo_seq);
+  CUDA_TRY(cudaGetLastError());
+  res.launches += 5;
 }
 
 // Reads back the error word and the number of queries redone exactly by the last call that used

@@ -2,6 +2,7 @@
 
 #include <nvtx3/nvToolsExt.h>
 
+#include <atomic>
 #include <mutex>
 
 namespace cuvs_b200 {
@@ -60,6 +61,7 @@ resources::resources()
   smem_optin = static_cast<int>(prop.sharedMemPerBlockOptin);
   cc_major   = prop.major;
   CUDA_TRY(cudaMallocHost(&pinned, 64));
+  pinned[12] = 0;
 }
 
 resources::~resources()
@@ -67,14 +69,17 @@ resources::~resources()
   for (auto& ev : pending) {
     for (auto& e : ev.e) { cudaEventDestroy(e); }
   }
-  if (tc_redo_event) { cudaEventDestroy(tc_redo_event); }
   if (d_stats) { cudaFree(d_stats); }
-  if (pinned) { cudaFreeHost(pinned); }
+  if (pinned) {
+    if (tc_redo_pending) { cudaDeviceSynchronize(); }  // a kernel may still write its verdict there
+    cudaFreeHost(pinned);
+  }
 }
 
 void resources::adopt_tc_verdict()
 {
-  if (!tc_redo_pending || cudaEventQuery(tc_redo_event) != cudaSuccess) { return; }
+  if (!tc_redo_pending || *static_cast<volatile uint32_t*>(pinned + 12) != tc_redo_seq) { return; }
+  std::atomic_thread_fence(std::memory_order_acquire);
   tc_redo_pending = false;
   if (pinned[8] != 0u) {
     // the coarse GEMM of that batch gave up on a bounded wait; its probes were all recomputed exactly

@@ -99,7 +99,8 @@ template <> __device__ __forceinline__ int8_t map_to_int8<int8_t>(int8_t x) { re
 template <> __device__ __forceinline__ int8_t map_to_int8<uint8_t>(uint8_t x) { return static_cast<int8_t>(x >> 1); }
 
 // One block per query.  fq = mapping<float>(query) padded to dim_ext with -0.5 (L2) or 0 in column
-// `dim`; rot_q = R * fq[:dim], each output accumulated by one thread in ascending k with FMA.
+// `dim`; rot_q = R * fq[:dim], each output accumulated in ascending k with FMA: here where R is the identity, else as a
+// product (exact_rows_product; a thread per output read R with a stride of a row: 148 us for 5,003 queries of 100 x 192).
 // kInt8 (coarse_search_dtype = CUDA_R_8I, ivf_pq_search.cuh:171-256 and :996-1025): fq holds the
 // int8 image of the query as numbers, dim_ext = round_up(dim + 2, 16) with 1 - m in column `dim` and
 // -128 (L2) or 0 in the m - 1 columns after it; `rotation` is the int8 image of the rotation matrix
@@ -109,9 +110,10 @@ template <> __device__ __forceinline__ int8_t map_to_int8<uint8_t>(uint8_t x) { 
 template <typename T, int kMode>
 __global__ void prep_queries_kernel(const T* __restrict__ queries, uint32_t dim, uint32_t dim_ext,
                                     uint32_t rot_dim, int is_l2, int cosine, int identity,
-                                    const float* __restrict__ rotation, float* __restrict__ fq,
-                                    float* __restrict__ rot_q)
+                                    float* __restrict__ fq, float* __restrict__ rot_q, uint32_t* __restrict__ counters)
 {
+  // the first kernel of a batch clears the counters of the later ones
+  if (counters != nullptr && blockIdx.x == 0 && threadIdx.x < 4) { counters[threadIdx.x] = 0u; }
   constexpr bool kInt8 = kMode == 1;
   extern __shared__ float s_buf[];  // [dim] query, [rot_dim] rotated (cosine only)
   float* s_q         = s_buf;
@@ -135,17 +137,10 @@ __global__ void prep_queries_kernel(const T* __restrict__ queries, uint32_t dim,
     dst[i] = v;
   }
   __syncthreads();
+  if (!identity) { return; }  // rotated by exact_rows_product
   float* out = rot_q + size_t(q) * rot_dim;
   for (uint32_t r = threadIdx.x; r < rot_dim; r += blockDim.x) {
-    float acc;
-    if (identity) {
-      acc = s_q[r];
-    } else {
-      const float* row = rotation + size_t(r) * dim;
-      acc              = 0.0f;
-      for (uint32_t k = 0; k < dim; k++) { acc = __fmaf_rn(__ldg(row + k), s_q[k], acc); }
-      if constexpr (kInt8) { acc = __fmul_rn(acc, 1.0f / 16384.0f); }
-    }
+    const float acc = s_q[r];
     if (cosine) {
       s_r[r] = acc;
     } else {
@@ -165,6 +160,34 @@ __global__ void prep_queries_kernel(const T* __restrict__ queries, uint32_t dim,
     for (uint32_t r = threadIdx.x; r < rot_dim; r += blockDim.x) {
       out[r] = nrm > 0.0f ? __fdiv_rn(s_r[r], nrm) : s_r[r];
     }
+  }
+}
+
+// Cosine: rows of rot_q divided by their norm (a chain of fused multiply-adds in ascending order, one thread per row, out
+// of shared memory).  32 rows per block.
+__global__ void __launch_bounds__(256)
+normalize_rows_kernel(float* __restrict__ rot_q, uint32_t n_rows, uint32_t rot_dim)
+{
+  extern __shared__ float s_rows[];  // [32][rot_dim | 1]
+  __shared__ float s_norm[32];
+  const uint32_t r0 = blockIdx.x * 32u, nr = min(32u, n_rows - r0), ld = rot_dim | 1u;
+  float* rows = rot_q + size_t(r0) * rot_dim;
+  for (uint32_t i = threadIdx.x; i < nr * rot_dim; i += 256u) {
+    const uint32_t r = i / rot_dim;
+    s_rows[r * ld + (i - r * rot_dim)] = rows[i];
+  }
+  __syncthreads();
+  if (threadIdx.x < nr) {
+    const float* v = s_rows + threadIdx.x * ld;
+    float ss       = 0.0f;
+    for (uint32_t i = 0; i < rot_dim; i++) { ss = __fmaf_rn(v[i], v[i], ss); }
+    s_norm[threadIdx.x] = __fsqrt_rn(ss);
+  }
+  __syncthreads();
+  for (uint32_t i = threadIdx.x; i < nr * rot_dim; i += 256u) {
+    const uint32_t r = i / rot_dim;
+    const float nrm  = s_norm[r];
+    if (nrm > 0.0f) { rows[i] = __fdiv_rn(s_rows[r * ld + (i - r * rot_dim)], nrm); }
   }
 }
 
@@ -400,10 +423,47 @@ __global__ void final_merge_kernel(const uint64_t* __restrict__ keys,
   queue.init(int(k));
   const uint64_t* src = keys + size_t(q) * n_probes * k;
   const uint32_t n    = n_probes * k;
-  for (uint32_t t0 = 0; t0 < n; t0 += 32) {
-    const uint32_t t = t0 + lane;
-    uint64_t key     = t < n ? src[t] : kEmptyKey;
-    queue.offer(key, t < n);
+  bool done           = false;
+  if constexpr (KPL == 1) {
+    // k <= 24: at least k keys have scores at or below the k-th smallest of the 32 lanes' smallest scores, and few others
+    // do: they are gathered and sorted once (a batch merge for every 32 keys took 7 us for 32 probes of one query)
+    __shared__ uint64_t s_found[4][64];
+    uint64_t* found = s_found[threadIdx.x >> 5];
+    if (k <= 24u) {
+      uint32_t mn = kEmptyScore;
+#pragma unroll 4
+      for (uint32_t t = lane; t < n; t += 32) { mn = min(mn, uint32_t(__ldg(src + t) >> 32)); }
+      uint32_t T = 0;
+#pragma unroll
+      for (int bit = 31; bit >= 8; bit--) {
+        const uint32_t c = T | (1u << bit);
+        if (uint32_t(__popc(__ballot_sync(kFullMask, mn < c))) < k) { T = c; }
+      }
+      T |= 0xFFu;
+      uint32_t count = 0;
+      for (uint32_t t0 = 0; t0 < n; t0 += 32) {
+        const uint64_t key = t0 + lane < n ? __ldg(src + t0 + lane) : kEmptyKey;
+        const bool in      = key != kEmptyKey && uint32_t(key >> 32) <= T;
+        const unsigned m   = __ballot_sync(kFullMask, in);
+        const uint32_t at  = count + __popc(m & ((1u << lane) - 1u));
+        if (in && at < 64u) { found[at] = key; }
+        count += __popc(m);
+      }
+      if (count <= 64u) {
+        __syncwarp();
+        uint64_t a0 = lane < count ? found[lane] : kEmptyKey, a1 = lane + 32u < count ? found[lane + 32u] : kEmptyKey;
+        warp_sort64<uint64_t, false>(a0, a1);
+        queue.a[0] = a0;
+        done       = true;
+      }
+    }
+  }
+  if (!done) {
+    for (uint32_t t0 = 0; t0 < n; t0 += 32) {
+      const uint32_t t = t0 + lane;
+      uint64_t key     = t < n ? src[t] : kEmptyKey;
+      queue.offer(key, t < n);
+    }
   }
   const uint32_t* ci = chunk_index + size_t(q) * n_probes;
   const uint32_t* pr = probes + size_t(q) * n_probes;
@@ -533,7 +593,8 @@ int coarse_mode() { return coarse_mode_ref(); }
 
 // `rotation_alt`: the int8 (mode 1) or half-rounded (mode 2) image of the rotation matrix.
 void launch_prep(raft::resources& res, const index<int64_t>& idx, const void* qptr, elem_t qtype,
-                 uint32_t nq, float* d_fq, float* d_rq, const float* rotation_alt = nullptr, int mode = 0)
+                 uint32_t nq, float* d_fq, float* d_rq, const float* rotation_alt = nullptr, int mode = 0,
+                 uint32_t* counters = nullptr)
 {
   const DistanceType metric = idx.metric();
   const int is_l2  = metric == DistanceType::L2Expanded || metric == DistanceType::L2SqrtExpanded;
@@ -551,13 +612,13 @@ void launch_prep(raft::resources& res, const index<int64_t>& idx, const void* qp
     using T = std::remove_const_t<std::remove_pointer_t<decltype(q)>>;
     if (mode == 1) {
       prep_queries_kernel<T, 1><<<nq, threads, smem, stream>>>(q, idx.dim(), dim_ext, idx.rot_dim(), is_l2,
-                                                               cosine, ident, rot, d_fq, d_rq);
+                                                               cosine, ident, d_fq, d_rq, counters);
     } else if (mode == 2) {
       prep_queries_kernel<T, 2><<<nq, threads, smem, stream>>>(q, idx.dim(), dim_ext, idx.rot_dim(), is_l2,
-                                                               cosine, ident, rot, d_fq, d_rq);
+                                                               cosine, ident, d_fq, d_rq, counters);
     } else {
       prep_queries_kernel<T, 0><<<nq, threads, smem, stream>>>(q, idx.dim(), dim_ext, idx.rot_dim(), is_l2,
-                                                               cosine, ident, rot, d_fq, d_rq);
+                                                               cosine, ident, d_fq, d_rq, counters);
     }
   };
   switch (qtype) {
@@ -568,6 +629,17 @@ void launch_prep(raft::resources& res, const index<int64_t>& idx, const void* qp
   }
   CUDA_TRY(cudaGetLastError());
   res.launches++;
+  if (!ident) {
+    // (int8 images: the sums are integers below 2^24, scaled by 1 / 128^2)
+    exact_rows_product(res, rot, idx.rot_dim(), d_fq, nq, dim_ext, idx.dim(), mode == 1 ? 1.0f / 16384.0f : 1.0f, d_rq);
+    if (cosine) {
+      const size_t smem_n = size_t(32) * (idx.rot_dim() | 1u) * 4;
+      ensure_dynamic_smem(reinterpret_cast<const void*>(normalize_rows_kernel), smem_n);
+      normalize_rows_kernel<<<ceildiv(nq, 32u), 256, smem_n, stream>>>(d_rq, nq, idx.rot_dim());
+      CUDA_TRY(cudaGetLastError());
+      res.launches++;
+    }
+  }
 }
 
 }  // namespace
@@ -872,7 +944,7 @@ void search_any(raft::resources& res, const search_params& params, const index<i
 
     // 1. cast / pad / rotate
     launch_prep(res, idx, qptr, qtype, nq, d_fq, d_rq, coarse_i8 ? op8.rotation : (coarse_h ? oph.rotation : nullptr),
-                coarse_i8 ? 1 : (coarse_h ? 2 : 0));
+                coarse_i8 ? 1 : (coarse_h ? 2 : 0), d_counter);
 
     if (stats) { res.stats_mark(ev, 1); }
     // 2. coarse selection: probes sorted by (score, list id)
@@ -917,7 +989,6 @@ void search_any(raft::resources& res, const search_params& params, const index<i
       auto* d_qscale  = reinterpret_cast<float*>(ws + o_qscale);
       auto* d_operand = reinterpret_cast<__half*>(ws + o_operand);
       // 3. tiles, and the query operand of every pair, ordered by list; d_counter: pairs, tiles, error word
-      CUDA_TRY(cudaMemsetAsync(d_counter, 0, 16, stream));
       if (f_small) {
         launch_tiles_small(d_probes, idx.list_sizes(), idx.row_offsets(), n_lists, nq, n_probes, d_chunk, d_groups, d_tiles,
                            d_counter, stream);
@@ -1040,7 +1111,6 @@ void search_any(raft::resources& res, const search_params& params, const index<i
     const bool sorted_pairs = stats || n_pairs > 4096;
     if (!sorted_pairs) {
       // small batch: one launch, pairs in arrival order (a sort by list has nothing to gain here)
-      CUDA_TRY(cudaMemsetAsync(d_counter, 0, 8, stream));
       small_batch_pairs_kernel<<<ceildiv<uint32_t>(nq * 32, 128), 128, 0, stream>>>(
         d_probes, idx.list_sizes(), n_lists, idx.row_offsets(), nq, n_probes, d_chunk, d_order, d_counter + 1, d_kth,
         store_all ? nullptr : d_keys, k);

@@ -98,9 +98,10 @@ void assign_nearest(raft::resources& res, const float* centers, uint32_t n_lists
 void assign_nearest_listed(raft::resources& res, const float* centers, uint32_t n_lists, uint32_t dim_ext, float alpha,
                            const float* x_ext, uint32_t n_rows, const uint32_t* row_list, const uint32_t* n_listed,
                            uint32_t* labels, unsigned long long* best);
-// out[i, j] = sum over ascending k of b[j, k] * a[i, k], one fp32 fused multiply-add chain each.
-void exact_rows_product(raft::resources& res, const float* b, uint32_t n_cols, const float* a, uint32_t n_rows, uint32_t k,
-                        float* out);
+// out[i, j] = alpha * sum over ascending k of b[j, k] * a[i, k], one fp32 fused multiply-add chain each; rows of `a` are
+// a_stride apart.
+void exact_rows_product(raft::resources& res, const float* b, uint32_t n_cols, const float* a, uint32_t n_rows, uint32_t a_stride,
+                        uint32_t k, float alpha, float* out);
 
 // The same labels on the tensor cores (label_tc.cu).  `model`: label_model_bytes of device memory that
 // prepare_label_model fills from the centres; `workspace`: label_workspace_bytes.  Nothing synchronises.

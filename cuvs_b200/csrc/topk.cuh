@@ -209,4 +209,39 @@ __device__ __forceinline__ void warp_sort64(T& a0, T& a1)
   }
 }
 
+// The digit (0..255) at which the running count of `hist` reaches `rem`, and how many of that digit are wanted; one whole
+// warp calls it.  Fewer than `rem` in all: false, digit 255 and `left` = rem.
+__device__ __forceinline__ bool find_digit(const uint32_t* hist, uint32_t rem, uint32_t& digit, uint32_t& left)
+{
+  const uint32_t lane = threadIdx.x & 31u;
+  uint32_t c[8], sum = 0;
+#pragma unroll
+  for (int i = 0; i < 8; i++) {
+    c[i] = hist[lane * 8u + i];
+    sum += c[i];
+  }
+  uint32_t inc = sum;
+#pragma unroll
+  for (int d = 1; d < 32; d <<= 1) {
+    const uint32_t o = __shfl_up_sync(kFullMask, inc, d);
+    if (lane >= uint32_t(d)) { inc += o; }
+  }
+  const unsigned reach = __ballot_sync(kFullMask, inc >= rem);
+  digit = 255u;
+  left  = rem;
+  if (reach == 0u) { return false; }
+  const int src = __ffs(reach) - 1;
+  uint32_t d = lane * 8u, r = rem - (inc - sum);
+#pragma unroll
+  for (int i = 0; i < 7; i++) {
+    if (d == lane * 8u + i && c[i] < r) {
+      r -= c[i];
+      d++;
+    }
+  }
+  digit = __shfl_sync(kFullMask, d, src);
+  left  = __shfl_sync(kFullMask, r, src);
+  return true;
+}
+
 }  // namespace cuvs_b200

@@ -158,7 +158,7 @@ struct resources {
   // Tensor-core coarse stage: products of the TF32 split per K step used by this handle (start at
   // two; raised when a finished batch had to redo more than 1/256 of its queries exactly, lowered when
   // all but 1/1024 of a batch would have passed the guard with one product less); the counters of the
-  // last batch arrive in pinned[8..11] once tc_redo_event has completed.
+  // last batch are in pinned[8..11] once pinned[12] holds tc_redo_seq.
   // List-sharded multi-GPU search: when set, the fine search scans the pairs of every query's nearest
   // probe first, calls this with (stream, per-query bounds on the k-th best ordered score, n_queries)
   // -- the caller enqueues a min-reduction of the bounds over the ranks -- and then scans the rest.
@@ -171,7 +171,7 @@ struct resources {
   };
   std::map<uint32_t, tc_level> tc_levels;
   uint32_t tc_redo_n_probes  = 0;  // n_probes of the batch whose counters are in flight
-  cudaEvent_t tc_redo_event  = nullptr;
+  uint32_t tc_redo_seq       = 0;
   bool tc_redo_pending       = false;
   uint32_t tc_redo_queries   = 0;
   bool tc_redo_adapts        = false;
