@@ -863,8 +863,10 @@ void search_any(raft::resources& res, const search_params& params, const index<i
   const uint32_t max_groups = uint32_t(ceildiv<uint64_t>(uint64_t(idx.accum_sorted_sizes()[n_probes]) + 31ull * n_probes, 32));
   // (below some 4,000 pairs, and for k > 128, the look-up-table scan is as fast or faster: 162 against 178 us for 100
   // queries of 20 probes, 632 against 754 us for 500 queries with k = 1000)
+  // (a list-sharded search exchanges bounds in the middle of the look-up-table scan: a collective, so that all its ranks
+  // take that path)
   const int home = scan_codebook_home();
-  if (home == 4 || (home == 0 && uint64_t(batch) * n_probes > 4096 && k <= 128)) {
+  if (!res.scan_phase_hook && (home == 4 || (home == 0 && uint64_t(batch) * n_probes > 4096 && k <= 128))) {
     // bounds of one internal batch: within 2 GiB
     batch = uint32_t(std::max<uint64_t>(1, std::min<uint64_t>(batch, (1ull << 31) / (uint64_t(max_groups) * 16))));
     fplan = plan_filter(res, idx, lut_kind, out_half, is_ip, k, n_probes, batch);
