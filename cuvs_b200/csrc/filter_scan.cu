@@ -534,7 +534,7 @@ __global__ void count_pairs_kernel(const uint32_t* __restrict__ probes, const ui
 // lists' pairs still fit a tile).  A list with more pairs has tiles of its own, its queries dealt evenly over
 // tiles of at most 128.  The block's pairs are ordered accordingly: first the sharing lists'.
 constexpr uint32_t kPackPairs   = kTileQ / 8;
-// (64 lists per block; 16 where 64 would leave SMs without one: 111 us against 40 us for 4,000 lists of 1,000 rows)
+// (64 lists per block; 16 where 64 would leave SMs without one: 111 us against 50 us for 4,000 lists of 1,000 rows)
 template <uint32_t kListsPerBlock>
 __global__ void __launch_bounds__(256)
 make_tiles_kernel(uint32_t* __restrict__ list_count, const uint32_t* __restrict__ list_sizes,
