@@ -9,6 +9,7 @@
 // This file holds the exact SIMT path: a register-tiled fp32 product (each output accumulated by
 // one thread in ascending k, so it equals the defining chain bit for bit) and a per-query radix
 // select.  It is the general path (any n_probes up to 4096, any shape).
+#include "common.hpp"
 #include "search_internal.hpp"
 #include "topk.cuh"
 
@@ -51,6 +52,7 @@ exact_gemm_kernel(const float* __restrict__ b, uint32_t n_cols, const float* __r
                   uint32_t kdim, float alpha, int half_scores, float* __restrict__ out, unsigned long long* __restrict__ best,
                   const uint32_t* __restrict__ row_list, const uint32_t* __restrict__ n_listed)
 {
+  chain_begin();
   __shared__ __align__(16) float s_a[2][kTileK][kTile + 4];
   __shared__ __align__(16) float s_b[2][kTileK][kTile + 4];
   const uint32_t j0 = blockIdx.x * kTile, i0 = blockIdx.y * kTile;
@@ -185,6 +187,7 @@ __global__ void __launch_bounds__(128)
 few_rows_kernel(const float* __restrict__ b, uint32_t n_cols, const float* __restrict__ a, uint32_t n_rows, uint32_t a_stride,
                 uint32_t kdim, float alpha, int half_scores, float* __restrict__ out)
 {
+  chain_begin();
   extern __shared__ float s_few[];  // [32][kdim | 1], then [n_rows][kdim]
   constexpr uint32_t kPer = kFewRows / 4;
   const uint32_t j0 = blockIdx.x * 32u, tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
@@ -235,7 +238,7 @@ void launch_exact_gemm(const float* b, uint32_t n_cols, const float* a, uint32_t
     const size_t smem = (size_t(32) * (kdim | 1u) + size_t(n_rows) * kdim) * 4;
     if (n_rows <= kFewRows && smem <= 200 * 1024) {
       ensure_dynamic_smem(reinterpret_cast<const void*>(few_rows_kernel), smem);
-      few_rows_kernel<<<ceildiv(n_cols, 32u), 128, smem, stream>>>(b, n_cols, a, n_rows, a_stride, kdim, alpha, half_scores, out);
+      launch_chained(few_rows_kernel, ceildiv(n_cols, 32u), 128, smem, stream, b, n_cols, a, n_rows, a_stride, kdim, alpha, half_scores, out);
       CUDA_TRY(cudaGetLastError());
       return;
     }
@@ -250,9 +253,9 @@ void launch_exact_gemm(const float* b, uint32_t n_cols, const float* a, uint32_t
     unsigned long long* bs = best ? best + r0 : nullptr;
     const bool vec = kdim % 4 == 0 && a_stride % 4 == 0 && ((reinterpret_cast<uintptr_t>(b) | reinterpret_cast<uintptr_t>(ar)) & 15u) == 0;
     if (vec) {
-      exact_gemm_kernel<true, kArgmin><<<grid, 256, 0, stream>>>(b, n_cols, ar, nr, a_stride, kdim, alpha, half_scores, o, bs, row_list, n_listed);
+      launch_chained(exact_gemm_kernel<true, kArgmin>, grid, 256, 0, stream, b, n_cols, ar, nr, a_stride, kdim, alpha, half_scores, o, bs, row_list, n_listed);
     } else {
-      exact_gemm_kernel<false, kArgmin><<<grid, 256, 0, stream>>>(b, n_cols, ar, nr, a_stride, kdim, alpha, half_scores, o, bs, row_list, n_listed);
+      launch_chained(exact_gemm_kernel<false, kArgmin>, grid, 256, 0, stream, b, n_cols, ar, nr, a_stride, kdim, alpha, half_scores, o, bs, row_list, n_listed);
     }
     CUDA_TRY(cudaGetLastError());
   }
@@ -296,6 +299,7 @@ select_kernel(const float* __restrict__ scores, uint32_t row_stride, uint32_t ro
               uint32_t ends_stride, uint32_t want, uint32_t cap /* keys of shared memory */, uint32_t* __restrict__ out_idx,
               float* __restrict__ out_scores)
 {
+  chain_begin();
   extern __shared__ uint64_t s_keys[];  // [cap]
   __shared__ uint32_t s_hist[256];
   __shared__ uint32_t s_prefix, s_remaining, s_count, s_eq_taken;
@@ -448,7 +452,7 @@ void launch_select(const float* scores, uint32_t n_rows, uint32_t row_stride, ui
   auto go = [&](auto kernel, int threads) {
     const size_t smem = size_t(cap) * 8;
     if (smem > 48 * 1024) { ensure_dynamic_smem(reinterpret_cast<const void*>(kernel), smem); }
-    kernel<<<n_rows, threads, smem, stream>>>(scores, row_stride, row_len, row_ends, ends_stride, want, cap, out_idx,
+    launch_chained(kernel, n_rows, threads, smem, stream, scores, row_stride, row_len, row_ends, ends_stride, want, cap, out_idx,
                                               out_scores);
     CUDA_TRY(cudaGetLastError());
   };

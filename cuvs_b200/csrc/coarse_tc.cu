@@ -33,6 +33,7 @@
 //      bounding |tensor-core - exact| for the number of products in use.  A query whose guard
 //      fails is queued.
 //   4. coarse_fallback_kernel: queued queries (rare) are redone exactly over all lists.
+#include "common.hpp"
 #include "search_internal.hpp"
 #include "tc_ptx.cuh"
 #include "topk.cuh"
@@ -104,6 +105,7 @@ __global__ void split_queries_kernel(const float* __restrict__ fq, uint32_t n_qu
                                      uint32_t ext_col, float col_scale, float cmax, float* __restrict__ hi,
                                      float* __restrict__ lo, float* __restrict__ row_scale, uint32_t* __restrict__ words)
 {
+  chain_begin();
   if (blockIdx.x == 0 && threadIdx.x < 4) { words[threadIdx.x] = 0u; }  // error, queries redone, redo and would-fail counters
   const uint32_t q    = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const uint32_t lane = threadIdx.x & 31u;
@@ -187,6 +189,7 @@ coarse_tc_kernel(const __grid_constant__ CUtensorMap map_a_hi, const __grid_cons
                  const __grid_constant__ CUtensorMap map_b_hi, const __grid_constant__ CUtensorMap map_b_lo,
                  const tc_params p)
 {
+  chain_begin();
   static_assert(!kARes || kProducts <= 2, "the resident-query variant stages one list operand");
   // Only the operands the chosen number of products reads are staged, and the 192 KB of stage memory
   // hold as many stages of that size as fit: 4 x 48 KB (three products), 6 x 32 KB (two), 8 x 24 KB
@@ -527,6 +530,7 @@ coarse_finish_kernel(const uint32_t* __restrict__ cand_key, const uint32_t* __re
                      const uint32_t* __restrict__ error_word, uint32_t ext_col, float ext_scale,
                      const float* __restrict__ row_scale, float down_thr, int by_maxima)
 {
+  chain_begin();
   // the GEMM gave up on a wait: its candidates are incomplete, every query is redone exactly
   if (*error_word != 0u) { return; }
   extern __shared__ uint64_t s_keys[];                 // [cap] keys; the query; the values to select among
@@ -758,6 +762,7 @@ coarse_finish_small_kernel(const uint32_t* __restrict__ cand_key, const uint32_t
                            uint32_t rows_per_round, const uint32_t* __restrict__ error_word, uint32_t ext_col,
                            float ext_scale, const float* __restrict__ row_scale, float down_thr)
 {
+  chain_begin();
   // the GEMM gave up on a wait: its candidates are incomplete, every query is redone exactly
   if (*error_word != 0u) { return; }
   // dynamic: query [dim_ext] | rows to rescore [rows_per_round][dim_ext + 1]
@@ -952,6 +957,7 @@ coarse_fallback_scores_kernel(const uint32_t* __restrict__ redo_list, const uint
                               float* __restrict__ scratch, uint32_t n_slots,
                               const uint32_t* __restrict__ error_word)
 {
+  chain_begin();
   extern __shared__ float s_f[];
   float* s_tile = s_f;             // [256 lists][32 columns + 1]
   float* s_qs   = s_f + 256 * 33;  // [kFbGroup][dim_ext]
@@ -1007,6 +1013,7 @@ coarse_fallback_kernel(const uint32_t* __restrict__ redo_list, const uint32_t* _
                        uint32_t* __restrict__ probes, float* __restrict__ scores_out,
                        uint32_t* __restrict__ words, volatile uint32_t* __restrict__ host_words, uint32_t host_seq)
 {
+  chain_begin();
   const uint32_t* error_word = words;
   extern __shared__ uint64_t s_keys[];  // [cap], then the query
   float* s_q = reinterpret_cast<float*>(s_keys + cap);
@@ -1294,8 +1301,7 @@ void select_clusters_tc(raft::resources& res, const float* centers, const float*
   cudaStream_t stream = res.stream;
 
   if (ext_scale == 1.0f) { ext_col = dim_ext; }
-  split_queries_kernel<<<ceildiv<uint32_t>(n_queries * 32u, 256u), 256, 0, stream>>>(
-    fq, n_queries, dim_ext, ext_col, ext_scale, cmax, fq_hi, fq_lo, row_scale, words);
+  launch_chained(split_queries_kernel, ceildiv<uint32_t>(n_queries * 32u, 256u), 256, 0, stream, fq, n_queries, dim_ext, ext_col, ext_scale, cmax, fq_hi, fq_lo, row_scale, words);
 
   const CUtensorMap m_a_hi = make_map(fq_hi, n_queries, dim_ext, kBM);
   const CUtensorMap m_a_lo = make_map(fq_lo, n_queries, dim_ext, kBM);
@@ -1332,7 +1338,7 @@ void select_clusters_tc(raft::resources& res, const float* centers, const float*
   auto launch = [&](auto kernel) {
     // every instantiation needs its shared-memory limit raised once per device
     ensure_dynamic_smem(reinterpret_cast<const void*>(kernel), kSmemBytes);
-    kernel<<<grid, kThreads, kSmemBytes, stream>>>(m_a_hi, m_a_lo, m_b_hi, m_b_lo, p);
+    launch_chained(kernel, grid, kThreads, kSmemBytes, stream, m_a_hi, m_a_lo, m_b_hi, m_b_lo, p);
   };
   // query operand resident in shared memory when it leaves room for at least four list stages
   const uint32_t a_bytes = p.k_blocks * uint32_t(kBM * kBK * 4) * (products >= 2 ? 2u : 1u);
@@ -1368,17 +1374,15 @@ void select_clusters_tc(raft::resources& res, const float* centers, const float*
   const size_t fin_small_smem = (size_t(dim_ext) + size_t(fin_rows) * (dim_ext + 1)) * 4;
   if (n_tiles * 2 <= kFinMaxHalfTiles && C <= kFinMaxC && C * 4 <= n_tiles * 2 && fin_small_smem <= 48 * 1024) {
     if (kph == 16) {
-      coarse_finish_small_kernel<16><<<n_queries, 256, fin_small_smem, stream>>>(
-        cand_key, cand_bnd, n_cand, centers, fq, n_lists, dim_ext, alpha, n_probes, C, cmax, eps_rel, probes,
+      launch_chained(coarse_finish_small_kernel<16>, n_queries, 256, fin_small_smem, stream, cand_key, cand_bnd, n_cand, centers, fq, n_lists, dim_ext, alpha, n_probes, C, cmax, eps_rel, probes,
         scores_out, redo_list, words + 2, fin_rows, words, ext_col, ext_scale, row_scale, down_thr);
     } else {
-      coarse_finish_small_kernel<8><<<n_queries, 256, fin_small_smem, stream>>>(
-        cand_key, cand_bnd, n_cand, centers, fq, n_lists, dim_ext, alpha, n_probes, C, cmax, eps_rel, probes,
+      launch_chained(coarse_finish_small_kernel<8>, n_queries, 256, fin_small_smem, stream, cand_key, cand_bnd, n_cand, centers, fq, n_lists, dim_ext, alpha, n_probes, C, cmax, eps_rel, probes,
         scores_out, redo_list, words + 2, fin_rows, words, ext_col, ext_scale, row_scale, down_thr);
     }
   } else {
     if (fin_smem > 48 * 1024) { ensure_dynamic_smem(reinterpret_cast<const void*>(coarse_finish_kernel), fin_smem); }
-    coarse_finish_kernel<<<n_queries, 256, fin_smem, stream>>>(cand_key, cand_bnd, n_cand, kph, centers, fq,
+    launch_chained(coarse_finish_kernel, n_queries, 256, fin_smem, stream, cand_key, cand_bnd, n_cand, kph, centers, fq,
                                                                n_lists, dim_ext, alpha, n_probes, C, cap,
                                                                cmax, eps_rel, probes, scores_out, redo_list,
                                                                words + 2, words, ext_col, ext_scale, row_scale, down_thr, by_maxima ? 1 : 0);
@@ -1388,8 +1392,7 @@ void select_clusters_tc(raft::resources& res, const float* centers, const float*
   const size_t fb_smem = size_t(cap_fb) * 8 + size_t(dim_ext) * 4;
   const size_t fs_smem = (size_t(256) * 33 + size_t(kFbGroup) * dim_ext) * 4;
   ensure_dynamic_smem(reinterpret_cast<const void*>(coarse_fallback_scores_kernel), fs_smem);
-  coarse_fallback_scores_kernel<<<ceildiv<uint32_t>(n_lists, 256u), 256, fs_smem, stream>>>(
-    redo_list, words + 2, centers, fq, n_queries, n_lists, dim_ext, alpha, scratch, kFbSlots, words);
+  launch_chained(coarse_fallback_scores_kernel, ceildiv<uint32_t>(n_lists, 256u), 256, fs_smem, stream, redo_list, words + 2, centers, fq, n_queries, n_lists, dim_ext, alpha, scratch, kFbSlots, words);
   // the error word and how many queries this batch redid exactly: written to pinned memory by the kernel, looked at
   // before a later batch and at the handle's next synchronisation
   uint32_t* host_words = nullptr;
@@ -1401,7 +1404,7 @@ void select_clusters_tc(raft::resources& res, const float* centers, const float*
     res.tc_redo_pending  = true;
     res.tc_redo_seq++;
   }
-  coarse_fallback_kernel<<<kFbSlots, 256, fb_smem, stream>>>(redo_list, words + 2, centers, fq, n_queries, n_lists,
+  launch_chained(coarse_fallback_kernel, kFbSlots, 256, fb_smem, stream, redo_list, words + 2, centers, fq, n_queries, n_lists,
                                                        dim_ext, alpha, n_probes, cap_fb, scratch, probes,
                                                        scores_out, words, host_words, res.tc_redo_seq);
   CUDA_TRY(cudaGetLastError());

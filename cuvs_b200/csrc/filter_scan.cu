@@ -23,6 +23,7 @@
 //
 // What bounds it: for few queries per list the gathers of the decode (one 4-byte look-up per code for two
 // dimensions per subspace, 3.4 wavefronts each on random codes); for many, the epilogue and the operand feed.
+#include "common.hpp"
 #include "filter_scan.hpp"
 #include "search_internal.hpp"
 #include "tc_ptx.cuh"
@@ -123,6 +124,7 @@ __global__ void __launch_bounds__(kFilterThreads, 1)
 filter_kernel(const __grid_constant__ CUtensorMap map_16, const __grid_constant__ CUtensorMap map_64,
               const __grid_constant__ CUtensorMap map_128, const filter_params p)
 {
+  chain_begin();
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw_a  = smem_u32(smem_raw);
   const uint32_t base_a = (raw_a + 1023u) & ~1023u;
@@ -498,6 +500,7 @@ __global__ void count_pairs_kernel(const uint32_t* __restrict__ probes, const ui
                                    uint32_t* __restrict__ chunk_index, uint32_t* __restrict__ group_index,
                                    uint32_t* __restrict__ list_count)
 {
+  chain_begin();
   const uint32_t q    = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const uint32_t lane = threadIdx.x & 31;
   if (q >= n_queries) { return; }
@@ -541,6 +544,7 @@ make_tiles_kernel(uint32_t* __restrict__ list_count, const uint32_t* __restrict_
                   const uint64_t* __restrict__ row_off, uint32_t n_lists, filter_tile* __restrict__ tiles,
                   uint32_t* __restrict__ counters)
 {
+  chain_begin();
   // exclusive sums over the block's lists: pairs and groups of sharing lists, pairs and tiles of the others
   constexpr uint32_t kScan = kListsPerBlock < 32u ? 32u : kListsPerBlock;
   __shared__ uint32_t s_off[4][kScan + 1], s_count[kScan], s_size[kScan], s_arena[kScan], s_warp[4], s_base[2];
@@ -641,6 +645,7 @@ pair_operands_kernel(const operand_params p, const uint32_t* __restrict__ probes
                      uint32_t max_groups, uint32_t* __restrict__ cursor, __half* __restrict__ operand,
                      float4* __restrict__ pair_rec, float* __restrict__ pair_norm)
 {
+  chain_begin();
   const uint32_t i    = (blockIdx.x * 256u + threadIdx.x) >> 4;
   const uint32_t lane = threadIdx.x & 15u;
   const unsigned half_mask = 0xFFFFu << (threadIdx.x & 16u);
@@ -745,6 +750,7 @@ __global__ void small_tiles_kernel(const uint32_t* __restrict__ probes, const ui
                                    uint32_t* __restrict__ group_index, filter_tile* __restrict__ tiles,
                                    uint32_t* __restrict__ counters)
 {
+  chain_begin();
   const uint32_t q    = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const uint32_t lane = threadIdx.x & 31;
   if (q >= n_queries) { return; }
@@ -791,6 +797,7 @@ __global__ void small_tiles_kernel(const uint32_t* __restrict__ probes, const ui
 __global__ void query_scale_kernel(const float* __restrict__ rot_q, uint32_t n_queries, uint32_t rot_dim,
                                    float* __restrict__ q_scale)
 {
+  chain_begin();
   const uint32_t q    = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const uint32_t lane = threadIdx.x & 31;
   if (q >= n_queries) { return; }
@@ -889,8 +896,7 @@ void launch_count_pairs(const uint32_t* probes, const uint32_t* list_sizes, uint
                         uint32_t n_probes, uint32_t* chunk_index, uint32_t* group_index, uint32_t* list_count,
                         cudaStream_t stream)
 {
-  count_pairs_kernel<<<ceildiv<uint32_t>(n_queries * 32, 256), 256, 0, stream>>>(
-    probes, list_sizes, n_lists, n_queries, n_probes, chunk_index, group_index, list_count);
+  launch_chained(count_pairs_kernel, ceildiv<uint32_t>(n_queries * 32, 256), 256, 0, stream, probes, list_sizes, n_lists, n_queries, n_probes, chunk_index, group_index, list_count);
   CUDA_TRY(cudaGetLastError());
 }
 
@@ -898,9 +904,9 @@ void launch_tiles(const uint32_t* list_sizes, const uint64_t* row_off, uint32_t 
                   filter_tile* tiles, uint32_t* counters, cudaStream_t stream)
 {
   if (n_lists >= 32768) {
-    make_tiles_kernel<64><<<ceildiv(n_lists, 64u), 256, 0, stream>>>(list_count, list_sizes, row_off, n_lists, tiles, counters);
+    launch_chained(make_tiles_kernel<64>, ceildiv(n_lists, 64u), 256, 0, stream, list_count, list_sizes, row_off, n_lists, tiles, counters);
   } else {
-    make_tiles_kernel<16><<<ceildiv(n_lists, 16u), 256, 0, stream>>>(list_count, list_sizes, row_off, n_lists, tiles, counters);
+    launch_chained(make_tiles_kernel<16>, ceildiv(n_lists, 16u), 256, 0, stream, list_count, list_sizes, row_off, n_lists, tiles, counters);
   }
   CUDA_TRY(cudaGetLastError());
 }
@@ -909,8 +915,7 @@ void launch_tiles_small(const uint32_t* probes, const uint32_t* list_sizes, cons
                         uint32_t n_queries, uint32_t n_probes, uint32_t* chunk_index, uint32_t* group_index,
                         filter_tile* tiles, uint32_t* counters, cudaStream_t stream)
 {
-  small_tiles_kernel<<<ceildiv<uint32_t>(n_queries * 32, 128), 128, 0, stream>>>(
-    probes, list_sizes, row_off, n_lists, n_queries, n_probes, chunk_index, group_index, tiles, counters);
+  launch_chained(small_tiles_kernel, ceildiv<uint32_t>(n_queries * 32, 128), 128, 0, stream, probes, list_sizes, row_off, n_lists, n_queries, n_probes, chunk_index, group_index, tiles, counters);
   CUDA_TRY(cudaGetLastError());
 }
 
@@ -918,14 +923,14 @@ void launch_pair_operands(const operand_params& p, const uint32_t* probes, const
                           const uint32_t* group_index, uint32_t n_pairs, uint32_t n_probes, uint32_t max_groups,
                           uint32_t* cursor, __half* operand, float4* pair_rec, float* pair_norm, cudaStream_t stream)
 {
-  pair_operands_kernel<<<ceildiv(n_pairs, 16u), 256, 0, stream>>>(p, probes, list_sizes, n_lists, group_index, n_pairs, n_probes,
+  launch_chained(pair_operands_kernel, ceildiv(n_pairs, 16u), 256, 0, stream, p, probes, list_sizes, n_lists, group_index, n_pairs, n_probes,
                                                                  max_groups, cursor, operand, pair_rec, pair_norm);
   CUDA_TRY(cudaGetLastError());
 }
 
 void launch_query_scale(const float* rot_q, uint32_t n_queries, uint32_t rot_dim, float* q_scale, cudaStream_t stream)
 {
-  query_scale_kernel<<<ceildiv<uint32_t>(n_queries * 32, 256), 256, 0, stream>>>(rot_q, n_queries, rot_dim, q_scale);
+  launch_chained(query_scale_kernel, ceildiv<uint32_t>(n_queries * 32, 256), 256, 0, stream, rot_q, n_queries, rot_dim, q_scale);
   CUDA_TRY(cudaGetLastError());
 }
 
@@ -948,7 +953,7 @@ void launch_filter(const filter_params& p, const __half* operand, uint32_t n_pai
   const CUtensorMap m128 = make_map_2d(CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, operand, n_pairs, k, 128, kBlockK, CU_TENSOR_MAP_SWIZZLE_128B);
   auto go = [&](auto kernel) {
     ensure_dynamic_smem(reinterpret_cast<const void*>(kernel), smem);
-    kernel<<<grid, kFilterThreads, smem, stream>>>(m16, m64, m128, p);
+    launch_chained(kernel, grid, kFilterThreads, smem, stream, m16, m64, m128, p);
     CUDA_TRY(cudaGetLastError());
   };
   auto by_len = [&](auto bits, auto words) {

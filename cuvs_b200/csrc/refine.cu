@@ -10,6 +10,7 @@
 //   L2Expanded / L2Unexpanded : sum (q - x)^2        L2Sqrt*: its square root
 //   InnerProduct              : sum q * x (largest first)
 //   CosineExpanded            : 1 - q.x / (|q| |x|)
+#include "common.hpp"
 #include "ivf_pq.hpp"
 #include "topk.cuh"
 
@@ -88,6 +89,7 @@ refine_kernel(const T* __restrict__ dataset, int64_t n_rows, uint32_t dim,
               int mode, uint32_t log_lanes, uint32_t log_wpq, uint32_t q_floats,
               int64_t* __restrict__ indices, float* __restrict__ distances)
 {
+  chain_begin();
   constexpr uint32_t kWords = ROW == ROW_VEC16 ? 4u : 1u;          // 4-byte words per load step
   constexpr uint32_t kPerWord = 4u / uint32_t(sizeof(T));
   constexpr uint32_t kElems = kWords * kPerWord;
@@ -271,8 +273,7 @@ void launch_refine_rows(raft::resources& res, const T* dataset, int64_t n_rows, 
       CUVS_EXPECTS(smem <= size_t(res.smem_optin) - 1024, "refine: dim = %u is too large", dim);
       ensure_dynamic_smem(reinterpret_cast<const void*>(kernel), smem);
     }
-    kernel<<<ceildiv(n_queries, qpb), warps * 32, smem, res.stream>>>(
-      dataset, n_rows, dim, queries, n_queries, candidates, n_cand, k, mode, log_lanes, log_wpq, q_floats, indices,
+    launch_chained(kernel, ceildiv(n_queries, qpb), warps * 32, smem, res.stream, dataset, n_rows, dim, queries, n_queries, candidates, n_cand, k, mode, log_lanes, log_wpq, q_floats, indices,
       distances);
     CUDA_TRY(cudaGetLastError());
   };

@@ -20,6 +20,7 @@
 //
 // What bounds it: gathers from the fp32 codebook (one 8-byte look-up per code for two dimensions per subspace);
 // it sits in shared memory once per CTA and thread groups of 32 to 1024 take one query at a time.
+#include "common.hpp"
 #include "filter_scan.hpp"
 #include "scan.cuh"
 #include "search_internal.hpp"
@@ -274,6 +275,7 @@ __device__ __forceinline__ bool score_row(const rescore_params& p, const float* 
 template <int LutKind, bool OutHalf, bool IsIP, int kLen, int kBits, bool kSmem>
 __global__ void __launch_bounds__(1024, 1) rescore_kernel(const rescore_params p)
 {
+  chain_begin();
   extern __shared__ __align__(16) uint8_t smem[];
   const uint32_t gt = p.group_threads;
   const uint32_t g = threadIdx.x / gt, t = threadIdx.x % gt;
@@ -665,7 +667,7 @@ void launch_rescore(const rescore_params& p, int lut_kind, bool out_half, bool i
 {
   auto go = [&](auto kernel) {
     ensure_dynamic_smem(reinterpret_cast<const void*>(kernel), smem);
-    kernel<<<grid, int(p.groups * p.group_threads), smem, stream>>>(p);
+    launch_chained(kernel, grid, int(p.groups * p.group_threads), smem, stream, p);
     CUDA_TRY(cudaGetLastError());
   };
   // straight-line code for 8- and 4-bit codes of two or four components (whole 16-byte groups of components)

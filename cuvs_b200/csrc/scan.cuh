@@ -697,6 +697,7 @@ __device__ __forceinline__ void score_part(accum<LutKind, OutHalf, IsIP>& acc, c
 template <int PqBits, int LutKind, bool OutHalf, bool IsIP, int KPL, int PQD = 0, int GT = 0, int LEN = 0>
 __global__ void __launch_bounds__(1024, 1) scan_kernel(const scan_params p)
 {
+  chain_begin();
   using lut_t               = typename lut_elem<LutKind>::type;
   constexpr uint32_t kBook  = 1u << PqBits;
   constexpr int kPerPiece   = 128 / PqBits;
@@ -1153,6 +1154,7 @@ __global__ void __launch_bounds__(1024, 1) scan_kernel(const scan_params p)
 template <int PqBits, int LutKind, bool OutHalf, bool IsIP, int KPL>
 __global__ void __launch_bounds__(256) scan_glut_kernel(const scan_params p)
 {
+  chain_begin();
   using lut_t              = typename lut_elem<LutKind>::type;
   constexpr uint32_t kBook = 1u << PqBits;
   constexpr uint32_t kMask = kBook - 1u;

@@ -14,7 +14,7 @@ template <typename Kernel>
 void launch_kernel(Kernel kernel, const scan_params& p, int grid, size_t smem, cudaStream_t stream)
 {
   ensure_dynamic_smem(reinterpret_cast<const void*>(kernel), smem);
-  kernel<<<grid, 1024, smem, stream>>>(p);
+  launch_chained(kernel, grid, 1024, smem, stream, p);
   CUDA_TRY(cudaGetLastError());
 }
 
@@ -102,7 +102,7 @@ void launch_glut_kpl(const scan_params& p, int kpl, int grid, size_t smem, cudaS
 {
   auto go = [&](auto kernel) {
     ensure_dynamic_smem(reinterpret_cast<const void*>(kernel), smem);
-    kernel<<<grid, 256, smem, stream>>>(p);
+    launch_chained(kernel, grid, 256, smem, stream, p);
     CUDA_TRY(cudaGetLastError());
   };
   if (kpl == 0) {

@@ -10,6 +10,7 @@
 //   scan_kernel ............... compute_similarity (scan.cuh)
 //   final_merge_kernel ........ cross-probe select_k (:646-655) + postprocess_distances
 //                               (ivf_common.cuh:175-252) + postprocess_neighbors (:112-169), fused
+#include "common.hpp"
 #include "filter_scan.hpp"
 #include "ivf_pq.hpp"
 #include "scan.cuh"
@@ -112,6 +113,7 @@ __global__ void prep_queries_kernel(const T* __restrict__ queries, uint32_t dim,
                                     uint32_t rot_dim, int is_l2, int cosine, int identity,
                                     float* __restrict__ fq, float* __restrict__ rot_q, uint32_t* __restrict__ counters)
 {
+  chain_begin();
   // the first kernel of a batch clears the counters of the later ones
   if (counters != nullptr && blockIdx.x == 0 && threadIdx.x < 4) { counters[threadIdx.x] = 0u; }
   constexpr bool kInt8 = kMode == 1;
@@ -168,6 +170,7 @@ __global__ void prep_queries_kernel(const T* __restrict__ queries, uint32_t dim,
 __global__ void __launch_bounds__(256)
 normalize_rows_kernel(float* __restrict__ rot_q, uint32_t n_rows, uint32_t rot_dim)
 {
+  chain_begin();
   extern __shared__ float s_rows[];  // [32][rot_dim | 1]
   __shared__ float s_norm[32];
   const uint32_t r0 = blockIdx.x * 32u, nr = min(32u, n_rows - r0), ld = rot_dim | 1u;
@@ -201,6 +204,7 @@ __global__ void chunk_and_count_kernel(const uint32_t* __restrict__ probes,
                                        uint32_t n_queries, uint32_t n_probes,
                                        uint32_t* __restrict__ chunk_index, uint32_t* __restrict__ list_count)
 {
+  chain_begin();
   const uint32_t q    = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const uint32_t lane = threadIdx.x & 31;
   if (q >= n_queries) { return; }
@@ -234,6 +238,7 @@ __global__ void chunk_and_count_kernel(const uint32_t* __restrict__ probes,
 __global__ void __launch_bounds__(1024) exclusive_scan_kernel(uint32_t* __restrict__ data, uint32_t n,
                                                               uint32_t* __restrict__ work_words)
 {
+  chain_begin();
   __shared__ uint32_t s_warp[32];
   const uint32_t tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
   const uint32_t per = round_up<uint32_t>(ceildiv<uint32_t>(n, 1024u), 4u);
@@ -338,6 +343,7 @@ __global__ void scatter_pairs_kernel(const uint32_t* __restrict__ probes,
                                      uint4* __restrict__ work, uint64_t* __restrict__ out_keys, uint32_t k,
                                      uint32_t* __restrict__ query_kth, uint32_t n_queries)
 {
+  chain_begin();
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n_pairs) { return; }
   if (i < n_queries) { query_kth[i] = kEmptyScore; }  // no bound on any query's k-th best yet
@@ -368,6 +374,7 @@ __global__ void small_batch_pairs_kernel(const uint32_t* __restrict__ probes,
                                          uint32_t* __restrict__ query_kth, uint64_t* __restrict__ out_keys,
                                          uint32_t k)
 {
+  chain_begin();
   const uint32_t q    = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const uint32_t lane = threadIdx.x & 31;
   if (q >= n_queries) { return; }
@@ -416,6 +423,7 @@ __global__ void final_merge_kernel(const uint64_t* __restrict__ keys,
                                    uint32_t n_probes, uint32_t k, int metric, float scale,
                                    int64_t* __restrict__ neighbors, float* __restrict__ distances)
 {
+  chain_begin();
   const uint32_t q    = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const uint32_t lane = threadIdx.x & 31;
   if (q >= n_queries) { return; }
@@ -506,6 +514,7 @@ __global__ void translate_selected_kernel(const float* __restrict__ sel_scores,
                                           uint32_t n_probes, uint32_t k, int metric, float scale,
                                           int64_t* __restrict__ neighbors, float* __restrict__ distances)
 {
+  chain_begin();
   const uint64_t i = blockIdx.x * uint64_t(blockDim.x) + threadIdx.x;
   if (i >= uint64_t(n_queries) * k) { return; }
   const uint32_t q   = uint32_t(i / k);
@@ -611,13 +620,13 @@ void launch_prep(raft::resources& res, const index<int64_t>& idx, const void* qp
   auto launch = [&](auto* q) {
     using T = std::remove_const_t<std::remove_pointer_t<decltype(q)>>;
     if (mode == 1) {
-      prep_queries_kernel<T, 1><<<nq, threads, smem, stream>>>(q, idx.dim(), dim_ext, idx.rot_dim(), is_l2,
+      launch_chained(prep_queries_kernel<T, 1>, nq, threads, smem, stream, q, idx.dim(), dim_ext, idx.rot_dim(), is_l2,
                                                                cosine, ident, d_fq, d_rq, counters);
     } else if (mode == 2) {
-      prep_queries_kernel<T, 2><<<nq, threads, smem, stream>>>(q, idx.dim(), dim_ext, idx.rot_dim(), is_l2,
+      launch_chained(prep_queries_kernel<T, 2>, nq, threads, smem, stream, q, idx.dim(), dim_ext, idx.rot_dim(), is_l2,
                                                                cosine, ident, d_fq, d_rq, counters);
     } else {
-      prep_queries_kernel<T, 0><<<nq, threads, smem, stream>>>(q, idx.dim(), dim_ext, idx.rot_dim(), is_l2,
+      launch_chained(prep_queries_kernel<T, 0>, nq, threads, smem, stream, q, idx.dim(), dim_ext, idx.rot_dim(), is_l2,
                                                                cosine, ident, d_fq, d_rq, counters);
     }
   };
@@ -635,7 +644,7 @@ void launch_prep(raft::resources& res, const index<int64_t>& idx, const void* qp
     if (cosine) {
       const size_t smem_n = size_t(32) * (idx.rot_dim() | 1u) * 4;
       ensure_dynamic_smem(reinterpret_cast<const void*>(normalize_rows_kernel), smem_n);
-      normalize_rows_kernel<<<ceildiv(nq, 32u), 256, smem_n, stream>>>(d_rq, nq, idx.rot_dim());
+      launch_chained(normalize_rows_kernel, ceildiv(nq, 32u), 256, smem_n, stream, d_rq, nq, idx.rot_dim());
       CUDA_TRY(cudaGetLastError());
       res.launches++;
     }
@@ -1113,25 +1122,22 @@ void search_any(raft::resources& res, const search_params& params, const index<i
     const bool sorted_pairs = stats || n_pairs > 4096;
     if (!sorted_pairs) {
       // small batch: one launch, pairs in arrival order (a sort by list has nothing to gain here)
-      small_batch_pairs_kernel<<<ceildiv<uint32_t>(nq * 32, 128), 128, 0, stream>>>(
-        d_probes, idx.list_sizes(), n_lists, idx.row_offsets(), nq, n_probes, d_chunk, d_order, d_counter + 1, d_kth,
+      launch_chained(small_batch_pairs_kernel, ceildiv<uint32_t>(nq * 32, 128), 128, 0, stream, d_probes, idx.list_sizes(), n_lists, idx.row_offsets(), nq, n_probes, d_chunk, d_order, d_counter + 1, d_kth,
         store_all ? nullptr : d_keys, k);
       CUDA_TRY(cudaGetLastError());
       res.launches += 1;
     } else {
       // counting sort of the pairs by list
       CUDA_TRY(cudaMemsetAsync(d_count, 0, (size_t(n_lists) * 2 + 1) * 4, stream));
-      chunk_and_count_kernel<<<ceildiv<uint32_t>(nq * 32, 256), 256, 0, stream>>>(
-        d_probes, idx.list_sizes(), n_lists, nq, n_probes, d_chunk, d_count);
+      launch_chained(chunk_and_count_kernel, ceildiv<uint32_t>(nq * 32, 256), 256, 0, stream, d_probes, idx.list_sizes(), n_lists, nq, n_probes, d_chunk, d_count);
       if (stats) {
         scan_stats_kernel<<<ceildiv<uint32_t>(n_lists, 256), 256, 0, stream>>>(d_count, idx.list_sizes(),
                                                                                 n_lists, 2, res.d_stats);
         res.stat_pairs += n_pairs;
       }
       // d_counter[0] = 0 (work counter), d_counter[1] = d_count[2 * n_lists] = number of work items
-      exclusive_scan_kernel<<<1, 1024, 0, stream>>>(d_count, n_lists * 2, d_counter);
-      scatter_pairs_kernel<<<ceildiv<uint32_t>(n_pairs, 256), 256, 0, stream>>>(
-        d_probes, d_chunk, idx.list_sizes(), n_lists, idx.row_offsets(), n_pairs, n_probes, d_count, d_order,
+      launch_chained(exclusive_scan_kernel, 1, 1024, 0, stream, d_count, n_lists * 2, d_counter);
+      launch_chained(scatter_pairs_kernel, ceildiv<uint32_t>(n_pairs, 256), 256, 0, stream, d_probes, d_chunk, idx.list_sizes(), n_lists, idx.row_offsets(), n_pairs, n_probes, d_count, d_order,
         store_all ? nullptr : d_keys, k, d_kth, nq);
       CUDA_TRY(cudaGetLastError());
       res.launches += 3;
@@ -1210,8 +1216,7 @@ void search_any(raft::resources& res, const search_params& params, const index<i
       auto* sel_idx    = reinterpret_cast<uint32_t*>(d_keys) + size_t(nq) * k;
       // (a row of scores ends where the query's last probe does; the scan writes every one of them)
       select_rows(res, d_all, nq, max_samples, k, sel_idx, sel_scores, d_chunk, n_probes);
-      translate_selected_kernel<<<unsigned(ceildiv<uint64_t>(uint64_t(nq) * k, 256)), 256, 0, stream>>>(
-        sel_scores, sel_idx, d_probes, d_chunk, idx.row_offsets(), idx.ids(), nq, n_probes, k,
+      launch_chained(translate_selected_kernel, unsigned(ceildiv<uint64_t>(uint64_t(nq) * k, 256)), 256, 0, stream, sel_scores, sel_idx, d_probes, d_chunk, idx.row_offsets(), idx.ids(), nq, n_probes, k,
         int(metric), scale, neighbors + size_t(q0) * k, distances + size_t(q0) * k);
       CUDA_TRY(cudaGetLastError());
       res.launches++;
@@ -1221,17 +1226,17 @@ void search_any(raft::resources& res, const search_params& params, const index<i
       float* ds        = distances + size_t(q0) * k;
       switch (kpl) {
         case 1:
-          final_merge_kernel<1><<<blocks, 128, 0, stream>>>(d_keys, d_probes, d_chunk,
+          launch_chained(final_merge_kernel<1>, blocks, 128, 0, stream, d_keys, d_probes, d_chunk,
                                                             idx.row_offsets(), idx.ids(), nq, n_probes,
                                                             k, int(metric), scale, nb, ds);
           break;
         case 2:
-          final_merge_kernel<2><<<blocks, 128, 0, stream>>>(d_keys, d_probes, d_chunk,
+          launch_chained(final_merge_kernel<2>, blocks, 128, 0, stream, d_keys, d_probes, d_chunk,
                                                             idx.row_offsets(), idx.ids(), nq, n_probes,
                                                             k, int(metric), scale, nb, ds);
           break;
         default:
-          final_merge_kernel<4><<<blocks, 128, 0, stream>>>(d_keys, d_probes, d_chunk,
+          launch_chained(final_merge_kernel<4>, blocks, 128, 0, stream, d_keys, d_probes, d_chunk,
                                                             idx.row_offsets(), idx.ids(), nq, n_probes,
                                                             k, int(metric), scale, nb, ds);
       }
