@@ -189,7 +189,6 @@ coarse_tc_kernel(const __grid_constant__ CUtensorMap map_a_hi, const __grid_cons
                  const __grid_constant__ CUtensorMap map_b_hi, const __grid_constant__ CUtensorMap map_b_lo,
                  const tc_params p)
 {
-  chain_begin();
   static_assert(!kARes || kProducts <= 2, "the resident-query variant stages one list operand");
   // Only the operands the chosen number of products reads are staged, and the 192 KB of stage memory
   // hold as many stages of that size as fit: 4 x 48 KB (three products), 6 x 32 KB (two), 8 x 24 KB
@@ -245,6 +244,7 @@ coarse_tc_kernel(const __grid_constant__ CUtensorMap map_a_hi, const __grid_cons
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  chain_begin();
   const uint32_t tmem_base = *reinterpret_cast<volatile uint32_t*>(tmem_slot);
 
   // Persistent CTAs (one per SM) over the n_work = query tiles x list tiles, list tile fastest, every SM

@@ -124,7 +124,6 @@ __global__ void __launch_bounds__(kFilterThreads, 1)
 filter_kernel(const __grid_constant__ CUtensorMap map_16, const __grid_constant__ CUtensorMap map_64,
               const __grid_constant__ CUtensorMap map_128, const filter_params p)
 {
-  chain_begin();
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw_a  = smem_u32(smem_raw);
   const uint32_t base_a = (raw_a + 1023u) & ~1023u;
@@ -137,9 +136,9 @@ filter_kernel(const __grid_constant__ CUtensorMap map_16, const __grid_constant_
   const uint32_t bar_tempty = bar_tfull + 2 * 8;
   uint32_t* tmem_slot       = reinterpret_cast<uint32_t*>(bars + 2 * kMaxStages + 4);
   const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
-  const uint32_t n_tiles  = __ldg(p.n_tiles);
   const uint32_t n_blocks = (p.k_chunks + 7u) >> 3;
 
+  // (barriers, tensor memory and the codebook, which is the index's: while the kernel before this one ends)
   if (threadIdx.x == 0) {
     for (uint32_t s = 0; s < p.n_stages; s++) {
       mbar_init(bar_full + s * 8, kDecodeWarps + 1);
@@ -165,7 +164,9 @@ filter_kernel(const __grid_constant__ CUtensorMap map_16, const __grid_constant_
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  chain_begin();
   const uint32_t tmem_base = *reinterpret_cast<volatile uint32_t*>(tmem_slot);
+  const uint32_t n_tiles   = __ldg(p.n_tiles);
   bool ok = true;
 
   if (warp < kDecodeWarps) {

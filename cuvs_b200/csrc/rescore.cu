@@ -275,7 +275,6 @@ __device__ __forceinline__ bool score_row(const rescore_params& p, const float* 
 template <int LutKind, bool OutHalf, bool IsIP, int kLen, int kBits, bool kSmem>
 __global__ void __launch_bounds__(1024, 1) rescore_kernel(const rescore_params p)
 {
-  chain_begin();
   extern __shared__ __align__(16) uint8_t smem[];
   const uint32_t gt = p.group_threads;
   const uint32_t g = threadIdx.x / gt, t = threadIdx.x % gt;
@@ -313,6 +312,7 @@ __global__ void __launch_bounds__(1024, 1) rescore_kernel(const rescore_params p
     }
   }
   __syncthreads();
+  chain_begin();  // (the codebook is the index's: copied while the kernel before this one ends)
   const bool all          = *p.error != 0u;
   const uint32_t n_groups = blockDim.x / gt;
 

@@ -697,7 +697,6 @@ __device__ __forceinline__ void score_part(accum<LutKind, OutHalf, IsIP>& acc, c
 template <int PqBits, int LutKind, bool OutHalf, bool IsIP, int KPL, int PQD = 0, int GT = 0, int LEN = 0>
 __global__ void __launch_bounds__(1024, 1) scan_kernel(const scan_params p)
 {
-  chain_begin();
   using lut_t               = typename lut_elem<LutKind>::type;
   constexpr uint32_t kBook  = 1u << PqBits;
   constexpr int kPerPiece   = 128 / PqBits;
@@ -769,6 +768,7 @@ __global__ void __launch_bounds__(1024, 1) scan_kernel(const scan_params p)
   }
   __syncthreads();
   tmem_fence_after();
+  chain_begin();  // (the codebook is the index's: copied while the kernel before this one ends)
   // this warp's window into tensor memory: lanes 32 * (warp % 4) .. + 31
   const uint32_t tmem_lane_a = tmem_base + (((uint32_t(tid) >> 5) & 3u) << 21);
 
