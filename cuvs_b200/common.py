@@ -47,6 +47,12 @@ class Resources:
         if self._fixed_stream is None:
             L.check(self._lib.cuvsStreamSet(self.handle, _current_stream()))
 
+    def stream_at_call(self, device: int) -> int:
+        """The stream that a call made now uses: the fixed one, else torch's current one."""
+        if self._fixed_stream is not None:
+            return self._fixed_stream
+        return _raw_stream(device) if _raw_stream is not None else _current_stream()
+
     def sync(self):
         L.check(self._lib.cuvsStreamSync(self.handle))
 
@@ -65,8 +71,9 @@ class Resources:
 _default_resources = {}
 
 
-def default_resources() -> Resources:
-    dev = torch.cuda.current_device()
+def default_resources(dev: int | None = None) -> Resources:
+    if dev is None:
+        dev = torch.cuda.current_device()
     r = _default_resources.get(dev)
     if r is None:
         r = _default_resources[dev] = Resources()

@@ -500,6 +500,23 @@ extern "C" cuvsError_t cuvsIvfPqTransform(cuvsResources_t res, cuvsIvfPqIndex_t 
 // search / serialize / deserialize
 // ------------------------------------------------------------------------------------------------
 namespace {
+void search_arrays(cuvsResources_t res, cuvsIvfPqSearchParams_t params, const index_t& ix, const void* queries,
+                   ivf_pq::elem_t type, int64_t n_queries, int64_t dim, int64_t k, int64_t* neighbors, float* distances,
+                   ivf_pq::bitset_view filter)
+{
+  CUVS_EXPECTS(dim == int64_t(ix.dim()),
+               "Number of query dimensions should equal number of dimensions in the index.");
+  ivf_pq::search_params sp;
+  sp.n_probes                 = params->n_probes;
+  sp.lut_dtype                = params->lut_dtype;
+  sp.internal_distance_dtype  = params->internal_distance_dtype;
+  sp.preferred_shmem_carveout = params->preferred_shmem_carveout;
+  sp.coarse_search_dtype      = params->coarse_search_dtype;
+  sp.max_internal_batch_size  = params->max_internal_batch_size;
+  ivf_pq::search_any(*res_of(res), sp, ix, queries, type, uint32_t(n_queries), uint32_t(k), neighbors, distances,
+                     nullptr, filter);
+}
+
 void search_entry(cuvsResources_t res, cuvsIvfPqSearchParams_t params, cuvsIvfPqIndex_t index,
                   DLManagedTensor* queries_tensor, DLManagedTensor* neighbors_tensor,
                   DLManagedTensor* distances_tensor, ivf_pq::bitset_view filter)
@@ -527,19 +544,31 @@ void search_entry(cuvsResources_t res, cuvsIvfPqSearchParams_t params, cuvsIvfPq
                "of queries.");
   CUVS_EXPECTS(neighbors.shape[1] == distances.shape[1],
                "Number of columns in output neighbors and distances matrices must equal k");
-  CUVS_EXPECTS(queries.shape[1] == int64_t(ix->dim()),
-               "Number of query dimensions should equal number of dimensions in the index.");
-  ivf_pq::search_params sp;
-  sp.n_probes                 = params->n_probes;
-  sp.lut_dtype                = params->lut_dtype;
-  sp.internal_distance_dtype  = params->internal_distance_dtype;
-  sp.preferred_shmem_carveout = params->preferred_shmem_carveout;
-  sp.coarse_search_dtype      = params->coarse_search_dtype;
-  sp.max_internal_batch_size  = params->max_internal_batch_size;
-  ivf_pq::search_any(*res_of(res), sp, *ix, q, et, uint32_t(queries.shape[0]),
-                     uint32_t(neighbors.shape[1]), nb, ds, nullptr, filter);
+  search_arrays(res, params, *ix, q, et, queries.shape[0], queries.shape[1], neighbors.shape[1], nb, ds, filter);
 }
 }  // namespace
+
+extern "C" cuvsError_t cuvsB200IvfPqSearchArrays(cuvsResources_t res, cudaStream_t stream, void* params, void* index,
+                                                 const void* queries, int dtype_code, int dtype_bits,
+                                                 int64_t n_queries, int64_t dim, int64_t k, int64_t* neighbors,
+                                                 float* distances, const uint32_t* filter_bits, int64_t filter_words,
+                                                 bool sync)
+{
+  return translate_exceptions([=] {
+    CUVS_EXPECTS(params != nullptr, "null argument");
+    auto* r   = res_of(res);
+    r->stream = stream;
+    const DLDataType type{uint8_t(dtype_code), uint8_t(dtype_bits), 1};
+    ivf_pq::bitset_view view{};
+    if (filter_bits != nullptr) {
+      view.bits   = filter_bits;
+      view.n_bits = uint64_t(filter_words) * 32u;
+    }
+    search_arrays(res, static_cast<cuvsIvfPqSearchParams_t>(params), *index_of(static_cast<cuvsIvfPqIndex_t>(index)), queries, elem_of_dtype(type, "queries"),
+                  n_queries, dim, k, neighbors, distances, view);
+    if (sync) { r->sync(); }
+  });
+}
 
 extern "C" cuvsError_t cuvsIvfPqSearch(cuvsResources_t res, cuvsIvfPqSearchParams_t params,
                                        cuvsIvfPqIndex_t index, DLManagedTensor* queries_tensor,

@@ -55,6 +55,17 @@ CUVS_EXPORT cuvsError_t cuvsB200SetCoarseMode(int mode);
  * which 0 chooses for large batches only. */
 CUVS_EXPORT cuvsError_t cuvsB200SetScanCodebookHome(int home);
 
+/* No counterpart in the reference: cuvsIvfPqSearch(WithFilter) on row-major device arrays given by their addresses, for
+ * callers to whom three tensor descriptors and three calls cost more than the launches (one query takes tens of
+ * microseconds).  `stream` becomes the handle's stream; `queries` is [n_queries, dim] of `dtype`, the outputs are
+ * [n_queries, k]; `filter_words` 32-bit words of a bitset, or NULL; `sync`: wait for the result. */
+CUVS_EXPORT cuvsError_t cuvsB200IvfPqSearchArrays(cuvsResources_t res, cudaStream_t stream,
+                                                  void* params /* cuvsIvfPqSearchParams_t */,
+                                                  void* index /* cuvsIvfPqIndex_t */, const void* queries,
+                                                  int dtype_code, int dtype_bits, int64_t n_queries, int64_t dim, int64_t k,
+                                                  int64_t* neighbors, float* distances, const uint32_t* filter_bits,
+                                                  int64_t filter_words, bool sync);
+
 /* No counterpart in the reference.  Every wait inside the tensor-core probe-selection kernel is bounded;
  * when one runs out the kernel sets an error word, frees what it holds and returns, the stages behind
  * it recompute the probes of every query of that batch with the exact path, and the handle counts the
