@@ -166,6 +166,8 @@ SIGNATURES = {
                              _P(DLManagedTensor), C.c_int, _P(C.c_uint32)],
     "cuvsB200IvfPqSearchArrays": [C.c_size_t, C.c_void_p, _P(SearchParamsStruct), _P(IndexStruct), C.c_void_p, C.c_int, C.c_int,
                                   C.c_int64, C.c_int64, C.c_int64, C.c_void_p, C.c_void_p, C.c_void_p, C.c_int64, C.c_bool],
+    "cuvsB200RefineArrays": [C.c_size_t, C.c_void_p, C.c_void_p, C.c_int64, C.c_int64, C.c_int, C.c_int, C.c_void_p,
+                             C.c_int64, C.c_void_p, C.c_int64, C.c_int, C.c_void_p, C.c_void_p, C.c_int64, C.c_bool],
     "cuvsB200SetCoarseMode": [C.c_int],
     "cuvsB200SetScanCodebookHome": [C.c_int],
     "cuvsB200CoarseTimeouts": [C.c_size_t, _P(C.c_uint64)],

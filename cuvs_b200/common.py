@@ -80,6 +80,16 @@ def default_resources(dev: int | None = None) -> Resources:
     return r
 
 
+CUDA_DEVICES = [torch.device("cuda", i) for i in range(64)]
+# (type code, bits) of vectors
+ELEMENT_TYPES = {t: _TORCH_DL[t] for t in (torch.float32, torch.float16, torch.int8, torch.uint8)}
+
+
+def is_cuda_matrix(t, dtype) -> bool:
+    """A row-major matrix of `dtype` that native code can be given by its address."""
+    return type(t) is torch.Tensor and t.dtype == dtype and t.is_cuda and t.dim() == 2 and t.is_contiguous()
+
+
 # ndim | dtype code << 32 | bits << 40 | lanes << 48, as the words of a DLTensor hold them
 _TORCH_WORD = {t: (code << 32) | (bits << 40) | (1 << 48) for t, (code, bits) in _TORCH_DL.items()}
 _NP_WORD = {t: (code << 32) | (bits << 40) | (1 << 48) for t, (code, bits) in _NP_DL.items()}

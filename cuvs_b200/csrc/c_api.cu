@@ -916,6 +916,22 @@ extern "C" cuvsError_t cuvsRefine(cuvsResources_t res, DLManagedTensor* dataset,
   });
 }
 
+extern "C" cuvsError_t cuvsB200RefineArrays(cuvsResources_t res, cudaStream_t stream, const void* dataset, int64_t n_rows,
+                                            int64_t dim, int dtype_code, int dtype_bits, const void* queries,
+                                            int64_t n_queries, const int64_t* candidates, int64_t n_candidates, int metric,
+                                            int64_t* indices, float* distances, int64_t k, bool sync)
+{
+  return translate_exceptions([=] {
+    auto* r   = res_of(res);
+    r->stream = stream;
+    const DLDataType type{uint8_t(dtype_code), uint8_t(dtype_bits), 1};
+    cuvs::neighbors::refine_any(*r, dataset, elem_of_dtype(type, "dataset"), n_rows, uint32_t(dim), queries,
+                                uint32_t(n_queries), candidates, uint32_t(n_candidates), ivf_pq::DistanceType(metric),
+                                indices, distances, uint32_t(k));
+    if (sync) { r->sync(); }
+  });
+}
+
 extern "C" cuvsError_t cuvsMultiGpuIvfPqSelectProbes(cuvsResources_t res, cuvsIvfPqIndex_t index,
                                                      DLManagedTensor* queries, DLManagedTensor* probes)
 {

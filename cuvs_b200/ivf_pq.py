@@ -12,7 +12,8 @@ import numpy as np
 import torch
 
 from . import _lib as L
-from .common import _TORCH_DL, DLTensorRef, Resources, default_resources, view_to_torch
+from .common import (CUDA_DEVICES, ELEMENT_TYPES, DLTensorRef, Resources, default_resources, is_cuda_matrix,
+                     view_to_torch)
 
 _METRICS = {"sqeuclidean": 0, "euclidean": 1, "cosine": 2, "inner_product": 6}
 _METRIC_NAMES = {v: k for k, v in _METRICS.items()}
@@ -237,29 +238,24 @@ def build_precomputed(index_params: IndexParams, dim, pq_centers, centers, cente
     return idx
 
 
-_CUDA = [torch.device("cuda", i) for i in range(64)]
-# (type code, bits) of the queries that a search takes
-_QUERY_TYPES = {t: _TORCH_DL[t] for t in (torch.float32, torch.float16, torch.int8, torch.uint8)}
-
-
 def _search_arrays(search_params, index, queries, k, neighbors, distances, resources, sync, filter):
     """The whole of a search of CUDA tensors in one native call (three tensor descriptors and three calls took 12 of the
     56 us of one query).  None where an argument is not what that call takes: the general path then says what is wrong."""
-    word = _QUERY_TYPES.get(queries.dtype)
+    word = ELEMENT_TYPES.get(queries.dtype)
     shape = queries.shape
     if word is None or len(shape) != 2 or not queries.is_contiguous():
         return None
     device = torch.cuda.current_device()
-    if device >= len(_CUDA):
+    if device >= len(CUDA_DEVICES):
         return None
     n = shape[0]
     if neighbors is None:
-        neighbors = torch.empty((n, k), dtype=torch.int64, device=_CUDA[device])
-    elif not _is_matrix(neighbors, torch.int64):
+        neighbors = torch.empty((n, k), dtype=torch.int64, device=CUDA_DEVICES[device])
+    elif not is_cuda_matrix(neighbors, torch.int64):
         return None
     if distances is None:
-        distances = torch.empty((n, k), dtype=torch.float32, device=_CUDA[device])
-    elif not _is_matrix(distances, torch.float32):
+        distances = torch.empty((n, k), dtype=torch.float32, device=CUDA_DEVICES[device])
+    elif not is_cuda_matrix(distances, torch.float32):
         return None
     out = neighbors.shape
     if out != distances.shape or out[0] != n or out.numel() == 0:
@@ -278,10 +274,6 @@ def _search_arrays(search_params, index, queries, k, neighbors, distances, resou
                                                word[0], word[1], n, shape[1], out[1], neighbors.data_ptr(),
                                                distances.data_ptr(), bits, words, bool(sync)))
     return distances, neighbors
-
-
-def _is_matrix(t, dtype):
-    return type(t) is torch.Tensor and t.dtype == dtype and t.is_cuda and t.dim() == 2 and t.is_contiguous()
 
 
 def search(search_params: SearchParams, index: Index, queries, k, neighbors=None, distances=None,

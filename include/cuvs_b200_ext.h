@@ -66,6 +66,14 @@ CUVS_EXPORT cuvsError_t cuvsB200IvfPqSearchArrays(cuvsResources_t res, cudaStrea
                                                   int64_t* neighbors, float* distances, const uint32_t* filter_bits,
                                                   int64_t filter_words, bool sync);
 
+/* No counterpart in the reference: cuvsRefine on row-major device arrays given by their addresses, as above; dataset and
+ * queries have the same element type. */
+CUVS_EXPORT cuvsError_t cuvsB200RefineArrays(cuvsResources_t res, cudaStream_t stream, const void* dataset,
+                                             int64_t n_rows, int64_t dim, int dtype_code, int dtype_bits,
+                                             const void* queries, int64_t n_queries, const int64_t* candidates,
+                                             int64_t n_candidates, int metric, int64_t* indices, float* distances,
+                                             int64_t k, bool sync);
+
 /* No counterpart in the reference.  Every wait inside the tensor-core probe-selection kernel is bounded;
  * when one runs out the kernel sets an error word, frees what it holds and returns, the stages behind
  * it recompute the probes of every query of that batch with the exact path, and the handle counts the
