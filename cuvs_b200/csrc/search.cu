@@ -870,12 +870,22 @@ void search_any(raft::resources& res, const search_params& params, const index<i
   // look-up-table kernels
   filter_plan fplan{};
   const uint32_t max_groups = uint32_t(ceildiv<uint64_t>(uint64_t(idx.accum_sorted_sizes()[n_probes]) + 31ull * n_probes, 32));
-  // (below some 4,000 pairs, and for k > 128, the look-up-table scan is as fast or faster: 162 against 178 us for 100
-  // queries of 20 probes, 632 against 754 us for 500 queries with k = 1000)
+  // Below some 4,000 pairs, and for k > 128, the look-up-table scan is as fast or faster: 162 against 178 us for 100
+  // queries of 20 probes, 632 against 754 us for 500 queries with k = 1000.  Where exact scores cost more it takes more
+  // pairs to win: 8-bit tables and half sums (wide bounds: 65 queries of 128 probes 296 against 342 us), and codes that
+  // the general loop scores (5 or 6 bits, or other lengths: 10,530 pairs 293 against 449 us, 28,034 pairs 544 against
+  // 278).  8-bit tables over other than 8-bit codes never do (64,065 pairs 1,022 against 2,977 us), half sums over codes of
+  // the general loop where a query has many probes for its k (777 queries, 40 probes, k 10: 288 against 255 us; 4,216
+  // queries, 10 probes, k 50: 624 against 748).
+  const bool wide_bounds = lut_kind == LUT_FP8 || out_half;
+  const bool straight    = idx.rot_dim() % 4 == 0 && ((idx.pq_bits() == 8 && (idx.pq_len() == 2 || idx.pq_len() == 4)) ||
+                                                   (idx.pq_bits() == 4 && idx.pq_len() == 2));
+  const bool never       = (lut_kind == LUT_FP8 && !(straight && idx.pq_bits() == 8)) || (out_half && !straight && n_probes < 2 * k);
+  const uint64_t enough  = straight && !wide_bounds ? 4096 : 16384;
   // (a list-sharded search exchanges bounds in the middle of the look-up-table scan: a collective, so that all its ranks
   // take that path)
   const int home = scan_codebook_home();
-  if (!res.scan_phase_hook && (home == 4 || (home == 0 && uint64_t(batch) * n_probes > 4096 && k <= 128))) {
+  if (!res.scan_phase_hook && (home == 4 || (home == 0 && !never && uint64_t(batch) * n_probes > enough && k <= 128))) {
     // bounds of one internal batch: within 2 GiB
     batch = uint32_t(std::max<uint64_t>(1, std::min<uint64_t>(batch, (1ull << 31) / (uint64_t(max_groups) * 16))));
     fplan = plan_filter(res, idx, lut_kind, out_half, is_ip, k, n_probes, batch);
