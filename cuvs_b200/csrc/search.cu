@@ -166,14 +166,15 @@ __global__ void prep_queries_kernel(const T* __restrict__ queries, uint32_t dim,
 }
 
 // Cosine: rows of rot_q divided by their norm (a chain of fused multiply-adds in ascending order, one thread per row, out
-// of shared memory).  32 rows per block.
+// of shared memory).  `per_block` rows per block: a warp's 32, or as many long rows as shared memory takes.
+constexpr uint32_t kNormRows = 32;
 __global__ void __launch_bounds__(256)
-normalize_rows_kernel(float* __restrict__ rot_q, uint32_t n_rows, uint32_t rot_dim)
+normalize_rows_kernel(float* __restrict__ rot_q, uint32_t n_rows, uint32_t rot_dim, uint32_t per_block)
 {
   chain_begin();
-  extern __shared__ float s_rows[];  // [32][rot_dim | 1]
-  __shared__ float s_norm[32];
-  const uint32_t r0 = blockIdx.x * 32u, nr = min(32u, n_rows - r0), ld = rot_dim | 1u;
+  extern __shared__ float s_rows[];  // [per_block][rot_dim | 1]
+  __shared__ float s_norm[kNormRows];
+  const uint32_t r0 = blockIdx.x * per_block, nr = min(per_block, n_rows - r0), ld = rot_dim | 1u;
   float* rows = rot_q + size_t(r0) * rot_dim;
   for (uint32_t i = threadIdx.x; i < nr * rot_dim; i += 256u) {
     const uint32_t r = i / rot_dim;
@@ -642,9 +643,12 @@ void launch_prep(raft::resources& res, const index<int64_t>& idx, const void* qp
     // (int8 images: the sums are integers below 2^24, scaled by 1 / 128^2)
     exact_rows_product(res, rot, idx.rot_dim(), d_fq, nq, dim_ext, idx.dim(), mode == 1 ? 1.0f / 16384.0f : 1.0f, d_rq);
     if (cosine) {
-      const size_t smem_n = size_t(32) * (idx.rot_dim() | 1u) * 4;
+      const size_t row   = size_t(idx.rot_dim() | 1u) * 4;
+      const auto rows    = uint32_t(std::min<size_t>(kNormRows, (size_t(res.smem_optin) - 1024) / row));
+      CUVS_EXPECTS(rows > 0, "IVF-PQ search: rot_dim = %u is too large for this engine", idx.rot_dim());
+      const size_t smem_n = rows * row;
       ensure_dynamic_smem(reinterpret_cast<const void*>(normalize_rows_kernel), smem_n);
-      launch_chained(normalize_rows_kernel, ceildiv(nq, 32u), 256, smem_n, stream, d_rq, nq, idx.rot_dim());
+      launch_chained(normalize_rows_kernel, ceildiv(nq, rows), 256, smem_n, stream, d_rq, nq, idx.rot_dim(), rows);
       CUDA_TRY(cudaGetLastError());
       res.launches++;
     }

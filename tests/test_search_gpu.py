@@ -514,3 +514,14 @@ def test_a_table_larger_than_shared_memory_goes_to_global_memory(ivf, oracle_mod
         d, i = gpu_search(ivf, g, q, k, p, "f32")
         do, io = O.search(ix, q, k, n_probes=p)
         assert_parity(d, i, do, io, 1e-5)
+
+
+# rotated dimensions around the size where 32 rows no longer fit one SM's shared memory, and well above; 33 queries: the
+# last block of rows is a remainder
+@pytest.mark.parametrize("dim,pq_dim", [(1799, 120), (1899, 100), (2047, 128)])
+def test_cosine_with_a_wide_rotation(ivf, oracle_mod, tmp_path, dim, pq_dim):
+    x, q, ix, path = build_case(oracle_mod, tmp_path, "wide_cosine", n=400, dim=dim, n_lists=4, pq_dim=pq_dim, pq_bits=4,
+                                metric=2, nq=33)
+    d, i = gpu_search(ivf, ivf.load(path), q, 10, 3)
+    do, io = oracle_mod.search(ix, q, 10, n_probes=3)
+    assert_parity(d, i, do, io, 1e-5)
