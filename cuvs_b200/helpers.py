@@ -117,5 +117,8 @@ def erase_list(index: Index, label: int, resources: Resources | None = None) -> 
 
 
 def reset_index(index: Index, resources: Resources | None = None) -> None:
-    """Remove every row of every list; the trained model stays (ivf_pq.hpp:3166)."""
+    """Remove every row of every list; the trained model stays (ivf_pq.hpp:3166).
+
+    The index keeps up to 64 MiB of each of its two arenas (codes, ids) for the rows to come; what is above that goes
+    back to the device."""
     L.check(L.load().cuvsIvfPqHelpersResetIndex(_res(resources).handle, index._h))

@@ -188,10 +188,10 @@ class dev_array {
     n_   = n;
     cap_ = n;
   }
-  // as resize, but keeps the allocation where it is large enough
-  void resize_within(size_t n)
+  // as resize, but keeps the allocation where it is large enough and at most `excess` bytes larger than asked for
+  void resize_within(size_t n, size_t excess)
   {
-    if (n > cap_) { resize(n); }
+    if (n > cap_ || (cap_ - n) * sizeof(T) > excess) { resize(n); }
     n_ = n;
   }
   void reset()
@@ -566,7 +566,8 @@ void extend_list_with_contiguous_codes(raft::resources& res, index<int64_t>* idx
 void extend_list(raft::resources& res, index<int64_t>* idx, const void* new_vectors, elem_t dtype,
                  const int64_t* new_indices, uint32_t n_rows, uint32_t label);
 }  // namespace codepacker
-// Remove all rows of one list / of every list (ivf_pq.hpp:3144, :3166).
+// Remove all rows of one list / of every list (ivf_pq.hpp:3144, :3166).  An emptied index holds at most 64 MiB of each of
+// its two arenas (codes, ids) for the rows to come; what is above that goes back to the device.
 void erase_list(raft::resources& res, index<int64_t>* idx, uint32_t label);
 void reset_index(raft::resources& res, index<int64_t>* idx);
 }  // namespace helpers

@@ -60,7 +60,8 @@ CUVS_EXPORT cuvsError_t cuvsIvfPqHelpersExtendList(cuvsResources_t res, cuvsIvfP
                                                    DLManagedTensor* new_vectors,
                                                    DLManagedTensor* new_indices, uint32_t label);
 
-/* Remove every row of one list / of all lists; the trained model stays. */
+/* Remove every row of one list / of all lists; the trained model stays.  An emptied index holds at most 64 MiB of each of
+ * its two arenas (codes, ids) for the rows to come; what is above that goes back to the device. */
 CUVS_EXPORT cuvsError_t cuvsIvfPqHelpersEraseList(cuvsResources_t res, cuvsIvfPqIndex_t index,
                                                   uint32_t label);
 CUVS_EXPORT cuvsError_t cuvsIvfPqHelpersResetIndex(cuvsResources_t res, cuvsIvfPqIndex_t index);

@@ -194,6 +194,37 @@ def test_erase_list_and_reset_index(mods, oracle_mod, tmp_path):
     assert len(g) == 6000
 
 
+@pytest.mark.parametrize("rows,kept", [(300_000, True), (1_300_000, False)])
+def test_an_emptied_index_gives_its_memory_back(mods, rows, kept):
+    """64 bytes per row of codes: 18 MiB stay for the next rows, 79 MiB go back to the device."""
+    ivf, H = mods
+    to = lambda a: torch.from_numpy(np.ascontiguousarray(a, dtype=np.float32)).cuda()  # noqa: E731
+    rng = np.random.default_rng(3)
+    centers = rng.standard_normal((8, 64))
+    g = ivf.build_precomputed(ivf.IndexParams(n_lists=8, pq_dim=64), 64, to(rng.standard_normal((64, 1, 256))), to(centers),
+                              to(centers), to(np.eye(64)))
+    x, ids = torch.randn(rows, 64, device="cuda"), torch.arange(rows, device="cuda")
+
+    def free():
+        torch.cuda.synchronize()
+        torch.cuda.empty_cache()
+        return torch.cuda.mem_get_info()[0]
+
+    ivf.extend(g, x, ids)
+    d0, i0 = ivf.search(ivf.SearchParams(n_probes=8), g, x[:50].contiguous(), 5)
+    filled = free()
+    H.reset_index(g)
+    back = free() - filled
+    assert back == 0 if kept else back >= 64 << 20
+    # fewer rows than before, then as many: the same answers
+    ivf.extend(g, x[:1000].contiguous(), ids[:1000].contiguous())
+    assert len(g) == 1000
+    H.reset_index(g)
+    ivf.extend(g, x, ids)
+    d1, i1 = ivf.search(ivf.SearchParams(n_probes=8), g, x[:50].contiguous(), 5)
+    assert bool((i0 == i1).all()) and bool((d0 == d1).all())
+
+
 def test_row_ranges_are_checked(mods):
     ivf, H = mods
     from cuvs_b200._lib import CuvsError
