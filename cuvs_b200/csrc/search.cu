@@ -873,6 +873,8 @@ void search_any(raft::resources& res, const search_params& params, const index<i
   // the two-step path (filter_scan.hpp) where it applies; a test override of the table's home asks for the
   // look-up-table kernels
   filter_plan fplan{};
+  const uint32_t f_data     = ceildiv(idx.pq_dim() * idx.filter_model().len_pad, 8u);
+  const uint32_t f_chunks   = round_up(f_data + 1u, 2u);  // 16-byte chunks of a row of the query operand
   const uint32_t max_groups = uint32_t(ceildiv<uint64_t>(uint64_t(idx.accum_sorted_sizes()[n_probes]) + 31ull * n_probes, 32));
   // Below some 4,000 pairs, and for k > 128, the look-up-table scan is as fast or faster: 162 against 178 us for 100
   // queries of 20 probes, 632 against 754 us for 500 queries with k = 1000.  Where exact scores cost more it takes more
@@ -890,9 +892,15 @@ void search_any(raft::resources& res, const search_params& params, const index<i
   // take that path)
   const int home = scan_codebook_home();
   if (!res.scan_phase_hook && (home == 4 || (home == 0 && !never && uint64_t(batch) * n_probes > enough && k <= 128))) {
-    // bounds of one internal batch: within 2 GiB
-    batch = uint32_t(std::max<uint64_t>(1, std::min<uint64_t>(batch, (1ull << 31) / (uint64_t(max_groups) * 16))));
     fplan = plan_filter(res, idx, lut_kind, out_half, is_ip, k, n_probes, batch);
+    // the bounds and the query operand of one internal batch: within 2 GiB each
+    const uint64_t per_query = std::max(uint64_t(max_groups), uint64_t(n_probes) * f_chunks) * 16;
+    const auto fits          = uint32_t(std::max<uint64_t>(1, (1ull << 31) / per_query));
+    if (fplan.use && fits < batch) {
+      // (the plan shares threads out by the number of queries; the look-up-table scan needs no smaller batch)
+      fplan = plan_filter(res, idx, lut_kind, out_half, is_ip, k, n_probes, fits);
+      if (fplan.use) { batch = fits; }
+    }
   }
   if (store_all && !fplan.use) {
     // keep the score matrix of one internal batch within 1 GiB
@@ -923,8 +931,6 @@ void search_any(raft::resources& res, const search_params& params, const index<i
   const size_t o_tiles   = lay.add(n_tiles * sizeof(filter_tile));
   const size_t o_units   = lay.add(f_use ? size_t(batch) * max_groups * 16 : 0);
   const size_t o_qscale  = lay.add(f_use && is_ip ? size_t(batch) * 4 : 0);
-  const uint32_t f_data  = f_use ? ceildiv(idx.pq_dim() * idx.filter_model().len_pad, 8u) : 0;
-  const uint32_t f_chunks = round_up(f_data + 1u, 2u);  // 16-byte chunks of an operand row
   const size_t o_operand = lay.add(f_use ? n_pairs_max * f_chunks * 16 : 0);
   const size_t o_order   = lay.add(f_use ? 0 : n_pairs_max * 32);
   const size_t o_count   = lay.add((size_t(n_lists) * 2 + 1) * 4);  // two segments of buckets, one per list each

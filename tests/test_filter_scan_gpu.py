@@ -102,3 +102,32 @@ def test_data_scale(ivf, oracle_mod, tmp_path, scale):
     ix.save(path)
     for lut in ("f32", "fp8") + (("f16",) if scale < 1e3 else ()):
         check(ivf, O, ix, path, q, 10, 6, lut, "f32", 1e-5 if lut == "f32" else 1e-2)
+
+
+@pytest.mark.parametrize("dim,pq_dim,bits,n_lists,rows,n_queries,metric,lut,batches", [
+    # bounds of 501 KB per query, but the look-up tables score these: one batch
+    (16, 8, 8, 64, 1_000_000, 5000, "inner_product", np.uint8, 1),
+    # the same size with bounds, and a query operand of 803 KB: 2 GiB at a time
+    (16, 8, 8, 64, 1_000_000, 5000, "inner_product", np.float16, 2),
+    (768, 384, 4, 512, 20_000, 3000, "inner_product", np.float16, 2)])
+def test_size_of_an_internal_batch(ivf, dim, pq_dim, bits, n_lists, rows, n_queries, metric, lut, batches):
+    import ctypes as C
+    from cuvs_b200 import _lib as L
+    from cuvs_b200.common import Resources
+    g = torch.Generator(device="cuda").manual_seed(4)
+    normal = lambda *shape: torch.randn(*shape, generator=g, device="cuda")  # noqa: E731
+    centers = normal(n_lists, dim)
+    index = ivf.build_precomputed(ivf.IndexParams(n_lists=n_lists, pq_dim=pq_dim, pq_bits=bits, metric=metric), dim,
+                                  normal(pq_dim, dim // pq_dim, 1 << bits) * 0.3, centers, centers,
+                                  torch.eye(dim, device="cuda"))
+    x = centers[torch.arange(rows, device="cuda") % n_lists] + 0.3 * normal(rows, dim)
+    ivf.extend(index, x, torch.arange(rows, device="cuda"))
+    q = x[:n_queries] + 0.1 * normal(n_queries, dim)
+    res, lib, stats = Resources(), L.load(), L.SearchStats()
+    L.check(lib.cuvsB200StatsEnable(res.handle, True))
+    p = dict(n_probes=n_lists, lut_dtype=lut)
+    d, i = ivf.search(ivf.SearchParams(max_internal_batch_size=n_queries, **p), index, q, 10, resources=res)
+    L.check(lib.cuvsB200StatsGet(res.handle, C.byref(stats), True))
+    assert stats.batches == batches
+    d2, i2 = ivf.search(ivf.SearchParams(max_internal_batch_size=1000, **p), index, q, 10, resources=res)
+    assert bool((i == i2).all()) and bool((d == d2).all())
