@@ -333,7 +333,8 @@ filter_kernel(const __grid_constant__ CUtensorMap map_16, const __grid_constant_
             }
           }
         }
-        if (!mbar_wait(bar_empty + stage * 8, phase ^ 1u, p.spin_limit)) {
+        // (the whole warp leaves, or none of it: the lanes meet again below)
+        if (!__all_sync(kFullMask, mbar_wait(bar_empty + stage * 8, phase ^ 1u, p.spin_limit))) {
           ok = false;
           break;
         }
