@@ -775,7 +775,7 @@ extern "C" cuvsError_t cuvsB200CoarseTimeouts(cuvsResources_t res, uint64_t* n_b
     CUVS_EXPECTS(n_batches != nullptr, "null output pointer");
     auto* r = res_of(res);
     r->adopt_tc_verdict();
-    *n_batches = r->tc_timeouts;
+    *n_batches = r->tc_timeouts + *static_cast<volatile uint32_t*>(r->pinned + 13);
   });
 }
 
@@ -784,7 +784,7 @@ extern "C" cuvsError_t cuvsB200SetCoarseWaitTest(uint32_t spin_limit, uint32_t s
   return translate_exceptions([=] {
     // a limit below 1000 iterations could fire on a healthy but busy GPU
     CUVS_EXPECTS(spin_limit == 0 || spin_limit >= 1000, "spin_limit must be 0 or at least 1000");
-    ivf_pq::set_coarse_tc_wait_test(spin_limit, skip_stage);
+    ivf_pq::set_tc_wait_test(spin_limit, skip_stage);
   });
 }
 

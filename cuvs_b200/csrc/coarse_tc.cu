@@ -1153,13 +1153,9 @@ bool& tc_resident_ref()
   return on;
 }
 
-// test hook: a shorter limit for the bounded waits and one operand stage left unfilled
-struct tc_fault {
-  uint32_t spin_limit = 0, skip_kb = 0;
-};
-tc_fault& tc_fault_ref()
+wait_limits& wait_limits_ref()
 {
-  static tc_fault f;
+  static wait_limits f{kSpinLimit, 0};
   return f;
 }
 
@@ -1192,10 +1188,10 @@ CUtensorMap make_map_2d(CUtensorMapDataType type, uint32_t elem_bytes, const voi
 
 void set_coarse_tc_products(int products) { tc_products_ref() = products; }
 void set_coarse_tc_resident(bool on) { tc_resident_ref() = on; }
-void set_coarse_tc_wait_test(uint32_t spin_limit, uint32_t skip_kb)
+wait_limits tc_wait_limits() { return wait_limits_ref(); }
+void set_tc_wait_test(uint32_t spin_limit, uint32_t skip_kb)
 {
-  tc_fault_ref().spin_limit = spin_limit;
-  tc_fault_ref().skip_kb    = skip_kb;
+  wait_limits_ref() = {spin_limit ? spin_limit : kSpinLimit, skip_kb};
 }
 
 bool coarse_tc_usable(uint32_t n_lists, uint32_t n_probes, uint32_t dim_ext)
@@ -1316,8 +1312,9 @@ void select_clusters_tc(raft::resources& res, const float* centers, const float*
   p.cand_key  = cand_key;
   p.cand_bound = cand_bnd;
   p.error     = words;
-  p.spin_limit = tc_fault_ref().spin_limit ? tc_fault_ref().spin_limit : kSpinLimit;
-  p.skip_kb    = tc_fault_ref().skip_kb;
+  const wait_limits wl = tc_wait_limits();
+  p.spin_limit         = wl.spin_limit;
+  p.skip_kb            = wl.skip_kb;
   const uint32_t q_tiles = ceildiv<uint32_t>(n_queries, kBM);
   p.n_work               = q_tiles * n_tiles;
   const uint32_t grid    = std::min<uint32_t>(uint32_t(res.sm_count), p.n_work);

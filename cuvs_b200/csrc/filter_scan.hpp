@@ -53,7 +53,7 @@ struct filter_params {
   float4* units;           // [n_q, max_groups] bounds of the four units of a 32-row group
   uint32_t n_stages;
   uint32_t* error;
-  uint32_t spin_limit;
+  uint32_t spin_limit, skip_kb;  // tc_wait_limits
 };
 
 struct rescore_params {
@@ -70,6 +70,7 @@ struct rescore_params {
   const float4* units;
   const float* pair_norm;
   const uint32_t* error;
+  uint32_t* timeouts;           // pinned host word: batches with the error word set
   const uint32_t* filter_bits;
   uint64_t filter_nbits;
   uint32_t n_lists, n_queries, n_probes, k, max_groups;

@@ -222,7 +222,7 @@ struct label_params {
   uint4* seconds;    // second largest keys of their units
   uint4* lists;      // their lists
   uint32_t* error;
-  uint32_t spin_limit;
+  uint32_t spin_limit, skip_kb;  // tc_wait_limits
 };
 
 __global__ void __launch_bounds__(kThreads, 1)
@@ -304,9 +304,12 @@ label_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
               break;
             }
             const uint32_t dst = stage_base + stage * stage_size, bar = bar_full + stage * 8;
-            mbar_arrive_expect_tx(bar, stage_size);
-            tma_load_2d(dst, &map_b, bar, int(kb * kBlockK), int(t * kLists));
-            if (!p.a_resident) { tma_load_2d(dst + kBBlock, &map_a, bar, int(kb * kBlockK), row0); }
+            // (test only: a block that never comes, so that the wait for it runs out)
+            if (kb + 1 != p.skip_kb || t != t0 || item != blockIdx.x) {
+              mbar_arrive_expect_tx(bar, stage_size);
+              tma_load_2d(dst, &map_b, bar, int(kb * kBlockK), int(t * kLists));
+              if (!p.a_resident) { tma_load_2d(dst + kBBlock, &map_a, bar, int(kb * kBlockK), row0); }
+            }
             if (++stage == p.n_stages) {
               stage = 0;
               phase ^= 1u;
@@ -486,6 +489,7 @@ struct label_records {
   const uint4* lists;
   const float* eps;
   const uint32_t* error;
+  uint32_t* timeouts;  // pinned host word: calls with the error word set
   uint32_t splits, n_rows, n_lists;
 };
 
@@ -526,6 +530,7 @@ label_finish_kernel(const label_records p, const float* __restrict__ x, const fl
     out = fmaxf(out, __shfl_xor_sync(mask, out, o));
   }
   const float t = top - 2.0f * __ldg(p.eps + r);
+  if (*p.error != 0u && blockIdx.x == 0 && threadIdx.x == 0) { count_timeout(p.timeouts); }
   // (negated: an infinite or undefined bound is not proof)
   if (*p.error != 0u || !(out < t)) {
     if (u == 0) { redo[atomicAdd(counts, 1u)] = r; }
@@ -732,13 +737,15 @@ void label_rows_tc(raft::resources& res, const float* centers, const void* model
   p.lists      = reinterpret_cast<uint4*>(ws + y.o_lists);
   p.seconds    = reinterpret_cast<uint4*>(ws + y.o_seconds);
   p.error      = words;
-  p.spin_limit = kSpinLimit;
+  const wait_limits wl = tc_wait_limits();
+  p.spin_limit = wl.spin_limit;
+  p.skip_kb    = wl.skip_kb;
   const CUtensorMap ma = make_map_2d(CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, a, n_rows, uint64_t(width) * products, kRows, kBlockK, CU_TENSOR_MAP_SWIZZLE_128B);
   const CUtensorMap mb = make_map_2d(CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, b, n_lists, width, kLists, kBlockK, CU_TENSOR_MAP_SWIZZLE_128B);
   const size_t smem    = kRoom + 1024 + 256;
   ensure_dynamic_smem(reinterpret_cast<const void*>(label_tc_kernel), smem);
   label_tc_kernel<<<std::min(uint32_t(res.sm_count), p.n_items), kThreads, smem, stream>>>(ma, mb, p);
-  const label_records rec{p.keys, p.seconds, p.lists, eps, words, p.splits, n_rows, n_lists};
+  const label_records rec{p.keys, p.seconds, p.lists, eps, words, res.pinned + 13, p.splits, n_rows, n_lists};
   label_finish_kernel<<<ceildiv(n_rows, 64u), 256, 0, stream>>>(rec, x_ext, centers, dim_ext, alpha, labels, redo, words + 1);
   label_units_kernel<<<std::min<uint32_t>(uint32_t(res.sm_count) * 8, blocks), 256, 0, stream>>>(rec, x_ext, centers, dim_ext, alpha,
                                                                                                labels, redo, words + 1);

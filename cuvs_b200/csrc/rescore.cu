@@ -24,6 +24,7 @@
 #include "filter_scan.hpp"
 #include "scan.cuh"
 #include "search_internal.hpp"
+#include "tc_ptx.cuh"
 #include "topk.cuh"
 
 #include <algorithm>
@@ -314,6 +315,7 @@ __global__ void __launch_bounds__(1024, 1) rescore_kernel(const rescore_params p
   __syncthreads();
   chain_begin();  // (the codebook is the index's: copied while the kernel before this one ends)
   const bool all          = *p.error != 0u;
+  if (all && blockIdx.x == 0 && threadIdx.x == 0) { count_timeout(p.timeouts); }
   const uint32_t n_groups = blockDim.x / gt;
 
   // the first query of a group by its number, the next ones from a counter (claimed one ahead)

@@ -62,6 +62,7 @@ resources::resources()
   cc_major   = prop.major;
   CUDA_TRY(cudaMallocHost(&pinned, 64));
   pinned[12] = 0;
+  pinned[13] = 0;
 }
 
 resources::~resources()

@@ -1082,7 +1082,9 @@ void search_any(raft::resources& res, const search_params& params, const index<i
       fp.units        = d_units;
       fp.n_stages     = fplan.n_stages;
       fp.error        = d_counter + 2;
-      fp.spin_limit   = kSpinLimit;
+      const wait_limits wl = tc_wait_limits();
+      fp.spin_limit   = wl.spin_limit;
+      fp.skip_kb      = wl.skip_kb;
       launch_filter(fp, d_operand, n_pairs, int(std::min<size_t>(size_t(res.sm_count), n_tiles)), fplan.filter_smem, stream);
       res.launches++;
       if (stats) { res.stats_mark(ev, 4); }
@@ -1101,6 +1103,7 @@ void search_any(raft::resources& res, const search_params& params, const index<i
       rp.units        = d_units;
       rp.pair_norm    = d_norm;
       rp.error        = d_counter + 2;
+      rp.timeouts     = res.pinned + 13;
       rp.filter_bits  = filter.bits;
       rp.filter_nbits = filter.n_bits;
       rp.n_lists      = n_lists;

@@ -80,9 +80,13 @@ void set_coarse_tc_products(int products);
 // process-wide override used by tests: false = the tensor-core coarse GEMM streams both operands even
 // where the query tile could stay resident in shared memory
 void set_coarse_tc_resident(bool on);
-// test hook of the bounded waits of the tensor-core coarse kernel: iterations a wait may take (0 = the
-// default) and 1 + index of an operand stage left unfilled (0 = none)
-void set_coarse_tc_wait_test(uint32_t spin_limit, uint32_t skip_kb);
+// Bounded waits of the tensor-core kernels (coarse_tc.cu, filter_scan.cu, label_tc.cu): iterations a wait may take, and for
+// tests 1 + index of the K block of every CTA's first tile that is never brought (0 = none).  Process-wide.
+struct wait_limits {
+  uint32_t spin_limit, skip_kb;
+};
+wait_limits tc_wait_limits();
+void set_tc_wait_test(uint32_t spin_limit /* 0 = the default */, uint32_t skip_kb);
 void set_coarse_mode(int mode);  // process-wide override used by tests: 0 auto, 1 SIMT, 2 tensor core
 // process-wide override used by tests: 0 = the per-subspace codebook goes to tensor memory where it
 // fits, 1 = never (shared memory, else global memory)

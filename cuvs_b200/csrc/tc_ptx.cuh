@@ -42,6 +42,14 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, uint32_
   }
   return false;
 }
+// A batch whose tensor-core pass timed out, counted in the handle's pinned word: by one thread of the kernel behind that
+// pass (the kernels of a handle run one after the other).
+__device__ __forceinline__ void count_timeout(uint32_t* word)
+{
+  volatile uint32_t* w = word;
+  *w                   = *w + 1u;
+  __threadfence_system();
+}
 __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, uint32_t bar, int x,
                                             int y)
 {

@@ -176,7 +176,8 @@ struct resources {
   uint32_t tc_redo_queries   = 0;
   bool tc_redo_adapts        = false;
   void adopt_tc_verdict();
-  // batches whose coarse GEMM gave up on a bounded wait (their probes were recomputed exactly)
+  // batches whose coarse GEMM gave up on a bounded wait (their probes were recomputed exactly); those of the fine search's
+  // bounds and of the labelling are counted by the kernels behind them in pinned[13]
   uint64_t tc_timeouts       = 0;
 
   resources();

@@ -131,3 +131,32 @@ def test_size_of_an_internal_batch(ivf, dim, pq_dim, bits, n_lists, rows, n_quer
     assert stats.batches == batches
     d2, i2 = ivf.search(ivf.SearchParams(max_internal_batch_size=1000, **p), index, q, 10, resources=res)
     assert bool((i == i2).all()) and bool((d == d2).all())
+
+
+@pytest.mark.parametrize("lut,internal,bits,k", [("f32", "f32", 8, 10), ("fp8", "f32", 8, 100), ("f16", "f16", 6, 17)])
+def test_a_wait_that_runs_out_scores_every_row(ivf, oracle_mod, tmp_path, lut, internal, bits, k):
+    """One block of every CTA's first tile never comes and the limit is about a millisecond: the bounding kernel gives up,
+    the exact pass scores every row of the probed lists, the handle counts the batch, and the next search is a healthy
+    one.  (Sixteen lists: the coarse search does not run on the tensor cores.)"""
+    import ctypes as C
+    from cuvs_b200 import _lib as L
+    from cuvs_b200.common import Resources
+    x, q, ix, path = build_case(oracle_mod, tmp_path, "t", n=3000, dim=48, n_lists=16, pq_dim=24, pq_bits=bits, nq=40)
+    do, io = oracle_mod.search(ix, q, k, n_probes=9, lut_dtype=LUT[lut][1], internal_dtype=LUT[internal][1])
+    g, lib, res = ivf.load(path), L.load(), Resources()
+    sp = ivf.SearchParams(n_probes=9, lut_dtype=LUT[lut][0], internal_distance_dtype=LUT[internal][0])
+
+    def search():
+        d, i = ivf.search(sp, g, torch.from_numpy(q).cuda(), k, resources=res)
+        n = C.c_uint64(0)
+        L.check(lib.cuvsStreamSync(res.handle))
+        L.check(lib.cuvsB200CoarseTimeouts(res.handle, C.byref(n)))
+        assert_parity(d.cpu().numpy(), i.cpu().numpy(), do, io, 1e-5 if lut == "f32" else 1e-2)
+        return n.value
+
+    try:
+        L.check(lib.cuvsB200SetCoarseWaitTest(1000, 1))
+        assert search() == 1
+    finally:
+        L.check(lib.cuvsB200SetCoarseWaitTest(0, 0))
+    assert search() == 1

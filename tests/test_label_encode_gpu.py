@@ -85,3 +85,33 @@ def test_codes(ivf, bits, pq_dim, length, n):
     d = ((r[:, :, :, None].astype(np.float64) - books[None]) ** 2).sum(2)
     got = np.take_along_axis(d, codes[:, :, None], 2)[:, :, 0]
     assert (got <= d.min(2) * (1 + 1e-5) + 1e-9).all() and (codes == d.argmin(2)).mean() > 0.999
+
+
+# resident row tile with two products, with one, and row tile streamed beside the lists
+@pytest.mark.parametrize("n,dim,n_lists", [(20000, 62, 1000), (17000, 300, 1100), (17000, 768, 1100)])
+def test_a_wait_that_runs_out_redoes_every_label(ivf, n, dim, n_lists):
+    """One list block of every CTA's first tile never comes and the limit is about a millisecond: the labelling kernel gives
+    up, every row is labelled by the exact product, and the handle counts the call."""
+    import ctypes as C
+    from cuvs_b200 import _lib as L
+    from cuvs_b200.common import Resources
+    index, _, _, _ = model(ivf, dim, n_lists, 4, 8)
+    x = torch.from_numpy(make_mixture(n, dim, 40, 0.3, 5)).cuda()
+    lib, res = L.load(), Resources()
+
+    def labels():
+        out = ivf.transform(index, x, resources=res)[0]
+        m = C.c_uint64(0)
+        L.check(lib.cuvsStreamSync(res.handle))
+        L.check(lib.cuvsB200CoarseTimeouts(res.handle, C.byref(m)))
+        return out.to(torch.int64), m.value
+
+    healthy, m0 = labels()
+    try:
+        L.check(lib.cuvsB200SetCoarseWaitTest(1000, 1))
+        timed_out, m1 = labels()
+    finally:
+        L.check(lib.cuvsB200SetCoarseWaitTest(0, 0))
+    again, m2 = labels()
+    assert m0 == 0 and m1 >= 1 and m2 == m1
+    assert bool((healthy == timed_out).all()) and bool((healthy == again).all())
