@@ -556,7 +556,7 @@ __global__ void __launch_bounds__(1024, 1) rescore_kernel(const rescore_params p
         for (uint32_t u = 0; u < 4; u++) {
           // (negated: a NaN is taken; +inf stands for a pair without bounds)
           if (all || !(x[u] > vmax) || x[u] == INFINITY) {
-            const bool front    = x[u] <= vk;
+            const bool front    = !all && x[u] <= vk;  // (after a time-out the values are anything)
             const uint32_t slot = atomicAdd(&s.word[front ? W_FRONT : W_BACK], 1u);
             if (slot < p.list_cap) {
               s.list[front ? slot : p.list_cap - 1u - slot] = make_uint2((gi << 2) | u, __float_as_uint(x[u]));
