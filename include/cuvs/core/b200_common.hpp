@@ -41,6 +41,7 @@ struct error : public std::runtime_error {
   do {                                                                                       \
     cudaError_t e__ = (call);                                                                \
     if (e__ != cudaSuccess) {                                                                \
+      cudaGetLastError(); /* reported here: not to be found by the next call's check */      \
       ::cuvs_b200::fail("CUDA error %s at %s:%d: %s", cudaGetErrorName(e__), __FILE__,       \
                         __LINE__, cudaGetErrorString(e__));                                  \
     }                                                                                        \

@@ -131,3 +131,16 @@ def test_database_vectors_find_themselves(big):
     sp = ivf.SearchParams(n_probes=10, lut_dtype=np.float32)
     _, i = ivf.search(sp, big["index"], big["x"][rows].contiguous(), 5)
     assert ((i == rows.unsqueeze(1)).any(dim=1).float().mean().item()) >= 0.95
+
+
+def test_an_allocation_that_fails_is_reported_once(big):
+    """A workspace no GPU holds is refused; the same handle then searches as if nothing had been asked."""
+    from cuvs_b200._lib import CuvsError
+    from cuvs_b200.common import Resources
+    ivf, res = big["ivf"], Resources()
+    sp = ivf.SearchParams(n_probes=30)
+    d0, i0 = ivf.search(sp, big["index"], big["q"], K)
+    with pytest.raises(CuvsError, match="cudaErrorMemoryAllocation"):
+        res.set_workspace_pool(1 << 46)
+    d, i = ivf.search(sp, big["index"], big["q"], K, resources=res)
+    assert (i == i0).all() and (d == d0).all()
