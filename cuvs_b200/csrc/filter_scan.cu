@@ -640,8 +640,8 @@ make_tiles_kernel(uint32_t* __restrict__ list_count, const uint32_t* __restrict_
   }
 }
 
-// The query operand: sixteen lanes per (query, probe) pair.  `cursor` (optional): next place of every list's pairs,
-// which orders the pairs by list; without it a pair's place is its number.  A pair of an empty list has none.
+// The query operand: sixteen lanes per (query, probe) pair.  `cursor`: next place of every list's pairs, which orders the
+// pairs by list.  A pair of an empty list has none.
 // Row of the operand: L2 -2 (q - c) s, inner product -q s_q, in half precision, then 1, 1, mask, 0, 1, 1, 0, 0
 // against the row side's |r|^2 and mask.  Record: {factor, constant, first group of the pair's bounds, -}.
 __global__ void __launch_bounds__(256)
@@ -658,11 +658,9 @@ pair_operands_kernel(const operand_params p, const uint32_t* __restrict__ probes
   const uint32_t label = __ldg(probes + i);
   if (label >= n_lists || __ldg(list_sizes + label) == 0) { return; }
   const uint32_t q = i / n_probes, pi = i - q * n_probes;
-  uint32_t pos     = i;
-  if (cursor != nullptr) {
-    if (lane == 0) { pos = atomicAdd(cursor + label, 1u); }
-    pos = __shfl_sync(half_mask, pos, 0, 16);
-  }
+  uint32_t pos     = 0;
+  if (lane == 0) { pos = atomicAdd(cursor + label, 1u); }
+  pos = __shfl_sync(half_mask, pos, 0, 16);
   const float* qr = p.rot_q + size_t(q) * p.rot_dim;
   const float* cr = p.centers + size_t(label) * p.rot_dim;
   const float sq  = p.is_ip ? __ldg(p.q_scale + q) : p.scale;
@@ -744,57 +742,6 @@ pair_operands_kernel(const operand_params p, const uint32_t* __restrict__ probes
     }
     pair_rec[pos] = make_float4(mul, add, __uint_as_float(q * max_groups + (pi > 0 ? __ldg(group_index + i - 1) : 0u)), 0.0f);
     pair_norm[i]  = norm;
-  }
-}
-
-// A few queries: nothing is ordered by list.  One warp per query writes the offsets, and the groups of 32 of its probes
-// at a time form one stream that is cut into tiles (all 32 pairs are a tile's queries, each group counts for one).
-__global__ void small_tiles_kernel(const uint32_t* __restrict__ probes, const uint32_t* __restrict__ list_sizes,
-                                   const uint64_t* __restrict__ row_off, uint32_t n_lists, uint32_t n_queries,
-                                   uint32_t n_probes, uint32_t* __restrict__ chunk_index,
-                                   uint32_t* __restrict__ group_index, filter_tile* __restrict__ tiles,
-                                   uint32_t* __restrict__ counters)
-{
-  chain_begin();
-  const uint32_t q    = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const uint32_t lane = threadIdx.x & 31;
-  if (q >= n_queries) { return; }
-  uint32_t carry = 0, gcarry = 0;
-  for (uint32_t p0 = 0; p0 < n_probes; p0 += 32) {
-    const uint32_t p    = p0 + lane;
-    const uint32_t pair = q * n_probes + p;
-    uint32_t label = 0, size = 0;
-    if (p < n_probes) {
-      label = probes[pair];
-      size  = label < n_lists ? list_sizes[label] : 0u;
-    }
-    const uint32_t ng = (size + 31u) >> 5;
-    uint32_t v = size, g = ng;
-#pragma unroll
-    for (int d = 1; d < 32; d <<= 1) {
-      const uint32_t a = __shfl_up_sync(kFullMask, v, d), b = __shfl_up_sync(kFullMask, g, d);
-      if (lane >= uint32_t(d)) {
-        v += a;
-        g += b;
-      }
-    }
-    const uint32_t total = __shfl_sync(kFullMask, g, 31);
-    uint32_t tile0 = 0;
-    if (lane == 0 && total > 0) { tile0 = atomicAdd(counters + 1, (total + 7u) >> 3); }
-    tile0 = __shfl_sync(kFullMask, tile0, 0);
-    if (p < n_probes) {
-      chunk_index[pair] = carry + v;
-      group_index[pair] = gcarry + g;
-      const uint32_t arena = ng > 0 ? uint32_t(row_off[label] >> 5) : 0u;
-      for (uint32_t k = 0; k < ng; k++) {
-        const uint32_t y = g - ng + k;
-        uint4* t         = reinterpret_cast<uint4*>(tiles + tile0 + (y >> 3));
-        t[1 + (y & 7u)]  = make_uint4(arena + k, min(32u, size - k * 32u) | (lane << 8) | (1u << 16), k, 0u);
-        if ((y & 7u) == 0u) { t[0] = make_uint4(q * n_probes + p0, min(32u, n_probes - p0), min(8u, total - y), 0u); }
-      }
-    }
-    carry += __shfl_sync(kFullMask, v, 31);
-    gcarry += total;
   }
 }
 
@@ -916,14 +863,6 @@ void launch_tiles(const uint32_t* list_sizes, const uint64_t* row_off, uint32_t 
   CUDA_TRY(cudaGetLastError());
 }
 
-void launch_tiles_small(const uint32_t* probes, const uint32_t* list_sizes, const uint64_t* row_off, uint32_t n_lists,
-                        uint32_t n_queries, uint32_t n_probes, uint32_t* chunk_index, uint32_t* group_index,
-                        filter_tile* tiles, uint32_t* counters, cudaStream_t stream)
-{
-  launch_chained(small_tiles_kernel, ceildiv<uint32_t>(n_queries * 32, 128), 128, 0, stream, probes, list_sizes, row_off, n_lists, n_queries, n_probes, chunk_index, group_index, tiles, counters);
-  CUDA_TRY(cudaGetLastError());
-}
-
 void launch_pair_operands(const operand_params& p, const uint32_t* probes, const uint32_t* list_sizes, uint32_t n_lists,
                           const uint32_t* group_index, uint32_t n_pairs, uint32_t n_probes, uint32_t max_groups,
                           uint32_t* cursor, __half* operand, float4* pair_rec, float* pair_norm, cudaStream_t stream)
@@ -939,11 +878,10 @@ void launch_query_scale(const float* rot_q, uint32_t n_queries, uint32_t rot_dim
   CUDA_TRY(cudaGetLastError());
 }
 
-uint64_t max_filter_tiles(const index<int64_t>& idx, uint64_t n_pairs, bool small)
+uint64_t max_filter_tiles(const index<int64_t>& idx, uint64_t n_pairs)
 {
   // tiles of the longest list, the most that one more group of 128 queries can add
   const uint64_t longest = ceildiv<uint64_t>(uint64_t(idx.accum_sorted_sizes()[1]), kTileR);
-  if (small) { return n_pairs * longest; }
   // every list once (row tiles of the whole index), and the extra query groups
   const uint64_t all = uint64_t(idx.total_rows_padded()) / kTileR + idx.n_lists();
   return std::min<uint64_t>(n_pairs * longest, all + (n_pairs / kTileQ) * longest);

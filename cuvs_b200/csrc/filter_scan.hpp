@@ -63,7 +63,6 @@ struct rescore_params {
   const uint8_t* codes;
   const int64_t* ids;
   const uint64_t* row_off;
-  const uint32_t* list_sizes;
   const uint32_t* probes;       // [n_q, n_probes]
   const uint32_t* chunk_index;  // [n_q, n_probes] inclusive sums of list sizes
   const uint32_t* group_index;  // [n_q, n_probes] inclusive sums of 32-row groups
@@ -76,7 +75,7 @@ struct rescore_params {
   uint32_t n_lists, n_queries, n_probes, k, max_groups;
   uint32_t pq_dim, pq_len, pq_bits, rot_dim, n_pieces, book_size;
   // shared-memory plan; book_bytes 0: the codebook stays in global memory
-  uint32_t groups, group_threads, group_bytes, book_bytes, cap, list_cap, tops;
+  uint32_t groups, group_threads, group_bytes, book_bytes, cap, list_cap;
   int cosine, metric;
   float post_scale;
   // error model (see rescore.cu)
@@ -92,11 +91,11 @@ struct filter_plan {
   bool use = false;
   uint32_t n_stages = 0;
   size_t filter_smem = 0;
-  uint32_t groups = 0, group_threads = 0, group_bytes = 0, book_bytes = 0, cap = 0, list_cap = 0, tops = 0;
+  uint32_t groups = 0, group_threads = 0, group_bytes = 0, book_bytes = 0, cap = 0, list_cap = 0;
   size_t rescore_smem = 0;
 };
 
-// Whether (and with which shared-memory plan) a search runs on the two-step path.
+// Whether (and with which shared-memory plan) a search runs on the two-step path (k <= 128).
 filter_plan plan_filter(const raft::resources& res, const index<int64_t>& idx, int lut_kind, bool out_half, bool is_ip,
                         uint32_t k, uint32_t n_probes, uint32_t n_queries);
 
@@ -114,18 +113,14 @@ void launch_count_pairs(const uint32_t* probes, const uint32_t* list_sizes, uint
 // [1] tiles (zero on entry).
 void launch_tiles(const uint32_t* list_sizes, const uint64_t* row_off, uint32_t n_lists, uint32_t* list_count,
                   filter_tile* tiles, uint32_t* counters, cudaStream_t stream);
-// Tiles of a few queries without ordering by list: one pair per tile; writes the offsets too.
-void launch_tiles_small(const uint32_t* probes, const uint32_t* list_sizes, const uint64_t* row_off, uint32_t n_lists,
-                        uint32_t n_queries, uint32_t n_probes, uint32_t* chunk_index, uint32_t* group_index,
-                        filter_tile* tiles, uint32_t* counters, cudaStream_t stream);
-// The query operand of every pair, at the pair's place (`cursor`: ordered by list; null: by number), its record, and
+// The query operand of every pair, at the pair's place (`cursor`: the next one of every list), its record, and
 // pair_norm [n_q * n_probes]: |q - c| (L2; negative: flagged) or |c| (inner product).
 void launch_pair_operands(const operand_params& p, const uint32_t* probes, const uint32_t* list_sizes, uint32_t n_lists,
                           const uint32_t* group_index, uint32_t n_pairs, uint32_t n_probes, uint32_t max_groups,
                           uint32_t* cursor, __half* operand, float4* pair_rec, float* pair_norm, cudaStream_t stream);
 void launch_query_scale(const float* rot_q, uint32_t n_queries, uint32_t rot_dim, float* q_scale, cudaStream_t stream);
 // Upper bound on the number of tiles.
-uint64_t max_filter_tiles(const index<int64_t>& idx, uint64_t n_pairs, bool small);
+uint64_t max_filter_tiles(const index<int64_t>& idx, uint64_t n_pairs);
 
 // Half-precision codebooks: `out` [pq_dim][book][len_pad], stats[0] = sum over subspaces of the largest squared
 // codeword norm, stats[1] = largest |component|, both of the fp32 codebook; `scale_out` the power of two.

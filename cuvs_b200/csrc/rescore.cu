@@ -19,7 +19,7 @@
 // their rows are dropped there.
 //
 // What bounds it: gathers from the fp32 codebook (one 8-byte look-up per code for two dimensions per subspace);
-// it sits in shared memory once per CTA and thread groups of 32 to 1024 take one query at a time.
+// it sits in shared memory once per CTA and thread groups of 32 to 256 take one query at a time.
 #include "common.hpp"
 #include "filter_scan.hpp"
 #include "scan.cuh"
@@ -126,7 +126,8 @@ struct group_mem {
   uint32_t* label;   // [P]
   uint32_t* word;    // [8]
 };
-constexpr uint32_t kListPerThread = 4;  // list_cap <= kListPerThread * threads of a group
+constexpr uint32_t kListPerThread   = 4;    // list_cap = kListPerThread * threads of a group
+constexpr uint32_t kMaxGroupThreads = 256;  // threads per query
 enum { W_KEYS = 0, W_FRONT = 1, W_BACK = 2, W_BOUND = 3, W_VK = 4, W_VMAX = 5, W_NEXT = 6 };
 __host__ __device__ inline uint32_t group_mem_bytes(uint32_t cap, uint32_t list_cap, uint32_t n_probes, uint32_t rot_dim)
 {
@@ -345,23 +346,15 @@ __global__ void __launch_bounds__(1024, 1) rescore_kernel(const rescore_params p
     const uint32_t n_units4 = __ldg(p.group_index + size_t(q) * P + P - 1);
     const float4* units     = p.units + size_t(q) * p.max_groups;
 
-    // ---- V: the k-th smallest value of the units (every thread contributes its `tops` smallest) ----
-    float best[8];
-#pragma unroll
-    for (int i = 0; i < 8; i++) { best[i] = INFINITY; }
+    // ---- V: the k-th smallest value of the units (every thread contributes its two smallest) ----
+    float best[2] = {INFINITY, INFINITY};
     if (!all) {
       auto take = [&](const float4& v) {
         const float x[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
         for (int u = 0; u < 4; u++) {
-          if (p.tops == 2) {
-            best[1] = fminf(best[1], fmaxf(best[0], x[u]));
-            best[0] = fminf(best[0], x[u]);
-          } else if (x[u] < best[7]) {
-#pragma unroll
-            for (int i = 7; i > 0; i--) { best[i] = fminf(best[i], fmaxf(best[i - 1], x[u])); }
-            best[0] = fminf(best[0], x[u]);
-          }
+          best[1] = fminf(best[1], fmaxf(best[0], x[u]));
+          best[0] = fminf(best[0], x[u]);
         }
       };
       const float4 none = make_float4(INFINITY, INFINITY, INFINITY, INFINITY);
@@ -373,11 +366,9 @@ __global__ void __launch_bounds__(1024, 1) rescore_kernel(const rescore_params p
         for (uint32_t i = 0; i < 4; i++) { take(v[i]); }
       }
       if (gt > 32u) {
-        uint32_t* top = reinterpret_cast<uint32_t*>(s.buf);  // tops * gt <= 2 * cap words
-#pragma unroll
-        for (uint32_t i = 0; i < 8; i++) {
-          if (i < p.tops) { top[i * gt + t] = float_to_ordered(best[i]); }
-        }
+        uint32_t* top = reinterpret_cast<uint32_t*>(s.buf);  // 2 * gt <= 2 * cap words
+        top[t]        = float_to_ordered(best[0]);
+        top[gt + t]   = float_to_ordered(best[1]);
       }
     }
     sync();
@@ -390,9 +381,8 @@ __global__ void __launch_bounds__(1024, 1) rescore_kernel(const rescore_params p
         qn = sqrtf(qn) * 1.00001f;
       }
       // 22 bits of the k-th smallest, rounded up
-      const uint32_t n_top = p.tops * gt;
-      float vk             = INFINITY;
-      if (k <= n_top) {
+      float vk = INFINITY;
+      if (k <= 2u * gt) {
         uint32_t lo = 0;  // largest multiple of the step with fewer than k values below it
         auto bisect = [&](auto count) {
           for (int bit = 31; bit >= 10; bit--) {
@@ -402,30 +392,19 @@ __global__ void __launch_bounds__(1024, 1) rescore_kernel(const rescore_params p
         };
         if (gt == 32u) {
           bisect([&](uint32_t c) {
-            uint32_t n = 0;
-#pragma unroll
-            for (uint32_t i = 0; i < 8; i++) { n += float_to_ordered(best[i]) < c ? 1u : 0u; }  // beyond `tops`: +inf
-            return n;
+            return (float_to_ordered(best[0]) < c ? 1u : 0u) + (float_to_ordered(best[1]) < c ? 1u : 0u);
           });
         } else {
           const uint32_t* top = reinterpret_cast<const uint32_t*>(s.buf);
-          if (n_top <= 512u) {
-            uint32_t v[16];
+          uint32_t v[2 * kMaxGroupThreads / 32];
 #pragma unroll
-            for (uint32_t i = 0; i < 16; i++) { v[i] = i * 32u < n_top ? top[i * 32u + lane] : 0xFFFFFFFFu; }
-            bisect([&](uint32_t c) {
-              uint32_t n = 0;
+          for (uint32_t i = 0; i < 2 * kMaxGroupThreads / 32; i++) { v[i] = i * 16u < gt ? top[i * 32u + lane] : 0xFFFFFFFFu; }
+          bisect([&](uint32_t c) {
+            uint32_t n = 0;
 #pragma unroll
-              for (int i = 0; i < 16; i++) { n += v[i] < c ? 1u : 0u; }
-              return n;
-            });
-          } else {
-            bisect([&](uint32_t c) {
-              uint32_t n = 0;
-              for (uint32_t i = lane; i < n_top; i += 32) { n += top[i] < c ? 1u : 0u; }
-              return n;
-            });
-          }
+            for (uint32_t i = 0; i < 2 * kMaxGroupThreads / 32; i++) { n += v[i] < c ? 1u : 0u; }
+            return n;
+          });
         }
         vk = ordered_to_float(lo | 0x3FFu);
       }
@@ -725,7 +704,7 @@ filter_plan plan_filter(const raft::resources& res, const index<int64_t>& idx, i
   // (inner product with 8-bit tables or half-precision sums) cancel, so their rounding is not small against the
   // differences between scores.  Codebooks per list have no shared operand.
   if (idx.codebook_kind() != codebook_gen::PER_SUBSPACE || (is_ip && (lut_kind == LUT_FP8 || out_half))) { return plan; }
-  if (k > 1024) { return plan; }
+  if (k > 128) { return plan; }
   const size_t limit  = size_t(res.smem_optin) - 1024;
   const auto& m       = idx.filter_model();
   const size_t fixed  = m.book.size() * 2 + 256 + 1024;
@@ -738,20 +717,15 @@ filter_plan plan_filter(const raft::resources& res, const index<int64_t>& idx, i
   // Threads per query: enough that a thread sees at most about 16 groups of units and that keys and candidate rows
   // spread over the warps; more when there are too few queries to fill the chip.
   const uint64_t avg_groups = ceildiv<uint64_t>(uint64_t(idx.size()) * n_probes, uint64_t(idx.n_lists()) * 32) + n_probes / 2;
-  uint32_t gt = k <= 16 ? 32 : (k <= 64 ? 64 : (k <= 256 ? 128 : 512));
-  while (gt < 256 && avg_groups > 16ull * gt) { gt <<= 1; }
-  while (gt < 256 && uint64_t(n_queries) * gt < uint64_t(res.sm_count) * 1024) { gt <<= 1; }
+  uint32_t gt = k <= 16 ? 32 : (k <= 64 ? 64 : 128);
+  while (gt < kMaxGroupThreads && avg_groups > 16ull * gt) { gt <<= 1; }
+  while (gt < kMaxGroupThreads && uint64_t(n_queries) * gt < uint64_t(res.sm_count) * 1024) { gt <<= 1; }
   const size_t book = round_up<size_t>(idx.pq_centers_size() * 4, 16);
   const bool few    = n_queries <= uint32_t(res.sm_count);
-  plan.tops = 2;
-  if (2 * k > 2 * gt) { plan.tops = 8; }
-  if (k > plan.tops * gt) { return plan; }
   uint32_t cap = 128;
-  while (cap < 2 * k + gt || 2 * cap < plan.tops * gt) { cap <<= 1; }
+  while (cap < 2 * k + gt) { cap <<= 1; }
   plan.cap           = cap;
-  // (wide bounds re-list what a first round of exact scores leaves, a fixed number of units per thread)
-  const bool sharpen = lut_kind == LUT_FP8 || out_half;
-  plan.list_cap      = sharpen ? kListPerThread * gt : std::max(kListPerThread * gt, k > 128 ? 4 * round_up(k, 64u) / 2 : 0u);
+  plan.list_cap      = kListPerThread * gt;
   plan.group_threads = gt;
   plan.group_bytes   = group_mem_bytes(cap, plan.list_cap, n_probes, idx.rot_dim());
   // As many groups per CTA as threads and shared memory allow, beside the codebook in shared memory where that leaves at

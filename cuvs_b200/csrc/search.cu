@@ -891,7 +891,7 @@ void search_any(raft::resources& res, const search_params& params, const index<i
   // (a list-sharded search exchanges bounds in the middle of the look-up-table scan: a collective, so that all its ranks
   // take that path)
   const int home = scan_codebook_home();
-  if (!res.scan_phase_hook && (home == 4 || (home == 0 && !never && uint64_t(batch) * n_probes > enough && k <= 128))) {
+  if (!res.scan_phase_hook && !store_all && (home == 4 || (home == 0 && !never && uint64_t(batch) * n_probes > enough))) {
     fplan = plan_filter(res, idx, lut_kind, out_half, is_ip, k, n_probes, batch);
     // the bounds and the query operand of one internal batch: within 2 GiB each
     const uint64_t per_query = std::max(uint64_t(max_groups), uint64_t(n_probes) * f_chunks) * 16;
@@ -902,7 +902,7 @@ void search_any(raft::resources& res, const search_params& params, const index<i
       if (fplan.use) { batch = fits; }
     }
   }
-  if (store_all && !fplan.use) {
+  if (store_all) {
     // keep the score matrix of one internal batch within 1 GiB
     const uint64_t cap_q = std::max<uint64_t>(1, (1ull << 30) / (uint64_t(max_samples) * 4));
     batch                = uint32_t(std::min<uint64_t>(batch, cap_q));
@@ -923,8 +923,7 @@ void search_any(raft::resources& res, const search_params& params, const index<i
   const size_t o_probes  = lay.add(n_pairs_max * 4);
   const size_t o_chunk   = lay.add(n_pairs_max * 4);
   const bool f_use       = fplan.use;
-  const bool f_small     = n_pairs_max <= 4096 && !res.stats_enabled;  // every pair its own tile, nothing ordered by list
-  const size_t n_tiles   = f_use ? size_t(max_filter_tiles(idx, n_pairs_max, f_small)) : 0;
+  const size_t n_tiles   = f_use ? size_t(max_filter_tiles(idx, n_pairs_max)) : 0;
   const size_t o_groups  = lay.add(f_use ? n_pairs_max * 4 : 0);
   const size_t o_rec     = lay.add(f_use ? n_pairs_max * 16 : 0);
   const size_t o_norm    = lay.add(f_use ? n_pairs_max * 4 : 0);
@@ -937,7 +936,7 @@ void search_any(raft::resources& res, const search_params& params, const index<i
   const size_t o_kth     = lay.add(size_t(batch) * 4);
   const size_t o_counter = lay.add(256);
   const size_t o_keys    = lay.add(f_use ? 0 : (store_all ? size_t(batch) * k * 8 : n_pairs_max * k * 8));
-  const size_t o_all     = lay.add(store_all && !f_use ? size_t(batch) * max_samples * 4 : 0);
+  const size_t o_all     = lay.add(store_all ? size_t(batch) * max_samples * 4 : 0);
   // half-precision scores tie in large groups, which the tensor-core path's guard (made for fp32
   // scores) does not settle: the fp16 coarse search runs on the exact SIMT path
   const bool use_tc = !coarse_h && coarse_mode() != 1 && coarse_tc_usable(n_lists, n_probes, cdim_ext);
@@ -1020,21 +1019,15 @@ void search_any(raft::resources& res, const search_params& params, const index<i
       auto* d_qscale  = reinterpret_cast<float*>(ws + o_qscale);
       auto* d_operand = reinterpret_cast<__half*>(ws + o_operand);
       // 3. tiles, and the query operand of every pair, ordered by list; d_counter: pairs, tiles, error word
-      if (f_small) {
-        launch_tiles_small(d_probes, idx.list_sizes(), idx.row_offsets(), n_lists, nq, n_probes, d_chunk, d_groups, d_tiles,
-                           d_counter, stream);
-        res.launches++;
-      } else {
-        CUDA_TRY(cudaMemsetAsync(d_count, 0, size_t(n_lists) * 4, stream));
-        launch_count_pairs(d_probes, idx.list_sizes(), n_lists, nq, n_probes, d_chunk, d_groups, d_count, stream);
-        if (stats) {
-          scan_stats_kernel<<<ceildiv<uint32_t>(n_lists, 256), 256, 0, stream>>>(d_count, idx.list_sizes(), n_lists, 1,
-                                                                                 res.d_stats);
-          res.stat_pairs += n_pairs;
-        }
-        launch_tiles(idx.list_sizes(), idx.row_offsets(), n_lists, d_count, d_tiles, d_counter, stream);
-        res.launches += 2;
+      CUDA_TRY(cudaMemsetAsync(d_count, 0, size_t(n_lists) * 4, stream));
+      launch_count_pairs(d_probes, idx.list_sizes(), n_lists, nq, n_probes, d_chunk, d_groups, d_count, stream);
+      if (stats) {
+        scan_stats_kernel<<<ceildiv<uint32_t>(n_lists, 256), 256, 0, stream>>>(d_count, idx.list_sizes(), n_lists, 1,
+                                                                               res.d_stats);
+        res.stat_pairs += n_pairs;
       }
+      launch_tiles(idx.list_sizes(), idx.row_offsets(), n_lists, d_count, d_tiles, d_counter, stream);
+      res.launches += 2;
       if (is_ip) {
         launch_query_scale(d_rq, nq, idx.rot_dim(), d_qscale, stream);
         res.launches++;
@@ -1057,7 +1050,7 @@ void search_any(raft::resources& res, const search_params& params, const index<i
       op.entry_limit = lut_kind == LUT_F16 || out_half ? 6.0e4f : (lut_kind == LUT_FP8 ? 1.2e5f : INFINITY);
       op.rcomp_max   = fm.comp_max;
       launch_pair_operands(op, d_probes, idx.list_sizes(), n_lists, d_groups, n_pairs, n_probes, max_groups,
-                           f_small ? nullptr : d_count, d_operand, d_rec, d_norm, stream);
+                           d_count, d_operand, d_rec, d_norm, stream);
       res.launches++;
       if (stats) { res.stats_mark(ev, 3); }
       // 4. bounds
@@ -1096,7 +1089,6 @@ void search_any(raft::resources& res, const search_params& params, const index<i
       rp.codes        = idx.codes();
       rp.ids          = idx.ids();
       rp.row_off      = idx.row_offsets();
-      rp.list_sizes   = idx.list_sizes();
       rp.probes       = d_probes;
       rp.chunk_index  = d_chunk;
       rp.group_index  = d_groups;
@@ -1123,7 +1115,6 @@ void search_any(raft::resources& res, const search_params& params, const index<i
       rp.group_bytes  = fplan.group_bytes;
       rp.book_bytes   = fplan.book_bytes;
       rp.cap          = fplan.cap;
-      rp.tops         = fplan.tops;
       rp.claim        = d_counter + 3;
       rp.cosine       = cosine;
       rp.metric       = int(metric);

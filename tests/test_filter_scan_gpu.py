@@ -45,6 +45,7 @@ def test_code_widths_and_lengths(ivf, oracle_mod, tmp_path, bits, dim, pq_dim, m
 
 @pytest.mark.parametrize("metric,lut,internal", [(0, "f32", "f32"), (1, "f16", "f32"), (0, "fp8", "f32"), (0, "f16", "f16"),
                                                  (0, "fp8", "f16"), (2, "f32", "f32"), (2, "f16", "f32"), (6, "f16", "f32")])
+# (k > 128 takes the look-up tables, forced or not)
 @pytest.mark.parametrize("k", [1, 16, 17, 64, 65, 100, 128, 300])
 def test_k_and_types(ivf, oracle_mod, tmp_path, metric, lut, internal, k):
     x, q, ix, path = build_case(oracle_mod, tmp_path, "k", n=4000, dim=48, n_lists=16, pq_dim=24, metric=metric, nq=24)
