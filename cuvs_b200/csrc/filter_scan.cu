@@ -542,7 +542,10 @@ __global__ void count_pairs_kernel(const uint32_t* __restrict__ probes, const ui
 // lists' pairs still fit a tile).  A list with more pairs has tiles of its own, its queries dealt evenly over
 // tiles of at most 128.  The block's pairs are ordered accordingly: first the sharing lists'.
 constexpr uint32_t kPackPairs   = kTileQ / 8;
-// (64 lists per block; 16 where 64 would leave SMs without one: 111 us against 50 us for 4,000 lists of 1,000 rows)
+// 64 lists per block share tiles better, 16 give more blocks: 16 below 32,768 lists.  A whole call of 10,000 queries x 20
+// probes over 3 M rows, 16 / 64 lists per block (us): 1,000 lists 1,029 / 1,073, 4,000 642 / 649, 9,000 684 / 685, 16,000
+// 771 / 772, 24,000 711 / 707, 32,000 766 / 762, 50,000 920 / 912.  (The kernel alone, 4,000 lists of 1,000 rows and 64
+// probes: 50 / 111.)
 template <uint32_t kListsPerBlock>
 __global__ void __launch_bounds__(256)
 make_tiles_kernel(uint32_t* __restrict__ list_count, const uint32_t* __restrict__ list_sizes,

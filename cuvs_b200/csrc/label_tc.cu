@@ -11,12 +11,14 @@
 //      columns carry |c|^2 / 2 - m.c + |m|^2 / 2, so that the accumulator holds F (score + a constant of the row), F = 2^e /
 //      cp, within (-0.5, 0.5).  `eps` of a row bounds how far that is from the exact value: the measured norms of what
 //      rounding took from row and lists, accumulation, the defining chain's own rounding, the rounding of the keys.
-//      Where the epilogue is the longer part (up to 190 dimensions) the row operand comes as two halfs, hi + lo, and two
-//      products: its rounding drops out of eps at no cost in time.
+//      Up to 190 dimensions (where both fit shared memory beside three list stages) the row operand comes as two halfs, hi +
+//      lo, and two products: its rounding drops out of eps.  The second product is on the critical path: at 96 dimensions the
+//      MMA thread issues the 14 products of a tile in about 3,400 clocks, the epilogue needs 2,200.
 //   2. label_tc_kernel: a persistent CTA takes a tile of 128 rows against all (or a share) of the lists, 256 at a time.
 //      Per row and unit of 64 lists the epilogue finds the largest value as a packed key (value in fixed point, low bits
 //      the column: see coarse_tc.cu) and the second largest; across the tiles it keeps, per row and column quarter, the
-//      units with the four largest.  Three float additions and three min / max per value, which bound the kernel.
+//      units with the four largest.  Three float additions and three min / max per value; the issue of the MMAs bounds the
+//      kernel.
 //   3. label_finish_kernel: units within 2 eps of the largest value are looked at.  One such unit whose second value is
 //      outside: that is the label.  Several: their lists are rescored with the defining chain.  Units whose second value
 //      is inside too go to label_units_kernel, which rescores all 64 lists of them.  If the fourth unit kept is inside,

@@ -876,13 +876,23 @@ void search_any(raft::resources& res, const search_params& params, const index<i
   const uint32_t f_data     = ceildiv(idx.pq_dim() * idx.filter_model().len_pad, 8u);
   const uint32_t f_chunks   = round_up(f_data + 1u, 2u);  // 16-byte chunks of a row of the query operand
   const uint32_t max_groups = uint32_t(ceildiv<uint64_t>(uint64_t(idx.accum_sorted_sizes()[n_probes]) + 31ull * n_probes, 32));
-  // Below some 4,000 pairs, and for k > 128, the look-up-table scan is as fast or faster: 162 against 178 us for 100
-  // queries of 20 probes, 632 against 754 us for 500 queries with k = 1000.  Where exact scores cost more it takes more
-  // pairs to win: 8-bit tables and half sums (wide bounds: 65 queries of 128 probes 296 against 342 us), and codes that
-  // the general loop scores (5 or 6 bits, or other lengths: 10,530 pairs 293 against 449 us, 28,034 pairs 544 against
-  // 278).  8-bit tables over other than 8-bit codes never do (64,065 pairs 1,022 against 2,977 us), half sums over codes of
-  // the general loop where a query has many probes for its k (777 queries, 40 probes, k 10: 288 against 255 us; 4,216
-  // queries, 10 probes, k 50: 624 against 748).
+  // Which path: lines on the number of pairs, measured on both sides (look-up tables / two steps in us, or the ratio of the
+  // two; about 1 M rows of 64 to 768 dimensions, fp32, half and 8-bit ones, in lists of 120 to 1,000 rows).
+  // - Codes with straight-line exact scores: from 4,096 pairs on, where small k breaks even (k 10, half-precision tables: 5,000
+  //   pairs 102 / 112, 8,000 120 / 126, 12,000 139 / 130; fp32 tables 5,000 116 / 112) and k 100 has long won (2,500 pairs
+  //   248 / 184).
+  // - Codes of the general loop (5 to 7 bits, other lengths): from 16,384 on, again where small k breaks even (64 x 6 bits, k
+  //   10: 12,000 pairs 145 / 163, 17,000 174 / 172, 40,000 302 / 225; k 100 wins from 5,000: 270 / 229).
+  // - Wide bounds (8-bit tables, half sums) leave more rows to the exact scores: from 16,384 on.  The line is on the safe side
+  //   for 8-bit straight-line codes (8-bit table, k 10: 8,310 pairs of 15 probes 233 / 165) and needed by the others (8-bit
+  //   codes of length 3: 12,000 pairs of 15 probes 254 / 309, 17,000 325 / 329).
+  // - Never: 8-bit tables over codes that are not straight-line 8-bit ones, because with few probes the exact scores cost more
+  //   than the tables however many the pairs (64,000 pairs of 15 probes, 64 x 6 bits: 713 / 862 at k 10, 1,232 / 1,717 at k
+  //   100; ratios 0.5 to 1.6).  And half sums over codes of the general loop where a query has few probes for its k (n_probes
+  //   < 2 k), which loses on some shapes (64,000 pairs of 15 probes, 64 x 6 bits, k 50: 801 / 1,048) and gains on more (ratios
+  //   0.7 to 2.9).  Both refusals are on the safe side: queries of 40 probes would mostly gain (ratios 0.8 to 4.4), those of
+  //   128 always (1.8 to 9.8).
+  // k > 128 takes the tables (500 queries with k 1000: 634, and 754 for two steps with eight values kept per thread).
   const bool wide_bounds = lut_kind == LUT_FP8 || out_half;
   const bool straight    = idx.rot_dim() % 4 == 0 && ((idx.pq_bits() == 8 && (idx.pq_len() == 2 || idx.pq_len() == 4)) ||
                                                    (idx.pq_bits() == 4 && idx.pq_len() == 2));
