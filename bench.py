@@ -14,13 +14,14 @@ stand in for them.
 A step = one search of the whole query batch.  `value` is queries/s with queries resident in HBM;
 `e2e` is the same through the C interface with pinned host buffers and the copies inside the timed
 region.  Times come from CUDA events on the stream the library launches on (torch's current
-stream); the code-scan kernel is timed by the library's own events around its launch.  `parity`
+stream); the kernels of the fine search are timed by the library's own events around their launches.  `parity`
 compares, id for id, what the GPU search returned for the CPU leg's sample of queries with what the
 CPU oracle returned for them; with several GPUs `mg_parity` compares the merged result with the
 single-GPU result of the same index.
 
---impl reference times the CPU oracle (the port of the reference search arithmetic, all host
-threads) on a bounded sample of the same queries against the same index.
+`cpu_baseline` is the CPU oracle (the port of the reference search arithmetic, all host threads) on a
+bounded sample of the same queries against the same index.  --impl reference reports that the
+reference itself cannot be built offline.
 """
 from __future__ import annotations
 
@@ -406,12 +407,40 @@ def hbm_peak():
     return FALLBACK_HBM_GBS, "fallback"
 
 
-# DRAM bytes (read + write) per DISTINCT 32-row group scanned in a launch, from the ncu capture of the
-# scan kernel on a 4 M-row case of this workload (312.3 MB over 134,482 distinct groups of
-# 3 x 512 B: the work list makes two passes over the lists, so a list can be fetched twice).  Traffic
+# DRAM bytes (read + write) of the bounding kernel per DISTINCT 32-row group of a launch, from an ncu
+# capture on a 2 M-row case of this workload (129.8 MB over 67,421 distinct groups of 3 x 512 B).  Traffic
 # grows with the distinct groups of a launch, so the full-size figure is this constant times the
 # launch's distinct groups.
-DRAM_BYTES_PER_UNIQUE_GROUP = 2322.0
+DRAM_BYTES_PER_UNIQUE_GROUP = 1926.0
+
+
+def fine_search_record(stats, wl, two_steps, peak):
+    """Roofline figures of the kernel that goes over the probed lists, from the library's counters.
+
+    Two steps (large batches): `filter_kernel` decodes every probed list once for up to 128 queries, so its bytes
+    are the codes of the distinct lists, one operand row per (query, list) pair and four bounds per pair and
+    32-row group; `rescore_kernel` then scores exactly what the bounds leave.  Tables: `scan_kernel` goes over the
+    codes of every pair.  `pair_scan`: the codes of every pair's list (what scanning each pair on its own would
+    read) over the time of the whole fine search, to compare the two and several GPUs; a list that many queries
+    share makes it exceed the peak."""
+    nb = max(1, stats.batches)
+    scan_ms, merge_ms = stats.scan_ms / nb, stats.merge_ms / nb
+    group = -(-wl["pq_dim"] // (128 // wl["pq_bits"])) * 512
+    pair_bytes, unique_bytes = stats.scan_groups / nb * group, stats.unique_groups / nb * group
+    algo, kernel = pair_bytes, "scan_kernel (LUT build + code scan + top-k)"
+    if two_steps:
+        length = wl["dim"] // wl["pq_dim"]          # 2 in every workload: no padding in the operand
+        chunks = -(-(wl["pq_dim"] * length // 8 + 1) // 2) * 2
+        algo = unique_bytes + stats.pairs / nb * chunks * 16 + stats.scan_groups / nb * 16
+        kernel = "filter_kernel (tensor-core bounds of every row of the probed lists)"
+    ms = scan_ms + (merge_ms if two_steps else 0.0)
+    rate = lambda b, t: round(b / (t * 1e-3) / 1e9, 1) if t > 0 else None  # noqa: E731
+    ach = rate(algo, scan_ms)
+    return {"bound": "hbm", "kernel": kernel, "achieved": ach, "peak": peak, "unit": "GB/s",
+            "frac": round(ach / peak, 4) if ach else None, "kernel_ms": round(scan_ms, 4),
+            "algorithmic_bytes_per_launch": int(algo), "unique_bytes_per_launch": int(unique_bytes),
+            "pair_scan": {"bytes": int(pair_bytes), "ms": round(ms, 4), "rate": rate(pair_bytes, ms), "unit": "GB/s",
+                          "kernels": "filter_kernel + rescore_kernel" if two_steps else "scan_kernel"}}
 
 
 def workload_from_args(args):
@@ -434,7 +463,7 @@ def workload_from_args(args):
 
 
 def long_list_record(res, device, peak, steps):
-    """The scan kernel on long lists: a 4 M-row slice of configuration 3 (lists of about 1,000 rows,
+    """The fine search on long lists: a 4 M-row slice of configuration 3 (lists of about 1,000 rows,
     8-bit look-up table, k = 100, n_probes 64), its own roofline figures."""
     import ctypes as C
 
@@ -459,19 +488,12 @@ def long_list_record(res, device, peak, steps):
     L.check(lib.cuvsB200StatsGet(res.handle, C.byref(stats), True))
     L.check(lib.cuvsB200StatsEnable(res.handle, False))
     b = max(1, stats.batches)
-    n_pieces = -(-wl["pq_dim"] // (128 // wl["pq_bits"]))
-    scan_ms = stats.scan_ms / b
-    algo = stats.scan_groups / b * n_pieces * 512
-    ach = algo / (scan_ms * 1e-3) / 1e9
     del index
     torch.cuda.empty_cache()
     return {"workload": wl["name"], "n_lists": wl["n_lists"], "n_probes": p, "k": k, "lut_dtype": "uint8",
             "recall_at_k": round(rec, 4), "ms_per_batch": round(sum(getattr(stats, f) for f in
                                                                     ("prep_ms", "coarse_ms", "sort_ms", "scan_ms", "merge_ms")) / b, 4),
-            "roofline": {"bound": "hbm", "kernel": "scan_kernel", "achieved": round(ach, 1), "peak": peak,
-                         "unit": "GB/s", "frac": round(ach / peak, 4), "kernel_ms": round(scan_ms, 4),
-                         "algorithmic_bytes_per_launch": int(algo),
-                         "unique_bytes_per_launch": int(stats.unique_groups / b * n_pieces * 512)}}
+            "roofline": fine_search_record(stats, wl, True, peak)}
 
 
 def run_ours(args):
@@ -634,11 +656,14 @@ def run_ours(args):
     nb = max(1, stats.batches)
     scan_ms = stats.scan_ms / nb
     n_pieces = -(-wl["pq_dim"] // (128 // wl["pq_bits"]))
-    bytes_scan = stats.scan_groups / nb * n_pieces * 512
-    bytes_unique = stats.unique_groups / nb * n_pieces * 512
     unique_groups = stats.unique_groups / nb
+    # which kernels a batch takes (every workload here has straight-line codes): see the library's dispatch
+    two_steps = comm is None and nq * p_star > 16384 and k0 <= 128
+    peak, peak_kind = hbm_peak()
+    roofline = fine_search_record(stats, wl, two_steps, peak)
     if comm is None:
-        stage = {k2: round(getattr(stats, k2) / nb, 4)
+        names = {"scan_ms": "bounds_ms", "merge_ms": "exact_scores_ms"} if two_steps else {}
+        stage = {names.get(k2, k2): round(getattr(stats, k2) / nb, 4)
                  for k2 in ("prep_ms", "coarse_ms", "sort_ms", "scan_ms", "merge_ms")}
     else:
         # the one-call step of a rank: its own five stages; the scan stage contains the fine search
@@ -789,9 +814,7 @@ def run_ours(args):
             dist.destroy_process_group()
         return
 
-    peak, peak_kind = hbm_peak()
-    achieved = bytes_scan / (scan_ms * 1e-3) / 1e9 if scan_ms > 0 else None
-    traffic = int(DRAM_BYTES_PER_UNIQUE_GROUP * unique_groups) if wl["gen"] == "deep" else None
+    traffic = int(DRAM_BYTES_PER_UNIQUE_GROUP * unique_groups) if wl["gen"] == "deep" and two_steps else None
     config = {"workload": wl["name"], "n_rows": wl["n_rows"], "dim": wl["dim"],
               "n_lists": wl["n_lists"], "pq_dim": wl["pq_dim"], "pq_bits": wl["pq_bits"], "metric": metric,
               "k": k, "recall_k": k, "batch": nq, "n_probes": p_star, "lut_dtype": wl["lut"],
@@ -825,13 +848,7 @@ def run_ours(args):
                 rkey: round(e2e_rec, 4)},
         "gpu_launches": gpu_launches,
         "clocks": clocks,
-        "roofline": {"bound": "hbm", "kernel": "scan_kernel (LUT build + code scan + top-k)",
-                     "achieved": round(achieved, 1) if achieved else None, "peak": peak,
-                     "peak_kind": f"of {peak_kind}", "unit": "GB/s",
-                     "frac": round(achieved / peak, 4) if achieved else None,
-                     "traffic": traffic, "algorithmic_bytes_per_launch": int(bytes_scan),
-                     "unique_bytes_per_launch": int(bytes_unique),
-                     "kernel_ms": round(scan_ms, 4)},
+        "roofline": dict(roofline, peak_kind=f"of {peak_kind}", traffic=traffic),
     }
     if mg_parity is not None:
         line["mg_parity"] = mg_parity
@@ -871,58 +888,12 @@ def run_ours(args):
 
 
 def run_reference(args):
-    """The reference arm: the CPU port of the reference search on the host cores."""
-    rank = int(os.environ.get("RANK", "0"))
-    if rank != 0:
-        return
-    wl = workload_from_args(args)
-    import torch
-    if not torch.cuda.is_available():
+    """The reference arm would time the reference's own build.  There is none: see the line it prints."""
+    if int(os.environ.get("RANK", "0")) == 0:
         emit({"impl": "reference",
-              "unavailable": "the index fixture is built on the GPU; no GPU here"})
-        return
-    torch.cuda.set_device(0)
-    k = wl["k"]
-    k0 = k0_of(wl)
-    fx = prepare_fixture(wl, torch.device("cuda", 0), need_dataset=k0 > k)
-    if os.path.getsize(fx["index_path"]) / 1e9 > 3.0:
-        emit({"impl": "reference",
-              "unavailable": "the CPU port loads the index through Python; this configuration's index is too large for that"})
-        return
-    # operating point: the same rule as the GPU arm, evaluated with the GPU search (fixture work)
-    from cuvs_b200 import ivf_pq, refine
-    index = ivf_pq.load(fx["index_path"])
-    recs = []
-    for p in wl["probes"]:
-        d, i = ivf_pq.search(ivf_pq.SearchParams(n_probes=p, lut_dtype=lut_np(wl),
-                                                 max_internal_batch_size=fx["queries"].shape[0]),
-                             index, fx["queries"], k0)
-        if k0 > k:
-            d, i = refine(fx["dataset"], fx["queries"], i, k=k, metric=wl["metric"])
-        recs.append((p, recall_at_k(i, fx["truth"])))
-    ok = [p for p, r in recs if r >= 0.95]
-    best = max(r for _, r in recs)
-    p_star = ok[0] if ok else [p for p, r in recs if r >= best - 0.005][0]
-    del index
-    dataset_np = fx["dataset"].cpu().numpy() if k0 > k else None
-    fx.pop("dataset", None)
-    torch.cuda.empty_cache()
-    cb, dt, n, _ = cpu_baseline(fx["index_path"], fx["queries"].cpu().numpy(), wl, p_star,
-                                budget_s=8.0, steps=args.steps, warmup=args.warmup, dataset_np=dataset_np)
-    line = {"impl": "reference", "metric": METRIC, "value": round(cb["value"], 1), "unit": "queries/s",
-            "n_gpus": int(os.environ.get("WORLD_SIZE", "1")), "steps": args.steps, "warmup": args.warmup,
-            "ms_per_step": round(dt * 1e3, 3), "higher_is_better": True, "scaling": "strong",
-            "vs_baseline": None, "dtype": "f32", "data": "synthetic",
-            "config": {"workload": wl["name"], "n_rows": wl["n_rows"], "dim": wl["dim"],
-                       "n_lists": wl["n_lists"], "pq_dim": wl["pq_dim"], "pq_bits": wl["pq_bits"],
-                       "metric": wl["metric"], "k": wl["k"], "batch": n, "n_probes": p_star,
-                       "lut_dtype": wl["lut"], "internal_distance_dtype": wl["internal"],
-                       "refine_ratio": wl["refine_ratio"]},
-            "cpu_baseline": dict(cb, value=round(cb["value"], 1)),
-            "e2e": {"value": round(cb["value"], 1), "unit": "queries/s", "h2d_bytes_per_step": 0,
-                    "d2h_bytes_per_step": 0},
-            "gpu_launches": 0}
-    emit(line)
+              "unavailable": "the reference needs RAFT, RMM and other RAPIDS sources that are not available offline: it "
+                             "cannot be built or installed here (its arithmetic restated for the host cores is timed as "
+                             "cpu_baseline of the other arm)"})
 
 
 def emit(line: dict):

@@ -884,8 +884,8 @@ void search_any(raft::resources& res, const search_params& params, const index<i
   // - Codes of the general loop (5 to 7 bits, other lengths): from 16,384 on, again where small k breaks even (64 x 6 bits, k
   //   10: 12,000 pairs 145 / 163, 17,000 174 / 172, 40,000 302 / 225; k 100 wins from 5,000: 270 / 229).
   // - Wide bounds (8-bit tables, half sums) leave more rows to the exact scores: from 16,384 on.  The line is on the safe side
-  //   for 8-bit straight-line codes (8-bit table, k 10: 8,310 pairs of 15 probes 233 / 165) and needed by the others (8-bit
-  //   codes of length 3: 12,000 pairs of 15 probes 254 / 309, 17,000 325 / 329).
+  //   for 8-bit straight-line codes (8-bit table, k 10: 8,310 pairs of 15 probes 233 / 165) and needed by half sums over codes
+  //   of the general loop (64 x 6 bits, 40 probes, k 10: 12,000 pairs 145 / 163, 17,000 175 / 174).
   // - Never: 8-bit tables over codes that are not straight-line 8-bit ones, because with few probes the exact scores cost more
   //   than the tables however many the pairs (64,000 pairs of 15 probes, 64 x 6 bits: 713 / 862 at k 10, 1,232 / 1,717 at k
   //   100; ratios 0.5 to 1.6).  And half sums over codes of the general loop where a query has few probes for its k (n_probes

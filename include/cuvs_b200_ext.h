@@ -18,9 +18,11 @@ typedef struct {
   double prep_ms;    /* query cast / pad / rotate */
   double coarse_ms;  /* probe selection */
   double sort_ms;    /* sample offsets + ordering of (query, probe) pairs by list */
-  double scan_ms;    /* look-up table build + code scan + per-pair top-k (one kernel per batch) */
-  double merge_ms;   /* final selection, id translation, distance post-processing */
-  uint64_t batches;        /* internal batches = launches of the scan kernel */
+  double scan_ms;    /* look-up table build + code scan + per-pair top-k (one kernel per batch); large batches: the
+                      * tensor-core bounds of the rows of the probed lists (one kernel) */
+  double merge_ms;   /* final selection, id translation, distance post-processing; large batches: exact scores of the
+                      * rows that the bounds leave, as well (one kernel) */
+  uint64_t batches;        /* internal batches = launches of the scan kernel, or of the two that replace it */
   uint64_t pairs;          /* (query, probe) pairs scanned */
   uint64_t scan_groups;    /* sum over pairs of ceil(list size / 32) */
   uint64_t unique_groups;  /* sum over distinct probed lists, per batch, of ceil(list size / 32) */
