@@ -128,6 +128,9 @@ struct group_mem {
 };
 constexpr uint32_t kListPerThread   = 4;    // list_cap = kListPerThread * threads of a group
 constexpr uint32_t kMaxGroupThreads = 256;  // threads per query
+// No bound: every score is kept but NaN (its bits order as 0xFFFFFFFF), which is no result, as in the scan (scan.cuh).  As a
+// float a NaN itself, which nothing exceeds.
+constexpr uint32_t kNoBound = 0xFFFFFFFEu;
 enum { W_KEYS = 0, W_FRONT = 1, W_BACK = 2, W_BOUND = 3, W_VK = 4, W_VMAX = 5, W_NEXT = 6 };
 __host__ __device__ inline uint32_t group_mem_bytes(uint32_t cap, uint32_t list_cap, uint32_t n_probes, uint32_t rot_dim)
 {
@@ -339,7 +342,7 @@ __global__ void __launch_bounds__(1024, 1) rescore_kernel(const rescore_params p
       s.word[W_KEYS]  = 0;
       s.word[W_FRONT] = 0;
       s.word[W_BACK]  = 0;
-      s.word[W_BOUND] = 0xFFFFFFFFu;
+      s.word[W_BOUND] = kNoBound;
       s.word[W_VK]    = __float_as_uint(-INFINITY);
       s.word[W_VMAX]  = __float_as_uint(INFINITY);
     }

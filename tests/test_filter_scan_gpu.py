@@ -161,3 +161,29 @@ def test_a_wait_that_runs_out_scores_every_row(ivf, oracle_mod, tmp_path, lut, i
     finally:
         L.check(lib.cuvsB200SetCoarseWaitTest(0, 0))
     assert search() == 1
+
+
+def odd_queries(q):
+    """NaN, infinities, zeros, and values at the ends of the ranges of fp32, half precision and the 8-bit float."""
+    q = q.copy()
+    q[0, 3], q[1], q[2, 5], q[3], q[4] = np.nan, np.nan, np.inf, -np.inf, 0.0
+    q[5], q[6, 0], q[8], q[9, 1], q[10], q[11], q[12] = 1e30, -1e30, 1e4, 3e4, 1e19, 3e18, 300.0
+    q[7] *= 1e-7
+    return q
+
+
+@pytest.mark.parametrize("metric,bits,dim,pq_dim", [(0, 8, 64, 32), (1, 8, 64, 64), (0, 6, 48, 24), (2, 8, 40, 24), (6, 8, 64, 32),
+                                                    (6, 4, 64, 32)])
+@pytest.mark.parametrize("lut,internal", [("f32", "f32"), ("f16", "f32"), ("f16", "f16"), ("fp8", "f16")])
+def test_odd_queries_answer_as_with_tables(ivf, oracle_mod, tmp_path, metric, bits, dim, pq_dim, lut, internal):
+    from cuvs_b200 import _lib as L
+    x, q, _, path = build_case(oracle_mod, tmp_path, "o", n=2500, dim=dim, n_lists=16, pq_dim=pq_dim, pq_bits=bits, metric=metric,
+                               nq=80)
+    g, q = ivf.load(path), odd_queries(q)
+    for k in (1, 10, 100):
+        d2, i2 = gpu_search(ivf, g, q, k, 7, lut, internal)
+        L.check(L.load().cuvsB200SetScanCodebookHome(2))
+        d0, i0 = gpu_search(ivf, g, q, k, 7, lut, internal)
+        L.check(L.load().cuvsB200SetScanCodebookHome(4))
+        assert (i0 == i2).all(), np.nonzero((i0 != i2).any(1))[0]
+        assert (d0.view(np.uint32) == d2.view(np.uint32)).all(), np.nonzero((d0.view(np.uint32) != d2.view(np.uint32)).any(1))[0]
