@@ -174,7 +174,7 @@ def odd_queries(q):
 
 @pytest.mark.parametrize("metric,bits,dim,pq_dim", [(0, 8, 64, 32), (1, 8, 64, 64), (0, 6, 48, 24), (2, 8, 40, 24), (6, 8, 64, 32),
                                                     (6, 4, 64, 32)])
-@pytest.mark.parametrize("lut,internal", [("f32", "f32"), ("f16", "f32"), ("f16", "f16"), ("fp8", "f16")])
+@pytest.mark.parametrize("lut,internal", [("f32", "f32"), ("f16", "f32"), ("fp8", "f32"), ("f16", "f16"), ("fp8", "f16")])
 def test_odd_queries_answer_as_with_tables(ivf, oracle_mod, tmp_path, metric, bits, dim, pq_dim, lut, internal):
     from cuvs_b200 import _lib as L
     x, q, _, path = build_case(oracle_mod, tmp_path, "o", n=2500, dim=dim, n_lists=16, pq_dim=pq_dim, pq_bits=bits, metric=metric,
