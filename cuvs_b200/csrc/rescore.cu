@@ -50,6 +50,9 @@ __device__ __forceinline__ float min3(float a, float b, float c)
   return d;
 }
 
+// Bound of a query's norm from its square; below 1e-15 squares may have underflowed and products may: no bounds then.
+__device__ __forceinline__ float query_norm(float square) { return square >= 1e-30f ? sqrtf(square) * 1.00001f : INFINITY; }
+
 // lo of a unit's value v in a pair with norm `norm` (a NaN compares as "cannot be ruled out").
 template <bool kIP>
 __device__ __forceinline__ float unit_lo(const rescore_params& p, float v, float norm, float qn)
@@ -384,7 +387,7 @@ __global__ void __launch_bounds__(1024, 1) rescore_kernel(const rescore_params p
         for (uint32_t i = lane; i < p.rot_dim; i += 32) { qn = __fmaf_rn(s.rq[i], s.rq[i], qn); }
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) { qn += __shfl_xor_sync(kFullMask, qn, o); }
-        qn = sqrtf(qn) * 1.00001f;
+        qn = query_norm(qn);
       }
       // 22 bits of the k-th smallest, rounded up
       float vk = INFINITY;
@@ -443,7 +446,7 @@ __global__ void __launch_bounds__(1024, 1) rescore_kernel(const rescore_params p
         for (uint32_t i = lane; i < p.rot_dim; i += 32) { qn = __fmaf_rn(s.rq[i], s.rq[i], qn); }
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) { qn += __shfl_xor_sync(kFullMask, qn, o); }
-        qn = sqrtf(qn) * 1.00001f;
+        qn = query_norm(qn);
       }
     }
     // 8-bit tables: does the query hold a NaN?  (A select on every entry, or such rows scored by a function of their own, cost
@@ -722,6 +725,10 @@ filter_plan plan_filter(const raft::resources& res, const index<int64_t>& idx, i
   // (inner product with 8-bit tables or half-precision sums) cancel, so their rounding is not small against the
   // differences between scores.  Codebooks per list have no shared operand.
   if (idx.codebook_kind() != codebook_gen::PER_SUBSPACE || (is_ip && (lut_kind == LUT_FP8 || out_half))) { return plan; }
+  // The error model counts rounding relative to the terms: codewords whose squares, or products with them, may underflow or
+  // overflow fp32 are left to the look-up tables.
+  const float rmax = idx.filter_model().rmax;
+  if (idx.filter_model().comp_max != 0.0f && !(rmax >= 1e-15f && rmax <= 1e15f)) { return plan; }
   if (k > 128) { return plan; }
   const size_t limit  = size_t(res.smem_optin) - 1024;
   const auto& m       = idx.filter_model();

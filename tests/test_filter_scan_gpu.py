@@ -187,3 +187,24 @@ def test_odd_queries_answer_as_with_tables(ivf, oracle_mod, tmp_path, metric, bi
         L.check(L.load().cuvsB200SetScanCodebookHome(4))
         assert (i0 == i2).all(), np.nonzero((i0 != i2).any(1))[0]
         assert (d0.view(np.uint32) == d2.view(np.uint32)).all(), np.nonzero((d0.view(np.uint32) != d2.view(np.uint32)).any(1))[0]
+
+
+# (squares and products that underflow fp32 partly or wholly, and large ones)
+@pytest.mark.parametrize("data_scale,query_scale", [(1.0, 1e-14), (1.0, 1e-17), (1.0, 1e-20), (1.0, 1e-38), (1.0, 1e18), (1e-13, 1e-13),
+                                                    (1e-17, 1e-17), (1e-19, 1e-19), (1e-20, 1.0), (1e16, 1e16)])
+@pytest.mark.parametrize("metric", [0, 6])
+def test_scales_at_the_ends_of_fp32_answer_as_with_tables(ivf, oracle_mod, tmp_path, metric, data_scale, query_scale):
+    from cuvs_b200 import _lib as L
+    x, q, ix, path = build_case(oracle_mod, tmp_path, "e", n=2500, dim=48, n_lists=16, pq_dim=24, metric=metric, nq=80)
+    for a in (ix.pq_centers, ix.centers, ix.centers_rot):
+        a *= np.float32(data_scale)
+    ix.centers[:, 48] *= np.float32(data_scale)
+    ix.save(path)
+    g, q = ivf.load(path), (q * np.float32(query_scale)).astype(np.float32)
+    for lut in ("f32", "f16"):
+        d2, i2 = gpu_search(ivf, g, q, 10, 7, lut)
+        L.check(L.load().cuvsB200SetScanCodebookHome(2))
+        d0, i0 = gpu_search(ivf, g, q, 10, 7, lut)
+        L.check(L.load().cuvsB200SetScanCodebookHome(4))
+        assert (i0 == i2).all(), np.nonzero((i0 != i2).any(1))[0]
+        assert (d0.view(np.uint32) == d2.view(np.uint32)).all()
