@@ -59,6 +59,7 @@ __device__ __forceinline__ float unit_lo(const rescore_params& p, float v, float
 {
   if (v == INFINITY) { return -INFINITY; }  // a pair without bounds
   if constexpr (kIP) {
+    if (!(qn * (p.rmax + norm) < p.sum_limit)) { return -INFINITY; }  // entries may be -inf
     return v + (p.cosine ? 1.0f : 0.0f) - (qn * (p.rmax * p.ip_gemm + (p.rmax + norm) * p.ip_lut) + p.eta);
   } else {
     if (norm < 0.0f && p.saturates) { return -INFINITY; }

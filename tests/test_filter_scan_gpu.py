@@ -169,6 +169,7 @@ def odd_queries(q):
     q[0, 3], q[1], q[2, 5], q[3], q[4] = np.nan, np.nan, np.inf, -np.inf, 0.0
     q[5], q[6, 0], q[8], q[9, 1], q[10], q[11], q[12] = 1e30, -1e30, 1e4, 3e4, 1e19, 3e18, 300.0
     q[7] *= 1e-7
+    q[13] *= 1e12
     return q
 
 
