@@ -881,13 +881,19 @@ void launch_query_scale(const float* rot_q, uint32_t n_queries, uint32_t rot_dim
   CUDA_TRY(cudaGetLastError());
 }
 
-uint64_t max_filter_tiles(const index<int64_t>& idx, uint64_t n_pairs)
+uint64_t max_filter_tiles(const index<int64_t>& idx, uint32_t n_queries, uint32_t n_probes, bool distinct)
 {
-  // tiles of the longest list, the most that one more group of 128 queries can add
+  const uint64_t n_pairs = uint64_t(n_queries) * n_probes;
+  // every list once (row tiles of the whole index), and the extra query groups: one more per 128 pairs of a list
+  const uint64_t all     = uint64_t(idx.total_rows_padded()) / kTileR + idx.n_lists();
   const uint64_t longest = ceildiv<uint64_t>(uint64_t(idx.accum_sorted_sizes()[1]), kTileR);
-  // every list once (row tiles of the whole index), and the extra query groups
-  const uint64_t all = uint64_t(idx.total_rows_padded()) / kTileR + idx.n_lists();
-  return std::min<uint64_t>(n_pairs * longest, all + (n_pairs / kTileQ) * longest);
+  uint64_t tiles         = std::min(n_pairs * longest, all + (n_pairs / kTileQ) * longest);
+  if (distinct) {
+    // a list has at most n_queries pairs: at worst all of them in the n_probes longest lists
+    const uint64_t probed = uint64_t(idx.accum_sorted_sizes()[n_probes]) / kTileR + n_probes;
+    tiles                 = std::min(tiles, all + ceildiv<uint64_t>(n_queries, kTileQ) * probed);
+  }
+  return tiles;
 }
 
 void launch_filter(const filter_params& p, const __half* operand, uint32_t n_pairs, int grid, size_t smem,

@@ -119,8 +119,8 @@ void launch_pair_operands(const operand_params& p, const uint32_t* probes, const
                           const uint32_t* group_index, uint32_t n_pairs, uint32_t n_probes, uint32_t max_groups,
                           uint32_t* cursor, __half* operand, float4* pair_rec, float* pair_norm, cudaStream_t stream);
 void launch_query_scale(const float* rot_q, uint32_t n_queries, uint32_t rot_dim, float* q_scale, cudaStream_t stream);
-// Upper bound on the number of tiles.
-uint64_t max_filter_tiles(const index<int64_t>& idx, uint64_t n_pairs);
+// Upper bound on the number of tiles; `distinct`: no query probes a list twice (caller-given probes may).
+uint64_t max_filter_tiles(const index<int64_t>& idx, uint32_t n_queries, uint32_t n_probes, bool distinct);
 
 // Half-precision codebooks: `out` [pq_dim][book][len_pad], stats[0] = sum over subspaces of the largest squared
 // codeword norm, stats[1] = largest |component|, both of the fp32 codebook; `scale_out` the power of two.

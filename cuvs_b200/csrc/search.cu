@@ -933,7 +933,7 @@ void search_any(raft::resources& res, const search_params& params, const index<i
   const size_t o_probes  = lay.add(n_pairs_max * 4);
   const size_t o_chunk   = lay.add(n_pairs_max * 4);
   const bool f_use       = fplan.use;
-  const size_t n_tiles   = f_use ? size_t(max_filter_tiles(idx, n_pairs_max)) : 0;
+  const size_t n_tiles   = f_use ? size_t(max_filter_tiles(idx, batch, n_probes, given_probes == nullptr)) : 0;
   const size_t o_groups  = lay.add(f_use ? n_pairs_max * 4 : 0);
   const size_t o_rec     = lay.add(f_use ? n_pairs_max * 16 : 0);
   const size_t o_norm    = lay.add(f_use ? n_pairs_max * 4 : 0);

@@ -209,3 +209,29 @@ def test_scales_at_the_ends_of_fp32_answer_as_with_tables(ivf, oracle_mod, tmp_p
         L.check(L.load().cuvsB200SetScanCodebookHome(4))
         assert (i0 == i2).all(), np.nonzero((i0 != i2).any(1))[0]
         assert (d0.view(np.uint32) == d2.view(np.uint32)).all()
+
+
+def test_workspace_of_a_skewed_index(ivf):
+    """One list of 400,000 rows, 4,000 of 25, each query probes 512 of them: bounds 2.1 GB, operand 0.33 GB, and tiles for what
+    10,000 queries can probe (25 MB; a bound by the longest list alone asks for 9 GB)."""
+    from cuvs_b200.common import Resources
+    g = torch.Generator(device="cuda").manual_seed(4)
+    n_lists, dim, long_list = 4001, 16, 400_000
+    centers = torch.randn(n_lists, dim, generator=g, device="cuda") * 4
+    index = ivf.build_precomputed(ivf.IndexParams(n_lists=n_lists, pq_dim=8), dim,
+                                  torch.randn(8, 2, 256, generator=g, device="cuda") * 0.3, centers, centers,
+                                  torch.eye(dim, device="cuda"))
+    which = torch.cat([torch.zeros(long_list, dtype=torch.int64, device="cuda"),
+                       torch.arange(100_000, device="cuda") % (n_lists - 1) + 1])
+    x = centers[which] + 0.2 * torch.randn(which.numel(), dim, generator=g, device="cuda")
+    ivf.extend(index, x, torch.arange(which.numel(), device="cuda"))
+    assert int(index.list_sizes.to(torch.int64).max()) > 300_000
+    q = x[torch.randint(0, x.shape[0], (10_000,), generator=g, device="cuda")].contiguous()
+    sp = lambda b: ivf.SearchParams(n_probes=512, lut_dtype=np.float16, max_internal_batch_size=b)  # noqa: E731
+    torch.cuda.empty_cache()
+    free, res = torch.cuda.mem_get_info()[0], Resources()
+    d, i = ivf.search(sp(10_000), index, q, 10, resources=res)
+    used = free - torch.cuda.mem_get_info()[0]
+    assert used < 4 << 30, used
+    d2, i2 = ivf.search(sp(500), index, q, 10)
+    assert bool((i == i2).all()) and bool((d == d2).all())
