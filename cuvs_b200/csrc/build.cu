@@ -1427,7 +1427,10 @@ void extend_any(raft::resources& res, const void* new_vectors, elem_t dtype, int
   ws_layout lay;
   const size_t row_bytes = size_t(dim) * elem_size(dtype);
   const size_t o_x       = lay.add(chunk * dim_ext * 4);
-  const size_t o_labels  = lay.add(n * 4);
+  // (the labels of more rows than these are released on return: they grow with the call, not with its chunks)
+  constexpr uint64_t kKeptLabels = 1ull << 26;
+  dev_array<uint32_t> many_labels(n > kKeptLabels ? n : 0);
+  const size_t o_labels  = lay.add(n > kKeptLabels ? 0 : n * 4);
   const size_t o_counts  = lay.add(size_t(n_lists) * 4);
   const size_t o_fill    = lay.add(size_t(n_lists) * 4);
   const size_t o_iota    = lay.add(chunk * 4);
@@ -1442,7 +1445,7 @@ void extend_any(raft::resources& res, const void* new_vectors, elem_t dtype, int
   res.scratch.reserve(lay.total());
   char* ws        = res.scratch.base();
   auto* x_ext     = reinterpret_cast<float*>(ws + o_x);
-  auto* labels    = reinterpret_cast<uint32_t*>(ws + o_labels);
+  auto* labels    = n > kKeptLabels ? many_labels.data() : reinterpret_cast<uint32_t*>(ws + o_labels);
   auto* counts    = reinterpret_cast<uint32_t*>(ws + o_counts);
   auto* fill      = reinterpret_cast<uint32_t*>(ws + o_fill);  // rows already placed in each list
   auto* iota      = reinterpret_cast<uint32_t*>(ws + o_iota);

@@ -136,7 +136,7 @@ struct resources {
   int smem_optin        = 0;        // max dynamic shared memory per block (opt-in)
   int cc_major          = 0;
   workspace ws;       // search
-  workspace scratch;  // extend and transform (bounded by their chunk size and the labels of the rows given)
+  workspace scratch;  // extend and transform: some 2 GB at most (what their chunks need, and the labels of 2^26 rows)
   // small pinned host word for an occasional device->host scalar
   uint32_t* pinned = nullptr;
   // counters read by the benchmark ("how many kernels of ours ran")

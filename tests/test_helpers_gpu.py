@@ -225,6 +225,27 @@ def test_an_emptied_index_gives_its_memory_back(mods, rows, kept):
     assert bool((i0 == i1).all()) and bool((d0 == d1).all())
 
 
+def test_what_a_handle_keeps_does_not_grow_with_the_rows_given(mods):
+    """70 million rows: their labels (267 MiB) are released on return, the scratch of a chunk stays."""
+    from cuvs_b200.common import Resources
+    ivf, _ = mods
+    n, g = 70_000_000, torch.Generator(device="cuda").manual_seed(1)
+    centers = torch.rand(8, 4, generator=g, device="cuda")
+    x = torch.randint(0, 256, (n, 4), generator=g, device="cuda", dtype=torch.uint8)
+    ids = torch.arange(n, device="cuda")
+    index = ivf.build_precomputed(ivf.IndexParams(n_lists=8, pq_dim=2), 4, torch.rand(2, 2, 256, generator=g, device="cuda") * 0.2,
+                                  centers, centers, torch.eye(4, device="cuda"))
+    torch.cuda.empty_cache()
+    free, res = torch.cuda.mem_get_info()[0], Resources()
+    ivf.extend(index, x, ids, resources=res)
+    assert len(index) == n
+    labels, _ = ivf.transform(index, x[:1000].contiguous())
+    assert (torch.bincount(labels.to(torch.int64), minlength=8) > 0).sum() > 1 and int(index.list_sizes.to(torch.int64).sum()) == n
+    del index, labels
+    torch.cuda.empty_cache()
+    assert free - torch.cuda.mem_get_info()[0] < 192 << 20
+
+
 def test_row_ranges_are_checked(mods):
     ivf, H = mods
     from cuvs_b200._lib import CuvsError
