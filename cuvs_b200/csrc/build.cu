@@ -20,6 +20,7 @@
 // labelling makes unnecessary here.  Unlike the reference's atomic slot allocation, vectors are placed
 // in a list in input order, so extend is deterministic.
 #include "ivf_pq.hpp"
+#include "packed.cuh"
 #include "search_internal.hpp"
 #include "topk.cuh"
 
@@ -375,38 +376,6 @@ __global__ void train_codebooks_kernel(const float* __restrict__ resid, uint32_t
 // ------------------------------------------------------------------------------------------------
 // encoder
 // ------------------------------------------------------------------------------------------------
-__device__ __forceinline__ uint64_t sub2(uint64_t a, uint64_t b)
-{
-  uint64_t d;
-  asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-  return d;
-}
-__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b)
-{
-  uint64_t d;
-  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-  return d;
-}
-__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c)
-{
-  uint64_t d;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
-  return d;
-}
-__device__ __forceinline__ uint64_t dup2(float x)
-{
-  uint64_t v;
-  asm("mov.b64 %0, {%1, %1};" : "=l"(v) : "f"(x));
-  return v;
-}
-__device__ __forceinline__ float lo2(uint64_t v) { return __uint_as_float(uint32_t(v)); }
-__device__ __forceinline__ float hi2(uint64_t v) { return __uint_as_float(uint32_t(v >> 32)); }
-__device__ __forceinline__ float min3(float a, float b, float c)
-{
-  float d;
-  asm("min.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
-  return d;
-}
 
 // Differences of the rows (taken in `order`) to the centres of their lists.  One thread per component.
 __global__ void difference_kernel(const float* __restrict__ x_ext, const uint32_t* __restrict__ labels,

@@ -564,8 +564,8 @@ extern "C" cuvsError_t cuvsB200IvfPqSearchArrays(cuvsResources_t res, cudaStream
       view.bits   = filter_bits;
       view.n_bits = uint64_t(filter_words) * 32u;
     }
-    search_arrays(res, static_cast<cuvsIvfPqSearchParams_t>(params), *index_of(static_cast<cuvsIvfPqIndex_t>(index)), queries, elem_of_dtype(type, "queries"),
-                  n_queries, dim, k, neighbors, distances, view);
+    search_arrays(res, static_cast<cuvsIvfPqSearchParams_t>(params), *index_of(static_cast<cuvsIvfPqIndex_t>(index)),
+                  queries, elem_of_dtype(type, "queries"), n_queries, dim, k, neighbors, distances, view);
     if (sync) { r->sync(); }
   });
 }

@@ -10,6 +10,7 @@
 // one thread in ascending k, so it equals the defining chain bit for bit) and a per-query radix
 // select.  It is the general path (any n_probes up to 4096, any shape).
 #include "common.hpp"
+#include "packed.cuh"
 #include "search_internal.hpp"
 #include "topk.cuh"
 
@@ -23,19 +24,7 @@ namespace {
 
 constexpr uint32_t kMaxProbes = 4096;
 
-__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c)
-{
-  uint64_t d;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
-  return d;
-}
 
-__device__ __forceinline__ uint64_t dup2(float x)
-{
-  uint64_t v;
-  asm("mov.b64 %0, {%1, %1};" : "=l"(v) : "f"(x));
-  return v;
-}
 
 // out[i, j] = alpha * sum over ascending k of b[j, k] * a[i, k], one fused multiply-add chain per output (the chain that
 // defines a coarse score, a rotation, a label).  kArgmin: instead of storing, best[i] = min over j of
@@ -238,7 +227,8 @@ void launch_exact_gemm(const float* b, uint32_t n_cols, const float* a, uint32_t
     const size_t smem = (size_t(32) * (kdim | 1u) + size_t(n_rows) * kdim) * 4;
     if (n_rows <= kFewRows && smem <= 200 * 1024) {
       ensure_dynamic_smem(reinterpret_cast<const void*>(few_rows_kernel), smem);
-      launch_chained(few_rows_kernel, ceildiv(n_cols, 32u), 128, smem, stream, b, n_cols, a, n_rows, a_stride, kdim, alpha, half_scores, out);
+      launch_chained(few_rows_kernel, ceildiv(n_cols, 32u), 128, smem, stream, b, n_cols, a, n_rows, a_stride, kdim,
+                     alpha, half_scores, out);
       CUDA_TRY(cudaGetLastError());
       return;
     }
@@ -253,9 +243,11 @@ void launch_exact_gemm(const float* b, uint32_t n_cols, const float* a, uint32_t
     unsigned long long* bs = best ? best + r0 : nullptr;
     const bool vec = kdim % 4 == 0 && a_stride % 4 == 0 && ((reinterpret_cast<uintptr_t>(b) | reinterpret_cast<uintptr_t>(ar)) & 15u) == 0;
     if (vec) {
-      launch_chained(exact_gemm_kernel<true, kArgmin>, grid, 256, 0, stream, b, n_cols, ar, nr, a_stride, kdim, alpha, half_scores, o, bs, row_list, n_listed);
+      launch_chained(exact_gemm_kernel<true, kArgmin>, grid, 256, 0, stream, b, n_cols, ar, nr, a_stride, kdim, alpha,
+                     half_scores, o, bs, row_list, n_listed);
     } else {
-      launch_chained(exact_gemm_kernel<false, kArgmin>, grid, 256, 0, stream, b, n_cols, ar, nr, a_stride, kdim, alpha, half_scores, o, bs, row_list, n_listed);
+      launch_chained(exact_gemm_kernel<false, kArgmin>, grid, 256, 0, stream, b, n_cols, ar, nr, a_stride, kdim, alpha,
+                     half_scores, o, bs, row_list, n_listed);
     }
     CUDA_TRY(cudaGetLastError());
   }
@@ -452,8 +444,8 @@ void launch_select(const float* scores, uint32_t n_rows, uint32_t row_stride, ui
   auto go = [&](auto kernel, int threads) {
     const size_t smem = size_t(cap) * 8;
     if (smem > 48 * 1024) { ensure_dynamic_smem(reinterpret_cast<const void*>(kernel), smem); }
-    launch_chained(kernel, n_rows, threads, smem, stream, scores, row_stride, row_len, row_ends, ends_stride, want, cap, out_idx,
-                                              out_scores);
+    launch_chained(kernel, n_rows, threads, smem, stream, scores, row_stride, row_len, row_ends, ends_stride, want, cap,
+                   out_idx, out_scores);
     CUDA_TRY(cudaGetLastError());
   };
   if (want <= 160) {

@@ -1297,7 +1297,8 @@ void select_clusters_tc(raft::resources& res, const float* centers, const float*
   cudaStream_t stream = res.stream;
 
   if (ext_scale == 1.0f) { ext_col = dim_ext; }
-  launch_chained(split_queries_kernel, ceildiv<uint32_t>(n_queries * 32u, 256u), 256, 0, stream, fq, n_queries, dim_ext, ext_col, ext_scale, cmax, fq_hi, fq_lo, row_scale, words);
+  launch_chained(split_queries_kernel, ceildiv<uint32_t>(n_queries * 32u, 256u), 256, 0, stream, fq, n_queries, dim_ext,
+                 ext_col, ext_scale, cmax, fq_hi, fq_lo, row_scale, words);
 
   const CUtensorMap m_a_hi = make_map(fq_hi, n_queries, dim_ext, kBM);
   const CUtensorMap m_a_lo = make_map(fq_lo, n_queries, dim_ext, kBM);
@@ -1371,25 +1372,27 @@ void select_clusters_tc(raft::resources& res, const float* centers, const float*
   const size_t fin_small_smem = (size_t(dim_ext) + size_t(fin_rows) * (dim_ext + 1)) * 4;
   if (n_tiles * 2 <= kFinMaxHalfTiles && C <= kFinMaxC && C * 4 <= n_tiles * 2 && fin_small_smem <= 48 * 1024) {
     if (kph == 16) {
-      launch_chained(coarse_finish_small_kernel<16>, n_queries, 256, fin_small_smem, stream, cand_key, cand_bnd, n_cand, centers, fq, n_lists, dim_ext, alpha, n_probes, C, cmax, eps_rel, probes,
-        scores_out, redo_list, words + 2, fin_rows, words, ext_col, ext_scale, row_scale, down_thr);
+      launch_chained(coarse_finish_small_kernel<16>, n_queries, 256, fin_small_smem, stream, cand_key, cand_bnd, n_cand,
+                     centers, fq, n_lists, dim_ext, alpha, n_probes, C, cmax, eps_rel, probes, scores_out, redo_list,
+                     words + 2, fin_rows, words, ext_col, ext_scale, row_scale, down_thr);
     } else {
-      launch_chained(coarse_finish_small_kernel<8>, n_queries, 256, fin_small_smem, stream, cand_key, cand_bnd, n_cand, centers, fq, n_lists, dim_ext, alpha, n_probes, C, cmax, eps_rel, probes,
-        scores_out, redo_list, words + 2, fin_rows, words, ext_col, ext_scale, row_scale, down_thr);
+      launch_chained(coarse_finish_small_kernel<8>, n_queries, 256, fin_small_smem, stream, cand_key, cand_bnd, n_cand,
+                     centers, fq, n_lists, dim_ext, alpha, n_probes, C, cmax, eps_rel, probes, scores_out, redo_list,
+                     words + 2, fin_rows, words, ext_col, ext_scale, row_scale, down_thr);
     }
   } else {
     if (fin_smem > 48 * 1024) { ensure_dynamic_smem(reinterpret_cast<const void*>(coarse_finish_kernel), fin_smem); }
     launch_chained(coarse_finish_kernel, n_queries, 256, fin_smem, stream, cand_key, cand_bnd, n_cand, kph, centers, fq,
-                                                               n_lists, dim_ext, alpha, n_probes, C, cap,
-                                                               cmax, eps_rel, probes, scores_out, redo_list,
-                                                               words + 2, words, ext_col, ext_scale, row_scale, down_thr, by_maxima ? 1 : 0);
+                   n_lists, dim_ext, alpha, n_probes, C, cap, cmax, eps_rel, probes, scores_out, redo_list, words + 2,
+                   words, ext_col, ext_scale, row_scale, down_thr, by_maxima ? 1 : 0);
   }
   uint32_t cap_fb = 2;
   while (cap_fb < n_probes) { cap_fb <<= 1; }
   const size_t fb_smem = size_t(cap_fb) * 8 + size_t(dim_ext) * 4;
   const size_t fs_smem = (size_t(256) * 33 + size_t(kFbGroup) * dim_ext) * 4;
   ensure_dynamic_smem(reinterpret_cast<const void*>(coarse_fallback_scores_kernel), fs_smem);
-  launch_chained(coarse_fallback_scores_kernel, ceildiv<uint32_t>(n_lists, 256u), 256, fs_smem, stream, redo_list, words + 2, centers, fq, n_queries, n_lists, dim_ext, alpha, scratch, kFbSlots, words);
+  launch_chained(coarse_fallback_scores_kernel, ceildiv<uint32_t>(n_lists, 256u), 256, fs_smem, stream, redo_list,
+                 words + 2, centers, fq, n_queries, n_lists, dim_ext, alpha, scratch, kFbSlots, words);
   // the error word and how many queries this batch redid exactly: written to pinned memory by the kernel, looked at
   // before a later batch and at the handle's next synchronisation
   uint32_t* host_words = nullptr;
@@ -1401,9 +1404,9 @@ void select_clusters_tc(raft::resources& res, const float* centers, const float*
     res.tc_redo_pending  = true;
     res.tc_redo_seq++;
   }
-  launch_chained(coarse_fallback_kernel, kFbSlots, 256, fb_smem, stream, redo_list, words + 2, centers, fq, n_queries, n_lists,
-                                                       dim_ext, alpha, n_probes, cap_fb, scratch, probes,
-                                                       scores_out, words, host_words, res.tc_redo_seq);
+  launch_chained(coarse_fallback_kernel, kFbSlots, 256, fb_smem, stream, redo_list, words + 2, centers, fq, n_queries,
+                 n_lists, dim_ext, alpha, n_probes, cap_fb, scratch, probes, scores_out, words, host_words,
+                 res.tc_redo_seq);
   CUDA_TRY(cudaGetLastError());
   res.launches += 5;
 }

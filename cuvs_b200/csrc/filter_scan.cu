@@ -25,6 +25,7 @@
 // dimensions per subspace, 3.4 wavefronts each on random codes); for many, the epilogue and the operand feed.
 #include "common.hpp"
 #include "filter_scan.hpp"
+#include "packed.cuh"
 #include "search_internal.hpp"
 #include "tc_ptx.cuh"
 #include "topk.cuh"
@@ -50,12 +51,6 @@ constexpr uint32_t kDecodeWarps = 16, kEpiWarp = 16, kEpiWarps = 8, kMmaWarp = 2
 constexpr uint32_t kFilterThreads = 26 * 32;
 constexpr float kMaskHalf    = 32768.0f;                // mask x mask = 2^30 in the scaled domain
 
-__device__ __forceinline__ float min3(float a, float b, float c)
-{
-  float d;
-  asm("min.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
-  return d;
-}
 // acc += h * h in fp32 (the half widens exactly)
 __device__ __forceinline__ float fma_half_sq(uint32_t h2, bool hi, float acc)
 {
@@ -107,14 +102,6 @@ __device__ __forceinline__ void lds128(uint32_t a, uint32_t& x, uint32_t& y, uin
 // byte offset of 16-byte chunk c (0..7) of row r inside a swizzled K block
 __device__ __forceinline__ uint32_t swz(uint32_t r, uint32_t c) { return r * 128u + ((c ^ (r & 7u)) << 4); }
 
-template <uint32_t kN, uint32_t kI = 0, typename Fn>
-__device__ __forceinline__ void static_for(Fn&& fn)
-{
-  if constexpr (kI < kN) {
-    fn(std::integral_constant<uint32_t, kI>{});
-    static_for<kN, kI + 1>(fn);
-  }
-}
 
 // kBits 8 or 4 (kWords): the codes of half a K block are extracted from whole words with constant shifts; other widths,
 // and subspaces of more than eight components, code by code.  kLP: halfs per subspace in the K layout (1, 2, 4 or 8;
@@ -851,7 +838,8 @@ void launch_count_pairs(const uint32_t* probes, const uint32_t* list_sizes, uint
                         uint32_t n_probes, uint32_t* chunk_index, uint32_t* group_index, uint32_t* list_count,
                         cudaStream_t stream)
 {
-  launch_chained(count_pairs_kernel, ceildiv<uint32_t>(n_queries * 32, 256), 256, 0, stream, probes, list_sizes, n_lists, n_queries, n_probes, chunk_index, group_index, list_count);
+  launch_chained(count_pairs_kernel, ceildiv<uint32_t>(n_queries * 32, 256), 256, 0, stream, probes, list_sizes,
+                 n_lists, n_queries, n_probes, chunk_index, group_index, list_count);
   CUDA_TRY(cudaGetLastError());
 }
 
@@ -859,9 +847,11 @@ void launch_tiles(const uint32_t* list_sizes, const uint64_t* row_off, uint32_t 
                   filter_tile* tiles, uint32_t* counters, cudaStream_t stream)
 {
   if (n_lists >= 32768) {
-    launch_chained(make_tiles_kernel<64>, ceildiv(n_lists, 64u), 256, 0, stream, list_count, list_sizes, row_off, n_lists, tiles, counters);
+    launch_chained(make_tiles_kernel<64>, ceildiv(n_lists, 64u), 256, 0, stream, list_count, list_sizes, row_off,
+                   n_lists, tiles, counters);
   } else {
-    launch_chained(make_tiles_kernel<16>, ceildiv(n_lists, 16u), 256, 0, stream, list_count, list_sizes, row_off, n_lists, tiles, counters);
+    launch_chained(make_tiles_kernel<16>, ceildiv(n_lists, 16u), 256, 0, stream, list_count, list_sizes, row_off,
+                   n_lists, tiles, counters);
   }
   CUDA_TRY(cudaGetLastError());
 }
@@ -870,14 +860,15 @@ void launch_pair_operands(const operand_params& p, const uint32_t* probes, const
                           const uint32_t* group_index, uint32_t n_pairs, uint32_t n_probes, uint32_t max_groups,
                           uint32_t* cursor, __half* operand, float4* pair_rec, float* pair_norm, cudaStream_t stream)
 {
-  launch_chained(pair_operands_kernel, ceildiv(n_pairs, 16u), 256, 0, stream, p, probes, list_sizes, n_lists, group_index, n_pairs, n_probes,
-                                                                 max_groups, cursor, operand, pair_rec, pair_norm);
+  launch_chained(pair_operands_kernel, ceildiv(n_pairs, 16u), 256, 0, stream, p, probes, list_sizes, n_lists,
+                 group_index, n_pairs, n_probes, max_groups, cursor, operand, pair_rec, pair_norm);
   CUDA_TRY(cudaGetLastError());
 }
 
 void launch_query_scale(const float* rot_q, uint32_t n_queries, uint32_t rot_dim, float* q_scale, cudaStream_t stream)
 {
-  launch_chained(query_scale_kernel, ceildiv<uint32_t>(n_queries * 32, 256), 256, 0, stream, rot_q, n_queries, rot_dim, q_scale);
+  launch_chained(query_scale_kernel, ceildiv<uint32_t>(n_queries * 32, 256), 256, 0, stream, rot_q, n_queries, rot_dim,
+                 q_scale);
   CUDA_TRY(cudaGetLastError());
 }
 

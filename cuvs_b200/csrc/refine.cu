@@ -273,8 +273,8 @@ void launch_refine_rows(raft::resources& res, const T* dataset, int64_t n_rows, 
       CUVS_EXPECTS(smem <= size_t(res.smem_optin) - 1024, "refine: dim = %u is too large", dim);
       ensure_dynamic_smem(reinterpret_cast<const void*>(kernel), smem);
     }
-    launch_chained(kernel, ceildiv(n_queries, qpb), warps * 32, smem, res.stream, dataset, n_rows, dim, queries, n_queries, candidates, n_cand, k, mode, log_lanes, log_wpq, q_floats, indices,
-      distances);
+    launch_chained(kernel, ceildiv(n_queries, qpb), warps * 32, smem, res.stream, dataset, n_rows, dim, queries,
+                   n_queries, candidates, n_cand, k, mode, log_lanes, log_wpq, q_floats, indices, distances);
     CUDA_TRY(cudaGetLastError());
   };
   if (k <= 32) {

@@ -22,6 +22,7 @@
 // it sits in shared memory once per CTA and thread groups of 32 to 256 take one query at a time.
 #include "common.hpp"
 #include "filter_scan.hpp"
+#include "packed.cuh"
 #include "scan.cuh"
 #include "search_internal.hpp"
 #include "tc_ptx.cuh"
@@ -42,12 +43,6 @@ __device__ __forceinline__ float sqrt_approx(float x)
   float r;
   asm("sqrt.approx.f32 %0, %1;" : "=f"(r) : "f"(x));
   return r;
-}
-__device__ __forceinline__ float min3(float a, float b, float c)
-{
-  float d;
-  asm("min.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
-  return d;
 }
 
 // Bound of a query's norm from its square; below 1e-15 squares may have underflowed and products may: no bounds then.
@@ -182,14 +177,6 @@ __device__ __forceinline__ float component(float entry, float q, float c, float 
   }
 }
 
-template <uint32_t kN, uint32_t kI = 0, typename Fn>
-__device__ __forceinline__ void static_for(Fn&& fn)
-{
-  if constexpr (kI < kN) {
-    fn(std::integral_constant<uint32_t, kI>{});
-    static_for<kN, kI + 1>(fn);
-  }
-}
 // Codebook loads at [address + constant]; the contents do not change, so they may move freely.
 template <uint32_t kOff>
 __device__ __forceinline__ void book_ld2(uint32_t a, float* b)

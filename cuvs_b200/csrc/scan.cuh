@@ -33,6 +33,7 @@
 // that no shared-memory plan can hold.
 #pragma once
 
+#include "packed.cuh"
 #include "topk.cuh"
 
 #include <cuda_fp16.h>
@@ -92,41 +93,9 @@ __device__ __forceinline__ uint64_t pack2(float x, float y)
 {
   return pack_b32x2(__float_as_uint(x), __float_as_uint(y));
 }
-__device__ __forceinline__ float lo2(uint64_t v)
-{
-  float lo, hi;
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
-  return lo;
-}
-__device__ __forceinline__ float hi2(uint64_t v)
-{
-  float lo, hi;
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
-  return hi;
-}
 __device__ __forceinline__ void sts_2xb32(uint32_t a, uint32_t x, uint32_t y)
 {
   asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(a), "r"(x), "r"(y) : "memory");
-}
-__device__ __forceinline__ uint64_t sub2(uint64_t a, uint64_t b)
-{
-  uint64_t d;
-  asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-  return d;
-}
-// a * b: the first term of a sum that starts from +0 (fma(a, a, +0) rounds to the same value, and
-// a square is never -0), without materialising a zero register pair
-__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b)
-{
-  uint64_t d;
-  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-  return d;
-}
-__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c)
-{
-  uint64_t d;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
-  return d;
 }
 
 // ---- 8-bit float, 5 exponent bits (ivf_pq_fp_8bit.cuh) -----------------------------------------
@@ -236,12 +205,6 @@ __device__ __forceinline__ void lds_2xb64(uint32_t a, uint64_t& x, uint64_t& y)
 __device__ __forceinline__ void sts_b128(uint32_t a, uint64_t x, uint64_t y)
 {
   asm volatile("st.shared.v2.b64 [%0], {%1, %2};" ::"r"(a), "l"(x), "l"(y) : "memory");
-}
-__device__ __forceinline__ uint64_t dup2(float x)
-{
-  uint64_t v;
-  asm("mov.b64 %0, {%1, %1};" : "=l"(v) : "f"(x));
-  return v;
 }
 
 // LUT of one pair from a codebook resident in shared memory.  A thread owns four adjacent codebook

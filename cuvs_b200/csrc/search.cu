@@ -622,13 +622,13 @@ void launch_prep(raft::resources& res, const index<int64_t>& idx, const void* qp
     using T = std::remove_const_t<std::remove_pointer_t<decltype(q)>>;
     if (mode == 1) {
       launch_chained(prep_queries_kernel<T, 1>, nq, threads, smem, stream, q, idx.dim(), dim_ext, idx.rot_dim(), is_l2,
-                                                               cosine, ident, d_fq, d_rq, counters);
+                     cosine, ident, d_fq, d_rq, counters);
     } else if (mode == 2) {
       launch_chained(prep_queries_kernel<T, 2>, nq, threads, smem, stream, q, idx.dim(), dim_ext, idx.rot_dim(), is_l2,
-                                                               cosine, ident, d_fq, d_rq, counters);
+                     cosine, ident, d_fq, d_rq, counters);
     } else {
       launch_chained(prep_queries_kernel<T, 0>, nq, threads, smem, stream, q, idx.dim(), dim_ext, idx.rot_dim(), is_l2,
-                                                               cosine, ident, d_fq, d_rq, counters);
+                     cosine, ident, d_fq, d_rq, counters);
     }
   };
   switch (qtype) {
@@ -1146,14 +1146,16 @@ void search_any(raft::resources& res, const search_params& params, const index<i
     const bool sorted_pairs = stats || n_pairs > 4096;
     if (!sorted_pairs) {
       // small batch: one launch, pairs in arrival order (a sort by list has nothing to gain here)
-      launch_chained(small_batch_pairs_kernel, ceildiv<uint32_t>(nq * 32, 128), 128, 0, stream, d_probes, idx.list_sizes(), n_lists, idx.row_offsets(), nq, n_probes, d_chunk, d_order, d_counter + 1, d_kth,
-        store_all ? nullptr : d_keys, k);
+      launch_chained(small_batch_pairs_kernel, ceildiv<uint32_t>(nq * 32, 128), 128, 0, stream, d_probes,
+                     idx.list_sizes(), n_lists, idx.row_offsets(), nq, n_probes, d_chunk, d_order, d_counter + 1, d_kth,
+                     store_all ? nullptr : d_keys, k);
       CUDA_TRY(cudaGetLastError());
       res.launches += 1;
     } else {
       // counting sort of the pairs by list
       CUDA_TRY(cudaMemsetAsync(d_count, 0, (size_t(n_lists) * 2 + 1) * 4, stream));
-      launch_chained(chunk_and_count_kernel, ceildiv<uint32_t>(nq * 32, 256), 256, 0, stream, d_probes, idx.list_sizes(), n_lists, nq, n_probes, d_chunk, d_count);
+      launch_chained(chunk_and_count_kernel, ceildiv<uint32_t>(nq * 32, 256), 256, 0, stream, d_probes,
+                     idx.list_sizes(), n_lists, nq, n_probes, d_chunk, d_count);
       if (stats) {
         scan_stats_kernel<<<ceildiv<uint32_t>(n_lists, 256), 256, 0, stream>>>(d_count, idx.list_sizes(),
                                                                                 n_lists, 2, res.d_stats);
@@ -1161,8 +1163,9 @@ void search_any(raft::resources& res, const search_params& params, const index<i
       }
       // d_counter[0] = 0 (work counter), d_counter[1] = d_count[2 * n_lists] = number of work items
       launch_chained(exclusive_scan_kernel, 1, 1024, 0, stream, d_count, n_lists * 2, d_counter);
-      launch_chained(scatter_pairs_kernel, ceildiv<uint32_t>(n_pairs, 256), 256, 0, stream, d_probes, d_chunk, idx.list_sizes(), n_lists, idx.row_offsets(), n_pairs, n_probes, d_count, d_order,
-        store_all ? nullptr : d_keys, k, d_kth, nq);
+      launch_chained(scatter_pairs_kernel, ceildiv<uint32_t>(n_pairs, 256), 256, 0, stream, d_probes, d_chunk,
+                     idx.list_sizes(), n_lists, idx.row_offsets(), n_pairs, n_probes, d_count, d_order,
+                     store_all ? nullptr : d_keys, k, d_kth, nq);
       CUDA_TRY(cudaGetLastError());
       res.launches += 3;
     }
@@ -1240,8 +1243,9 @@ void search_any(raft::resources& res, const search_params& params, const index<i
       auto* sel_idx    = reinterpret_cast<uint32_t*>(d_keys) + size_t(nq) * k;
       // (a row of scores ends where the query's last probe does; the scan writes every one of them)
       select_rows(res, d_all, nq, max_samples, k, sel_idx, sel_scores, d_chunk, n_probes);
-      launch_chained(translate_selected_kernel, unsigned(ceildiv<uint64_t>(uint64_t(nq) * k, 256)), 256, 0, stream, sel_scores, sel_idx, d_probes, d_chunk, idx.row_offsets(), idx.ids(), nq, n_probes, k,
-        int(metric), scale, neighbors + size_t(q0) * k, distances + size_t(q0) * k);
+      launch_chained(translate_selected_kernel, unsigned(ceildiv<uint64_t>(uint64_t(nq) * k, 256)), 256, 0, stream,
+                     sel_scores, sel_idx, d_probes, d_chunk, idx.row_offsets(), idx.ids(), nq, n_probes, k, int(metric),
+                     scale, neighbors + size_t(q0) * k, distances + size_t(q0) * k);
       CUDA_TRY(cudaGetLastError());
       res.launches++;
     } else {
@@ -1250,19 +1254,16 @@ void search_any(raft::resources& res, const search_params& params, const index<i
       float* ds        = distances + size_t(q0) * k;
       switch (kpl) {
         case 1:
-          launch_chained(final_merge_kernel<1>, blocks, 128, 0, stream, d_keys, d_probes, d_chunk,
-                                                            idx.row_offsets(), idx.ids(), nq, n_probes,
-                                                            k, int(metric), scale, nb, ds);
+          launch_chained(final_merge_kernel<1>, blocks, 128, 0, stream, d_keys, d_probes, d_chunk, idx.row_offsets(),
+                         idx.ids(), nq, n_probes, k, int(metric), scale, nb, ds);
           break;
         case 2:
-          launch_chained(final_merge_kernel<2>, blocks, 128, 0, stream, d_keys, d_probes, d_chunk,
-                                                            idx.row_offsets(), idx.ids(), nq, n_probes,
-                                                            k, int(metric), scale, nb, ds);
+          launch_chained(final_merge_kernel<2>, blocks, 128, 0, stream, d_keys, d_probes, d_chunk, idx.row_offsets(),
+                         idx.ids(), nq, n_probes, k, int(metric), scale, nb, ds);
           break;
         default:
-          launch_chained(final_merge_kernel<4>, blocks, 128, 0, stream, d_keys, d_probes, d_chunk,
-                                                            idx.row_offsets(), idx.ids(), nq, n_probes,
-                                                            k, int(metric), scale, nb, ds);
+          launch_chained(final_merge_kernel<4>, blocks, 128, 0, stream, d_keys, d_probes, d_chunk, idx.row_offsets(),
+                         idx.ids(), nq, n_probes, k, int(metric), scale, nb, ds);
       }
       CUDA_TRY(cudaGetLastError());
       res.launches++;
