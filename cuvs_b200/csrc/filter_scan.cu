@@ -320,11 +320,8 @@ filter_kernel(const __grid_constant__ CUtensorMap map_16, const __grid_constant_
             }
           }
         }
-        // (the whole warp leaves, or none of it: the lanes meet again below)
-        if (!__all_sync(kFullMask, mbar_wait(bar_empty + stage * 8, phase ^ 1u, p.spin_limit))) {
-          ok = false;
-          break;
-        }
+        // (a lane whose wait runs out goes through the tile's blocks without another one, so that the warp stays together)
+        if (ok) { ok = mbar_wait(bar_empty + stage * 8, phase ^ 1u, p.spin_limit); }
         if (in) {
           const uint32_t dst = base_a + stage * kStage + kABytes;
 #pragma unroll
@@ -347,6 +344,10 @@ filter_kernel(const __grid_constant__ CUtensorMap map_16, const __grid_constant_
           stage = 0;
           phase ^= 1u;
         }
+      }
+      if (__any_sync(kFullMask, !ok)) {
+        ok = false;
+        break;
       }
     }
   } else if (warp == kTmaWarp) {
