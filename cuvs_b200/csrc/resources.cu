@@ -72,7 +72,7 @@ resources::~resources()
   }
   if (d_stats) { cudaFree(d_stats); }
   if (pinned) {
-    if (tc_redo_pending) { cudaDeviceSynchronize(); }  // a kernel may still write its verdict there
+    cudaDeviceSynchronize();  // a kernel may still write its verdict or count a time-out there
     cudaFreeHost(pinned);
   }
 }
