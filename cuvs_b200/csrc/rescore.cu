@@ -137,9 +137,8 @@ __host__ __device__ inline uint32_t group_mem_bytes(uint32_t cap, uint32_t list_
                               (n_probes + 1u) * 8u + n_probes * 8u + 32u, 16u);
 }
 
-// One code's contribution in the reference's arithmetic, added to the running score.  kNaN: entries may be NaN (8-bit tables
-// give those a code of their own, which the clamp does not reproduce).
-template <int LutKind, bool OutHalf, bool IsIP, bool kNaN>
+// One code's contribution in the reference's arithmetic, added to the running score.
+template <int LutKind, bool OutHalf, bool IsIP>
 __device__ __forceinline__ void add_entry(float entry, float& f, __half& h)
 {
   if constexpr (!OutHalf) {
@@ -147,16 +146,15 @@ __device__ __forceinline__ void add_entry(float entry, float& f, __half& h)
       f = __fadd_rn(f, entry);
     } else if constexpr (LutKind == LUT_F16) {
       f = __fadd_rn(f, __half2float(__float2half_rn(entry)));
-    } else if constexpr (kNaN) {
-      f = __fadd_rn(f, fp8_to_float<IsIP>(fp8_encode<IsIP>(entry)));
     } else {
       // fp8_to_float(fp8_encode(entry)) of a non-negative entry: clamped to the type's range, all but the three
-      // upper mantissa bits replaced by half a step
+      // upper mantissa bits replaced by half a step; a NaN (a query with NaN components) has code 0x7F, which reads 1.9375
       static_assert(!IsIP, "inner products do not take this path");
       constexpr float kMin = 1.0f / 32768.0f;
       const float kMax     = __uint_as_float(0x3F800000u - (15u << 23) + (255u << 20));  // smallest value of the last code
       const float a        = fminf(fmaxf(entry, kMin), kMax);
-      f = __fadd_rn(f, __uint_as_float((__float_as_uint(a) & 0xFFF00000u) | 0x00080000u));
+      const float read     = __uint_as_float((__float_as_uint(a) & 0xFFF00000u) | 0x00080000u);
+      f = __fadd_rn(f, entry == entry ? read : 1.9375f);
     }
   } else {
     if constexpr (LutKind == LUT_F16) {
@@ -192,8 +190,8 @@ __device__ __forceinline__ void book_ld4(uint32_t a, float* b)
 // Exact score of one row: `src` its first 16-byte code piece (the next ones 512 bytes apart), c the rotated centre of
 // its list.  Stops early (false) when a partial sum of non-negative terms has passed `bound`.
 // kLen 2 or 4 with kBits 8 or 4: straight-line code over a piece; else the general loop.  kSmem: the codebook is in
-// shared memory.  kNaN: see add_entry.
-template <int LutKind, bool OutHalf, bool IsIP, int kLen, int kBits, bool kSmem, bool kNaN = false>
+// shared memory.
+template <int LutKind, bool OutHalf, bool IsIP, int kLen, int kBits, bool kSmem>
 __device__ __forceinline__ bool score_row(const rescore_params& p, const float* s_book, const float* rq, const float* c,
                                           const uint4* src, float bound, float& f, __half& h)
 {
@@ -236,7 +234,7 @@ __device__ __forceinline__ bool score_row(const rescore_params& p, const float* 
           float e = 0.0f;
 #pragma unroll
           for (uint32_t kk = 0; kk < kLen; kk++) { e = component<IsIP>(e, qa[s * kLen + kk], ca[s * kLen + kk], b[kk]); }
-          add_entry<LutKind, OutHalf, IsIP, kNaN>(e, f, h);
+          add_entry<LutKind, OutHalf, IsIP>(e, f, h);
         });
       };
       if (nj == kCodes) {
@@ -261,7 +259,7 @@ __device__ __forceinline__ bool score_row(const rescore_params& p, const float* 
         for (uint32_t kk = 0; kk < len; kk++) {
           e = component<IsIP>(e, rq[j * len + kk], __ldg(c + j * len + kk), kSmem ? b[kk] : __ldg(b + kk * book));
         }
-        add_entry<LutKind, OutHalf, IsIP, kNaN>(e, f, h);
+        add_entry<LutKind, OutHalf, IsIP>(e, f, h);
       }
     }
     if constexpr (!IsIP) {
@@ -437,14 +435,6 @@ __global__ void __launch_bounds__(1024, 1) rescore_kernel(const rescore_params p
         qn = query_norm(qn);
       }
     }
-    // 8-bit tables: does the query hold a NaN?  (A select on every entry, or such rows scored by a function of their own, cost
-    // more: the latter 2.6% of 10,000 queries of 64 probes, k 100; this 0.4%.)
-    constexpr bool kMayBeNaN = LutKind == LUT_FP8 && !OutHalf;
-    bool has_nan = false;
-    if constexpr (kMayBeNaN) {
-      for (uint32_t i = lane; i < p.rot_dim; i += 32) { has_nan = has_nan || s.rq[i] != s.rq[i]; }
-      has_nan = __any_sync(kFullMask, has_nan);
-    }
     const float vk = __uint_as_float(s.word[W_VK]), vmax = __uint_as_float(s.word[W_VMAX]);
 
     // Sorts the first n2 (a power of two) keys of buf across the group.
@@ -502,11 +492,7 @@ __global__ void __launch_bounds__(1024, 1) rescore_kernel(const rescore_params p
         if (valid) {
           const uint4* src = reinterpret_cast<const uint4*>(p.codes + ((row & ~uint64_t(31)) * p.n_pieces) * 16u) + (row & 31u);
           const float* c   = p.centers + size_t(s.label[pi]) * p.rot_dim;
-          if (kMayBeNaN && has_nan) {
-            valid = score_row<LutKind, OutHalf, IsIP, 0, 0, kSmem, kMayBeNaN>(p, s_book, s.rq, c, src, bound, f, h);
-          } else {
-            valid = score_row<LutKind, OutHalf, IsIP, kLen, kBits, kSmem>(p, s_book, s.rq, c, src, bound, f, h);
-          }
+          valid = score_row<LutKind, OutHalf, IsIP, kLen, kBits, kSmem>(p, s_book, s.rq, c, src, bound, f, h);
         }
         float score;
         if constexpr (!OutHalf) {
