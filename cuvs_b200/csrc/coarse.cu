@@ -33,9 +33,9 @@ constexpr uint32_t kMaxProbes = 4096;
 // as packed pairs of columns (fma.rn.f32x2: two chains per instruction), a warp 4 x 8 threads so that its loads are
 // 64 and 128 distinct bytes; the next eight k are on their way while eight are used.
 // 10,000 x 4,000 x 136: 487 us with 64 x 64 outputs per block and scalar FMAs, 238 us so.  kVec: rows of both operands are
-// 16-byte aligned and k is a multiple of four.
+// 16-byte aligned and k is a multiple of four.  kListed: the rows of `a` (and of `best`) named by row_list, *n_listed of them.
 constexpr uint32_t kTile = 128, kTileK = 8;
-template <bool kVec, bool kArgmin>
+template <bool kVec, bool kArgmin, bool kListed>
 __global__ void __launch_bounds__(256, 2)
 exact_gemm_kernel(const float* __restrict__ b, uint32_t n_cols, const float* __restrict__ a, uint32_t n_rows, uint32_t a_stride,
                   uint32_t kdim, float alpha, int half_scores, float* __restrict__ out, unsigned long long* __restrict__ best,
@@ -44,127 +44,132 @@ exact_gemm_kernel(const float* __restrict__ b, uint32_t n_cols, const float* __r
   chain_begin();
   __shared__ __align__(16) float s_a[2][kTileK][kTile + 4];
   __shared__ __align__(16) float s_b[2][kTileK][kTile + 4];
-  const uint32_t j0 = blockIdx.x * kTile, i0 = blockIdx.y * kTile;
+  const uint32_t j0 = blockIdx.x * kTile;
   const uint32_t tid = threadIdx.x;
   const uint32_t tx = ((tid >> 5) & 1u) * 8u + (tid & 7u), ty = (tid >> 6) * 4u + ((tid >> 3) & 3u);
-  // `row_list` (optional): the rows of `a` (and of `best`) to do, *n_listed of them
-  if (row_list != nullptr) {
-    n_rows = min(n_rows, __ldg(n_listed));
-    if (i0 >= n_rows) { return; }
-  }
-  // one row and four k of either operand per thread
-  const uint32_t lrow = tid >> 1, lk = (tid & 1u) * 4u;
-  const bool in_a = i0 + lrow < n_rows, in_b = j0 + lrow < n_cols;
-  const float* pa = a + size_t(row_list != nullptr && in_a ? __ldg(row_list + i0 + lrow) : i0 + lrow) * a_stride + lk;
-  const float* pb = b + size_t(j0 + lrow) * kdim + lk;
-  float ra[4], rb[4];
-  auto load = [&](uint32_t k0) {
-    if constexpr (kVec) {
-      const float4 z = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-      const float4 x = in_a && k0 + lk < kdim ? __ldg(reinterpret_cast<const float4*>(pa + k0)) : z;
-      const float4 y = in_b && k0 + lk < kdim ? __ldg(reinterpret_cast<const float4*>(pb + k0)) : z;
-      ra[0] = x.x; ra[1] = x.y; ra[2] = x.z; ra[3] = x.w;
-      rb[0] = y.x; rb[1] = y.y; rb[2] = y.z; rb[3] = y.w;
-    } else {
+  if constexpr (kListed) { n_rows = min(n_rows, __ldg(n_listed)); }
+  // (listed rows: the blocks take the tiles in turn, since the host does not know how many there are; else each has one)
+  uint32_t i0 = blockIdx.y * kTile;
+  if (kListed && i0 >= n_rows) { return; }
+  do {
+    // one row and four k of either operand per thread
+    const uint32_t lrow = tid >> 1, lk = (tid & 1u) * 4u;
+    const bool in_a = i0 + lrow < n_rows, in_b = j0 + lrow < n_cols;
+    const float* pa = a + size_t(kListed && in_a ? __ldg(row_list + i0 + lrow) : i0 + lrow) * a_stride + lk;
+    const float* pb = b + size_t(j0 + lrow) * kdim + lk;
+    float ra[4], rb[4];
+    auto load = [&](uint32_t k0) {
+      if constexpr (kVec) {
+        const float4 z = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        const float4 x = in_a && k0 + lk < kdim ? __ldg(reinterpret_cast<const float4*>(pa + k0)) : z;
+        const float4 y = in_b && k0 + lk < kdim ? __ldg(reinterpret_cast<const float4*>(pb + k0)) : z;
+        ra[0] = x.x; ra[1] = x.y; ra[2] = x.z; ra[3] = x.w;
+        rb[0] = y.x; rb[1] = y.y; rb[2] = y.z; rb[3] = y.w;
+      } else {
 #pragma unroll
-      for (uint32_t e = 0; e < 4; e++) {
-        const bool in = k0 + lk + e < kdim;
-        ra[e]         = in && in_a ? __ldg(pa + k0 + e) : 0.0f;
-        rb[e]         = in && in_b ? __ldg(pb + k0 + e) : 0.0f;
-      }
-    }
-  };
-  auto store = [&](uint32_t buf) {
-#pragma unroll
-    for (uint32_t e = 0; e < 4; e++) {
-      s_a[buf][lk + e][lrow] = ra[e];
-      s_b[buf][lk + e][lrow] = rb[e];
-    }
-  };
-  // rows ty * 4 + {0..3} and 64 + ..., columns tx * 4 + {0..3} and 64 + ...
-  uint64_t acc[8][4];
-#pragma unroll
-  for (int i = 0; i < 8; i++) {
-#pragma unroll
-    for (int j = 0; j < 4; j++) { acc[i][j] = 0ull; }
-  }
-  load(0);
-  store(0);
-  __syncthreads();
-  uint32_t buf = 0;
-  for (uint32_t k0 = 0; k0 < kdim; k0 += kTileK, buf ^= 1u) {
-    const bool more = k0 + kTileK < kdim;
-    if (more) { load(k0 + kTileK); }
-    // (a partial last tile stops at kdim: a product with zero would leave the chain's value alone, except for -0 and
-    // infinities)
-    const uint32_t kn = min(kTileK, kdim - k0);
-    auto step = [&](uint32_t k) {
-      const float4 x0 = *reinterpret_cast<const float4*>(&s_a[buf][k][ty * 4u]);
-      const float4 x1 = *reinterpret_cast<const float4*>(&s_a[buf][k][64u + ty * 4u]);
-      const ulonglong2 c0 = *reinterpret_cast<const ulonglong2*>(&s_b[buf][k][tx * 4u]);
-      const ulonglong2 c1 = *reinterpret_cast<const ulonglong2*>(&s_b[buf][k][64u + tx * 4u]);
-      const uint64_t x[8] = {dup2(x0.x), dup2(x0.y), dup2(x0.z), dup2(x0.w), dup2(x1.x), dup2(x1.y), dup2(x1.z), dup2(x1.w)};
-      const uint64_t c[4] = {c0.x, c0.y, c1.x, c1.y};
-#pragma unroll
-      for (int i = 0; i < 8; i++) {
-#pragma unroll
-        for (int j = 0; j < 4; j++) { acc[i][j] = fma2(c[j], x[i], acc[i][j]); }
+        for (uint32_t e = 0; e < 4; e++) {
+          const bool in = k0 + lk + e < kdim;
+          ra[e]         = in && in_a ? __ldg(pa + k0 + e) : 0.0f;
+          rb[e]         = in && in_b ? __ldg(pb + k0 + e) : 0.0f;
+        }
       }
     };
-    if (kn == kTileK) {
+    auto store = [&](uint32_t buf) {
 #pragma unroll
-      for (uint32_t k = 0; k < kTileK; k++) { step(k); }
-    } else {
-      for (uint32_t k = 0; k < kn; k++) { step(k); }
-    }
-    if (more) {
-      store(buf ^ 1u);
-      __syncthreads();
-    }
-  }
-#pragma unroll
-  for (int i = 0; i < 8; i++) {
-    const uint32_t row = i0 + (i < 4 ? ty * 4u + i : 64u + ty * 4u + (i - 4));
-    [[maybe_unused]] unsigned long long m = ~0ull;
-#pragma unroll
-    for (int h = 0; h < 2; h++) {
-      const uint32_t col = j0 + h * 64u + tx * 4u;
-      float v[4];
-#pragma unroll
-      for (int e = 0; e < 4; e++) {
-        const uint64_t pair = acc[i][h * 2 + (e >> 1)];
-        v[e] = __fmul_rn(alpha, __uint_as_float(uint32_t((e & 1) ? (pair >> 32) : pair)));
-        // fp16 coarse search: the score is a half-precision number
-        if (half_scores) { v[e] = __half2float(__float2half_rn(v[e])); }
+      for (uint32_t e = 0; e < 4; e++) {
+        s_a[buf][lk + e][lrow] = ra[e];
+        s_b[buf][lk + e][lrow] = rb[e];
       }
-      if constexpr (kArgmin) {
+    };
+    // rows ty * 4 + {0..3} and 64 + ..., columns tx * 4 + {0..3} and 64 + ...
+    uint64_t acc[8][4];
+#pragma unroll
+    for (int i = 0; i < 8; i++) {
+#pragma unroll
+      for (int j = 0; j < 4; j++) { acc[i][j] = 0ull; }
+    }
+    load(0);
+    store(0);
+    __syncthreads();
+    uint32_t buf = 0;
+    for (uint32_t k0 = 0; k0 < kdim; k0 += kTileK, buf ^= 1u) {
+      const bool more = k0 + kTileK < kdim;
+      if (more) { load(k0 + kTileK); }
+      // (a partial last tile stops at kdim: a product with zero would leave the chain's value alone, except for -0 and
+      // infinities)
+      const uint32_t kn = min(kTileK, kdim - k0);
+      auto step = [&](uint32_t k) {
+        const float4 x0 = *reinterpret_cast<const float4*>(&s_a[buf][k][ty * 4u]);
+        const float4 x1 = *reinterpret_cast<const float4*>(&s_a[buf][k][64u + ty * 4u]);
+        const ulonglong2 c0 = *reinterpret_cast<const ulonglong2*>(&s_b[buf][k][tx * 4u]);
+        const ulonglong2 c1 = *reinterpret_cast<const ulonglong2*>(&s_b[buf][k][64u + tx * 4u]);
+        const uint64_t x[8] = {dup2(x0.x), dup2(x0.y), dup2(x0.z), dup2(x0.w), dup2(x1.x), dup2(x1.y), dup2(x1.z), dup2(x1.w)};
+        const uint64_t c[4] = {c0.x, c0.y, c1.x, c1.y};
+#pragma unroll
+        for (int i = 0; i < 8; i++) {
+#pragma unroll
+          for (int j = 0; j < 4; j++) { acc[i][j] = fma2(c[j], x[i], acc[i][j]); }
+        }
+      };
+      if (kn == kTileK) {
+#pragma unroll
+        for (uint32_t k = 0; k < kTileK; k++) { step(k); }
+      } else {
+        for (uint32_t k = 0; k < kn; k++) { step(k); }
+      }
+      if (more) {
+        store(buf ^ 1u);
+        __syncthreads();
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < 8; i++) {
+      const uint32_t row = i0 + (i < 4 ? ty * 4u + i : 64u + ty * 4u + (i - 4));
+      [[maybe_unused]] unsigned long long m = ~0ull;
+#pragma unroll
+      for (int h = 0; h < 2; h++) {
+        const uint32_t col = j0 + h * 64u + tx * 4u;
+        float v[4];
 #pragma unroll
         for (int e = 0; e < 4; e++) {
-          const unsigned long long key = ((unsigned long long)float_to_ordered(v[e]) << 32) | (col + e);
-          if (col + e < n_cols) { m = key < m ? key : m; }
+          const uint64_t pair = acc[i][h * 2 + (e >> 1)];
+          v[e] = __fmul_rn(alpha, __uint_as_float(uint32_t((e & 1) ? (pair >> 32) : pair)));
+          // fp16 coarse search: the score is a half-precision number
+          if (half_scores) { v[e] = __half2float(__float2half_rn(v[e])); }
         }
-      } else if (row < n_rows) {
-        float* o = out + size_t(row) * n_cols + col;
-        if (n_cols % 4 == 0 && col < n_cols) {
-          *reinterpret_cast<float4*>(o) = make_float4(v[0], v[1], v[2], v[3]);
-        } else {
+        if constexpr (kArgmin) {
 #pragma unroll
           for (int e = 0; e < 4; e++) {
-            if (col + e < n_cols) { o[e] = v[e]; }
+            const unsigned long long key = ((unsigned long long)float_to_ordered(v[e]) << 32) | (col + e);
+            if (col + e < n_cols) { m = key < m ? key : m; }
+          }
+        } else if (row < n_rows) {
+          float* o = out + size_t(row) * n_cols + col;
+          if (n_cols % 4 == 0 && col < n_cols) {
+            *reinterpret_cast<float4*>(o) = make_float4(v[0], v[1], v[2], v[3]);
+          } else {
+#pragma unroll
+            for (int e = 0; e < 4; e++) {
+              if (col + e < n_cols) { o[e] = v[e]; }
+            }
           }
         }
       }
-    }
-    if constexpr (kArgmin) {
-      // eight lanes of a warp share a row: reduce before touching memory
+      if constexpr (kArgmin) {
+        // eight lanes of a warp share a row: reduce before touching memory
 #pragma unroll
-      for (int d = 4; d > 0; d >>= 1) {
-        const unsigned long long o = __shfl_xor_sync(kFullMask, m, d);
-        m = o < m ? o : m;
+        for (int d = 4; d > 0; d >>= 1) {
+          const unsigned long long o = __shfl_xor_sync(kFullMask, m, d);
+          m = o < m ? o : m;
+        }
+        if ((tid & 7u) == 0 && row < n_rows) { atomicMin(best + (kListed ? __ldg(row_list + row) : row), m); }
       }
-      if ((tid & 7u) == 0 && row < n_rows) { atomicMin(best + (row_list != nullptr ? __ldg(row_list + row) : row), m); }
     }
-  }
+    if constexpr (kListed) {
+      __syncthreads();
+      i0 += gridDim.y * kTile;
+    }
+  } while (kListed && i0 < n_rows);
 }
 
 // The same product for a few rows (at most kFewRows), where the tiles above would leave the chip empty and the time is
@@ -218,7 +223,7 @@ few_rows_kernel(const float* __restrict__ b, uint32_t n_cols, const float* __res
   }
 }
 
-template <bool kArgmin>
+template <bool kArgmin, bool kListed = false>
 void launch_exact_gemm(const float* b, uint32_t n_cols, const float* a, uint32_t n_rows, uint32_t a_stride, uint32_t kdim, float alpha,
                        bool half_scores, float* out, unsigned long long* best, cudaStream_t stream,
                        const uint32_t* row_list = nullptr, const uint32_t* n_listed = nullptr)
@@ -237,17 +242,20 @@ void launch_exact_gemm(const float* b, uint32_t n_cols, const float* a, uint32_t
   const uint32_t most = 65535u * kTile;
   for (uint32_t r0 = 0; r0 < n_rows; r0 += most) {
     const uint32_t nr = std::min(most, n_rows - r0);
-    const dim3 grid(ceildiv(n_cols, kTile), ceildiv(nr, kTile));
+    dim3 grid(ceildiv(n_cols, kTile), ceildiv(nr, kTile));
+    // some eight blocks per SM: 4,096 x 128 blocks that found nothing to do took 0.6 ms
+    if (kListed) { grid.y = std::min(grid.y, ceildiv(1184u, grid.x)); }
     const float* ar = a + size_t(r0) * a_stride;
     float* o        = out ? out + size_t(r0) * n_cols : nullptr;
     unsigned long long* bs = best ? best + r0 : nullptr;
     const bool vec = kdim % 4 == 0 && a_stride % 4 == 0 && ((reinterpret_cast<uintptr_t>(b) | reinterpret_cast<uintptr_t>(ar)) & 15u) == 0;
+    auto go = [&](auto kernel) {
+      launch_chained(kernel, grid, 256, 0, stream, b, n_cols, ar, nr, a_stride, kdim, alpha, half_scores, o, bs, row_list, n_listed);
+    };
     if (vec) {
-      launch_chained(exact_gemm_kernel<true, kArgmin>, grid, 256, 0, stream, b, n_cols, ar, nr, a_stride, kdim, alpha,
-                     half_scores, o, bs, row_list, n_listed);
+      go(exact_gemm_kernel<true, kArgmin, kListed>);
     } else {
-      launch_chained(exact_gemm_kernel<false, kArgmin>, grid, 256, 0, stream, b, n_cols, ar, nr, a_stride, kdim, alpha,
-                     half_scores, o, bs, row_list, n_listed);
+      go(exact_gemm_kernel<false, kArgmin, kListed>);
     }
     CUDA_TRY(cudaGetLastError());
   }
@@ -463,6 +471,7 @@ __global__ void unpack_labels_kernel(const unsigned long long* __restrict__ best
                                      const uint32_t* __restrict__ row_list, const uint32_t* __restrict__ n_listed,
                                      uint32_t* __restrict__ labels)
 {
+  chain_begin();
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= (row_list != nullptr ? min(n, __ldg(n_listed)) : n)) { return; }
   const uint32_t r = row_list != nullptr ? __ldg(row_list + i) : i;
@@ -544,9 +553,9 @@ void assign_nearest_listed(raft::resources& res, const float* centers, uint32_t 
                            uint32_t* labels, unsigned long long* best)
 {
   CUVS_EXPECTS(n_rows <= 65535u * kTile, "too many rows");
-  CUDA_TRY(cudaMemsetAsync(best, 0xFF, size_t(n_rows) * 8, res.stream));
-  launch_exact_gemm<true>(centers, n_lists, x_ext, n_rows, dim_ext, dim_ext, alpha, false, nullptr, best, res.stream, row_list, n_listed);
-  unpack_labels_kernel<<<ceildiv<uint32_t>(n_rows, 256), 256, 0, res.stream>>>(best, n_rows, row_list, n_listed, labels);
+  launch_exact_gemm<true, true>(centers, n_lists, x_ext, n_rows, dim_ext, dim_ext, alpha, false, nullptr, best, res.stream, row_list,
+                                n_listed);
+  launch_chained(unpack_labels_kernel, ceildiv<uint32_t>(n_rows, 256), 256, 0, res.stream, best, n_rows, row_list, n_listed, labels);
   CUDA_TRY(cudaGetLastError());
   res.launches += 2;
 }

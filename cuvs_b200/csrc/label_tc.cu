@@ -3,27 +3,28 @@
 //
 // Reference: kmeans_balanced::predict (cpp/src/cluster/detail/kmeans_balanced.cuh:100-160).
 //
-// The probe selection of coarse_tc.cu with n_probes = 1 answers the same question, but keeps eight keys of every 64
-// lists in global memory and finishes with a block per row: 12 of 23 ms for 1 M rows x 16,384 lists.  For the nearest list
-// alone, one maximum per 64 lists is enough:
+// For the nearest list alone, one maximum per few lists is enough:
 //   1. operands in half precision (the same 11 significant bits as TF32 at twice the rate), relative to the mean m of the
-//      centres: rows (q - m) 2^e, lists (c - m) / cp, with cp the power of two above the largest |c - m|; two more
-//      columns carry |c|^2 / 2 - m.c + |m|^2 / 2, so that the accumulator holds F (score + a constant of the row), F = 2^e /
-//      cp, within (-0.5, 0.5).  `eps` of a row bounds how far that is from the exact value: the measured norms of what
-//      rounding took from row and lists, accumulation, the defining chain's own rounding, the rounding of the keys.
-//      Up to 190 dimensions (where both fit shared memory beside three list stages) the row operand comes as two halfs, hi +
-//      lo, and two products: its rounding drops out of eps.  The second product is on the critical path: at 96 dimensions the
-//      MMA thread issues the 14 products of a tile in about 3,400 clocks, the epilogue needs 2,200.
-//   2. label_tc_kernel: a persistent CTA takes a tile of 128 rows against all (or a share) of the lists, 256 at a time.
-//      Per row and unit of 64 lists the epilogue finds the largest value as a packed key (value in fixed point, low bits
-//      the column: see coarse_tc.cu) and the second largest; across the tiles it keeps, per row and column quarter, the
-//      units with the four largest.  Three float additions and three min / max per value; the issue of the MMAs bounds the
-//      kernel.
-//   3. label_finish_kernel: units within 2 eps of the largest value are looked at.  One such unit whose second value is
-//      outside: that is the label.  Several: their lists are rescored with the defining chain.  Units whose second value
-//      is inside too go to label_units_kernel, which rescores all 64 lists of them.  If the fourth unit kept is inside,
-//      a fifth might be: the row is redone exactly over all lists.
+//      centres: rows (q - m) 2^e, lists (c - m) / cp, with cp the power of two above the largest |c - m|, so that products lie
+//      within (-0.5, 0.5); the epilogue subtracts the list's norm term |c|^2 / 2 - m.c + |m|^2 / 2 times a factor of the row,
+//      which gives F (score + a constant of the row).  The bounds of a row say how far that can be from the exact value: the
+//      measured norms of what rounding took from row and lists, accumulation, the defining chain's own rounding, the keys.
+//   2. label_tc_kernel: a persistent CTA takes a tile of 256 rows against all (or a share) of the lists, 256 at a time: two
+//      accumulators of 128 rows, so that a list tile is read once for both and the epilogue of one runs beside the products of
+//      the other.  Per row and unit of 8 lists the epilogue finds the largest value (its low bits replaced by the unit's
+//      number); across the tiles it keeps, per row and column quarter, the four largest: 1.3 comparisons per value.
+//   3. label_finish_kernel looks at the units within 2 eps of the largest value: first their operands' products in fp32, then
+//      what is left in ever finer sums, the defining chain last.
+//   4. If the fourth unit kept is inside, a fifth might be: such rows (2.7% of 1 M rows x 16,384 lists of 96 dimensions) go
+//      through 2 and 3 once more with the lists in eight shares; only what that does not settle is redone exactly over all lists.
+// What bounds label_tc_kernel: the issue and execution of the MMAs (1,300 clocks per 128 x 256 x 96; the products alone take 880),
+// then the comparisons (740).  1,000,003 rows x 16,384 lists x 96 dimensions, all of the labelling: 9.4 ms with two products
+// (row operand as two halfs), units of 64 lists whose largest two values were kept with their columns, and 2% of the rows
+// redone over all lists; 3.8 ms so.  (One product widens the bounds from 5.2e-5 to 6.5e-5: 2.6 instead of 2.2 lists within
+// reach.)
 // Every wait is bounded: on a time-out the kernel raises the error word and returns, and all rows are redone.
+#include "common.hpp"
+#include "packed.cuh"
 #include "search_internal.hpp"
 #include "tc_ptx.cuh"
 #include "topk.cuh"
@@ -36,17 +37,32 @@ using namespace cuvs_b200;
 
 namespace {
 
-constexpr uint32_t kRows = 128, kLists = 256, kBlockK = 64, kUnit = 64, kKeep = 4;
+constexpr uint32_t kRows = 128, kTileRows = 2 * kRows, kLists = 256, kBlockK = 64, kUnit = 8, kKeep = 4;
+constexpr uint32_t kUnitsPerTile = 64 / kUnit;        // units of a tile in one column quarter
+constexpr uint32_t kSplitTiles   = 64;                // most list tiles of an item: nine bits number its units
 constexpr uint32_t kEpiWarps = 16;
 constexpr uint32_t kThreads  = (2 + kEpiWarps) * 32;  // warp 0 TMA, warp 1 MMA, warps 2..17 epilogue
 constexpr uint32_t kABlock = kRows * kBlockK * 2, kBBlock = kLists * kBlockK * 2;  // 16 and 32 KB
-constexpr uint32_t kMaxStages = 6;
 constexpr uint32_t kRoom      = 6 * kBBlock;          // shared memory for operands: 192 KB
+constexpr uint32_t kMaxStages = 4;
+constexpr uint32_t kNormSlots = 8;                    // list tiles whose norm terms are on hand
+constexpr uint32_t kNormBytes = kLists * 4;
+constexpr float kNoList       = 1e30f;                // norm term of a list that is not there
 
 // Model: words {bits of the largest max(|c - m|^2, 2 |norm column|), of the largest |c|^2 or norm column, of the largest
-// squared norm of what rounding took from a list}, the sum of the centres at kMeanAt, the list operand at operand_at(dim).
+// squared norm of what rounding took from a list}, the sum of the centres at kMeanAt, the lists' norm terms at norms_at(dim) (whole
+// tiles of them), the list operand behind, and once more by units at unit_operand_at: [units][width / 8][8 lists] 16-byte chunks.
 constexpr uint32_t kMeanAt = 256;
-__host__ __device__ __forceinline__ size_t operand_at(uint32_t dim) { return kMeanAt + round_up<size_t>(size_t(dim) * 4, 256); }
+__host__ __device__ __forceinline__ size_t norms_at(uint32_t dim) { return kMeanAt + round_up<size_t>(size_t(dim) * 4, 256); }
+__host__ __device__ __forceinline__ size_t operand_at(uint32_t n_lists, uint32_t dim)
+{
+  return norms_at(dim) + size_t(round_up(n_lists, kLists)) * 4;
+}
+
+__host__ __device__ __forceinline__ size_t unit_operand_at(uint32_t n_lists, uint32_t dim, uint32_t width)
+{
+  return operand_at(n_lists, dim) + round_up<size_t>(size_t(n_lists) * width * 2, 256);
+}
 
 __global__ void center_sum_kernel(const float* __restrict__ centers, uint32_t n_lists, uint32_t dim, uint32_t dim_ext,
                                   float* __restrict__ sum)
@@ -117,61 +133,108 @@ __device__ __forceinline__ float center_scale(const uint32_t* words, float& bn)
   return cp;
 }
 
-// One warp per list.
+// One warp per list (of whole tiles: there is nothing in those beyond the last one but their norm terms).
 __global__ void center_operand_kernel(const float* __restrict__ centers, uint32_t n_lists, uint32_t dim, uint32_t dim_ext,
                                       uint32_t width, const float* __restrict__ sum, uint32_t* __restrict__ words,
-                                      __half* __restrict__ out)
+                                      float* __restrict__ norms, __half* __restrict__ out, __half* __restrict__ by_unit)
 {
   const uint32_t l = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31u;
-  if (l >= n_lists) { return; }
+  if (l >= n_lists) {
+    if (l < round_up(n_lists, kLists) && lane == 0) { norms[l] = kNoList; }
+    return;
+  }
   float bn, cc, dd;
   const float inv   = 1.0f / center_scale(words, bn);
   const float inv_n = 1.0f / float(n_lists);
   const float* c    = centers + size_t(l) * dim_ext;
   double norm;
   list_norms(c, sum, inv_n, dim, cc, dd, norm);
-  const float nf = float(norm * double(inv) * double(inv));
-  const float hi = __half2float(__float2half_rn(nf));
   __half* dst    = out + size_t(l) * width;
   float lost     = 0.0f;
   for (uint32_t k = lane; k < width; k += 32) {
-    const float v  = k < dim ? (c[k] - sum[k] * inv_n) * inv : (k == dim ? hi : (k == dim + 1 ? nf - hi : 0.0f));
+    const float v  = k < dim ? (c[k] - sum[k] * inv_n) * inv : 0.0f;
     const __half h = __float2half_rn(v);
     dst[k]         = h;
-    if (k < dim) {
-      const float d = v - __half2float(h);
-      lost          = __fmaf_rn(d, d, lost);
-    }
+    by_unit[((size_t(l / kUnit) * (width / 8u) + k / 8u) * kUnit + l % kUnit) * 8u + (k & 7u)] = h;
+    const float d  = v - __half2float(h);
+    lost           = __fmaf_rn(d, d, lost);
   }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) { lost += __shfl_xor_sync(kFullMask, lost, o); }
-  if (lane == 0) { atomicMax(words + 2, __float_as_uint(lost * 1.001f)); }
+  if (lane == 0) {
+    atomicMax(words + 2, __float_as_uint(lost * 1.001f));
+    norms[l] = float(norm * double(inv) * double(inv));
+  }
 }
 
-// One warp per row: the operand row (kSplit: hi, then lo, `width` halfs each), and eps (infinite: redo the row).
-template <bool kSplit>
-__global__ void row_operand_kernel(const float* __restrict__ x, uint32_t n_rows, uint32_t n_lists, uint32_t dim, uint32_t dim_ext,
-                                   uint32_t width, const float* __restrict__ sum, const uint32_t* __restrict__ words,
-                                   __half* __restrict__ out, float* __restrict__ eps)
+// Eight lanes per row: the operand row, the factor of the lists' norm terms, and three bounds: {of a key, of a sum of the half-precision operands in fp32, of the
+// defining chain and of any other fp32 sum of its products, the last in units of the chain} (infinite: the row is redone).
+// What bounds it: memory (dim_ext floats in, `width` halfs out).  A warp per row spent its time on the arithmetic of the
+// bounds: 161 us for 524,288 rows of 96 dimensions.  kRegs: the row stays in registers (width <= 128).
+template <bool kRegs>
+__global__ void __launch_bounds__(256)
+row_operand_kernel(const float* __restrict__ x, uint32_t n_rows, uint32_t n_lists, uint32_t dim, uint32_t dim_ext, uint32_t width,
+                   const float* __restrict__ sum, const uint32_t* __restrict__ words, float key_error, __half* __restrict__ out,
+                   float* __restrict__ factor, float4* __restrict__ eps, uint4* __restrict__ clear)
 {
-  const uint32_t r    = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const uint32_t lane = threadIdx.x & 31u;
+  chain_begin();
+  if (blockIdx.x == 0 && threadIdx.x == 0) { *clear = make_uint4(0u, 0u, 0u, 0u); }  // errors and counts of the kernels behind
+  const uint32_t r    = (blockIdx.x * blockDim.x + threadIdx.x) >> 3;
+  const uint32_t lane = threadIdx.x & 7u;
+  const unsigned mask = 0xFFu << (threadIdx.x & 24u);
   if (r >= n_rows) { return; }
-  float bn;
-  const float cp    = center_scale(words, bn);
   const float inv_n = 1.0f / float(n_lists);
-  const float* q    = x + size_t(r) * dim_ext;
-  float ss = 0.0f, qq = 0.0f;
-  for (uint32_t k = lane; k < dim; k += 32) {
-    const float v = q[k], d = v - sum[k] * inv_n;
-    ss = __fmaf_rn(d, d, ss);
-    qq = __fmaf_rn(v, v, qq);
-  }
+  const float4* q   = reinterpret_cast<const float4*>(x + size_t(r) * dim_ext);  // dim_ext is a multiple of 8
+  constexpr uint32_t kIters = kRegs ? 4u : 1u;
+  float4 a4[kIters];
+  if constexpr (kRegs) {
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    ss += __shfl_xor_sync(kFullMask, ss, o);
-    qq += __shfl_xor_sync(kFullMask, qq, o);
+    for (uint32_t i = 0; i < kIters; i++) {
+      const uint32_t k = lane * 4u + i * 32u;
+      a4[i]            = k < dim_ext ? __ldg(q + (k >> 2)) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    }
   }
+  // four components of the row and of its difference to the mean (zero from `dim` on)
+  auto load = [&](uint32_t k, uint32_t i, float (&v)[4], float (&d)[4]) {
+    float4 a;
+    if constexpr (kRegs) {
+      a = a4[i];
+    } else {
+      a = k < dim_ext ? __ldg(q + (k >> 2)) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    }
+    v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
+#pragma unroll
+    for (uint32_t e = 0; e < 4; e++) {
+      const bool in = k + e < dim;
+      v[e]          = in ? v[e] : 0.0f;
+      d[e]          = in ? v[e] - __ldg(sum + k + e) * inv_n : 0.0f;
+    }
+  };
+  auto steps = [&](auto&& fn) {
+    if constexpr (kRegs) {
+#pragma unroll
+      for (uint32_t i = 0; i < kIters; i++) { fn(lane * 4u + i * 32u, i); }
+    } else {
+      for (uint32_t k = lane * 4u; k < width; k += 32u) { fn(k, 0u); }
+    }
+  };
+  float ss = 0.0f, qq = 0.0f;
+  steps([&](uint32_t k, uint32_t i) {
+    float v[4], d[4];
+    load(k, i, v, d);
+#pragma unroll
+    for (uint32_t e = 0; e < 4; e++) {
+      ss = __fmaf_rn(d[e], d[e], ss);
+      qq = __fmaf_rn(v[e], v[e], qq);
+    }
+  });
+#pragma unroll
+  for (int o = 4; o > 0; o >>= 1) {
+    ss += __shfl_xor_sync(mask, ss, o);
+    qq += __shfl_xor_sync(mask, qq, o);
+  }
+  float bn;
+  const float cp = center_scale(words, bn);
   const float dn = sqrtf(ss) * 1.0001f, qn = sqrtf(qq) * 1.0001f;
   // 2^e (|q - m| + cp / 2) in [0.25, 0.5)
   const float b     = (dn + 0.5f * cp) * 1.01f;
@@ -179,86 +242,111 @@ __global__ void row_operand_kernel(const float* __restrict__ x, uint32_t n_rows,
   const bool fine   = E >= 2 && E <= 250;
   const float scale = fine ? __uint_as_float(uint32_t(252 - E) << 23) : 0.0f;
   const float a     = scale * cp;
-  __half2* dst      = reinterpret_cast<__half2*>(out + size_t(r) * width * (kSplit ? 2u : 1u));
   float lost        = 0.0f;
-  for (uint32_t k2 = lane; k2 < width / 2; k2 += 32) {
-    float v[2];
+  steps([&](uint32_t k, uint32_t i) {
+    float v[4], d[4];
+    load(k, i, v, d);
 #pragma unroll
-    for (uint32_t e = 0; e < 2; e++) {
-      const uint32_t k = 2 * k2 + e;
-      v[e]             = k < dim ? (q[k] - sum[k] * inv_n) * scale : (k < dim + 2 ? -a : 0.0f);
-    }
-    const __half2 h = __floats2half2_rn(v[0], v[1]);
-    float2 f        = __half22float2(h);
-    dst[k2]         = h;
-    f               = make_float2(v[0] - f.x, v[1] - f.y);
-    if constexpr (kSplit) {
-      const __half2 lo     = __floats2half2_rn(f.x, f.y);
-      const float2 g       = __half22float2(lo);
-      dst[width / 2 + k2] = lo;
-      f                    = make_float2(f.x - g.x, f.y - g.y);
-    }
-    lost = __fmaf_rn(f.x, f.x, lost);
-    lost = __fmaf_rn(f.y, f.y, lost);
-  }
+    for (uint32_t e = 0; e < 4; e++) { d[e] *= scale; }
+    const __half2 h0 = __floats2half2_rn(d[0], d[1]), h1 = __floats2half2_rn(d[2], d[3]);
+    const float2 f0 = __half22float2(h0), f1 = __half22float2(h1);
+    d[0] -= f0.x; d[1] -= f0.y; d[2] -= f1.x; d[3] -= f1.y;
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) { lost += __shfl_xor_sync(kFullMask, lost, o); }
+    for (uint32_t e = 0; e < 4; e++) { lost = __fmaf_rn(d[e], d[e], lost); }
+    uint2 w;
+    w.x = *reinterpret_cast<const uint32_t*>(&h0);
+    w.y = *reinterpret_cast<const uint32_t*>(&h1);
+    if (k < width) { *reinterpret_cast<uint2*>(out + size_t(r) * width + k) = w; }  // width is a multiple of 16
+  });
+#pragma unroll
+  for (int o = 4; o > 0; o >>= 1) { lost += __shfl_xor_sync(mask, lost, o); }
   if (lane == 0) {
     const float an = dn * scale, w = float(width);
     const float bl = sqrtf(__uint_as_float(__ldg(words + 2))), cn = sqrtf(__uint_as_float(__ldg(words + 1)));
-    const float orig = qn * cn + 0.5f * cn * cn;  // bounds every partial sum of the defining chain
-    float e = (sqrtf(lost) * (bn + bl) + an * bl) * 1.01f       // rounding of the operands
-              + (w + 24.0f) * (kSplit ? 1.8e-7f : 1.2e-7f)      // accumulation of sums below 0.5 by the tensor core
-              + (scale / cp) * orig * (float(dim_ext) + 4.0f) * 1.2e-7f  // the defining chain, and q - m
-              + 8.2e-6f;                                        // norm columns, keys
+    const float orig  = qn * cn + 0.5f * cn * cn;  // bounds every partial sum of the defining chain
+    const float chain = orig * (float(dim_ext) + 4.0f) * 1.2e-7f;
+    float e = (sqrtf(lost) * (bn + bl) + an * bl) * 1.01f  // rounding of the operands
+              + (scale / cp) * chain                       // the defining chain, and q - m
+              + 0.6e-6f;                                   // norm terms
     if (!fine || !(a >= 6.2e-5f)) { e = INFINITY; }
-    eps[r] = e;
+    // accumulation of sums below 0.5 by the tensor core, and in fp32
+    factor[r] = a;
+    eps[r] = make_float4(e + (w + 24.0f) * 1.2e-7f + key_error, e + w * 6.1e-8f, chain, 0.0f);
+  }
+}
+
+// Operand rows and factors of the listed rows, one after the other.  One warp per row at a time.
+__global__ void __launch_bounds__(256)
+gather_operand_kernel(const __half* __restrict__ a, const float* __restrict__ factor, const uint32_t* __restrict__ rows,
+                      const uint32_t* __restrict__ count, uint32_t cap, uint32_t width, __half* __restrict__ out,
+                      float* __restrict__ factor_out)
+{
+  chain_begin();
+  const uint32_t n = min(__ldg(count), cap), lane = threadIdx.x & 31u;
+  for (uint32_t i = (blockIdx.x * 256u + threadIdx.x) >> 5; i < n; i += gridDim.x * 8u) {
+    const uint32_t r = __ldg(rows + i);
+    const uint4* src = reinterpret_cast<const uint4*>(a + size_t(r) * width);
+    uint4* dst       = reinterpret_cast<uint4*>(out + size_t(i) * width);
+    for (uint32_t c = lane; c < width / 8u; c += 32u) { dst[c] = __ldg(src + c); }
+    if (lane == 0) { factor_out[i] = __ldg(factor + r); }
   }
 }
 
 struct label_params {
-  uint32_t n_rows, n_lists, k_steps /* of 16 halfs */, k_blocks;
-  uint32_t n_tiles, tiles_per_split, n_items, splits;
-  uint32_t a_resident, n_stages, products, width;
-  uint4* keys;       // [splits, n_rows, 4] largest keys of a column quarter
-  uint4* seconds;    // second largest keys of their units
-  uint4* lists;      // their lists
+  uint32_t n_rows;       // rows of the operand (and of `keys`)
+  const uint32_t* count; // where given: only so many of them count
+  uint32_t k_steps /* of 16 halfs */, k_blocks;
+  uint32_t n_tiles, tiles_per_split, splits;
+  uint32_t tag_mask;     // low bits of a key: number of the unit among those of an item's column quarter
+  const float* norms;    // of the lists, whole tiles
+  const float* factor;   // of the rows
+  float4* keys;          // [splits, n_rows, 4] largest keys of a column quarter
   uint32_t* error;
   uint32_t spin_limit, skip_kb;  // tc_wait_limits
 };
 
+// kKB: K blocks of 64 halfs; up to three of both halves of the row tile stay in shared memory beside a ring of kSlots list
+// tiles.  0: any number, row blocks stream beside the list blocks.
+template <uint32_t kKB>
 __global__ void __launch_bounds__(kThreads, 1)
 label_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, const label_params p)
 {
+  constexpr bool kResident   = kKB > 0;
+  constexpr uint32_t kSlots  = kKB == 1 ? 4u : (kKB == 2 ? 2u : 1u);
+  constexpr uint32_t kStages = kResident ? kSlots * kKB : kRoom / (2 * kABlock + kBBlock);
+  static_assert(kStages <= kMaxStages && kKB * (2 * kABlock + kSlots * kBBlock) <= kRoom, "shared memory");
+  // [row tile, when resident: two halves of kKB blocks][stages: list block, then the two row blocks when not][norm terms]
+  constexpr uint32_t kABytes    = kResident ? 2u * kKB * kABlock : 0u;
+  constexpr uint32_t kStageSize = kBBlock + (kResident ? 0u : 2u * kABlock);
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw_a  = smem_u32(smem_raw);
   const uint32_t base_a = (raw_a + 1023u) & ~1023u;
   uint8_t* base_p       = smem_raw + (base_a - raw_a);
-  uint64_t* bars        = reinterpret_cast<uint64_t*>(base_p + kRoom);
+  uint64_t* bars        = reinterpret_cast<uint64_t*>(base_p + kRoom + kNormSlots * kNormBytes);
   const uint32_t bar_full   = smem_u32(bars);
   const uint32_t bar_empty  = bar_full + kMaxStages * 8;
   const uint32_t bar_tfull  = bar_empty + kMaxStages * 8;
   const uint32_t bar_tempty = bar_tfull + 2 * 8;
   const uint32_t bar_afull  = bar_tempty + 2 * 8;
   const uint32_t bar_aempty = bar_afull + 8;
-  uint32_t* tmem_slot       = reinterpret_cast<uint32_t*>(bars + 2 * kMaxStages + 6);
-  // [row tile, when resident][stages: list block, then row block when not]
-  const uint32_t a_bytes    = p.a_resident ? p.products * p.k_blocks * kABlock : 0u;
-  const uint32_t stage_size = kBBlock + (p.a_resident ? 0u : kABlock);
-  const uint32_t stage_base = base_a + a_bytes;
+  const uint32_t bar_norms  = bar_aempty + 8;
+  uint32_t* tmem_slot       = reinterpret_cast<uint32_t*>(bars + 2 * kMaxStages + 6 + kNormSlots);
+  const uint32_t stage_base = base_a + kABytes;
+  const uint32_t norm_base  = base_a + kRoom;
   const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
 
   if (threadIdx.x == 0) {
-    for (uint32_t s = 0; s < p.n_stages; s++) {
+    for (uint32_t s = 0; s < kStages; s++) {
       mbar_init(bar_full + s * 8, 1);
       mbar_init(bar_empty + s * 8, 1);
     }
     for (uint32_t a = 0; a < 2; a++) {
       mbar_init(bar_tfull + a * 8, 1);
-      mbar_init(bar_tempty + a * 8, kEpiWarps);
+      mbar_init(bar_tempty + a * 8, kEpiWarps / 2);
     }
     mbar_init(bar_afull, 1);
     mbar_init(bar_aempty, 1);
+    for (uint32_t s = 0; s < kNormSlots; s++) { mbar_init(bar_norms + s * 8, 1); }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 1) {
@@ -269,7 +357,11 @@ label_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  chain_begin();
   const uint32_t tmem_base = *reinterpret_cast<volatile uint32_t*>(tmem_slot);
+  const uint32_t n_rows    = p.count != nullptr ? min(__ldg(p.count), p.n_rows) : p.n_rows;
+  const uint32_t n_items   = ceildiv(n_rows, kTileRows) * p.splits;
+  const uint32_t k_blocks  = kResident ? kKB : p.k_blocks;
   bool ok = true;
   // the list tiles of an item
   auto tiles_of = [&](uint32_t item, uint32_t& t0, uint32_t& t1) {
@@ -281,38 +373,48 @@ label_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
   if (warp == 0) {
     // ---------------- TMA producer ----------------
     if (lane == 0) {
-      uint32_t stage = 0, phase = 0, n_a = 0;
-      for (uint32_t item = blockIdx.x; ok && item < p.n_items; item += gridDim.x) {
-        const int row0 = int((item / p.splits) * kRows);
+      uint32_t stage = 0, phase = 0, n_a = 0, it = 0;
+      for (uint32_t item = blockIdx.x; ok && item < n_items; item += gridDim.x) {
+        const int row0 = int((item / p.splits) * kTileRows);
         uint32_t t0, t1;
         tiles_of(item, t0, t1);
-        if (p.a_resident) {
+        if constexpr (kResident) {
           if (!mbar_wait(bar_aempty, (n_a & 1u) ^ 1u, p.spin_limit)) {
             ok = false;
             break;
           }
           n_a++;
-          mbar_arrive_expect_tx(bar_afull, a_bytes);
-          for (uint32_t i = 0; i < p.products; i++) {
-            for (uint32_t kb = 0; kb < p.k_blocks; kb++) {
-              tma_load_2d(base_a + (i * p.k_blocks + kb) * kABlock, &map_a, bar_afull, int(i * p.width + kb * kBlockK), row0);
+          mbar_arrive_expect_tx(bar_afull, kABytes);
+          for (uint32_t h = 0; h < 2; h++) {
+            for (uint32_t kb = 0; kb < kKB; kb++) {
+              tma_load_2d(base_a + (h * kKB + kb) * kABlock, &map_a, bar_afull, int(kb * kBlockK), row0 + int(h * kRows));
             }
           }
         }
-        for (uint32_t t = t0; ok && t < t1; t++) {
-          for (uint32_t kb = 0; kb < p.k_blocks; kb++) {
+        for (uint32_t t = t0; ok && t < t1; t++, it++) {
+          for (uint32_t kb = 0; kb < k_blocks; kb++) {
             if (!mbar_wait(bar_empty + stage * 8, phase ^ 1u, p.spin_limit)) {
               ok = false;
               break;
             }
-            const uint32_t dst = stage_base + stage * stage_size, bar = bar_full + stage * 8;
+            if (kb == 0) {
+              // the slot's last reader is kNormSlots tiles back, and the tile of the stage just freed, whose products wait
+              // for the epilogue of the one before, at most kSlots
+              const uint32_t slot = it % kNormSlots, bar = bar_norms + slot * 8;
+              mbar_arrive_expect_tx(bar, kNormBytes);
+              bulk_load(norm_base + slot * kNormBytes, p.norms + size_t(t) * kLists, kNormBytes, bar);
+            }
+            const uint32_t dst = stage_base + stage * kStageSize, bar = bar_full + stage * 8;
             // (test only: a block that never comes, so that the wait for it runs out)
             if (kb + 1 != p.skip_kb || t != t0 || item != blockIdx.x) {
-              mbar_arrive_expect_tx(bar, stage_size);
+              mbar_arrive_expect_tx(bar, kStageSize);
               tma_load_2d(dst, &map_b, bar, int(kb * kBlockK), int(t * kLists));
-              if (!p.a_resident) { tma_load_2d(dst + kBBlock, &map_a, bar, int(kb * kBlockK), row0); }
+              if constexpr (!kResident) {
+                tma_load_2d(dst + kBBlock, &map_a, bar, int(kb * kBlockK), row0);
+                tma_load_2d(dst + kBBlock + kABlock, &map_a, bar, int(kb * kBlockK), row0 + int(kRows));
+              }
             }
-            if (++stage == p.n_stages) {
+            if (++stage == kStages) {
               stage = 0;
               phase ^= 1u;
             }
@@ -323,146 +425,177 @@ label_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
     __syncwarp();
   } else if (warp == 1) {
     // ---------------- MMA issuer ----------------
-    if (lane == 0) {
-      // fp32 accumulate, half x half, both K-major, M = 128, N = 256
-      constexpr uint32_t idesc = (1u << 4) | ((kLists >> 3) << 17) | ((kRows >> 4) << 24);
-      uint32_t stage = 0, phase = 0, n_a = 0, it = 0;
-      for (uint32_t item = blockIdx.x; ok && item < p.n_items; item += gridDim.x) {
-        uint32_t t0, t1;
-        tiles_of(item, t0, t1);
-        if (p.a_resident) {
-          if (!mbar_wait(bar_afull, n_a & 1u, p.spin_limit)) {
-            ok = false;
-            break;
-          }
-          n_a++;
-        }
-        for (uint32_t t = t0; ok && t < t1; t++, it++) {
-          const uint32_t acc = it & 1u;
-          if (!mbar_wait(bar_tempty + acc * 8, ((it >> 1) & 1u) ^ 1u, p.spin_limit)) {
-            ok = false;
-            break;
-          }
-          tc_fence_after();
-          const uint32_t tmem_d = tmem_base + acc * kLists;
-          for (uint32_t kb = 0; kb < p.k_blocks; kb++) {
-            if (!mbar_wait(bar_full + stage * 8, phase, p.spin_limit)) {
-              ok = false;
-              break;
-            }
-            tc_fence_after();
-            const uint32_t sa = stage_base + stage * stage_size;
-            const uint32_t la = desc_sw128_lo(p.a_resident ? base_a + kb * kABlock : sa + kBBlock);
-            const uint32_t lb = desc_sw128_lo(sa);
-            const uint32_t nk = p.k_steps - kb * 4u;  // 32 bytes of K (2 descriptor units) per step
-            if (kb == 0) {
-              tc_mma_f16_lo<false>(tmem_d, la, lb, idesc);
-            } else {
-              tc_mma_f16_lo<true>(tmem_d, la, lb, idesc);
-            }
-            auto rest = [&](uint32_t a) {
-              if (nk >= 4u) {
-                tc_mma_f16_lo<true>(tmem_d, a + 2u, lb + 2u, idesc);
-                tc_mma_f16_lo<true>(tmem_d, a + 4u, lb + 4u, idesc);
-                tc_mma_f16_lo<true>(tmem_d, a + 6u, lb + 6u, idesc);
-              } else {
-                if (nk >= 2u) { tc_mma_f16_lo<true>(tmem_d, a + 2u, lb + 2u, idesc); }
-                if (nk >= 3u) { tc_mma_f16_lo<true>(tmem_d, a + 4u, lb + 4u, idesc); }
+    // (the warp goes through the loops as a whole; one lane issues: see elect_one)
+    // fp32 accumulate, half x half, both K-major, M = 128, N = 256
+    constexpr uint32_t idesc = (1u << 4) | ((kLists >> 3) << 17) | ((kRows >> 4) << 24);
+    const uint32_t tmem_d    = __shfl_sync(kFullMask, tmem_base, 0);
+    const uint32_t last_k    = p.k_steps - (k_blocks - 1u) * 4u;  // steps of the last K block
+    // the steps of one K block (32 bytes of K, 2 descriptor units, each)
+    auto block = [&](uint32_t d, uint32_t la, uint32_t lb, auto first, bool last) {
+      tc_mma_f16_lo<!decltype(first)::value>(d, la, lb, idesc);
+      if (!last || last_k >= 2u) { tc_mma_f16_lo<true>(d, la + 2u, lb + 2u, idesc); }
+      if (!last || last_k >= 3u) { tc_mma_f16_lo<true>(d, la + 4u, lb + 4u, idesc); }
+      if (!last || last_k >= 4u) { tc_mma_f16_lo<true>(d, la + 6u, lb + 6u, idesc); }
+    };
+    uint32_t stage = 0, phase = 0, n_a = 0, it = 0;
+    for (uint32_t item = blockIdx.x; ok && item < n_items; item += gridDim.x) {
+      uint32_t t0, t1;
+      tiles_of(item, t0, t1);
+      if constexpr (kResident) {
+        ok = mbar_wait_warp(bar_afull, n_a & 1u, p.spin_limit);
+        if (!ok) { break; }
+        n_a++;
+      }
+      for (uint32_t t = t0; t < t1; t++, it++) {
+        const uint32_t t_empty = (it & 1u) ^ 1u;
+        if constexpr (kResident) {
+          // one half of the rows after the other, both against the list blocks of the tile
+          const uint32_t slot = it % kSlots, full = (it / kSlots) & 1u;
+          const uint32_t lb   = desc_sw128_lo(stage_base) + slot * (kKB * kBBlock >> 4);
+          const uint32_t la   = desc_sw128_lo(base_a);
+          auto half = [&](auto hc) {
+            constexpr uint32_t h = decltype(hc)::value;
+            if (!mbar_wait_warp(bar_tempty + h * 8, t_empty, p.spin_limit)) { return false; }
+            bool fine = true;
+            static_for<kKB>([&](auto kc) {
+              constexpr uint32_t kb = decltype(kc)::value;
+              const uint32_t s      = slot * kKB + kb;
+              if (h == 0 && fine) { fine = mbar_wait_warp(bar_full + s * 8, full, p.spin_limit); }
+              if (!fine) { return; }
+              tc_fence_after();
+              if (elect_one()) {
+                block(tmem_d + h * kLists, la + (h * kKB + kb) * (kABlock >> 4), lb + kb * (kBBlock >> 4),
+                      std::integral_constant<bool, kb == 0>{}, kb + 1 == kKB);
+                if constexpr (h == 1) { tc_commit(bar_empty + s * 8); }
+                if constexpr (kb + 1 == kKB) { tc_commit(bar_tfull + h * 8); }
               }
-            };
-            rest(la);
-            if (p.products == 2u) {
-              const uint32_t ll = la + p.k_blocks * (kABlock >> 4);
-              tc_mma_f16_lo<true>(tmem_d, ll, lb, idesc);
-              rest(ll);
+              __syncwarp();
+            });
+            return fine;
+          };
+          ok = half(std::integral_constant<uint32_t, 0>{}) && half(std::integral_constant<uint32_t, 1>{});
+          if (!ok) { break; }
+        } else {
+          for (uint32_t kb = 0; kb < k_blocks; kb++) {
+            ok = mbar_wait_warp(bar_full + stage * 8, phase, p.spin_limit);
+            if (!ok) { break; }
+            const uint32_t sa = stage_base + stage * kStageSize;
+            for (uint32_t h = 0; h < 2; h++) {
+              if (kb == 0) {
+                ok = mbar_wait_warp(bar_tempty + h * 8, t_empty, p.spin_limit);
+                if (!ok) { break; }
+              }
+              tc_fence_after();
+              if (elect_one()) {
+                const uint32_t la = desc_sw128_lo(sa + kBBlock + h * kABlock), lb = desc_sw128_lo(sa);
+                if (kb == 0) {
+                  block(tmem_d + h * kLists, la, lb, std::true_type{}, kb + 1 == k_blocks);
+                } else {
+                  block(tmem_d + h * kLists, la, lb, std::false_type{}, kb + 1 == k_blocks);
+                }
+                if (kb + 1 == k_blocks) { tc_commit(bar_tfull + h * 8); }
+                if (h == 1) { tc_commit(bar_empty + stage * 8); }
+              }
+              __syncwarp();
             }
-            tc_commit(bar_empty + stage * 8);
-            if (++stage == p.n_stages) {
+            if (!ok) { break; }
+            if (++stage == kStages) {
               stage = 0;
               phase ^= 1u;
             }
           }
-          if (ok) { tc_commit(bar_tfull + acc * 8); }
+          if (!ok) { break; }
         }
-        if (ok && p.a_resident) { tc_commit(bar_aempty); }  // the row tile may be replaced once these MMAs are done
       }
+      // the row tile may be replaced once these MMAs are done
+      if (kResident && ok && elect_one()) { tc_commit(bar_aempty); }
+      __syncwarp();
     }
-    __syncwarp();
   } else {
-    // ---------------- epilogue: thread = row, warp = (lane quarter, 64 columns) ----------------
-    const uint32_t quarter = warp & 3u, unit = (warp - 2) >> 2;
+    // ---------------- epilogue: thread = row, warp = (half of the rows, half of the columns, lane quarter) ----------------
+    // (eight warps per accumulator, so that one half's loads run beside the other half's comparisons)
+    const uint32_t quarter = warp & 3u, side = ((warp - 2) >> 2) & 1u, h = (warp - 2) >> 3;
     uint32_t it            = 0;
-    for (uint32_t item = blockIdx.x; ok && item < p.n_items; item += gridDim.x) {
+    for (uint32_t item = blockIdx.x; ok && item < n_items; item += gridDim.x) {
       uint32_t t0, t1;
       tiles_of(item, t0, t1);
-      uint32_t key[kKeep] = {0u, 0u, 0u, 0u}, second[kKeep] = {0u, 0u, 0u, 0u}, list[kKeep] = {0u, 0u, 0u, 0u};
+      const uint32_t row = (item / p.splits) * kTileRows + h * kRows + quarter * 32u + lane;
+      const uint64_t neg = dup2(row < n_rows ? -__ldg(p.factor + row) : 0.0f);
+      float key[2][kKeep];  // of two column quarters
+#pragma unroll
+      for (uint32_t c = 0; c < 2; c++) {
+#pragma unroll
+        for (uint32_t i = 0; i < kKeep; i++) { key[c][i] = -3e38f; }
+      }
       for (uint32_t t = t0; t < t1; t++, it++) {
-        const uint32_t acc = it & 1u;
-        if (ok && !mbar_wait(bar_tfull + acc * 8, (it >> 1) & 1u, p.spin_limit)) { ok = false; }
+        const uint32_t id   = (t - t0) * kUnitsPerTile;
+        const uint32_t slot = it % kNormSlots;
+        if (ok && !mbar_wait(bar_norms + slot * 8, (it / kNormSlots) & 1u, p.spin_limit)) { ok = false; }
+        if (ok && !mbar_wait(bar_tfull + h * 8, it & 1u, p.spin_limit)) { ok = false; }
         if (__any_sync(kFullMask, !ok)) {
           ok = false;
           break;
         }
         tc_fence_after();
-        const uint32_t n0 = t * kLists + unit * kUnit;
-        uint32_t l0 = 0u, l1 = 0u;
-        auto chunk = [&](const uint32_t (&x)[32], auto second, auto full) {
-          constexpr uint32_t c = decltype(second)::value ? 32u : 0u;
+        const uint32_t tm = tmem_base + ((quarter * 32u) << 16) + h * kLists + side * 128u;
+        const uint32_t na = norm_base + slot * kNormBytes + side * 512u;
+        // four units of eight columns each
+        auto chunk = [&](uint32_t (&x)[32], auto cc) {
+          constexpr uint32_t c = decltype(cc)::value;
+          float m[4];
+          static_for<4>([&](auto uc) {
+            constexpr uint32_t u = decltype(uc)::value;
+            float v[8];
 #pragma unroll
-          for (uint32_t e = 0; e < 32; e++) {
-            // value rounded to a multiple of 2^-16, + 1.5 + tag 2^-23: bits that sort, low 7 the tag 63 - column
-            float f = __fadd_rn(__uint_as_float(x[e]), 192.0f);
-            f       = __fadd_rn(f, -192.0f);
-            f       = __fadd_rn(f, 1.5f + float(63u - c - e) * 0x1p-23f);
-            uint32_t k = __float_as_uint(f);
-            if constexpr (!decltype(full)::value) {
-              if (n0 + c + e >= p.n_lists) { k = 0u; }
+            for (uint32_t e = 0; e < 8; e += 4) {
+              uint64_t n01, n23;
+              lds128(na + (c * 32u + u * 8u + e) * 4u, n01, n23);
+              const uint64_t a = fma2(n01, neg, pack2(x[u * 8u + e], x[u * 8u + e + 1]));
+              const uint64_t b = fma2(n23, neg, pack2(x[u * 8u + e + 2], x[u * 8u + e + 3]));
+              v[e] = lo2(a); v[e + 1] = hi2(a); v[e + 2] = lo2(b); v[e + 3] = hi2(b);
             }
-            l1 = max(l1, min(l0, k));
-            l0 = max(l0, k);
+            const float y = max3(max3(max3(v[0], v[1], v[2]), v[3], v[4]), v[5], v[6]);
+            m[u] = __uint_as_float((__float_as_uint(fmaxf(y, v[7])) & ~p.tag_mask) | (id + (c & 1u) * 4u + u));
+          });
+          // two units at a time into the four largest: the m-th largest of two ordered runs a and b is the maximum over
+          // i + j = m of min(a[i - 1], b[j - 1])
+          float (&k)[kKeep] = key[c >> 1];
+#pragma unroll
+          for (uint32_t u = 0; u < 4; u += 2) {
+            const float hi = fmaxf(m[u], m[u + 1]), lo = fminf(m[u], m[u + 1]);
+            const float k3 = max3(k[3], fminf(k[2], hi), fminf(k[1], lo));
+            const float k2 = max3(k[2], fminf(k[1], hi), fminf(k[0], lo));
+            const float k1 = max3(k[1], fminf(k[0], hi), lo);
+            k[0]           = fmaxf(k[0], hi);
+            k[1]           = k1;
+            k[2]           = k2;
+            k[3]           = k3;
           }
         };
-        // (the second half is on its way while the first is looked at)
-        const uint32_t tm = tmem_base + ((quarter * 32u) << 16) + acc * kLists + unit * kUnit;
+        using std::integral_constant;
         uint32_t x0[32], x1[32];
         tmem_ld32(tm, x0);
         tmem_ld32_async(tm + 32u, x1);
-        if (n0 + kUnit <= p.n_lists) {
-          chunk(x0, std::false_type{}, std::true_type{});
-          tmem_ld_wait(x1);
-          chunk(x1, std::true_type{}, std::true_type{});
-        } else {
-          chunk(x0, std::false_type{}, std::false_type{});
-          tmem_ld_wait(x1);
-          chunk(x1, std::true_type{}, std::false_type{});
-        }
+        chunk(x0, integral_constant<uint32_t, 0>{});
+        tmem_ld_wait(x1);
+        tmem_ld32_async(tm + 64u, x0);
+        chunk(x1, integral_constant<uint32_t, 1>{});
+        tmem_ld_wait(x0);
+        tmem_ld32_async(tm + 96u, x1);
+        chunk(x0, integral_constant<uint32_t, 2>{});
+        tmem_ld_wait(x1);
+        // (the last values are in registers: the accumulator is free)
         tc_fence_before();
         __syncwarp();
-        if (lane == 0) { mbar_arrive(bar_tempty + acc * 8); }
-        if (l0 > key[kKeep - 1]) {
-          key[kKeep - 1]    = l0;
-          second[kKeep - 1] = l1;
-          list[kKeep - 1] = n0 + (63u - (l0 & 127u));
-#pragma unroll
-          for (int i = int(kKeep) - 1; i > 0; i--) {
-            if (key[i] > key[i - 1]) {
-              const uint32_t a = key[i], b = list[i], c = second[i];
-              key[i]        = key[i - 1];
-              list[i]       = list[i - 1];
-              second[i]     = second[i - 1];
-              key[i - 1]    = a;
-              list[i - 1]   = b;
-              second[i - 1] = c;
-            }
-          }
-        }
+        if (lane == 0) { mbar_arrive(bar_tempty + h * 8); }
+        chunk(x1, integral_constant<uint32_t, 3>{});
       }
-      const uint32_t row = (item / p.splits) * kRows + quarter * 32u + lane;
-      if (ok && row < p.n_rows) {
-        const size_t at = (size_t(item % p.splits) * p.n_rows + row) * 4u + unit;
-        p.keys[at]      = make_uint4(key[0], key[1], key[2], key[3]);
-        p.lists[at]     = make_uint4(list[0], list[1], list[2], list[3]);
-        p.seconds[at]   = make_uint4(second[0], second[1], second[2], second[3]);
+      if (ok && row < n_rows) {
+#pragma unroll
+        for (uint32_t c = 0; c < 2; c++) {
+          p.keys[(size_t(item % p.splits) * p.n_rows + row) * 4u + side * 2u + c] =
+            make_float4(key[c][0], key[c][1], key[c][2], key[c][3]);
+        }
       }
     }
   }
@@ -480,21 +613,6 @@ label_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
   }
 }
 
-__device__ __forceinline__ float key_value(uint32_t key)
-{
-  return key >= 0x00800000u ? __fadd_rn(__uint_as_float(key & ~127u), -1.5f) : -INFINITY;
-}
-
-struct label_records {
-  const uint4* keys;
-  const uint4* seconds;
-  const uint4* lists;
-  const float* eps;
-  const uint32_t* error;
-  uint32_t* timeouts;  // pinned host word: calls with the error word set
-  uint32_t splits, n_rows, n_lists;
-};
-
 // the defining chain of one list
 __device__ __forceinline__ uint64_t exact_key(const float* q, const float* centers, uint32_t list, uint32_t dim_ext, float alpha)
 {
@@ -511,130 +629,242 @@ __device__ __forceinline__ uint64_t exact_key(const float* q, const float* cente
   return make_key(__fmul_rn(alpha, acc), list);
 }
 
-// Four lanes per row: lane u reads what column quarter u kept (of every split).  Rows for the other two passes are
-// listed: redo[0 .. counts[0]) from the front, whole units from the back (counts[1] of them).
-__global__ void __launch_bounds__(256)
-label_finish_kernel(const label_records p, const float* __restrict__ x, const float* __restrict__ centers, uint32_t dim_ext,
-                    float alpha, uint32_t* __restrict__ labels, uint32_t* __restrict__ redo, uint32_t* __restrict__ counts)
+struct finish_params {
+  const float* keys;       // [splits, stride, 16]
+  const float4* eps;
+  const uint32_t* error;
+  uint32_t* timeouts;      // pinned host word: passes with the error word set
+  uint32_t splits, stride, n_lists, tiles_per_split, tag_mask, width, block_rows;
+  uint32_t n_rows;
+  const uint32_t* count;   // where given: so many rows (at most n_rows), named by `rows`
+  const uint32_t* rows;
+  const __half* a;         // operands of all rows, and of all lists by units; factors and norm terms
+  const __half* b;
+  const float* factor;
+  const float* norms;
+  const float* x;
+  const float* centers;
+  uint32_t dim_ext;
+  float alpha;
+  uint32_t* labels;
+  // rows that more units reach than are kept: to `next` while it has room, else to `last`
+  uint32_t* next;
+  uint32_t* next_count;
+  uint32_t next_cap;
+  uint32_t* last;
+  uint32_t* last_count;
+  unsigned long long* best;  // set to "none yet" for rows that go to `last`
+};
+
+// acc += a.lo b.lo + a.hi b.hi in fp32 (the halfs widen exactly)
+__device__ __forceinline__ float fma_half2(uint32_t a, uint32_t b, float acc)
 {
-  const uint32_t r = (blockIdx.x * 256u + threadIdx.x) >> 2, u = threadIdx.x & 3u;
-  const unsigned mask = 0xFu << (threadIdx.x & 28u);
-  if (r >= p.n_rows) { return; }
-  float top = -INFINITY, out = -INFINITY;  // largest value, largest that bounds units not kept
-  for (uint32_t s = 0; s < p.splits; s++) {
-    const uint4 k = __ldg(p.keys + (size_t(s) * p.n_rows + r) * 4u + u);
-    top           = fmaxf(top, key_value(k.x));
-    out           = fmaxf(out, key_value(k.w));
-  }
-#pragma unroll
-  for (int o = 2; o > 0; o >>= 1) {
-    top = fmaxf(top, __shfl_xor_sync(mask, top, o));
-    out = fmaxf(out, __shfl_xor_sync(mask, out, o));
-  }
-  const float t = top - 2.0f * __ldg(p.eps + r);
-  if (*p.error != 0u && blockIdx.x == 0 && threadIdx.x == 0) { count_timeout(p.timeouts); }
-  // (negated: an infinite or undefined bound is not proof)
-  if (*p.error != 0u || !(out < t)) {
-    if (u == 0) { redo[atomicAdd(counts, 1u)] = r; }
-    return;
-  }
-  uint32_t n = 0, only = 0xFFFFFFFFu;
-  bool more  = false;
-  for (uint32_t s = 0; s < p.splits; s++) {
-    const size_t at = (size_t(s) * p.n_rows + r) * 4u + u;
-    const uint4 k   = __ldg(p.keys + at);
-    if (key_value(k.x) >= t) {
-      const uint4 b = __ldg(p.seconds + at);
-      only          = __ldg(&p.lists[at].x);
-      n += 1u + (key_value(k.y) >= t ? 1u : 0u) + (key_value(k.z) >= t ? 1u : 0u);
-      more = more || key_value(b.x) >= t || (key_value(k.y) >= t && key_value(b.y) >= t) ||
-             (key_value(k.z) >= t && key_value(b.z) >= t);
-    }
-  }
-  uint32_t all = n;
-#pragma unroll
-  for (int o = 2; o > 0; o >>= 1) { all += __shfl_xor_sync(mask, all, o); }
-  if (__any_sync(mask, more)) {
-    if (u == 0) { redo[p.n_rows - 1u - atomicAdd(counts + 1, 1u)] = r; }
-    return;
-  }
-  if (all == 1u) {
-    if (n == 1u) { labels[r] = only; }
-    return;
-  }
-  // each lane rescores its own (rarely more than one)
-  uint64_t best = kEmptyKey;
-  if (n > 0) {
-    for (uint32_t s = 0; s < p.splits; s++) {
-      const size_t at      = (size_t(s) * p.n_rows + r) * 4u + u;
-      const uint4 k        = __ldg(p.keys + at), l = __ldg(p.lists + at);
-      const uint32_t kk[3] = {k.x, k.y, k.z}, ll[3] = {l.x, l.y, l.z};
-#pragma unroll
-      for (int i = 0; i < 3; i++) {
-        if (key_value(kk[i]) < t) { continue; }
-        const uint64_t key = exact_key(x + size_t(r) * dim_ext, centers, ll[i], dim_ext, alpha);
-        best               = key < best ? key : best;
-      }
-    }
-  }
-#pragma unroll
-  for (int o = 2; o > 0; o >>= 1) {
-    const uint32_t hi = __shfl_xor_sync(mask, uint32_t(best >> 32), o), lo = __shfl_xor_sync(mask, uint32_t(best), o);
-    const uint64_t other = (uint64_t(hi) << 32) | lo;
-    best                 = other < best ? other : best;
-  }
-  if (u == 0) { labels[r] = uint32_t(best); }
+  asm("{\n\t.reg .b16 al, ah, bl, bh;\n\tmov.b32 {al, ah}, %1;\n\tmov.b32 {bl, bh}, %2;\n\t"
+      "fma.rn.f32.f16 %0, al, bl, %0;\n\tfma.rn.f32.f16 %0, ah, bh, %0;\n\t}" : "+f"(acc) : "r"(a), "r"(b));
+  return acc;
 }
 
-// Rows with units whose second value is within reach: one warp per row rescores every list of such units, and the single
-// lists of the others.
-__global__ void __launch_bounds__(256)
-label_units_kernel(const label_records p, const float* __restrict__ x, const float* __restrict__ centers, uint32_t dim_ext,
-                   float alpha, uint32_t* __restrict__ labels, const uint32_t* __restrict__ redo, const uint32_t* __restrict__ counts)
+// A block per `block_rows` rows (at most kFinishRows), in steps that share the work evenly over its half warps:
+//   1. two threads per row: which kept units are within 2 eps of the largest value;
+//   2. a half warp per unit: the operands' products of its eight lists in fp32, two lanes per list (that takes the tensor
+//      core's accumulation and the keys out of the bound), and which lists are within reach of the row's best one;
+//   3. rows with several such lists, a half warp per list: the product summed in fp32 (that takes the rounding of the
+//      operands out);
+//   4. where that leaves several, a thread per list: the defining chain.
+// What bounds it: latency, then L2 -- 8 operand rows per unit, 2.6 units per row on 1 M rows x 16,384 lists of 96 dimensions.
+// With a warp, or half a warp, to itself a row's dependent reads took 1.3 and 1.1 ms there.
+constexpr uint32_t kFinishRows = 64, kSecondRows = 32, kFinishUnits = 640, kFinishLists = 640;
+__device__ __forceinline__ uint32_t half_warp_max(uint32_t v)
 {
-  const uint32_t lane = threadIdx.x & 31u;
-  const uint32_t n    = __ldg(counts + 1);
-  for (uint32_t i = (blockIdx.x * 256u + threadIdx.x) >> 5; i < n; i += gridDim.x * 8u) {
-    const uint32_t r = redo[p.n_rows - 1u - i];
-    const float* q   = x + size_t(r) * dim_ext;
-    // lane 4 u + j: unit j of column quarter u
-    const uint32_t* keys = reinterpret_cast<const uint32_t*>(p.keys);
-    auto at = [&](uint32_t s) { return (size_t(s) * p.n_rows + r) * 16u + (lane & 15u); };
-    float top = -INFINITY;
-    for (uint32_t s = 0; s < p.splits; s++) { top = fmaxf(top, key_value(__ldg(keys + at(s)))); }
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) { top = fmaxf(top, __shfl_xor_sync(kFullMask, top, o)); }
-    const float t = top - 2.0f * __ldg(p.eps + r);
-    uint64_t best = kEmptyKey;
-    for (uint32_t s = 0; s < p.splits; s++) {
-      const bool in       = lane < 16u && key_value(__ldg(keys + at(s))) >= t;
-      const bool whole    = in && key_value(__ldg(reinterpret_cast<const uint32_t*>(p.seconds) + at(s))) >= t;
-      const uint32_t list = in ? __ldg(reinterpret_cast<const uint32_t*>(p.lists) + at(s)) : 0u;
-      if (in && !whole) {
-        const uint64_t key = exact_key(q, centers, list, dim_ext, alpha);
-        best               = key < best ? key : best;
+  for (int o = 8; o > 0; o >>= 1) { v = max(v, __shfl_xor_sync(kFullMask, v, o)); }
+  return v;
+}
+__global__ void __launch_bounds__(256, 6)
+label_finish_kernel(const finish_params p)
+{
+  __shared__ uint32_t s_unit[kFinishUnits];        // unit's first list
+  __shared__ uint8_t s_unit_row[kFinishUnits];
+  __shared__ float s_val[kFinishUnits * kUnit];
+  __shared__ uint32_t s_list[kFinishLists];
+  __shared__ uint8_t s_list_row[kFinishLists];
+  __shared__ float s_sum[kFinishLists];
+  __shared__ unsigned long long s_key[kFinishRows];
+  __shared__ float4 s_eps[kFinishRows];
+  __shared__ uint32_t s_row[kFinishRows], s_best[kFinishRows], s_sum_best[kFinishRows], s_label[kFinishRows], s_n_sum[kFinishRows];
+  __shared__ uint32_t s_n_list[kFinishRows], s_redo[kFinishRows], s_count[2];
+  chain_begin();
+  const uint32_t tid = threadIdx.x, lane = tid & 31u, l16 = lane & 15u, hw = tid >> 4;
+  const uint32_t n   = p.count != nullptr ? min(__ldg(p.count), p.n_rows) : p.n_rows;
+  const uint32_t w8 = p.width / 8u, n4 = p.dim_ext / 4u;
+  const bool failed = *p.error != 0u;
+  if (failed && n > 0 && blockIdx.x == 0 && tid == 0) { count_timeout(p.timeouts); }
+  for (uint32_t i0 = blockIdx.x * p.block_rows; i0 < n; i0 += gridDim.x * p.block_rows) {
+    if (tid < 2) { s_count[tid] = 0u; }
+    __syncthreads();
+    // ---- 1. units within reach ----
+    if (tid < 2u * p.block_rows) {  // (whole warps)
+      const uint32_t lr = tid >> 1, side = tid & 1u;  // thread: two column quarters of row lr
+      const uint32_t i = min(i0 + lr, n - 1u);
+      const uint32_t r = p.rows != nullptr ? __ldg(p.rows + i) : i;
+      const float4 e   = __ldg(p.eps + r);
+      auto keys_of = [&](uint32_t s, uint32_t c) {
+        return __ldg(reinterpret_cast<const float4*>(p.keys) + (size_t(s) * p.stride + i) * 4u + side * 2u + c);
+      };
+      float top = -INFINITY, out = -INFINITY;  // largest value, largest that bounds units not kept
+      for (uint32_t s = 0; s < p.splits; s++) {
+        const float4 a = keys_of(s, 0), b = keys_of(s, 1);
+        top = max3(top, a.x, b.x);
+        out = max3(out, a.w, b.w);
       }
-      unsigned m = __ballot_sync(kFullMask, whole);
-      while (m) {
-        const uint32_t base = __shfl_sync(kFullMask, list, __ffs(m) - 1) & ~(kUnit - 1u);
-        m &= m - 1;
-        for (uint32_t l = base + lane; l < min(base + kUnit, p.n_lists); l += 32) {
-          const uint64_t key = exact_key(q, centers, l, dim_ext, alpha);
-          best               = key < best ? key : best;
+      top           = fmaxf(top, __shfl_xor_sync(kFullMask, top, 1));
+      out           = fmaxf(out, __shfl_xor_sync(kFullMask, out, 1));
+      const float t = top - 2.0f * e.x;
+      // (negated: an infinite or undefined bound is not proof)
+      bool redo = failed || !(out < t);
+      for (uint32_t s = 0; !redo && s < p.splits; s++) {
+#pragma unroll
+        for (uint32_t c = 0; c < 2; c++) {
+          const float4 a   = keys_of(s, c);
+          const float k[3] = {a.x, a.y, a.z};
+          const uint32_t m = (k[0] >= t ? 1u : 0u) + (k[1] >= t ? 1u : 0u) + (k[2] >= t ? 1u : 0u);  // (they are in order)
+          if (m == 0u || redo) { continue; }
+          const uint32_t at = atomicAdd(&s_count[0], m);
+          if (at + m > kFinishUnits) { redo = true; }
+#pragma unroll
+          for (uint32_t j = 0; j < 3; j++) {
+            if (j >= m || at + j >= kFinishUnits) { continue; }
+            const uint32_t id   = __float_as_uint(k[j]) & p.tag_mask;
+            s_unit[at + j]      = (s * p.tiles_per_split + id / kUnitsPerTile) * kLists + (side * 2u + c) * 64u + (id % kUnitsPerTile) * kUnit;
+            s_unit_row[at + j]  = uint8_t(lr);
+          }
+        }
+      }
+      redo = __shfl_xor_sync(kFullMask, redo ? 1 : 0, 1) != 0 || redo;
+      if (side == 0u) {
+        s_row[lr]      = r;
+        s_eps[lr]      = e;
+        s_redo[lr]     = redo ? 1u : 0u;
+        s_best[lr]     = 0u;
+        s_sum_best[lr] = 0u;
+        s_n_list[lr]   = 0u;
+        s_n_sum[lr]    = 0u;
+        s_key[lr]      = ~0ull;
+      }
+    }
+    __syncthreads();
+    // (every entry below this is written; units that had no room are not there: their rows are redone)
+    const uint32_t n_units = min(s_count[0], kFinishUnits);
+    // ---- 2. their lists ----
+    for (uint32_t u0 = 0; u0 < n_units; u0 += 16u) {
+      const uint32_t u  = u0 + hw;
+      const bool has    = u < n_units;
+      const uint32_t lr = has ? s_unit_row[u] : 0u, list0 = has ? s_unit[u] : 0u, list = list0 + (l16 & 7u);
+      const bool look   = has && s_redo[lr] == 0u, valid = look && list < p.n_lists;
+      float acc = 0.0f, acc1 = 0.0f;
+      if (look) {
+        // (lanes 0-7 and 8-15: neighbouring 16-byte chunks of the eight lists)
+        const uint32_t r = s_row[lr];
+        const uint4* av  = reinterpret_cast<const uint4*>(p.a + size_t(r) * p.width);
+        const uint4* bv  = reinterpret_cast<const uint4*>(p.b) + size_t(list0 / kUnit) * w8 * kUnit + l16;
+#pragma unroll 6
+        for (uint32_t c = 0; c < w8; c += 2u) {
+          const uint4 ac = __ldg(av + c + (l16 >> 3)), bc = __ldg(bv + c * kUnit);
+          acc  = fma_half2(ac.x, bc.x, acc);
+          acc1 = fma_half2(ac.y, bc.y, acc1);
+          acc  = fma_half2(ac.z, bc.z, acc);
+          acc1 = fma_half2(ac.w, bc.w, acc1);
+        }
+        if (l16 < 8u && valid) { acc1 = __fmaf_rn(__ldg(p.norms + list), -__ldg(p.factor + r), acc1); }
+      }
+      acc += acc1;
+      acc += __shfl_xor_sync(kFullMask, acc, 8);
+      const uint32_t mx = half_warp_max(valid ? float_to_ordered(acc) : 0u);
+      if (has) {
+        if (l16 < 8u) { s_val[u * kUnit + l16] = valid ? acc : -INFINITY; }
+        if (l16 == 0u && mx != 0u) { atomicMax(&s_best[lr], mx); }
+      }
+    }
+    __syncthreads();
+    for (uint32_t v = tid; v < n_units * kUnit; v += 256u) {
+      const uint32_t lr = s_unit_row[v / kUnit];
+      if (s_redo[lr] == 0u && s_val[v] >= ordered_to_float(s_best[lr]) - 2.0f * s_eps[lr].y) {
+        const uint32_t at = atomicAdd(&s_count[1], 1u), list = s_unit[v / kUnit] + v % kUnit;
+        atomicAdd(&s_n_list[lr], 1u);
+        s_label[lr] = list;  // (the only one, or another is found below)
+        if (at < kFinishLists) {
+          s_list[at]     = list;
+          s_list_row[at] = uint8_t(lr);
+        } else {
+          s_n_list[lr] = 1u << 30;  // no room: the row is redone
         }
       }
     }
+    __syncthreads();
+    const uint32_t n_lists = min(s_count[1], kFinishLists);
+    // ---- 3. rows with several ----
+    for (uint32_t c0 = 0; c0 < n_lists; c0 += 16u) {
+      const uint32_t c  = c0 + hw;
+      const uint32_t lr = c < n_lists ? s_list_row[c] : 0u;
+      const bool has    = c < n_lists && s_n_list[lr] > 1u;
+      if (!__any_sync(kFullMask, has)) { continue; }
+      float acc = 0.0f;
+      if (has) {
+        const float4* x  = reinterpret_cast<const float4*>(p.x + size_t(s_row[lr]) * p.dim_ext);
+        const float4* cv = reinterpret_cast<const float4*>(p.centers + size_t(s_list[c]) * p.dim_ext);
+#pragma unroll 2
+        for (uint32_t k4 = l16; k4 < n4; k4 += 16u) {
+          const float4 a = __ldg(cv + k4), b = __ldg(x + k4);
+          acc = __fmaf_rn(a.x, b.x, __fmaf_rn(a.y, b.y, __fmaf_rn(a.z, b.z, __fmaf_rn(a.w, b.w, acc))));
+        }
+      }
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      const uint64_t other = shfl_u64(best, int(lane) ^ o);
-      best                 = other < best ? other : best;
+      for (int o = 8; o > 0; o >>= 1) { acc += __shfl_xor_sync(kFullMask, acc, o); }
+      if (has && l16 == 0u) {
+        s_sum[c] = acc;
+        atomicMax(&s_sum_best[lr], float_to_ordered(acc));
+      }
     }
-    if (lane == 0) { labels[r] = uint32_t(best); }
+    __syncthreads();
+    auto close = [&](uint32_t c, uint32_t lr) {
+      return s_n_list[lr] > 1u && s_sum[c] >= ordered_to_float(s_sum_best[lr]) - 2.0f * s_eps[lr].z;
+    };
+    for (uint32_t c = tid; c < n_lists; c += 256u) {
+      const uint32_t lr = s_list_row[c];
+      if (close(c, lr)) {
+        atomicAdd(&s_n_sum[lr], 1u);
+        s_label[lr] = s_list[c];
+      }
+    }
+    __syncthreads();
+    // ---- 4. near ties ----
+    for (uint32_t c = tid; c < n_lists; c += 256u) {
+      const uint32_t lr = s_list_row[c];
+      if (s_n_sum[lr] > 1u && close(c, lr)) {
+        atomicMin(&s_key[lr], exact_key(p.x + size_t(s_row[lr]) * p.dim_ext, p.centers, s_list[c], p.dim_ext, p.alpha));
+      }
+    }
+    __syncthreads();
+    if (tid < p.block_rows && i0 + tid < n) {
+      const uint32_t r = s_row[tid];
+      if (s_redo[tid] != 0u || s_n_list[tid] >= (1u << 30)) {
+        uint32_t at = p.next_cap;
+        if (!failed && p.next_cap > 0) { at = atomicAdd(p.next_count, 1u); }
+        if (at < p.next_cap) {
+          p.next[at] = r;
+        } else {
+          p.last[atomicAdd(p.last_count, 1u)] = r;
+          p.best[r]                           = ~0ull;
+        }
+      } else {
+        p.labels[r] = s_n_sum[tid] > 1u ? uint32_t(s_key[tid]) : s_label[tid];
+      }
+    }
+    __syncthreads();
   }
 }
 
-uint32_t operand_width(uint32_t dim) { return round_up(dim + 2u, 16u); }
-uint32_t operand_products(uint32_t dim) { return ceildiv(operand_width(dim), kBlockK) <= 3u ? 2u : 1u; }
+uint32_t operand_width(uint32_t dim) { return round_up(dim, 16u); }
 
 }  // namespace
 
@@ -644,116 +874,184 @@ bool label_tc_usable(uint32_t n_rows, uint32_t n_lists)
   return n_lists >= 256 && uint64_t(n_rows) * n_lists >= (1ull << 24);
 }
 
-size_t label_model_bytes(uint32_t n_lists, uint32_t dim) { return operand_at(dim) + size_t(n_lists) * operand_width(dim) * 2; }
+size_t label_model_bytes(uint32_t n_lists, uint32_t dim) { return unit_operand_at(n_lists, dim, operand_width(dim)) + size_t(round_up(n_lists, kUnit)) * operand_width(dim) * 2; }
 
 void prepare_label_model(cudaStream_t stream, const float* centers, uint32_t n_lists, uint32_t dim, uint32_t dim_ext, void* model)
 {
   auto* words = static_cast<uint32_t*>(model);
   auto* sum   = reinterpret_cast<float*>(static_cast<char*>(model) + kMeanAt);
-  auto* b     = reinterpret_cast<__half*>(static_cast<char*>(model) + operand_at(dim));
-  CUDA_TRY(cudaMemsetAsync(model, 0, operand_at(dim), stream));
+  auto* norms = reinterpret_cast<float*>(static_cast<char*>(model) + norms_at(dim));
+  auto* b     = reinterpret_cast<__half*>(static_cast<char*>(model) + operand_at(n_lists, dim));
+  auto* units = reinterpret_cast<__half*>(static_cast<char*>(model) + unit_operand_at(n_lists, dim, operand_width(dim)));
+  CUDA_TRY(cudaMemsetAsync(model, 0, norms_at(dim), stream));
   const uint32_t shares = std::min<uint32_t>(64, ceildiv(n_lists, 64u));
   center_sum_kernel<<<dim3(ceildiv(dim, 32u), shares), dim3(32, 8), 0, stream>>>(centers, n_lists, dim, dim_ext, sum);
   center_stats_kernel<<<ceildiv<uint32_t>(n_lists, 8u), 256, 0, stream>>>(centers, n_lists, dim, dim_ext, sum, words);
-  center_operand_kernel<<<ceildiv<uint32_t>(n_lists, 8u), 256, 0, stream>>>(centers, n_lists, dim, dim_ext, operand_width(dim), sum,
-                                                                           words, b);
+  center_operand_kernel<<<round_up(n_lists, kLists) / 8u, 256, 0, stream>>>(centers, n_lists, dim, dim_ext, operand_width(dim), sum,
+                                                                           words, norms, b, units);
   CUDA_TRY(cudaGetLastError());
 }
 
 namespace {
-struct label_layout {
-  uint32_t splits, tiles_per_split;
-  size_t o_a, o_eps, o_keys, o_seconds, o_lists, o_redo, o_words, o_best, total;
+// One pass of label_tc_kernel over up to `rows` rows: the lists are shared out (`splits`) where row tiles alone do not fill
+// the SMs four times, and so that an item has at most kSplitTiles list tiles.
+struct label_pass {
+  uint32_t splits, tiles_per_split, tag_mask;
+  label_pass(uint32_t rows, uint32_t n_lists, uint32_t items)
+  {
+    const uint32_t row_tiles = ceildiv(rows, kTileRows), n_tiles = ceildiv(n_lists, kLists);
+    splits = ceildiv(n_tiles, kSplitTiles);
+    while (splits < n_tiles && row_tiles * splits < items && splits < 16) { splits <<= 1; }
+    splits          = std::min(splits, n_tiles);
+    tiles_per_split = ceildiv(n_tiles, splits);
+    splits          = ceildiv(n_tiles, tiles_per_split);
+    tag_mask        = 1;
+    while (tag_mask < tiles_per_split * kUnitsPerTile) { tag_mask <<= 1; }
+    tag_mask--;
+  }
 };
-label_layout layout_for(uint32_t n_rows, uint32_t n_lists, uint32_t dim, int sm_count)
-{
-  label_layout y{};
-  const uint32_t row_tiles = ceildiv(n_rows, kRows), n_tiles = ceildiv(n_lists, kLists);
-  // few row tiles: the lists are shared out, so that there are about four items per SM
-  y.splits = 1;
-  while (y.splits < n_tiles && row_tiles * y.splits < 4u * uint32_t(sm_count) && y.splits < 16) { y.splits <<= 1; }
-  y.splits          = std::min(y.splits, n_tiles);
-  y.tiles_per_split = ceildiv(n_tiles, y.splits);
-  y.splits          = ceildiv(n_tiles, y.tiles_per_split);
-  const size_t recs = size_t(y.splits) * n_rows * 4;
-  ws_layout lay;
-  y.o_a      = lay.add(size_t(n_rows) * operand_width(dim) * operand_products(dim) * 2);
-  y.o_eps    = lay.add(size_t(n_rows) * 4);
-  y.o_keys   = lay.add(recs * 16);
-  y.o_lists  = lay.add(recs * 16);
-  y.o_seconds = lay.add(recs * 16);
-  y.o_redo   = lay.add(size_t(n_rows) * 4);
-  y.o_words  = lay.add(256);
-  y.o_best   = lay.add(size_t(n_rows) * 8);
-  y.total    = lay.total();
-  return y;
-}
+// Rows whose reach the first pass does not settle go through a second one with the lists in eight shares, whose records keep
+// eight times as many units: room for this many rows (what exceeds it is redone by the exact product).  On 300,000 8-bit rows
+// against 4,000 lists a tenth of the rows go there.
+constexpr uint32_t kSecondShares = 8;
+uint32_t second_rows(uint32_t n_rows) { return round_up(std::max(n_rows / 4u, std::min(n_rows, 1024u)), kTileRows); }
+
+struct label_layout {
+  label_pass first, second;
+  uint32_t cap;
+  // (few rows: the first pass has as many shares already)
+  bool second_pass() const { return second.splits > first.splits; }
+  size_t o_a, o_factor, o_eps, o_keys, o_a2, o_factor2, o_keys2, o_next, o_last, o_words, o_best, total;
+  label_layout(uint32_t n_rows, uint32_t n_lists, uint32_t dim, int sm_count)
+    : first(n_rows, n_lists, 4u * uint32_t(sm_count)), second(1, n_lists, kSecondShares), cap(second_pass() ? second_rows(n_rows) : 0)
+  {
+    const size_t row = size_t(operand_width(dim)) * 2;
+    ws_layout lay;
+    o_a     = lay.add(n_rows * row);
+    o_factor = lay.add(size_t(n_rows) * 4);
+    o_eps   = lay.add(size_t(n_rows) * 16);
+    o_keys  = lay.add(size_t(first.splits) * n_rows * 64);
+    o_a2    = lay.add(cap * row);
+    o_factor2 = lay.add(size_t(cap) * 4);
+    o_keys2 = lay.add(size_t(second.splits) * cap * 64);
+    o_next  = lay.add(size_t(cap) * 4);
+    o_last  = lay.add(size_t(n_rows) * 4);
+    o_words = lay.add(256);
+    o_best  = lay.add(size_t(n_rows) * 8);
+    total   = lay.total();
+  }
+};
 }  // namespace
 
 size_t label_workspace_bytes(const raft::resources& res, uint32_t n_rows, uint32_t n_lists, uint32_t dim)
 {
-  return layout_for(n_rows, n_lists, dim, res.sm_count).total;
+  return label_layout(n_rows, n_lists, dim, res.sm_count).total;
 }
 
 void label_rows_tc(raft::resources& res, const float* centers, const void* model, uint32_t n_lists, uint32_t dim,
                    uint32_t dim_ext, float alpha, const float* x_ext, uint32_t n_rows, uint32_t* labels, void* workspace)
 {
   if (n_rows == 0) { return; }
-  const label_layout y = layout_for(n_rows, n_lists, dim, res.sm_count);
+  const label_layout y(n_rows, n_lists, dim, res.sm_count);
   const uint32_t width = operand_width(dim);
   char* ws             = static_cast<char*>(workspace);
   auto* a              = reinterpret_cast<__half*>(ws + y.o_a);
-  auto* eps            = reinterpret_cast<float*>(ws + y.o_eps);
-  auto* words          = reinterpret_cast<uint32_t*>(ws + y.o_words);  // error, rows to redo
-  auto* redo           = reinterpret_cast<uint32_t*>(ws + y.o_redo);
+  auto* a2             = reinterpret_cast<__half*>(ws + y.o_a2);
+  auto* factor         = reinterpret_cast<float*>(ws + y.o_factor);
+  auto* factor2        = reinterpret_cast<float*>(ws + y.o_factor2);
+  auto* eps            = reinterpret_cast<float4*>(ws + y.o_eps);
+  auto* keys           = reinterpret_cast<float4*>(ws + y.o_keys);
+  auto* keys2          = reinterpret_cast<float4*>(ws + y.o_keys2);
+  auto* next           = reinterpret_cast<uint32_t*>(ws + y.o_next);
+  auto* last           = reinterpret_cast<uint32_t*>(ws + y.o_last);
   auto* best           = reinterpret_cast<unsigned long long*>(ws + y.o_best);
+  auto* words          = reinterpret_cast<uint32_t*>(ws + y.o_words);  // errors of the passes, rows in `next` and `last`
   const auto* stats    = static_cast<const uint32_t*>(model);
   const auto* sum      = reinterpret_cast<const float*>(static_cast<const char*>(model) + kMeanAt);
-  const auto* b        = reinterpret_cast<const __half*>(static_cast<const char*>(model) + operand_at(dim));
+  const auto* norms    = reinterpret_cast<const float*>(static_cast<const char*>(model) + norms_at(dim));
+  const auto* b        = reinterpret_cast<const __half*>(static_cast<const char*>(model) + operand_at(n_lists, dim));
   cudaStream_t stream  = res.stream;
-  CUDA_TRY(cudaMemsetAsync(words, 0, 12, stream));
-  const uint32_t products = operand_products(dim);
-  const uint32_t blocks   = ceildiv<uint32_t>(n_rows, 8u);
-  if (products == 2) {
-    row_operand_kernel<true><<<blocks, 256, 0, stream>>>(x_ext, n_rows, n_lists, dim, dim_ext, width, sum, stats, a, eps);
+  // (a key's low bits number its unit: of a value below 0.5 that takes less than tag_mask + 1 units of 2^-25)
+  const float key_error = float(std::max(y.first.tag_mask, y.second.tag_mask) + 1u) * 0x1p-25f;
+  auto operand = [&](auto kernel) {
+    launch_chained(kernel, ceildiv<uint32_t>(n_rows, 32u), 256, 0, stream, x_ext, n_rows, n_lists, dim, dim_ext, width, sum, stats,
+                   key_error, a, factor, eps, reinterpret_cast<uint4*>(words));
+  };
+  if (width <= 128) {
+    operand(row_operand_kernel<true>);
   } else {
-    row_operand_kernel<false><<<blocks, 256, 0, stream>>>(x_ext, n_rows, n_lists, dim, dim_ext, width, sum, stats, a, eps);
+    operand(row_operand_kernel<false>);
   }
   label_params p{};
-  p.n_rows          = n_rows;
-  p.n_lists         = n_lists;
-  p.k_steps         = width / 16;
-  p.k_blocks        = ceildiv(width, kBlockK);
-  p.n_tiles         = ceildiv(n_lists, kLists);
-  p.tiles_per_split = y.tiles_per_split;
-  p.splits          = y.splits;
-  p.n_items         = ceildiv(n_rows, kRows) * y.splits;
-  // the row tile stays in shared memory where that leaves at least three list stages
-  const uint32_t a_size = products * p.k_blocks * kABlock;
-  p.products   = products;
-  p.width      = width;
-  p.a_resident = a_size + 3 * kBBlock <= kRoom;
-  CUVS_EXPECTS(p.a_resident || products == 1, "internal error: split row operands are resident");
-  p.n_stages   = p.a_resident ? std::min(kMaxStages, (kRoom - a_size) / kBBlock) : kRoom / (kABlock + kBBlock);
-  p.keys       = reinterpret_cast<uint4*>(ws + y.o_keys);
-  p.lists      = reinterpret_cast<uint4*>(ws + y.o_lists);
-  p.seconds    = reinterpret_cast<uint4*>(ws + y.o_seconds);
-  p.error      = words;
+  p.k_steps  = width / 16;
+  p.k_blocks = ceildiv(width, kBlockK);
+  p.n_tiles  = ceildiv(n_lists, kLists);
+  p.norms    = norms;
   const wait_limits wl = tc_wait_limits();
   p.spin_limit = wl.spin_limit;
   p.skip_kb    = wl.skip_kb;
-  const CUtensorMap ma = make_map_2d(CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, a, n_rows, uint64_t(width) * products, kRows, kBlockK, CU_TENSOR_MAP_SWIZZLE_128B);
   const CUtensorMap mb = make_map_2d(CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, b, n_lists, width, kLists, kBlockK, CU_TENSOR_MAP_SWIZZLE_128B);
-  const size_t smem    = kRoom + 1024 + 256;
-  ensure_dynamic_smem(reinterpret_cast<const void*>(label_tc_kernel), smem);
-  label_tc_kernel<<<std::min(uint32_t(res.sm_count), p.n_items), kThreads, smem, stream>>>(ma, mb, p);
-  const label_records rec{p.keys, p.seconds, p.lists, eps, words, res.pinned + 13, p.splits, n_rows, n_lists};
-  label_finish_kernel<<<ceildiv(n_rows, 64u), 256, 0, stream>>>(rec, x_ext, centers, dim_ext, alpha, labels, redo, words + 1);
-  label_units_kernel<<<std::min<uint32_t>(uint32_t(res.sm_count) * 8, blocks), 256, 0, stream>>>(rec, x_ext, centers, dim_ext, alpha,
-                                                                                               labels, redo, words + 1);
-  CUDA_TRY(cudaGetLastError());
-  assign_nearest_listed(res, centers, n_lists, dim_ext, alpha, x_ext, n_rows, redo, words + 1, labels, best);
-  res.launches += 4;
+  const size_t smem    = kRoom + kNormSlots * kNormBytes + 1024 + 256;
+  finish_params f{};
+  f.eps = eps;
+  f.timeouts = res.pinned + 13;
+  f.n_lists = n_lists;
+  f.width = width;
+  f.a = a;
+  f.b = reinterpret_cast<const __half*>(static_cast<const char*>(model) + unit_operand_at(n_lists, dim, width));
+  f.factor = factor;
+  f.norms = norms;
+  f.x = x_ext;
+  f.centers = centers;
+  f.dim_ext = dim_ext;
+  f.alpha = alpha;
+  f.labels = labels;
+  f.last = last;
+  f.last_count = words + 3;
+  f.best = best;
+  auto pass = [&](const label_pass& s, const __half* operand, const float* factors, float4* k, uint32_t rows, uint32_t* error, const uint32_t* count,
+                  uint32_t block_rows, uint32_t finish_blocks) {
+    p.n_rows = f.n_rows = f.stride = rows;
+    f.block_rows = block_rows;
+    p.count = f.count = count;
+    p.splits = f.splits = s.splits;
+    p.tiles_per_split = f.tiles_per_split = s.tiles_per_split;
+    p.tag_mask = f.tag_mask = s.tag_mask;
+    p.keys = k;
+    p.factor = factors;
+    f.keys = reinterpret_cast<const float*>(k);
+    p.error = error;
+    f.error = error;
+    const CUtensorMap ma = make_map_2d(CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, operand, rows, width, kRows, kBlockK, CU_TENSOR_MAP_SWIZZLE_128B);
+    const uint32_t items = ceildiv(rows, kTileRows) * s.splits;
+    auto go = [&](auto kernel) {
+      ensure_dynamic_smem(reinterpret_cast<const void*>(kernel), smem);
+      launch_chained(kernel, std::min(uint32_t(res.sm_count), items), kThreads, smem, stream, ma, mb, p);
+    };
+    switch (p.k_blocks) {
+      case 1: go(label_tc_kernel<1>); break;
+      case 2: go(label_tc_kernel<2>); break;
+      case 3: go(label_tc_kernel<3>); break;
+      default: go(label_tc_kernel<0>);
+    }
+    launch_chained(label_finish_kernel, finish_blocks, 256, 0, stream, f);
+    CUDA_TRY(cudaGetLastError());
+  };
+  f.next = next;
+  f.next_count = words + 2;
+  f.next_cap = y.second_pass() ? y.cap : 0;
+  pass(y.first, a, factor, keys, n_rows, words, nullptr, kFinishRows, ceildiv(n_rows, kFinishRows));
+  res.launches += 3;
+  if (y.second_pass()) {
+    const uint32_t few = std::min<uint32_t>(uint32_t(res.sm_count) * 8, ceildiv(y.cap, 8u));
+    launch_chained(gather_operand_kernel, few, 256, 0, stream, a, factor, next, words + 2, y.cap, width, a2, factor2);
+    f.rows = next;
+    f.next_cap = 0;
+    pass(y.second, a2, factor2, keys2, y.cap, words + 1, words + 2,
+         kSecondRows, std::min<uint32_t>(uint32_t(res.sm_count) * 4, ceildiv(y.cap, kSecondRows)));
+    res.launches += 3;
+  }
+  assign_nearest_listed(res, centers, n_lists, dim_ext, alpha, x_ext, n_rows, last, words + 3, labels, best);
 }
 
 }  // namespace cuvs::neighbors::ivf_pq

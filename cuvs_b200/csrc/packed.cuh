@@ -1,5 +1,5 @@
 // Register-level helpers that several kernels share: two floats in one 64-bit register (one packed instruction for
-// both), the three-input minimum, and a loop whose counter is a compile-time constant.
+// both), the three-input minimum and maximum, and a loop whose counter is a compile-time constant.
 #pragma once
 
 #include <cstdint>
@@ -12,6 +12,17 @@ __device__ __forceinline__ uint64_t dup2(float x)
   uint64_t v;
   asm("mov.b64 %0, {%1, %1};" : "=l"(v) : "f"(x));
   return v;
+}
+__device__ __forceinline__ uint64_t pack2(uint32_t lo, uint32_t hi)
+{
+  uint64_t v;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "r"(lo), "r"(hi));
+  return v;
+}
+// four floats of shared memory as two pairs (volatile: asynchronous copies write them)
+__device__ __forceinline__ void lds128(uint32_t a, uint64_t& x, uint64_t& y)
+{
+  asm volatile("ld.shared.v2.b64 {%0, %1}, [%2];" : "=l"(x), "=l"(y) : "r"(a) : "memory");
 }
 __device__ __forceinline__ float lo2(uint64_t v)
 {
@@ -50,6 +61,13 @@ __device__ __forceinline__ float min3(float a, float b, float c)
 {
   float d;
   asm("min.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
+  return d;
+}
+
+__device__ __forceinline__ float max3(float a, float b, float c)
+{
+  float d;
+  asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
   return d;
 }
 

@@ -98,7 +98,8 @@ void assign_nearest(raft::resources& res, const float* centers, uint32_t n_lists
                     float alpha, const float* x_ext, uint32_t n_rows, uint32_t* labels,
                     unsigned long long* best);
 
-// The same for the rows named in row_list[0 .. *n_listed) (both on the device); other labels stay as they are.
+// The same for the rows named in row_list[0 .. *n_listed) (both on the device), whose `best` is all ones; other labels stay as
+// they are.
 void assign_nearest_listed(raft::resources& res, const float* centers, uint32_t n_lists, uint32_t dim_ext, float alpha,
                            const float* x_ext, uint32_t n_rows, const uint32_t* row_list, const uint32_t* n_listed,
                            uint32_t* labels, unsigned long long* best);

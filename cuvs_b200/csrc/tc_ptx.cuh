@@ -14,6 +14,15 @@ __device__ __forceinline__ uint32_t smem_u32(const void* p)
 {
   return uint32_t(__cvta_generic_to_shared(p));
 }
+// One lane of a converged warp.  tcgen05 instructions take their operands from uniform registers: issued under this predicate
+// by a warp that goes through its loops as a whole they cost a few clocks, in the branch of a given lane (`lane == 0`) some
+// hundred each, for then the compiler cannot know that one thread is there.
+__device__ __forceinline__ bool elect_one()
+{
+  uint32_t e;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xFFFFFFFF;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(e));
+  return e != 0;
+}
 __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count)
 {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count));
@@ -42,6 +51,11 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, uint32_
   }
   return false;
 }
+// The same for a whole warp, with one answer for all of it.
+__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, uint32_t limit)
+{
+  return __all_sync(0xFFFFFFFFu, mbar_wait(bar, parity, limit));
+}
 // A batch whose tensor-core pass timed out, counted in the handle's pinned word: by one thread of the kernel behind that
 // pass (the kernels of a handle run one after the other).
 __device__ __forceinline__ void count_timeout(uint32_t* word)
@@ -57,6 +71,13 @@ __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map
     "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
     ::"r"(dst), "l"(map), "r"(bar), "r"(x), "r"(y)
     : "memory");
+}
+// `bytes` (a multiple of 16) from 16-byte aligned global memory
+__device__ __forceinline__ void bulk_load(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar)
+{
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+               ::"r"(dst), "l"(src), "r"(bytes), "r"(bar)
+               : "memory");
 }
 // generic-proxy writes of shared memory become visible to the tensor core and to TMA
 __device__ __forceinline__ void fence_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }

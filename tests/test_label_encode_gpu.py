@@ -87,7 +87,7 @@ def test_codes(ivf, bits, pq_dim, length, n):
     assert (got <= d.min(2) * (1 + 1e-5) + 1e-9).all() and (codes == d.argmin(2)).mean() > 0.999
 
 
-# resident row tile with two products, with one, and row tile streamed beside the lists
+# one and several K blocks: row tile resident, and streamed beside the lists
 @pytest.mark.parametrize("n,dim,n_lists", [(20000, 62, 1000), (17000, 300, 1100), (17000, 768, 1100)])
 def test_a_wait_that_runs_out_redoes_every_label(ivf, n, dim, n_lists):
     """One list block of every CTA's first tile never comes and the limit is about a millisecond: the labelling kernel gives
@@ -115,3 +115,34 @@ def test_a_wait_that_runs_out_redoes_every_label(ivf, n, dim, n_lists):
     again, m2 = labels()
     assert m0 == 0 and m1 >= 1 and m2 == m1
     assert bool((healthy == timed_out).all()) and bool((healthy == again).all())
+
+
+# more lists within reach of a row than the first pass keeps (four units of eight per column quarter), than a block of the
+# finish kernel has room for, and than the second pass keeps; one, two, three and more K blocks
+@pytest.mark.parametrize("n,dim,n_lists,alike", [(4097, 40, 4096, 64), (9000, 96, 4100, 12), (8200, 128, 2050, 10), (8200, 130, 2050, 10),
+                                                 (17000, 200, 1030, 6), (20000, 64, 1024, 512)])
+def test_many_lists_within_reach(ivf, n, dim, n_lists, alike):
+    """Centres in groups that differ by some 1e-5 of their length: the labels equal those of the exact product (the labelling
+    kernel's waits made to run out)."""
+    from cuvs_b200 import _lib as L
+    rng = np.random.default_rng(dim)
+    groups = make_mixture(-(-n_lists // alike), dim, 40, 0.3, 1)
+    centers = groups[rng.permutation(n_lists) % len(groups)] + 1e-5 * rng.standard_normal((n_lists, dim))
+    centers = centers.astype(np.float32)
+    books = rng.standard_normal((4, dim // 2, 16)).astype(np.float32) if dim % 4 else \
+        rng.standard_normal((4, dim // 4, 16)).astype(np.float32)
+    if dim % 4:
+        books = books[:2]
+    to = lambda a: torch.from_numpy(np.ascontiguousarray(a)).cuda()  # noqa: E731
+    eye = np.eye(dim, dtype=np.float32)
+    index = ivf.build_precomputed(ivf.IndexParams(n_lists=n_lists, pq_dim=len(books), pq_bits=4), dim, to(books), to(centers),
+                                  to(centers), to(eye))
+    x = to((groups[rng.integers(0, len(groups), n)] + 0.05 * rng.standard_normal((n, dim))).astype(np.float32))
+    labels = ivf.transform(index, x)[0].to(torch.int64)
+    lib = L.load()
+    try:
+        L.check(lib.cuvsB200SetCoarseWaitTest(1000, 1))
+        exact = ivf.transform(index, x)[0].to(torch.int64)
+    finally:
+        L.check(lib.cuvsB200SetCoarseWaitTest(0, 0))
+    assert bool((labels == exact).all())
