@@ -559,6 +559,457 @@ encode_subspaces_kernel(const float* __restrict__ x, uint32_t x_stride, const ui
   }
 }
 
+// The same codes through a table of cells, for codewords of at most four components and many vectors: the space around a
+// subspace's codewords is cut into kCells cells, and a cell names the codewords that can be the nearest one of a point in it,
+// so that a vector looks at those instead of all of them: of 256 codewords some 2 with one or two components, 5 with three,
+// 12 with four (k-means codebooks of normal and of heavy-tailed residuals).
+//
+// An axis is cut evenly in u = z / sqrt(1 + z^2), z the distance to the mean codeword in units of twice the mean deviation: fine
+// cells where codewords are dense (even cuts of the axis itself: 6 codewords instead of 2 on heavy tails).
+//
+// A codeword c is left out of a cell where some other c' is nearer at every point of it by more than rounding can hide:
+// |x - c'|^2 - |x - c|^2 is linear in x, so its maximum over the cell (a little enlarged: the cell of a point is found with
+// rounding) is that of a corner.  What is left always holds the codeword that the comparison of all distances finds, and
+// is compared in the same order with the same arithmetic; points far outside, NaN among them, are compared with all.
+constexpr uint32_t kCells = 4096, kCellSpill = 16384;
+template <uint32_t kLen>
+struct cell_shape {
+  static constexpr uint32_t axis  = kLen == 1 ? 4096u : (kLen == 2 ? 64u : (kLen == 3 ? 16u : 8u));
+  static constexpr uint32_t bytes = kLen <= 2 ? 8u : 16u;   // of a cell
+  static constexpr uint32_t codes = bytes - 1u;             // that fit it
+  static constexpr uint32_t subs  = kLen <= 2 ? 4u : 2u;    // subspaces of a block of the encoder
+  static constexpr uint32_t sure  = kLen <= 2 ? 3u : (kLen == 3 ? 4u : 8u);  // codewords looked at without asking how many there are
+  // cells of a warp along axis k, and warps of a patch of 256 cells
+  static __host__ __device__ constexpr uint32_t lanes(uint32_t k)
+  {
+    return kLen == 1 ? 32u : (kLen == 2 ? (k == 0 ? 8u : 4u) : (kLen == 3 ? (k == 2 ? 2u : 4u) : (k == 0 ? 4u : 2u)));
+  }
+  static __host__ __device__ constexpr uint32_t warps(uint32_t k) { return kLen == 1 ? 8u : (kLen == 2 ? (k == 0 ? 2u : 4u) : (kLen == 4 && k == 0 ? 1u : 2u)); }
+};
+// A table: cells, then the codes of long cells.  A cell: count, codes (unused places repeat the last one); count kCellLong:
+// {-, codes (byte 1), -, offset of them in `spill` (bytes 4-7)}; kCellAll: every codeword.  frame: per component {mean, 1 / deviation,
+// low end in u, cells per u}, ends: {lowest, highest} value that the edge cells hold.
+constexpr uint32_t kCellLong = 0xFEu, kCellAll = 0xFFu;
+template <uint32_t kLen>
+struct code_table {
+  uint4 cell[kCells * cell_shape<kLen>::bytes / 16];
+  uint8_t spill[kCellSpill];
+  float4 frame[kLen];
+  float2 ends[4];
+  uint32_t n_spill, pad[3];
+};
+
+// Block: a patch of 256 cells of subspace blockIdx.x.  The codewords that can matter are found for the patch, of those the ones
+// for a warp's 32 cells, of those the ones for a cell.  What bounds it: the instructions of the comparisons (from the whole
+// codebook for every cell: 119 us instead of 43 for 64 subspaces of two components and 256 codewords).
+template <uint32_t kLen>
+__global__ void __launch_bounds__(256)
+code_cells_kernel(const float* __restrict__ pq_centers, uint32_t book, code_table<kLen>* __restrict__ tables)
+{
+  using shape = cell_shape<kLen>;
+  constexpr uint32_t kAxis = shape::axis, kShort = 64;
+  __shared__ float s_c[kLen][256];
+  constexpr uint32_t kFirst = kLen <= 2 ? 4u : 16u;  // codewords nearest to a warp's middle that the others are compared with
+  __shared__ uint8_t s_left[256], s_near[8][256], s_first[8][kFirst];  // codewords that matter to the patch, to a warp: ascending
+  __shared__ uint8_t s_kept[256][kShort + 4];
+  __shared__ float s_red[3][8];
+  __shared__ unsigned long long s_mid[8];
+  __shared__ uint32_t s_warp[8];
+  const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
+  auto& t = tables[blockIdx.x];
+  for (uint32_t i = tid; i < kLen * book; i += 256) { s_c[i / book][i % book] = pq_centers[size_t(blockIdx.x) * kLen * book + i]; }
+  __syncthreads();
+  auto block_reduce = [&](float a, float b, float c, float& mn, float& mx, float& sum) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      a = fminf(a, __shfl_xor_sync(kFullMask, a, o));
+      b = fmaxf(b, __shfl_xor_sync(kFullMask, b, o));
+      c += __shfl_xor_sync(kFullMask, c, o);
+    }
+    if (lane == 0) {
+      s_red[0][warp] = a;
+      s_red[1][warp] = b;
+      s_red[2][warp] = c;
+    }
+    __syncthreads();
+    mn = s_red[0][0]; mx = s_red[1][0]; sum = s_red[2][0];
+    for (uint32_t w = 1; w < 8; w++) {
+      mn = fminf(mn, s_red[0][w]);
+      mx = fmaxf(mx, s_red[1][w]);
+      sum += s_red[2][w];
+    }
+    __syncthreads();
+  };
+  float lo[kLen], hi[kLen], mean[kLen], dev[kLen], range = 0.0f;
+  bool usable = true;
+#pragma unroll
+  for (uint32_t k = 0; k < kLen; k++) {
+    const float v = s_c[k][min(tid, book - 1u)], in = tid < book ? 1.0f : 0.0f;
+    float x0, x1, sum;
+    block_reduce(v, v, v * in, lo[k], hi[k], sum);
+    mean[k] = sum / float(book);
+    block_reduce(v, v, fabsf(v - mean[k]) * in, x0, x1, sum);
+    dev[k] = 2.0f * sum / float(book);
+    range  = fmaxf(range, hi[k] - lo[k]);
+    usable = __syncthreads_and(fabsf(v) < 1e12f) && usable;  // (false for NaN)
+  }
+  // (all codewords equal: the first one wins everywhere)
+  const bool alone = usable && range == 0.0f;
+  // (squares of a box this small or large would leave fp32)
+  usable = usable && range > 1e-12f;
+  constexpr float kFarOut = kLen <= 2 ? 1.0f : 0.25f;  // (edge cells that reach farther name more codewords)
+  float u0[kLen], du[kLen], end0[kLen], end1[kLen];  // low end and width of the cells in u, ends of the edge cells
+#pragma unroll
+  for (uint32_t k = 0; k < kLen; k++) {
+    dev[k]        = fmaxf(dev[k], 0.01f * range);
+    const float r = fmaxf(hi[k] - lo[k], 0.01f * range);
+    const float z0 = (lo[k] - 0.25f * r - mean[k]) / dev[k], z1 = (hi[k] + 0.25f * r - mean[k]) / dev[k];
+    u0[k]   = z0 * rsqrtf(1.0f + z0 * z0);
+    du[k]   = (z1 * rsqrtf(1.0f + z1 * z1) - u0[k]) / float(kAxis);
+    end0[k] = lo[k] - 0.25f * r - kFarOut * range;
+    end1[k] = hi[k] + 0.25f * r + kFarOut * range;
+    // (the ends of a cell are off by rounding of their own size: 1/64 of its width has to cover that)
+    usable = usable && dev[k] * du[k] > 1.6e-5f * fmaxf(fabsf(lo[k]), fabsf(hi[k]));
+    if (blockIdx.y == 0 && tid == 0) {
+      t.frame[k] = make_float4(mean[k], 1.0f / dev[k], u0[k], 1.0f / du[k]);
+    }
+  }
+  if (blockIdx.y == 0 && tid == 0) {
+    // (not usable: nothing lies between the ends)
+#pragma unroll
+    for (uint32_t k = 0; k < kLen; k++) {
+      t.ends[k] = usable ? make_float2(end0[k], end1[k]) : (alone ? make_float2(-INFINITY, INFINITY) : make_float2(INFINITY, -INFINITY));
+    }
+  }
+  // value at cell position p of axis k
+  auto at = [&](uint32_t k, float p) {
+    const float u = fminf(fmaxf(u0[k] + p * du[k], -0.9999999f), 0.9999999f);
+    return mean[k] + dev[k] * u * rsqrtf(1.0f - u * u);
+  };
+  // ends of cells i .. i + n of axis k, enlarged by 1/64 of a cell (a point's cell position is off by less than 2^-8)
+  auto span = [&](uint32_t k, uint32_t i, uint32_t n, float& a, float& b) {
+    a = i == 0 ? end0[k] : at(k, float(i) - 0.015625f);
+    b = i + n == kAxis ? end1[k] : at(k, float(i + n) + 0.015625f);
+  };
+  // `far`: no point of the box is farther from a codeword (squared); rounding of two distances and of the difference below is
+  // at most 20 roundings of 2^-24 of it
+  auto far_of = [&](const float (&a)[kLen], const float (&b)[kLen]) {
+    float far = 0.0f;
+#pragma unroll
+    for (uint32_t k = 0; k < kLen; k++) {
+      const float d = fmaxf(b[k] - lo[k], hi[k] - a[k]);
+      far           = __fmaf_rn(d, d, far);
+    }
+    return far;
+  };
+  // codeword p is nearer than e in all of the box
+  auto beats = [&](uint32_t p, uint32_t e, const float (&a)[kLen], const float (&b)[kLen], float margin) {
+    float g = 0.0f;
+#pragma unroll
+    for (uint32_t k = 0; k < kLen; k++) {
+      const float cp = s_c[k][p], ce = s_c[k][e], d = cp - ce;
+      g += fmaxf(d * ((cp - a[k]) + (ce - a[k])), d * ((cp - b[k]) + (ce - b[k])));
+    }
+    return g < -margin;
+  };
+  auto to_middle = [&](uint32_t e, const float (&a)[kLen], const float (&b)[kLen]) {
+    float d2 = 0.0f;
+#pragma unroll
+    for (uint32_t k = 0; k < kLen; k++) {
+      const float d = 0.5f * (a[k] + b[k]) - s_c[k][e];
+      d2            = __fmaf_rn(d, d, d2);
+    }
+    return d2;
+  };
+  // this thread's cell, its warp's and the block's
+  uint32_t cell = 0, stride = 1, patch = blockIdx.y, in_lane = lane, in_warp = warp;
+  float a[kLen], b[kLen], wa[kLen], wb[kLen], pa[kLen], pb[kLen];
+#pragma unroll
+  for (uint32_t k = 0; k < kLen; k++) {
+    const uint32_t nl = shape::lanes(k), nw = shape::warps(k), np = kAxis / (nl * nw);
+    const uint32_t p0 = (patch % np) * nl * nw, w0 = p0 + (in_warp % nw) * nl, i = w0 + in_lane % nl;
+    patch /= np;
+    in_warp /= nw;
+    in_lane /= nl;
+    cell += i * stride;
+    stride *= kAxis;
+    span(k, i, 1, a[k], b[k]);
+    span(k, w0, nl, wa[k], wb[k]);
+    span(k, p0, nl * nw, pa[k], pb[k]);
+  }
+  // e is beaten by one of the n codewords of `list` in the box, or equals one of lower code (which wins every tie)
+  auto beaten_by = [&](const uint8_t* list, uint32_t n, uint32_t e, const float (&a)[kLen], const float (&b)[kLen], float margin) {
+    for (uint32_t o = 0; o < n; o++) {
+      const uint32_t p = list[o];
+      bool same        = p < e;
+#pragma unroll
+      for (uint32_t k = 0; k < kLen; k++) { same = same && s_c[k][p] == s_c[k][e]; }
+      if (same || beats(p, e, a, b, margin)) { return true; }
+    }
+    return false;
+  };
+  uint32_t n_near = 0;
+  if (usable) {
+    // the patch: what the one nearest to its middle leaves
+    auto nearest = [&](uint64_t key) {
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) {
+        const uint64_t other = shfl_u64(key, int(lane) ^ o);
+        key                  = other < key ? other : key;
+      }
+      return key;
+    };
+    auto key_of = [&](uint32_t e, const float (&a)[kLen], const float (&b)[kLen]) {
+      return (uint64_t(__float_as_uint(to_middle(e, a, b))) << 32) | e;
+    };
+    uint64_t key = nearest(tid < book ? key_of(tid, pa, pb) : ~0ull);
+    if (lane == 0) { s_mid[warp] = key; }
+    __syncthreads();
+    for (uint32_t w = 0; w < 8; w++) { key = s_mid[w] < key ? s_mid[w] : key; }
+    const bool stays = tid < book && !beats(uint32_t(key), tid, pa, pb, far_of(pa, pb) * 4e-6f);
+    const unsigned m = __ballot_sync(kFullMask, stays);
+    if (lane == 0) { s_warp[warp] = __popc(m); }
+    __syncthreads();
+    uint32_t at = 0, n_left = 0;
+    for (uint32_t w = 0; w < 8; w++) {
+      if (w < warp) { at += s_warp[w]; }
+      n_left += s_warp[w];
+    }
+    if (stays) { s_left[at + __popc(m & ((1u << lane) - 1u))] = uint8_t(tid); }
+    __syncthreads();
+    // the warp: what the kFirst nearest to its middle leave
+    uint64_t keys[8];
+#pragma unroll
+    for (uint32_t i = 0; i < 8; i++) { keys[i] = i * 32u + lane < n_left ? key_of(s_left[i * 32u + lane], wa, wb) : ~0ull; }
+    const uint32_t n_first = min(kFirst, n_left);
+    for (uint32_t f = 0; f < n_first; f++) {
+      uint64_t mine = keys[0];
+#pragma unroll
+      for (uint32_t i = 1; i < 8; i++) { mine = keys[i] < mine ? keys[i] : mine; }
+      const uint64_t first = nearest(mine);
+#pragma unroll
+      for (uint32_t i = 0; i < 8; i++) { keys[i] = keys[i] == first ? ~0ull : keys[i]; }
+      if (lane == 0) { s_first[warp][f] = uint8_t(first); }
+    }
+    __syncwarp();
+    const float w_margin = far_of(wa, wb) * 4e-6f;
+    for (uint32_t i0 = 0; i0 < n_left; i0 += 32) {
+      const uint32_t c    = i0 + lane < n_left ? s_left[i0 + lane] : 0u;
+      const bool in       = i0 + lane < n_left && !beaten_by(s_first[warp], n_first, c, wa, wb, w_margin);
+      const unsigned in_m = __ballot_sync(kFullMask, in);
+      if (in) { s_near[warp][n_near + __popc(in_m & ((1u << lane) - 1u))] = uint8_t(c); }
+      n_near += __popc(in_m);
+    }
+    __syncwarp();
+  }
+  uint32_t n = 0xFFFFu;
+  if (alone) {
+    n              = 1;
+    s_kept[tid][0] = 0;
+  }
+  if (usable) {
+    // the cell
+    const float margin = far_of(a, b) * 4e-6f;
+    uint32_t mid = 0;
+    float best   = INFINITY;
+    for (uint32_t i = 0; i < n_near; i++) {
+      const float d2 = to_middle(s_near[warp][i], a, b);
+      if (d2 < best) {
+        best = d2;
+        mid  = s_near[warp][i];
+      }
+    }
+    // (most are beaten by the one nearest to the middle, nearly all others by one already kept)
+    n = 0;
+    for (uint32_t i = 0; i < n_near && n <= kShort; i++) {
+      const uint32_t e = s_near[warp][i];
+      if (!beats(mid, e, a, b, margin) && !beaten_by(s_kept[tid], n, e, a, b, margin)) {
+        if (n < kShort) { s_kept[tid][n] = uint8_t(e); }
+        n++;
+      }
+    }
+    if (n <= kShort) {
+      // without those that one kept after them beats
+      uint32_t m = 0;
+      for (uint32_t i = 0; i < n; i++) {
+        const uint32_t e = s_kept[tid][i];
+        if (!beaten_by(s_kept[tid] + i + 1, n - i - 1, e, a, b, margin)) { s_kept[tid][m++] = uint8_t(e); }
+      }
+      n = m;
+    }
+  }
+  uint32_t w[shape::bytes / 4] = {kCellAll};
+  if (n <= shape::codes) {
+    w[0] = n;
+#pragma unroll
+    for (uint32_t i = 0; i < shape::codes; i++) { w[(i + 1) / 4] |= uint32_t(s_kept[tid][min(i, n - 1u)]) << (((i + 1) & 3u) * 8u); }
+  } else if (n <= kShort) {
+    const uint32_t from = atomicAdd(&t.n_spill, n);
+    if (from + n <= kCellSpill) {
+      for (uint32_t i = 0; i < n; i++) { t.spill[from + i] = s_kept[tid][i]; }
+      w[0] = kCellLong | (n << 8);
+      w[1] = from;
+    }
+  }
+  auto* out = reinterpret_cast<uint32_t*>(t.cell) + cell * (shape::bytes / 4);
+#pragma unroll
+  for (uint32_t i = 0; i < shape::bytes / 4; i++) { out[i] = w[i]; }
+}
+
+// Block: the tables of a few subspaces in shared memory, `rows_per_block` vectors, a thread per vector.  What bounds it: the
+// instructions and shared-memory wavefronts of the look-ups (a cell, then the components of a few codewords, each at random
+// places).  1,000,003 rows of 48 x 2 components, 256 codewords: 2,180 us by comparing all, 361 us so.
+template <uint32_t kLen>
+__global__ void __launch_bounds__(1024, 1)
+encode_cells_kernel(const float* __restrict__ x, uint32_t x_stride, const uint32_t* __restrict__ order,
+                    const uint32_t* __restrict__ labels, const float* __restrict__ centers, uint32_t c_stride, uint32_t n,
+                    const float* __restrict__ pq_centers, const code_table<kLen>* __restrict__ tables, uint32_t pq_dim,
+                    uint32_t book, uint32_t rows_per_block, int vec, uint8_t* __restrict__ codes)
+{
+  using shape = cell_shape<kLen>;
+  constexpr uint32_t kSub = shape::subs, kN = kSub * kLen, kAxis = shape::axis, kWords = shape::bytes / 4;
+  extern __shared__ __align__(16) uint8_t s_tables[];
+  auto* s_book = reinterpret_cast<float*>(s_tables + size_t(kSub) * kCells * shape::bytes);  // [kSub][book][kLen]
+  const uint32_t tid = threadIdx.x;
+  const uint32_t j0 = blockIdx.x * kSub, nj = min(kSub, pq_dim - j0);
+  constexpr uint32_t kPer = kCells * shape::bytes / 16;
+  for (uint32_t i = tid; i < nj * kPer; i += 1024u) { reinterpret_cast<uint4*>(s_tables)[i] = __ldg(tables[j0 + i / kPer].cell + i % kPer); }
+  for (uint32_t i = tid; i < nj * kLen * book; i += 1024u) {
+    const uint32_t s = i / (kLen * book), k = i / book % kLen, e = i % book;
+    s_book[(s * book + e) * kLen + k] = __ldg(pq_centers + size_t(j0) * kLen * book + i);
+  }
+  __shared__ float4 s_frame[kN];
+  __shared__ float2 s_ends[kN];
+  if (tid < nj * kLen) {
+    s_frame[tid] = __ldg(&tables[j0 + tid / kLen].frame[tid % kLen]);
+    s_ends[tid]  = __ldg(&tables[j0 + tid / kLen].ends[tid % kLen]);
+  }
+  __syncthreads();
+  const uint32_t end = min(n, (blockIdx.y + 1u) * rows_per_block);
+  for (uint32_t i = blockIdx.y * rows_per_block + tid; i < end; i += 1024u) {
+    const uint32_t row = order ? __ldg(order + i) : i;
+    const float* xr    = x + size_t(row) * x_stride + j0 * kLen;
+    const float* cr    = centers ? centers + size_t(__ldg(labels + row)) * c_stride + j0 * kLen : nullptr;
+    float r[kN];
+    if (kN % 4 == 0 && vec && nj == kSub) {
+#pragma unroll
+      for (uint32_t v = 0; v + 4 <= kN; v += 4) {
+        const float4 q = __ldg(reinterpret_cast<const float4*>(xr + v));
+        r[v] = q.x; r[v + 1] = q.y; r[v + 2] = q.z; r[v + 3] = q.w;
+      }
+      if (centers) {
+#pragma unroll
+        for (uint32_t v = 0; v + 4 <= kN; v += 4) {
+          const float4 c = __ldg(reinterpret_cast<const float4*>(cr + v));
+          r[v] = __fsub_rn(r[v], c.x); r[v + 1] = __fsub_rn(r[v + 1], c.y);
+          r[v + 2] = __fsub_rn(r[v + 2], c.z); r[v + 3] = __fsub_rn(r[v + 3], c.w);
+        }
+      }
+    } else {
+#pragma unroll
+      for (uint32_t v = 0; v < kN; v++) {
+        r[v] = v < nj * kLen ? __ldg(xr + v) : 0.0f;
+        if (centers && v < nj * kLen) { r[v] = __fsub_rn(r[v], __ldg(cr + v)); }
+      }
+    }
+    uint32_t cell[kSub][kWords], from[kSub], code[kSub];
+    float best[kSub];
+    auto look = [&](uint32_t s, uint32_t e) {
+      const float* c = s_book + (s * book + e) * kLen;
+      float y[kLen];
+      if constexpr (kLen == 2) {
+        const float2 v = *reinterpret_cast<const float2*>(c);
+        y[0] = v.x; y[1] = v.y;
+      } else if constexpr (kLen == 4) {
+        const float4 v = *reinterpret_cast<const float4*>(c);
+        y[0] = v.x; y[1] = v.y; y[2] = v.z; y[3] = v.w;
+      } else {
+#pragma unroll
+        for (uint32_t k = 0; k < kLen; k++) { y[k] = c[k]; }
+      }
+      float d2 = 0.0f;
+#pragma unroll
+      for (uint32_t k = 0; k < kLen; k++) {
+        const float d = __fsub_rn(r[s * kLen + k], y[k]);
+        d2            = k == 0 ? __fmul_rn(d, d) : __fmaf_rn(d, d, d2);  // the chain starts from +0
+      }
+      if (d2 < best[s]) {
+        best[s] = d2;
+        code[s] = e;
+      }
+    };
+#pragma unroll
+    for (uint32_t s = 0; s < kSub; s++) {
+      uint32_t pos = 0, stride = 1;
+      bool in = s < nj;
+#pragma unroll
+      for (uint32_t k = 0; k < kLen; k++) {
+        const float4 f = s_frame[s * kLen + k];
+        const float2 e = s_ends[s * kLen + k];
+        const float v = r[s * kLen + k], z = (v - f.x) * f.y, u = z * rsqrtf(1.0f + z * z);
+        in          = in && v >= e.x && v <= e.y;
+        const int p = min(max(int((u - f.z) * f.w), 0), int(kAxis) - 1);
+        pos += uint32_t(p) * stride;
+        stride *= kAxis;
+      }
+      from[s]        = (s * kCells + pos) * shape::bytes;
+      const auto* cw = reinterpret_cast<const uint32_t*>(s_tables + (s < nj ? from[s] : 0u));
+#pragma unroll
+      for (uint32_t i = 0; i < kWords; i += 2) {
+        const uint2 v = *reinterpret_cast<const uint2*>(cw + i);
+        cell[s][i] = v.x; cell[s][i + 1] = v.y;
+      }
+      if (!in) { cell[s][0] = kCellAll; }
+      best[s] = INFINITY;
+      code[s] = 0;
+    }
+#pragma unroll
+    for (uint32_t q = 0; q < shape::sure; q++) {
+#pragma unroll
+      for (uint32_t s = 0; s < kSub; s++) {
+        if ((cell[s][0] & 0xFFu) <= shape::codes) { look(s, (cell[s][(q + 1) / 4] >> (((q + 1) & 3u) * 8u)) & 0xFFu); }
+      }
+    }
+#pragma unroll
+    for (uint32_t s = 0; s < kSub; s++) {
+      const uint32_t count = cell[s][0] & 0xFFu;
+      if (count <= shape::codes) {
+        for (uint32_t q = shape::sure; q < count; q++) { look(s, s_tables[from[s] + 1u + q]); }
+      } else if (count == kCellLong) {
+        const uint8_t* more = tables[j0 + s].spill + cell[s][1];
+        for (uint32_t q = 0; q < ((cell[s][0] >> 8) & 0xFFu); q++) { look(s, __ldg(more + q)); }
+      } else if (s < nj) {
+        for (uint32_t e = 0; e < book; e++) { look(s, e); }
+      }
+    }
+    uint8_t* o = codes + size_t(i) * pq_dim + j0;
+    if (kSub == 4 && nj == 4 && (reinterpret_cast<uintptr_t>(o) & 3u) == 0) {
+      uint32_t w = 0;
+#pragma unroll
+      for (uint32_t s = 0; s < kSub; s++) { w |= code[s] << (8u * s); }
+      *reinterpret_cast<uint32_t*>(o) = w;
+    } else {
+#pragma unroll
+      for (uint32_t s = 0; s < kSub; s++) {
+        if (s < nj) { o[s] = uint8_t(code[s]); }
+      }
+    }
+  }
+}
+
+// fn(std::integral_constant<uint32_t, components per subspace>) for the lengths that have tables of cells
+template <typename Fn>
+auto with_cell_len(uint32_t len, Fn&& fn)
+{
+  using std::integral_constant;
+  switch (len) {
+    case 1: return fn(integral_constant<uint32_t, 1>{});
+    case 2: return fn(integral_constant<uint32_t, 2>{});
+    case 3: return fn(integral_constant<uint32_t, 3>{});
+    default: return fn(integral_constant<uint32_t, 4>{});
+  }
+}
+
 // Byte codes of vectors taken in `order` -> interleaved list slots (and ids).  A warp handles 32 vectors and one 16-byte
 // piece at a time: neighbours in a list are neighbours in the warp, so its stores are runs of 16-byte pieces.
 __global__ void place_interleaved_kernel(const uint8_t* __restrict__ codes, const uint32_t* __restrict__ labels,
@@ -1027,10 +1478,24 @@ void make_rotation(uint32_t rot_dim, uint32_t dim, bool force_random, std::vecto
 }
 
 // Scratch of launch_encode for up to n vectors: byte codes, and with a rotation the differences before and after it.
-size_t encode_scratch_bytes(const index<int64_t>& idx, uint64_t n)
+// Whether n vectors are encoded through tables of cells: where making those costs less than they save.  256 codewords, 96
+// dimensions, making + encoding / comparing all (us): one component 36 + 24 / 67 at 20,000 rows, 40 + 137 / 468 at 200,000; two
+// 51 + 17 / 70 and 55 + 83 / 449; three 158 + 69 / 159 at 60,000, 149 + 167 / 450 at 200,000; four 640 + 187 / 449 at 200,000.
+bool encode_by_cells(const index<int64_t>& idx, uint64_t n)
+{
+  const uint32_t len = idx.pq_len();
+  if (idx.codebook_kind() != codebook_gen::PER_SUBSPACE || len > 4 || idx.pq_bits() < 7) { return false; }
+  return n >= (len <= 2 ? 24'576u : (len == 3 ? 131'072u : 393'216u));
+}
+size_t code_table_bytes(const index<int64_t>& idx)
+{
+  return idx.pq_dim() * with_cell_len(idx.pq_len(), [](auto len) { return sizeof(code_table<decltype(len)::value>); });
+}
+size_t encode_scratch_bytes(const index<int64_t>& idx, uint64_t n, bool cells)
 {
   if (idx.codebook_kind() == codebook_gen::PER_CLUSTER) { return 0; }
   ws_layout lay;
+  if (cells) { lay.add(code_table_bytes(idx)); }
   lay.add(n * idx.pq_dim());
   if (!idx.rotation_is_identity()) {
     lay.add(n * idx.dim() * 4);
@@ -1039,11 +1504,12 @@ size_t encode_scratch_bytes(const index<int64_t>& idx, uint64_t n)
   return lay.total();
 }
 
-// `to_lists`: write slots of the index's lists (and ids); else plain rows of codes_out.
+// `to_lists`: write slots of the index's lists (and ids); else plain rows of codes_out.  `cells`: through tables of cells, made
+// first where make_tables is set (else they are in `scratch` from the call before).
 void launch_encode(raft::resources& res, const index<int64_t>& idx, const float* x_ext,
                    const uint32_t* labels, const uint32_t* order, const uint32_t* slots, uint32_t n,
                    bool to_lists, uint8_t* codes_out, int64_t* ids_out, const int64_t* src_ids,
-                   int64_t id_base, void* scratch)
+                   int64_t id_base, void* scratch, bool cells, bool make_tables)
 {
   if (n == 0) { return; }
   const uint32_t row_bytes = ceildiv(idx.pq_dim() * idx.pq_bits(), 8u);
@@ -1067,6 +1533,7 @@ void launch_encode(raft::resources& res, const index<int64_t>& idx, const float*
   const uint32_t pq_dim = idx.pq_dim(), book = idx.pq_book_size();
   ws_layout lay;
   char* ws     = static_cast<char*>(scratch);
+  void* tables = cells ? ws + lay.add(code_table_bytes(idx)) : nullptr;
   auto* bytes  = reinterpret_cast<uint8_t*>(ws + lay.add(size_t(n) * pq_dim));
   // plain rows of 8-bit codes are the byte codes themselves
   const bool direct = !to_lists && idx.pq_bits() == 8;
@@ -1098,14 +1565,38 @@ void launch_encode(raft::resources& res, const index<int64_t>& idx, const float*
       x, x_stride, x_order, labels, c, dim_ext, n, idx.pq_centers(), pq_dim, len, book, in_smem, bytes, pq_dim);
     CUDA_TRY(cudaGetLastError());
   };
+  auto go_cells = [&](auto lenc) {
+    constexpr uint32_t kLen = decltype(lenc)::value;
+    using shape             = cell_shape<kLen>;
+    auto* tab               = static_cast<code_table<kLen>*>(tables);
+    if (make_tables) {
+      CUDA_TRY(cudaMemset2DAsync(&tab->n_spill, sizeof(*tab), 0, 4, pq_dim, res.stream));
+      code_cells_kernel<kLen><<<dim3(pq_dim, kCells / 256), 256, 0, res.stream>>>(idx.pq_centers(), book, tab);
+      res.launches++;
+    }
+    const size_t smem = size_t(shape::subs) * (kCells * shape::bytes + book * kLen * 4);
+    ensure_dynamic_smem(reinterpret_cast<const void*>(encode_cells_kernel<kLen>), smem);
+    // about two blocks per SM, each reading its tables once
+    const uint32_t groups = ceildiv(pq_dim, shape::subs);
+    const uint32_t shares = std::max(1u, 2u * uint32_t(res.sm_count) / groups);
+    const uint32_t rows   = round_up(ceildiv(n, shares), 1024u);
+    const bool vec        = x_stride % 4 == 0 && dim_ext % 4 == 0 && (reinterpret_cast<uintptr_t>(x) & 15u) == 0;
+    encode_cells_kernel<kLen><<<dim3(groups, ceildiv(n, rows)), 1024, smem, res.stream>>>(
+      x, x_stride, x_order, labels, c, dim_ext, n, idx.pq_centers(), tab, pq_dim, book, rows, vec, bytes);
+    CUDA_TRY(cudaGetLastError());
+  };
   using std::integral_constant;
-  switch (len) {
-    case 1: go(integral_constant<uint32_t, 1>{}); break;
-    case 2: go(integral_constant<uint32_t, 2>{}); break;
-    case 3: go(integral_constant<uint32_t, 3>{}); break;
-    case 4: go(integral_constant<uint32_t, 4>{}); break;
-    case 8: go(integral_constant<uint32_t, 8>{}); break;
-    default: go(integral_constant<uint32_t, 0>{});
+  if (cells) {
+    with_cell_len(len, go_cells);
+  } else {
+    switch (len) {
+      case 1: go(integral_constant<uint32_t, 1>{}); break;
+      case 2: go(integral_constant<uint32_t, 2>{}); break;
+      case 3: go(integral_constant<uint32_t, 3>{}); break;
+      case 4: go(integral_constant<uint32_t, 4>{}); break;
+      case 8: go(integral_constant<uint32_t, 8>{}); break;
+      default: go(integral_constant<uint32_t, 0>{});
+    }
   }
   res.launches++;
   if (direct) { return; }
@@ -1337,7 +1828,7 @@ void extend_list(raft::resources& res, index<int64_t>* idx, const void* new_vect
   const label_ctx lc = labeling_of(idx->metric());
   dev_array<float> x_ext(size_t(n_rows) * idx->dim_ext());
   dev_array<uint32_t> labels(n_rows), slots(n_rows);
-  dev_array<uint8_t> scratch(encode_scratch_bytes(*idx, n_rows));
+  dev_array<uint8_t> scratch(encode_scratch_bytes(*idx, n_rows, false));
   to_float_ext(res, new_vectors, dtype, n_rows, 1, idx->dim(), idx->dim_ext(), lc.pad, lc.normalize,
                x_ext.data());
   fill_u32_kernel<<<ceildiv(n_rows, 256u), 256, 0, res.stream>>>(labels.data(), n_rows, label);
@@ -1346,7 +1837,7 @@ void extend_list(raft::resources& res, index<int64_t>* idx, const void* new_vect
   res.launches += 3;
   // ids were written by extend_list_prepare: the encoder gets the same array, so it rewrites them
   launch_encode(res, *idx, x_ext.data(), labels.data(), nullptr, slots.data(), n_rows, true, idx->codes(),
-                idx->ids(), new_indices, 0, scratch.data());
+                idx->ids(), new_indices, 0, scratch.data(), false, false);
   res.sync();
 }
 
@@ -1385,6 +1876,7 @@ void extend_any(raft::resources& res, const void* new_vectors, elem_t dtype, int
   const uint32_t dim = idx->dim(), dim_ext = idx->dim_ext(), n_lists = idx->n_lists();
   const label_ctx lc   = labeling_of(idx->metric());
   const uint64_t chunk = std::min<uint64_t>(n, chunk_rows_for(dim_ext));
+  const bool cells     = encode_by_cells(*idx, n);
 
   int end_bit = 1;
   while ((1ull << end_bit) < n_lists) { end_bit++; }
@@ -1410,7 +1902,7 @@ void extend_any(raft::resources& res, const void* new_vectors, elem_t dtype, int
   const size_t o_staging = lay.add(on_device ? 0 : chunk * row_bytes);
   const size_t o_ids     = lay.add(on_device || !new_indices ? 0 : chunk * 8);
   // (labelling and encoding take turns)
-  const size_t o_work    = lay.add(std::max(nearest_labeler::bytes(res, chunk, n_lists, dim), encode_scratch_bytes(*idx, chunk)));
+  const size_t o_work    = lay.add(std::max(nearest_labeler::bytes(res, chunk, n_lists, dim), encode_scratch_bytes(*idx, chunk, cells)));
   res.scratch.reserve(lay.total());
   char* ws        = res.scratch.base();
   auto* x_ext     = reinterpret_cast<float*>(ws + o_x);
@@ -1465,7 +1957,7 @@ void extend_any(raft::resources& res, const void* new_vectors, elem_t dtype, int
       ids_chunk = reinterpret_cast<const int64_t*>(ws + o_ids);
     }
     launch_encode(res, *idx, x_ext, labels + r0, order, slots, nr, true, idx->codes(), idx->ids(), ids_chunk, int64_t(r0),
-                  ws + o_work);
+                  ws + o_work, cells, r0 == 0);
     if (r0 + chunk < n) {
       // rows of the chunk are placed
       histogram_kernel<<<ceildiv(nr, 256u), 256, 0, stream>>>(labels + r0, nr, fill);
@@ -1489,11 +1981,12 @@ void transform_any(raft::resources& res, const index<int64_t>& idx, const void* 
   const uint32_t dim = idx.dim(), dim_ext = idx.dim_ext();
   const label_ctx lc   = labeling_of(idx.metric());
   const uint64_t chunk = std::min<uint64_t>(n, chunk_rows_for(dim_ext));
+  const bool cells     = encode_by_cells(idx, n);
   const uint32_t flat  = ceildiv(idx.pq_dim() * idx.pq_bits(), 8u);
   ws_layout lay;
   const size_t o_x     = lay.add(chunk * dim_ext * 4);
   const size_t o_label = lay.add(nearest_labeler::bytes(res, chunk, idx.n_lists(), dim));
-  const size_t o_enc   = lay.add(encode_scratch_bytes(idx, chunk));
+  const size_t o_enc   = lay.add(encode_scratch_bytes(idx, chunk, cells));
   res.scratch.reserve(lay.total());
   char* ws    = res.scratch.base();
   auto* x_ext = reinterpret_cast<float*>(ws + o_x);
@@ -1504,7 +1997,7 @@ void transform_any(raft::resources& res, const index<int64_t>& idx, const void* 
     to_float_ext(res, src, dtype, nr, 1, dim, dim_ext, lc.pad, lc.normalize, x_ext);
     labeler.run(x_ext, nr, out_labels + r0);
     launch_encode(res, idx, x_ext, out_labels + r0, nullptr, nullptr, nr, false, out_codes + r0 * flat, nullptr, nullptr, 0,
-                  ws + o_enc);
+                  ws + o_enc, cells, r0 == 0);
   }
   res.sync();
 }

@@ -87,6 +87,43 @@ def test_codes(ivf, bits, pq_dim, length, n):
     assert (got <= d.min(2) * (1 + 1e-5) + 1e-9).all() and (codes == d.argmin(2)).mean() > 0.999
 
 
+# through tables of cells (at most four components, 7 and 8 bits, so many rows or more), against the comparison of all distances
+# (fewer rows at a time), bit for bit: normal and heavy-tailed residuals, equal codewords, a subspace whose codewords are
+# all equal or far from zero for their spread, components that do not count, rows far outside, infinities and NaN
+@pytest.mark.parametrize("length,n", [(1, 24576), (2, 24577), (3, 131073), (4, 393217)])
+@pytest.mark.parametrize("bits", [7, 8])
+@pytest.mark.parametrize("rotated", [False, True])
+def test_codes_by_cells(ivf, length, n, bits, rotated):
+    pq_dim, n_lists = 8 if bits < 8 else 7, 20
+    dim = pq_dim * length - (1 if rotated else 0)
+    rot_dim, book = pq_dim * length, 1 << bits
+    rng = np.random.default_rng(10 * length + bits)
+    books = rng.standard_normal((pq_dim, length, book)).astype(np.float32)
+    books[1] *= np.exp(rng.uniform(-4, 1, book)).astype(np.float32)          # heavy tails
+    books[2, :, book // 2:] = books[2, :, :book - book // 2]                 # every codeword twice
+    books[3] = 0.25                                                          # all equal
+    books[4] = 100.0 + 1e-4 * books[4]                                       # far from zero for their spread
+    books[5, 0] = -0.5                                                       # a component that is always the same
+    centers = rng.standard_normal((n_lists, dim)).astype(np.float32)
+    rot = np.eye(dim) if not rotated else np.linalg.qr(rng.standard_normal((rot_dim, rot_dim)))[0][:, :dim]
+    rot = rot.astype(np.float32)
+    to = lambda a: torch.from_numpy(np.ascontiguousarray(a)).cuda()  # noqa: E731
+    index = ivf.build_precomputed(ivf.IndexParams(n_lists=n_lists, pq_dim=pq_dim, pq_bits=bits), dim, to(books), to(centers),
+                                  to(centers @ rot.T), to(rot))
+    x = (centers[rng.integers(0, n_lists, n)] + rng.standard_normal((n, dim)) * np.exp(rng.uniform(-5, 1, (n, 1)))).astype(np.float32)
+    x[::7] = x[::7] * 30.0
+    x[5], x[6, 0], x[7, 0] = 1e30, np.inf, np.nan
+    if not rotated:
+        near = centers[3].reshape(pq_dim, length)                            # midway between codewords, and on them
+        x[100:100 + book] = (near + books.transpose(2, 0, 1)).reshape(book, dim)
+        x[1000:1000 + book] = (near + 0.5 * (books + np.roll(books, 1, 2)).transpose(2, 0, 1)).reshape(book, dim)
+    labels, codes = ivf.transform(index, to(x))
+    for r0 in range(0, n, 20000):
+        few_labels, few = ivf.transform(index, to(x[r0:r0 + 20000]))
+        assert bool((few_labels == labels[r0:r0 + 20000]).all())
+        assert bool((few == codes[r0:r0 + 20000]).all())
+
+
 # one and several K blocks: row tile resident, and streamed beside the lists
 @pytest.mark.parametrize("n,dim,n_lists", [(20000, 62, 1000), (17000, 300, 1100), (17000, 768, 1100)])
 def test_a_wait_that_runs_out_redoes_every_label(ivf, n, dim, n_lists):
