@@ -1392,7 +1392,7 @@ class nearest_labeler {
   {
     const uint32_t batch = batch_of(n_rows);
     return label_tc_usable(batch, n_lists)
-             ? round_up<size_t>(label_model_bytes(n_lists, dim), 256) + label_workspace_bytes(res, batch, n_lists, dim)
+             ? round_up<size_t>(label_model_bytes(n_lists, dim, true), 256) + label_workspace_bytes(res, batch, n_lists, dim)
              : size_t(batch) * 8;
   }
   // `dim`: index of the |c|^2 column of the centre rows (rows carry -0.5 there); n_rows: the most that run() is given
@@ -1407,7 +1407,7 @@ class nearest_labeler {
   void refresh()
   {
     if (!use_tc_) { return; }
-    prepare_label_model(res_.stream, centers_, n_lists_, dim_, dim_ext_, mem_);
+    prepare_label_model(res_.stream, centers_, n_lists_, dim_, dim_ext_, 0.5f, true, mem_);
     res_.launches += 3;
   }
   // labels[i] = nearest list of row i of x_ext [n_rows, dim_ext]
@@ -1418,7 +1418,7 @@ class nearest_labeler {
       const float* x    = x_ext + r0 * dim_ext_;
       if (use_tc_) {
         label_rows_tc(res_, centers_, mem_, n_lists_, dim_, dim_ext_, alpha_, x, nr, labels + r0,
-                      mem_ + round_up<size_t>(label_model_bytes(n_lists_, dim_), 256));
+                      mem_ + round_up<size_t>(label_model_bytes(n_lists_, dim_, true), 256));
       } else {
         assign_nearest(res_, centers_, n_lists_, dim_ext_, alpha_, x, nr, labels + r0, reinterpret_cast<unsigned long long*>(mem_));
       }

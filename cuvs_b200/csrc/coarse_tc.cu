@@ -1386,13 +1386,6 @@ void select_clusters_tc(raft::resources& res, const float* centers, const float*
                    n_lists, dim_ext, alpha, n_probes, C, cap, cmax, eps_rel, probes, scores_out, redo_list, words + 2,
                    words, ext_col, ext_scale, row_scale, down_thr, by_maxima ? 1 : 0);
   }
-  uint32_t cap_fb = 2;
-  while (cap_fb < n_probes) { cap_fb <<= 1; }
-  const size_t fb_smem = size_t(cap_fb) * 8 + size_t(dim_ext) * 4;
-  const size_t fs_smem = (size_t(256) * 33 + size_t(kFbGroup) * dim_ext) * 4;
-  ensure_dynamic_smem(reinterpret_cast<const void*>(coarse_fallback_scores_kernel), fs_smem);
-  launch_chained(coarse_fallback_scores_kernel, ceildiv<uint32_t>(n_lists, 256u), 256, fs_smem, stream, redo_list,
-                 words + 2, centers, fq, n_queries, n_lists, dim_ext, alpha, scratch, kFbSlots, words);
   // the error word and how many queries this batch redid exactly: written to pinned memory by the kernel, looked at
   // before a later batch and at the handle's next synchronisation
   uint32_t* host_words = nullptr;
@@ -1404,11 +1397,29 @@ void select_clusters_tc(raft::resources& res, const float* centers, const float*
     res.tc_redo_pending  = true;
     res.tc_redo_seq++;
   }
-  launch_chained(coarse_fallback_kernel, kFbSlots, 256, fb_smem, stream, redo_list, words + 2, centers, fq, n_queries,
-                 n_lists, dim_ext, alpha, n_probes, cap_fb, scratch, probes, scores_out, words, host_words,
-                 res.tc_redo_seq);
+  launch_probe_redo(res, redo_list, words, centers, fq, n_queries, n_lists, dim_ext, alpha, n_probes, scratch, probes, scores_out,
+                    host_words, res.tc_redo_seq);
+  res.launches += 3;
+}
+
+size_t probe_redo_bytes(uint32_t n_lists) { return size_t(kFbSlots) * n_lists * 4; }
+
+void launch_probe_redo(raft::resources& res, const uint32_t* redo_list, uint32_t* words, const float* centers, const float* fq,
+                       uint32_t n_queries, uint32_t n_lists, uint32_t dim_ext, float alpha, uint32_t n_probes, float* scratch,
+                       uint32_t* probes, float* scores_out, uint32_t* host_words, uint32_t host_seq)
+{
+  uint32_t cap_fb = 2;
+  while (cap_fb < n_probes) { cap_fb <<= 1; }
+  const size_t fb_smem = size_t(cap_fb) * 8 + size_t(dim_ext) * 4;
+  const size_t fs_smem = (size_t(256) * 33 + size_t(kFbGroup) * dim_ext) * 4;
+  ensure_dynamic_smem(reinterpret_cast<const void*>(coarse_fallback_scores_kernel), fs_smem);
+  if (fb_smem > 48 * 1024) { ensure_dynamic_smem(reinterpret_cast<const void*>(coarse_fallback_kernel), fb_smem); }
+  launch_chained(coarse_fallback_scores_kernel, ceildiv<uint32_t>(n_lists, 256u), 256, fs_smem, res.stream, redo_list,
+                 words + 2, centers, fq, n_queries, n_lists, dim_ext, alpha, scratch, kFbSlots, words);
+  launch_chained(coarse_fallback_kernel, kFbSlots, 256, fb_smem, res.stream, redo_list, words + 2, centers, fq, n_queries,
+                 n_lists, dim_ext, alpha, n_probes, cap_fb, scratch, probes, scores_out, words, host_words, host_seq);
   CUDA_TRY(cudaGetLastError());
-  res.launches += 5;
+  res.launches += 2;
 }
 
 // Reads back the error word and the number of queries redone exactly by the last call that used

@@ -1,5 +1,6 @@
 // Nearest list of many rows on the tensor cores, exact: labels[i] = argmin over lists l of (score, l) with the score's
-// defining fp32 chain (coarse.cu) -- what k-means steps, extend and transform need.
+// defining fp32 chain (coarse.cu) -- what k-means steps, extend and transform need.  At the end: the nearest lists (probes) of a
+// batch of queries, by the same products.
 //
 // Reference: kmeans_balanced::predict (cpp/src/cluster/detail/kmeans_balanced.cuh:100-160).
 //
@@ -9,7 +10,7 @@
 //      within (-0.5, 0.5); the epilogue subtracts the list's norm term |c|^2 / 2 - m.c + |m|^2 / 2 times a factor of the row,
 //      which gives F (score + a constant of the row).  The bounds of a row say how far that can be from the exact value: the
 //      measured norms of what rounding took from row and lists, accumulation, the defining chain's own rounding, the keys.
-//   2. label_tc_kernel: a persistent CTA takes a tile of 256 rows against all (or a share) of the lists, 256 at a time: two
+//   2. row_list_kernel: a persistent CTA takes a tile of 256 rows against all (or a share) of the lists, 256 at a time: two
 //      accumulators of 128 rows, so that a list tile is read once for both and the epilogue of one runs beside the products of
 //      the other.  Per row and unit of 8 lists the epilogue finds the largest value (its low bits replaced by the unit's
 //      number); across the tiles it keeps, per row and column quarter, the four largest: 1.3 comparisons per value.
@@ -17,7 +18,7 @@
 //      what is left in ever finer sums, the defining chain last.
 //   4. If the fourth unit kept is inside, a fifth might be: such rows (2.7% of 1 M rows x 16,384 lists of 96 dimensions) go
 //      through 2 and 3 once more with the lists in eight shares; only what that does not settle is redone exactly over all lists.
-// What bounds label_tc_kernel: the issue and execution of the MMAs (1,300 clocks per 128 x 256 x 96; the products alone take 880),
+// What bounds row_list_kernel: the issue and execution of the MMAs (1,300 clocks per 128 x 256 x 96; the products alone take 880),
 // then the comparisons (740).  1,000,003 rows x 16,384 lists x 96 dimensions, all of the labelling: 9.4 ms with two products
 // (row operand as two halfs), units of 64 lists whose largest two values were kept with their columns, and 2% of the rows
 // redone over all lists; 3.8 ms so.  (One product widens the bounds from 5.2e-5 to 6.5e-5: 2.6 instead of 2.2 lists within
@@ -84,8 +85,9 @@ __global__ void center_sum_kernel(const float* __restrict__ centers, uint32_t n_
   }
 }
 
-// |c|^2 / 2 - m.c + |m|^2 / 2 of a list, by one warp (any m gives valid results: it only has to be the same everywhere)
-__device__ __forceinline__ void list_norms(const float* c, const float* sum, float inv_n, uint32_t dim, float& cc, float& dd, double& norm)
+// weight |c|^2 - m.c + |m|^2 / 2 of a list, by one warp (any m gives valid results: it only has to be the same everywhere)
+__device__ __forceinline__ void list_norms(const float* c, const float* sum, float inv_n, uint32_t dim, float weight, float& cc, float& dd,
+                                           double& norm)
 {
   const uint32_t lane = threadIdx.x & 31u;
   double mc = 0.0, mm = 0.0;
@@ -104,18 +106,18 @@ __device__ __forceinline__ void list_norms(const float* c, const float* sum, flo
     cc += __shfl_xor_sync(kFullMask, cc, o);
     dd += __shfl_xor_sync(kFullMask, dd, o);
   }
-  norm = 0.5 * double(c[dim]) - mc + 0.5 * mm;
+  norm = double(weight) * double(c[dim]) - mc + 0.5 * mm;
 }
 
 __global__ void center_stats_kernel(const float* __restrict__ centers, uint32_t n_lists, uint32_t dim, uint32_t dim_ext,
-                                    const float* __restrict__ sum, uint32_t* __restrict__ words)
+                                    float weight, const float* __restrict__ sum, uint32_t* __restrict__ words)
 {
   const uint32_t l = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   if (l >= n_lists) { return; }
   const float* c = centers + size_t(l) * dim_ext;
   float cc, dd;
   double norm;
-  list_norms(c, sum, 1.0f / float(n_lists), dim, cc, dd, norm);
+  list_norms(c, sum, 1.0f / float(n_lists), dim, weight, cc, dd, norm);
   if ((threadIdx.x & 31u) == 0) {
     atomicMax(words, __float_as_uint(fmaxf(dd, 2.0f * fabsf(float(norm))) * 1.0001f));
     atomicMax(words + 1, __float_as_uint(fmaxf(cc, fabsf(c[dim])) * 1.0001f));
@@ -135,7 +137,7 @@ __device__ __forceinline__ float center_scale(const uint32_t* words, float& bn)
 
 // One warp per list (of whole tiles: there is nothing in those beyond the last one but their norm terms).
 __global__ void center_operand_kernel(const float* __restrict__ centers, uint32_t n_lists, uint32_t dim, uint32_t dim_ext,
-                                      uint32_t width, const float* __restrict__ sum, uint32_t* __restrict__ words,
+                                      uint32_t width, float weight, const float* __restrict__ sum, uint32_t* __restrict__ words,
                                       float* __restrict__ norms, __half* __restrict__ out, __half* __restrict__ by_unit)
 {
   const uint32_t l = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31u;
@@ -148,14 +150,14 @@ __global__ void center_operand_kernel(const float* __restrict__ centers, uint32_
   const float inv_n = 1.0f / float(n_lists);
   const float* c    = centers + size_t(l) * dim_ext;
   double norm;
-  list_norms(c, sum, inv_n, dim, cc, dd, norm);
+  list_norms(c, sum, inv_n, dim, weight, cc, dd, norm);
   __half* dst    = out + size_t(l) * width;
   float lost     = 0.0f;
   for (uint32_t k = lane; k < width; k += 32) {
     const float v  = k < dim ? (c[k] - sum[k] * inv_n) * inv : 0.0f;
     const __half h = __float2half_rn(v);
     dst[k]         = h;
-    by_unit[((size_t(l / kUnit) * (width / 8u) + k / 8u) * kUnit + l % kUnit) * 8u + (k & 7u)] = h;
+    if (by_unit != nullptr) { by_unit[((size_t(l / kUnit) * (width / 8u) + k / 8u) * kUnit + l % kUnit) * 8u + (k & 7u)] = h; }
     const float d  = v - __half2float(h);
     lost           = __fmaf_rn(d, d, lost);
   }
@@ -300,16 +302,24 @@ struct label_params {
   uint32_t tag_mask;     // low bits of a key: number of the unit among those of an item's column quarter
   const float* norms;    // of the lists, whole tiles
   const float* factor;   // of the rows
-  float4* keys;          // [splits, n_rows, 4] largest keys of a column quarter
+  float4* keys;          // kKeys: [splits, n_rows, 4] largest keys of a column quarter
+  float* maxima;         // kMaxima: [n_rows, max_stride] largest value of every `unit` (8, 32, 64 or 128) lists
+  uint32_t unit, max_stride;
+  const float* threshold;  // kEmit: of the rows
+  uint32_t* found;         // [n_rows, 2 splits, found_cap] lists whose value reaches it
+  uint32_t* n_found;       // [n_rows, 2 splits]
+  uint32_t found_cap;
   uint32_t* error;
   uint32_t spin_limit, skip_kb;  // tc_wait_limits
 };
+// What the epilogue makes of the values
+enum row_list_mode { kKeys, kMaxima, kEmit };
 
 // kKB: K blocks of 64 halfs; up to three of both halves of the row tile stay in shared memory beside a ring of kSlots list
 // tiles.  0: any number, row blocks stream beside the list blocks.
-template <uint32_t kKB>
+template <uint32_t kKB, row_list_mode kMode>
 __global__ void __launch_bounds__(kThreads, 1)
-label_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, const label_params p)
+row_list_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, const label_params p)
 {
   constexpr bool kResident   = kKB > 0;
   constexpr uint32_t kSlots  = kKB == 1 ? 4u : (kKB == 2 ? 2u : 1u);
@@ -521,11 +531,20 @@ label_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
       tiles_of(item, t0, t1);
       const uint32_t row = (item / p.splits) * kTileRows + h * kRows + quarter * 32u + lane;
       const uint64_t neg = dup2(row < n_rows ? -__ldg(p.factor + row) : 0.0f);
-      float key[2][kKeep];  // of two column quarters
+      [[maybe_unused]] float key[2][kKeep];  // kKeys: of two column quarters
+      if constexpr (kMode == kKeys) {
 #pragma unroll
-      for (uint32_t c = 0; c < 2; c++) {
+        for (uint32_t c = 0; c < 2; c++) {
 #pragma unroll
-        for (uint32_t i = 0; i < kKeep; i++) { key[c][i] = -3e38f; }
+          for (uint32_t i = 0; i < kKeep; i++) { key[c][i] = -3e38f; }
+        }
+      }
+      // kEmit: this thread's own places (nothing is taken for a row that is not there)
+      [[maybe_unused]] float threshold  = INFINITY;
+      [[maybe_unused]] uint32_t n_found = 0;
+      [[maybe_unused]] const size_t seg = size_t(row) * (2u * p.splits) + (item % p.splits) * 2u + side;
+      if constexpr (kMode == kEmit) {
+        if (row < n_rows) { threshold = __ldg(p.threshold + row); }
       }
       for (uint32_t t = t0; t < t1; t++, it++) {
         const uint32_t id   = (t - t0) * kUnitsPerTile;
@@ -539,10 +558,13 @@ label_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
         tc_fence_after();
         const uint32_t tm = tmem_base + ((quarter * 32u) << 16) + h * kLists + side * 128u;
         const uint32_t na = norm_base + slot * kNormBytes + side * 512u;
-        // four units of eight columns each
+        [[maybe_unused]] float* out = p.maxima;
+        if constexpr (kMode == kMaxima) { out += size_t(row) * p.max_stride + (t * kLists + side * 128u) / p.unit; }
+        [[maybe_unused]] float wide[4];
         auto chunk = [&](uint32_t (&x)[32], auto cc) {
           constexpr uint32_t c = decltype(cc)::value;
-          float m[4];
+          [[maybe_unused]] float m[4];
+          [[maybe_unused]] uint32_t hits = 0;
           static_for<4>([&](auto uc) {
             constexpr uint32_t u = decltype(uc)::value;
             float v[8];
@@ -554,22 +576,57 @@ label_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
               const uint64_t b = fma2(n23, neg, pack2(x[u * 8u + e + 2], x[u * 8u + e + 3]));
               v[e] = lo2(a); v[e + 1] = hi2(a); v[e + 2] = lo2(b); v[e + 3] = hi2(b);
             }
-            const float y = max3(max3(max3(v[0], v[1], v[2]), v[3], v[4]), v[5], v[6]);
-            m[u] = __uint_as_float((__float_as_uint(fmaxf(y, v[7])) & ~p.tag_mask) | (id + (c & 1u) * 4u + u));
-          });
-          // two units at a time into the four largest: the m-th largest of two ordered runs a and b is the maximum over
-          // i + j = m of min(a[i - 1], b[j - 1])
-          float (&k)[kKeep] = key[c >> 1];
+            if constexpr (kMode == kEmit) {
 #pragma unroll
-          for (uint32_t u = 0; u < 4; u += 2) {
-            const float hi = fmaxf(m[u], m[u + 1]), lo = fminf(m[u], m[u + 1]);
-            const float k3 = max3(k[3], fminf(k[2], hi), fminf(k[1], lo));
-            const float k2 = max3(k[2], fminf(k[1], hi), fminf(k[0], lo));
-            const float k1 = max3(k[1], fminf(k[0], hi), lo);
-            k[0]           = fmaxf(k[0], hi);
-            k[1]           = k1;
-            k[2]           = k2;
-            k[3]           = k3;
+              for (uint32_t e = 0; e < 8; e++) {
+                if (v[e] >= threshold) { hits |= 1u << (u * 8u + e); }
+              }
+            } else {
+              const float y = fmaxf(max3(max3(max3(v[0], v[1], v[2]), v[3], v[4]), v[5], v[6]), v[7]);
+              m[u] = kMode == kKeys ? __uint_as_float((__float_as_uint(y) & ~p.tag_mask) | (id + (c & 1u) * 4u + u)) : y;
+            }
+          });
+          if constexpr (kMode == kEmit) {
+            while (hits != 0u) {
+              if (n_found < p.found_cap) {
+                p.found[seg * p.found_cap + n_found] = t * kLists + side * 128u + c * 32u + uint32_t(__ffs(int(hits))) - 1u;
+              }
+              n_found++;
+              hits &= hits - 1u;
+            }
+          }
+          if constexpr (kMode == kMaxima) {
+            if (p.unit == 8u) {
+              if (row < n_rows) { *reinterpret_cast<float4*>(out + c * 4u) = make_float4(m[0], m[1], m[2], m[3]); }
+            } else {
+              wide[c] = fmaxf(max3(m[0], m[1], m[2]), m[3]);
+              if (c == 3u && row < n_rows) {
+                const float w0 = fmaxf(wide[0], wide[1]), w1 = fmaxf(wide[2], wide[3]);
+                if (p.unit == 32u) {
+                  *reinterpret_cast<float4*>(out) = make_float4(wide[0], wide[1], wide[2], wide[3]);
+                } else if (p.unit == 64u) {
+                  *reinterpret_cast<float2*>(out) = make_float2(w0, w1);
+                } else {
+                  *out = fmaxf(w0, w1);
+                }
+              }
+            }
+          }
+          if constexpr (kMode == kKeys) {
+            // two units at a time into the four largest: the m-th largest of two ordered runs a and b is the maximum over
+            // i + j = m of min(a[i - 1], b[j - 1])
+            float (&k)[kKeep] = key[c >> 1];
+#pragma unroll
+            for (uint32_t u = 0; u < 4; u += 2) {
+              const float hi = fmaxf(m[u], m[u + 1]), lo = fminf(m[u], m[u + 1]);
+              const float k3 = max3(k[3], fminf(k[2], hi), fminf(k[1], lo));
+              const float k2 = max3(k[2], fminf(k[1], hi), fminf(k[0], lo));
+              const float k1 = max3(k[1], fminf(k[0], hi), lo);
+              k[0]           = fmaxf(k[0], hi);
+              k[1]           = k1;
+              k[2]           = k2;
+              k[3]           = k3;
+            }
           }
         };
         using std::integral_constant;
@@ -591,11 +648,14 @@ label_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
         chunk(x1, integral_constant<uint32_t, 3>{});
       }
       if (ok && row < n_rows) {
+        if constexpr (kMode == kKeys) {
 #pragma unroll
-        for (uint32_t c = 0; c < 2; c++) {
-          p.keys[(size_t(item % p.splits) * p.n_rows + row) * 4u + side * 2u + c] =
-            make_float4(key[c][0], key[c][1], key[c][2], key[c][3]);
+          for (uint32_t c = 0; c < 2; c++) {
+            p.keys[(size_t(item % p.splits) * p.n_rows + row) * 4u + side * 2u + c] =
+              make_float4(key[c][0], key[c][1], key[c][2], key[c][3]);
+          }
         }
+        if constexpr (kMode == kEmit) { p.n_found[seg] = n_found; }
       }
     }
   }
@@ -874,26 +934,47 @@ bool label_tc_usable(uint32_t n_rows, uint32_t n_lists)
   return n_lists >= 256 && uint64_t(n_rows) * n_lists >= (1ull << 24);
 }
 
-size_t label_model_bytes(uint32_t n_lists, uint32_t dim) { return unit_operand_at(n_lists, dim, operand_width(dim)) + size_t(round_up(n_lists, kUnit)) * operand_width(dim) * 2; }
+size_t label_model_bytes(uint32_t n_lists, uint32_t dim, bool by_units)
+{
+  return unit_operand_at(n_lists, dim, operand_width(dim)) + (by_units ? size_t(round_up(n_lists, kUnit)) * operand_width(dim) * 2 : 0);
+}
 
-void prepare_label_model(cudaStream_t stream, const float* centers, uint32_t n_lists, uint32_t dim, uint32_t dim_ext, void* model)
+void prepare_label_model(cudaStream_t stream, const float* centers, uint32_t n_lists, uint32_t dim, uint32_t dim_ext, float weight,
+                         bool by_units, void* model)
 {
   auto* words = static_cast<uint32_t*>(model);
   auto* sum   = reinterpret_cast<float*>(static_cast<char*>(model) + kMeanAt);
   auto* norms = reinterpret_cast<float*>(static_cast<char*>(model) + norms_at(dim));
   auto* b     = reinterpret_cast<__half*>(static_cast<char*>(model) + operand_at(n_lists, dim));
-  auto* units = reinterpret_cast<__half*>(static_cast<char*>(model) + unit_operand_at(n_lists, dim, operand_width(dim)));
+  auto* units = by_units ? reinterpret_cast<__half*>(static_cast<char*>(model) + unit_operand_at(n_lists, dim, operand_width(dim))) : nullptr;
   CUDA_TRY(cudaMemsetAsync(model, 0, norms_at(dim), stream));
   const uint32_t shares = std::min<uint32_t>(64, ceildiv(n_lists, 64u));
   center_sum_kernel<<<dim3(ceildiv(dim, 32u), shares), dim3(32, 8), 0, stream>>>(centers, n_lists, dim, dim_ext, sum);
-  center_stats_kernel<<<ceildiv<uint32_t>(n_lists, 8u), 256, 0, stream>>>(centers, n_lists, dim, dim_ext, sum, words);
-  center_operand_kernel<<<round_up(n_lists, kLists) / 8u, 256, 0, stream>>>(centers, n_lists, dim, dim_ext, operand_width(dim), sum,
+  center_stats_kernel<<<ceildiv<uint32_t>(n_lists, 8u), 256, 0, stream>>>(centers, n_lists, dim, dim_ext, weight, sum, words);
+  center_operand_kernel<<<round_up(n_lists, kLists) / 8u, 256, 0, stream>>>(centers, n_lists, dim, dim_ext, operand_width(dim), weight, sum,
                                                                            words, norms, b, units);
   CUDA_TRY(cudaGetLastError());
 }
 
 namespace {
-// One pass of label_tc_kernel over up to `rows` rows: the lists are shared out (`splits`) where row tiles alone do not fill
+template <row_list_mode kMode>
+void launch_row_list(const label_params& p, const CUtensorMap& ma, const CUtensorMap& mb, uint32_t items, int sm_count, cudaStream_t stream)
+{
+  constexpr size_t smem = kRoom + kNormSlots * kNormBytes + 1024 + 256;
+  auto go = [&](auto kernel) {
+    ensure_dynamic_smem(reinterpret_cast<const void*>(kernel), smem);
+    launch_chained(kernel, std::min(uint32_t(sm_count), items), kThreads, smem, stream, ma, mb, p);
+    CUDA_TRY(cudaGetLastError());
+  };
+  switch (p.k_blocks) {
+    case 1: go(row_list_kernel<1, kMode>); break;
+    case 2: go(row_list_kernel<2, kMode>); break;
+    case 3: go(row_list_kernel<3, kMode>); break;
+    default: go(row_list_kernel<0, kMode>);
+  }
+}
+
+// One pass of row_list_kernel over up to `rows` rows: the lists are shared out (`splits`) where row tiles alone do not fill
 // the SMs four times, and so that an item has at most kSplitTiles list tiles.
 struct label_pass {
   uint32_t splits, tiles_per_split, tag_mask;
@@ -991,7 +1072,6 @@ void label_rows_tc(raft::resources& res, const float* centers, const void* model
   p.spin_limit = wl.spin_limit;
   p.skip_kb    = wl.skip_kb;
   const CUtensorMap mb = make_map_2d(CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, b, n_lists, width, kLists, kBlockK, CU_TENSOR_MAP_SWIZZLE_128B);
-  const size_t smem    = kRoom + kNormSlots * kNormBytes + 1024 + 256;
   finish_params f{};
   f.eps = eps;
   f.timeouts = res.pinned + 13;
@@ -1024,16 +1104,7 @@ void label_rows_tc(raft::resources& res, const float* centers, const void* model
     f.error = error;
     const CUtensorMap ma = make_map_2d(CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, operand, rows, width, kRows, kBlockK, CU_TENSOR_MAP_SWIZZLE_128B);
     const uint32_t items = ceildiv(rows, kTileRows) * s.splits;
-    auto go = [&](auto kernel) {
-      ensure_dynamic_smem(reinterpret_cast<const void*>(kernel), smem);
-      launch_chained(kernel, std::min(uint32_t(res.sm_count), items), kThreads, smem, stream, ma, mb, p);
-    };
-    switch (p.k_blocks) {
-      case 1: go(label_tc_kernel<1>); break;
-      case 2: go(label_tc_kernel<2>); break;
-      case 3: go(label_tc_kernel<3>); break;
-      default: go(label_tc_kernel<0>);
-    }
+    launch_row_list<kKeys>(p, ma, mb, items, res.sm_count, stream);
     launch_chained(label_finish_kernel, finish_blocks, 256, 0, stream, f);
     CUDA_TRY(cudaGetLastError());
   };
@@ -1052,6 +1123,379 @@ void label_rows_tc(raft::resources& res, const float* centers, const void* model
     res.launches += 3;
   }
   assign_nearest_listed(res, centers, n_lists, dim_ext, alpha, x_ext, n_rows, last, words + 3, labels, best);
+}
+
+// ------------------------------------------------------------------------------------------------
+// The nearest lists of a batch of queries (search's coarse stage), exact: probes ordered by (score, list), the score being
+// the defining fp32 chain.
+//
+// Two passes of row_list_kernel and no score matrix.  The first writes the largest value of every `unit` lists; the n_probes-th
+// largest of a query's maxima, T, is a value that n_probes lists reach, so a wanted list has a value of at least T - 2 eps.
+// The second emits the lists that do (some n_probes of them where lists are many).  Those are scored with the defining
+// chain and ranked.  Queries that have no bound, or more lists within reach than there is room for, are redone exactly
+// over all lists (coarse_tc.cu).
+//
+// Measured (us, coarse stage): 10,000 queries x 50,000 lists, 20 probes: 553 by candidate keys (coarse_tc.cu) -> 270; 4,000 x
+// 12,288, 128 probes: 585 by the exact product and row selection -> 290; 10,000 x 4,000, 64 probes: 436 -> 230.  What is left is the
+// exact scores (half), then the two passes.
+// ------------------------------------------------------------------------------------------------
+namespace {
+
+// A warp per query: a value that at least n_probes of its maxima reach, from twelve halvings of their range, less 2 eps.
+template <uint32_t kPer>
+__global__ void __launch_bounds__(256)
+probe_threshold_kernel(const float* __restrict__ maxima, uint32_t n_units, uint32_t stride, uint32_t n_rows, uint32_t n_probes,
+                       const float4* __restrict__ eps, float* __restrict__ threshold, uint32_t* __restrict__ redo,
+                       uint32_t* __restrict__ n_redo)
+{
+  chain_begin();
+  const uint32_t r = (blockIdx.x * 256u + threadIdx.x) >> 5, lane = threadIdx.x & 31u;
+  if (r >= n_rows) { return; }
+  const float4* src = reinterpret_cast<const float4*>(maxima + size_t(r) * stride);  // the stride is a multiple of four
+  float v[kPer];
+  float lo = INFINITY, hi = -INFINITY;
+#pragma unroll
+  for (uint32_t i = 0; i < kPer; i += 4) {
+    const uint32_t at = i * 8u + lane;
+    const float4 x    = at * 4u < n_units ? __ldg(src + at) : make_float4(-INFINITY, -INFINITY, -INFINITY, -INFINITY);
+    v[i] = x.x; v[i + 1] = x.y; v[i + 2] = x.z; v[i + 3] = x.w;
+#pragma unroll
+    for (uint32_t e = 0; e < 4; e++) {
+      // (nothing, or nothing but lists that are not there)
+      if (at * 4u + e >= n_units || v[i + e] < -1e20f) { v[i + e] = -INFINITY; }
+      hi = fmaxf(hi, v[i + e]);
+      lo = v[i + e] > -INFINITY ? fminf(lo, v[i + e]) : lo;
+    }
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    lo = fminf(lo, __shfl_xor_sync(kFullMask, lo, o));
+    hi = fmaxf(hi, __shfl_xor_sync(kFullMask, hi, o));
+  }
+  // (all of them reach the smallest, and there are at least n_probes)
+  for (int step = 0; step < 12; step++) {
+    const float mid = 0.5f * (lo + hi);
+    uint32_t n      = 0;
+#pragma unroll
+    for (uint32_t i = 0; i < kPer; i++) { n += v[i] >= mid ? 1u : 0u; }
+    n = __reduce_add_sync(kFullMask, n);
+    if (n >= n_probes) {
+      lo = mid;
+    } else {
+      hi = mid;
+    }
+  }
+  if (lane == 0) {
+    float t         = lo - 2.0f * __ldg(eps + r).x;
+    const bool fine = t > -INFINITY && t < INFINITY;  // (false for NaN)
+    if (!fine) {
+      redo[atomicAdd(n_redo, 1u)] = r;
+      t                           = INFINITY;
+    }
+    threshold[r] = t;
+  }
+}
+
+constexpr uint32_t kMaxSegments   = 64;
+constexpr uint32_t kChainCols     = 64;   // columns staged at a time
+
+// A warp per query: the lists found, 32 at a time through shared memory, one per lane with the defining chain (the next
+// columns are on their way while some are used); a list's rank is the number of lists before it.
+// What bounds it: the shared-memory pipe, two thirds busy (8,000 queries x 128 probes x 96 dimensions: 135 us).  Bulk copies of a
+// lane's own row, 256 bytes each, took as long or longer (768 dimensions: 300 against 250 us).
+constexpr uint32_t kProbeWarps = 4, kChainPitch = kChainCols + 4u;
+// (a cap that is a multiple of eight, fourteen bytes each: the next warp's rows start on 16)
+__host__ __device__ __forceinline__ uint32_t probe_warp_bytes(uint32_t cap)
+{
+  return (32u * kChainPitch + kChainCols) * 4u + cap * 14u;
+}
+__global__ void __launch_bounds__(kProbeWarps * 32)
+probe_finish_kernel(const uint32_t* __restrict__ found, const uint32_t* __restrict__ n_found, uint32_t segments, uint32_t found_cap,
+                    const float* __restrict__ fq, const float* __restrict__ centers, uint32_t dim_ext, float alpha,
+                    uint32_t n_queries, uint32_t n_probes, uint32_t cap, const float* __restrict__ threshold,
+                    const uint32_t* __restrict__ error, uint32_t* __restrict__ timeouts, uint32_t* __restrict__ probes,
+                    uint32_t* __restrict__ redo, uint32_t* __restrict__ n_redo)
+{
+  // per warp: [32][kChainPitch] columns, [kChainCols] of the query, [cap] scores (order-preserving), lists, places and ranks
+  extern __shared__ __align__(16) uint8_t s_probe[];
+  __shared__ uint32_t s_first[kProbeWarps][kMaxSegments];
+  const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, q = blockIdx.x * kProbeWarps + warp;
+  const uint32_t bytes = probe_warp_bytes(cap);
+  float* s_rows  = reinterpret_cast<float*>(s_probe + warp * bytes);
+  float* s_query = s_rows + 32u * kChainPitch;
+  auto* s_score  = reinterpret_cast<uint32_t*>(s_query + kChainCols);
+  uint32_t *s_list = s_score + cap, *s_place = s_list + cap;
+  auto* s_rank   = reinterpret_cast<uint16_t*>(s_place + cap);
+  chain_begin();
+  const bool there      = q < n_queries;
+  const uint32_t failed = __ldg(error);
+  const float limit     = there ? __ldg(threshold + q) : INFINITY;
+  // (at most 64 segments, two per lane)
+  uint32_t n_seg[2], sum = 0;
+  bool fits = true;
+#pragma unroll
+  for (uint32_t i = 0; i < 2; i++) {
+    n_seg[i] = there && 2u * lane + i < segments ? __ldg(n_found + size_t(q) * segments + 2u * lane + i) : 0u;
+    fits     = fits && n_seg[i] <= found_cap;
+    n_seg[i] = min(n_seg[i], cap + 1u);
+    sum += n_seg[i];
+  }
+  if (failed != 0u) {  // every query is redone
+    if (q == 0 && lane == 0) { count_timeout(timeouts); }
+    return;
+  }
+  if (limit == INFINITY) { return; }  // (listed already)
+  uint32_t inc = sum;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const uint32_t x = __shfl_up_sync(kFullMask, inc, o);
+    if (lane >= uint32_t(o)) { inc += x; }
+  }
+  const uint32_t n = __shfl_sync(kFullMask, inc, 31);
+  if (!__all_sync(kFullMask, fits) || n > cap || n < n_probes) {
+    if (lane == 0) { redo[atomicAdd(n_redo, 1u)] = q; }
+    return;
+  }
+  s_first[warp][2u * lane]      = inc - sum;
+  s_first[warp][2u * lane + 1u] = inc - n_seg[1];
+  __syncwarp();
+  for (uint32_t i = lane; i < n; i += 32u) {
+    // the last segment that starts at or before i (an empty one starts where the next does)
+    uint32_t seg = 0;
+#pragma unroll
+    for (uint32_t step = kMaxSegments / 2u; step > 0; step >>= 1) { seg += s_first[warp][seg + step] <= i ? step : 0u; }
+    s_list[i] = __ldg(found + (size_t(q) * segments + seg) * found_cap + (i - s_first[warp][seg]));
+  }
+  __syncwarp();
+  // sixteen lanes per row; step: (32 lists, kChainCols columns)
+  float4 v[16], x;
+  auto load = [&](uint32_t c0, uint32_t k0) {
+    const uint32_t k4 = k0 / 4u + (lane & 15u);
+    const bool in     = k4 < dim_ext / 4u;
+#pragma unroll
+    for (uint32_t i = 0; i < 16; i++) {
+      const uint32_t c = c0 + 2u * i + (lane >> 4);
+      if (in && c < n) { v[i] = __ldg(reinterpret_cast<const float4*>(centers + size_t(s_list[c]) * dim_ext) + k4); }
+    }
+    if (in && lane < 16u) { x = __ldg(reinterpret_cast<const float4*>(fq + size_t(q) * dim_ext) + k4); }
+  };
+  load(0, 0);
+  float acc = 0.0f;
+  for (uint32_t c0 = 0, k0 = 0; c0 < n;) {
+#pragma unroll
+    for (uint32_t i = 0; i < 16; i++) {
+      *reinterpret_cast<float4*>(s_rows + (2u * i + (lane >> 4)) * kChainPitch + (lane & 15u) * 4u) = v[i];
+    }
+    if (lane < 16u) { *reinterpret_cast<float4*>(s_query + lane * 4u) = x; }
+    __syncwarp();
+    const uint32_t kn = min(kChainCols, dim_ext - k0) / 4u;  // dim_ext is a multiple of 8
+    uint32_t next_c = c0, next_k = k0 + kChainCols;
+    if (next_k >= dim_ext) {
+      next_k = 0;
+      next_c += 32u;
+    }
+    if (next_c < n) { load(next_c, next_k); }
+    const float* mine = s_rows + lane * kChainPitch;
+#pragma unroll 4
+    for (uint32_t k = 0; k < kn; k++) {
+      const float4 c = *reinterpret_cast<const float4*>(mine + k * 4u);
+      const float4 y = *reinterpret_cast<const float4*>(s_query + k * 4u);
+      acc = __fmaf_rn(c.x, y.x, acc);
+      acc = __fmaf_rn(c.y, y.y, acc);
+      acc = __fmaf_rn(c.z, y.z, acc);
+      acc = __fmaf_rn(c.w, y.w, acc);
+    }
+    if (next_k == 0) {
+      if (c0 + lane < n) { s_score[c0 + lane] = float_to_ordered(__fmul_rn(alpha, acc)); }
+      acc = 0.0f;
+    }
+    c0 = next_c;
+    k0 = next_k;
+    __syncwarp();
+  }
+  // the rank by score, four lists of a lane at a time
+  if (lane < 3u && n + lane < cap) { s_score[n + lane] = 0xFFFFFFFFu; }  // (read below in fours)
+  __syncwarp();
+  for (uint32_t c0 = 0; c0 < n; c0 += 128u) {
+    uint32_t mine[4], rank[4] = {0u, 0u, 0u, 0u};
+#pragma unroll
+    for (uint32_t i = 0; i < 4; i++) { mine[i] = c0 + i * 32u + lane < n ? s_score[c0 + i * 32u + lane] : 0u; }
+    for (uint32_t o = 0; o < n; o += 4) {
+      const uint4 y = *reinterpret_cast<const uint4*>(s_score + o);
+#pragma unroll
+      for (uint32_t i = 0; i < 4; i++) {
+        rank[i] += (y.x < mine[i] ? 1u : 0u) + (y.y < mine[i] ? 1u : 0u);
+        rank[i] += (y.z < mine[i] ? 1u : 0u) + (y.w < mine[i] ? 1u : 0u);
+      }
+    }
+#pragma unroll
+    for (uint32_t i = 0; i < 4; i++) {
+      const uint32_t c = c0 + i * 32u + lane;
+      if (c < n) {
+        s_place[rank[i]] = c;
+        s_rank[c]        = uint16_t(rank[i]);
+      }
+    }
+  }
+  __syncwarp();
+  // lists of equal score met at one place: then the order is by (score, list)
+  bool tied = false;
+  for (uint32_t c = lane; c < n; c += 32u) { tied = tied || s_place[s_rank[c]] != c; }
+  if (__any_sync(kFullMask, tied)) {
+    for (uint32_t c = lane; c < n; c += 32u) {
+      const uint32_t score = s_score[c], list = s_list[c];
+      uint32_t rank        = 0;
+      for (uint32_t o = 0; o < n; o++) { rank += s_score[o] < score || (s_score[o] == score && s_list[o] < list) ? 1u : 0u; }
+      if (rank < n_probes) { probes[size_t(q) * n_probes + rank] = list; }
+    }
+    return;
+  }
+  for (uint32_t r = lane; r < n_probes; r += 32u) { probes[size_t(q) * n_probes + r] = s_list[s_place[r]]; }
+}
+// Lists within reach that a query can have.
+uint32_t probe_cap(uint32_t n_probes) { return round_up(2u * n_probes + 48u, 8u); }
+
+// Lists per unit: as many as leave six times as many units as wanted lists, so that the maxima select sharply (8% more lists
+// reach the threshold than are wanted); no fewer than a warp can hold the maxima of.
+uint32_t probe_unit(uint32_t n_lists, uint32_t n_probes)
+{
+  for (uint32_t unit : {128u, 64u, 32u}) {
+    if (n_lists / unit >= 6u * n_probes && n_lists <= unit * 2048u) { return unit; }
+  }
+  return n_lists <= 16384u ? 8u : (n_lists <= 65536u ? 32u : 64u);
+}
+
+struct probe_layout {
+  uint32_t unit, n_units, max_stride, splits, tiles_per_split, found_cap;
+  size_t o_a, o_factor, o_eps, o_maxima, o_threshold, o_found, o_n_found, o_redo, o_words, o_scratch, total;
+  probe_layout(uint32_t n_queries, uint32_t n_lists, uint32_t n_probes, uint32_t dim, int sm_count)
+  {
+    const uint32_t row_tiles = ceildiv(n_queries, kTileRows), n_tiles = ceildiv(n_lists, kLists);
+    unit       = probe_unit(n_lists, n_probes);
+    n_units    = n_tiles * (kLists / unit);
+    max_stride = round_up(n_units, 4u);
+    // the split of the lists whose last wave is fullest: clocks of a list tile (products, or the epilogue) and of an item's
+    // start (its row tile)
+    const uint64_t tile = std::max(2u * 140u * (operand_width(dim) / 16u), 2600u), start = 4000;
+    uint64_t best       = ~0ull;
+    splits = tiles_per_split = 1;
+    for (uint32_t s = 1; s <= std::min(n_tiles, kMaxSegments / 2u); s++) {
+      const uint32_t per = ceildiv(n_tiles, s), n = ceildiv(n_tiles, per);
+      const uint64_t cost = ceildiv<uint64_t>(uint64_t(row_tiles) * n, uint64_t(sm_count)) * (per * tile + start);
+      if (cost < best) {
+        best            = cost;
+        splits          = n;
+        tiles_per_split = per;
+      }
+    }
+    found_cap = round_up(std::min(n_probes + n_probes / 4u + 32u, tiles_per_split * 128u), 4u);
+    ws_layout lay;
+    o_a         = lay.add(size_t(n_queries) * operand_width(dim) * 2);
+    o_factor    = lay.add(size_t(n_queries) * 4);
+    o_eps       = lay.add(size_t(n_queries) * 16);
+    o_maxima    = lay.add(size_t(n_queries) * max_stride * 4);
+    o_threshold = lay.add(size_t(n_queries) * 4);
+    o_found     = lay.add(size_t(n_queries) * splits * 2 * found_cap * 4);
+    o_n_found   = lay.add(size_t(n_queries) * splits * 2 * 4);
+    o_redo      = lay.add(size_t(n_queries) * 4);
+    o_words     = lay.add(256);
+    o_scratch   = lay.add(probe_redo_bytes(n_lists));
+    total       = lay.total();
+  }
+};
+
+}  // namespace
+
+// From 2 M (query, list) pairs on.  A whole call with 20 probes, by coarse_tc.cu or the exact product / so (us): 500 x 2,048 95 / 95,
+// 1,000 x 2,048 117 / 117, 2,000 x 1,024 145 / 145, 500 x 4,096 112 / 112, 1,000 x 4,096 146 / 122, 200 x 10,000 110 / 105, 500 x
+// 10,000 121 / 107, 4,000 x 10,000 378 / 214.
+bool probes_tc_usable(uint32_t n_queries, uint32_t n_lists, uint32_t n_probes, uint32_t dim)
+{
+  const uint32_t unit = probe_unit(n_lists, n_probes);
+  return n_lists >= 256 && n_lists <= 131072 && n_probes <= 256 && n_lists / unit >= 2 * n_probes && dim <= 4096 &&
+         uint64_t(n_queries) * n_lists >= (1ull << 21);
+}
+
+size_t probes_workspace_bytes(const raft::resources& res, uint32_t n_queries, uint32_t n_lists, uint32_t n_probes, uint32_t dim)
+{
+  return probe_layout(n_queries, n_lists, n_probes, dim, res.sm_count).total;
+}
+
+void select_probes_tc(raft::resources& res, const float* centers, const void* model, uint32_t n_lists, uint32_t dim, uint32_t dim_ext,
+                      float alpha, const float* fq, uint32_t n_queries, uint32_t max_queries, uint32_t n_probes, uint32_t* probes,
+                      void* workspace)
+{
+  const probe_layout y(max_queries, n_lists, n_probes, dim, res.sm_count);
+  const uint32_t width = operand_width(dim);
+  char* ws             = static_cast<char*>(workspace);
+  auto* a              = reinterpret_cast<__half*>(ws + y.o_a);
+  auto* factor         = reinterpret_cast<float*>(ws + y.o_factor);
+  auto* eps            = reinterpret_cast<float4*>(ws + y.o_eps);
+  auto* maxima         = reinterpret_cast<float*>(ws + y.o_maxima);
+  auto* threshold      = reinterpret_cast<float*>(ws + y.o_threshold);
+  auto* found          = reinterpret_cast<uint32_t*>(ws + y.o_found);
+  auto* n_found        = reinterpret_cast<uint32_t*>(ws + y.o_n_found);
+  auto* redo           = reinterpret_cast<uint32_t*>(ws + y.o_redo);
+  auto* words          = reinterpret_cast<uint32_t*>(ws + y.o_words);  // error, queries redone, queries to redo
+  const auto* sum      = reinterpret_cast<const float*>(static_cast<const char*>(model) + kMeanAt);
+  const auto* norms    = reinterpret_cast<const float*>(static_cast<const char*>(model) + norms_at(dim));
+  const auto* b        = reinterpret_cast<const __half*>(static_cast<const char*>(model) + operand_at(n_lists, dim));
+  cudaStream_t stream  = res.stream;
+  auto operand = [&](auto kernel) {
+    launch_chained(kernel, ceildiv<uint32_t>(n_queries, 32u), 256, 0, stream, fq, n_queries, n_lists, dim, dim_ext, width, sum,
+                   static_cast<const uint32_t*>(model), 0.0f, a, factor, eps, reinterpret_cast<uint4*>(words));
+  };
+  if (width <= 128) {
+    operand(row_operand_kernel<true>);
+  } else {
+    operand(row_operand_kernel<false>);
+  }
+  label_params p{};
+  p.n_rows = n_queries;
+  p.k_steps = width / 16;
+  p.k_blocks = ceildiv(width, kBlockK);
+  p.n_tiles = ceildiv(n_lists, kLists);
+  p.tiles_per_split = y.tiles_per_split;
+  p.splits = y.splits;
+  p.norms = norms;
+  p.factor = factor;
+  p.maxima = maxima;
+  p.unit = y.unit;
+  p.max_stride = y.max_stride;
+  p.threshold = threshold;
+  p.found = found;
+  p.n_found = n_found;
+  p.found_cap = y.found_cap;
+  p.error = words;
+  const wait_limits wl = tc_wait_limits();
+  p.spin_limit = wl.spin_limit;
+  p.skip_kb = wl.skip_kb;
+  const CUtensorMap ma = make_map_2d(CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, a, n_queries, width, kRows, kBlockK, CU_TENSOR_MAP_SWIZZLE_128B);
+  const CUtensorMap mb = make_map_2d(CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, b, n_lists, width, kLists, kBlockK, CU_TENSOR_MAP_SWIZZLE_128B);
+  const uint32_t items = ceildiv(n_queries, kTileRows) * y.splits;
+  launch_row_list<kMaxima>(p, ma, mb, items, res.sm_count, stream);
+  auto threshold_of = [&](auto kernel) {
+    launch_chained(kernel, ceildiv(n_queries, 8u), 256, 0, stream, maxima, y.n_units, y.max_stride, n_queries, n_probes, eps, threshold, redo, words + 2);
+  };
+  if (y.n_units <= 256) {
+    threshold_of(probe_threshold_kernel<8>);
+  } else if (y.n_units <= 512) {
+    threshold_of(probe_threshold_kernel<16>);
+  } else if (y.n_units <= 1024) {
+    threshold_of(probe_threshold_kernel<32>);
+  } else {
+    threshold_of(probe_threshold_kernel<64>);
+  }
+  launch_row_list<kEmit>(p, ma, mb, items, res.sm_count, stream);
+  const size_t finish_smem = kProbeWarps * probe_warp_bytes(probe_cap(n_probes));
+  ensure_dynamic_smem(reinterpret_cast<const void*>(probe_finish_kernel), finish_smem);
+  launch_chained(probe_finish_kernel, ceildiv(n_queries, kProbeWarps), kProbeWarps * 32, finish_smem, stream, found, n_found,
+                 2u * y.splits, y.found_cap, fq, centers, dim_ext, alpha, n_queries, n_probes, probe_cap(n_probes), threshold, words,
+                 res.pinned + 13, probes, redo, words + 2);
+  CUDA_TRY(cudaGetLastError());
+  launch_probe_redo(res, redo, words, centers, fq, n_queries, n_lists, dim_ext, alpha, n_probes, reinterpret_cast<float*>(ws + y.o_scratch),
+                    probes, nullptr, nullptr, 0);
+  res.launches += 5;
 }
 
 }  // namespace cuvs::neighbors::ivf_pq

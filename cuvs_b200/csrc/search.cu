@@ -949,11 +949,15 @@ void search_any(raft::resources& res, const search_params& params, const index<i
   const size_t o_all     = lay.add(store_all ? size_t(batch) * max_samples * 4 : 0);
   // half-precision scores tie in large groups, which the tensor-core path's guard (made for fp32
   // scores) does not settle: the fp16 coarse search runs on the exact SIMT path
+  // large batches: no score matrix; else the other tensor-core path or the exact product
+  const bool use_probes_tc =
+    !coarse_h && !coarse_i8 && coarse_mode() == 0 && probes_tc_usable(batch, n_lists, n_probes, idx.dim());
   const bool use_tc = !coarse_h && coarse_mode() != 1 && coarse_tc_usable(n_lists, n_probes, cdim_ext);
   const size_t coarse_ws =
-    given_probes ? 0
-                 : (use_tc ? coarse_tc_workspace_bytes(batch, n_lists, cdim_ext)
-                           : coarse_workspace_bytes(batch, n_lists, n_probes));
+    given_probes    ? 0
+    : use_probes_tc ? probes_workspace_bytes(res, batch, n_lists, n_probes, idx.dim())
+    : use_tc        ? coarse_tc_workspace_bytes(batch, n_lists, cdim_ext)
+                    : coarse_workspace_bytes(batch, n_lists, n_probes);
   const size_t o_coarse  = lay.add(coarse_ws);
   // tables in global memory: one per CTA of the (smaller) grid of that variant
   const uint32_t glut_grid = uint32_t(std::min<size_t>(n_pairs_max, size_t(res.sm_count) * 4));
@@ -1007,6 +1011,9 @@ void search_any(raft::resources& res, const search_params& params, const index<i
         select_clusters(res, op8.centers, n_lists, cdim_ext, is_l2 ? -2.0f : -1.0f, d_fq, nq, n_probes,
                         d_probes, nullptr, d_coarse, coarse_ws);
       }
+    } else if (use_probes_tc) {
+      select_probes_tc(res, idx.centers(), idx.list_model(), n_lists, idx.dim(), idx.dim_ext(), is_l2 ? -2.0f : -1.0f, d_fq, nq,
+                       batch, n_probes, d_probes, d_coarse);
     } else if (use_tc) {
       select_clusters_tc(res, idx.centers(), idx.centers_hi(), idx.centers_lo(), idx.centers_max_norm(),
                          n_lists, idx.dim_ext(), is_l2 ? -2.0f : -1.0f, d_fq, nq, n_probes, d_probes,
@@ -1315,11 +1322,14 @@ void select_probes_any(raft::resources& res, const index<int64_t>& idx, const vo
   if (coarse_h) { oph = idx.half_coarse_operands(res.stream); }
   const bool use_tc = !coarse_h && coarse_mode() != 1 && coarse_tc_usable(n_lists, n_probes, cdim_ext);
   const uint32_t batch = std::min<uint32_t>(n_queries, 16384);
+  const bool use_probes_tc =
+    !coarse_h && !coarse_i8 && coarse_mode() == 0 && probes_tc_usable(batch, n_lists, n_probes, idx.dim());
   ws_layout lay;
   const size_t o_fq = lay.add(size_t(batch) * cdim_ext * 4);
   const size_t o_rq = lay.add(size_t(batch) * idx.rot_dim() * 4);
-  const size_t cws  = use_tc ? coarse_tc_workspace_bytes(batch, n_lists, cdim_ext)
-                             : coarse_workspace_bytes(batch, n_lists, n_probes);
+  const size_t cws  = use_probes_tc ? probes_workspace_bytes(res, batch, n_lists, n_probes, idx.dim())
+                      : use_tc      ? coarse_tc_workspace_bytes(batch, n_lists, cdim_ext)
+                                    : coarse_workspace_bytes(batch, n_lists, n_probes);
   const size_t o_c  = lay.add(cws);
   res.ws.reserve(lay.total());
   char* ws   = res.ws.base();
@@ -1343,6 +1353,9 @@ void select_probes_any(raft::resources& res, const index<int64_t>& idx, const vo
         select_clusters(res, op8.centers, n_lists, cdim_ext, alpha, d_fq, nq, n_probes, out, nullptr,
                         ws + o_c, cws);
       }
+    } else if (use_probes_tc) {
+      select_probes_tc(res, idx.centers(), idx.list_model(), n_lists, idx.dim(), idx.dim_ext(), alpha, d_fq, nq, batch, n_probes, out,
+                       ws + o_c);
     } else if (use_tc) {
       select_clusters_tc(res, idx.centers(), idx.centers_hi(), idx.centers_lo(), idx.centers_max_norm(),
                          n_lists, idx.dim_ext(), alpha, d_fq, nq, n_probes, out, nullptr, ws + o_c, cws, false,

@@ -111,11 +111,29 @@ void exact_rows_product(raft::resources& res, const float* b, uint32_t n_cols, c
 // The same labels on the tensor cores (label_tc.cu).  `model`: label_model_bytes of device memory that
 // prepare_label_model fills from the centres; `workspace`: label_workspace_bytes.  Nothing synchronises.
 bool label_tc_usable(uint32_t n_rows, uint32_t n_lists);
-size_t label_model_bytes(uint32_t n_lists, uint32_t dim);
-void prepare_label_model(cudaStream_t stream, const float* centers, uint32_t n_lists, uint32_t dim, uint32_t dim_ext,
-                         void* model);
+// `weight`: the factor of the rows' column `dim` in the score, negated (0.5 for L2 distances, 0 where the column does not count);
+// by_units: with what label_rows_tc needs (select_probes_tc does not).
+size_t label_model_bytes(uint32_t n_lists, uint32_t dim, bool by_units);
+void prepare_label_model(cudaStream_t stream, const float* centers, uint32_t n_lists, uint32_t dim, uint32_t dim_ext, float weight,
+                         bool by_units, void* model);
 size_t label_workspace_bytes(const raft::resources& res, uint32_t n_rows, uint32_t n_lists, uint32_t dim);
 void label_rows_tc(raft::resources& res, const float* centers, const void* model, uint32_t n_lists, uint32_t dim,
                    uint32_t dim_ext, float alpha, const float* x_ext, uint32_t n_rows, uint32_t* labels, void* workspace);
+
+// The probes of a batch on the tensor cores without a score matrix (label_tc.cu): same contract and bit-identical probes as
+// select_clusters.  `model`: of the same centres, by prepare_label_model; `workspace`: probes_workspace_bytes for max_queries.
+bool probes_tc_usable(uint32_t n_queries, uint32_t n_lists, uint32_t n_probes, uint32_t dim);
+size_t probes_workspace_bytes(const raft::resources& res, uint32_t n_queries, uint32_t n_lists, uint32_t n_probes, uint32_t dim);
+void select_probes_tc(raft::resources& res, const float* centers, const void* model, uint32_t n_lists, uint32_t dim, uint32_t dim_ext,
+                      float alpha, const float* fq, uint32_t n_queries, uint32_t max_queries, uint32_t n_probes, uint32_t* probes,
+                      void* workspace);
+
+// Queries redone exactly over all lists: redo_list[0 .. words[2]), or all of them where words[0], the error word, is set.  `words[1]`
+// receives their number; host_words (optional, pinned): {words[0], number, words[2], words[3], host_seq}.  `scratch`:
+// probe_redo_bytes.
+size_t probe_redo_bytes(uint32_t n_lists);
+void launch_probe_redo(raft::resources& res, const uint32_t* redo_list, uint32_t* words, const float* centers, const float* fq,
+                       uint32_t n_queries, uint32_t n_lists, uint32_t dim_ext, float alpha, uint32_t n_probes, float* scratch,
+                       uint32_t* probes, float* scores_out, uint32_t* host_words, uint32_t host_seq);
 
 }  // namespace cuvs::neighbors::ivf_pq

@@ -302,6 +302,9 @@ class index<int64_t> {
     float scale = 1.0f, rmax = 0.0f, comp_max = 0.0f;
   };
   const filter_operand& filter_model() const { return filter_; }
+  // The centres in half precision with their norm terms, for the coarse search of large batches; made with the other derived
+  // state.
+  const void* list_model() const { return list_model_.data(); }
 
   // (Re)create the arenas for the given list sizes; contents are zero codes / -1 ids.
   void allocate_lists(const std::vector<uint32_t>& sizes, cudaStream_t stream);
@@ -313,6 +316,7 @@ class index<int64_t> {
   // model arrays are public to the builder / loader
   dev_array<float> pq_centers_, centers_, centers_rot_, rotation_;
   dev_array<float> centers_hi_, centers_lo_;
+  dev_array<uint8_t> list_model_;
   float centers_max_norm_ = 0.0f;
   float centers_ext_scale_ = 1.0f;
   mutable dev_array<float> centers_i8f_, rotation_i8f_;

@@ -1,0 +1,105 @@
+"""Probe selection of large batches (two passes over the lists' values, no score matrix) against the exact product with
+row selection: the same probes in the same order, bit for bit."""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+from conftest import make_mixture
+
+pytestmark = pytest.mark.gpu
+torch = pytest.importorskip("torch")
+
+
+@pytest.fixture(scope="module")
+def mods():
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    from cuvs_b200 import _lib, ivf_pq, mg
+    return ivf_pq, mg, _lib
+
+
+def index_of(ivf, centers, metric):
+    n_lists, dim = centers.shape
+    rng = np.random.default_rng(1)
+    books = rng.standard_normal((2, dim // 2, 16)).astype(np.float32)
+    to = lambda a: torch.from_numpy(np.ascontiguousarray(a, dtype=np.float32)).cuda()  # noqa: E731
+    return ivf.build_precomputed(ivf.IndexParams(n_lists=n_lists, pq_dim=2, pq_bits=4, metric=metric), dim, to(books), to(centers),
+                                 to(centers), to(np.eye(dim)))
+
+
+def both(mods, index, q, n_probes):
+    """(probes as search selects them, probes of the exact product)"""
+    ivf, mg, L = mods
+    lib, got = L.load(), []
+    for mode in (0, 1):
+        try:
+            lib.cuvsB200SetCoarseMode(mode)
+            got.append(mg.select_probes(index, q, n_probes).to(torch.int64))
+        finally:
+            lib.cuvsB200SetCoarseMode(0)
+    return got
+
+
+# edges of the 256-query and 256-list tiles; 8, 32, 64 and 128 lists per maximum; one, two, three and more K blocks
+@pytest.mark.parametrize("metric", ["sqeuclidean", "inner_product", "cosine"])
+@pytest.mark.parametrize("n_lists,n_q,dim,n_probes", [(257, 8200, 14, 1), (513, 4300, 62, 32), (1024, 2305, 130, 20), (4001, 700, 96, 128),
+                                                      (4096, 513, 256, 256), (9000, 257, 128, 20), (20000, 255, 66, 200),
+                                                      (40000, 100, 32, 50)])
+def test_probes(mods, n_lists, n_q, dim, n_probes, metric):
+    centers = make_mixture(n_lists, dim, 60, 0.4, 2)
+    q = make_mixture(n_q, dim, 60, 0.4, 3)
+    if metric == "cosine":
+        centers /= np.linalg.norm(centers, axis=1, keepdims=True)
+    index = index_of(mods[0], centers, metric)
+    fast, exact = both(mods, index, torch.from_numpy(q).cuda(), n_probes)
+    assert bool((fast == exact).all())
+
+
+def test_odd_queries_and_equal_lists(mods):
+    """Queries without a bound (NaN, infinities, values at the ends of fp32, zeros) and lists that are equal or nearly so in numbers
+    beyond what a query has room for."""
+    rng = np.random.default_rng(5)
+    centers = make_mixture(4096, 48, 60, 0.4, 2)
+    centers[100:130] = centers[7]                                  # ties: lowest list first
+    centers[1000:1600] = centers[8] + 1e-6 * rng.standard_normal((600, 48))
+    q = make_mixture(1500, 48, 60, 0.4, 3)
+    q[0], q[1, 3], q[2, 4], q[3] = 0.0, np.nan, np.inf, 1e30
+    q[4] *= 1e-30
+    q[5] *= 1e18
+    q[10:40] = centers[7]
+    q[40:80] = centers[8]
+    for metric in ("sqeuclidean", "inner_product"):
+        index = index_of(mods[0], centers, metric)
+        fast, exact = both(mods, index, torch.from_numpy(q.astype(np.float32)).cuda(), 40)
+        fine = torch.ones(len(q), dtype=torch.bool, device="cuda")
+        fine[1] = fine[2] = False                                  # (NaN scores have no order)
+        assert bool((fast == exact).all(1)[fine].all())
+
+
+# one product pass times out; every query is redone exactly and the handle counts the batch
+@pytest.mark.parametrize("dim", [40, 300])
+def test_a_wait_that_runs_out_redoes_every_query(mods, dim):
+    ivf, mg, L = mods
+    from cuvs_b200.common import Resources
+    centers = make_mixture(2100, dim, 60, 0.4, 2)
+    q = torch.from_numpy(make_mixture(1100, dim, 60, 0.4, 3)).cuda()
+    index = index_of(ivf, centers, "sqeuclidean")
+    lib, res = L.load(), Resources()
+
+    def run():
+        out = mg.select_probes(index, q, 20, resources=res).to(torch.int64)
+        m = C.c_uint64(0)
+        L.check(lib.cuvsStreamSync(res.handle))
+        L.check(lib.cuvsB200CoarseTimeouts(res.handle, C.byref(m)))
+        return out, m.value
+
+    healthy, m0 = run()
+    try:
+        L.check(lib.cuvsB200SetCoarseWaitTest(1000, 1))
+        timed_out, m1 = run()
+    finally:
+        L.check(lib.cuvsB200SetCoarseWaitTest(0, 0))
+    again, m2 = run()
+    assert m0 == 0 and m1 == 1 and m2 == m1
+    assert bool((healthy == timed_out).all()) and bool((healthy == again).all())
