@@ -106,7 +106,7 @@ __device__ __forceinline__ uint32_t swz(uint32_t r, uint32_t c) { return r * 128
 // kBits 8 or 4 (kWords): the codes of half a K block are extracted from whole words with constant shifts; other widths,
 // and subspaces of more than eight components, code by code.  kLP: halfs per subspace in the K layout (1, 2, 4 or 8;
 // without kWords 8 stands for every multiple of 8).
-template <int kBits, int kLP, bool kWords>
+template <int kBits, int kLP, bool kWords, bool kCodes>
 __global__ void __launch_bounds__(kFilterThreads, 1)
 filter_kernel(const __grid_constant__ CUtensorMap map_16, const __grid_constant__ CUtensorMap map_64,
               const __grid_constant__ CUtensorMap map_128, const filter_params p)
@@ -436,6 +436,8 @@ filter_kernel(const __grid_constant__ CUtensorMap map_16, const __grid_constant_
       const uint4 d0 = nx_d, dg = nx_g;
       const float mul = nx_rec.x, add = nx_rec.y;
       float4* out    = p.units + __float_as_uint(nx_rec.z);
+      uint4* codes   = kCodes ? p.row_codes + __float_as_uint(nx_rec.z) : nullptr;
+      const uint64_t per = dup2(nx_rec.w);
       if (t + gridDim.x < n_tiles) { load_tile(t + gridDim.x); }
       const uint32_t acc = it & 1u;
       if (ok && !mbar_wait(bar_tfull + acc * 8, (it >> 1) & 1u, p.spin_limit)) { ok = false; }
@@ -453,15 +455,35 @@ filter_kernel(const __grid_constant__ CUtensorMap map_16, const __grid_constant_
           const uint32_t pr = __shfl_sync(kFullMask, dg.y, int(g)), gl = __shfl_sync(kFullMask, dg.z, int(g));
           const uint32_t p0 = (pr >> 8) & 0xFFu, np = (pr >> 16) & 0xFFu;  // the group's pairs
           tmem_ld_wait(x);
-          float m[4];
+          float m[4], least[4];
 #pragma unroll
           for (int u = 0; u < 4; u++) {
             float a = min3(__uint_as_float(x[8 * u]), __uint_as_float(x[8 * u + 1]), __uint_as_float(x[8 * u + 2]));
             a       = min3(a, __uint_as_float(x[8 * u + 3]), __uint_as_float(x[8 * u + 4]));
             a       = min3(a, __uint_as_float(x[8 * u + 5]), __uint_as_float(x[8 * u + 6]));
-            m[u]    = __fmaf_rn(fminf(a, __uint_as_float(x[8 * u + 7])), mul, add);
+            a       = fminf(a, __uint_as_float(x[8 * u + 7]));
+            m[u]    = __fmaf_rn(a, mul, add);
+            least[u] = a;
           }
-          if (r - p0 < np) { out[gl] = make_float4(m[0], m[1], m[2], m[3]); }
+          const bool mine = r - p0 < np;
+          if (mine) { out[gl] = make_float4(m[0], m[1], m[2], m[3]); }
+          if constexpr (kCodes) {
+            // rows above it in whole steps, at most 15: the nearest integer of (steps - 1/2), which never exceeds the steps, in the
+            // low bits of a float of 1.5 2^23; shifted and summed, all but those bits come to a constant
+            uint32_t code[4];
+#pragma unroll
+            for (int u = 0; u < 4; u++) {
+              const uint64_t low = dup2(least[u]);
+              code[u]            = 0u - 0x3F400000u;
+#pragma unroll
+              for (int e = 0; e < 8; e += 2) {
+                const uint64_t d = fma2(sub2(pack2(x[8 * u + e], x[8 * u + e + 1]), low), per, dup2(-0.5f));
+                code[u] += __float_as_uint(fminf(lo2(d), 15.0f) + 12582912.0f) << (4 * e);
+                code[u] += __float_as_uint(fminf(hi2(d), 15.0f) + 12582912.0f) << (4 * e + 4);
+              }
+            }
+            if (mine) { codes[gl] = make_uint4(code[0], code[1], code[2], code[3]); }
+          }
         }
       }
       tc_fence_before();
@@ -634,7 +656,7 @@ make_tiles_kernel(uint32_t* __restrict__ list_count, const uint32_t* __restrict_
 // The query operand: sixteen lanes per (query, probe) pair.  `cursor`: next place of every list's pairs, which orders the
 // pairs by list.  A pair of an empty list has none.
 // Row of the operand: L2 -2 (q - c) s, inner product -q s_q, in half precision, then 1, 1, mask, 0, 1, 1, 0, 0
-// against the row side's |r|^2 and mask.  Record: {factor, constant, first group of the pair's bounds, -}.
+// against the row side's |r|^2 and mask.  Record: {factor, constant, first group of the pair's bounds, steps per value}.
 __global__ void __launch_bounds__(256)
 pair_operands_kernel(const operand_params p, const uint32_t* __restrict__ probes, const uint32_t* __restrict__ list_sizes,
                      uint32_t n_lists, const uint32_t* __restrict__ group_index, uint32_t n_pairs, uint32_t n_probes,
@@ -717,21 +739,26 @@ pair_operands_kernel(const operand_params p, const uint32_t* __restrict__ probes
     b_sum         = p.is_ip ? b_sum + x : fmaxf(b_sum, x);
   }
   if (lane == 0) {
-    float mul, add, norm;
+    float mul, add, norm, per;
     if (p.is_ip) {
       mul  = 1.0f / (sq * p.scale);
       add  = -b_sum;
       norm = sqrtf(a_sum) * 1.00001f;
+      per  = mul * sq / p.row_step;
     } else {
       mul  = p.inv_scale2;
       add  = a_sum * p.inv_scale2;
       norm = sqrtf(add) * 1.00001f;
       const float far = b_sum + p.rcomp_max;
+      per  = mul / (p.row_step * add);
       // differences that do not fit half precision: no bound for this pair
       if (!(b_sum * p.scale <= 16384.0f)) { add = INFINITY; }
       if (!(float(p.pq_len) * far * far < p.entry_limit)) { norm = -norm - 1e-30f; }
     }
-    pair_rec[pos] = make_float4(mul, add, __uint_as_float(q * max_groups + (pi > 0 ? __ldg(group_index + i - 1) : 0u)), 0.0f);
+    // (no steps that make sense: every row counts as its unit)
+    if (!(per > 0.0f && per < 1e25f && add < INFINITY)) { per = 0.0f; }
+    pair_rec[pos] = make_float4(mul, add, __uint_as_float(q * max_groups + (pi > 0 ? __ldg(group_index + i - 1) : 0u)),
+                                per * 0.9999f);
     pair_norm[i]  = norm;
   }
 }
@@ -895,7 +922,8 @@ void launch_filter(const filter_params& p, const __half* operand, uint32_t n_pai
   const CUtensorMap m16  = make_map_2d(CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, operand, n_pairs, k, 16, kBlockK, CU_TENSOR_MAP_SWIZZLE_128B);
   const CUtensorMap m64  = make_map_2d(CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, operand, n_pairs, k, 64, kBlockK, CU_TENSOR_MAP_SWIZZLE_128B);
   const CUtensorMap m128 = make_map_2d(CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, operand, n_pairs, k, 128, kBlockK, CU_TENSOR_MAP_SWIZZLE_128B);
-  auto go = [&](auto kernel) {
+  auto go = [&](auto with_codes, auto without) {
+    auto kernel = p.row_codes != nullptr ? with_codes : without;
     ensure_dynamic_smem(reinterpret_cast<const void*>(kernel), smem);
     launch_chained(kernel, grid, kFilterThreads, smem, stream, m16, m64, m128, p);
     CUDA_TRY(cudaGetLastError());
@@ -904,10 +932,10 @@ void launch_filter(const filter_params& p, const __half* operand, uint32_t n_pai
     constexpr int kB     = decltype(bits)::value;
     constexpr bool kWord = decltype(words)::value;
     switch (p.len_pad) {
-      case 1: go(filter_kernel<kB, 1, kWord>); break;
-      case 2: go(filter_kernel<kB, 2, kWord>); break;
-      case 4: go(filter_kernel<kB, 4, kWord>); break;
-      default: go(filter_kernel<kB, 8, kWord>);
+      case 1: go(filter_kernel<kB, 1, kWord, true>, filter_kernel<kB, 1, kWord, false>); break;
+      case 2: go(filter_kernel<kB, 2, kWord, true>, filter_kernel<kB, 2, kWord, false>); break;
+      case 4: go(filter_kernel<kB, 4, kWord, true>, filter_kernel<kB, 4, kWord, false>); break;
+      default: go(filter_kernel<kB, 8, kWord, true>, filter_kernel<kB, 8, kWord, false>);
     }
   };
   using std::integral_constant;
@@ -916,7 +944,7 @@ void launch_filter(const filter_params& p, const __half* operand, uint32_t n_pai
       if (p.len_pad <= 8) {
         by_len(integral_constant<int, 8>{}, std::true_type{});
       } else {
-        go(filter_kernel<8, 8, false>);
+        go(filter_kernel<8, 8, false, true>, filter_kernel<8, 8, false, false>);
       }
       break;
     case 7: by_len(integral_constant<int, 7>{}, std::false_type{}); break;
@@ -926,7 +954,7 @@ void launch_filter(const filter_params& p, const __half* operand, uint32_t n_pai
       if (p.len_pad <= 8) {
         by_len(integral_constant<int, 4>{}, std::true_type{});
       } else {
-        go(filter_kernel<4, 8, false>);
+        go(filter_kernel<4, 8, false, true>, filter_kernel<4, 8, false, false>);
       }
   }
 }

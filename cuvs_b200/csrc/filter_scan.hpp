@@ -35,6 +35,7 @@ struct operand_params {
   int is_ip;
   float scale, inv_scale2;                  // power of two s: codewords and differences are multiplied by it
   float entry_limit, rcomp_max;             // a table entry that may exceed the limit flags its pair
+  float row_step;                           // see row_step of rescore_params
 };
 
 struct filter_params {
@@ -49,8 +50,9 @@ struct filter_params {
   int is_ip;
   const filter_tile* tiles;
   const uint32_t* n_tiles;
-  const float4* pair_rec;  // per pair, in the operand's order: {factor, constant, first group of its units, -}
+  const float4* pair_rec;  // per pair, in the operand's order: {factor, constant, first group of its units, row codes per value}
   float4* units;           // [n_q, max_groups] bounds of the four units of a 32-row group
+  uint4* row_codes;        // optional: [n_q, max_groups] how far above it its rows are, four bits each, in steps (row_step)
   uint32_t n_stages;
   uint32_t* error;
   uint32_t spin_limit, skip_kb;  // tc_wait_limits
@@ -67,7 +69,9 @@ struct rescore_params {
   const uint32_t* chunk_index;  // [n_q, n_probes] inclusive sums of list sizes
   const uint32_t* group_index;  // [n_q, n_probes] inclusive sums of 32-row groups
   const float4* units;
+  const uint4* row_codes;       // optional
   const float* pair_norm;
+  const float* q_scale;         // inner product
   const uint32_t* error;
   uint32_t* timeouts;           // pinned host word: batches with the error word set
   const uint32_t* filter_bits;
@@ -80,6 +84,8 @@ struct rescore_params {
   float post_scale;
   // error model (see rescore.cu)
   float e1, kappa, e0, delta_lo, delta_hi, eta, sum_limit, rmax, ip_gemm, ip_lut;
+  // step of the row codes: L2 |d|^2 row_step, inner product row_step over the query's scale (less what rounding may do)
+  float row_step;
   int sharpen;    // wide bounds: score what is certainly wanted first
   int saturates;  // the table type saturates (8-bit tables)
   uint32_t* claim;  // zero on entry: next query to take
@@ -97,7 +103,7 @@ struct filter_plan {
 
 // Whether (and with which shared-memory plan) a search runs on the two-step path (k <= 128).
 filter_plan plan_filter(const raft::resources& res, const index<int64_t>& idx, int lut_kind, bool out_half, bool is_ip,
-                        uint32_t k, uint32_t n_probes, uint32_t n_queries);
+                        uint32_t k, uint32_t n_probes, uint32_t n_queries, bool row_codes);
 
 // `operand`: [n_pairs, k_chunks * 8] halfs written by launch_pair_operands.
 void launch_filter(const filter_params& p, const __half* operand, uint32_t n_pairs, int grid, size_t smem,

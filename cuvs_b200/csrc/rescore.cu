@@ -116,6 +116,7 @@ __device__ __forceinline__ uint32_t find_offset(const uint32_t* off, uint32_t n,
 // Shared memory of one thread group.
 struct group_mem {
   uint64_t* buf;     // [cap] keys
+  uint32_t* rows;    // [2 * threads, with row codes] rows of the query's groups, expanded from units and not scored yet
   uint2* list;       // [list_cap] {unit, value}: from the front the units among the k smallest, from the back the rest
   float* rq;         // [rot_dim]
   uint64_t* row;     // [P] arena row of the probe's list
@@ -130,10 +131,10 @@ constexpr uint32_t kMaxGroupThreads = 256;  // threads per query
 // No bound: every score is kept but NaN (its bits order as 0xFFFFFFFF), which is no result, as in the scan (scan.cuh).  As a
 // float a NaN itself, which nothing exceeds.
 constexpr uint32_t kNoBound = 0xFFFFFFFEu;
-enum { W_KEYS = 0, W_FRONT = 1, W_BACK = 2, W_BOUND = 3, W_VK = 4, W_VMAX = 5, W_NEXT = 6 };
-__host__ __device__ inline uint32_t group_mem_bytes(uint32_t cap, uint32_t list_cap, uint32_t n_probes, uint32_t rot_dim)
+enum { W_KEYS = 0, W_FRONT = 1, W_BACK = 2, W_BOUND = 3, W_VK = 4, W_VMAX = 5, W_NEXT = 6, W_ROWS = 7 };
+__host__ __device__ inline uint32_t group_mem_bytes(uint32_t cap, uint32_t list_cap, uint32_t rows_cap, uint32_t n_probes, uint32_t rot_dim)
 {
-  return round_up<uint32_t>(cap * 8u + list_cap * 8u + n_probes * 8u + round_up<uint32_t>(rot_dim, 4u) * 4u +
+  return round_up<uint32_t>(cap * 8u + list_cap * 8u + rows_cap * 4u + n_probes * 8u + round_up<uint32_t>(rot_dim, 4u) * 4u +
                               (n_probes + 1u) * 8u + n_probes * 8u + 32u, 16u);
 }
 
@@ -269,7 +270,7 @@ __device__ __forceinline__ bool score_row(const rescore_params& p, const float* 
   return true;
 }
 
-template <int LutKind, bool OutHalf, bool IsIP, int kLen, int kBits, bool kSmem>
+template <int LutKind, bool OutHalf, bool IsIP, int kLen, int kBits, bool kSmem, bool kCodes>
 __global__ void __launch_bounds__(1024, 1) rescore_kernel(const rescore_params p)
 {
   extern __shared__ __align__(16) uint8_t smem[];
@@ -289,7 +290,8 @@ __global__ void __launch_bounds__(1024, 1) rescore_kernel(const rescore_params p
     uint8_t* b = smem + p.book_bytes + size_t(g) * p.group_bytes;
     s.buf      = reinterpret_cast<uint64_t*>(b);
     s.list     = reinterpret_cast<uint2*>(s.buf + p.cap);
-    s.rq       = reinterpret_cast<float*>(s.list + p.list_cap);
+    s.rows     = reinterpret_cast<uint32_t*>(s.list + p.list_cap);
+    s.rq       = reinterpret_cast<float*>(s.rows + (kCodes ? 2u * gt : 0u));
     s.row      = reinterpret_cast<uint64_t*>(s.rq + round_up<uint32_t>(p.rot_dim, 4u));
     s.goff     = reinterpret_cast<uint32_t*>(s.row + P);
     s.soff     = s.goff + P + 1;
@@ -334,12 +336,15 @@ __global__ void __launch_bounds__(1024, 1) rescore_kernel(const rescore_params p
       s.word[W_KEYS]  = 0;
       s.word[W_FRONT] = 0;
       s.word[W_BACK]  = 0;
+      s.word[W_ROWS]  = 0;
       s.word[W_BOUND] = kNoBound;
       s.word[W_VK]    = __float_as_uint(-INFINITY);
       s.word[W_VMAX]  = __float_as_uint(INFINITY);
     }
     const uint32_t n_units4 = __ldg(p.group_index + size_t(q) * P + P - 1);
     const float4* units     = p.units + size_t(q) * p.max_groups;
+    const auto* codes       = kCodes ? reinterpret_cast<const uint32_t*>(p.row_codes + size_t(q) * p.max_groups) : nullptr;
+    const float row_step    = kCodes && IsIP ? p.row_step / __ldg(p.q_scale + q) : 0.0f;
 
     // ---- V: the k-th smallest value of the units (every thread contributes its two smallest) ----
     float best[2] = {INFINITY, INFINITY};
@@ -472,21 +477,71 @@ __global__ void __launch_bounds__(1024, 1) rescore_kernel(const rescore_params p
       }
       sync();
     };
-    // exact scores of the rows of the listed units [first, last)
+    // exact scores of the rows of the listed units [first, last).  With row codes, eight threads per unit leave the rows that the
+    // bound does not rule out (a unit's value and the row's code bound the row's value from below) and a thread per row scores them:
+    // some 350 rows per query of a 64-probe batch with 8-bit tables and k 100, whose whole units are 2,000.
+    // Kernels of their own with and without codes, here and in step 1: one for both took 253 against 247 us without codes (777 x 40
+    // pairs, half sums) and 1,204 against 1,187 with them (10,000 queries x 50,000 lists).
     auto score_listed = [&](uint32_t first, uint32_t last) {
-      for (uint32_t b0 = first; b0 < last; b0 += gt / kUnitRows) {
-        if (n_most + gt > p.cap) { compact(); }
+      uint32_t n_rows = 0;  // rows waiting
+      for (uint32_t u0 = first; u0 < last || n_rows > 0;) {
+        uint32_t gi, pi, lrow;  // group of the query, its probe, row of that list
+        bool valid;
+        if constexpr (kCodes) {
+          while (u0 < last && n_rows < gt) {
+            const uint32_t ui = u0 + t / kUnitRows;
+            bool live         = ui < last;
+            const uint2 e     = s.list[live ? ui : first];
+            gi                = e.x >> 2;
+            pi                = find_offset(s.goff, P, gi);
+            const uint32_t lr = (e.x & 3u) * kUnitRows + (lane & 7u);
+            live              = live && (gi - s.goff[pi]) * 32u + lr < s.soff[pi + 1] - s.soff[pi];
+            if (!all && live) {
+              float value          = __uint_as_float(e.y);
+              const float norm     = s.norm[pi];
+              const uint32_t steps = (__ldg(codes + e.x) >> (4u * (lane & 7u))) & 15u;
+              if (steps != 0u && value < INFINITY) { value = __fmaf_rd(float(steps), IsIP ? row_step : norm * norm * p.row_step, value); }
+              live = !(unit_lo<IsIP>(p, value, norm, qn) > ordered_to_float(s.word[W_BOUND]));
+            }
+            u0 += gt / kUnitRows;
+            const unsigned m = __ballot_sync(kFullMask, live);
+            if (m != 0u) {
+              uint32_t base = 0;
+              if (lane == 0) { base = atomicAdd(&s.word[W_ROWS], uint32_t(__popc(m))); }
+              base = __shfl_sync(kFullMask, base, 0);
+              if (live) { s.rows[base + __popc(m & ((1u << lane) - 1u))] = (gi << 5) | lr; }
+            }
+            sync();
+            n_rows = s.word[W_ROWS];
+            sync();  // everybody has read it before anybody adds to it
+          }
+          if (n_rows == 0) { break; }
+          // (the last ones; fewer than gt are left to wait)
+          const uint32_t from = n_rows > gt ? n_rows - gt : 0u;
+          valid               = from + t < n_rows;
+          const uint32_t row_of = s.rows[valid ? from + t : from];
+          n_rows              = from;
+          gi                  = row_of >> 5;
+          pi                  = find_offset(s.goff, P, gi);
+          lrow                = (gi - s.goff[pi]) * 32u + (row_of & 31u);
+          if (n_most + gt > p.cap) { compact(); }
+        } else {
+          if (n_most + gt > p.cap) { compact(); }
+          const uint32_t ui = u0 + t / kUnitRows;
+          valid             = ui < last;
+          const uint2 e     = s.list[valid ? ui : first];
+          gi                = e.x >> 2;
+          pi                = find_offset(s.goff, P, gi);
+          lrow              = (gi - s.goff[pi]) * 32u + (e.x & 3u) * kUnitRows + (lane & 7u);
+          valid             = valid && lrow < s.soff[pi + 1] - s.soff[pi];
+          if (!all) { valid = valid && !(unit_lo<IsIP>(p, __uint_as_float(e.y), s.norm[pi], qn) > ordered_to_float(s.word[W_BOUND])); }
+          u0 += gt / kUnitRows;
+        }
         n_most += gt;
-        const uint32_t ui   = b0 + t / kUnitRows;
-        const bool live     = ui < last;
-        const uint2 e       = s.list[live ? ui : first];
-        const uint32_t gi = e.x >> 2, pi = find_offset(s.goff, P, gi);
-        const uint32_t lrow = (gi - s.goff[pi]) * 32u + (e.x & 3u) * kUnitRows + (lane & 7u);  // row of the list
         const uint64_t row  = s.row[pi] + lrow;
         const uint32_t b_ord = s.word[W_BOUND];
         const float bound    = ordered_to_float(b_ord);  // NaN: none
-        bool valid = live && lrow < s.soff[pi + 1] - s.soff[pi];
-        if (!all) { valid = valid && !(unit_lo<IsIP>(p, __uint_as_float(e.y), s.norm[pi], qn) > bound); }
+        if (kCodes && t == 0) { s.word[W_ROWS] = n_rows; }
         float f  = 0.0f;
         __half h = __ushort_as_half(0);
         if (valid) {
@@ -648,24 +703,37 @@ void launch_rescore(const rescore_params& p, int lut_kind, bool out_half, bool i
   };
   // straight-line code for 8- and 4-bit codes of two or four components (whole 16-byte groups of components)
   const bool whole = p.rot_dim % 4 == 0;
-  auto shape_home = [&](auto lut, auto oh, auto ip, auto smem_book) {
+  auto shape_home = [&](auto lut, auto oh, auto ip, auto smem_book, auto codes) {
     constexpr int kL   = decltype(lut)::value;
-    constexpr bool kOH = decltype(oh)::value, kIP = decltype(ip)::value, kS = decltype(smem_book)::value;
+    constexpr bool kOH = decltype(oh)::value, kIP = decltype(ip)::value, kS = decltype(smem_book)::value, kC = decltype(codes)::value;
     if (whole && p.pq_bits == 8 && p.pq_len == 2) {
-      go(rescore_kernel<kL, kOH, kIP, 2, 8, kS>);
+      go(rescore_kernel<kL, kOH, kIP, 2, 8, kS, kC>);
     } else if (whole && p.pq_bits == 8 && p.pq_len == 4) {
-      go(rescore_kernel<kL, kOH, kIP, 4, 8, kS>);
+      go(rescore_kernel<kL, kOH, kIP, 4, 8, kS, kC>);
     } else if (whole && p.pq_bits == 4 && p.pq_len == 2) {
-      go(rescore_kernel<kL, kOH, kIP, 2, 4, kS>);
+      go(rescore_kernel<kL, kOH, kIP, 2, 4, kS, kC>);
     } else {
-      go(rescore_kernel<kL, kOH, kIP, 0, 0, kS>);
+      go(rescore_kernel<kL, kOH, kIP, 0, 0, kS, kC>);
     }
   };
   auto shape = [&](auto lut, auto oh, auto ip) {
-    if (p.book_bytes != 0u) {
-      shape_home(lut, oh, ip, std::true_type{});
+    auto home = [&](auto codes) {
+      if (p.book_bytes != 0u) {
+        shape_home(lut, oh, ip, std::true_type{}, codes);
+      } else {
+        shape_home(lut, oh, ip, std::false_type{}, codes);
+      }
+    };
+    // (tight bounds always come with row codes)
+    if constexpr (decltype(lut)::value == LUT_FP8 || decltype(oh)::value) {
+      if (p.row_codes == nullptr) {
+        home(std::false_type{});
+      } else {
+        home(std::true_type{});
+      }
     } else {
-      shape_home(lut, oh, ip, std::false_type{});
+      CUVS_EXPECTS(p.row_codes != nullptr, "two-step search: no row codes");
+      home(std::true_type{});
     }
   };
   using std::bool_constant;
@@ -692,7 +760,7 @@ void launch_rescore(const rescore_params& p, int lut_kind, bool out_half, bool i
 }
 
 filter_plan plan_filter(const raft::resources& res, const index<int64_t>& idx, int lut_kind, bool out_half, bool is_ip,
-                        uint32_t k, uint32_t n_probes, uint32_t n_queries)
+                        uint32_t k, uint32_t n_probes, uint32_t n_queries, bool row_codes)
 {
   filter_plan plan{};
   // Where the bounds say too little the look-up-table scan is the better one: signed sums of coarse entries
@@ -726,7 +794,7 @@ filter_plan plan_filter(const raft::resources& res, const index<int64_t>& idx, i
   plan.cap           = cap;
   plan.list_cap      = kListPerThread * gt;
   plan.group_threads = gt;
-  plan.group_bytes   = group_mem_bytes(cap, plan.list_cap, n_probes, idx.rot_dim());
+  plan.group_bytes   = group_mem_bytes(cap, plan.list_cap, row_codes ? 2 * gt : 0, n_probes, idx.rot_dim());
   // As many groups per CTA as threads and shared memory allow, beside the codebook in shared memory where that leaves at
   // least half of the threads; with fewer queries than SMs, one query per CTA reading the codebook through the caches
   // (a copy would cost more than the look-ups it serves).

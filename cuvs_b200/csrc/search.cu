@@ -898,17 +898,23 @@ void search_any(raft::resources& res, const search_params& params, const index<i
                                                    (idx.pq_bits() == 4 && idx.pq_len() == 2));
   const bool never       = (lut_kind == LUT_FP8 && !(straight && idx.pq_bits() == 8)) || (out_half && !straight && n_probes < 2 * k);
   const uint64_t enough  = straight && !wide_bounds ? 4096 : 16384;
+  // Codes of the rows beside the units' bounds leave the exact scores a sixth to a half of the rows and cost the first step 3 to 15%.
+  // Whole calls without / with them (us): half-precision tables, k 20, 10,000 queries x 50,000 lists 1,190 / 1,187; fp32 tables
+  // whose codebook exceeds shared memory, k 10 612 / 509; 4-bit inner product, k 10 1,094 / 1,074; 8-bit tables, k 100 3,115 / 2,734.
+  // With wide bounds and few neighbours the scores are too few to pay: 8-bit tables, k 10 1,143 / 1,190; half sums, k 10 247 / 269.
+  const bool row_codes = !wide_bounds || k > 64;
   // (a list-sharded search exchanges bounds in the middle of the look-up-table scan: a collective, so that all its ranks
   // take that path)
   const int home = scan_codebook_home();
   if (!res.scan_phase_hook && !store_all && (home == 4 || (home == 0 && !never && uint64_t(batch) * n_probes > enough))) {
-    fplan = plan_filter(res, idx, lut_kind, out_half, is_ip, k, n_probes, batch);
-    // the bounds and the query operand of one internal batch: within 2 GiB each
-    const uint64_t per_query = std::max(uint64_t(max_groups), uint64_t(n_probes) * f_chunks) * 16;
-    const auto fits          = uint32_t(std::max<uint64_t>(1, (1ull << 31) / per_query));
+    fplan = plan_filter(res, idx, lut_kind, out_half, is_ip, k, n_probes, batch, row_codes);
+    // the bounds (with the row codes), and the query operand of one internal batch: within 2 (3) and 2 GiB
+    const uint64_t fits_bounds  = row_codes ? (3ull << 30) / (uint64_t(max_groups) * 32) : (1ull << 31) / (uint64_t(max_groups) * 16);
+    const uint64_t fits_operand = (1ull << 31) / (uint64_t(n_probes) * f_chunks * 16);
+    const auto fits             = uint32_t(std::max<uint64_t>(1, std::min(fits_bounds, fits_operand)));
     if (fplan.use && fits < batch) {
       // (the plan shares threads out by the number of queries; the look-up-table scan needs no smaller batch)
-      fplan = plan_filter(res, idx, lut_kind, out_half, is_ip, k, n_probes, fits);
+      fplan = plan_filter(res, idx, lut_kind, out_half, is_ip, k, n_probes, fits, row_codes);
       if (fplan.use) { batch = fits; }
     }
   }
@@ -939,6 +945,7 @@ void search_any(raft::resources& res, const search_params& params, const index<i
   const size_t o_norm    = lay.add(f_use ? n_pairs_max * 4 : 0);
   const size_t o_tiles   = lay.add(n_tiles * sizeof(filter_tile));
   const size_t o_units   = lay.add(f_use ? size_t(batch) * max_groups * 16 : 0);
+  const size_t o_rowcode = lay.add(f_use && row_codes ? size_t(batch) * max_groups * 16 : 0);
   const size_t o_qscale  = lay.add(f_use && is_ip ? size_t(batch) * 4 : 0);
   const size_t o_operand = lay.add(f_use ? n_pairs_max * f_chunks * 16 : 0);
   const size_t o_order   = lay.add(f_use ? 0 : n_pairs_max * 32);
@@ -1033,6 +1040,7 @@ void search_any(raft::resources& res, const search_params& params, const index<i
       auto* d_norm    = reinterpret_cast<float*>(ws + o_norm);
       auto* d_tiles   = reinterpret_cast<filter_tile*>(ws + o_tiles);
       auto* d_units   = reinterpret_cast<float4*>(ws + o_units);
+      auto* d_rowcode = reinterpret_cast<uint4*>(ws + o_rowcode);
       auto* d_qscale  = reinterpret_cast<float*>(ws + o_qscale);
       auto* d_operand = reinterpret_cast<__half*>(ws + o_operand);
       // 3. tiles, and the query operand of every pair, ordered by list; d_counter: pairs, tiles, error word
@@ -1066,6 +1074,9 @@ void search_any(raft::resources& res, const search_params& params, const index<i
       op.inv_scale2  = 1.0f / (fm.scale * fm.scale);
       op.entry_limit = lut_kind == LUT_F16 || out_half ? 6.0e4f : (lut_kind == LUT_FP8 ? 1.2e5f : INFINITY);
       op.rcomp_max   = fm.comp_max;
+      // Steps of the row codes: 15 of them reach as far above a unit's value as the bounds leave rows.  L2: in shares of |d|^2;
+      // inner product: an eighth of what a component of a residual of the largest norm is on average.
+      op.row_step    = is_ip ? 90.0f * fm.rmax / (8.0f * std::sqrt(float(idx.rot_dim()))) : (wide_bounds ? 1.0f / 32 : 1.0f / 64);
       launch_pair_operands(op, d_probes, idx.list_sizes(), n_lists, d_groups, n_pairs, n_probes, max_groups,
                            d_count, d_operand, d_rec, d_norm, stream);
       res.launches++;
@@ -1090,6 +1101,7 @@ void search_any(raft::resources& res, const search_params& params, const index<i
       fp.n_tiles      = d_counter + 1;
       fp.pair_rec     = d_rec;
       fp.units        = d_units;
+      fp.row_codes    = row_codes ? d_rowcode : nullptr;
       fp.n_stages     = fplan.n_stages;
       fp.error        = d_counter + 2;
       const wait_limits wl = tc_wait_limits();
@@ -1110,6 +1122,9 @@ void search_any(raft::resources& res, const search_params& params, const index<i
       rp.chunk_index  = d_chunk;
       rp.group_index  = d_groups;
       rp.units        = d_units;
+      rp.row_codes    = fp.row_codes;
+      rp.q_scale      = d_qscale;
+      rp.row_step     = 0.999f * op.row_step;
       rp.pair_norm    = d_norm;
       rp.error        = d_counter + 2;
       rp.timeouts     = res.pinned + 13;

@@ -3,6 +3,7 @@ against the CPU oracle: ids and distance bits."""
 import numpy as np
 import pytest
 
+from conftest import make_mixture
 from test_search_gpu import LUT, assert_parity, build_case, gpu_search
 
 pytestmark = pytest.mark.gpu
@@ -235,3 +236,23 @@ def test_workspace_of_a_skewed_index(ivf):
     assert used < 4 << 30, used
     d2, i2 = ivf.search(sp(500), index, q, 10)
     assert bool((i == i2).all()) and bool((d == d2).all())
+
+
+# rows left by their distance above the unit's value: tight bounds (steps saturate), wide bounds with many neighbours, signed scores,
+# lists that end inside a unit; against the tables bit for bit
+@pytest.mark.parametrize("metric,lut,k", [("sqeuclidean", "f16", 20), ("sqeuclidean", "f32", 128), ("sqeuclidean", "fp8", 100),
+                                          ("inner_product", "f16", 10), ("cosine", "f32", 65)])
+@pytest.mark.parametrize("dim,pq_dim,bits", [(96, 48, 8), (64, 32, 4), (50, 24, 6)])
+def test_row_codes_leave_what_the_tables_find(ivf, metric, lut, k, dim, pq_dim, bits):
+    from cuvs_b200 import _lib as L
+    x = make_mixture(60_001, dim, 60, 0.3, seed=dim)
+    q = make_mixture(900, dim, 60, 0.3, seed=dim + 1)
+    g = ivf.build(ivf.IndexParams(n_lists=150, pq_dim=pq_dim, pq_bits=bits, metric=metric, kmeans_n_iters=3), torch.from_numpy(x).cuda())
+    L.check(L.load().cuvsB200SetScanCodebookHome(4))
+    try:
+        d2, i2 = gpu_search(ivf, g, q, k, 20, lut, "f32")
+        L.check(L.load().cuvsB200SetScanCodebookHome(2))
+        d0, i0 = gpu_search(ivf, g, q, k, 20, lut, "f32")
+    finally:
+        L.check(L.load().cuvsB200SetScanCodebookHome(0))
+    assert (i0 == i2).all() and (d0.view(np.uint32) == d2.view(np.uint32)).all()
