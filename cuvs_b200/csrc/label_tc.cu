@@ -18,10 +18,10 @@
 //      what is left in ever finer sums, the defining chain last.
 //   4. If the fourth unit kept is inside, a fifth might be: such rows (2.7% of 1 M rows x 16,384 lists of 96 dimensions) go
 //      through 2 and 3 once more with the lists in eight shares; only what that does not settle is redone exactly over all lists.
-// What bounds row_list_kernel: the issue and execution of the MMAs (1,300 clocks per 128 x 256 x 96; the products alone take 880),
-// then the comparisons (740).  1,000,003 rows x 16,384 lists x 96 dimensions, all of the labelling: 9.4 ms with two products
-// (row operand as two halfs), units of 64 lists whose largest two values were kept with their columns, and 2% of the rows
-// redone over all lists; 3.8 ms so.  (One product widens the bounds from 5.2e-5 to 6.5e-5: 2.6 instead of 2.2 lists within
+// What bounds row_list_kernel: the epilogue.  A 128 x 256 x 96 tile takes 1,260 clocks, 860 with the epilogue left out of a copy
+// of the kernel, and its products alone 770.  1,000,003 rows x 16,384 lists x 96 dimensions, all of the labelling: 9.4 ms with two
+// products (row operand as two halfs), units of 64 lists whose largest two values were kept with their columns, and 2% of the
+// rows redone over all lists; 3.8 ms so.  (One product widens the bounds from 5.2e-5 to 6.5e-5: 2.6 instead of 2.2 lists within
 // reach.)
 // Every wait is bounded: on a time-out the kernel raises the error word and returns, and all rows are redone.
 #include "common.hpp"
