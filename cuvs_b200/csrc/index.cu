@@ -234,15 +234,16 @@ void index<int64_t>::recompute_model_state(cudaStream_t stream)
     centers_lo_.resize(nc);
   }
   const bool norm_column = metric_ == DistanceType::L2Expanded || metric_ == DistanceType::L2SqrtExpanded;
-  prepare_tc_centers(stream, centers_.data(), n_lists_, dim_ext(), norm_column ? dim_ : dim_ext(),
-                     centers_hi_.data(), centers_lo_.data(), &centers_max_norm_, &centers_ext_scale_);
-  // and the half-precision operand of large batches
+  // and the half-precision operand of large batches; enqueued first, so that the synchronisation that ends
+  // prepare_tc_centers covers it: a caller may search on another stream as soon as this returns
   const size_t model_bytes = label_model_bytes(n_lists_, dim_, false);
   if (list_model_.size() != model_bytes) { list_model_.resize(model_bytes); }
   if (n_lists_ > 0) {
     prepare_label_model(stream, centers_.data(), n_lists_, dim_, dim_ext(), norm_column ? 0.5f : 0.0f, false,
                         list_model_.data());
   }
+  prepare_tc_centers(stream, centers_.data(), n_lists_, dim_ext(), norm_column ? dim_ : dim_ext(),
+                     centers_hi_.data(), centers_lo_.data(), &centers_max_norm_, &centers_ext_scale_);
   // codebooks in half precision for the fine search's tensor-core pass
   if (codebook_kind_ == codebook_gen::PER_SUBSPACE) {
     const uint32_t len = pq_len();

@@ -103,3 +103,22 @@ def test_a_wait_that_runs_out_redoes_every_query(mods, dim):
     again, m2 = run()
     assert m0 == 0 and m1 == 1 and m2 == m1
     assert bool((healthy == timed_out).all()) and bool((healthy == again).all())
+
+
+@pytest.mark.parametrize("per_cluster", [False, True])
+def test_a_model_is_complete_on_return(mods, per_cluster):
+    """Nothing of the derived state is still being made when the C call that lays out a model returns: a handle on another
+    stream may search at once."""
+    from cuvs_b200.common import DLTensorRef, Resources
+    ivf, _, L = mods
+    n_lists, dim = 30_000, 128
+    to = lambda a: torch.from_numpy(np.ascontiguousarray(a, dtype=np.float32)).cuda()  # noqa: E731
+    centers = to(make_mixture(n_lists, dim, 60, 0.4, 2))
+    books = torch.rand((n_lists if per_cluster else 2, dim // 2, 16), device="cuda")
+    params = ivf.IndexParams(n_lists=n_lists, pq_dim=2, pq_bits=4, codebook_kind="cluster" if per_cluster else "subspace")
+    stream = torch.cuda.Stream()
+    res, index = Resources(stream.cuda_stream), ivf.Index()
+    refs = [DLTensorRef(t) for t in (books, centers, centers, to(np.eye(dim)))]
+    torch.cuda.synchronize()
+    L.check(L.load().cuvsIvfPqBuildPrecomputed(res.handle, params._p, C.c_uint32(dim), *[r.ref() for r in refs], index._h))
+    assert stream.query()
