@@ -779,6 +779,18 @@ extern "C" cuvsError_t cuvsB200CoarseTimeouts(cuvsResources_t res, uint64_t* n_b
   });
 }
 
+extern "C" cuvsError_t cuvsB200RedoCounts(cuvsResources_t res, uint64_t* counts)
+{
+  return translate_exceptions([=] {
+    CUVS_EXPECTS(counts != nullptr, "null output pointer");
+    auto* r = res_of(res);
+    unsigned long long c[raft::resources::N_REDO_COUNTS];
+    CUDA_TRY(cudaMemcpyAsync(c, r->redo_counts, sizeof(c), cudaMemcpyDeviceToHost, r->stream));
+    r->sync();
+    std::copy(std::begin(c), std::end(c), counts);
+  });
+}
+
 extern "C" cuvsError_t cuvsB200SetCoarseWaitTest(uint32_t spin_limit, uint32_t skip_stage)
 {
   return translate_exceptions([=] {

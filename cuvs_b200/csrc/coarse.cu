@@ -469,11 +469,13 @@ void launch_select(const float* scores, uint32_t n_rows, uint32_t row_stride, ui
 
 __global__ void unpack_labels_kernel(const unsigned long long* __restrict__ best, uint32_t n,
                                      const uint32_t* __restrict__ row_list, const uint32_t* __restrict__ n_listed,
-                                     uint32_t* __restrict__ labels)
+                                     uint32_t* __restrict__ labels, unsigned long long* __restrict__ listed)
 {
   chain_begin();
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= (row_list != nullptr ? min(n, __ldg(n_listed)) : n)) { return; }
+  if (row_list != nullptr) { n = min(n, __ldg(n_listed)); }
+  if (i >= n) { return; }
+  if (i == 0 && listed != nullptr) { atomicAdd(listed, static_cast<unsigned long long>(n)); }
   const uint32_t r = row_list != nullptr ? __ldg(row_list + i) : i;
   labels[r]        = uint32_t(best[r]);
 }
@@ -543,7 +545,7 @@ void assign_nearest(raft::resources& res, const float* centers, uint32_t n_lists
   if (n_rows == 0) { return; }
   CUDA_TRY(cudaMemsetAsync(best, 0xFF, size_t(n_rows) * 8, res.stream));
   launch_exact_gemm<true>(centers, n_lists, x_ext, n_rows, dim_ext, dim_ext, alpha, false, nullptr, best, res.stream);
-  unpack_labels_kernel<<<ceildiv<uint32_t>(n_rows, 256), 256, 0, res.stream>>>(best, n_rows, nullptr, nullptr, labels);
+  unpack_labels_kernel<<<ceildiv<uint32_t>(n_rows, 256), 256, 0, res.stream>>>(best, n_rows, nullptr, nullptr, labels, nullptr);
   CUDA_TRY(cudaGetLastError());
   res.launches += 2;
 }
@@ -555,7 +557,8 @@ void assign_nearest_listed(raft::resources& res, const float* centers, uint32_t 
   CUVS_EXPECTS(n_rows <= 65535u * kTile, "too many rows");
   launch_exact_gemm<true, true>(centers, n_lists, x_ext, n_rows, dim_ext, dim_ext, alpha, false, nullptr, best, res.stream, row_list,
                                 n_listed);
-  launch_chained(unpack_labels_kernel, ceildiv<uint32_t>(n_rows, 256), 256, 0, res.stream, best, n_rows, row_list, n_listed, labels);
+  launch_chained(unpack_labels_kernel, ceildiv<uint32_t>(n_rows, 256), 256, 0, res.stream, best, n_rows, row_list, n_listed, labels,
+                 res.redo_counts + raft::resources::LABELS_REDONE);
   CUDA_TRY(cudaGetLastError());
   res.launches += 2;
 }

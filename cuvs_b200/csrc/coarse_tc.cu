@@ -1011,7 +1011,8 @@ coarse_fallback_kernel(const uint32_t* __restrict__ redo_list, const uint32_t* _
                        uint32_t dim_ext, float alpha, uint32_t n_probes, uint32_t cap,
                        float* __restrict__ scratch /* [gridDim.x, n_lists] */,
                        uint32_t* __restrict__ probes, float* __restrict__ scores_out,
-                       uint32_t* __restrict__ words, volatile uint32_t* __restrict__ host_words, uint32_t host_seq)
+                       uint32_t* __restrict__ words, volatile uint32_t* __restrict__ host_words, uint32_t host_seq,
+                       unsigned long long* __restrict__ redone)
 {
   chain_begin();
   const uint32_t* error_word = words;
@@ -1026,6 +1027,7 @@ coarse_fallback_kernel(const uint32_t* __restrict__ redo_list, const uint32_t* _
   const uint32_t n_redo = redo_all ? n_queries : min(*redo_count, n_queries);
   if (blockIdx.x == 0 && tid == 0) {
     words[1] = n_redo;
+    if (n_redo > 0) { atomicAdd(redone, static_cast<unsigned long long>(n_redo)); }
     if (host_words != nullptr) {
       // the batch's verdict straight into the handle's pinned words (a copy and an event cost the host 8 us per call)
       host_words[0] = words[0];
@@ -1417,7 +1419,8 @@ void launch_probe_redo(raft::resources& res, const uint32_t* redo_list, uint32_t
   launch_chained(coarse_fallback_scores_kernel, ceildiv<uint32_t>(n_lists, 256u), 256, fs_smem, res.stream, redo_list,
                  words + 2, centers, fq, n_queries, n_lists, dim_ext, alpha, scratch, kFbSlots, words);
   launch_chained(coarse_fallback_kernel, kFbSlots, 256, fb_smem, res.stream, redo_list, words + 2, centers, fq, n_queries,
-                 n_lists, dim_ext, alpha, n_probes, cap_fb, scratch, probes, scores_out, words, host_words, host_seq);
+                 n_lists, dim_ext, alpha, n_probes, cap_fb, scratch, probes, scores_out, words, host_words, host_seq,
+                 res.redo_counts + raft::resources::PROBES_REDONE);
   CUDA_TRY(cudaGetLastError());
   res.launches += 2;
 }

@@ -281,10 +281,11 @@ row_operand_kernel(const float* __restrict__ x, uint32_t n_rows, uint32_t n_list
 __global__ void __launch_bounds__(256)
 gather_operand_kernel(const __half* __restrict__ a, const float* __restrict__ factor, const uint32_t* __restrict__ rows,
                       const uint32_t* __restrict__ count, uint32_t cap, uint32_t width, __half* __restrict__ out,
-                      float* __restrict__ factor_out)
+                      float* __restrict__ factor_out, unsigned long long* __restrict__ listed)
 {
   chain_begin();
   const uint32_t n = min(__ldg(count), cap), lane = threadIdx.x & 31u;
+  if (n > 0 && blockIdx.x == 0 && threadIdx.x == 0) { atomicAdd(listed, static_cast<unsigned long long>(n)); }
   for (uint32_t i = (blockIdx.x * 256u + threadIdx.x) >> 5; i < n; i += gridDim.x * 8u) {
     const uint32_t r = __ldg(rows + i);
     const uint4* src = reinterpret_cast<const uint4*>(a + size_t(r) * width);
@@ -1115,7 +1116,8 @@ void label_rows_tc(raft::resources& res, const float* centers, const void* model
   res.launches += 3;
   if (y.second_pass()) {
     const uint32_t few = std::min<uint32_t>(uint32_t(res.sm_count) * 8, ceildiv(y.cap, 8u));
-    launch_chained(gather_operand_kernel, few, 256, 0, stream, a, factor, next, words + 2, y.cap, width, a2, factor2);
+    launch_chained(gather_operand_kernel, few, 256, 0, stream, a, factor, next, words + 2, y.cap, width, a2, factor2,
+                   res.redo_counts + raft::resources::LABELS_SECOND);
     f.rows = next;
     f.next_cap = 0;
     pass(y.second, a2, factor2, keys2, y.cap, words + 1, words + 2,

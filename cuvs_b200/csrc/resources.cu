@@ -63,6 +63,8 @@ resources::resources()
   CUDA_TRY(cudaMallocHost(&pinned, 64));
   pinned[12] = 0;
   pinned[13] = 0;
+  CUDA_TRY(cudaMalloc(&redo_counts, N_REDO_COUNTS * sizeof(*redo_counts)));
+  CUDA_TRY(cudaMemset(redo_counts, 0, N_REDO_COUNTS * sizeof(*redo_counts)));
 }
 
 resources::~resources()
@@ -71,6 +73,7 @@ resources::~resources()
     for (auto& e : ev.e) { cudaEventDestroy(e); }
   }
   if (d_stats) { cudaFree(d_stats); }
+  if (redo_counts) { cudaFree(redo_counts); }
   if (pinned) {
     cudaDeviceSynchronize();  // a kernel may still write its verdict or count a time-out there
     cudaFreeHost(pinned);

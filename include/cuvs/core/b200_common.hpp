@@ -180,6 +180,10 @@ struct resources {
   // batches whose coarse GEMM gave up on a bounded wait (their probes were recomputed exactly); those of the fine search's
   // bounds and of the labelling are counted by the kernels behind them in pinned[13]
   uint64_t tc_timeouts       = 0;
+  // Device words that the kernels add to: queries whose probes, rows whose label a tensor-core pass left to the exact product
+  // over all lists; between them, rows whose label took a second pass.
+  enum { PROBES_REDONE = 0, LABELS_SECOND = 1, LABELS_REDONE = 2, N_REDO_COUNTS = 3 };
+  unsigned long long* redo_counts = nullptr;
 
   resources();
   ~resources();

@@ -83,7 +83,13 @@ CUVS_EXPORT cuvsError_t cuvsB200RefineArrays(cuvsResources_t res, cudaStream_t s
  * waiting for nothing: it reports the batches whose verdict has arrived; cuvsStreamSync first makes that all of
  * them). */
 CUVS_EXPORT cuvsError_t cuvsB200CoarseTimeouts(cuvsResources_t res, uint64_t* n_batches);
-/* No counterpart in the reference; for tests of the above.  spin_limit: iterations (about a microsecond
+/* No counterpart in the reference.  What the tensor-core passes of this handle left to slower ones since its creation:
+ * counts[0] = queries whose probes, counts[2] = rows whose label was worked out over all lists with the defining
+ * arithmetic, because more lists lay within the error bound than there is room for (or a wait ran out);
+ * counts[1] = rows whose label took a second pass for the same reason.  The results are the same; many of them mean
+ * that the lists lie too close together for the bound.  Synchronises the stream. */
+CUVS_EXPORT cuvsError_t cuvsB200RedoCounts(cuvsResources_t res, uint64_t* counts /* [3] */);
+/* No counterpart in the reference; for tests of the time-outs.  spin_limit: iterations (about a microsecond
  * each) a wait of those kernels may take, 0 = the default of about two seconds; skip_stage: 1 + index of
  * an operand stage of each CTA's first tile that is never filled, so that the wait for it runs out;
  * 0 = none.  Process-wide. */

@@ -1,5 +1,7 @@
 """Labels and codes of `transform` against a float64 statement: the labelling on the tensor cores (and the exact pass below
 its size), and the encoder for every number of components per subspace."""
+import ctypes as C
+
 import numpy as np
 import pytest
 
@@ -155,13 +157,17 @@ def test_a_wait_that_runs_out_redoes_every_label(ivf, n, dim, n_lists):
 
 
 # more lists within reach of a row than the first pass keeps (four units of eight per column quarter), than a block of the
-# finish kernel has room for, and than the second pass keeps; one, two, three and more K blocks
-@pytest.mark.parametrize("n,dim,n_lists,alike", [(4097, 40, 4096, 64), (9000, 96, 4100, 12), (8200, 128, 2050, 10), (8200, 130, 2050, 10),
-                                                 (17000, 200, 1030, 6), (20000, 64, 1024, 512)])
-def test_many_lists_within_reach(ivf, n, dim, n_lists, alike):
+# finish kernel has room for, and than the second pass keeps; one, two, three and more K blocks.  second, full: rows go through
+# a second pass (there is none for so few rows that the first has as many shares), and to the exact product over all lists.
+@pytest.mark.parametrize("n,dim,n_lists,alike,second,full",
+                         [(4097, 40, 4096, 64, False, True), (9000, 96, 4100, 12, False, True), (8200, 128, 2050, 10, False, True),
+                          (8200, 130, 2050, 10, False, True), (17000, 200, 1030, 6, False, True), (20000, 64, 1024, 512, False, True),
+                          (41000, 96, 4096, 12, True, True), (40001, 130, 2050, 64, True, True), (150000, 32, 2048, 8, True, False)])
+def test_many_lists_within_reach(ivf, n, dim, n_lists, alike, second, full):
     """Centres in groups that differ by some 1e-5 of their length: the labels equal those of the exact product (the labelling
     kernel's waits made to run out)."""
     from cuvs_b200 import _lib as L
+    from cuvs_b200.common import Resources
     rng = np.random.default_rng(dim)
     groups = make_mixture(-(-n_lists // alike), dim, 40, 0.3, 1)
     centers = groups[rng.permutation(n_lists) % len(groups)] + 1e-5 * rng.standard_normal((n_lists, dim))
@@ -175,8 +181,10 @@ def test_many_lists_within_reach(ivf, n, dim, n_lists, alike):
     index = ivf.build_precomputed(ivf.IndexParams(n_lists=n_lists, pq_dim=len(books), pq_bits=4), dim, to(books), to(centers),
                                   to(centers), to(eye))
     x = to((groups[rng.integers(0, len(groups), n)] + 0.05 * rng.standard_normal((n, dim))).astype(np.float32))
-    labels = ivf.transform(index, x)[0].to(torch.int64)
-    lib = L.load()
+    lib, res, counts = L.load(), Resources(), (C.c_uint64 * 3)()
+    labels = ivf.transform(index, x, resources=res)[0].to(torch.int64)
+    L.check(lib.cuvsB200RedoCounts(res.handle, counts))
+    assert (counts[1] > 0) == second and (counts[2] > 0) == full
     try:
         L.check(lib.cuvsB200SetCoarseWaitTest(1000, 1))
         exact = ivf.transform(index, x)[0].to(torch.int64)

@@ -28,17 +28,25 @@ def index_of(ivf, centers, metric):
                                  to(centers), to(np.eye(dim)))
 
 
+def redone(mods, res):
+    """Queries whose probes were worked out over all lists, since the handle was made."""
+    counts = (C.c_uint64 * 3)()
+    mods[2].check(mods[2].load().cuvsB200RedoCounts(res.handle, counts))
+    return counts[0]
+
+
 def both(mods, index, q, n_probes):
-    """(probes as search selects them, probes of the exact product)"""
+    """(probes as search selects them, probes of the exact product, queries that the former left to all lists)"""
+    from cuvs_b200.common import Resources
     ivf, mg, L = mods
-    lib, got = L.load(), []
+    lib, got, res = L.load(), [], Resources()
     for mode in (0, 1):
         try:
             lib.cuvsB200SetCoarseMode(mode)
-            got.append(mg.select_probes(index, q, n_probes).to(torch.int64))
+            got.append(mg.select_probes(index, q, n_probes, resources=res).to(torch.int64))
         finally:
             lib.cuvsB200SetCoarseMode(0)
-    return got
+    return *got, redone(mods, res)
 
 
 # edges of the 256-query and 256-list tiles; 8, 32, 64 and 128 lists per maximum; one, two, three and more K blocks
@@ -52,8 +60,9 @@ def test_probes(mods, n_lists, n_q, dim, n_probes, metric):
     if metric == "cosine":
         centers /= np.linalg.norm(centers, axis=1, keepdims=True)
     index = index_of(mods[0], centers, metric)
-    fast, exact = both(mods, index, torch.from_numpy(q).cuda(), n_probes)
+    fast, exact, n = both(mods, index, torch.from_numpy(q).cuda(), n_probes)
     assert bool((fast == exact).all())
+    assert n <= n_q // 256                                         # ordinary data: the two passes settle it
 
 
 def test_odd_queries_and_equal_lists(mods):
@@ -71,7 +80,8 @@ def test_odd_queries_and_equal_lists(mods):
     q[40:80] = centers[8]
     for metric in ("sqeuclidean", "inner_product"):
         index = index_of(mods[0], centers, metric)
-        fast, exact = both(mods, index, torch.from_numpy(q.astype(np.float32)).cuda(), 40)
+        fast, exact, n = both(mods, index, torch.from_numpy(q.astype(np.float32)).cuda(), 40)
+        assert 41 <= n <= 120                                      # those at centers[8], without a bound, and few others
         fine = torch.ones(len(q), dtype=torch.bool, device="cuda")
         fine[1] = fine[2] = False                                  # (NaN scores have no order)
         assert bool((fast == exact).all(1)[fine].all())
