@@ -65,6 +65,25 @@ __host__ __device__ __forceinline__ size_t unit_operand_at(uint32_t n_lists, uin
   return operand_at(n_lists, dim) + round_up<size_t>(size_t(n_lists) * width * 2, 256);
 }
 
+// The list at a place of the operand that probes are selected from: a fixed shuffle of 0 .. n - 1 (odd multiples and shifted
+// exclusive-ors, each a permutation of the numbers of some bits, repeated while it leads beyond n).  A unit's maximum stands for
+// 8 to 128 neighbouring places: where neighbouring lists are alike -- a data set stored by cluster or by time, whose evenly taken
+// rows k-means starts from, or a model trained in levels -- few units hold all lists that are near, and a value that n_probes
+// units reach lies far below that of the n_probes-th list (4,000 lists sorted by component, 64 probes: every query had more
+// lists within reach than there is room for).
+__device__ __forceinline__ uint32_t list_at(uint32_t place, uint32_t n)
+{
+  const uint32_t bits = 32u - uint32_t(__clz(int(n - 1u))), shift = max(bits / 2u, 1u);
+  const uint32_t mask = bits < 32u ? (1u << bits) - 1u : ~0u;
+  do {
+    place = (place * 0x9E3779B1u) & mask;
+    place ^= place >> shift;
+    place = (place * 0x6A09E667u) & mask;
+    place ^= place >> shift;
+  } while (place >= n);
+  return place;
+}
+
 __global__ void center_sum_kernel(const float* __restrict__ centers, uint32_t n_lists, uint32_t dim, uint32_t dim_ext,
                                   float* __restrict__ sum)
 {
@@ -135,7 +154,8 @@ __device__ __forceinline__ float center_scale(const uint32_t* words, float& bn)
   return cp;
 }
 
-// One warp per list (of whole tiles: there is nothing in those beyond the last one but their norm terms).
+// One warp per place (of whole tiles: there is nothing in those beyond the last list but their norm terms).  Without `by_unit` the
+// lists are shuffled (list_at).
 __global__ void center_operand_kernel(const float* __restrict__ centers, uint32_t n_lists, uint32_t dim, uint32_t dim_ext,
                                       uint32_t width, float weight, const float* __restrict__ sum, uint32_t* __restrict__ words,
                                       float* __restrict__ norms, __half* __restrict__ out, __half* __restrict__ by_unit)
@@ -148,7 +168,7 @@ __global__ void center_operand_kernel(const float* __restrict__ centers, uint32_
   float bn, cc, dd;
   const float inv   = 1.0f / center_scale(words, bn);
   const float inv_n = 1.0f / float(n_lists);
-  const float* c    = centers + size_t(l) * dim_ext;
+  const float* c    = centers + size_t(by_unit != nullptr ? l : list_at(l, n_lists)) * dim_ext;
   double norm;
   list_norms(c, sum, inv_n, dim, weight, cc, dd, norm);
   __half* dst    = out + size_t(l) * width;
@@ -307,7 +327,7 @@ struct label_params {
   float* maxima;         // kMaxima: [n_rows, max_stride] largest value of every `unit` (8, 32, 64 or 128) lists
   uint32_t unit, max_stride;
   const float* threshold;  // kEmit: of the rows
-  uint32_t* found;         // [n_rows, 2 splits, found_cap] lists whose value reaches it
+  uint32_t* found;         // [n_rows, 2 splits, found_cap] places of the lists whose value reaches it
   uint32_t* n_found;       // [n_rows, 2 splits]
   uint32_t found_cap;
   uint32_t* error;
@@ -1201,7 +1221,7 @@ probe_threshold_kernel(const float* __restrict__ maxima, uint32_t n_units, uint3
 constexpr uint32_t kMaxSegments   = 64;
 constexpr uint32_t kChainCols     = 64;   // columns staged at a time
 
-// A warp per query: the lists found, 32 at a time through shared memory, one per lane with the defining chain (the next
+// A warp per query: the places found, whose lists go 32 at a time through shared memory, one per lane with the defining chain (the next
 // columns are on their way while some are used); a list's rank is the number of lists before it.
 // What bounds it: the shared-memory pipe, two thirds busy (8,000 queries x 128 probes x 96 dimensions: 135 us).  Bulk copies of a
 // lane's own row, 256 bytes each, took as long or longer (768 dimensions: 300 against 250 us).
@@ -1213,8 +1233,8 @@ __host__ __device__ __forceinline__ uint32_t probe_warp_bytes(uint32_t cap)
 }
 __global__ void __launch_bounds__(kProbeWarps * 32)
 probe_finish_kernel(const uint32_t* __restrict__ found, const uint32_t* __restrict__ n_found, uint32_t segments, uint32_t found_cap,
-                    const float* __restrict__ fq, const float* __restrict__ centers, uint32_t dim_ext, float alpha,
-                    uint32_t n_queries, uint32_t n_probes, uint32_t cap, const float* __restrict__ threshold,
+                    const float* __restrict__ fq, const float* __restrict__ centers, uint32_t n_lists, uint32_t dim_ext,
+                    float alpha, uint32_t n_queries, uint32_t n_probes, uint32_t cap, const float* __restrict__ threshold,
                     const uint32_t* __restrict__ error, uint32_t* __restrict__ timeouts, uint32_t* __restrict__ probes,
                     uint32_t* __restrict__ redo, uint32_t* __restrict__ n_redo)
 {
@@ -1266,7 +1286,7 @@ probe_finish_kernel(const uint32_t* __restrict__ found, const uint32_t* __restri
     uint32_t seg = 0;
 #pragma unroll
     for (uint32_t step = kMaxSegments / 2u; step > 0; step >>= 1) { seg += s_first[warp][seg + step] <= i ? step : 0u; }
-    s_list[i] = __ldg(found + (size_t(q) * segments + seg) * found_cap + (i - s_first[warp][seg]));
+    s_list[i] = list_at(__ldg(found + (size_t(q) * segments + seg) * found_cap + (i - s_first[warp][seg])), n_lists);
   }
   __syncwarp();
   // sixteen lanes per row; step: (32 lists, kChainCols columns)
@@ -1358,7 +1378,7 @@ probe_finish_kernel(const uint32_t* __restrict__ found, const uint32_t* __restri
 uint32_t probe_cap(uint32_t n_probes) { return round_up(2u * n_probes + 48u, 8u); }
 
 // Lists per unit: as many as leave six times as many units as wanted lists, so that the maxima select sharply (8% more lists
-// reach the threshold than are wanted); no fewer than a warp can hold the maxima of.
+// reach the threshold than are wanted, the lists of a unit being chosen at random: list_at); no fewer than a warp can hold the maxima of.
 uint32_t probe_unit(uint32_t n_lists, uint32_t n_probes)
 {
   for (uint32_t unit : {128u, 64u, 32u}) {
@@ -1492,7 +1512,7 @@ void select_probes_tc(raft::resources& res, const float* centers, const void* mo
   const size_t finish_smem = kProbeWarps * probe_warp_bytes(probe_cap(n_probes));
   ensure_dynamic_smem(reinterpret_cast<const void*>(probe_finish_kernel), finish_smem);
   launch_chained(probe_finish_kernel, ceildiv(n_queries, kProbeWarps), kProbeWarps * 32, finish_smem, stream, found, n_found,
-                 2u * y.splits, y.found_cap, fq, centers, dim_ext, alpha, n_queries, n_probes, probe_cap(n_probes), threshold, words,
+                 2u * y.splits, y.found_cap, fq, centers, n_lists, dim_ext, alpha, n_queries, n_probes, probe_cap(n_probes), threshold, words,
                  res.pinned + 13, probes, redo, words + 2);
   CUDA_TRY(cudaGetLastError());
   launch_probe_redo(res, redo, words, centers, fq, n_queries, n_lists, dim_ext, alpha, n_probes, reinterpret_cast<float*>(ws + y.o_scratch),

@@ -112,7 +112,7 @@ void exact_rows_product(raft::resources& res, const float* b, uint32_t n_cols, c
 // prepare_label_model fills from the centres; `workspace`: label_workspace_bytes.  Nothing synchronises.
 bool label_tc_usable(uint32_t n_rows, uint32_t n_lists);
 // `weight`: the factor of the rows' column `dim` in the score, negated (0.5 for L2 distances, 0 where the column does not count);
-// by_units: with what label_rows_tc needs (select_probes_tc does not).
+// by_units: for label_rows_tc; without: for select_probes_tc, which takes the lists in a shuffled order.
 size_t label_model_bytes(uint32_t n_lists, uint32_t dim, bool by_units);
 void prepare_label_model(cudaStream_t stream, const float* centers, uint32_t n_lists, uint32_t dim, uint32_t dim_ext, float weight,
                          bool by_units, void* model);

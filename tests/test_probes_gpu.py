@@ -65,6 +65,30 @@ def test_probes(mods, n_lists, n_q, dim, n_probes, metric):
     assert n <= n_q // 256                                         # ordinary data: the two passes settle it
 
 
+# lists in the order of their components, or of the branches of a tree: neighbours are alike
+@pytest.mark.parametrize("metric", ["sqeuclidean", "inner_product"])
+@pytest.mark.parametrize("n_lists,n_q,dim,n_probes", [(2048, 2000, 96, 20), (4000, 2000, 128, 64), (12288, 1000, 64, 128),
+                                                      (20000, 1000, 64, 20), (65536, 300, 32, 50)])
+@pytest.mark.parametrize("tree", [False, True])
+def test_the_order_of_the_lists_does_not_matter(mods, n_lists, n_q, dim, n_probes, metric, tree):
+    rng = np.random.default_rng(n_lists)
+    if tree:
+        centers, level = np.zeros((1, dim)), 1.0
+        while len(centers) < n_lists:
+            level *= 0.7
+            centers = np.repeat(centers, 8, 0)
+            centers = centers + level * rng.standard_normal(centers.shape)
+        centers = centers[:n_lists]
+    else:
+        component = np.sort(rng.integers(0, n_lists // 16, n_lists))
+        centers = rng.standard_normal((n_lists // 16, dim))[component] + 0.3 * rng.standard_normal((n_lists, dim))
+    q = centers[rng.integers(0, n_lists, n_q)] + 0.3 * np.abs(centers).mean() * rng.standard_normal((n_q, dim))
+    index = index_of(mods[0], centers.astype(np.float32), metric)
+    fast, exact, n = both(mods, index, torch.from_numpy(q.astype(np.float32)).cuda(), n_probes)
+    assert bool((fast == exact).all())
+    assert n <= n_q // 256
+
+
 def test_odd_queries_and_equal_lists(mods):
     """Queries without a bound (NaN, infinities, values at the ends of fp32, zeros) and lists that are equal or nearly so in numbers
     beyond what a query has room for."""
