@@ -11,6 +11,7 @@
 // select.  It is the general path (any n_probes up to 4096, any shape).
 #include "common.hpp"
 #include "packed.cuh"
+#include "row_select.cuh"
 #include "search_internal.hpp"
 #include "topk.cuh"
 
@@ -261,38 +262,7 @@ void launch_exact_gemm(const float* b, uint32_t n_cols, const float* a, uint32_t
   }
 }
 
-// Sorts the first n2 (a power of two) keys ascending; the whole block calls it after a barrier.
-__device__ __forceinline__ void block_sort_keys(uint64_t* keys, uint32_t n2)
-{
-  for (uint32_t size = 2; size <= n2; size <<= 1) {
-    for (uint32_t stride = size >> 1; stride > 0; stride >>= 1) {
-      for (uint32_t i = threadIdx.x; i < n2 / 2; i += blockDim.x) {
-        const uint32_t lo = 2 * i - (i & (stride - 1));
-        const uint32_t hi = lo + stride;
-        const bool up     = (lo & size) == 0;
-        const uint64_t a = keys[lo], b = keys[hi];
-        if ((a > b) == up) {
-          keys[lo] = b;
-          keys[hi] = a;
-        }
-      }
-      __syncthreads();
-    }
-  }
-}
-
-// One block per row: the exact `want` smallest (score, position), written in ascending order.  A row holds row_len scores,
-// or row_ends[(row + 1) * ends_stride - 1] of them; where that is less than `want` the rest of the result is empty
-// (score NaN).
-//
-// First way: every thread keeps the kTops smallest scores of its strided part of the row; at least `want` scores are at or
-// below the want-th smallest of the kThreads * kTops kept ones, and few others are (expected 1.2 `want` at 64 of 256,
-// 1.4 at 128; 1.1 at 1,000 of 1,024 x 2), so two reads of the row find them all: keys (score, position) into shared
-// memory, one sort.  A radix select reads the row five times, and its first histogram is one bucket's serial atomics
-// (scores share their exponent): 252 us against 111 us for 64 of 4,000 scores in 10,000 rows, 280 against 85 us for 1,000 of
-// 15,000 in 500 rows.
-// Second way (more ties at the threshold than the buffer holds): radix select on the order-preserving image of the score
-// (4 passes of 8 bits), one gather pass, then the sort.
+// One block per row.  A row holds row_len scores, or row_ends[(row + 1) * ends_stride - 1] of them.
 template <uint32_t kThreads, uint32_t kTops>
 __global__ void __launch_bounds__(kThreads)
 select_kernel(const float* __restrict__ scores, uint32_t row_stride, uint32_t row_len, const uint32_t* __restrict__ row_ends,
@@ -301,154 +271,19 @@ select_kernel(const float* __restrict__ scores, uint32_t row_stride, uint32_t ro
 {
   chain_begin();
   extern __shared__ uint64_t s_keys[];  // [cap]
-  __shared__ uint32_t s_hist[256];
-  __shared__ uint32_t s_prefix, s_remaining, s_count, s_eq_taken;
-  const uint32_t q   = blockIdx.x;
-  const float* row   = scores + size_t(q) * row_stride;
-  const uint32_t tid = threadIdx.x;
-  const uint32_t len = row_ends ? row_ends[size_t(q + 1) * ends_stride - 1] : row_len;
-  const uint32_t n4  = row_stride % 4 == 0 ? len / 4 : 0u;  // rows start on 16-byte boundaries
-  // every score of the row with its position
-  auto for_row = [&](auto&& fn) {
-    const float4* r4 = reinterpret_cast<const float4*>(row);
-#pragma unroll 4
-    for (uint32_t i = tid; i < n4; i += kThreads) {
-      const float4 v = __ldg(r4 + i);
-      fn(float_to_ordered(v.x), 4 * i);
-      fn(float_to_ordered(v.y), 4 * i + 1);
-      fn(float_to_ordered(v.z), 4 * i + 2);
-      fn(float_to_ordered(v.w), 4 * i + 3);
-    }
-#pragma unroll 4
-    for (uint32_t i = 4 * n4 + tid; i < len; i += kThreads) { fn(float_to_ordered(__ldg(row + i)), i); }
-  };
-
-  uint32_t n_sort = 0;
-  {
-    uint32_t best[kTops];
-#pragma unroll
-    for (uint32_t i = 0; i < kTops; i++) { best[i] = 0xFFFFFFFFu; }
-    for_row([&](uint32_t o, uint32_t) {
-#pragma unroll
-      for (uint32_t i = kTops - 1; i > 0; i--) { best[i] = min(best[i], max(best[i - 1], o)); }
-      best[0] = min(best[0], o);
-    });
-    // 24 bits of the want-th smallest of the kept scores, rounded up
-    uint32_t lo = 0;
-    for (int bit = 31; bit >= 8; bit--) {
-      const uint32_t c = lo | (1u << bit);
-      uint32_t n       = 0;
-#pragma unroll
-      for (uint32_t i = 0; i < kTops; i++) { n += uint32_t(__syncthreads_count(best[i] < c)); }
-      if (n < want) { lo = c; }
-    }
-    const uint32_t T = lo | 0xFFu;
-    if (tid == 0) { s_count = 0; }
-    __syncthreads();
-    if (best[0] <= T) {  // (a thread whose smallest score is above the threshold has nothing)
-      for_row([&](uint32_t o, uint32_t l) {
-        if (o <= T) {
-          const uint32_t slot = atomicAdd(&s_count, 1u);
-          if (slot < cap) { s_keys[slot] = (uint64_t(o) << 32) | l; }
-        }
-      });
-    }
-    __syncthreads();
-    const uint32_t n = s_count;
-    if (n <= cap) {
-      n_sort = 64;
-      while (n_sort < n || n_sort < want) { n_sort <<= 1; }
-      for (uint32_t i = n + tid; i < n_sort; i += kThreads) { s_keys[i] = kEmptyKey; }
-    }
-    __syncthreads();
-  }
-  if (n_sort == 0) {
-    n_sort = 64;
-    while (n_sort < want) { n_sort <<= 1; }
-    if (tid == 0) {
-      s_prefix    = 0;
-      s_remaining = want;
-    }
-    // radix select: after the passes s_prefix is the ordered image T of the want-th smallest score
-    for (int pass = 0; pass < 4; pass++) {
-      const int shift = 24 - 8 * pass;
-      if (tid < 256) { s_hist[tid] = 0; }
-      __syncthreads();
-      const uint32_t prefix = s_prefix;
-      const uint32_t mask   = pass == 0 ? 0u : (0xFFFFFFFFu << (shift + 8));
-      for_row([&](uint32_t o, uint32_t) {
-        if ((o & mask) == prefix) { atomicAdd(&s_hist[(o >> shift) & 0xFFu], 1u); }
-      });
-      __syncthreads();
-      if (tid < 32) {
-        uint32_t d, left;
-        find_digit(s_hist, s_remaining, d, left);
-        if (tid == 0) {
-          s_prefix    = prefix | (d << shift);
-          s_remaining = left;  // how many elements are wanted among those sharing the new prefix
-        }
-      }
-      __syncthreads();
-    }
-    const uint32_t T       = s_prefix;
-    const uint32_t want_eq = s_remaining;  // elements equal to T that belong to the selection
-    if (tid == 0) {
-      s_count    = 0;
-      s_eq_taken = 0;
-    }
-    for (uint32_t i = tid; i < n_sort; i += kThreads) { s_keys[i] = kEmptyKey; }
-    __syncthreads();
-    // gather: everything below T, plus the want_eq lowest positions equal to T
-    for (uint32_t base = 0; base < len; base += kThreads) {
-      const uint32_t l = base + tid;
-      uint32_t o       = 0xFFFFFFFFu;
-      if (l < len) { o = float_to_ordered(row[l]); }
-      if (l < len && o < T) { s_keys[atomicAdd(&s_count, 1u)] = (uint64_t(o) << 32) | l; }
-      // ties at T are taken in order: ballot keeps order inside a warp, warps take turns
-      const bool eq = l < len && o == T;
-      if (__syncthreads_or(eq)) {
-        for (uint32_t w = 0; w < kThreads / 32; w++) {
-          if ((tid >> 5) == w) {
-            const unsigned m = __ballot_sync(kFullMask, eq);
-            if (m) {
-              const uint32_t start = s_eq_taken;
-              const uint32_t rank  = start + __popc(m & ((1u << (tid & 31)) - 1u));
-              if (eq && rank < want_eq) { s_keys[atomicAdd(&s_count, 1u)] = (uint64_t(o) << 32) | l; }
-              __syncwarp();
-              if ((tid & 31) == 0) { s_eq_taken = start + __popc(m); }
-            }
-          }
-          __syncthreads();
-        }
-      }
-    }
-    __syncthreads();
-  }
-  if (n_sort == 64) {
-    if (tid < 32) {
-      uint64_t a0 = s_keys[tid], a1 = s_keys[tid + 32];
-      warp_sort64<uint64_t, false>(a0, a1);
-      s_keys[tid]      = a0;
-      s_keys[tid + 32] = a1;
-    }
-    __syncthreads();
-  } else {
-    block_sort_keys(s_keys, n_sort);
-  }
-  for (uint32_t p = tid; p < want; p += kThreads) {
-    const uint64_t key             = s_keys[p];
-    out_idx[size_t(q) * want + p] = uint32_t(key);
-    if (out_scores) { out_scores[size_t(q) * want + p] = ordered_to_float(uint32_t(key >> 32)); }
-  }
+  __shared__ select_mem s_mem;
+  const uint32_t q = blockIdx.x;
+  select_row<kThreads, kTops>(scores + size_t(q) * row_stride, row_ends ? row_ends[size_t(q + 1) * ends_stride - 1] : row_len,
+                              row_stride % 4 == 0, want, cap, s_keys, s_mem, [](auto* p) { return __ldg(p); },
+                              out_idx + size_t(q) * want, out_scores ? out_scores + size_t(q) * want : nullptr);
 }
 
 // Threads and scores kept per thread: `want` stays below two thirds of what the block keeps, where the scores taken beyond
-// the wanted ones are few; the buffer holds them with room to spare (a power of two, as the sort needs).
+// the wanted ones are few.
 void launch_select(const float* scores, uint32_t n_rows, uint32_t row_stride, uint32_t row_len, const uint32_t* row_ends,
                    uint32_t ends_stride, uint32_t want, uint32_t* out_idx, float* out_scores, cudaStream_t stream)
 {
-  uint32_t cap = 64;
-  while (cap < want + (want <= 1024 ? want / 2 : want / 4) || (want <= 160 && cap < 3 * want)) { cap <<= 1; }
+  const uint32_t cap = select_cap(want);
   auto go = [&](auto kernel, int threads) {
     const size_t smem = size_t(cap) * 8;
     if (smem > 48 * 1024) { ensure_dynamic_smem(reinterpret_cast<const void*>(kernel), smem); }

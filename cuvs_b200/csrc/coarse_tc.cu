@@ -34,6 +34,8 @@
 //      fails is queued.
 //   4. coarse_fallback_kernel: queued queries (rare) are redone exactly over all lists.
 #include "common.hpp"
+#include "packed.cuh"
+#include "row_select.cuh"
 #include "search_internal.hpp"
 #include "tc_ptx.cuh"
 #include "topk.cuh"
@@ -943,85 +945,159 @@ coarse_finish_small_kernel(const uint32_t* __restrict__ cand_key, const uint32_t
 // ------------------------------------------------------------------------------------------------
 // exact redo of flagged queries
 // ------------------------------------------------------------------------------------------------
-constexpr uint32_t kFbSlots = 64;  // queries redone per round = blocks of coarse_fallback_kernel = scratch rows
-constexpr uint32_t kFbGroup = 8;   // queries whose chains one thread carries at a time
+constexpr uint32_t kFbSlots  = 64;   // up to so many queries are scored by the whole grid, one block each selects
+constexpr uint32_t kFbMost   = 16;   // queries whose chains a thread carries at a time
+constexpr uint32_t kFbBlocks = 296;  // two per SM
 
-// Exact scores of the first kFbSlots queries to redo, spread over the whole grid: one block per 256
-// lists; 256 lists x 32 columns at a time go through shared memory (a warp reads 128 contiguous bytes
-// of one row), every thread continues the defining chain (ascending k, fused multiply-add) of its own
-// list for up to kFbGroup queries.  scratch[slot][list] = alpha * dot.
-__global__ void __launch_bounds__(256)
-coarse_fallback_scores_kernel(const uint32_t* __restrict__ redo_list, const uint32_t* __restrict__ redo_count,
-                              const float* __restrict__ centers, const float* __restrict__ fq,
-                              uint32_t n_queries, uint32_t n_lists, uint32_t dim_ext, float alpha,
-                              float* __restrict__ scratch, uint32_t n_slots,
-                              const uint32_t* __restrict__ error_word)
+// Rows of scores that the redo works in: a block takes `group` queries at a time.  Large groups read the centres less often (they
+// come from L2); all rows together stay within 256 MB, unless lists are so many that 64 rows are more.
+struct redo_plan {
+  uint32_t group, blocks;
+  redo_plan(uint32_t n_queries, uint32_t n_lists)
+  {
+    const uint32_t most = uint32_t(std::max<uint64_t>(kFbSlots, (256ull << 20) / (uint64_t(n_lists) * 4)));
+    const uint32_t rows = std::min({most, std::max(n_queries, kFbSlots), kFbBlocks * kFbMost});
+    group  = std::min(kFbMost, std::max(rows / kFbBlocks, std::min(4u, rows / kFbSlots)));
+    blocks = std::min(kFbBlocks, rows / group);
+  }
+  size_t bytes(uint32_t n_lists) const { return size_t(group) * blocks * n_lists * 4; }
+};
+
+// Exact scores of nj queries (at most 2 kPairs) with the lists from `from` to `to`, rows[j][list] = alpha * dot: 256 lists x 32
+// columns at a time through shared memory, the queries' columns beside them; a thread continues the defining chain (ascending k,
+// fused multiply-add) of its own list for all queries, two per instruction.
+constexpr uint32_t kFbPitch = kFbMost + 4u;  // floats of the queries per column: 16-byte aligned, stores spread over the banks
+template <uint32_t kPairs>
+__device__ __forceinline__ void score_group(const float* __restrict__ centers, const float* __restrict__ fq, const uint32_t* s_ids, uint32_t nj,
+                                            uint32_t from, uint32_t to, uint32_t n_lists, uint32_t dim_ext, float alpha, float* s_tile,
+                                            float* s_qs, float* rows)
 {
-  chain_begin();
-  extern __shared__ float s_f[];
-  float* s_tile = s_f;             // [256 lists][32 columns + 1]
-  float* s_qs   = s_f + 256 * 33;  // [kFbGroup][dim_ext]
-  const uint32_t tid    = threadIdx.x;
-  const bool redo_all   = *error_word != 0u;
-  const uint32_t n_redo = redo_all ? n_queries : min(*redo_count, n_queries);
-  const uint32_t R      = min(n_redo, n_slots);
-  const uint32_t l0     = blockIdx.x * 256u;
-  for (uint32_t j0 = 0; j0 < R; j0 += kFbGroup) {
-    const uint32_t nj = min(kFbGroup, R - j0);
-    __syncthreads();
-    for (uint32_t i = tid; i < nj * dim_ext; i += 256) {
-      const uint32_t j = i / dim_ext, k = i - j * dim_ext;
-      const uint32_t q = redo_all ? (j0 + j) : redo_list[j0 + j];
-      s_qs[i]          = fq[size_t(q) * dim_ext + k];
+  const uint32_t tid = threadIdx.x, n4 = dim_ext / 4u;
+  // this thread's parts of a tile (eight threads per list, 16 bytes each) and of the queries' columns, on their way while the
+  // tile before is used
+  float4 v[8];
+  float x[2];
+  auto load = [&](uint32_t l0, uint32_t k0) {
+    const uint32_t c4 = k0 / 4u + (tid & 7u);
+#pragma unroll
+    for (uint32_t i = 0; i < 8; i++) {
+      const uint32_t l = l0 + i * 32u + (tid >> 3);
+      if (l < to && c4 < n4) { v[i] = __ldg(reinterpret_cast<const float4*>(centers + size_t(l) * dim_ext) + c4); }
     }
-    float acc[kFbGroup];
 #pragma unroll
-    for (uint32_t j = 0; j < kFbGroup; j++) { acc[j] = 0.0f; }
-    for (uint32_t k0 = 0; k0 < dim_ext; k0 += 32) {
-      const uint32_t kc = min(32u, dim_ext - k0);
-      __syncthreads();
-      for (uint32_t r = tid >> 5; r < 256; r += 8) {
-        const uint32_t l = l0 + r, lane = tid & 31u;
-        if (l < n_lists && lane < kc) { s_tile[r * 33 + lane] = __ldg(centers + size_t(l) * dim_ext + k0 + lane); }
+    for (uint32_t i = 0; i < 2; i++) {
+      const uint32_t j = i * 8u + (tid >> 5), k = k0 + (tid & 31u);
+      if (j < 2u * kPairs) { x[i] = j < nj && k < dim_ext ? __ldg(fq + size_t(s_ids[j]) * dim_ext + k) : 0.0f; }
+    }
+  };
+  uint64_t acc[kPairs];
+#pragma unroll
+  for (uint32_t j = 0; j < kPairs; j++) { acc[j] = 0ull; }
+  load(from, 0);
+  for (uint32_t l0 = from, k0 = 0; l0 < to;) {
+    __syncthreads();
+#pragma unroll
+    for (uint32_t i = 0; i < 8; i++) {
+      float* at = s_tile + (i * 32u + (tid >> 3)) * 33u + (tid & 7u) * 4u;
+      at[0] = v[i].x; at[1] = v[i].y; at[2] = v[i].z; at[3] = v[i].w;
+    }
+#pragma unroll
+    for (uint32_t i = 0; i < 2; i++) {
+      const uint32_t j = i * 8u + (tid >> 5);
+      if (j < 2u * kPairs) { s_qs[(tid & 31u) * kFbPitch + j] = x[i]; }
+    }
+    __syncthreads();
+    const uint32_t kc = min(32u, dim_ext - k0);  // a multiple of 8
+    uint32_t next_l = l0, next_k = k0 + 32u;
+    if (next_k >= dim_ext) {
+      next_k = 0;
+      next_l += 256u;
+    }
+    if (next_l < to) { load(next_l, next_k); }
+#pragma unroll 8
+    for (uint32_t k = 0; k < kc; k++) {
+      const uint64_t c = dup2(s_tile[tid * 33u + k]);
+#pragma unroll
+      for (uint32_t j = 0; j < kPairs; j += 2) {
+        const ulonglong2 y = *reinterpret_cast<const ulonglong2*>(s_qs + k * kFbPitch + j * 2u);
+        acc[j]             = fma2(c, y.x, acc[j]);
+        acc[j + 1]         = fma2(c, y.y, acc[j + 1]);
       }
-      __syncthreads();
-      if (l0 + tid < n_lists) {
-        for (uint32_t k = 0; k < kc; k++) {
-          const float c = s_tile[tid * 33 + k];
+    }
+    if (next_k == 0u) {
+      if (l0 + tid < to) {
 #pragma unroll
-          for (uint32_t j = 0; j < kFbGroup; j++) {
-            if (j < nj) { acc[j] = __fmaf_rn(c, s_qs[j * dim_ext + k0 + k], acc[j]); }
-          }
+        for (uint32_t j = 0; j < kPairs; j++) {
+          if (2u * j < nj) { rows[size_t(2u * j) * n_lists + l0 + tid] = __fmul_rn(alpha, lo2(acc[j])); }
+          if (2u * j + 1u < nj) { rows[size_t(2u * j + 1u) * n_lists + l0 + tid] = __fmul_rn(alpha, hi2(acc[j])); }
         }
       }
-    }
-    if (l0 + tid < n_lists) {
 #pragma unroll
-      for (uint32_t j = 0; j < kFbGroup; j++) {
-        if (j < nj) { scratch[size_t(j0 + j) * n_lists + l0 + tid] = __fmul_rn(alpha, acc[j]); }
-      }
+      for (uint32_t j = 0; j < kPairs; j++) { acc[j] = 0ull; }
     }
+    l0 = next_l;
+    k0 = next_k;
+  }
+}
+__device__ __forceinline__ void score_group(const float* centers, const float* fq, const uint32_t* s_ids, uint32_t nj, uint32_t from, uint32_t to,
+                                            uint32_t n_lists, uint32_t dim_ext, float alpha, float* s_tile, float* s_qs, float* rows)
+{
+  if (nj <= 4u) {
+    score_group<2>(centers, fq, s_ids, nj, from, to, n_lists, dim_ext, alpha, s_tile, s_qs, rows);
+  } else {
+    score_group<8>(centers, fq, s_ids, nj, from, to, n_lists, dim_ext, alpha, s_tile, s_qs, rows);
   }
 }
 
-__global__ void __launch_bounds__(256)
+// Exact scores of up to kFbSlots queries to redo (where there are more, coarse_fallback_kernel scores them), spread over the
+// whole grid: a block per 256 lists.  20 queries x 1,024 lists x 128 dimensions: 200 us with scalar loads, none of them ahead of
+// its use, 21 us so.
+__global__ void __launch_bounds__(256, 2)
+coarse_fallback_scores_kernel(const uint32_t* __restrict__ redo_list, const uint32_t* __restrict__ redo_count,
+                              const float* __restrict__ centers, const float* __restrict__ fq,
+                              uint32_t n_queries, uint32_t n_lists, uint32_t dim_ext, float alpha,
+                              float* __restrict__ scratch, const uint32_t* __restrict__ error_word)
+{
+  chain_begin();
+  extern __shared__ float s_tile[];  // [256 lists][32 columns + 1]
+  __shared__ __align__(16) float s_qs[32 * kFbPitch];
+  __shared__ uint32_t s_ids[kFbSlots];
+  const bool redo_all   = *error_word != 0u;
+  const uint32_t n_redo = redo_all ? n_queries : min(*redo_count, n_queries), tid = threadIdx.x;
+  if (n_redo == 0 || n_redo > kFbSlots) { return; }
+  if (tid < n_redo) { s_ids[tid] = redo_all ? tid : redo_list[tid]; }
+  __syncthreads();
+  const uint32_t l0 = blockIdx.x * 256u, l1 = min(n_lists, l0 + 256u);
+  for (uint32_t j0 = 0; j0 < n_redo; j0 += kFbMost) {
+    score_group(centers, fq, s_ids + j0, min(kFbMost, n_redo - j0), l0, l1, n_lists, dim_ext, alpha, s_tile, s_qs,
+                scratch + size_t(j0) * n_lists);
+  }
+}
+
+// The probes of the queries to redo, selected from their rows of scores.  Up to kFbSlots of them: a block each, whose rows
+// coarse_fallback_scores_kernel has filled.  More (centres too close together for the bounds, or one far out that widens them; a
+// time-out): every block scores `group` queries at a time itself.  All of 10,000 queries x 4,000 lists x 128 dimensions: 19 ms
+// with a query per block and each thread on rows of its own, 0.9 so; 10,000 x 50,000 x 96: 210 and 14 ms.  What bounds it: the
+// latency of a tile's loads and barriers at two blocks per SM, and the selection.
+template <uint32_t kTops>
+__global__ void __launch_bounds__(256, 2)
 coarse_fallback_kernel(const uint32_t* __restrict__ redo_list, const uint32_t* __restrict__ redo_count,
                        const float* __restrict__ centers,
                        const float* __restrict__ fq, uint32_t n_queries, uint32_t n_lists,
-                       uint32_t dim_ext, float alpha, uint32_t n_probes, uint32_t cap,
-                       float* __restrict__ scratch /* [gridDim.x, n_lists] */,
+                       uint32_t dim_ext, float alpha, uint32_t n_probes, uint32_t cap, uint32_t most_group,
+                       float* scratch /* [gridDim.x * most_group, n_lists] */,
                        uint32_t* __restrict__ probes, float* __restrict__ scores_out,
                        uint32_t* __restrict__ words, volatile uint32_t* __restrict__ host_words, uint32_t host_seq,
                        unsigned long long* __restrict__ redone)
 {
   chain_begin();
   const uint32_t* error_word = words;
-  extern __shared__ uint64_t s_keys[];  // [cap], then the query
-  float* s_q = reinterpret_cast<float*>(s_keys + cap);
-  __shared__ uint32_t s_hist[256];
-  __shared__ uint32_t s_prefix, s_remaining, s_count, s_eq_taken;
+  extern __shared__ uint64_t s_keys[];  // [cap], then columns of 256 lists [256][33]
+  float* s_tile = reinterpret_cast<float*>(s_keys + cap);
+  __shared__ __align__(16) float s_qs[32 * kFbPitch];
+  __shared__ uint32_t s_ids[kFbMost];
+  __shared__ select_mem s_mem;
   const uint32_t tid = threadIdx.x;
-  float* row         = scratch + size_t(blockIdx.x) * n_lists;
   // after a time-out of the GEMM nothing it produced is trusted: all queries are redone here
   const bool redo_all   = *error_word != 0u;
   const uint32_t n_redo = redo_all ? n_queries : min(*redo_count, n_queries);
@@ -1038,97 +1114,23 @@ coarse_fallback_kernel(const uint32_t* __restrict__ redo_list, const uint32_t* _
       host_words[4] = host_seq;
     }
   }
-  for (uint32_t ri = blockIdx.x; ri < n_redo; ri += gridDim.x) {
-    const uint32_t q = redo_all ? ri : redo_list[ri];
-    for (uint32_t i = tid; i < dim_ext; i += 256) { s_q[i] = fq[size_t(q) * dim_ext + i]; }
+  const bool scored    = n_redo <= kFbSlots;
+  const uint32_t group = scored ? 1u : min(most_group, (n_redo + gridDim.x - 1u) / gridDim.x);
+  float* rows          = scratch + size_t(blockIdx.x) * (scored ? 1u : most_group) * n_lists;
+  for (uint32_t r0 = blockIdx.x * group; r0 < n_redo; r0 += gridDim.x * group) {
+    const uint32_t nj = min(group, n_redo - r0);
+    if (tid < nj) { s_ids[tid] = redo_all ? r0 + tid : redo_list[r0 + tid]; }
     __syncthreads();
-    // the first gridDim.x queries were scored by coarse_fallback_scores_kernel (row = slot); later
-    // rounds (many queries to redo: rare) score here, one chain per thread
-    if (ri >= gridDim.x) {
-      for (uint32_t l = tid; l < n_lists; l += 256) {
-        const float* c = centers + size_t(l) * dim_ext;
-        float acc      = 0.0f;
-        for (uint32_t k = 0; k < dim_ext; k++) { acc = __fmaf_rn(__ldg(c + k), s_q[k], acc); }
-        row[l] = __fmul_rn(alpha, acc);
-      }
-    }
-    if (tid == 0) {
-      s_prefix    = 0;
-      s_remaining = n_probes;
-    }
-    __syncthreads();
-    for (int pass = 0; pass < 4; pass++) {
-      const int shift = 24 - 8 * pass;
-      s_hist[tid]     = 0;
-      __syncthreads();
-      const uint32_t prefix = s_prefix;
-      const uint32_t mask   = pass == 0 ? 0u : (0xFFFFFFFFu << (shift + 8));
-      for (uint32_t l = tid; l < n_lists; l += 256) {
-        const uint32_t o = float_to_ordered(row[l]);
-        if ((o & mask) == prefix) { atomicAdd(&s_hist[(o >> shift) & 0xFFu], 1u); }
-      }
-      __syncthreads();
-      if (tid < 32) {
-        uint32_t d, left;
-        find_digit(s_hist, s_remaining, d, left);
-        if (tid == 0) {
-          s_prefix    = prefix | (d << shift);
-          s_remaining = left;
-        }
-      }
+    if (!scored) {
+      score_group(centers, fq, s_ids, nj, 0, n_lists, n_lists, dim_ext, alpha, s_tile, s_qs, rows);
       __syncthreads();
     }
-    const uint32_t T = s_prefix, want_eq = s_remaining;
-    if (tid == 0) {
-      s_count    = 0;
-      s_eq_taken = 0;
+    for (uint32_t j = 0; j < nj; j++) {
+      const size_t at = size_t(s_ids[j]) * n_probes;
+      select_row<256, kTops>(rows + size_t(j) * n_lists, n_lists, n_lists % 4u == 0u, n_probes, cap, s_keys, s_mem,
+                             [](auto* p) { return *p; }, probes + at, scores_out ? scores_out + at : nullptr);
+      __syncthreads();
     }
-    for (uint32_t i = tid; i < cap; i += 256) { s_keys[i] = kEmptyKey; }
-    __syncthreads();
-    for (uint32_t base = 0; base < n_lists; base += 256) {
-      const uint32_t l = base + tid;
-      uint32_t o       = 0xFFFFFFFFu;
-      if (l < n_lists) { o = float_to_ordered(row[l]); }
-      if (l < n_lists && o < T) { s_keys[atomicAdd(&s_count, 1u)] = (uint64_t(o) << 32) | l; }
-      const bool eq = l < n_lists && o == T;
-      if (__syncthreads_or(eq)) {
-        for (int w = 0; w < 8; w++) {
-          if (int(tid >> 5) == w) {
-            const unsigned m = __ballot_sync(kFullMask, eq);
-            if (m) {
-              const uint32_t start = s_eq_taken;
-              const uint32_t rank  = start + __popc(m & ((1u << (tid & 31)) - 1u));
-              if (eq && rank < want_eq) { s_keys[atomicAdd(&s_count, 1u)] = (uint64_t(o) << 32) | l; }
-              __syncwarp();
-              if ((tid & 31) == 0) { s_eq_taken = start + __popc(m); }
-            }
-          }
-          __syncthreads();
-        }
-      }
-    }
-    __syncthreads();
-    for (uint32_t size = 2; size <= cap; size <<= 1) {
-      for (uint32_t stride = size >> 1; stride > 0; stride >>= 1) {
-        for (uint32_t i = tid; i < cap / 2; i += 256) {
-          const uint32_t lo = 2 * i - (i & (stride - 1));
-          const uint32_t hi = lo + stride;
-          const bool up     = (lo & size) == 0;
-          const uint64_t a = s_keys[lo], b = s_keys[hi];
-          if ((a > b) == up) {
-            s_keys[lo] = b;
-            s_keys[hi] = a;
-          }
-        }
-        __syncthreads();
-      }
-    }
-    for (uint32_t pi = tid; pi < n_probes; pi += 256) {
-      const uint64_t key               = s_keys[pi];
-      probes[size_t(q) * n_probes + pi] = uint32_t(key);
-      if (scores_out) { scores_out[size_t(q) * n_probes + pi] = ordered_to_float(uint32_t(key >> 32)); }
-    }
-    __syncthreads();
   }
 }
 
@@ -1196,6 +1198,8 @@ void set_tc_wait_test(uint32_t spin_limit, uint32_t skip_kb)
   wait_limits_ref() = {spin_limit ? spin_limit : kSpinLimit, skip_kb};
 }
 
+size_t probe_redo_bytes(uint32_t n_queries, uint32_t n_lists) { return redo_plan(n_queries, n_lists).bytes(n_lists); }
+
 bool coarse_tc_usable(uint32_t n_lists, uint32_t n_probes, uint32_t dim_ext)
 {
   if (n_lists < 2048 || (dim_ext % 4) != 0) { return false; }
@@ -1218,7 +1222,7 @@ size_t coarse_tc_workspace_bytes(uint32_t n_queries, uint32_t n_lists, uint32_t 
   lay.add(size_t(n_queries) * n_tiles * 4 * 4);          // bound per 64-column unit
   lay.add(size_t(n_queries) * 4);            // queries to redo exactly
   lay.add(256);                              // error word, fallback counter, redo counter
-  lay.add(size_t(kFbSlots) * n_lists * 4);   // fallback scratch rows
+  lay.add(probe_redo_bytes(n_queries, n_lists));  // fallback scratch rows
   lay.add(size_t(n_queries) * 4);            // power-of-two scale of every query row
   return lay.total();
 }
@@ -1294,7 +1298,7 @@ void select_clusters_tc(raft::resources& res, const float* centers, const float*
   auto* cand_bnd  = reinterpret_cast<uint32_t*>(ws + lay.add(size_t(n_queries) * n_tiles * 4 * 4));
   auto* redo_list = reinterpret_cast<uint32_t*>(ws + lay.add(size_t(n_queries) * 4));
   auto* words     = reinterpret_cast<uint32_t*>(ws + lay.add(256));
-  float* scratch  = reinterpret_cast<float*>(ws + lay.add(size_t(kFbSlots) * n_lists * 4));
+  float* scratch  = reinterpret_cast<float*>(ws + lay.add(probe_redo_bytes(n_queries, n_lists)));
   float* row_scale = reinterpret_cast<float*>(ws + lay.add(size_t(n_queries) * 4));
   cudaStream_t stream = res.stream;
 
@@ -1399,28 +1403,36 @@ void select_clusters_tc(raft::resources& res, const float* centers, const float*
     res.tc_redo_pending  = true;
     res.tc_redo_seq++;
   }
-  launch_probe_redo(res, redo_list, words, centers, fq, n_queries, n_lists, dim_ext, alpha, n_probes, scratch, probes, scores_out,
-                    host_words, res.tc_redo_seq);
+  launch_probe_redo(res, redo_list, words, centers, fq, n_queries, n_queries, n_lists, dim_ext, alpha, n_probes, scratch, probes,
+                    scores_out, host_words, res.tc_redo_seq);
   res.launches += 3;
 }
 
-size_t probe_redo_bytes(uint32_t n_lists) { return size_t(kFbSlots) * n_lists * 4; }
-
 void launch_probe_redo(raft::resources& res, const uint32_t* redo_list, uint32_t* words, const float* centers, const float* fq,
-                       uint32_t n_queries, uint32_t n_lists, uint32_t dim_ext, float alpha, uint32_t n_probes, float* scratch,
-                       uint32_t* probes, float* scores_out, uint32_t* host_words, uint32_t host_seq)
+                       uint32_t n_queries, uint32_t max_queries, uint32_t n_lists, uint32_t dim_ext, float alpha,
+                       uint32_t n_probes, float* scratch, uint32_t* probes, float* scores_out, uint32_t* host_words, uint32_t host_seq)
 {
-  uint32_t cap_fb = 2;
-  while (cap_fb < n_probes) { cap_fb <<= 1; }
-  const size_t fb_smem = size_t(cap_fb) * 8 + size_t(dim_ext) * 4;
-  const size_t fs_smem = (size_t(256) * 33 + size_t(kFbGroup) * dim_ext) * 4;
+  const uint32_t cap_fb = select_cap(n_probes);
+  const redo_plan plan(max_queries, n_lists);
+  const size_t fb_smem = size_t(cap_fb) * 8 + size_t(256) * 33 * 4;
+  const size_t fs_smem = size_t(256) * 33 * 4;
   ensure_dynamic_smem(reinterpret_cast<const void*>(coarse_fallback_scores_kernel), fs_smem);
-  if (fb_smem > 48 * 1024) { ensure_dynamic_smem(reinterpret_cast<const void*>(coarse_fallback_kernel), fb_smem); }
   launch_chained(coarse_fallback_scores_kernel, ceildiv<uint32_t>(n_lists, 256u), 256, fs_smem, res.stream, redo_list,
-                 words + 2, centers, fq, n_queries, n_lists, dim_ext, alpha, scratch, kFbSlots, words);
-  launch_chained(coarse_fallback_kernel, kFbSlots, 256, fb_smem, res.stream, redo_list, words + 2, centers, fq, n_queries,
-                 n_lists, dim_ext, alpha, n_probes, cap_fb, scratch, probes, scores_out, words, host_words, host_seq,
-                 res.redo_counts + raft::resources::PROBES_REDONE);
+                 words + 2, centers, fq, n_queries, n_lists, dim_ext, alpha, scratch, words);
+  // (scores kept per thread: see select_row)
+  auto go = [&](auto kernel) {
+    ensure_dynamic_smem(reinterpret_cast<const void*>(kernel), fb_smem);
+    launch_chained(kernel, plan.blocks, 256, fb_smem, res.stream, redo_list, words + 2, centers, fq, n_queries, n_lists, dim_ext,
+                   alpha, n_probes, cap_fb, plan.group, scratch, probes, scores_out, words, host_words, host_seq,
+                   res.redo_counts + raft::resources::PROBES_REDONE);
+  };
+  if (n_probes <= 160) {
+    go(coarse_fallback_kernel<1>);
+  } else if (n_probes <= 384) {
+    go(coarse_fallback_kernel<2>);
+  } else {
+    go(coarse_fallback_kernel<8>);
+  }
   CUDA_TRY(cudaGetLastError());
   res.launches += 2;
 }

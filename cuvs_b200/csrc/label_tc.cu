@@ -1421,7 +1421,7 @@ struct probe_layout {
     o_n_found   = lay.add(size_t(n_queries) * splits * 2 * 4);
     o_redo      = lay.add(size_t(n_queries) * 4);
     o_words     = lay.add(256);
-    o_scratch   = lay.add(probe_redo_bytes(n_lists));
+    o_scratch   = lay.add(probe_redo_bytes(n_queries, n_lists));
     total       = lay.total();
   }
 };
@@ -1515,8 +1515,8 @@ void select_probes_tc(raft::resources& res, const float* centers, const void* mo
                  2u * y.splits, y.found_cap, fq, centers, n_lists, dim_ext, alpha, n_queries, n_probes, probe_cap(n_probes), threshold, words,
                  res.pinned + 13, probes, redo, words + 2);
   CUDA_TRY(cudaGetLastError());
-  launch_probe_redo(res, redo, words, centers, fq, n_queries, n_lists, dim_ext, alpha, n_probes, reinterpret_cast<float*>(ws + y.o_scratch),
-                    probes, nullptr, nullptr, 0);
+  launch_probe_redo(res, redo, words, centers, fq, n_queries, max_queries, n_lists, dim_ext, alpha, n_probes,
+                    reinterpret_cast<float*>(ws + y.o_scratch), probes, nullptr, nullptr, 0);
   res.launches += 5;
 }
 

@@ -130,10 +130,10 @@ void select_probes_tc(raft::resources& res, const float* centers, const void* mo
 
 // Queries redone exactly over all lists: redo_list[0 .. words[2]), or all of them where words[0], the error word, is set.  `words[1]`
 // receives their number; host_words (optional, pinned): {words[0], number, words[2], words[3], host_seq}.  `scratch`:
-// probe_redo_bytes.
-size_t probe_redo_bytes(uint32_t n_lists);
+// probe_redo_bytes for max_queries.
+size_t probe_redo_bytes(uint32_t n_queries, uint32_t n_lists);
 void launch_probe_redo(raft::resources& res, const uint32_t* redo_list, uint32_t* words, const float* centers, const float* fq,
-                       uint32_t n_queries, uint32_t n_lists, uint32_t dim_ext, float alpha, uint32_t n_probes, float* scratch,
-                       uint32_t* probes, float* scores_out, uint32_t* host_words, uint32_t host_seq);
+                       uint32_t n_queries, uint32_t max_queries, uint32_t n_lists, uint32_t dim_ext, float alpha,
+                       uint32_t n_probes, float* scratch, uint32_t* probes, float* scores_out, uint32_t* host_words, uint32_t host_seq);
 
 }  // namespace cuvs::neighbors::ivf_pq

@@ -35,12 +35,12 @@ def redone(mods, res):
     return counts[0]
 
 
-def both(mods, index, q, n_probes):
+def both(mods, index, q, n_probes, mode=0):
     """(probes as search selects them, probes of the exact product, queries that the former left to all lists)"""
     from cuvs_b200.common import Resources
     ivf, mg, L = mods
     lib, got, res = L.load(), [], Resources()
-    for mode in (0, 1):
+    for mode in (mode, 1):
         try:
             lib.cuvsB200SetCoarseMode(mode)
             got.append(mg.select_probes(index, q, n_probes, resources=res).to(torch.int64))
@@ -109,6 +109,59 @@ def test_odd_queries_and_equal_lists(mods):
         fine = torch.ones(len(q), dtype=torch.bool, device="cuda")
         fine[1] = fine[2] = False                                  # (NaN scores have no order)
         assert bool((fast == exact).all(1)[fine].all())
+
+
+# queries that many equal lists are nearest to, beyond what there is room for: as many as the whole grid scores, one more, and
+# many; the scores in rows of 16 and of fewer queries per block; both paths that leave queries to the redo
+@pytest.mark.parametrize("n_lists,n_q,dim,n_probes", [(1024, 9000, 40, 20), (4001, 3000, 102, 64), (100_000, 700, 30, 10)])
+@pytest.mark.parametrize("m", [1, 64, 65, 500, 0])
+def test_queries_redone(mods, n_lists, n_q, dim, n_probes, m):
+    rng = np.random.default_rng(m)
+    centers = make_mixture(n_lists, dim, 60, 0.4, 2)
+    centers[rng.permutation(n_lists)[:600]] = centers[8] + 1e-6 * rng.standard_normal((600, dim))
+    q = make_mixture(n_q, dim, 60, 0.4, 3)
+    m = m or n_q
+    q[rng.permutation(n_q)[:m]] = centers[8] + 1e-3 * rng.standard_normal((m, dim))
+    index = index_of(mods[0], centers.astype(np.float32), "sqeuclidean")
+    for mode in (0, 2) if n_lists > 50_000 else (0,):              # (2: shapes that path covers)
+        fast, exact, n = both(mods, index, torch.from_numpy(q.astype(np.float32)).cuda(), n_probes, mode)
+        assert bool((fast == exact).all())
+        assert m <= n <= m + n_q // 16, (mode, n)
+
+
+def test_redoing_a_whole_batch_costs_a_few_exact_products(mods):
+    """One centre at thirty times the others' length widens every query's bound: the whole batch is redone.  Measured: 49 times
+    the exact product with a thread per list and its centre row read by itself, 2 to 3 times through shared memory."""
+    from cuvs_b200.common import Resources
+    ivf, mg, L = mods
+    centers = make_mixture(4000, 128, 60, 0.4, 2)
+    ordinary = index_of(ivf, centers, "sqeuclidean")
+    centers[5] *= 30.0 * np.linalg.norm(centers, axis=1).mean() / np.linalg.norm(centers[5])
+    index = index_of(ivf, centers, "sqeuclidean")
+    q = torch.from_numpy(make_mixture(10_000, 128, 60, 0.4, 3)).cuda()
+
+    def timed(index, res):
+        a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+        torch.cuda.synchronize()
+        a.record()
+        mg.select_probes(index, q, 64, resources=res)
+        b.record()
+        torch.cuda.synchronize()
+        return a.elapsed_time(b)
+
+    redo, exact = [], []
+    for _ in range(3):
+        res = Resources()
+        timed(ordinary, res)                                       # (buffers)
+        redo.append(timed(index, res))
+        assert redone(mods, res) >= 9000
+        try:
+            L.load().cuvsB200SetCoarseMode(1)
+            timed(index, res)
+            exact.append(timed(index, res))
+        finally:
+            L.load().cuvsB200SetCoarseMode(0)
+    assert min(redo) < 8.0 * min(exact)
 
 
 # one product pass times out; every query is redone exactly and the handle counts the batch
