@@ -315,12 +315,16 @@ __global__ void unpack_labels_kernel(const unsigned long long* __restrict__ best
   labels[r]        = uint32_t(best[r]);
 }
 
+// Most queries of a chunk: its scores stay around 64 MB, so that the select passes read them from L2.
+uint64_t most_queries(uint32_t n_lists)
+{
+  const uint64_t target = 64ull << 20;
+  return std::max<uint64_t>(kTile, target / (uint64_t(n_lists) * 4)) / kTile * kTile;
+}
+
 uint32_t chunk_queries(uint32_t n_queries, uint32_t n_lists)
 {
-  // keep one chunk of scores around 64 MB so that the select passes read it from L2
-  const uint64_t target = 64ull << 20;
-  uint64_t c            = std::max<uint64_t>(kTile, target / (uint64_t(n_lists) * 4));
-  c                     = (c / kTile) * kTile;
+  const uint64_t c = most_queries(n_lists);
   // equal chunks: a short last one would be a nearly empty wave
   const uint32_t n = uint32_t(ceildiv<uint64_t>(n_queries, c));
   return round_up<uint32_t>(ceildiv(n_queries, n), kTile);
@@ -331,7 +335,9 @@ uint32_t chunk_queries(uint32_t n_queries, uint32_t n_lists)
 size_t coarse_workspace_bytes(uint32_t n_queries, uint32_t n_lists, uint32_t n_probes)
 {
   (void)n_probes;
-  return size_t(chunk_queries(n_queries, n_lists)) * n_lists * 4;
+  // (enough for fewer queries too, whose chunks may be larger: two of 8,192 for 16,384 queries x 1,100 lists, one of 12,032
+  // for 12,000)
+  return size_t(std::min<uint64_t>(round_up(n_queries, kTile), most_queries(n_lists))) * n_lists * 4;
 }
 
 void select_clusters(raft::resources& res, const float* centers, uint32_t n_lists, uint32_t dim_ext,

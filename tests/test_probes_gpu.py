@@ -89,6 +89,16 @@ def test_the_order_of_the_lists_does_not_matter(mods, n_lists, n_q, dim, n_probe
     assert n <= n_q // 256
 
 
+def test_a_last_batch_with_larger_chunks(mods):
+    """The exact product of 12,000 queries takes one chunk, that of the 16,384 before them two smaller ones, in one workspace."""
+    ivf, mg, _ = mods
+    index = index_of(ivf, make_mixture(1100, 16, 60, 0.4, 2), "sqeuclidean")
+    q = torch.from_numpy(make_mixture(16_384 + 12_000, 16, 60, 0.4, 3)).cuda()
+    got = mg.select_probes(index, q, 300)                          # (more probes than the two product passes take)
+    assert bool((got[:16_384].to(torch.int64) == mg.select_probes(index, q[:16_384], 300).to(torch.int64)).all())
+    assert bool((got[16_384:].to(torch.int64) == mg.select_probes(index, q[16_384:], 300).to(torch.int64)).all())
+
+
 def test_odd_queries_and_equal_lists(mods):
     """Queries without a bound (NaN, infinities, values at the ends of fp32, zeros) and lists that are equal or nearly so in numbers
     beyond what a query has room for."""
