@@ -1394,15 +1394,7 @@ void select_clusters_tc(raft::resources& res, const float* centers, const float*
   }
   // the error word and how many queries this batch redid exactly: written to pinned memory by the kernel, looked at
   // before a later batch and at the handle's next synchronisation
-  uint32_t* host_words = nullptr;
-  if (!res.tc_redo_pending) {
-    host_words           = res.pinned + 8;
-    res.tc_redo_queries  = n_queries;
-    res.tc_redo_n_probes = n_probes;
-    res.tc_redo_adapts   = !exact_operands && tc_products_ref() == 0;
-    res.tc_redo_pending  = true;
-    res.tc_redo_seq++;
-  }
+  uint32_t* host_words = res.tc_redo_record(n_queries, n_probes, 0, !exact_operands && tc_products_ref() == 0);
   launch_probe_redo(res, redo_list, words, centers, fq, n_queries, n_queries, n_lists, dim_ext, alpha, n_probes, scratch, probes,
                     scores_out, host_words, res.tc_redo_seq);
   res.launches += 3;

@@ -1515,8 +1515,10 @@ void select_probes_tc(raft::resources& res, const float* centers, const void* mo
                  2u * y.splits, y.found_cap, fq, centers, n_lists, dim_ext, alpha, n_queries, n_probes, probe_cap(n_probes), threshold, words,
                  res.pinned + 13, probes, redo, words + 2);
   CUDA_TRY(cudaGetLastError());
+  // how many: looked at before a later batch, which may then go to the exact product
+  uint32_t* host_words = res.tc_redo_record(n_queries, n_probes, n_lists, true);
   launch_probe_redo(res, redo, words, centers, fq, n_queries, max_queries, n_lists, dim_ext, alpha, n_probes,
-                    reinterpret_cast<float*>(ws + y.o_scratch), probes, nullptr, nullptr, 0);
+                    reinterpret_cast<float*>(ws + y.o_scratch), probes, nullptr, host_words, res.tc_redo_seq);
   res.launches += 5;
 }
 

@@ -85,7 +85,18 @@ void resources::adopt_tc_verdict()
   if (!tc_redo_pending || *static_cast<volatile uint32_t*>(pinned + 12) != tc_redo_seq) { return; }
   std::atomic_thread_fence(std::memory_order_acquire);
   tc_redo_pending = false;
-  if (pinned[8] != 0u) {
+  if (tc_redo_n_lists != 0u) {
+    // (a time-out, which the kernels count, says nothing about the bounds)
+    if (pinned[8] == 0u && tc_redo_adapts) {
+      probe_level& lv = probe_levels[{tc_redo_n_lists, tc_redo_n_probes}];
+      if (uint64_t(pinned[9]) * 16 > tc_redo_queries) {
+        lv.rest      = lv.next_rest;
+        lv.next_rest = std::min(2 * lv.next_rest, 1024u);
+      } else {
+        lv.next_rest = 16;
+      }
+    }
+  } else if (pinned[8] != 0u) {
     // the coarse GEMM of that batch gave up on a bounded wait; its probes were all recomputed exactly
     tc_timeouts++;
   } else if (tc_redo_adapts) {
@@ -100,6 +111,28 @@ void resources::adopt_tc_verdict()
       lv.products--;
     }
   }
+}
+
+bool resources::probes_by_passes(uint32_t n_lists, uint32_t n_probes)
+{
+  adopt_tc_verdict();
+  if (probe_levels.size() > 4096) { probe_levels.clear(); }
+  const auto at = probe_levels.find({n_lists, n_probes});
+  if (at == probe_levels.end() || at->second.rest == 0u) { return true; }
+  at->second.rest--;
+  return false;
+}
+
+uint32_t* resources::tc_redo_record(uint32_t n_queries, uint32_t n_probes, uint32_t n_lists, bool adapts)
+{
+  if (tc_redo_pending) { return nullptr; }
+  tc_redo_queries  = n_queries;
+  tc_redo_n_probes = n_probes;
+  tc_redo_n_lists  = n_lists;
+  tc_redo_adapts   = adapts;
+  tc_redo_pending  = true;
+  tc_redo_seq++;
+  return pinned + 8;
 }
 
 void resources::sync()

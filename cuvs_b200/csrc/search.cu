@@ -956,15 +956,16 @@ void search_any(raft::resources& res, const search_params& params, const index<i
   const size_t o_all     = lay.add(store_all ? size_t(batch) * max_samples * 4 : 0);
   // half-precision scores tie in large groups, which the tensor-core path's guard (made for fp32
   // scores) does not settle: the fp16 coarse search runs on the exact SIMT path
-  // large batches: no score matrix; else the other tensor-core path or the exact product
-  const bool use_probes_tc =
-    !coarse_h && !coarse_i8 && coarse_mode() == 0 && probes_tc_usable(batch, n_lists, n_probes, idx.dim());
-  const bool use_tc = !coarse_h && coarse_mode() != 1 && coarse_tc_usable(n_lists, n_probes, cdim_ext);
+  // large batches: no score matrix, or the exact product where that left too many queries to the redo (the workspace holds
+  // either, so that a handle that changes over allocates nothing); else the other tensor-core path or the exact product
+  const bool large  = !given_probes && !coarse_h && !coarse_i8 && coarse_mode() == 0 && probes_tc_usable(batch, n_lists, n_probes, idx.dim());
+  const bool use_probes_tc = large && res.probes_by_passes(n_lists, n_probes);
+  const bool use_tc = !large && !coarse_h && coarse_mode() != 1 && coarse_tc_usable(n_lists, n_probes, cdim_ext);
   const size_t coarse_ws =
-    given_probes    ? 0
-    : use_probes_tc ? probes_workspace_bytes(res, batch, n_lists, n_probes, idx.dim())
-    : use_tc        ? coarse_tc_workspace_bytes(batch, n_lists, cdim_ext)
-                    : coarse_workspace_bytes(batch, n_lists, n_probes);
+    given_probes ? 0
+    : large      ? std::max(probes_workspace_bytes(res, batch, n_lists, n_probes, idx.dim()), coarse_workspace_bytes(batch, n_lists, n_probes))
+    : use_tc     ? coarse_tc_workspace_bytes(batch, n_lists, cdim_ext)
+                 : coarse_workspace_bytes(batch, n_lists, n_probes);
   const size_t o_coarse  = lay.add(coarse_ws);
   // tables in global memory: one per CTA of the (smaller) grid of that variant
   const uint32_t glut_grid = uint32_t(std::min<size_t>(n_pairs_max, size_t(res.sm_count) * 4));
@@ -1335,16 +1336,17 @@ void select_probes_any(raft::resources& res, const index<int64_t>& idx, const vo
   if (coarse_i8) { op8 = idx.int8_coarse_operands(res.stream); }
   index<int64_t>::half_operands oph{};
   if (coarse_h) { oph = idx.half_coarse_operands(res.stream); }
-  const bool use_tc = !coarse_h && coarse_mode() != 1 && coarse_tc_usable(n_lists, n_probes, cdim_ext);
   const uint32_t batch = std::min<uint32_t>(n_queries, 16384);
-  const bool use_probes_tc =
-    !coarse_h && !coarse_i8 && coarse_mode() == 0 && probes_tc_usable(batch, n_lists, n_probes, idx.dim());
+  const bool large  = !coarse_h && !coarse_i8 && coarse_mode() == 0 && probes_tc_usable(batch, n_lists, n_probes, idx.dim());
+  const bool use_probes_tc = large && res.probes_by_passes(n_lists, n_probes);
+  const bool use_tc = !large && !coarse_h && coarse_mode() != 1 && coarse_tc_usable(n_lists, n_probes, cdim_ext);
   ws_layout lay;
   const size_t o_fq = lay.add(size_t(batch) * cdim_ext * 4);
   const size_t o_rq = lay.add(size_t(batch) * idx.rot_dim() * 4);
-  const size_t cws  = use_probes_tc ? probes_workspace_bytes(res, batch, n_lists, n_probes, idx.dim())
-                      : use_tc      ? coarse_tc_workspace_bytes(batch, n_lists, cdim_ext)
-                                    : coarse_workspace_bytes(batch, n_lists, n_probes);
+  const size_t cws =
+    large    ? std::max(probes_workspace_bytes(res, batch, n_lists, n_probes, idx.dim()), coarse_workspace_bytes(batch, n_lists, n_probes))
+    : use_tc ? coarse_tc_workspace_bytes(batch, n_lists, cdim_ext)
+             : coarse_workspace_bytes(batch, n_lists, n_probes);
   const size_t o_c  = lay.add(cws);
   res.ws.reserve(lay.total());
   char* ws   = res.ws.base();

@@ -171,6 +171,23 @@ struct resources {
     int floor    = 1;  // raised when a level produced too many exact redos
   };
   std::map<uint32_t, tc_level> tc_levels;
+  // Probes of large batches by two product passes (label_tc.cu) are worth it while few queries are left to the redo over all
+  // lists, which depends on the centres (one far out, groups closer together than the bound) and on the queries.  A batch that
+  // left more than a sixteenth of its queries sends the next calls with as many lists and probes to the exact product, whose
+  // time does not depend on the data: 16 calls, then one more try, after another such batch 32 calls and so on up to 1,024.
+  // (The line: 10,000 queries, the passes / redoing all / the exact product in us: 1,024 lists x 20 probes 99 / 400 / 150, 4,000 x
+  // 64 196 / 900 / 385, 20,000 x 20 166 / 3,600 / 1,285, 50,000 x 20 271 / 13,900 / 3,375; 2,000 queries of 768 dimensions, 4,096 x 100
+  // 262 / 2,400 / 358.)
+  struct probe_level {
+    uint32_t rest      = 0;   // calls that go to the exact product before the next try
+    uint32_t next_rest = 16;
+  };
+  std::map<std::pair<uint32_t, uint32_t>, probe_level> probe_levels;  // by (lists, probes); at most a few thousand
+  bool probes_by_passes(uint32_t n_lists, uint32_t n_probes);         // how a call selects its probes
+  // The pinned words for a batch's counters, or nullptr while another batch's are in flight.  n_lists: 0 for the tensor-core
+  // coarse stage, whose level `adapts`; else a batch of two product passes.
+  uint32_t* tc_redo_record(uint32_t n_queries, uint32_t n_probes, uint32_t n_lists, bool adapts);
+  uint32_t tc_redo_n_lists   = 0;
   uint32_t tc_redo_n_probes  = 0;  // n_probes of the batch whose counters are in flight
   uint32_t tc_redo_seq       = 0;
   bool tc_redo_pending       = false;

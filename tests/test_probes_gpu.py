@@ -219,3 +219,37 @@ def test_a_model_is_complete_on_return(mods, per_cluster):
     torch.cuda.synchronize()
     L.check(L.load().cuvsIvfPqBuildPrecomputed(res.handle, params._p, C.c_uint32(dim), *[r.ref() for r in refs], index._h))
     assert stream.query()
+
+
+def test_a_handle_leaves_the_passes_where_they_do_not_pay(mods):
+    """A batch that left more than a sixteenth of its queries to the redo sends the next calls of that shape to the exact product;
+    other shapes stay, and after a while the passes are tried again."""
+    from cuvs_b200.common import Resources
+    ivf, mg, _ = mods
+    centers = make_mixture(2048, 64, 60, 0.4, 2)
+    ordinary = index_of(ivf, centers, "sqeuclidean")
+    far = centers.copy()
+    far[5] *= 30.0 * np.linalg.norm(centers, axis=1).mean() / np.linalg.norm(far[5])
+    index = index_of(ivf, far, "sqeuclidean")
+    q = torch.from_numpy(make_mixture(2000, 64, 60, 0.4, 3)).cuda()
+    res = Resources()
+
+    def run(index, n_probes=20):
+        before = redone(mods, res)                                 # (synchronises: the last batch's counters have arrived)
+        out = mg.select_probes(index, q, n_probes, resources=res).to(torch.int64)
+        return out, redone(mods, res) - before
+
+    first, n = run(index)
+    assert n > len(q) // 4
+    for _ in range(16):
+        out, n = run(index)
+        assert n == 0 and bool((out == first).all())
+    assert run(ordinary, 30)[1] <= len(q) // 256                   # (another shape takes the passes)
+    assert run(index)[1] > len(q) // 4                             # the next try
+    for _ in range(32):
+        assert run(index)[1] == 0
+    assert run(ordinary)[1] <= len(q) // 256                       # a try that succeeds
+    assert run(index)[1] > len(q) // 4
+    for _ in range(16):
+        assert run(index)[1] == 0
+    assert run(index)[1] > len(q) // 4
