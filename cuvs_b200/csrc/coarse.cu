@@ -35,7 +35,7 @@ constexpr uint32_t kMaxProbes = 4096;
 // 64 and 128 distinct bytes; the next eight k are on their way while eight are used.
 // 10,000 x 4,000 x 136: 487 us with 64 x 64 outputs per block and scalar FMAs, 238 us so.  kVec: rows of both operands are
 // 16-byte aligned and k is a multiple of four.  kListed: the rows of `a` (and of `best`) named by row_list, *n_listed of them.
-constexpr uint32_t kTile = 128, kTileK = 8;
+constexpr uint32_t kTile = 128, kTileK = 8, kListedBlocks = 2368;
 template <bool kVec, bool kArgmin, bool kListed>
 __global__ void __launch_bounds__(256, 2)
 exact_gemm_kernel(const float* __restrict__ b, uint32_t n_cols, const float* __restrict__ a, uint32_t n_rows, uint32_t a_stride,
@@ -45,43 +45,58 @@ exact_gemm_kernel(const float* __restrict__ b, uint32_t n_cols, const float* __r
   chain_begin();
   __shared__ __align__(16) float s_a[2][kTileK][kTile + 4];
   __shared__ __align__(16) float s_b[2][kTileK][kTile + 4];
-  const uint32_t j0 = blockIdx.x * kTile;
   const uint32_t tid = threadIdx.x;
   const uint32_t tx = ((tid >> 5) & 1u) * 8u + (tid & 7u), ty = (tid >> 6) * 4u + ((tid >> 3) & 3u);
   if constexpr (kListed) { n_rows = min(n_rows, __ldg(n_listed)); }
-  // (listed rows: the blocks take the tiles in turn, since the host does not know how many there are; else each has one)
-  uint32_t i0 = blockIdx.y * kTile;
-  if (kListed && i0 >= n_rows) { return; }
-  do {
-    // one row and four k of either operand per thread
-    const uint32_t lrow = tid >> 1, lk = (tid & 1u) * 4u;
-    const bool in_a = i0 + lrow < n_rows, in_b = j0 + lrow < n_cols;
-    const float* pa = a + size_t(kListed && in_a ? __ldg(row_list + i0 + lrow) : i0 + lrow) * a_stride + lk;
-    const float* pb = b + size_t(j0 + lrow) * kdim + lk;
-    float ra[4], rb[4];
-    auto load = [&](uint32_t k0) {
-      if constexpr (kVec) {
-        const float4 z = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        const float4 x = in_a && k0 + lk < kdim ? __ldg(reinterpret_cast<const float4*>(pa + k0)) : z;
-        const float4 y = in_b && k0 + lk < kdim ? __ldg(reinterpret_cast<const float4*>(pb + k0)) : z;
-        ra[0] = x.x; ra[1] = x.y; ra[2] = x.z; ra[3] = x.w;
-        rb[0] = y.x; rb[1] = y.y; rb[2] = y.z; rb[3] = y.w;
-      } else {
-#pragma unroll
-        for (uint32_t e = 0; e < 4; e++) {
-          const bool in = k0 + lk + e < kdim;
-          ra[e]         = in && in_a ? __ldg(pa + k0 + e) : 0.0f;
-          rb[e]         = in && in_b ? __ldg(pb + k0 + e) : 0.0f;
-        }
-      }
-    };
-    auto store = [&](uint32_t buf) {
+  // (listed rows: sixteen blocks per SM take the tiles in turn, since the host does not know how many there are; else each
+  // block has one)
+  uint32_t j0 = blockIdx.x * kTile, i0 = blockIdx.y * kTile, tile = blockIdx.x;
+  [[maybe_unused]] const uint32_t across = (n_cols + kTile - 1u) / kTile;
+  auto place = [&] {
+    j0 = tile % across * kTile;
+    i0 = tile / across * kTile;
+  };
+  if constexpr (kListed) {
+    place();
+    if (i0 >= n_rows) { return; }
+  }
+  // one row and four k of either operand per thread
+  const uint32_t lrow = tid >> 1, lk = (tid & 1u) * 4u;
+  bool in_a, in_b;
+  const float *pa, *pb;
+  float ra[4], rb[4];
+  auto rows_of_tile = [&] {
+    in_a = i0 + lrow < n_rows;
+    in_b = j0 + lrow < n_cols;
+    pa   = a + size_t(kListed && in_a ? __ldg(row_list + i0 + lrow) : i0 + lrow) * a_stride + lk;
+    pb   = b + size_t(j0 + lrow) * kdim + lk;
+  };
+  rows_of_tile();
+  auto load = [&](uint32_t k0) {
+    if constexpr (kVec) {
+      const float4 z = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+      const float4 x = in_a && k0 + lk < kdim ? __ldg(reinterpret_cast<const float4*>(pa + k0)) : z;
+      const float4 y = in_b && k0 + lk < kdim ? __ldg(reinterpret_cast<const float4*>(pb + k0)) : z;
+      ra[0] = x.x; ra[1] = x.y; ra[2] = x.z; ra[3] = x.w;
+      rb[0] = y.x; rb[1] = y.y; rb[2] = y.z; rb[3] = y.w;
+    } else {
 #pragma unroll
       for (uint32_t e = 0; e < 4; e++) {
-        s_a[buf][lk + e][lrow] = ra[e];
-        s_b[buf][lk + e][lrow] = rb[e];
+        const bool in = k0 + lk + e < kdim;
+        ra[e]         = in && in_a ? __ldg(pa + k0 + e) : 0.0f;
+        rb[e]         = in && in_b ? __ldg(pb + k0 + e) : 0.0f;
       }
-    };
+    }
+  };
+  auto store = [&](uint32_t buf) {
+#pragma unroll
+    for (uint32_t e = 0; e < 4; e++) {
+      s_a[buf][lk + e][lrow] = ra[e];
+      s_b[buf][lk + e][lrow] = rb[e];
+    }
+  };
+  load(0);
+  do {
     // rows ty * 4 + {0..3} and 64 + ..., columns tx * 4 + {0..3} and 64 + ...
     uint64_t acc[8][4];
 #pragma unroll
@@ -89,7 +104,6 @@ exact_gemm_kernel(const float* __restrict__ b, uint32_t n_cols, const float* __r
 #pragma unroll
       for (int j = 0; j < 4; j++) { acc[i][j] = 0ull; }
     }
-    load(0);
     store(0);
     __syncthreads();
     uint32_t buf = 0;
@@ -123,13 +137,23 @@ exact_gemm_kernel(const float* __restrict__ b, uint32_t n_cols, const float* __r
         __syncthreads();
       }
     }
+    [[maybe_unused]] const uint32_t row0 = i0, col0 = j0;
+    if constexpr (kListed) {
+      // the next tile's first columns are on their way while this one's results are handed over
+      tile += gridDim.x;
+      place();
+      if (i0 < n_rows) {
+        rows_of_tile();
+        load(0);
+      }
+    }
 #pragma unroll
     for (int i = 0; i < 8; i++) {
-      const uint32_t row = i0 + (i < 4 ? ty * 4u + i : 64u + ty * 4u + (i - 4));
+      const uint32_t row = row0 + (i < 4 ? ty * 4u + i : 64u + ty * 4u + (i - 4));
       [[maybe_unused]] unsigned long long m = ~0ull;
 #pragma unroll
       for (int h = 0; h < 2; h++) {
-        const uint32_t col = j0 + h * 64u + tx * 4u;
+        const uint32_t col = col0 + h * 64u + tx * 4u;
         float v[4];
 #pragma unroll
         for (int e = 0; e < 4; e++) {
@@ -166,10 +190,7 @@ exact_gemm_kernel(const float* __restrict__ b, uint32_t n_cols, const float* __r
         if ((tid & 7u) == 0 && row < n_rows) { atomicMin(best + (kListed ? __ldg(row_list + row) : row), m); }
       }
     }
-    if constexpr (kListed) {
-      __syncthreads();
-      i0 += gridDim.y * kTile;
-    }
+    if constexpr (kListed) { __syncthreads(); }
   } while (kListed && i0 < n_rows);
 }
 
@@ -244,8 +265,10 @@ void launch_exact_gemm(const float* b, uint32_t n_cols, const float* a, uint32_t
   for (uint32_t r0 = 0; r0 < n_rows; r0 += most) {
     const uint32_t nr = std::min(most, n_rows - r0);
     dim3 grid(ceildiv(n_cols, kTile), ceildiv(nr, kTile));
-    // some eight blocks per SM: 4,096 x 128 blocks that found nothing to do took 0.6 ms
-    if (kListed) { grid.y = std::min(grid.y, ceildiv(1184u, grid.x)); }
+    // A block per tile: 4,096 x 128 blocks that find nothing to do take 0.6 ms, these 3 us.  As many as are resident run out
+    // unevenly, and so did some eight per SM whose last wave was a sixth full.  100,000 rows labelled against 50,000 lists,
+    // all redone: 25.5 ms with a block per tile, 27.1 with 1,564 blocks, 26.4 with 296, 25.6 with 1,184, 25.35 so, 25.1 with 9,472.
+    if (kListed) { grid = dim3(uint32_t(std::min<uint64_t>(uint64_t(grid.x) * grid.y, kListedBlocks))); }
     const float* ar = a + size_t(r0) * a_stride;
     float* o        = out ? out + size_t(r0) * n_cols : nullptr;
     unsigned long long* bs = best ? best + r0 : nullptr;
