@@ -1360,15 +1360,31 @@ probe_finish_kernel(const uint32_t* __restrict__ found, const uint32_t* __restri
     }
   }
   __syncwarp();
-  // lists of equal score met at one place: then the order is by (score, list)
+  // Lists of equal score met at one place: then the order is by (score, list).  For each of them the warp counts the lists of
+  // equal score before it.  (Among 350 scores of fp32 two are often equal, and more so where all are large.  When every lane
+  // ranked its lists anew by both: 4,000 queries x 4,096 lists x 256 probes, 512 against 214 us for a whole selection; with centres
+  // around a common offset of ten times their spread, 1,193 against 248.)
+  constexpr uint32_t kMet = 1u << 31;
   bool tied = false;
   for (uint32_t c = lane; c < n; c += 32u) { tied = tied || s_place[s_rank[c]] != c; }
   if (__any_sync(kFullMask, tied)) {
     for (uint32_t c = lane; c < n; c += 32u) {
-      const uint32_t score = s_score[c], list = s_list[c];
-      uint32_t rank        = 0;
-      for (uint32_t o = 0; o < n; o++) { rank += s_score[o] < score || (s_score[o] == score && s_list[o] < list) ? 1u : 0u; }
-      if (rank < n_probes) { probes[size_t(q) * n_probes + rank] = list; }
+      if ((s_place[s_rank[c]] & ~kMet) != c) { atomicOr(s_place + s_rank[c], kMet); }
+    }
+    __syncwarp();
+    for (uint32_t c0 = 0; c0 < n; c0 += 32u) {
+      const uint32_t c = c0 + lane;
+      const bool met   = c < n && (s_place[s_rank[c]] & kMet) != 0u;
+      uint32_t rank    = c < n ? s_rank[c] : n_probes;
+      for (unsigned left = __ballot_sync(kFullMask, met); left != 0u; left &= left - 1u) {
+        const uint32_t one   = uint32_t(__ffs(int(left))) - 1u;
+        const uint32_t score = s_score[c0 + one], list = s_list[c0 + one];
+        uint32_t before      = 0;
+        for (uint32_t o = lane; o < n; o += 32u) { before += s_score[o] == score && s_list[o] < list ? 1u : 0u; }
+        before = __reduce_add_sync(kFullMask, before);
+        if (lane == one) { rank += before; }
+      }
+      if (rank < n_probes) { probes[size_t(q) * n_probes + rank] = s_list[c]; }
     }
     return;
   }

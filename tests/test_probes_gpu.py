@@ -89,6 +89,18 @@ def test_the_order_of_the_lists_does_not_matter(mods, n_lists, n_q, dim, n_probe
     assert n <= n_q // 256
 
 
+# small integers: most lists have the score of several others; two, or many of them, across the last probe
+@pytest.mark.parametrize("n_lists,n_q,dim,n_probes,top", [(2048, 1100, 16, 40, 16), (4096, 600, 30, 200, 9), (20000, 150, 12, 33, 8)])
+@pytest.mark.parametrize("metric", ["sqeuclidean", "inner_product"])
+def test_equal_scores(mods, n_lists, n_q, dim, n_probes, top, metric):
+    rng = np.random.default_rng(top)
+    centers, q = rng.integers(0, top, (n_lists, dim)), rng.integers(0, top, (n_q, dim))
+    index = index_of(mods[0], centers.astype(np.float32), metric)
+    fast, exact, n = both(mods, index, torch.from_numpy(q.astype(np.float32)).cuda(), n_probes)
+    assert bool((fast == exact).all())
+    assert n < n_q // 2                                            # (what is tested is the order of those ranked at once)
+
+
 def test_a_last_batch_with_larger_chunks(mods):
     """The exact product of 12,000 queries takes one chunk, that of the 16,384 before them two smaller ones, in one workspace."""
     ivf, mg, _ = mods
