@@ -1477,7 +1477,6 @@ void make_rotation(uint32_t rot_dim, uint32_t dim, bool force_random, std::vecto
   }
 }
 
-// Scratch of launch_encode for up to n vectors: byte codes, and with a rotation the differences before and after it.
 // Whether n vectors are encoded through tables of cells: where making those costs less than they save.  256 codewords, 96
 // dimensions, making + encoding / comparing all (us): one component 36 + 24 / 67 at 20,000 rows, 40 + 137 / 468 at 200,000; two
 // 51 + 17 / 70 and 55 + 83 / 449; three 158 + 69 / 159 at 60,000, 149 + 167 / 450 at 200,000; four 640 + 187 / 449 at 200,000.
@@ -1491,6 +1490,9 @@ size_t code_table_bytes(const index<int64_t>& idx)
 {
   return idx.pq_dim() * with_cell_len(idx.pq_len(), [](auto len) { return sizeof(code_table<decltype(len)::value>); });
 }
+// Scratch of launch_encode for up to n vectors: the tables of cells, at an offset that does not depend on n (the chunks of a call
+// after the first find them there, so nothing may write them in between), byte codes, and with a rotation the differences before
+// and after it.
 size_t encode_scratch_bytes(const index<int64_t>& idx, uint64_t n, bool cells)
 {
   if (idx.codebook_kind() == codebook_gen::PER_CLUSTER) { return 0; }
