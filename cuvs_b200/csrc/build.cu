@@ -1477,14 +1477,22 @@ void make_rotation(uint32_t rot_dim, uint32_t dim, bool force_random, std::vecto
   }
 }
 
-// Whether n vectors are encoded through tables of cells: where making those costs less than they save.  256 codewords, 96
-// dimensions, making + encoding / comparing all (us): one component 36 + 24 / 67 at 20,000 rows, 40 + 137 / 468 at 200,000; two
-// 51 + 17 / 70 and 55 + 83 / 449; three 158 + 69 / 159 at 60,000, 149 + 167 / 450 at 200,000; four 640 + 187 / 449 at 200,000.
+// Whether n vectors are encoded through tables of cells: where making those costs less than they save.  What a vector saves grows with
+// the subspaces, and so does the making of the tables beyond what a handful of them takes; few codewords (7 bits) leave less to save:
+// the two sides meet at some a + b / pq_dim vectors.  Whole calls of `transform` by comparing all / through tables (us), 256 codewords:
+// 64 subspaces of one component 112 / 107 at 24,576 vectors, 163 / 125 at 49,152; of two 166 / 154 and 261 / 196; of three 437 / 481 at
+// 65,536, 786 / 614 at 131,072; of four 998 / 1,310 at 131,072, 1,929 / 1,541 at 262,144; 16 subspaces of two 95 / 96 and, unit vectors,
+// 93 / 114 at 24,576, 128 / 113 at 40,000; 8 of four 331 / 467 at 262,144, 610 / 560 at 524,288; 2 of two 85 / 90 at 98,304.  128
+// codewords, 64 subspaces of two: 135 / 146 at 24,576, 202 / 182 at 49,152.
 bool encode_by_cells(const index<int64_t>& idx, uint64_t n)
 {
-  const uint32_t len = idx.pq_len();
-  if (idx.codebook_kind() != codebook_gen::PER_SUBSPACE || len > 4 || idx.pq_bits() < 7) { return false; }
-  return n >= (len <= 2 ? 24'576u : (len == 3 ? 131'072u : 393'216u));
+  const uint32_t len = idx.pq_len(), bits = idx.pq_bits();
+  if (idx.codebook_kind() != codebook_gen::PER_SUBSPACE || len > 4 || bits < 7) { return false; }
+  constexpr uint32_t kFixed[2][4] = {{25'000, 22'000, 100'000, 170'000}, {12'000, 14'000, 60'000, 175'000}};
+  constexpr uint32_t kShared[2][4] = {{1'000'000, 800'000, 1'500'000, 2'300'000}, {200'000, 250'000, 1'300'000, 2'600'000}};
+  // (four to eight subspaces leave the comparison of all too few blocks)
+  if (bits == 8 && len <= 2 && idx.pq_dim() >= 4 && idx.pq_dim() <= 8) { return n >= 24'576; }
+  return n >= kFixed[bits - 7][len - 1] + kShared[bits - 7][len - 1] / idx.pq_dim();
 }
 size_t code_table_bytes(const index<int64_t>& idx)
 {

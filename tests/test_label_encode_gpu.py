@@ -126,6 +126,42 @@ def test_codes_by_cells(ivf, length, n, bits, rotated):
         assert bool((few == codes[r0:r0 + 20000]).all())
 
 
+# at the number of rows from which the tables are used, which depends on the number of subspaces, and one row below it: against fewer
+# rows at a time, bit for bit (subspaces that do not fill the last block of either encoder)
+@pytest.mark.parametrize("length,bits,pq_dim,n", [(1, 8, 37, 17_405), (1, 7, 64, 40_625), (2, 8, 65, 17_846), (2, 7, 24, 55_333),
+                                                  (3, 8, 33, 99_393), (3, 7, 40, 137_500), (4, 8, 41, 238_414), (4, 7, 72, 201_944),
+                                                  (2, 8, 1, 264_000), (2, 8, 8, 24_576), (4, 8, 3, 1_041_666)])
+def test_where_tables_of_cells_begin(ivf, length, bits, pq_dim, n):
+    rng = np.random.default_rng(n)
+    dim, n_lists, book = pq_dim * length, 20, 1 << bits
+    books = (rng.standard_normal((pq_dim, length, book)) * np.exp(rng.uniform(-2, 1, (pq_dim, 1, 1)))).astype(np.float32)
+    centers = rng.standard_normal((n_lists, dim)).astype(np.float32)
+    to = lambda a: torch.from_numpy(np.ascontiguousarray(a, dtype=np.float32)).cuda()  # noqa: E731
+    index = ivf.build_precomputed(ivf.IndexParams(n_lists=n_lists, pq_dim=pq_dim, pq_bits=bits), dim, to(books), to(centers),
+                                  to(centers), to(np.eye(dim)))
+    x = to(centers)[torch.from_numpy(rng.integers(0, n_lists, n)).cuda()]
+    x = x + torch.randn(n, dim, generator=torch.Generator(device="cuda").manual_seed(n), device="cuda")
+    from cuvs_b200 import _lib as L
+    from cuvs_b200.common import Resources
+    res, launches, stats = Resources(), [0], L.SearchStats()
+
+    def transform(rows):
+        out = ivf.transform(index, rows, resources=res)
+        L.check(L.load().cuvsB200StatsGet(res.handle, C.byref(stats), False))
+        launches.append(stats.launches)
+        return out
+
+    labels_below, codes_below = transform(x[:n - 1])
+    labels, codes = transform(x)
+    # (the tables are made by one kernel more)
+    assert launches[2] - launches[1] == launches[1] + 1
+    assert bool((labels_below == labels[:n - 1]).all()) and bool((codes_below == codes[:n - 1]).all())
+    for r0 in range(0, n, 12_000):
+        few_labels, few = ivf.transform(index, x[r0:r0 + 12_000])
+        assert bool((few_labels == labels[r0:r0 + 12_000]).all())
+        assert bool((few == codes[r0:r0 + 12_000]).all())
+
+
 # one and several K blocks: row tile resident, and streamed beside the lists
 @pytest.mark.parametrize("n,dim,n_lists", [(20000, 62, 1000), (17000, 300, 1100), (17000, 768, 1100)])
 def test_a_wait_that_runs_out_redoes_every_label(ivf, n, dim, n_lists):
