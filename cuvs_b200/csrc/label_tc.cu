@@ -1444,14 +1444,25 @@ struct probe_layout {
 
 }  // namespace
 
-// From 2 M (query, list) pairs on.  A whole call with 20 probes, by coarse_tc.cu or the exact product / so (us): 500 x 2,048 95 / 95,
-// 1,000 x 2,048 117 / 117, 2,000 x 1,024 145 / 145, 500 x 4,096 112 / 112, 1,000 x 4,096 146 / 122, 200 x 10,000 110 / 105, 500 x
-// 10,000 121 / 107, 4,000 x 10,000 378 / 214.
+// From 2 M (query, list) pairs on, and more where a query has many probes for the lists: what the passes save grows with the pairs, what
+// they cost beside with the probes (the finish) and where the maxima select less sharply.  Whole calls, 96 dimensions, by coarse_tc.cu or
+// the exact product / so (us):
+// - 20 probes: 1,000 x 4,096 146 / 122, 500 x 10,000 121 / 107, 4,000 x 10,000 378 / 214;
+// - 1,000 lists: 32 probes, 2,200 queries 153 / 161, 4,500 231 / 231, 9,000 378 / 353; 48 probes 175 / 187, 274 / 280, 462 / 444;
+// - 2,048 lists: 64 probes, 1,074 queries 157 / 165, 2,197 220 / 215; 128 probes, 4,394 502 / 518, 8,789 914 / 910, 19,531 1,943 / 1,910;
+// - 4,096 lists: 128 probes, 1,098 queries 244 / 261, 2,197 351 / 345, 4,394 581 / 536; 256 probes, 2,197 511 / 558, 9,765 1,858 / 1,880
+//   (512 dimensions: 1,100 queries 706 / 851, 4,400 2,112 / 2,329);
+// - 8,192 lists: 256 probes, 549 queries 268 / 289, 1,098 425 / 444, 2,197 614 / 590; 16,384 lists: 549 288 / 297, 1,098 545 / 480.
+// Beyond 16,384 lists, few queries are a matter of latency, where coarse_tc.cu has fewer steps, but not with many probes of many lists:
+// 110 x 20,000, 20 probes 58 / 64, 100 probes 134 / 142, 300 queries, 20 probes 102 / 100; 100 x 32,768, 10 probes 49 / 59, 32 probes 64 /
+// 75, 64 probes 135 / 132; 256 queries, 10 probes 61 / 68, 700 queries 140 / 130.
 bool probes_tc_usable(uint32_t n_queries, uint32_t n_lists, uint32_t n_probes, uint32_t dim)
 {
   const uint32_t unit = probe_unit(n_lists, n_probes);
+  const double share  = double(n_probes) / n_lists;
   return n_lists >= 256 && n_lists <= 131072 && n_probes <= 256 && n_lists / unit >= 2 * n_probes && dim <= 4096 &&
-         uint64_t(n_queries) * n_lists >= (1ull << 21);
+         uint64_t(n_queries) * n_lists >= (1ull << 21) && n_queries >= 2.5e6 * share * share &&
+         (n_lists <= 16384 || (n_lists < 32768 ? n_queries > 128 : n_queries > 256 || n_probes >= 64));
 }
 
 size_t probes_workspace_bytes(const raft::resources& res, uint32_t n_queries, uint32_t n_lists, uint32_t n_probes, uint32_t dim)

@@ -65,6 +65,20 @@ def test_probes(mods, n_lists, n_q, dim, n_probes, metric):
     assert n <= n_q // 256                                         # ordinary data: the two passes settle it
 
 
+# the fewest queries that go through the two passes (by probes and lists, by pairs, beyond 16,384 lists by queries), and one less
+@pytest.mark.parametrize("metric", ["sqeuclidean", "inner_product"])
+@pytest.mark.parametrize("n_lists,n_q,dim,n_probes", [(513, 9728, 30, 32), (1000, 9000, 40, 60), (4001, 2559, 96, 128), (4096, 9766, 24, 256),
+                                                      (9000, 1235, 130, 200), (16384, 257, 66, 160), (20000, 129, 32, 30), (40000, 257, 32, 63), (32768, 64, 62, 64),
+                                                      (40000, 64, 98, 200), (1000, 2098, 20, 5)])
+def test_where_the_two_passes_begin(mods, n_lists, n_q, dim, n_probes, metric):
+    index = index_of(mods[0], make_mixture(n_lists, dim, 60, 0.4, 2), metric)
+    q = torch.from_numpy(make_mixture(n_q, dim, 60, 0.4, 3)).cuda()
+    fast, exact, n = both(mods, index, q, n_probes)
+    assert bool((fast == exact).all()) and n <= n_q // 256
+    below, exact, _ = both(mods, index, q[:n_q - 1], n_probes)     # (the other path's guard is wider: it redoes more)
+    assert bool((below == exact).all()) and bool((below == fast[:n_q - 1]).all())
+
+
 # lists in the order of their components, or of the branches of a tree: neighbours are alike
 @pytest.mark.parametrize("metric", ["sqeuclidean", "inner_product"])
 @pytest.mark.parametrize("n_lists,n_q,dim,n_probes", [(2048, 2000, 96, 20), (4000, 2000, 128, 64), (12288, 1000, 64, 128),
