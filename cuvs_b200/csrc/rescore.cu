@@ -724,15 +724,9 @@ void launch_rescore(const rescore_params& p, int lut_kind, bool out_half, bool i
         shape_home(lut, oh, ip, std::false_type{}, codes);
       }
     };
-    // (tight bounds always come with row codes)
-    if constexpr (decltype(lut)::value == LUT_FP8 || decltype(oh)::value) {
-      if (p.row_codes == nullptr) {
-        home(std::false_type{});
-      } else {
-        home(std::true_type{});
-      }
+    if (p.row_codes == nullptr) {
+      home(std::false_type{});
     } else {
-      CUVS_EXPECTS(p.row_codes != nullptr, "two-step search: no row codes");
       home(std::true_type{});
     }
   };

@@ -828,6 +828,33 @@ static void set_error_model(rescore_params& rp, const operand_params& fp, int lu
   }
 }
 
+// Whether the first of the two steps writes codes of the rows beside the units' bounds: where the rows that these spare the exact
+// scores cost more than the codes.  The codes cost arithmetic per tile of (128 pairs x 256 rows) and 16 bytes per query and 32 rows: some
+// 20 us for 1 M rows in lists that few queries share, 90 for 256 M (query, row) pairs.  What they spare grows with k and with the
+// components of a row, more so with 8-bit tables, whose bounds leave several times as many rows, and where the codebook is read through
+// L2; with few queries a second round of scores per query is all there is to spare.
+// Whole calls without / with them (us), 1 M rows, 96 dimensions, 48 x 8 bits, half-precision tables: 5,000 queries x 20 probes of 4,000
+// lists k 1 201 / 219, k 10 238 / 232, k 24 307 / 270, k 64 436 / 342; 1,000 queries k 10 143 / 160, k 40 164 / 169, k 64 192 / 184;
+// 3,000 x 64 of 2,000 k 10 279 / 300, k 24 305 / 306, k 64 420 / 353; 2 M rows, 4,000 x 128 of 4,000 k 10 604 / 702, k 64 760 / 761.
+// 128 dimensions, 64 x 8, 8-bit tables: 5,000 x 20 k 1 333 / 308, k 10 605 / 436; 1,000 x 20 k 1 182 / 198, k 10 207 / 204; 2 M rows, 4,000
+// x 128 k 10 814 / 835, k 24 893 / 841; half sums: 10,000 x 20 k 10 354 / 332, 2,000 x 64 k 10 271 / 292, k 64 361 / 316.
+// Codebook in L2 (100 dimensions, 96 x 8): 5,000 x 20 k 1 360 / 352, k 10 490 / 390; 1,000 x 20 k 10 308 / 327.
+// The estimate below (times in us, fitted to 420 such points) takes 0.3% longer than the better side on average, 10% at worst; codes with
+// narrow bounds or k > 64 and none else: 7% and 76%.
+bool row_codes_pay(const index<int64_t>& idx, int lut_kind, uint32_t k, uint32_t n_probes, uint32_t n_queries, bool book_at_hand)
+{
+  const double q = n_queries, n = double(idx.size()), pairs = q * n_probes * n / idx.n_lists();  // (query, row) pairs
+  const double cost = 18e-6 * std::max(std::min(n, pairs), pairs / 128) + 1e-7 * pairs;
+  double gain       = 0.0;  // ns per query and 96 components
+  if (lut_kind == LUT_FP8) {
+    gain = 4.0 + 0.75 * k;
+  } else {
+    gain = 0.4 * std::max(int(k) - 10, 0) + 0.1 * std::min(k, 10u) * (n_queries >= 4096 ? 4.5 : (n_queries >= 1536 ? 2.0 : 0.0)) +
+           (!book_at_hand && n_queries >= 1536 ? 10.0 : 0.0);
+  }
+  return gain * 1e-3 * q * idx.rot_dim() / 96.0 >= cost;
+}
+
 void search_any(raft::resources& res, const search_params& params, const index<int64_t>& idx,
                 const void* queries, elem_t qtype, uint32_t n_queries, uint32_t k,
                 int64_t* neighbors, float* distances, const uint32_t* given_probes, bitset_view filter)
@@ -898,16 +925,18 @@ void search_any(raft::resources& res, const search_params& params, const index<i
                                                    (idx.pq_bits() == 4 && idx.pq_len() == 2));
   const bool never       = (lut_kind == LUT_FP8 && !(straight && idx.pq_bits() == 8)) || (out_half && !straight && n_probes < 2 * k);
   const uint64_t enough  = straight && !wide_bounds ? 4096 : 16384;
-  // Codes of the rows beside the units' bounds leave the exact scores a sixth to a half of the rows and cost the first step 3 to 15%.
-  // Whole calls without / with them (us): half-precision tables, k 20, 10,000 queries x 50,000 lists 1,190 / 1,187; fp32 tables
-  // whose codebook exceeds shared memory, k 10 612 / 509; 4-bit inner product, k 10 1,094 / 1,074; 8-bit tables, k 100 3,115 / 2,734.
-  // With wide bounds and few neighbours the scores are too few to pay: 8-bit tables, k 10 1,143 / 1,190; half sums, k 10 247 / 269.
-  const bool row_codes = !wide_bounds || k > 64;
+  bool row_codes = false;
   // (a list-sharded search exchanges bounds in the middle of the look-up-table scan: a collective, so that all its ranks
   // take that path)
   const int home = scan_codebook_home();
   if (!res.scan_phase_hook && !store_all && (home == 4 || (home == 0 && !never && uint64_t(batch) * n_probes > enough))) {
-    fplan = plan_filter(res, idx, lut_kind, out_half, is_ip, k, n_probes, batch, row_codes);
+    fplan = plan_filter(res, idx, lut_kind, out_half, is_ip, k, n_probes, batch, false);
+    if (fplan.use && row_codes_pay(idx, lut_kind, k, n_probes, batch, fplan.book_bytes != 0)) {
+      const filter_plan with = plan_filter(res, idx, lut_kind, out_half, is_ip, k, n_probes, batch, true);
+      // (their buffer does not drive the codebook out of shared memory)
+      row_codes = with.use && (with.book_bytes != 0) == (fplan.book_bytes != 0);
+      if (row_codes) { fplan = with; }
+    }
     // the bounds (with the row codes), and the query operand of one internal batch: within 2 (3) and 2 GiB
     const uint64_t fits_bounds  = row_codes ? (3ull << 30) / (uint64_t(max_groups) * 32) : (1ull << 31) / (uint64_t(max_groups) * 16);
     const uint64_t fits_operand = (1ull << 31) / (uint64_t(n_probes) * f_chunks * 16);

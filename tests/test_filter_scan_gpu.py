@@ -256,3 +256,21 @@ def test_row_codes_leave_what_the_tables_find(ivf, metric, lut, k, dim, pq_dim, 
     finally:
         L.check(L.load().cuvsB200SetScanCodebookHome(0))
     assert (i0 == i2).all() and (d0.view(np.uint32) == d2.view(np.uint32)).all()
+
+
+# few neighbours (no row codes) and more (with them), narrow and wide bounds, every straight-line shape, the general loop, and a codebook that
+# exceeds shared memory; against the tables bit for bit
+@pytest.mark.parametrize("metric,lut,internal", [("sqeuclidean", "f32", "f32"), ("sqeuclidean", "f16", "f32"), ("sqeuclidean", "f16", "f16"),
+                                                 ("sqeuclidean", "fp8", "f32"), ("inner_product", "f16", "f32"), ("cosine", "f32", "f32")])
+@pytest.mark.parametrize("dim,pq_dim,bits", [(96, 48, 8), (64, 16, 8), (64, 32, 4), (81, 27, 8), (56, 40, 5), (200, 100, 8)])
+def test_with_and_without_row_codes(ivf, metric, lut, internal, dim, pq_dim, bits):
+    from cuvs_b200 import _lib as L
+    x = make_mixture(60_001, dim, 60, 0.3, seed=dim)
+    q = make_mixture(900, dim, 60, 0.3, seed=dim + 1)
+    g = ivf.build(ivf.IndexParams(n_lists=150, pq_dim=pq_dim, pq_bits=bits, metric=metric, kmeans_n_iters=3), torch.from_numpy(x).cuda())
+    for k in (1, 9, 40):
+        L.check(L.load().cuvsB200SetScanCodebookHome(4))
+        d2, i2 = gpu_search(ivf, g, q, k, 20, lut, internal)
+        L.check(L.load().cuvsB200SetScanCodebookHome(2))
+        d0, i0 = gpu_search(ivf, g, q, k, 20, lut, internal)
+        assert (i0 == i2).all() and (d0.view(np.uint32) == d2.view(np.uint32)).all()
