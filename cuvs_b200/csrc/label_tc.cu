@@ -1223,7 +1223,8 @@ constexpr uint32_t kChainCols     = 64;   // columns staged at a time
 
 // A warp per query: the places found, whose lists go 32 at a time through shared memory, one per lane with the defining chain (the next
 // columns are on their way while some are used); a list's rank is the number of lists before it.
-// What bounds it: the shared-memory pipe, two thirds busy (8,000 queries x 128 probes x 96 dimensions: 135 us).  Bulk copies of a
+// What bounds it: L1, which the centres' rows and shared memory share, 69% busy (8,000 queries x 128 probes x 96 dimensions: 123 us; 86% for
+// 2,000 x 100 x 768: 181), and the latency of shared memory, whose four or five blocks per SM are few warps.  Bulk copies of a
 // lane's own row, 256 bytes each, took as long or longer (768 dimensions: 300 against 250 us).
 constexpr uint32_t kProbeWarps = 4, kChainPitch = kChainCols + 4u;
 // (a cap that is a multiple of eight, fourteen bytes each: the next warp's rows start on 16)
