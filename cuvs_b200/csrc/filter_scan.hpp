@@ -83,7 +83,7 @@ struct rescore_params {
   int cosine, metric;
   float post_scale;
   // error model (see rescore.cu)
-  float e1, kappa, e0, delta_lo, delta_hi, eta, sum_limit, rmax, ip_gemm, ip_lut;
+  float e1, kappa, e0, e2, delta_lo, delta_hi, eta, sum_limit, rmax, ip_gemm, ip_lut;
   // step of the row codes: L2 |d|^2 row_step, inner product row_step over the query's scale (less what rounding may do)
   float row_step;
   int sharpen;    // wide bounds: score what is certainly wanted first

@@ -4,8 +4,9 @@
 // Bounds.  A unit (eight rows of a list) carries the smallest approximate score v of its rows.  With m >= |d| + |r|
 // (L2; d the difference to the list centre, r a row's decoded residual) the score that the reference's
 // arithmetic gives a row with approximation v lies in [lo(v), hi(v)]:
-//   sqrt(t) in [sqrt(v - kappa m^2) - e1 m - e0, sqrt(v + kappa m^2) + e1 m + e0]   (t: the real distance)
-//       e1: operands rounded to half precision; kappa: fp32 accumulation; e0: half-precision underflow
+//   sqrt(t) in [sqrt(v - w) - e1 m - e0, sqrt(v + w) + e1 m + e0], w = kappa m^2 + e2   (t: the real distance)
+//       e1: operands rounded to half precision; kappa: fp32 accumulation; e0, e2: half-precision underflow of components and of |r|^2
+//       (rows far shorter than the longest, whose |r|^2 sets the scale)
 //   lo = t_lo (1 - delta_lo) - eta,  hi = t_hi (1 + delta_hi) + eta
 //       delta, eta: what rounding table entries and partial sums does to a sum of non-negative terms
 // and for inner products t is within ip_gemm |q| rmax of v, the score within ip_lut |q| (rmax + |c|) + eta of t.
@@ -60,7 +61,7 @@ __device__ __forceinline__ float unit_lo(const rescore_params& p, float v, float
     if (norm < 0.0f && p.saturates) { return -INFINITY; }
     const float vp = fmaxf(v, 0.0f);
     const float m  = 2.0f * fabsf(norm) + sqrt_approx(vp);
-    const float a  = fmaxf(sqrt_approx(fmaxf(vp - p.kappa * m * m, 0.0f)) - __fmaf_rn(p.e1, m, p.e0), 0.0f);
+    const float a  = fmaxf(sqrt_approx(fmaxf(vp - __fmaf_rn(p.kappa * m, m, p.e2), 0.0f)) - __fmaf_rn(p.e1, m, p.e0), 0.0f);
     return a * a * (1.0f - p.delta_lo) - p.eta;
   }
 }
@@ -75,13 +76,13 @@ __device__ __forceinline__ float unit_hi(const rescore_params& p, float v, float
   } else {
     const float vp = fmaxf(v, 0.0f);
     const float m  = 2.0f * fabsf(norm) + sqrt_approx(vp);
-    const float b  = sqrt_approx(vp + p.kappa * m * m) + __fmaf_rn(p.e1, m, p.e0);
+    const float b  = sqrt_approx(vp + __fmaf_rn(p.kappa * m, m, p.e2)) + __fmaf_rn(p.e1, m, p.e0);
     hi             = b * b * (1.0f + p.delta_hi) + p.eta;
     return norm < 0.0f || !(hi < p.sum_limit) ? INFINITY : hi;
   }
 }
 // A value that every v with lo(v) <= bound stays below (L2: with x = sqrt(v) and A the distance that the bound allows,
-// x <= A + e0 + (e1 + sqrt(kappa)) (2 |d| + x), so 1.05 (A + e0) + 0.05 |d| exceeds x; one step from there).
+// x <= A + e0 + sqrt(e2) + (e1 + sqrt(kappa)) (2 |d| + x), so 1.05 (A + e0 + sqrt(e2)) + 0.05 |d| exceeds x; one step from there).
 template <bool kIP>
 __device__ __forceinline__ float value_limit(const rescore_params& p, float bound, float norm, float qn)
 {
@@ -92,9 +93,9 @@ __device__ __forceinline__ float value_limit(const rescore_params& p, float boun
   } else {
     const float dn = fabsf(norm);
     const float A  = sqrt_approx((fmaxf(bound, 0.0f) + p.eta) / (1.0f - p.delta_lo)) * 1.00001f;
-    const float m  = 2.0f * dn + 1.05f * (A + p.e0) + 0.05f * dn;
+    const float m  = 2.0f * dn + 1.05f * (A + p.e0 + sqrt_approx(p.e2)) + 0.05f * dn;
     const float x  = A + __fmaf_rn(p.e1, m, p.e0);
-    return (x * x + p.kappa * m * m) * 1.00001f;
+    return (x * x + __fmaf_rn(p.kappa * m, m, p.e2)) * 1.00001f;
   }
 }
 

@@ -798,6 +798,7 @@ static void set_error_model(rescore_params& rp, const operand_params& fp, int lu
   rp.kappa = float((K + 32.0) * std::ldexp(1.0, -22) * 1.1);
   rp.e1    = float(half * 1.03);
   rp.e0    = float(2.0 * std::sqrt(K) * tiny / double(fp.scale));
+  rp.e2    = float(2.0 * tiny * 1.2 / (double(fp.scale) * double(fp.scale)));  // (|r|^2: two halves of a row, each as two halfs)
   // table entries: their fp32 chain, then one rounding to the table type
   double up   = (double(fp.pq_len) + 4.0) * ulp, down = up;
   double zero = 0.0;  // absolute error of an entry near zero

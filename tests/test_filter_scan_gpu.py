@@ -274,3 +274,30 @@ def test_with_and_without_row_codes(ivf, metric, lut, internal, dim, pq_dim, bit
         L.check(L.load().cuvsB200SetScanCodebookHome(2))
         d0, i0 = gpu_search(ivf, g, q, k, 20, lut, internal)
         assert (i0 == i2).all() and (d0.view(np.uint32) == d2.view(np.uint32)).all()
+
+
+# rows and queries whose distances are many orders below the longest codeword, which sets the scale of the half-precision operands:
+# |r|^2 of the near rows underflows there.  Against the tables bit for bit
+@pytest.mark.parametrize("lut,internal", [("f32", "f32"), ("f16", "f32"), ("fp8", "f32"), ("f16", "f16")])
+@pytest.mark.parametrize("pq_dim,length,bits", [(16, 1, 8), (16, 2, 8), (24, 4, 8), (32, 2, 4), (16, 8, 8)])
+@pytest.mark.parametrize("longest,near", [(3.0, 1.0), (300.0, 0.05), (30_000.0, 0.05), (300.0, 1e-3)])
+def test_distances_far_below_the_longest_codeword(ivf, lut, internal, pq_dim, length, bits, longest, near):
+    from cuvs_b200 import _lib as L
+    rng = np.random.default_rng(pq_dim + length)
+    dim, n_lists, n, book = pq_dim * length, 20, 6000, 1 << bits
+    books = near * rng.standard_normal((pq_dim, length, book))
+    books[:, :, book - 2:] *= longest / near
+    centers = rng.standard_normal((n_lists, dim))
+    to = lambda a: torch.from_numpy(np.ascontiguousarray(a, dtype=np.float32)).cuda()  # noqa: E731
+    g = ivf.build_precomputed(ivf.IndexParams(n_lists=n_lists, pq_dim=pq_dim, pq_bits=bits), dim, to(books), to(centers), to(centers),
+                              to(np.eye(dim)))
+    rows = centers[rng.integers(0, n_lists, n)] + near * rng.standard_normal((n, dim))
+    rows[::50] += longest * rng.standard_normal((len(rows[::50]), dim))
+    ivf.extend(g, to(rows), torch.arange(n, device="cuda"))
+    q = (rows[rng.integers(0, n, 300)] + 0.01 * near * rng.standard_normal((300, dim))).astype(np.float32)
+    for k in (1, 10, 40):
+        L.check(L.load().cuvsB200SetScanCodebookHome(4))
+        d2, i2 = gpu_search(ivf, g, q, k, 4, lut, internal)
+        L.check(L.load().cuvsB200SetScanCodebookHome(2))
+        d0, i0 = gpu_search(ivf, g, q, k, 4, lut, internal)
+        assert (i0 == i2).all() and (d0.view(np.uint32) == d2.view(np.uint32)).all()
